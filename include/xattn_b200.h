@@ -221,7 +221,7 @@ int xattn_b200_mask_to_lists(const uint8_t* mask, int batch, int heads, int mask
  * out[b,h,i,:] = softmax_j(scale * q_i.k_j) v_j over keys j in kept blocks, and j <= i + (k_len-q_len)
  * when causal.  head_dim must be 128.  Rows with no visible key give zeros.
  * out has element strides (o_stride_b, o_stride_h, o_stride_l), unit stride along head_dim, same
- * dtype as the inputs.
+ * dtype as the inputs.  block_idx and block_cnt NULL: a dense call, every block that holds a visible key is listed.
  */
 int xattn_b200_block_sparse_attn(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv,
                                  int q_len, int k_len, int head_dim, int64_t q_stride_b, int64_t q_stride_h,
@@ -231,22 +231,17 @@ int xattn_b200_block_sparse_attn(const void* q, const void* k, const void* v, in
                                  int64_t o_stride_h, int64_t o_stride_l, int* status, void* cuda_stream);
 
 /*
- * The same operation with scratch memory, which lets the library treat the lists that long-context prefill
- * produces most -- one or two blocks (attention sink + diagonal), identical for all query heads of a kv head --
- * in a kernel of their own: K/V tiles loaded once per kv head and query block and shared by its query heads
- * (GQA head sharing), both Q.K^T products and both P.V products issued back to back, one softmax pass without
- * online rescaling.  Which rows qualify is decided on the device (no synchronisation); all other rows run through
- * the general kernel of xattn_b200_block_sparse_attn.  Because two kernels in a row cost a second tail, the split is
- * also only made, again decided on the device, when the qualifying rows list at least 92 % of the call's blocks
- * (Llama-3.1-8B at 128K tokens: 95 %, 8 % faster; at 64K: 89 %, no gain; at 32K: 66 %, a loss); below that the
- * general kernel computes everything and the attempt has cost 30-45 microseconds (so callers with short sequences
- * should use xattn_b200_block_sparse_attn; the Python layer offers the workspace from 96K tokens on).
- * xattn_b200_block_sparse_attn_split_share(percent) replaces the 92 for the calls enqueued after it (0: split
+ * The same operation with scratch memory.  Causal calls: rows whose kv group shares a list of one or two blocks (attention
+ * sink + diagonal) run in a kernel of their own, with K/V tiles loaded once per kv head and query block for all its query
+ * heads and one softmax pass over both blocks.  Which rows qualify is decided on the device (no synchronisation); all
+ * other rows run through the general kernel of xattn_b200_block_sparse_attn.  The split is only made, again decided on the
+ * device, when the qualifying rows list at least 92 % of the call's blocks; below that the general kernel computes
+ * everything.  xattn_b200_block_sparse_attn_split_share(percent) replaces the 92 for the calls enqueued after it (0: split
  * whenever anything qualifies, 101: never) and returns the previous value; a negative argument only reads it.
  * Same call-site contract (xattn/src/Xattention.py:377-391), same results up to the summation order.
- * A non-causal call uses the scratch memory differently: its work items (batch, query head, query block) are sorted
- * by list length, longest first, by one small kernel, and dealt to the SMs in that order; masks whose rows differ
- * widely in length (video diffusion: 5 to 891 blocks per row) otherwise leave the most loaded SM 16 % above the mean.
+ * A non-causal call uses the scratch memory differently: its work is ordered by list length (very long lists first, then
+ * kv head by kv head, longest first) by one small kernel before it is handed to the SMs; masks whose rows differ widely in
+ * length (video diffusion: 5 to 891 blocks per row) would otherwise leave single SMs at work at the end.
  * workspace: device memory of xattn_b200_block_sparse_attn_workspace_bytes() bytes, 16-byte aligned, contents
  * irrelevant on entry; the call's kernels use it until they finish.  With workspace == NULL the call equals
  * xattn_b200_block_sparse_attn.

@@ -1,0 +1,78 @@
+"""The attention kernel at the sizes where their tiling can go wrong, against plain fp32 attention."""
+import pytest
+import torch
+
+from oracle import xattn_oracle as orc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+# Probabilities and outputs are rounded to the 16-bit type, 2^-9 relative each for bf16 (2^-12 for fp16): an output, an
+# average of values of at most about 5, is off by at most 2 * 2^-9 * 5 = 2e-2; on average by a tenth of that.
+MAX_ABS, MEAN_ABS = 2e-2, 2e-3
+
+
+@pytest.fixture(autouse=True)
+def _status_clean():
+    import xattn_b200
+    yield
+    xattn_b200.check_device_status()
+
+
+def _close(got, want, scale=1.0):
+    err = (got.float().cpu() - want).abs()
+    assert torch.isfinite(got.float()).all()
+    assert err.max() < MAX_ABS * scale and err.mean() < MEAN_ABS * scale, (float(err.max()), float(err.mean()))
+
+
+def _qkv(seed, b, hq, hkv, lq, lk, dtype=torch.bfloat16):
+    g = torch.Generator().manual_seed(seed)
+    return [torch.randn(b, h, n, 128, generator=g).to(dtype) for h, n in ((hq, lq), (hkv, lk), (hkv, lk))]
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("batch,hq,hkv,lq,lk", [(1, 7, 1, 640, 640), (1, 3, 3, 300, 300), (2, 4, 2, 129, 1000), (1, 1, 1, 5, 5),
+                                                (1, 2, 2, 127, 4200), (1, 5, 1, 1, 257)])
+def test_dense_call_without_lists(causal, batch, hq, hkv, lq, lk):
+    """Odd groups, odd numbers of query blocks, a query offset that is no multiple of the block, lists of more than 32
+    blocks: every form of a work unit (two heads, two query blocks, one tile)."""
+    from xattn_b200 import ops
+    q, k, v = _qkv(lq + lk, batch, hq, hkv, lq, lk)
+    out = ops.block_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), None, None, causal)
+    rep = hq // hkv
+    keep = torch.ones(lq, lk, dtype=torch.bool).tril(lk - lq) if causal else None
+    want = torch.nn.functional.scaled_dot_product_attention(q.float(), k.float().repeat_interleave(rep, 1),
+                                                            v.float().repeat_interleave(rep, 1), attn_mask=keep)
+    _close(out, want)
+
+
+@pytest.mark.parametrize("causal,ordered", [(True, False), (False, False), (False, True)])
+@pytest.mark.parametrize("hq,hkv,L", [(6, 2, 128 * 81), (3, 3, 128 * 160 - 1), (7, 1, 128 * 61)])
+def test_more_units_than_sms(causal, ordered, hq, hkv, L):
+    """CTAs take over further units: lists of 0 to 40 blocks that differ between the two tiles of a unit, runs of rows that
+    list nothing, one row that lists everything."""
+    from xattn_b200 import ops
+    q, k, v = _qkv(L + hq, 1, hq, hkv, L, L)
+    nb = (L + 127) // 128
+    g = torch.Generator().manual_seed(L)
+    want_n = (torch.rand(1, hq, nb, 1, generator=g) ** 3 * 40).long()
+    mask = torch.rand(1, hq, nb, nb, generator=g).argsort(-1).argsort(-1) < want_n
+    mask[:, :, nb // 3:nb // 3 + 12] = False
+    mask[0, hq - 1, nb - 2] = True
+    if causal:
+        mask &= torch.tril(torch.ones(nb, nb, dtype=torch.bool))
+    idx, cnt = ops.mask_to_lists(mask.to(DEV), L, L, causal)
+    out = torch.full((1, hq, L, 128), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.block_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), idx, cnt, causal, out=out, use_workspace=ordered)
+    assert torch.isfinite(out.float()).all()
+    rows = sorted({0, 1, 2, nb // 3, nb // 3 + 11, nb // 2, nb - 3, nb - 2, nb - 1})
+    rep = hq // hkv
+    for r in rows:
+        r0, r1 = r * 128, min(L, (r + 1) * 128)
+        keep = mask[:, :, r].repeat_interleave(128, -1)[:, :, None, :L].expand(-1, -1, r1 - r0, -1)
+        if causal:
+            keep = keep & (torch.arange(L)[None, :] <= torch.arange(r0, r1)[:, None])
+        s = torch.einsum("bhqd,bhkd->bhqk", q[:, :, r0:r1].float(), k.float().repeat_interleave(rep, 1)) / 128 ** 0.5
+        p = torch.where(keep.any(-1, keepdim=True), s.masked_fill(~keep, float("-inf")), torch.zeros(()))
+        p = torch.where(keep, torch.softmax(p, -1), torch.zeros(()))
+        want = p @ v.float().repeat_interleave(rep, 1)
+        _close(out[:, :, r0:r1], want)

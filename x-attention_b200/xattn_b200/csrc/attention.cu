@@ -1,36 +1,45 @@
 // Phase 3 of the XAttention prefill path: block-sparse FlashAttention forward over 128x128 blocks.
 //
 // Replaces block_sparse_attn.block_sparse_attn_func (third-party CUDA package; call site
-// xattn/src/Xattention.py:377-391).  A work item is one (batch, head, 128-row query block) with its list
-// of kept key blocks.  Mask rows are short (often 2-10 blocks), so per-item latency chains
-// (Q load -> QK^T -> softmax -> PV -> store) matter as much as the inner loop.  The kernel is persistent
-// (one CTA per SM) and runs TWO independent item streams per CTA: the CTA's non-empty items alternate
-// between stream 0 and stream 1, each stream has its own Q / K / V tiles in shared memory, its own
-// score/probability buffer S and output accumulator O in tensor memory and its own softmax warpgroup,
-// so the bubbles of one stream's dependency chain are filled by the other stream's work.
+// xattn/src/Xattention.py:377-391).  A tile is one (batch, head, 128-row query block) with its list of kept key
+// blocks (or, for dense calls, the blocks 0 .. n-1 without a list in memory).  A unit of work is two tiles that read the
+// same kv head: two query heads of a kv group, or two neighbouring query blocks of one head.  The grid has a CTA per
+// unit, of which one per SM runs at a time and takes over further ones (cluster launch control).  Its two tiles are two
+// streams: each has its own Q tile in shared memory, its own score/probability buffer S and output accumulator O in
+// tensor memory and its own softmax warpgroup, so that one stream's softmax runs under the other's MMAs.  (Only the pass over
+// what the pair kernel leaves, whose length the host does not know, takes its units in strides of the grid instead.)
 //
-//   warps 0-3   softmax of stream 0  } one thread per query row.  A block is taken as two halves of 64 keys, each
-//   warps 4-7   softmax of stream 1  } an online-softmax step: the half's scores come out of TMEM once (two
-//                                      32-column loads in flight) and stay in registers for the row max (8
-//                                      independent chains) and the exp2; P packed to 16-bit goes back into S
-//                                      columns already read; lazy rescale of O only when the max grew by more
-//                                      than 2^8; the row sum of the item's last block goes to shared memory for
-//                                      the epilogue
-//   warps 8-11  epilogue of both streams: O / l from TMEM -> global memory, hands the O buffer back
-//   warps 12,14 TMA loader of stream 0 / 1 (lane 0 issues): Q, then K_j, V_j in list order, one TMA
-//               instruction per 128x128 tile
-//   warps 13,15 (1 thread each) tcgen05 issuer of stream 0 / 1: S = Q K^T (operands in shared memory), then
-//               O += P V (P from TMEM, V from shared memory as an MN-major operand)
+//   warps 0-3   softmax of stream 0  } one thread per query row.  A block's 128 scores leave TMEM once and stay in
+//   warps 4-7   softmax of stream 1  } registers for the row maximum (3-input max) and the exp2; P packed to 16-bit
+//                                      goes back into S columns, handed to the tensor pipe in two halves; lazy
+//                                      rescale of O only when the max grew by more than 2^8; the row sum of the
+//                                      tile's last block goes to shared memory for the epilogue
+//   warps 8-11  epilogue of both streams: O / l from TMEM, through shared memory, to TMA stores
+//   warp  12    loader of K and V: the union of the two lists passes once through a ring of two K and two V slots that
+//               both streams read; requests the units of work
+//   warp  13    tcgen05 issuer of both streams: S = Q K^T (operands in shared memory), then O += P V (P from TMEM, V
+//               from shared memory as an MN-major operand)
+//   warp  14    loader of Q
 //
-// Lists are walked from the last entry (the diagonal block when causal, which usually holds the row
-// maximum) to the first, so the running maximum settles at the first block and O is rarely rescaled.
-// The kernel is a template over how a stream walks a 128-key block (see kHalfModeMinBlocksX2): as one block
-// (K and V as 32 KiB tiles, one Q.K^T per block: the shortest chain per item, for short lists), or as two
-// 64-key halves (S of half h in its own 64-column TMEM buffer, so while the softmax warpgroup works on one half
-// the tensor pipe computes the other half's S and the previous half's P.V; K and V as four 16 KiB half-tiles
-// per block: for long lists).  Every CTA picks one of the two from its own list lengths.
-// TMEM columns: [0,128) S of stream 0 (two 64-column halves in half mode), [128,256) S of stream 1,
-// [256,384) O of stream 0, [384,512) O of stream 1.
+// What bounds it, and what follows from that (dense causal mask, 32 heads x 16384 tokens: 1110 -> 1372 TFLOP/s; 32768
+// tokens with 2.5 listed blocks per row: 254 -> 185 us):
+//   * A 128x128 block is 1024 cycles of MMA and 1024 cycles of ex2 (16 per cycle and SM), so the two streams have to be
+//     half a period apart.  One warp issues the MMAs of both in fixed alternation: a stream's batch then goes through
+//     the tensor pipe in one piece.  Two issuing warps' batches interleave, both streams' scores are complete at the
+//     same time, both exponentiate at half speed, and the tensor pipe idles.
+//   * tcgen05 takes its operands from uniform registers.  Issued from a single-thread branch an MMA cost 83 cycles, more
+//     than its 64 cycles of work; issued under a predicate in converged code, 10.
+//   * Shared memory (128 B per cycle) has to take the operand reads of Q.K^T (64 KiB a block), of P.V (32 KiB) and the TMA
+//     writes of K and V (64 KiB if every tile brings its own): 1280 cycles, against 1024 when two tiles share them; and
+//     L2 delivers half the bytes.
+//   * Short lists walk through all of the code every few microseconds.  At 74 KB of code the SMs that share an
+//     instruction cache took up to 1.6 times as long as the ones that do not (128K tokens: 980 us for the slowest,
+//     600 for the fastest; below 50 KB: 650 and 600).  Hence no division in the unit decoding, rolled loops in the
+//     epilogue and for masked blocks, TMA stores, one instantiation per data type.
+//
+// Lists are walked from the last entry (the diagonal block when causal, which usually holds the row maximum) to the
+// first, so the running maximum settles at the first block and O is rarely rescaled.
+// TMEM columns: [0,128) S of stream 0, [128,256) S of stream 1, [256,384) O of stream 0, [384,512) O of stream 1.
 #include <math.h>
 
 #include <atomic>
@@ -40,135 +49,176 @@
 namespace xb {
 
 constexpr int kAttnThreads = 512;
-constexpr int kHalfTile = 64 * 128 * 2;    // 64 keys x 128 columns: [2 column halves][64 rows][64 columns]
-constexpr int kAttnSmemTiles = kTile16 * 6;                   // Q, K, V per stream
-constexpr int kSchedCap = 2048;                               // work items one CTA can schedule
-constexpr int kStageBytes = 4 * 32 * 128;                     // per epilogue warp: 32 rows x 64 16-bit columns
-constexpr int kAttnSmem = kAttnSmemTiles + 2 * 2 * 128 * 4 /*row sums*/ + 512 /*barriers*/ +
-                          3 * kSchedCap * 2 /*schedule*/ + 16 + kStageBytes;
+constexpr int kAttnSmemTiles = kTile16 * 6;                   // Q0, Q1, then two slots of K, V
+constexpr int kStageBytes = 4 * 2 * 32 * 128;                 // per epilogue warp: 32 rows x 2 x 64 16-bit columns
+// A step of the K/V loader, published for the MMA issuer in a ring: which streams use the K/V pair, and whether it is the
+// first / the last block of their tile
+constexpr int kRingEntries = 8;
+constexpr int kStepUses = 1, kStepFirst = 4, kStepLast = 16, kStepEnd = 64;      // << stream, except the last
+// A unit, published by the K/V loader for the other roles: each stream's tile and its number of blocks
+struct UnitTile {
+  int b, h, qb, n;        // qb < 0: no tile; n < 0: no more units
+};
+constexpr int kUnitSlots = 4;
+constexpr int kUnitReaders = 13;                              // warps that read it
+constexpr int kAttnSmem = kAttnSmemTiles + kStageBytes + 2 * 2 * 128 * 4 /*row sums*/ + kRingEntries * 4 +
+                          kUnitSlots * 2 * 16 + 16 + 512 /*barriers*/;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
-// Register budget of a role.  The kernel is launched with 512 threads x 128 registers; setmaxnreg moves registers
-// between warpgroups inside that allocation (8 x softmax + 4 x epilogue + 4 x load/MMA warps = 2048 per lane).
-template <int N> __device__ __forceinline__ void reg_set() {
-  if constexpr (N > 128) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
-  if constexpr (N < 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
-}
-
-// Work item t -> (b, h, qb): heaviest query blocks (largest index) first, the heads of a kv group adjacent.
-// (Ordering the items kv group by kv group instead, so that all CTAs work on one kv head at a time, was measured:
-// +4 % on the 119K-token non-causal mask, -5 % to -15 % on causal masks, whose heavy rows then no longer all
-// come first.)
-struct Item {
-  int b, h, qb;
-  size_t row;
+struct Tile {
+  int b, h, qb;      // qb < 0: no tile
 };
-__device__ __forceinline__ Item decode_item(const AttnParams& p, int t) {
-  Item it;
-  if (p.item_list) t = __ldg(p.item_list + t);
-  it.h = t % p.hq;
-  const int rest = t / p.hq;
-  it.b = rest % p.batch;
-  it.qb = p.q_blocks - 1 - rest / p.batch;
-  it.row = (static_cast<size_t>(it.b) * p.hq + it.h) * p.q_blocks + it.qb;
-  return it;
+__device__ __forceinline__ size_t tile_row(const AttnParams& p, const Tile& t) {
+  return (static_cast<size_t>(t.b) * p.hq + t.h) * p.q_blocks + t.qb;
 }
-// Work slot of this CTA's i-th item and the number of its items.  Plain dealing: slot i * G + blockIdx.x.  With
-// `snake` (the item list is sorted by list length, longest first) odd rows of the deal run backwards, so that no
-// CTA gets the longest item of every row: the loads of the CTAs then differ by about one item of the first row.
-__device__ __forceinline__ int item_slot(const AttnParams& p, int i, int G) {
-  const int c = (p.snake && (i & 1)) ? G - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
-  return i * G + c;
+// The tiles of unit u.  With a tile list: its entries 2u and 2u+1 (-1: none), tile i being (b, h, qb) with qb from the last
+// to the first.  Otherwise a "super row" is two query blocks hi, hi-1; its hq units per batch entry are, for each kv head,
+// the pairs of query heads at hi, then those at hi-1, and for an odd group first one unit that takes the last head at hi
+// and hi-1.  Causal: super row by super row, the heaviest (last) first.  Non-causal: kv head by kv head, so that the CTAs
+// work on one head's K and V at a time.
+__device__ __forceinline__ void unit_tiles(const AttnParams& p, int u, Tile& t0, Tile& t1) {
+  if (p.tile_list) {
+    auto decode = [&](int i, Tile& t) {
+      t.b = t.h = 0;
+      t.qb = -1;
+      if (i < 0) return;
+      const int rest = fast_div(i, p.by_hq, t.h);
+      t.qb = p.q_blocks - 1 - fast_div(rest, p.by_batch, t.b);
+    };
+    int i0 = -1, i1 = -1;
+    if (2 * u < p.list_tiles) i0 = __ldg(p.tile_list + 2 * u);
+    if (2 * u + 1 < p.list_tiles) i1 = __ldg(p.tile_list + 2 * u + 1);
+    decode(i0, t0);
+    decode(i1, t1);
+  } else {
+    int x, j, g;
+    const int hi = fast_div(u, p.by_units, x), lo = fast_div(x, p.by_group, j);
+    const int r = p.causal ? hi : lo, bg = p.causal ? lo : hi;
+    t0.b = fast_div(bg, p.by_hkv, g);
+    const int group = static_cast<int>(p.by_group.d), odd = group & 1, pairs = group >> 1;
+    const int lower = j - odd >= pairs ? 1 : 0;
+    const int across = odd && j == 0 ? 1 : 0;
+    t0.qb = p.q_blocks - 1 - 2 * r - (across ? 0 : lower);
+    t0.h = g * group + (across ? group - 1 : 2 * (j - odd - lower * pairs));
+    t1.b = t0.b;
+    t1.qb = t0.qb - across;
+    t1.h = t0.h + 1 - across;
+  }
 }
-__device__ __forceinline__ int local_item_count(const AttnParams& p, int G) {
-  const int full = p.total_items / G, rem = p.total_items % G;
-  const int c = (p.snake && (full & 1)) ? G - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
-  return full + (c < rem ? 1 : 0);
+// number of listed blocks; a dense call lists every block that holds a key the tile's last row may see
+__device__ __forceinline__ int tile_count(const AttnParams& p, const int32_t* __restrict__ block_cnt, const Tile& t) {
+  if (t.qb < 0) return 0;
+  if (block_cnt) return __ldg(block_cnt + tile_row(p, t));
+  if (!p.causal) return p.list_k_blocks;
+  int last = t.qb * 128 + 127;
+  last = (last < p.q_len - 1 ? last : p.q_len - 1) + p.k_len - p.q_len;
+  const int n = last / 128 + 1;
+  return n < p.list_k_blocks ? n : p.list_k_blocks;
 }
-__device__ __forceinline__ int item_count(const AttnParams& p, const int32_t* __restrict__ cnt, int t) {
-  return t < p.total_items ? __ldg(cnt + decode_item(p, t).row) : 0;
+// A tile's list as its walkers see it: walk position j maps to list[n - 1 - j].
+struct List {
+  const int32_t* last;     // its last entry; null in a dense call
+  int n;
+};
+__device__ __forceinline__ List tile_list(const AttnParams& p, const int32_t* __restrict__ block_idx, const Tile& t, int n) {
+  List l;
+  l.last = block_idx ? block_idx + tile_row(p, t) * p.list_k_blocks + (n - 1) : nullptr;
+  l.n = n;
+  return l;
 }
-// lane's entry of the 32-wide window at walk position j0: walk position j maps to list[n-1-j]
-__device__ __forceinline__ int list_window(const AttnParams& p, const int32_t* __restrict__ block_idx, size_t row,
-                                           int n, int j0, int lane) {
-  const int e = n - 1 - (j0 + lane);
-  if (e < 0) return 0;
+// the lane's entry of the 32-wide window at walk position j0
+__device__ __forceinline__ int list_window(const List& l, int j0, int lane) {
+  const int j = j0 + lane;
+  if (j >= l.n) return 0;
+  if (!l.last) return l.n - 1 - j;
   // volatile asm pins the issue point: a plain read-only load would be sunk by the compiler to its first use,
   // which turns the intended prefetch into an exposed memory latency
   int v;
-  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(block_idx + row * p.list_k_blocks + e));
+  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(l.last - j));
   return v;
 }
 
-// Per-CTA schedule, built once in shared memory by the prologue: the block count of every item of this CTA
-// (item i is work item t = blockIdx.x + i * gridDim.x) and, per stream, the order of its items (the k-th
-// non-empty item of the CTA runs on stream k & 1).  Roles then walk their items without touching global memory.
-struct Sched {
-  const uint16_t* cnt;      // [n_local]
-  const uint16_t* seq[2];   // [n_seq[s]] CTA-local item indices of stream s
-  int n_local, n_seq[2];
+// Reader of the published units.
+struct Units {
+  const volatile UnitTile* ring;          // [slot][stream]
+  uint32_t full, empty;                   // shared-memory addresses of the slots' barriers
+  volatile int* abort_flag;
+  uint32_t k;
+  // whole warp: waits for the next unit; false after an abort
+  __device__ __forceinline__ bool wait() {
+    return __all_sync(0xffffffffu, mbar_wait(full + 8 * (k % kUnitSlots), (k / kUnitSlots) & 1, abort_flag));
+  }
+  __device__ __forceinline__ UnitTile tile(int s) const {
+    const int4 v = *reinterpret_cast<const int4*>(const_cast<const UnitTile*>(ring) + 2 * (k % kUnitSlots) + s);
+    UnitTile t;
+    t.b = v.x; t.h = v.y; t.qb = v.z; t.n = v.w;
+    return t;
+  }
+  __device__ __forceinline__ void release(int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty + 8 * (k % kUnitSlots));
+    ++k;
+  }
 };
 
-// kHalf selects how a stream walks a 128-key block: as two 64-key halves with their own S buffers (softmax of
-// one half overlaps the MMAs of the other: 62 % of the dense bf16 peak on long lists) or as one block (fewer
-// instructions and barriers: better when a row lists only a handful of blocks).  The kernel sums the CTA's
-// block counts while it builds the schedule and calls the body meant for its average list length, so the
-// choice needs no host synchronisation.
-// twice the average number of listed blocks per non-empty item from which the half-block body pays off
-// (random masks with n blocks per row, 16 heads x 16K, full / half body in TFLOP/s: n=3 583-596 / 532-542,
-// n=4 637-651 / 645-663, n=6 691-708 / 756-771, n=8 726-739 / 818-824; the 32K Llama mask with its masked diagonal
-// blocks, 2.5 blocks per row: 676 / 484)
-constexpr int kHalfModeMinBlocksX2 = 7;
-template <bool kHalf>
-__device__ __forceinline__ void attn_cta(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
-                                         const CUtensorMap& tmKf, const CUtensorMap& tmVf, const AttnParams& p,
-                                         const int32_t* __restrict__ block_idx, void* __restrict__ out, int* status) {
-  // Shared memory takes nearly the whole L1, so a register spilled to local memory costs an L2 round trip:
-  // the split below is the one with the fewest spills ptxas reports for this kernel (48 bytes, in cold paths).
-#ifdef XB_A_SM
-  constexpr int kRegSoftmax = XB_A_SM, kRegEpilogue = XB_A_EP, kRegLoadMma = XB_A_LM;
-#else
-  constexpr int kRegSoftmax = 152, kRegEpilogue = 112, kRegLoadMma = 96;
-#endif
+// kBf16: bf16 or fp16 (a template parameter: as a run-time switch every packed pair cost both conversions and a select).
+template <bool kBf16>
+__global__ void __launch_bounds__(kAttnThreads, 1)
+block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
+                         const AttnParams p_in,
+                         const int32_t* __restrict__ block_idx, const int32_t* __restrict__ block_cnt,
+                         const int32_t* __restrict__ rest_list, const int* __restrict__ pair_header,
+                         int pair_min_share, int* status) {
+  // The kernel is launched with 512 threads x 128 registers; setmaxnreg moves registers between warpgroups inside
+  // that allocation.  A softmax thread keeps a row's 128 scores in registers; shared memory takes nearly the whole
+  // L1, so a register spilled to local memory would cost an L2 round trip.
+  constexpr int kRegSoftmax = 192, kRegEpilogue = 64, kRegLoadMma = 64;
   static_assert(8 * kRegSoftmax + 4 * kRegEpilogue + 4 * kRegLoadMma <= 16 * 128, "register budget of the roles");
   extern __shared__ __align__(1024) uint8_t smem[];
-  // tiles: [stream][Q, K, V]
-  float* s_l = reinterpret_cast<float*>(smem + kAttnSmemTiles);          // [stream][2][128] final row sums
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kAttnSmemTiles + 2 * 2 * 128 * 4);
-  // per stream s: NBAR barriers at bars[NBAR*s + ...].  H_* : the four half-tile slots of a block
-  // (0: keys 0-63 of K, 1: keys 64-127 of K, 2: keys 0-63 of V, 3: keys 64-127 of V); S_FULL/P_READY: per half
-  enum { Q_FULL = 0, Q_EMPTY, H_FULL, H_EMPTY = H_FULL + 4, S_FULL = H_EMPTY + 4, P_READY = S_FULL + 2,
-         O_FULL = P_READY + 2, O_EMPTY, PV_DONE, NBAR };
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);     // (uniform for the compiler too)
+  const int lane = threadIdx.x & 31;
+  if ((smem_u32(smem) & 1023u) != 0) {              // the swizzled tiles need 1024-byte alignment
+    if (threadIdx.x == 0 && status) atomicExch(status, static_cast<int>(kDevBadSmemAlign));
+    return;
+  }
+  uint8_t* stage_base = smem + kAttnSmemTiles;
+  float* s_l = reinterpret_cast<float*>(stage_base + kStageBytes);                 // [stream][2][128] final row sums
+  volatile int* ring = reinterpret_cast<volatile int*>(s_l + 2 * 2 * 128);         // [step]
+  UnitTile* unit_ring = reinterpret_cast<UnitTile*>(s_l + 2 * 2 * 128 + kRingEntries);         // [slot][stream]
+  uint8_t* answer = reinterpret_cast<uint8_t*>(unit_ring + 2 * kUnitSlots);                    // of the request for a unit
+  uint64_t* bars = reinterpret_cast<uint64_t*>(answer + 16);
+  // per slot: K_*, V_*; per stream: the others; then UNIT_FULL, UNIT_EMPTY per unit slot, and the answer's
+  enum { K_FULL = 0, K_EMPTY, V_FULL, V_EMPTY, Q_FULL, Q_EMPTY, S_FULL, P_READY, O_FULL = P_READY + 2, O_EMPTY, NBAR };
   const uint32_t bar0 = smem_u32(bars);
   auto bar = [&](int s, int which) -> uint32_t { return bar0 + 8u * (NBAR * s + which); };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NBAR);
+  const uint32_t unit_full = bar0 + 8u * (2 * NBAR), unit_empty = unit_full + 8u * kUnitSlots,
+                 answer_full = unit_empty + 8u * kUnitSlots;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NBAR + 2 * kUnitSlots + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
 #ifdef XB_TRACE
   uint32_t trace_n = 0;
   const int trace_role = warp < 8 ? ((warp & 3) == 0 ? 2 + (warp >> 2) : 7 + 3 * (warp >> 2) + (warp & 3) - 1)
                                   : (warp < 12 ? 4 : (warp == 12 ? 0 : (warp == 13 ? 1 : (warp == 14 ? 5 : 6))));
 #endif
-
-  // schedule table, built by the kernel before it picked this instantiation
-  uint16_t* sch_cnt = reinterpret_cast<uint16_t*>(smem + kAttnSmemTiles + 2 * 2 * 128 * 4 + 512);
-  uint16_t* sch_seq0 = sch_cnt + kSchedCap;
-  uint16_t* sch_seq1 = sch_seq0 + kSchedCap;
-  int* sch_total = reinterpret_cast<int*>(sch_seq1 + kSchedCap);
-  uint8_t* stage_base = reinterpret_cast<uint8_t*>(sch_total) + 16;     // 16-byte aligned (sch_total: 2 ints)
-  const int G = gridDim.x;
-  const int n_local = local_item_count(p, G);                       // host guarantees <= kSchedCap
   if (threadIdx.x == 0) {
+#pragma unroll 1
     for (int s = 0; s < 2; ++s)
+#pragma unroll 1
       for (int w = 0; w < NBAR; ++w)
         mbar_init(bar(s, w), (w == P_READY || w == P_READY + 1 || w == O_EMPTY) ? 128 : 1);
+#pragma unroll 1
+    for (int w = 0; w < kUnitSlots; ++w) {
+      mbar_init(unit_full + 8u * w, 1);
+      mbar_init(unit_empty + 8u * w, kUnitReaders);
+    }
+    mbar_init(answer_full, 1);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
+    tma_prefetch_desc(&tmO);
   }
   if (warp == 13) {
     tmem_alloc(smem_u32(tmem_slot), 512);
@@ -177,361 +227,286 @@ __device__ __forceinline__ void attn_cta(const CUtensorMap& tmQ, const CUtensorM
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  Sched sch;
-  sch.cnt = sch_cnt;
-  sch.seq[0] = sch_seq0;
-  sch.seq[1] = sch_seq1;
-  sch.n_local = n_local;
-  sch.n_seq[0] = (*sch_total + 1) >> 1;
-  sch.n_seq[1] = *sch_total >> 1;
   const uint32_t tmem_base = *tmem_slot;
-  const int group = p.hq / p.hkv;
+  // The kernel may have been launched while the one before it in the stream was still running: up to here it has
+  // touched nothing that one writes.  With a pair kernel in front: the items it left (a list) if it ran, all items if
+  // it declined.
+  pdl_wait();
+  AttnParams p = p_in;
+  if (rest_list && pair_path_chosen(pair_header, pair_min_share)) {
+    p.tile_list = rest_list;
+    p.list_tiles = *reinterpret_cast<const volatile int*>(pair_header + kPairRestCount);
+  }
+  // (units of the pass over a pair kernel's leavings, or of the whole call if it declined)
+  const int rest_units = p.tile_list ? (p.list_tiles + 1) / 2 : (p.q_blocks + 1) / 2 * p.batch * p.hq;
+  Units units;
+  units.ring = unit_ring;
+  units.full = unit_full;
+  units.empty = unit_empty;
+  units.abort_flag = abort_flag;
+  units.k = 0;
 
   if (warp >= 12) {
-    reg_set<kRegLoadMma>();
-    const int s = (warp - 12) >> 1;                   // stream of this warp
-    uint8_t* tiles = smem + s * 3 * kTile16;          // Q, K, V tiles of the stream
-    if ((warp & 1) == 0) {
-      // ---------------------------------------------------------------- TMA loader of stream s (lane 0 issues)
-      const int n_items = sch.n_seq[s];
-      uint32_t bc = 0;
+    reg_set_from<kRegLoadMma, 128>();
+    if (warp == 12) {
+      // ------------------------------------------------------------ K/V loader: the union of the two lists
+      uint32_t step = 0;
       int ok = 1;
-      // list window of the first item; the next item's window is fetched while the current one is loaded
-      Item it = decode_item(p, n_items > 0 ? item_slot(p, sch.seq[s][0], G) : 0);
-      int n = n_items > 0 ? sch.cnt[sch.seq[s][0]] : 0;
-      int win = n_items > 0 ? list_window(p, block_idx, it.row, n, 0, lane) : 0;
-      for (int m = 0; m < n_items && ok; ++m) {
-        Item nit = it;
-        int nn = 0, nwin = 0;
-        if (m + 1 < n_items) {
-          const int i2 = sch.seq[s][m + 1];
-          nit = decode_item(p, item_slot(p, i2, G));
-          nn = sch.cnt[i2];
-          nwin = list_window(p, block_idx, nit.row, nn, 0, lane);
+      Tile t, tn;                                       // (tile of stream 0: both read the same kv head)
+      List l0, l1, l0n, l1n;
+      int w0n, w1n, unit = blockIdx.x;
+      // unit u, the CTA's k-th: published, its lists on their way
+      auto fetch = [&](int u, uint32_t k) {
+        l0n.n = l1n.n = -1;
+        Tile t1;
+        if (u >= 0) {
+          unit_tiles(p, u, tn, t1);
+          l0n = tile_list(p, block_idx, tn, tile_count(p, block_cnt, tn));
+          l1n = tile_list(p, block_idx, t1, tile_count(p, block_cnt, t1));
+          w0n = list_window(l0n, 0, lane);
+          w1n = list_window(l1n, 0, lane);
         }
-        const int hkv = it.h / group;
         if (lane == 0) {
-          if (mbar_wait(bar(s, Q_EMPTY), (m & 1) ^ 1, abort_flag)) {
-            XB_TRACE_EV(0x10, m);
-            mbar_expect_tx(bar(s, Q_FULL), kTile16);
-            tma_load_5d(smem_u32(tiles), &tmQ, bar(s, Q_FULL), 0, it.qb * 128, 0, it.h, it.b);
-            // the stream has one Q buffer, so the next item's Q can only be loaded when this item's last S is
-            // done: pull it into L2 now so that load does not wait on HBM
-            if (m + 1 < n_items) tma_prefetch_l2_5d(&tmQ, 0, nit.qb * 128, 0, nit.h, nit.b);
+          if (mbar_wait(unit_empty + 8 * (k % kUnitSlots), (k / kUnitSlots & 1) ^ 1, abort_flag)) {
+            int4* out = reinterpret_cast<int4*>(unit_ring + 2 * (k % kUnitSlots));
+            out[0] = make_int4(tn.b, tn.h, tn.qb, l0n.n);
+            out[1] = make_int4(t1.b, t1.h, t1.qb, l1n.n);
+            mbar_arrive(unit_full + 8 * (k % kUnitSlots));
           } else {
             ok = 0;
           }
         }
-        int w = win, w_next = list_window(p, block_idx, it.row, n, 32, lane);
-        for (int j = 0; j < n; ++j, ++bc) {
-          if (j > 0 && (j & 31) == 0) {
-            w = w_next;
-            w_next = list_window(p, block_idx, it.row, n, j + 32, lane);
-          }
-          const int k0 = __shfl_sync(0xffffffffu, w, j & 31) * 128;
-          if constexpr (kHalf) {
-          if (lane == 0 && ok) {
-#pragma unroll
-            for (int slot = 0; slot < 4; ++slot) {
-              if (!mbar_wait(bar(s, H_EMPTY + slot), (bc & 1) ^ 1, abort_flag)) { ok = 0; break; }
-              XB_TRACE_EV(0x12 + (slot >> 1), bc * 2 + (slot & 1));
-              mbar_expect_tx(bar(s, H_FULL + slot), kHalfTile);
-              tma_load_5d(smem_u32(tiles + kTile16 + slot * kHalfTile), slot < 2 ? &tmK : &tmV, bar(s, H_FULL + slot), 0,
-                          k0 + (slot & 1) * 64, 0, hkv, it.b);
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+      };
+      // the first turn of the loop has no lists to load, it only fetches those of the CTA's own unit; turn k works on the
+      // CTA's unit k - 1 and requests and fetches unit k
+      l0n.n = l1n.n = 0;
+      l0n.last = l1n.last = nullptr;
+      w0n = w1n = 0;
+      tn.b = tn.h = 0;
+#pragma unroll 1
+      for (uint32_t k = 0; unit >= 0 && ok; ++k) {
+        t = tn; l0 = l0n; l1 = l1n;
+        int w0 = w0n, w1 = w1n;
+        if (k > 0 && lane == 0 && !rest_list) {
+          mbar_expect_tx(answer_full, 16);
+          clc_try_cancel(smem_u32(answer), answer_full);
+        }
+        __syncwarp();
+        int g_;
+        const int kvh = fast_div(t.h, p.by_group, g_);
+        int i0 = 0, i1 = 0;
+        int w0x = list_window(l0, 32, lane), w1x = list_window(l1, 32, lane);
+        bool fetched = false;
+#pragma unroll 1
+        while (ok) {
+          if (i0 < l0.n || i1 < l1.n) {
+            const int c0 = i0 < l0.n ? __shfl_sync(0xffffffffu, w0, i0 & 31) : -1;
+            const int c1 = i1 < l1.n ? __shfl_sync(0xffffffffu, w1, i1 & 31) : -1;
+            const int blk = c0 > c1 ? c0 : c1;
+            const bool f0 = i0 < l0.n && c0 == blk, f1 = i1 < l1.n && c1 == blk;
+            if (lane == 0) {
+              const int sl = step & 1;
+              const uint32_t ph = ((step >> 1) & 1) ^ 1;
+              const uint32_t dst = smem_u32(smem + (2 + 2 * sl) * kTile16);
+              if (mbar_wait(bar(sl, K_EMPTY), ph, abort_flag)) {
+                XB_TRACE_EV(0x12, step);
+                ring[step & (kRingEntries - 1)] =
+                    (f0 ? kStepUses | (i0 == 0 ? kStepFirst : 0) | (i0 == l0.n - 1 ? kStepLast : 0) : 0) |
+                    (f1 ? kStepUses | (i1 == 0 ? kStepFirst : 0) | (i1 == l1.n - 1 ? kStepLast : 0) : 0) << 1;
+                mbar_expect_tx(bar(sl, K_FULL), kTile16);
+                tma_load_5d(dst, &tmK, bar(sl, K_FULL), 0, blk * 128, 0, kvh, t.b);
+              } else {
+                ok = 0;
+              }
+              if (ok && mbar_wait(bar(sl, V_EMPTY), ph, abort_flag)) {
+                XB_TRACE_EV(0x13, step);
+                mbar_expect_tx(bar(sl, V_FULL), kTile16);
+                tma_load_5d(dst + kTile16, &tmV, bar(sl, V_FULL), 0, blk * 128, 0, kvh, t.b);
+              } else {
+                ok = 0;
+              }
             }
-          }
-          } else {
-          if (lane == 0 && ok) {
-            if (mbar_wait(bar(s, H_EMPTY), (bc & 1) ^ 1, abort_flag)) {
-              XB_TRACE_EV(0x12, bc);
-              mbar_expect_tx(bar(s, H_FULL), kTile16);
-              tma_load_5d(smem_u32(tiles + kTile16), &tmKf, bar(s, H_FULL), 0, k0, 0, hkv, it.b);
-            } else {
-              ok = 0;
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (f0 && (++i0 & 31) == 0) {
+              w0 = w0x;
+              w0x = list_window(l0, i0 + 32, lane);
             }
-            if (ok && mbar_wait(bar(s, H_EMPTY + 2), (bc & 1) ^ 1, abort_flag)) {
-              XB_TRACE_EV(0x13, bc);
-              mbar_expect_tx(bar(s, H_FULL + 2), kTile16);
-              tma_load_5d(smem_u32(tiles + 2 * kTile16), &tmVf, bar(s, H_FULL + 2), 0, k0, 0, hkv, it.b);
-            } else {
-              ok = 0;
+            if (f1 && (++i1 & 31) == 0) {
+              w1 = w1x;
+              w1x = list_window(l1, i1 + 32, lane);
             }
+            ++step;
+          } else if (fetched) {
+            break;
           }
+          if (!fetched) {
+            // the next unit's lists, on their way while this unit's blocks are loaded
+            fetched = true;
+            if (rest_list) {
+              if (k > 0) unit += gridDim.x;
+              if (unit >= rest_units) unit = -1;
+            } else if (k > 0) {
+              if (!__all_sync(0xffffffffu, mbar_wait(answer_full, (k - 1) & 1, abort_flag))) { ok = 0; break; }
+              unit = clc_answer(smem_u32(answer));
+              fence_proxy_async_smem();                 // read before the next answer is written
+              __syncwarp();
+            }
+            fetch(unit, k);
           }
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        it = nit; n = nn; win = nwin;
       }
-    } else if (lane == 0) {
-      // ---------------------------------------------------------------- MMA issuer of stream s
-      const uint32_t idesc_pv = make_idesc_f16(128, 128, p.is_bf16 != 0, false, true);
-      if constexpr (kHalf) {
-      const uint32_t qa = smem_u32(tiles), ha = smem_u32(tiles + kTile16);      // Q tile, four half-tile slots
-      const uint32_t sd = tmem_base + s * 128;          // S / P, half h at +64*h
-      const uint32_t od = tmem_base + 256 + s * 128;    // O
-      // operand descriptors never change: build them once.  Q: [2][128 rows][64]; K half: [2][64 keys][64];
-      // V half: [2][64 keys][64], MN-major (16 keys per step = 16 x 128 B rows, next 64 columns 8 KiB away)
-      uint64_t dq[8], dk[2][8], dv[2][4];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        dq[k] = smem_desc_sw128(qa + (k >> 2) * kHalf16 + (k & 3) * 32, 16, 1024);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          dk[h][k] = smem_desc_sw128(ha + h * kHalfTile + (k >> 2) * (kHalfTile / 2) + (k & 3) * 32, 16, 1024);
+      // the end marker: a step that no stream uses
+      if (lane == 0 && ok && mbar_wait(bar(step & 1, K_EMPTY), ((step >> 1) & 1) ^ 1, abort_flag)) {
+        ring[step & (kRingEntries - 1)] = kStepEnd;
+        mbar_arrive(bar(step & 1, K_FULL));
       }
+    } else if (warp == 14) {
+      // ------------------------------------------------------------ Q loader of both streams
+      uint32_t m = 0;                                   // parity of the tiles so far, bit s: stream s
+      bool ok = true;
+#pragma unroll 1
+      while (ok && units.wait()) {
+        const UnitTile t0 = units.tile(0), t1 = units.tile(1);
+        units.release(lane);
+        if (t0.n < 0) break;
+        // a stream has one Q buffer, so a tile's Q can only be loaded when the last S of the stream's tile before it is
+        // done: both tiles of the unit are first pulled into L2, so that the loads do not wait on HBM
+        if (lane == 0) {
+          if (t0.n > 0) tma_prefetch_l2_5d(&tmQ, 0, t0.qb * 128, 0, t0.h, t0.b);
+          if (t1.n > 0) tma_prefetch_l2_5d(&tmQ, 0, t1.qb * 128, 0, t1.h, t1.b);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int s = 0; s < 2; ++s) {
+          const UnitTile t = s ? t1 : t0;
+          if (t.n == 0) continue;
+          if (!__all_sync(0xffffffffu, mbar_wait(bar(s, Q_EMPTY), (m >> s & 1) ^ 1, abort_flag))) { ok = false; break; }
+          if (lane == 0) {
+            XB_TRACE_EV(0x10 + s, m);
+            mbar_expect_tx(bar(s, Q_FULL), kTile16);
+            tma_load_5d(smem_u32(smem + s * kTile16), &tmQ, bar(s, Q_FULL), 0, t.qb * 128, 0, t.h, t.b);
+          }
+          __syncwarp();
+          m ^= 1u << s;
+        }
+      }
+    } else if (warp == 13) {
+      // ---------------------------------------------------------------- MMA issuer (converged warp, one thread issues: see
+      // mma_ss_lead)
+      constexpr uint32_t idesc_qk = make_idesc_f16(128, 128, kBf16, false, false);
+      constexpr uint32_t idesc_pv = make_idesc_f16(128, 128, kBf16, false, true);
+      const uint32_t lead = elect_one() ? 1u : 0u;
+      // K-major operands, k-step k: 16 columns = 32 B inside the 64-column half (k & 3), the second half 16 KiB on;
+      // V as MN-major operand: 16 keys per step = 16 x 128 B rows, the second 64 columns 16 KiB on
+      const uint64_t dq0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
+      const uint64_t dk0 = smem_desc_sw128(smem_u32(smem + 2 * kTile16), 16, 1024);
+      const uint64_t dv0 = smem_desc_sw128(smem_u32(smem + 3 * kTile16), kHalf16, 1024);
+      auto wait = [&](uint32_t b, uint32_t ph) -> bool { return __all_sync(0xffffffffu, mbar_wait(b, ph, abort_flag)); };
+      // S of stream s = Q K^T with the K tile of slot sl
+      auto issue_qk = [&](int s, int sl) {
+        const uint64_t dq = dq0 + static_cast<uint64_t>(s * (kTile16 >> 4));
+        const uint64_t dk = dk0 + static_cast<uint64_t>(sl * ((2 * kTile16) >> 4));
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+        for (int k = 0; k < 8; ++k) {
+          const uint32_t o = ((k >> 2) * kHalf16 + (k & 3) * 32) >> 4;
+          mma_ss_lead(tmem_base + s * 128, dq + o, dk + o, idesc_qk, k > 0 ? 1u : 0u, lead);
+        }
+      };
+      // O of stream s (+)= P V over keys 64 h .. 64 h + 63 of the V tile of slot sl
+      auto issue_pv = [&](int s, int sl, int h, uint32_t accumulate) {
+        const uint64_t dv = dv0 + static_cast<uint64_t>(sl * ((2 * kTile16) >> 4));
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          dv[h][k] = smem_desc_sw128(ha + (2 + h) * kHalfTile + k * 2048, kHalfTile / 2, 1024);
-      const uint32_t idesc_qk64 = make_idesc_f16(128, 64, p.is_bf16 != 0, false, false);
-      const int n_items = sch.n_seq[s];
-      bool ok = true;
-      // S of half h of block (m, j): needs Q (first block of an item) and K half h
-      auto issue_qk = [&](int m, int n, int j, uint32_t bc, int h) -> bool {
-        if (j == 0 && h == 0 && !mbar_wait(bar(s, Q_FULL), m & 1, abort_flag)) return false;
-        if (!mbar_wait(bar(s, H_FULL + h), bc & 1, abort_flag)) return false;
-        tc_fence_after();
-        XB_TRACE_EV(0x20 + h, bc);
-        mma_ss(sd + h * 64, dq[0], dk[h][0], idesc_qk64, 0u);
-#pragma unroll
-        for (int k = 1; k < 8; ++k) mma_ss(sd + h * 64, dq[k], dk[h][k], idesc_qk64, 1u);
-        mma_commit(bar(s, H_EMPTY + h));
-        mma_commit(bar(s, S_FULL + h));
-        if (h == 1 && j == n - 1) mma_commit(bar(s, Q_EMPTY));
-        return true;
+          mma_ts_lead(tmem_base + 256 + s * 128, tmem_base + s * 128 + (4 * h + k) * 8, dv + (((4 * h + k) * 2048) >> 4),
+                      idesc_pv, k > 0 ? 1u : accumulate, lead);
       };
-      // O += P V of half h: needs the softmax of that half and V half h
-      auto issue_pv = [&](int m, int n, int j, uint32_t bc, int h) -> bool {
-        if (j == 0 && h == 0 && !mbar_wait(bar(s, O_EMPTY), (m & 1) ^ 1, abort_flag)) return false;
-        if (!mbar_wait(bar(s, P_READY + h), bc & 1, abort_flag)) return false;
-        if (!mbar_wait(bar(s, H_FULL + 2 + h), bc & 1, abort_flag)) return false;
-        tc_fence_after();
-        XB_TRACE_EV(0x22 + h, bc);
-        mma_ts(od, sd + h * 64, dv[h][0], idesc_pv, (j > 0 || h > 0) ? 1u : 0u);
-#pragma unroll
-        for (int k = 1; k < 4; ++k) mma_ts(od, sd + h * 64 + k * 8, dv[h][k], idesc_pv, 1u);
-        mma_commit(bar(s, H_EMPTY + 2 + h));
-        mma_commit(bar(s, PV_DONE));
-        if (h == 1 && j == n - 1) mma_commit(bar(s, O_FULL));
-        return true;
-      };
-      // order inside the stream: ..., PV(b,0), QK(b+1,0), PV(b,1), QK(b+1,1), PV(b+1,0), ...
-      int m = 0, j = 0;
-      int n = n_items > 0 ? sch.cnt[sch.seq[s][0]] : 0;
-      uint32_t bc = 0;
-      if (n_items > 0) ok = issue_qk(m, n, j, bc, 0) && issue_qk(m, n, j, bc, 1);
-      while (ok && m < n_items) {
-        // the block after (m, j)
-        int m2 = m, j2 = j + 1, n2 = n;
-        if (j2 == n) { m2 = m + 1; j2 = 0; n2 = m2 < n_items ? sch.cnt[sch.seq[s][m2]] : 0; }
-        const bool has_next = m2 < n_items;
-        if (!issue_pv(m, n, j, bc, 0)) { ok = false; break; }
-        if (has_next && !issue_qk(m2, n2, j2, bc + 1, 0)) { ok = false; break; }
-        if (!issue_pv(m, n, j, bc, 1)) { ok = false; break; }
-        if (has_next && !issue_qk(m2, n2, j2, bc + 1, 1)) { ok = false; break; }
-        m = m2; j = j2; n = n2; ++bc;
-      }
-      } else {
-      const uint32_t idesc_qk = make_idesc_f16(128, 128, p.is_bf16 != 0, false, false);
-      const uint32_t qa = smem_u32(tiles), ka = smem_u32(tiles + kTile16), va = smem_u32(tiles + 2 * kTile16);
-      const uint32_t sd = tmem_base + s * 128;          // S / P
-      const uint32_t od = tmem_base + 256 + s * 128;    // O
-      // operand descriptors never change (one Q, K and V slot per stream): build them once
-      uint64_t dq[8], dk[8], dv[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t o = (k >> 2) * kHalf16 + (k & 3) * 32;
-        dq[k] = smem_desc_sw128(qa + o, 16, 1024);
-        dk[k] = smem_desc_sw128(ka + o, 16, 1024);
-        // 16 keys per step: V rows advance by 16 x 128 B (P columns by 8: two 16-bit values per column)
-        dv[k] = smem_desc_sw128(va + k * 2048, kHalf16, 1024);
-      }
-      const int n_items = sch.n_seq[s];
-      uint32_t bc = 0;
-      bool ok = true;
-      for (int m = 0; m < n_items && ok; ++m) {
-        const int n = sch.cnt[sch.seq[s][m]];
-        for (int j = 0; j < n && ok; ++j, ++bc) {
-          // S = Q K^T
-          if (j == 0 && !mbar_wait(bar(s, Q_FULL), m & 1, abort_flag)) { ok = false; break; }
-          if (!mbar_wait(bar(s, H_FULL), bc & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          XB_TRACE_EV(0x20, bc);
-          mma_ss(sd, dq[0], dk[0], idesc_qk, 0u);
-#pragma unroll
-          for (int k = 1; k < 8; ++k) mma_ss(sd, dq[k], dk[k], idesc_qk, 1u);
-          mma_commit(bar(s, H_EMPTY));
-          mma_commit(bar(s, S_FULL));
-          if (j == n - 1) mma_commit(bar(s, Q_EMPTY));
-          // O += P V, in two steps: keys 0-63 as soon as their half of P is written, so that this half of the
-          // product runs while the softmax warpgroup still exponentiates keys 64-127
-          if (!mbar_wait(bar(s, P_READY), bc & 1, abort_flag)) { ok = false; break; }
-          if (!mbar_wait(bar(s, H_FULL + 2), bc & 1, abort_flag)) { ok = false; break; }
-          if (j == 0 && !mbar_wait(bar(s, O_EMPTY), (m & 1) ^ 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          XB_TRACE_EV(0x22, bc);
-          mma_ts(od, sd, dv[0], idesc_pv, j > 0 ? 1u : 0u);
-#pragma unroll
-          for (int k = 1; k < 4; ++k) mma_ts(od, sd + k * 8, dv[k], idesc_pv, 1u);
-          mma_commit(bar(s, PV_DONE));                  // (a softmax warp that has to rescale O waits for this)
-          if (!mbar_wait(bar(s, P_READY + 1), bc & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-#pragma unroll
-          for (int k = 4; k < 8; ++k) mma_ts(od, sd + k * 8, dv[k], idesc_pv, 1u);
-          mma_commit(bar(s, PV_DONE));
-          mma_commit(bar(s, H_EMPTY + 2));
-          if (j == n - 1) mma_commit(bar(s, O_FULL));
+      // One bit per stream: pend, its block of step u - 1 has its P.V outstanding; todo, step u's K is outstanding; next, it
+      // has a block in step u.  In the fields of `st`: that block is the first / the last of its tile; parity of the
+      // stream's blocks and of its tiles.
+      constexpr int kFirst = 0, kLast = 2, kBlocks = 4, kTiles = 6;
+      uint32_t st = 0, u = 0, pend = 0, todo = 3, next = 0;
+      bool ok = true, have = false, v_used = false;     // have: the step's K is there and `e` is its entry
+      int e = 0;
+#pragma unroll 1
+      while (ok) {
+        const int sl = u & 1;
+        // Without K a stream's outstanding P.V is issued all the same: the block may be the last one for a while, and the
+        // next unit may even depend on it (its publication on the epilogue of this one).  So K is asked for before and
+        // after each stream's P.V, and waited for only when neither stream has one left.
+        auto look = [&](bool block) -> bool {
+          if (!have) {
+            have = block ? wait(bar(sl, K_FULL), (u >> 1) & 1)
+                         : __all_sync(0xffffffffu, mbar_test(bar(sl, K_FULL), (u >> 1) & 1));
+            if (have) e = __shfl_sync(0xffffffffu, ring[u & (kRingEntries - 1)], 0);
+          }
+          return have;
+        };
+        if (!look(pend == 0) && pend == 0) break;
+        // (first the stream that can start on this step at once, its last block being done, if the other cannot)
+        const int s0 = pend == 1 && have && (e & (kStepUses << 1)) ? 1 : 0;
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i) {
+          const int s = s0 ^ i;
+          auto bit = [&](int field) -> uint32_t { return st >> (field + s) & 1u; };
+          if (pend >> s & 1) {
+            // P.V of the block of step u - 1, in two steps: keys 0-63 as soon as their half of P is written, so that
+            // this half runs while the softmax warpgroup still exponentiates keys 64-127
+            const uint32_t par = bit(kBlocks);
+            if (!wait(bar(sl ^ 1, V_FULL), ((u - 1) >> 1) & 1)) { ok = false; break; }
+            if (bit(kFirst) && !wait(bar(s, O_EMPTY), bit(kTiles) ^ 1)) { ok = false; break; }
+            if (!wait(bar(s, P_READY), par)) { ok = false; break; }
+            tc_fence_after();
+            if (lead) XB_TRACE_EV(0x22 + 0x100 * s, u - 1);
+            issue_pv(s, sl ^ 1, 0, bit(kFirst) ^ 1u);
+            if (!wait(bar(s, P_READY + 1), par)) { ok = false; break; }
+            tc_fence_after();
+            if (lead) XB_TRACE_EV(0x25 + 0x100 * s, u - 1);
+            issue_pv(s, sl ^ 1, 1, 1u);
+            if (bit(kLast)) {
+              mma_commit_lead(bar(s, O_FULL), lead);
+              st ^= 1u << (kTiles + s);
+            }
+            st ^= 1u << (kBlocks + s);
+            st &= ~((1u << kFirst | 1u << kLast) << s);
+            pend &= ~(1u << s);
+          }
+          if (v_used && pend == 0) {
+            mma_commit_lead(bar(sl ^ 1, V_EMPTY), lead);
+            v_used = false;
+          }
+          if (!(todo >> s & 1) || !look(false)) continue;
+          todo &= ~(1u << s);
+          if (e >> s & kStepUses) {
+            if (e >> s & kStepFirst) {
+              if (!wait(bar(s, Q_FULL), bit(kTiles))) { ok = false; break; }
+              st |= 1u << (kFirst + s);
+            }
+            tc_fence_after();
+            if (lead) XB_TRACE_EV(0x20 + 0x100 * s, u);
+            issue_qk(s, sl);
+            mma_commit_lead(bar(s, S_FULL), lead);
+            if (e >> s & kStepLast) {
+              mma_commit_lead(bar(s, Q_EMPTY), lead);
+              st |= 1u << (kLast + s);
+            }
+            next |= 1u << s;
+          }
         }
-      }
+        if (todo) continue;                             // K was not there for both
+        if (e & kStepEnd) break;
+        mma_commit_lead(bar(sl, K_EMPTY), lead);
+        pend = next;
+        next = 0;
+        todo = 3;
+        have = false;
+        v_used = true;
+        ++u;
       }
     }
   } else if (warp < 8) {
     // -------------------------------------------------------------------- softmax of stream (warp >> 2)
-    reg_set<kRegSoftmax>();
-    if constexpr (kHalf) {
-    const int s = warp >> 2;
-    const int quad = warp & 3;
-    const int r = quad * 32 + lane;
-    const uint32_t lane_bits = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t ts0 = tmem_base + s * 128 + lane_bits;         // S / P of this stream, this row (half h at +64h)
-    const uint32_t tmem_o = tmem_base + 256 + s * 128 + lane_bits;
-    const int k_off = p.k_len - p.q_len;
-    const unsigned long long scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
-    const int n_items = sch.n_seq[s];
-    uint32_t bc = 0;
-    bool ok = true;
-    Item it = decode_item(p, n_items > 0 ? item_slot(p, sch.seq[s][0], G) : 0);
-    int n = n_items > 0 ? sch.cnt[sch.seq[s][0]] : 0;
-    int win = n_items > 0 ? list_window(p, block_idx, it.row, n, 0, lane) : 0;
-    for (int m = 0; m < n_items && ok; ++m) {
-      if (lane == 0) XB_TRACE_EV(0x36, m);
-      // the stream's next item: fetch its first list window while this one is processed
-      Item nit = it;
-      int nn = 0, nwin = 0;
-      if (m + 1 < n_items) {
-        const int i2 = sch.seq[s][m + 1];
-        nit = decode_item(p, item_slot(p, i2, G));
-        nn = sch.cnt[i2];
-        nwin = list_window(p, block_idx, nit.row, nn, 0, lane);
-      }
-      const size_t row = it.row;
-      const int q_pos = it.qb * 128 + r;
-      int row_last = p.k_len - 1;                       // last key position this row may see
-      if (p.causal && q_pos + k_off < row_last) row_last = q_pos + k_off;
-      float m_used = -INFINITY, l = 0.f;
-      int w = win, w_next = list_window(p, block_idx, row, n, 32, lane);
-      for (int j = 0; j < n && ok; ++j, ++bc) {
-        if (j > 0 && (j & 31) == 0) {
-          w = w_next;
-          w_next = list_window(p, block_idx, row, n, j + 32, lane);
-        }
-        const int k0 = __shfl_sync(0xffffffffu, w, j & 31) * 128;
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          const int limit = row_last - k0 - 64 * h;       // columns c <= limit of this half are visible
-          const bool masked = __any_sync(0xffffffffu, limit < 63);
-          const uint32_t ts = ts0 + h * 64;
-          if (lane == 0) XB_TRACE_EV(0x30, bc * 2 + h);
-          // waits are made warp-uniform: the tensor-memory loads/stores below are warp-collective
-          if (!__all_sync(0xffffffffu, mbar_wait(bar(s, S_FULL + h), bc & 1, abort_flag))) { ok = false; break; }
-          tc_fence_after();
-          if (lane == 0) XB_TRACE_EV(0x31, bc * 2 + h);
-          // ---- pass 1: row maximum over the 64 columns, 8 chains of 3-input max, both loads in flight
-          float mx8[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) mx8[q] = -INFINITY;
-          // the half's 64 scores stay in registers for both passes: one tensor-memory round trip per half
-          uint32_t v0[32], v1[32];
-          {
-            tmem_ld32(ts, v0);
-            tmem_ld32(ts + 32, v1);
-            tc_wait_ld();
-            if (!masked) {
-#pragma unroll
-              for (int k = 0; k < 16; ++k) {
-                mx8[k & 7] = max3(mx8[k & 7], __uint_as_float(v0[2 * k]), __uint_as_float(v0[2 * k + 1]));
-                mx8[(k + 4) & 7] = max3(mx8[(k + 4) & 7], __uint_as_float(v1[2 * k]), __uint_as_float(v1[2 * k + 1]));
-              }
-            } else {
-#pragma unroll
-              for (int k = 0; k < 16; ++k) {
-                mx8[k & 7] = max3(mx8[k & 7], 2 * k <= limit ? __uint_as_float(v0[2 * k]) : -INFINITY,
-                                  2 * k + 1 <= limit ? __uint_as_float(v0[2 * k + 1]) : -INFINITY);
-                mx8[(k + 4) & 7] = max3(mx8[(k + 4) & 7], 32 + 2 * k <= limit ? __uint_as_float(v1[2 * k]) : -INFINITY,
-                                        33 + 2 * k <= limit ? __uint_as_float(v1[2 * k + 1]) : -INFINITY);
-              }
-            }
-          }
-          const float mx = fmaxf(max3(mx8[0], mx8[1], mx8[2]), max3(max3(mx8[3], mx8[4], mx8[5]), mx8[6], mx8[7]));
-          const float m_new = fmaxf(m_used, mx * p.scale_log2);
-          const bool first = j == 0 && h == 0;
-          const bool need = m_new > m_used + kRescaleThreshold || first || (m_used == -INFINITY && m_new > -INFINITY);
-          if (__any_sync(0xffffffffu, need)) {
-            const float alpha = !need ? 1.f : (m_used == -INFINITY ? 0.f : fast_exp2(m_used - m_new));
-            if (!first) {
-              // O may be touched once every P.V issued so far for this stream has completed (the half before
-              // this one is the latest: its P.V cannot have been issued before this half's P is ready)
-              if (lane == 0) XB_TRACE_EV(0x32, bc * 2 + h);
-              const uint32_t hq = bc * 2 + h;
-              if (!__all_sync(0xffffffffu, mbar_wait(bar(s, PV_DONE), (hq - 1) & 1, abort_flag))) { ok = false; break; }
-              tc_fence_after();
-#pragma unroll 1
-              for (int c4 = 0; c4 < 4; ++c4) {
-                uint32_t v[32];
-                tmem_ld32(tmem_o + c4 * 32, v);
-                tc_wait_ld();
-#pragma unroll
-                for (int k = 0; k < 32; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * alpha);
-                tmem_st32(tmem_o + c4 * 32, v);
-              }
-            }
-            l *= alpha;
-            if (need) m_used = m_new;
-          }
-          const float m_ref = m_used == -INFINITY ? 0.f : m_used;
-          if (lane == 0) XB_TRACE_EV(0x35, bc * 2 + h);
-          // ---- pass 2: exp2 of the two 32-column chunks; P chunk c (16 packed columns) overwrites S columns that
-          // were read already
-          const unsigned long long nmref2 = pack_f32x2(-m_ref, -m_ref);
-          unsigned long long ls2[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) ls2[q] = 0ull;     // (+0.f, +0.f)
-          auto chunk = [&](const uint32_t (&v)[32], int c) {
-            uint32_t pk[16];
-            const int lim = limit - 32 * c;
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              float x0 = __uint_as_float(v[2 * k]), x1 = __uint_as_float(v[2 * k + 1]);
-              if (masked) {
-                x0 = 2 * k <= lim ? x0 : -INFINITY;
-                x1 = 2 * k + 1 <= lim ? x1 : -INFINITY;
-              }
-              float y0, y1;
-              unpack_f32x2(fma_f32x2(pack_f32x2(x0, x1), scale2, nmref2), y0, y1);
-              const float p0 = fast_exp2(y0), p1 = fast_exp2(y1);
-              ls2[k & 3] = add_f32x2(ls2[k & 3], pack_f32x2(p0, p1));
-              pk[k] = pack16(p0, p1, p.is_bf16);
-            }
-            tmem_st16(ts + c * 16, pk);
-          };
-          chunk(v0, 0);
-          chunk(v1, 1);
-          {
-            float a0, a1;
-            unpack_f32x2(add_f32x2(add_f32x2(ls2[0], ls2[1]), add_f32x2(ls2[2], ls2[3])), a0, a1);
-            l += a0 + a1;
-          }
-          if (j == n - 1 && h == 1) s_l[(s * 2 + (m & 1)) * 128 + r] = l;   // for the epilogue of this item
-          tc_wait_st();
-          tc_fence_before();
-          mbar_arrive(bar(s, P_READY + h));
-          if (lane == 0) XB_TRACE_EV(0x33, bc * 2 + h);
-        }
-      }
-      it = nit; n = nn; win = nwin;
-    }
-    } else {
+    reg_set_from<kRegSoftmax, 128>();
     const int s = warp >> 2;
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
@@ -539,248 +514,245 @@ __device__ __forceinline__ void attn_cta(const CUtensorMap& tmQ, const CUtensorM
     const uint32_t ts = tmem_base + s * 128 + lane_bits;          // S / P of this stream, this row
     const uint32_t tmem_o = tmem_base + 256 + s * 128 + lane_bits;
     const int k_off = p.k_len - p.q_len;
-    const uint32_t s_full = bar(s, S_FULL);
-    const int n_items = sch.n_seq[s];
+    const unsigned long long scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
     uint32_t bc = 0;
     bool ok = true;
-    Item it = decode_item(p, n_items > 0 ? item_slot(p, sch.seq[s][0], G) : 0);
-    int n = n_items > 0 ? sch.cnt[sch.seq[s][0]] : 0;
-    int win = n_items > 0 ? list_window(p, block_idx, it.row, n, 0, lane) : 0;
-    for (int m = 0; m < n_items && ok; ++m) {
-      if (lane == 0) XB_TRACE_EV(0x36, m);
-      // the stream's next item: fetch its first list window while this one is processed
-      Item nit = it;
-      int nn = 0, nwin = 0;
-      if (m + 1 < n_items) {
-        const int i2 = sch.seq[s][m + 1];
-        nit = decode_item(p, item_slot(p, i2, G));
-        nn = sch.cnt[i2];
-        nwin = list_window(p, block_idx, nit.row, nn, 0, lane);
+    // the stream's tile in the next unit, with its list's first window on its way from memory.  (One unit at a time: to
+    // wait here for a unit that lists anything would hold up the unit at hand, and with it the publication of the next.)
+    UnitTile nt;
+    int nwin = 0;
+    auto list_of = [&](const UnitTile& ut) -> List {
+      Tile tt;
+      tt.b = ut.b; tt.h = ut.h; tt.qb = ut.qb;
+      return tile_list(p, block_idx, tt, ut.n);
+    };
+    auto fetch = [&]() {
+      if (!units.wait()) {
+        nt.n = -1;
+        return;
       }
-      const size_t row = it.row;
-      const int q_pos = it.qb * 128 + r;
+      nt = units.tile(s);
+      units.release(lane);
+      if (nt.n > 0) nwin = list_window(list_of(nt), 0, lane);
+    };
+    int m = 0;
+    nt.n = 0;
+#pragma unroll 1
+    while (ok && nt.n >= 0) {
+      if (nt.n == 0) {                                  // (at the start, too)
+        fetch();
+        continue;
+      }
+      const UnitTile t = nt;
+      const List list = list_of(t);
+      if (lane == 0) XB_TRACE_EV(0x36, m);
+      const int n = list.n;
+      const int q_pos = t.qb * 128 + r;
       int row_last = p.k_len - 1;                       // last key position this row may see
       if (p.causal && q_pos + k_off < row_last) row_last = q_pos + k_off;
+      int row_last_lo = p.k_len - 1;                    // the same for the first row of the warp
+      if (p.causal && t.qb * 128 + quad * 32 + k_off < row_last_lo) row_last_lo = t.qb * 128 + quad * 32 + k_off;
       float m_used = -INFINITY, l = 0.f;
-      int w = win, w_next = list_window(p, block_idx, row, n, 32, lane);
-      if (lane == 0) XB_TRACE_EV(0x37, m);
+      int w = nwin, w_next = list_window(list, 32, lane);
+#pragma unroll 1
       for (int j = 0; j < n; ++j, ++bc) {
         if (j > 0 && (j & 31) == 0) {
           w = w_next;
-          w_next = list_window(p, block_idx, row, n, j + 32, lane);
+          w_next = list_window(list, j + 32, lane);
         }
         const int k0 = __shfl_sync(0xffffffffu, w, j & 31) * 128;
-        if (lane == 0) XB_TRACE_EV(0x38, bc);
         if (lane == 0) XB_TRACE_EV(0x30, bc);
         // waits are made warp-uniform: the tensor-memory loads/stores below are warp-collective
-        if (!__all_sync(0xffffffffu, mbar_wait(s_full, bc & 1, abort_flag))) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(bar(s, S_FULL), bc & 1, abort_flag))) { ok = false; break; }
         tc_fence_after();
         if (lane == 0) XB_TRACE_EV(0x31, bc);
-        // The block's 128 scores are taken in two halves of 64 columns, each an online-softmax step of its own:
-        // one tensor-memory round trip per half (both 32-column loads in flight), the 64 scores stay in registers
-        // for the maximum and for the exponentiation, and P of keys 0-63 is handed to the tensor pipe while keys
-        // 64-127 are still being worked on.  P (16-bit, two keys per column) of half h goes to columns
-        // [32h, 32h + 32), which hold scores that are in registers by then.
-        const unsigned long long scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          const int limit = row_last - k0 - 64 * h;       // columns c <= limit of this half are visible
-          const bool none_vis = __all_sync(0xffffffffu, limit < 0);
-          const bool masked = __any_sync(0xffffffffu, limit < 63);
-          if (none_vis) {
-            // (the upper half of the diagonal block for the first 64 rows) P = 0, nothing else changes
-            uint32_t z[16];
+        float mx8[8];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) z[k] = 0u;
-            tmem_st16(ts + h * 32, z);
-            tmem_st16(ts + h * 32 + 16, z);
-          } else {
-            float mx8[8];
+        for (int q = 0; q < 8; ++q) mx8[q] = -INFINITY;
+        auto chunk_max = [&](const uint32_t (&x)[32]) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) mx8[q] = -INFINITY;
-            uint32_t v0[32], v1[32];
-            tmem_ld32(ts + h * 64, v0);
-            tmem_ld32(ts + h * 64 + 32, v1);
-            tc_wait_ld();
-            if (!masked) {
+          for (int k = 0; k < 16; ++k)
+            mx8[k & 7] = max3(mx8[k & 7], __uint_as_float(x[2 * k]), __uint_as_float(x[2 * k + 1]));
+        };
+        unsigned long long ls2[4], nmref2 = 0ull;
 #pragma unroll
-              for (int k = 0; k < 16; ++k) {
-                mx8[k & 7] = max3(mx8[k & 7], __uint_as_float(v0[2 * k]), __uint_as_float(v0[2 * k + 1]));
-                mx8[(k + 4) & 7] = max3(mx8[(k + 4) & 7], __uint_as_float(v1[2 * k]), __uint_as_float(v1[2 * k + 1]));
-              }
-            } else {
+        for (int q = 0; q < 4; ++q) ls2[q] = 0ull;     // (+0.f, +0.f)
+        // exp2 of 32 scores, their sum, and P packed to 16 bit
+        auto chunk_exp = [&](const uint32_t (&x)[32], uint32_t (&pk)[16]) {
 #pragma unroll
-              for (int k = 0; k < 16; ++k) {
-                mx8[k & 7] = max3(mx8[k & 7], 2 * k <= limit ? __uint_as_float(v0[2 * k]) : -INFINITY,
-                                  2 * k + 1 <= limit ? __uint_as_float(v0[2 * k + 1]) : -INFINITY);
-                mx8[(k + 4) & 7] = max3(mx8[(k + 4) & 7], 32 + 2 * k <= limit ? __uint_as_float(v1[2 * k]) : -INFINITY,
-                                        33 + 2 * k <= limit ? __uint_as_float(v1[2 * k + 1]) : -INFINITY);
-              }
-            }
-            const float mx = fmaxf(max3(mx8[0], mx8[1], mx8[2]), max3(max3(mx8[3], mx8[4], mx8[5]), mx8[6], mx8[7]));
-            const float m_new = fmaxf(m_used, mx * p.scale_log2);
-            const bool first = j == 0 && h == 0;
-            const bool need = m_new > m_used + kRescaleThreshold || first || (m_used == -INFINITY && m_new > -INFINITY);
-            if (__any_sync(0xffffffffu, need)) {
-              const float alpha = !need ? 1.f : (m_used == -INFINITY ? 0.f : fast_exp2(m_used - m_new));
-              if (!first) {
-                // O may be touched once every P.V issued so far for this stream has completed (the half before
-                // this one is the latest: its P.V cannot have been issued before this half's P is ready)
-                if (lane == 0) XB_TRACE_EV(0x32, bc);
-                const uint32_t hq = bc * 2 + h;
-                if (!__all_sync(0xffffffffu, mbar_wait(bar(s, PV_DONE), (hq - 1) & 1, abort_flag))) { ok = false; break; }
-                tc_fence_after();
-#pragma unroll 1
-                for (int c4 = 0; c4 < 4; ++c4) {
-                  uint32_t v[32];
-                  tmem_ld32(tmem_o + c4 * 32, v);
-                  tc_wait_ld();
-#pragma unroll
-                  for (int k = 0; k < 32; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * alpha);
-                  tmem_st32(tmem_o + c4 * 32, v);
-                }
-              }
-              l *= alpha;
-              if (need) m_used = m_new;
-            }
-            const float m_ref = m_used == -INFINITY ? 0.f : m_used;
-            if (lane == 0) XB_TRACE_EV(0x35, bc);
-            const unsigned long long nmref2 = pack_f32x2(-m_ref, -m_ref);
-            unsigned long long ls2[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) ls2[q] = 0ull;     // (+0.f, +0.f)
-            auto chunk = [&](const uint32_t (&v)[32], int c) {
-              uint32_t pk[16];
-              const int lim = limit - 32 * c;
-#pragma unroll
-              for (int k = 0; k < 16; ++k) {
-                float x0 = __uint_as_float(v[2 * k]), x1 = __uint_as_float(v[2 * k + 1]);
-                if (masked) {
-                  x0 = 2 * k <= lim ? x0 : -INFINITY;
-                  x1 = 2 * k + 1 <= lim ? x1 : -INFINITY;
-                }
-                float y0, y1;
-                unpack_f32x2(fma_f32x2(pack_f32x2(x0, x1), scale2, nmref2), y0, y1);
-                const float p0 = fast_exp2(y0), p1 = fast_exp2(y1);
-                ls2[k & 3] = add_f32x2(ls2[k & 3], pack_f32x2(p0, p1));
-                pk[k] = pack16(p0, p1, p.is_bf16);
-              }
-              tmem_st16(ts + h * 32 + c * 16, pk);
-            };
-            chunk(v0, 0);
-            chunk(v1, 1);
-            float a0, a1;
-            unpack_f32x2(add_f32x2(add_f32x2(ls2[0], ls2[1]), add_f32x2(ls2[2], ls2[3])), a0, a1);
-            l += a0 + a1;
+          for (int k = 0; k < 16; ++k) {
+            float y0, y1;
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(x[2 * k]), __uint_as_float(x[2 * k + 1])), scale2, nmref2),
+                         y0, y1);
+            const float p0 = fast_exp2(y0), p1 = fast_exp2(y1);
+            ls2[k & 3] = add_f32x2(ls2[k & 3], pack_f32x2(p0, p1));
+            pk[k] = pack16t<kBf16>(p0, p1);
           }
-          if (j == n - 1 && h == 1) s_l[(s * 2 + (m & 1)) * 128 + r] = l;   // read by the epilogue once this item's last P.V is done
+        };
+        // the running maximum moves to cover this block (lazily); O is rescaled if it holds anything already
+        auto rescale = [&]() {
+          const float mx = fmaxf(max3(mx8[0], mx8[1], mx8[2]), max3(max3(mx8[3], mx8[4], mx8[5]), mx8[6], mx8[7]));
+          const float m_new = fmaxf(m_used, mx * p.scale_log2);
+          const bool need = m_new > m_used + kRescaleThreshold || j == 0 || (m_used == -INFINITY && m_new > -INFINITY);
+          if (__any_sync(0xffffffffu, need)) {
+            const float alpha = !need ? 1.f : (m_used == -INFINITY ? 0.f : fast_exp2(m_used - m_new));
+            if (j > 0) {
+              // O may be touched: S of this block is complete, and its MMAs were issued after the stream's P.V of all
+              // earlier blocks
+              if (lane == 0) XB_TRACE_EV(0x32, bc);
+#pragma unroll 1
+              for (int c4 = 0; c4 < 8; ++c4) {
+                uint32_t o[16];
+                tmem_ld16(tmem_o + c4 * 16, o);
+                tc_wait_ld();
+#pragma unroll
+                for (int k = 0; k < 16; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
+                tmem_st16(tmem_o + c4 * 16, o);
+              }
+            }
+            l *= alpha;
+            if (need) m_used = m_new;
+          }
+          const float m_ref = m_used == -INFINITY ? 0.f : m_used;
+          nmref2 = pack_f32x2(-m_ref, -m_ref);
+          if (lane == 0) XB_TRACE_EV(0x35, bc);
+        };
+        // P of chunk c (32 keys, 16 packed columns) goes to columns [16 c, 16 c + 16): scores that have been read by now
+        auto half_ready = [&](int h) {
           tc_wait_st();
           tc_fence_before();
           mbar_arrive(bar(s, P_READY + h));
-          if (lane == 0) XB_TRACE_EV(0x33, bc * 2 + h);
+        };
+        // last visible column of the warp's first row: every row of the warp sees the whole block, or some do not
+        const int lim_lo = row_last_lo - k0;
+        if (lim_lo < 127) {
+          // Some columns are hidden from some rows (diagonal blocks, the ragged last block): their scores are replaced by
+          // -inf in tensor memory, in a rolled loop over the chunks concerned, because the code has to stay small.
+          const int lim = row_last - k0;                // columns c <= lim are visible
+#pragma unroll 1
+          for (int c = lim_lo < 0 ? 0 : (lim_lo + 1) >> 5; c < 4; ++c) {
+            uint32_t x[32];
+            tmem_ld32(ts + c * 32, x);
+            tc_wait_ld();
+            const int lc = lim - 32 * c;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) x[k] = k <= lc ? x[k] : 0xff800000u;
+            tmem_st32(ts + c * 32, x);
+          }
+          tc_wait_st();
         }
-        if (!ok) break;
+        uint32_t v[4][32];
+        tmem_ld32(ts, v[0]);
+        tmem_ld32(ts + 32, v[1]);
+        tc_wait_ld();
+        tmem_ld32(ts + 64, v[2]);
+        tmem_ld32(ts + 96, v[3]);
+        chunk_max(v[0]);
+        chunk_max(v[1]);
+        tc_wait_ld();
+        chunk_max(v[2]);
+        chunk_max(v[3]);
+        rescale();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
+          chunk_exp(v[c], pk);
+          tmem_st16(ts + c * 16, pk);
+          if (c == 1) {
+            half_ready(0);
+            if (lane == 0) XB_TRACE_EV(0x34, bc);
+          }
+        }
+        {
+          float a0, a1;
+          unpack_f32x2(add_f32x2(add_f32x2(ls2[0], ls2[1]), add_f32x2(ls2[2], ls2[3])), a0, a1);
+          l += a0 + a1;
+        }
+        if (j == n - 1) s_l[(s * 2 + (m & 1)) * 128 + r] = l;   // read by the epilogue once this tile's last P.V is done
+        half_ready(1);
+        if (j == 0) fetch();
+        if (lane == 0) XB_TRACE_EV(0x33, bc);
       }
-      it = nit; n = nn; win = nwin;
-    }
+      ++m;
     }
   } else {
     // -------------------------------------------------------------------- epilogue (warps 8-11), both streams
-    reg_set<kRegEpilogue>();
+    reg_set_from<kRegEpilogue, 128>();
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
     const uint32_t lane_bits = static_cast<uint32_t>(quad * 32) << 16;
-    uint32_t seen = 0;                 // non-empty items so far: item `seen` runs on stream seen & 1
+    // A warp's 32 rows x 128 columns go, scaled and packed to 16 bit, to a staging tile of two 64-column halves in the
+    // 128-byte swizzle pattern (16-byte chunk c of row r at chunk c ^ (r & 7)) and leave as two TMA stores, which also
+    // clip the rows past q_len.  O leaves tensor memory before the stores, so that the stream's next tile can start
+    // accumulating while this one is still being stored.
+    uint8_t* stg = stage_base + quad * (2 * 32 * 128);
+    uint32_t done = 0;                 // tiles with a list so far, mod 2: stream 0 in bit 0, stream 1 in bit 1
     bool ok = true;
-    for (int i = 0; i < sch.n_local && ok; ++i) {
-      const int t = item_slot(p, i, G);
-      const int n = sch.cnt[i];
-      const Item it = decode_item(p, t);
-      const int q_pos = it.qb * 128 + r;
-      const bool store = q_pos < p.q_len;
-      uint8_t* orow = static_cast<uint8_t*>(out) +
-                      2 * (static_cast<int64_t>(it.b) * p.osb + static_cast<int64_t>(it.h) * p.osh +
-                           static_cast<int64_t>(store ? q_pos : 0) * p.osl);
-      if (n == 0) {
-        if (store) {
-          uint4* dst = reinterpret_cast<uint4*>(orow);
-#pragma unroll
-          for (int q4 = 0; q4 < 16; ++q4) dst[q4] = make_uint4(0u, 0u, 0u, 0u);
-        }
-        continue;
+    UnitTile t1;
+#pragma unroll 1
+    for (int i = 0; ok; ++i) {
+      const int s = i & 1;
+      UnitTile t = t1;
+      if (s == 0) {
+        if (!units.wait()) break;
+        t = units.tile(0);
+        t1 = units.tile(1);
+        units.release(lane);
       }
-      const int s = seen & 1;
-      const uint32_t m = seen >> 1;
-      ++seen;
-      if (threadIdx.x == 256) XB_TRACE_EV(0x40 + s, m);
-      if (!__all_sync(0xffffffffu, mbar_wait(bar(s, O_FULL), m & 1, abort_flag))) { ok = false; break; }
-      tc_fence_after();
-      if (threadIdx.x == 256) XB_TRACE_EV(0x42 + s, m);
-      const float l = s_l[(s * 2 + (m & 1)) * 128 + r];
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const int n = t.n;
+      if (n < 0) break;
+      if (t.qb < 0) continue;
+      float inv = 0.f;
+      if (n > 0) {
+        const uint32_t m = (done >> s) & 1;
+        done ^= 1u << s;
+        if (threadIdx.x == 256) XB_TRACE_EV(0x40 + s, m);
+        if (!__all_sync(0xffffffffu, mbar_wait(bar(s, O_FULL), m, abort_flag))) { ok = false; break; }
+        tc_fence_after();
+        if (threadIdx.x == 256) XB_TRACE_EV(0x42 + s, m);
+        const float l = s_l[(s * 2 + m) * 128 + r];
+        inv = l > 0.f ? 1.f / l : 0.f;
+      }
+      if (lane == 0) tma_store_wait_read();             // the staging tile's previous stores have read it
+      __syncwarp();
       const uint32_t tmem_o = tmem_base + 256 + s * 128 + lane_bits;
-      // A thread owns one output row, but a store instruction should write whole cache lines: each 64-column
-      // half of the warp's 32 rows goes through a 4 KiB shared-memory buffer (16-byte chunks XOR-swizzled by
-      // row against bank conflicts) and leaves as 8 instructions of 4 rows x 128 contiguous bytes.
-      uint8_t* stg = stage_base + quad * (32 * 128);
-      const int q_row0 = it.qb * 128 + quad * 32;                     // first row of this warp
-      uint8_t* obase = static_cast<uint8_t*>(out) +
-                       2 * (static_cast<int64_t>(it.b) * p.osb + static_cast<int64_t>(it.h) * p.osh);
-      // O leaves tensor memory first, half by half (scaled and packed to 16 bit; the first half is parked in the
-      // staging buffer, the second in registers), so that the stream's next item can start accumulating while
-      // this one is still being stored
-      auto load_half = [&](int half, uint4 (&pk)[8]) {
-        uint32_t v0[32], v1[32];
-        tmem_ld32(tmem_o + half * 64, v0);
-        tmem_ld32(tmem_o + half * 64 + 32, v1);
-        tc_wait_ld();
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        uint32_t pk[16];
+        if (n > 0) {
+          uint32_t v[32];
+          tmem_ld32(tmem_o + c * 32, v);
+          tc_wait_ld();
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          pk[q4] = make_uint4(
-              pack16(__uint_as_float(v0[q4 * 8 + 0]) * inv, __uint_as_float(v0[q4 * 8 + 1]) * inv, p.is_bf16),
-              pack16(__uint_as_float(v0[q4 * 8 + 2]) * inv, __uint_as_float(v0[q4 * 8 + 3]) * inv, p.is_bf16),
-              pack16(__uint_as_float(v0[q4 * 8 + 4]) * inv, __uint_as_float(v0[q4 * 8 + 5]) * inv, p.is_bf16),
-              pack16(__uint_as_float(v0[q4 * 8 + 6]) * inv, __uint_as_float(v0[q4 * 8 + 7]) * inv, p.is_bf16));
-          pk[4 + q4] = make_uint4(
-              pack16(__uint_as_float(v1[q4 * 8 + 0]) * inv, __uint_as_float(v1[q4 * 8 + 1]) * inv, p.is_bf16),
-              pack16(__uint_as_float(v1[q4 * 8 + 2]) * inv, __uint_as_float(v1[q4 * 8 + 3]) * inv, p.is_bf16),
-              pack16(__uint_as_float(v1[q4 * 8 + 4]) * inv, __uint_as_float(v1[q4 * 8 + 5]) * inv, p.is_bf16),
-              pack16(__uint_as_float(v1[q4 * 8 + 6]) * inv, __uint_as_float(v1[q4 * 8 + 7]) * inv, p.is_bf16));
+          for (int k = 0; k < 16; ++k)
+            pk[k] = pack16t<kBf16>(__uint_as_float(v[2 * k]) * inv, __uint_as_float(v[2 * k + 1]) * inv);
+        } else {                                        // an empty list: zeros
+#pragma unroll
+          for (int k = 0; k < 16; ++k) pk[k] = 0u;
         }
-      };
-      auto stage = [&](const uint4 (&pk)[8]) {
+        uint8_t* row = stg + (c >> 1) * (32 * 128) + lane * 128;
 #pragma unroll
-        for (int chunk = 0; chunk < 8; ++chunk)
-          *reinterpret_cast<uint4*>(stg + lane * 128 + ((chunk ^ (lane & 7)) << 4)) = pk[chunk];
-      };
-      auto store_half = [&](int half) {
-#pragma unroll
-        for (int i2 = 0; i2 < 8; ++i2) {
-          const int rr = 4 * i2 + (lane >> 3);                        // row within the warp's 32
-          const int chunk = lane & 7;
-          const uint4 wv = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((chunk ^ (rr & 7)) << 4));
-          const int q_pos_r = q_row0 + rr;
-          if (q_pos_r < p.q_len)
-            *reinterpret_cast<uint4*>(obase + 2 * static_cast<int64_t>(q_pos_r) * p.osl + half * 128 + chunk * 16) = wv;
-        }
-      };
-      {
-        uint4 pk[8];
-        load_half(0, pk);
-        stage(pk);
-        load_half(1, pk);
+        for (int q4 = 0; q4 < 4; ++q4)
+          *reinterpret_cast<uint4*>(row + (((((c & 1) << 2) | q4) ^ (lane & 7)) << 4)) =
+              make_uint4(pk[4 * q4], pk[4 * q4 + 1], pk[4 * q4 + 2], pk[4 * q4 + 3]);
+      }
+      if (n > 0) {
         tc_fence_before();
         mbar_arrive(bar(s, O_EMPTY));
-        __syncwarp();
-        store_half(0);
-        __syncwarp();
-        stage(pk);
-        __syncwarp();
-        store_half(1);
-        __syncwarp();
       }
-      if (threadIdx.x == 256) XB_TRACE_EV(0x44 + s, m);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        const int q_row0 = t.qb * 128 + quad * 32;      // first row of this warp
+        if (q_row0 < p.q_len) {
+          tma_store_5d(&tmO, smem_u32(stg), 0, q_row0, 0, t.h, t.b);
+          tma_store_5d(&tmO, smem_u32(stg + 32 * 128), 0, q_row0, 1, t.h, t.b);
+          tma_store_commit();
+        }
+      }
+      if (threadIdx.x == 256) XB_TRACE_EV(0x44 + s, 0);
     }
+    if (lane == 0) tma_store_wait_all();                // the staging tiles must outlive the stores that read them
   }
 
   // -------------------------------------------------------------------- teardown
@@ -798,107 +770,63 @@ __device__ __forceinline__ void attn_cta(const CUtensorMap& tmQ, const CUtensorM
   }
 }
 
-// The kernel: builds the CTA's schedule in shared memory, sums its list lengths and runs the instantiation that
-// fits them (a CTA executes only one of the two bodies, so only that one occupies its instruction cache).
-__global__ void __launch_bounds__(kAttnThreads, 1)
-block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmKf,
-                         const __grid_constant__ CUtensorMap tmVf, const AttnParams p_in,
-                         const int32_t* __restrict__ block_idx, const int32_t* __restrict__ block_cnt,
-                         const int32_t* __restrict__ rest_list, const int* __restrict__ pair_header,
-                         int pair_min_share, void* __restrict__ out, int* status) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  // with a pair kernel in front: the items it left (a list, spread evenly over the CTAs) if it ran, all items if it
-  // declined.  In that case this kernel was launched while the pair kernel was running and first waits for it (and
-  // so for the classify kernel before it) to end.
-  pdl_wait();
-  AttnParams p = p_in;
-  if (rest_list && pair_path_chosen(pair_header, pair_min_share)) {
-    p.item_list = rest_list;
-    p.total_items = *reinterpret_cast<const volatile int*>(pair_header + kPairRestCount);
-  }
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  if ((smem_u32(smem) & 1023u) != 0) {              // the swizzled tiles need 1024-byte alignment
-    if (threadIdx.x == 0 && status) atomicExch(status, static_cast<int>(kDevBadSmemAlign));
-    return;
-  }
-  uint16_t* sch_cnt = reinterpret_cast<uint16_t*>(smem + kAttnSmemTiles + 2 * 2 * 128 * 4 + 512);
-  uint16_t* sch_seq0 = sch_cnt + kSchedCap;
-  uint16_t* sch_seq1 = sch_seq0 + kSchedCap;
-  int* sch_total = reinterpret_cast<int*>(sch_seq1 + kSchedCap);
-  const int G = gridDim.x;
-  const int n_local = local_item_count(p, G);                       // host guarantees <= kSchedCap
-  for (int i = threadIdx.x; i < n_local; i += kAttnThreads) {
-    const int c = __ldg(block_cnt + decode_item(p, item_slot(p, i, G)).row);
-    sch_cnt[i] = static_cast<uint16_t>(c > 65534 ? 65534 : c);
-  }
-  __syncthreads();
-  if (warp == 0) {
-    int running = 0, blocks = 0;
-    for (int base = 0; base < n_local; base += 32) {
-      const int i = base + lane;
-      const int c = i < n_local ? sch_cnt[i] : 0;
-      const bool ne = c > 0;
-      const unsigned bal = __ballot_sync(0xffffffffu, ne);
-      const int k = running + __popc(bal & ((1u << lane) - 1u));
-      if (ne) ((k & 1) ? sch_seq1 : sch_seq0)[k >> 1] = static_cast<uint16_t>(i);
-      running += __popc(bal);
-      blocks += c;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) blocks += __shfl_xor_sync(0xffffffffu, blocks, o);
-    if (lane == 0) {
-      sch_total[0] = running;
-      sch_total[1] = blocks;
-    }
-  }
-  __syncthreads();
-  if (2 * sch_total[1] >= kHalfModeMinBlocksX2 * sch_total[0])
-    attn_cta<true>(tmQ, tmK, tmV, tmKf, tmVf, p, block_idx, out, status);
-  else
-    attn_cta<false>(tmQ, tmK, tmV, tmKf, tmVf, p, block_idx, out, status);
-}
-
-// ------------------------------------------------------------------------------------------------ item order
-// Orders the work items kv head by kv head and, inside a kv head, by list length, longest first; the attention
-// kernel then deals that list to its CTAs in rows of gridDim.x, in alternating direction.  Two effects, both for
-// masks without an order of their own (non-causal video-diffusion masks: rows list 5 to 891 of 931 blocks, anywhere
-// in the sequence):
-//  * all CTAs work on one kv head at a time and finish it together (every row of the deal holds items of similar
-//    length), so the K/V tiles they gather come from that head's tensors only -- 61 MB at 119K tokens, which stay in
-//    L2, where the natural order walks all 24 heads at once (1.46 GB) and re-reads every tile from HBM: measured on
-//    random 26-block lists at 119K tokens, 662 TFLOP/s with 24 heads against 914 with two;
-//  * no CTA gets the longest item of every row.
-// One CTA per (batch, kv head) sorts that head's items with a counting sort (lengths above kOrderBuckets - 1 share
-// the first bucket; the order inside a bucket is as the atomics fall, which changes nothing in the result) and
-// writes them into the head's segment of the list.
-constexpr int kOrderBuckets = 2048;
+// ------------------------------------------------------------------------------------------------ unit order
+// Non-causal masks have no order of their own (video diffusion: rows list 5 to 891 of 931 blocks, anywhere in the
+// sequence).  The units are put in this order: first the very long ones of all heads, then kv head by kv head the others,
+// longest first.  Two effects:
+//  * the CTAs work on one kv head at a time, so the K/V tiles they gather come from that head's tensors only -- 61 MB at
+//    119K tokens, which stay in L2, where a walk over all 24 heads at once (1.46 GB) re-reads every tile from HBM;
+//  * a unit that would keep a CTA busy for a good part of the whole call (the rows of the text tokens list nearly every
+//    block) starts at once instead of near the end.
+// One CTA per (batch, kv head) sorts that head's units with a counting sort by the two tiles' list lengths (sums above
+// kOrderBuckets - 1 share the first bucket; the order inside a bucket is as the atomics fall, which changes nothing in
+// the result) and counts the very long units of all heads by itself, so that the CTAs need not wait for one another.
+constexpr int kOrderBuckets = 4096;
 constexpr int kOrderThreads = 1024;
 __global__ void __launch_bounds__(kOrderThreads, 1)
-attn_order_kernel(const AttnParams p, const int32_t* __restrict__ block_cnt, int32_t* __restrict__ sorted) {
+attn_order_kernel(const AttnParams p, const int32_t* __restrict__ block_cnt, int sms, int32_t* __restrict__ sorted) {
   __shared__ int hist[kOrderBuckets];
   __shared__ int warp_sum[kOrderThreads / 32];
+  __shared__ unsigned long long s_blocks;
+  __shared__ int s_long[3];           // very long units: of all heads, of the heads before this one, of this one
   pdl_launch_dependents();            // the attention kernel may take its place; it waits for this grid to end
   const int tid = threadIdx.x;
-  const int group = p.hq / p.hkv;
-  const int b = blockIdx.x / p.hkv, g = blockIdx.x % p.hkv;
-  const int n_seg = group * p.q_blocks;                                  // items of this (batch, kv head)
-  const size_t row0 = (static_cast<size_t>(b) * p.hq + static_cast<size_t>(g) * group) * p.q_blocks;
-  int32_t* seg = sorted + static_cast<size_t>(blockIdx.x) * n_seg;
+  const int n_seg = static_cast<int>(p.by_units.d);                      // units of a (batch, kv head)
+  const int n_heads = gridDim.x, first = blockIdx.x * n_seg;
+  if (tid == 0) s_blocks = 0;
+  if (tid < 3) s_long[tid] = 0;
   for (int i = tid; i < kOrderBuckets; i += kOrderThreads) hist[i] = 0;
   __syncthreads();
-  // item j of the segment: query head g * group + j / q_blocks, query block j % q_blocks -- the count array's own
-  // order.  The bucket index grows as the list gets shorter.
-  auto bucket = [&](int j) {
-    const int c = __ldg(block_cnt + row0 + j);
-    return kOrderBuckets - 1 - (c < 0 ? 0 : (c > kOrderBuckets - 1 ? kOrderBuckets - 1 : c));
-  };
-  for (int j = tid; j < n_seg; j += kOrderThreads) atomicAdd(&hist[bucket(j)], 1);
+  // blocks listed by the whole call; a unit with more than an eighth of one SM's share of them is a very long one
+  const int rows = p.batch * p.hq * p.q_blocks;
+  unsigned long long sum = 0;
+  for (int i = tid; i < rows; i += kOrderThreads) sum += static_cast<unsigned>(__ldg(block_cnt + i));
+  atomicAdd(&s_blocks, sum);
   __syncthreads();
-  // exclusive prefix over the buckets, two per thread
-  const int h0 = hist[2 * tid], h1 = hist[2 * tid + 1];
-  int incl = h0 + h1;
+  unsigned long long lim64 = s_blocks / (8ull * sms);
+  const int limit = lim64 < 64 ? 64 : (lim64 > kOrderBuckets - 2 ? kOrderBuckets - 2 : static_cast<int>(lim64));
+  auto length = [&](int u) {
+    Tile t0, t1;
+    unit_tiles(p, u, t0, t1);
+    const int c = tile_count(p, block_cnt, t0) + tile_count(p, block_cnt, t1);
+    return c < 0 ? 0 : (c > kOrderBuckets - 1 ? kOrderBuckets - 1 : c);
+  };
+  for (int u = tid; u < n_heads * n_seg; u += kOrderThreads) {
+    const int c = length(u);
+    const bool own = u >= first && u < first + n_seg;
+    if (own) atomicAdd(&hist[kOrderBuckets - 1 - c], 1);                 // the bucket index grows as the lists get shorter
+    if (c > limit) {
+      atomicAdd(&s_long[0], 1);
+      if (own) atomicAdd(&s_long[2], 1);
+      else if (u < first) atomicAdd(&s_long[1], 1);
+    }
+  }
+  __syncthreads();
+  // exclusive prefix over the buckets, four per thread
+  int h[4], hsum = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) { h[q] = hsum; hsum += hist[4 * tid + q]; }
+  int incl = hsum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int v = __shfl_up_sync(0xffffffffu, incl, o);
@@ -916,20 +844,25 @@ attn_order_kernel(const AttnParams p, const int32_t* __restrict__ block_cnt, int
     warp_sum[tid] = w;                 // inclusive over the warps
   }
   __syncthreads();
-  const int base = ((tid >> 5) > 0 ? warp_sum[(tid >> 5) - 1] : 0) + incl - h0 - h1;
+  const int base = ((tid >> 5) > 0 ? warp_sum[(tid >> 5) - 1] : 0) + incl - hsum;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) hist[4 * tid + q] = base + h[q];           // from here on: the bucket's next free place
   __syncthreads();
-  hist[2 * tid] = base;                // from here on: the next free position of the bucket
-  hist[2 * tid + 1] = base + h0;
-  __syncthreads();
-  for (int j = tid; j < n_seg; j += kOrderThreads) {
-    const int h = g * group + j / p.q_blocks, qb = j % p.q_blocks;
-    // the attention kernel's item numbering (decode_item): t = ((q_blocks - 1 - qb) * batch + b) * hq + h
-    seg[atomicAdd(&hist[bucket(j)], 1)] = ((p.q_blocks - 1 - qb) * p.batch + b) * p.hq + h;
+  const int all_long = s_long[0], before = s_long[1], own_long = s_long[2];
+  for (int u = first + tid; u < first + n_seg; u += kOrderThreads) {
+    const int rank = atomicAdd(&hist[kOrderBuckets - 1 - length(u)], 1);
+    const int at = rank < own_long ? before + rank : all_long + first - before + (rank - own_long);
+    Tile t0, t1;
+    unit_tiles(p, u, t0, t1);
+    // the numbering of the tile list: ((q_blocks - 1 - qb) * batch + b) * hq + h
+    auto item = [&](const Tile& t) { return t.qb < 0 ? -1 : ((p.q_blocks - 1 - t.qb) * p.batch + t.b) * p.hq + t.h; };
+    sorted[2 * at] = item(t0);
+    sorted[2 * at + 1] = item(t1);
   }
 }
 
 size_t order_workspace_bytes(int batch, int hq, int q_len) {
-  return static_cast<size_t>(batch) * hq * ((static_cast<size_t>(q_len) + 127) / 128) * sizeof(int32_t);
+  return static_cast<size_t>(batch) * hq * (((static_cast<size_t>(q_len) + 127) / 128 + 1) / 2) * 2 * sizeof(int32_t);
 }
 
 size_t pair_workspace_bytes(int batch, int hq, int hkv, int q_len);
@@ -953,19 +886,19 @@ size_t block_sparse_attn_workspace_bytes(int batch, int hq, int hkv, int q_len, 
   return pair > order ? pair : order;
 }
 
-// With a workspace a causal call (with an even number >= 2 of query heads per kv head) runs in two parts: the group
-// items whose heads all list the same one or two blocks go to the pair kernel (attention_pair.cu), everything else
-// to the general kernel below, which takes its items from the list the pair path leaves.  A non-causal call with a
-// workspace has its items ordered kv head by kv head, longest list first inside a head (attn_order_kernel).  Without a workspace the general kernel
-// computes everything in the order of the item numbering (rows from the last query block to the first: under a
-// causal mask that is longest first already).
+// Without lists (block_idx and block_cnt null) the call is dense.  With a workspace a causal call (with an even number >= 2
+// of query heads per kv head) runs in two parts: the group items whose heads all list the same one or two blocks go to the
+// pair kernel (attention_pair.cu), everything else to the general kernel, which takes its tiles from the list the pair
+// path leaves (a group's query heads stand next to one another in it, so two entries read the same kv head).  A
+// non-causal call with a workspace has its units ordered first (attn_order_kernel).
 int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv,
                              int q_len, int k_len, int head_dim, int64_t qsb, int64_t qsh, int64_t qsl, int64_t ksb,
                              int64_t ksh, int64_t ksl, int64_t vsb, int64_t vsh, int64_t vsl,
                              const int32_t* block_idx, const int32_t* block_cnt, int causal, float scale, void* out,
                              int64_t osb, int64_t osh, int64_t osl, void* workspace, size_t workspace_bytes,
                              int* status, cudaStream_t stream) {
-  if (!q || !k || !v || !out || !block_idx || !block_cnt) return XATTN_B200_ERR_ARG;
+  if (!q || !k || !v || !out || (block_idx == nullptr) != (block_cnt == nullptr)) return XATTN_B200_ERR_ARG;
+  const bool dense = block_idx == nullptr;
   if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16) return XATTN_B200_ERR_ARG;
   if (head_dim != 128 || batch < 1 || hq < 1 || hkv < 1 || hq % hkv != 0 || q_len < 1 || k_len < 1)
     return XATTN_B200_ERR_ARG;
@@ -974,52 +907,54 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
   if (!(scale > 0.f)) return XATTN_B200_ERR_ARG;
   int rc;
   if ((rc = check_sm100())) return rc;
-  CUtensorMap tmQ, tmK, tmV, tmKf, tmVf;   // K/V as 64-key half tiles and as full 128-key tiles
+  CUtensorMap tmQ, tmK, tmV, tmO;
   if ((rc = make_qkv_map(&tmQ, q, q_len, hq, batch, qsb, qsh, qsl, 128))) return rc;
-  if ((rc = make_qkv_map(&tmK, k, k_len, hkv, batch, ksb, ksh, ksl, 64))) return rc;
-  if ((rc = make_qkv_map(&tmV, v, k_len, hkv, batch, vsb, vsh, vsl, 64))) return rc;
-  if ((rc = make_qkv_map(&tmKf, k, k_len, hkv, batch, ksb, ksh, ksl, 128))) return rc;
-  if ((rc = make_qkv_map(&tmVf, v, k_len, hkv, batch, vsb, vsh, vsl, 128))) return rc;
+  if ((rc = make_qkv_map(&tmK, k, k_len, hkv, batch, ksb, ksh, ksl, 128))) return rc;
+  if ((rc = make_qkv_map(&tmV, v, k_len, hkv, batch, vsb, vsh, vsl, 128))) return rc;
+  // the output: a store box is 32 rows of one 64-column half
+  if ((rc = make_qkv_map(&tmO, out, q_len, hq, batch, osb, osh, osl, 32, 1))) return rc;
   AttnParams p;
   p.batch = batch; p.hq = hq; p.hkv = hkv; p.q_len = q_len; p.k_len = k_len;
   p.q_blocks = (q_len + 127) / 128; p.list_k_blocks = (k_len + 127) / 128;
   p.causal = causal ? 1 : 0; p.is_bf16 = dtype == XATTN_B200_BF16 ? 1 : 0;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.osb = osb; p.osh = osh; p.osl = osl;
-  p.item_list = nullptr;
-  p.snake = 0;
-  if (cudaFuncSetAttribute(block_sparse_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem) !=
-      cudaSuccess)
-    return XATTN_B200_ERR_CUDA;
-  const long long items = static_cast<long long>(batch) * hq * p.q_blocks;
-  if (items > 0x7fffffffLL) return XATTN_B200_ERR_LIMIT;
-  p.total_items = static_cast<int>(items);
-  const int sms = sm_count();
-  const int grid = items < sms ? static_cast<int>(items) : sms;
-  if ((items + grid - 1) / grid > kSchedCap || p.list_k_blocks > 65534) return XATTN_B200_ERR_LIMIT;
+  p.tile_list = nullptr;
+  p.list_tiles = 0;
+  const int super_rows = (p.q_blocks + 1) / 2;
+  const long long units = static_cast<long long>(super_rows) * batch * hq;
+  if (units > 0x3fffffffLL || p.list_k_blocks > 65534) return XATTN_B200_ERR_LIMIT;
+  p.by_units = make_fast_div(causal ? batch * hq : super_rows * (hq / hkv));
+  p.by_hq = make_fast_div(hq);
+  p.by_batch = make_fast_div(batch);
+  p.by_group = make_fast_div(hq / hkv);
+  p.by_hkv = make_fast_div(hkv);
   const int32_t* rest = nullptr;
   const int* pair_header = nullptr;
   const int min_share = g_pair_min_share.load();
-  if (workspace && !causal) {
+  if (workspace && !dense && !causal) {
     if (workspace_bytes < order_workspace_bytes(batch, hq, q_len)) return XATTN_B200_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace) & 15) != 0) return XATTN_B200_ERR_ARG;
     int32_t* sorted = static_cast<int32_t*>(workspace);
-    attn_order_kernel<<<batch * hkv, kOrderThreads, 0, stream>>>(p, block_cnt, sorted);
+    attn_order_kernel<<<batch * hkv, kOrderThreads, 0, stream>>>(p, block_cnt, sm_count(), sorted);
     if ((rc = launch_status())) return rc;
-    p.item_list = sorted;
-    p.snake = 1;
-    return launch_dependent(block_sparse_attn_kernel, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tmQ, tmK, tmV,
-                            tmKf, tmVf, p, block_idx, block_cnt, static_cast<const int32_t*>(nullptr),
-                            static_cast<const int*>(nullptr), min_share, out, status);
-  }
-  if (workspace && pair_path_applies(hq, hkv, k_len)) {
-    if ((rc = block_sparse_attn_pair_launch(tmQ, tmKf, tmVf, p, block_idx, block_cnt, out, workspace, workspace_bytes,
+    p.tile_list = sorted;
+    p.list_tiles = static_cast<int>(2 * units);
+  } else if (workspace && !dense && pair_path_applies(hq, hkv, k_len)) {
+    if ((rc = block_sparse_attn_pair_launch(tmQ, tmK, tmV, p, block_idx, block_cnt, out, workspace, workspace_bytes,
                                             &rest, &pair_header, min_share, status, stream)))
       return rc;
   }
   // (a dependent launch in every case: after the pair kernel, or after whatever kernel produced the block lists)
-  return launch_dependent(block_sparse_attn_kernel, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tmQ, tmK, tmV,
-                          tmKf, tmVf, p, block_idx, block_cnt, rest, pair_header, min_share, out, status);
+  const long long sms = sm_count();
+  const unsigned grid = static_cast<unsigned>(rest && units > sms ? sms : units);
+  auto launch = [&](auto kern) -> int {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem) != cudaSuccess)
+      return XATTN_B200_ERR_CUDA;
+    return launch_dependent(kern, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tmQ, tmK,
+                            tmV, tmO, p, block_idx, block_cnt, rest, pair_header, min_share, status);
+  };
+  return p.is_bf16 ? launch(block_sparse_attn_kernel<true>) : launch(block_sparse_attn_kernel<false>);
 }
 
 }  // namespace xb

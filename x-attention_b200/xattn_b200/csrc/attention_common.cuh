@@ -11,15 +11,34 @@ namespace xb {
 constexpr int kTile16 = 128 * 128 * 2;     // one 128x128 16-bit tile = two 64-column TMA boxes
 constexpr int kHalf16 = kTile16 / 2;
 
+// Division of numbers below 2^31 by a divisor known on the host: a multiplication and a shift instead of the ~25
+// instructions of an integer division, which add up in code that every role of a kernel has to decode its work with.
+struct FastDiv {
+  uint32_t d, mul, shift;
+};
+static inline FastDiv make_fast_div(uint32_t d) {
+  FastDiv f;
+  f.d = d;
+  f.shift = 0;
+  while ((1ull << f.shift) < d) ++f.shift;
+  f.mul = static_cast<uint32_t>((((1ull << f.shift) - d) << 32) / d + 1);
+  return f;
+}
+__device__ __forceinline__ int fast_div(int n, const FastDiv& f, int& rem) {
+  const uint32_t q = (__umulhi(static_cast<uint32_t>(n), f.mul) + static_cast<uint32_t>(n)) >> f.shift;
+  rem = n - static_cast<int>(q * f.d);
+  return static_cast<int>(q);
+}
+
 struct AttnParams {
   int batch, hq, hkv, q_len, k_len;
   int q_blocks, list_k_blocks;
   int causal, is_bf16;
-  int total_items;
   float scale_log2;
   int64_t osb, osh, osl;
-  const int32_t* item_list;     // general kernel: its work items (null: all of them, 0 .. total_items - 1)
-  int snake;                    // general kernel: deal the items to the CTAs in alternating direction (sorted list)
+  FastDiv by_units, by_hq, by_batch, by_group, by_hkv;          // (general kernel: see unit_tile) hq, batch, hq / hkv, hkv
+  const int32_t* tile_list;     // general kernel: its tiles, two per unit (null: all, in their natural order)
+  int list_tiles;               // entries of that list
 };
 
 __device__ __forceinline__ uint32_t pack16(float lo, float hi, int is_bf16) {
@@ -30,6 +49,8 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi, int is_bf16) {
   __half2 v = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
+
+template <bool kBf16> __device__ __forceinline__ uint32_t pack16t(float lo, float hi) { return pack16(lo, hi, kBf16 ? 1 : 0); }
 
 // Development aid, compiled only with -DXB_TRACE: per-role timestamps of the first CTAs, written behind the
 // status word (which must then point to a device buffer of at least 64 + 16*14*XB_TRACE_CAP bytes).  Roles: 0/5

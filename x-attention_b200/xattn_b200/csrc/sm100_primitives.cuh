@@ -82,19 +82,26 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity
   return ok != 0;
 }
 // Bounded wait.  `abort_flag` lives in shared memory and is shared by all roles of the CTA.  Waiting threads
-// are suspended by the hardware in slices of at most 20 us, so co-resident warps keep their issue slots.
+// are suspended by the hardware in slices of at most 20 us, so co-resident warps keep their issue slots.  (Inlined at
+// dozens of places in kernels whose instruction footprint matters: a 32-bit clock is enough for limits below 2^32.)
+__device__ __forceinline__ uint32_t clock32() {
+  uint32_t c;
+  asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
+  return c;
+}
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  static_assert(kWaitCycleLimit > 0 && kWaitCycleLimit < (1LL << 32), "wait limit");
   if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
+  const uint32_t t0 = clock32();
 #pragma unroll 1
-  while (true) {
-    if (mbar_try_wait_hint(bar, parity, 20000u)) return true;
+  while (!mbar_try_wait_hint(bar, parity, 20000u)) {
     if (*abort_flag) return false;
-    if (clock64() - t0 > kWaitCycleLimit) {
+    if (clock32() - t0 > static_cast<uint32_t>(kWaitCycleLimit)) {
       *abort_flag = 1;
       return false;
     }
   }
+  return true;
 }
 
 // Bounded wait that polls without ever suspending the thread: for the single-thread roles (TMA issue, MMA
@@ -174,6 +181,29 @@ __device__ __forceinline__ void tma_prefetch_l2_5d(const CUtensorMap* m, int c0,
                : "memory");
 }
 
+// ------------------------------------------------------------------ cluster launch control (work stealing)
+// A running CTA asks for a CTA of the same grid that has not been launched yet and takes over its work: the grid has one
+// CTA per unit of work, the ones that fit run, and each then cancels further ones until a request is declined.  The
+// 16-byte answer arrives in shared memory and completes 16 bytes on the mbarrier.  After a declined request no other
+// may be made.
+__device__ __forceinline__ void clc_try_cancel(uint32_t dst, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(dst), "r"(bar) : "memory");
+}
+// blockIdx.x of the cancelled CTA, or -1 if the request was declined
+__device__ __forceinline__ int clc_answer(uint32_t src) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t.reg .b32 a, b, c;\n\t"
+      "ld.shared.b128 h, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "mov.b32 a, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {a, b, c, _}, h;\n\t"
+      "mov.b32 %0, a;\n\t}"
+      : "=r"(x) : "r"(src) : "memory");
+  return x;
+}
+
 // ------------------------------------------------------------------ tcgen05 / TMEM
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_result_addr, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result_addr), "r"(ncols)
@@ -213,6 +243,32 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// The same, to be executed by a converged warp of which the one thread with `lead` issues.  tcgen05 takes its operands
+// from uniform registers: inside a single-thread branch every descriptor has to be moved there word by word (measured:
+// 83 cycles per MMA, 100 per commit, as much as the MMA itself takes), in converged code they are computed there.
+__device__ __forceinline__ void mma_ss_lead(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                            uint32_t accumulate, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ts_lead(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                            uint32_t accumulate, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit_lead(uint32_t bar, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(bar), "r"(lead) : "memory");
+}
+
 // 32 lanes x 32 columns of 32-bit: thread t of the warp gets lane (base_lane + t), columns [col, col+32)
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -223,6 +279,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
         "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
 }

@@ -4,8 +4,8 @@ Reference: eval/HunyuanVideo/hyvideo/modules/attenion.py:132-166.  The sequence 
 [valid image+text tokens | padded text tail]; the two segments attend only within themselves
 (`cu_seqlens = [0, valid, total]`).  The valid segment goes through XAttention (non-causal; dense attention
 instead when threshold >= 1, which the model uses during its warm-up steps, models.py:211), the tail is dense.
-Both dense cases run through the block-sparse kernel with an all-ones block list, so no third-party attention
-package is involved.
+Both dense cases run through the same attention kernel without block lists, so no third-party attention package is
+involved.
 """
 from __future__ import annotations
 
@@ -15,12 +15,7 @@ from . import ops
 
 
 def _dense(q, k, v, out):
-    B, H, Lq, _ = q.shape
-    Lk = k.shape[2]
-    qb, kb = (Lq + 127) // 128, (Lk + 127) // 128
-    idx = torch.arange(kb, dtype=torch.int32, device=q.device).expand(B, H, qb, kb).contiguous()
-    cnt = torch.full((B, H, qb), kb, dtype=torch.int32, device=q.device)
-    ops.block_sparse_attention(q, k, v, idx, cnt, causal=False, out=out)
+    ops.block_sparse_attention(q, k, v, None, None, causal=False, out=out)
 
 
 def _xattn(q, k, v, out, threshold, stride):

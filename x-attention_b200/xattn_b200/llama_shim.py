@@ -6,7 +6,7 @@ RoPE and the cache update (which stay the model's business) its core is: repeat 
 (q_len == 1 against a longer cache) -> a dense single-query attention from a third-party package (:188-197).
 `attention_core` is that core for callers that hold q/k/v after RoPE: K/V are NOT repeated (the kernels read
 kv head h // (Hq/Hkv)), prefill goes to the sm_100a XAttention path, decode and the "full" metric run dense
-through the same block-sparse attention kernel with an all-ones block list.
+through the same attention kernel without block lists.
 
 `llama_attention_forward` / `patch_llama_attention` are the whole patch for Hugging Face's `LlamaAttention`
 (projections, in-place RoPE on the projection outputs, cache update, prefill or decode core, `o_proj` fed
@@ -55,13 +55,6 @@ def default_threshold_table(stride: int) -> torch.Tensor:
     return torch.from_numpy(z[f"fuse_{stride}"].copy())
 
 
-def _dense_lists(batch, heads, q_len, k_len, device):
-    qb, kb = (q_len + 127) // 128, (k_len + 127) // 128
-    idx = torch.arange(kb, dtype=torch.int32, device=device).expand(batch, heads, qb, kb).contiguous()
-    cnt = torch.full((batch, heads, qb), kb, dtype=torch.int32, device=device)
-    return idx, cnt
-
-
 def attention_core(query_states: torch.Tensor, key_states: torch.Tensor, value_states: torch.Tensor,
                    layer_idx: int, config: FastPrefillConfig) -> torch.Tensor:
     """q [B,Hq,q_len,D], k/v [B,Hkv,k_len,D] (after RoPE and the cache update) -> [B,Hq,q_len,D]."""
@@ -73,8 +66,7 @@ def attention_core(query_states: torch.Tensor, key_states: torch.Tensor, value_s
         return Xattention_prefill(query_states, key_states, value_states, config.stride, norm=1, threshold=thr,
                                   use_triton=True)
     # decode, or dense prefill: every key block that a row may see (token-level causal inside the kernel)
-    idx, cnt = _dense_lists(B, Hq, q_len, k_len, query_states.device)
-    return ops.block_sparse_attention(query_states, key_states, value_states, idx, cnt, causal=True)
+    return ops.block_sparse_attention(query_states, key_states, value_states, None, None, causal=True)
 
 
 def rope_and_attend(q_proj_out: torch.Tensor, k_proj_out: torch.Tensor, v_proj_out: torch.Tensor,

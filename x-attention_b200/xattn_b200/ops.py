@@ -246,15 +246,9 @@ def mask_to_lists(mask: torch.Tensor, q_len: int, k_len: int, causal: bool):
 
 
 # ------------------------------------------------------------------------------ phase 3
-# The split has fixed costs: the classify kernel (8 us) and the general kernel's pass over the rows the pair kernel
-# leaves (a few items per SM, each a full latency chain), against 8-12 % of the call won when 95 % of the blocks
-# qualify (Llama-3.1-8B at 128K tokens); and an attempt that the library declines costs 15-45 us (at 32K or 64K
-# tokens it does decline: 66 % / 89 % qualify).  Measured on 1 / 2 / 4 / 8 kv heads of the 128K-token layer (4096 /
-# 8192 / 16384 / 32768 items): general kernel alone 117 / 221 / 430 / 830 us, with the split 134 / 219 / 393 / 750.
-# So the scratch memory is offered by default only for sequences of at least 96K tokens (PAIR_MIN_K_BLOCKS key
-# blocks) and calls of at least PAIR_MIN_ITEMS (batch, query head, query block) items.
-PAIR_MIN_K_BLOCKS = 768
-PAIR_MIN_ITEMS = 12288
+# Causal calls are not offered scratch memory by default: the general kernel now loads K/V once for two query heads of a
+# kv group itself, and the split into two kernels no longer gains (Llama-3.1-8B at 128K tokens, where 95 % of the blocks
+# qualify for the pair kernel: 700 us with the split, 610 us without).
 # Non-causal calls: sorting the items by list length is one launch of a few microseconds; with only a few items per
 # SM there is nothing to balance.
 ORDER_MIN_ITEMS = 16 * 148
@@ -267,21 +261,21 @@ def pair_split_share(percent: Optional[int] = None) -> int:
     return int(_lib.load().xattn_b200_block_sparse_attn_split_share(-1 if percent is None else int(percent)))
 
 
-def block_sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, block_idx: torch.Tensor,
-                           block_cnt: torch.Tensor, causal: bool = True, scale: Optional[float] = None,
+def block_sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, block_idx: Optional[torch.Tensor],
+                           block_cnt: Optional[torch.Tensor], causal: bool = True, scale: Optional[float] = None,
                            out: Optional[torch.Tensor] = None, use_workspace: Optional[bool] = None) -> torch.Tensor:
     """q [B,Hq,Lq,128], k/v [B,Hkv,Lk,128] (bf16/fp16; fp32 is computed in bf16) -> [B,Hq,Lq,128], returned
     as a transposed view of [B,Lq,Hq,128] storage, like the reference's output (Xattention.py:392-394).
+    Without lists (block_idx and block_cnt None) the call is dense: every block that holds a visible key.
     `out`, if given, is a [B,Hq,Lq,128] tensor of the compute dtype (any strides, unit stride on the last
     dimension, 16-byte aligned rows) that receives the result instead.  `use_workspace=True` hands the library
     scratch memory (xattn_b200_block_sparse_attn_ws).  Causal calls: it may then send the rows whose kv group shares a
-    list of one or two blocks to the kernel that loads K/V once per group and treats both blocks in one softmax pass;
-    the library takes that route only when those rows list at least `pair_split_share()` per cent of the blocks,
-    which it finds out on the device, and a declined attempt costs 30-45 us, so by default (None) the memory is
-    offered only for sequences of at least PAIR_MIN_K_BLOCKS key blocks and calls of at least PAIR_MIN_ITEMS items.  Non-causal calls: the work items are sorted
-    by list length before they are dealt to the SMs (one small kernel); offered by default from ORDER_MIN_ITEMS
-    items on.  False: the general kernel alone, items in their natural order."""
-    _require_cuda(q, k, v, block_idx, block_cnt)
+    list of one or two blocks to a kernel of their own, provided those rows list at least `pair_split_share()` per cent
+    of the blocks, which it finds out on the device; by default (None) no memory is offered.  Non-causal calls: the
+    work is sorted by list length before it is handed to the SMs (one small kernel); offered by default from
+    ORDER_MIN_ITEMS items on.  False: the general kernel alone, work in its natural order."""
+    dense = block_idx is None and block_cnt is None
+    _require_cuda(q, k, v, *(() if dense else (block_idx, block_cnt)))
     lib = _lib.load()
     B, Hq, Lq, D = q.shape
     Hkv, Lk = k.shape[1], k.shape[2]
@@ -301,21 +295,22 @@ def block_sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bl
             raise ValueError("out must be a CUDA tensor [B,Hq,Lq,D] of the compute dtype with unit inner stride")
         out_view = out
     lqb, lkb = (Lq + 127) // 128, (Lk + 127) // 128
-    if tuple(block_idx.shape) != (B, Hq, lqb, lkb) or tuple(block_cnt.shape) != (B, Hq, lqb):
+    if not dense and (tuple(block_idx.shape) != (B, Hq, lqb, lkb) or tuple(block_cnt.shape) != (B, Hq, lqb)):
         raise ValueError("block lists have the wrong shape")
-    if use_workspace is None:
+    if dense:
+        use_workspace = False
+    elif use_workspace is None:
         forced = os.environ.get("XATTN_B200_ATTN_WORKSPACE")         # "0" / "1": overrides the rule (for measurements)
         if forced in ("0", "1"):
             use_workspace = forced == "1"
         else:
-            use_workspace = ((lkb >= PAIR_MIN_K_BLOCKS and B * Hq * lqb >= PAIR_MIN_ITEMS) if causal
-                             else B * Hq * lqb >= ORDER_MIN_ITEMS)
+            use_workspace = not causal and B * Hq * lqb >= ORDER_MIN_ITEMS
     ws_bytes = lib.xattn_b200_block_sparse_attn_workspace_bytes(B, Hq, Hkv, Lq, Lk) if use_workspace else 0
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device) if ws_bytes else None
     _lib.check(lib.xattn_b200_block_sparse_attn_ws(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), _DT[q.dtype], B, Hq, Hkv, Lq, Lk, D,
-        *_strides3(q), *_strides3(k), *_strides3(v), block_idx.contiguous().data_ptr(),
-        block_cnt.contiguous().data_ptr(), int(causal), scale, out_view.data_ptr(),
+        *_strides3(q), *_strides3(k), *_strides3(v), 0 if dense else block_idx.contiguous().data_ptr(),
+        0 if dense else block_cnt.contiguous().data_ptr(), int(causal), scale, out_view.data_ptr(),
         out_view.stride(0), out_view.stride(1), out_view.stride(2), ws.data_ptr() if ws is not None else 0, ws_bytes,
         _status(q.device).data_ptr(), _stream(q)), "block_sparse_attn")
     return out_view.to(in_dtype) if (in_dtype == torch.float32 and out is None) else out_view
