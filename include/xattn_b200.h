@@ -256,6 +256,20 @@ int xattn_b200_block_sparse_attn_ws(const void* q, const void* k, const void* v,
                                     void* out, int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_l,
                                     void* workspace, size_t workspace_bytes, int* status, void* cuda_stream);
 
+/*
+ * Decode step: dense attention of one query token per sequence (q [batch, hq, 1, 128]) against its key cache, which it may
+ * see completely.  Replaces the third-party single-query attention of the reference's Llama patch
+ * (xattn/src/load_llama.py:188-197); the same result as the general kernel up to the summation order.  hq / hkv <= 16
+ * (XATTN_B200_ERR_LIMIT otherwise: use xattn_b200_block_sparse_attn without lists).  The cache is split over the SMs; the
+ * parts are merged through `workspace` (device memory, 16-byte aligned, contents irrelevant on entry).
+ */
+size_t xattn_b200_decode_workspace_bytes(int batch, int hq, int hkv, int k_len);
+int xattn_b200_decode_attn(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv, int k_len,
+                           int head_dim, int64_t q_stride_b, int64_t q_stride_h, int64_t k_stride_b, int64_t k_stride_h,
+                           int64_t k_stride_l, int64_t v_stride_b, int64_t v_stride_h, int64_t v_stride_l, float scale,
+                           void* out, int64_t o_stride_b, int64_t o_stride_h, void* workspace, size_t workspace_bytes,
+                           int* status, void* cuda_stream);
+
 #ifdef __cplusplus
 }
 #endif

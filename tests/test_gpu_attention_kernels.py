@@ -1,4 +1,4 @@
-"""The attention kernel at the sizes where their tiling can go wrong, against plain fp32 attention."""
+"""The attention and decode kernels at the sizes where their tiling can go wrong, against plain fp32 attention."""
 import pytest
 import torch
 
@@ -27,6 +27,24 @@ def _close(got, want, scale=1.0):
 def _qkv(seed, b, hq, hkv, lq, lk, dtype=torch.bfloat16):
     g = torch.Generator().manual_seed(seed)
     return [torch.randn(b, h, n, 128, generator=g).to(dtype) for h, n in ((hq, lq), (hkv, lk), (hkv, lk))]
+
+
+@pytest.mark.parametrize("k_len", [1, 17, 63, 64, 65, 129, 1000, 4097])       # edges of a warp's 16 keys, of a stage, of a split
+@pytest.mark.parametrize("dtype,batch,hq,hkv", [(torch.bfloat16, 1, 8, 2), (torch.float16, 2, 7, 1), (torch.bfloat16, 1, 3, 3),
+                                                (torch.bfloat16, 1, 16, 1), (torch.bfloat16, 1, 17, 1)])
+def test_decode_step(k_len, dtype, batch, hq, hkv):
+    from xattn_b200 import ops
+    q, k, v = _qkv(k_len + hq, batch, hq, hkv, 1, k_len, dtype)
+    k[:, :, k_len // 2] *= 4.0                                               # a dominant key: the running maximum moves
+    cache = [torch.zeros(batch, hkv, k_len + 37, 128, dtype=dtype, device=DEV) for _ in range(2)]
+    for c, x in zip(cache, (k, v)):
+        c[:, :, :k_len] = x.to(DEV)
+    out = ops.decode_attention(q.to(DEV), cache[0][:, :, :k_len], cache[1][:, :, :k_len])     # a slice of a longer cache
+    assert out.shape == q.shape and out.dtype == dtype
+    rep = hq // hkv
+    want = torch.nn.functional.scaled_dot_product_attention(q.float(), k.float().repeat_interleave(rep, 1),
+                                                            v.float().repeat_interleave(rep, 1))
+    _close(out, want)
 
 
 @pytest.mark.parametrize("causal", [True, False])

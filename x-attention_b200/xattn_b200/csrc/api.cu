@@ -27,6 +27,11 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
                              int* status, cudaStream_t stream);
 size_t block_sparse_attn_workspace_bytes(int batch, int hq, int hkv, int q_len, int k_len);
 int pair_min_share_pct(int set_to);
+size_t decode_workspace_bytes(int batch, int hq, int hkv, int k_len);
+int decode_launch(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv, int k_len,
+                  int head_dim, int64_t qsb, int64_t qsh, int64_t ksb, int64_t ksh, int64_t ksl, int64_t vsb, int64_t vsh,
+                  int64_t vsl, float scale, void* out, int64_t osb, int64_t osh, void* workspace, size_t workspace_bytes,
+                  int* status, cudaStream_t stream);
 }  // namespace xb
 
 extern "C" {
@@ -166,6 +171,20 @@ int xattn_b200_block_sparse_attn_ws(const void* q, const void* k, const void* v,
                                       v_stride_l, block_idx, block_cnt, causal, scale, out, o_stride_b, o_stride_h,
                                       o_stride_l, workspace, workspace_bytes, status,
                                       static_cast<cudaStream_t>(cuda_stream));
+}
+
+size_t xattn_b200_decode_workspace_bytes(int batch, int hq, int hkv, int k_len) {
+  return xb::decode_workspace_bytes(batch, hq, hkv, k_len);
+}
+
+int xattn_b200_decode_attn(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv, int k_len,
+                           int head_dim, int64_t q_stride_b, int64_t q_stride_h, int64_t k_stride_b, int64_t k_stride_h,
+                           int64_t k_stride_l, int64_t v_stride_b, int64_t v_stride_h, int64_t v_stride_l, float scale,
+                           void* out, int64_t o_stride_b, int64_t o_stride_h, void* workspace, size_t workspace_bytes,
+                           int* status, void* cuda_stream) {
+  return xb::decode_launch(q, k, v, dtype, batch, hq, hkv, k_len, head_dim, q_stride_b, q_stride_h, k_stride_b, k_stride_h,
+                           k_stride_l, v_stride_b, v_stride_h, v_stride_l, scale, out, o_stride_b, o_stride_h, workspace,
+                           workspace_bytes, status, static_cast<cudaStream_t>(cuda_stream));
 }
 
 }  // extern "C"

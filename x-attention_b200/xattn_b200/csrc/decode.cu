@@ -1,0 +1,322 @@
+// Decode step: dense attention of ONE query token per sequence against its key cache.
+//
+// The reference runs it through a third-party single-query kernel (xattn/src/load_llama.py:188-197); the general
+// attention kernel here can compute it too, but as a 128-row tile with one valid row per head: a serial walk over the
+// cache on as many SMs as there are pairs of heads (128K tokens, 32 / 8 heads: 1.8 ms).
+//
+// The step reads K and V once and does next to nothing with them, so it is HBM-bound (128K tokens, 8 kv heads: 537 MB, 83 us
+// at the measured copy bandwidth; measured 95 us) or, for short caches, pure latency.  Therefore:
+//   * the cache is split along its length so that every SM has two CTAs' worth of it; a CTA streams its keys through a ring
+//     of TMA stages (64 keys of K and V, 32 KiB each), three stages per CTA = 192 KiB in flight per SM, which covers the
+//     HBM latency (6.5 TB/s x 1 us / 148 SMs = 44 KiB) several times over;
+//   * all query heads of a kv group are rows of one MMA (m16n8k16), so K and V are read once per kv head.  These are warp
+//     MMAs on purpose: with at most 16 useful rows a 128-row tcgen05 tile would be seven eighths padding, and the products
+//     take under a tenth of the time the bytes do;
+//   * every warp takes 16 keys of a stage and keeps a running softmax of its own; the four warps of a CTA are merged
+//     through shared memory at the end, the CTAs of a (batch, kv head) by a small second kernel (launched as a dependent
+//     one, so its launch latency runs under the first), or not at all when the cache needs no split.
+#include "attention_common.cuh"
+
+namespace xb {
+
+constexpr int kDecWarps = 4;
+constexpr int kDecThreads = kDecWarps * 32;
+constexpr int kDecKeys = 64;                              // keys per stage: 16 per warp
+constexpr int kDecTile = kDecKeys * 128 * 2;              // [2 column halves][64 keys][64 columns], 128-byte swizzle
+constexpr int kDecStages = 3;
+constexpr int kDecMaxRows = 16;                           // query heads per kv head
+constexpr int kDecSmem = kDecStages * 2 * kDecTile + 1024 /*alignment slack*/ + 256 /*barriers*/;
+constexpr float kDecRescale = 8.0f;                       // log2 units: the running maximum moves lazily
+
+struct DecodeParams {
+  int batch, hkv, group, k_len, splits, stages;           // stages: 64-key stages of the whole cache
+  float scale_log2;
+  int64_t qsb, qsh, osb, osh;
+};
+
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+template <bool kBf16>
+__device__ __forceinline__ void warp_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (kBf16)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// part: [batch * hkv][splits][group][128] un-normalised outputs, then [..][splits][group] (max, sum) pairs
+template <bool kBf16>
+__global__ void __launch_bounds__(kDecThreads, 2)
+decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                   const uint16_t* __restrict__ q, const DecodeParams p, float* __restrict__ part,
+                   float2* __restrict__ part_ml, uint16_t* __restrict__ out, int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kDecStages * 2 * kDecTile);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kDecStages);
+  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kDecStages);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int split = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
+  // stages [s0, s1) of the cache
+  const int s0 = static_cast<int>(static_cast<long long>(p.stages) * split / p.splits);
+  const int s1 = static_cast<int>(static_cast<long long>(p.stages) * (split + 1) / p.splits);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kDecStages; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, kDecWarps);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  pdl_launch_dependents();              // the merging kernel may take its place; it waits for this grid to end
+  auto load_stage = [&](int i) {        // one thread: the CTA's i-th stage
+    const int st = i % kDecStages;
+    const uint32_t dst = smem_u32(smem) + st * 2 * kDecTile;
+    mbar_expect_tx(full0 + 8 * st, 2 * kDecTile);
+    tma_load_5d(dst, &tmK, full0 + 8 * st, 0, (s0 + i) * kDecKeys, 0, g, b);
+    tma_load_5d(dst + kDecTile, &tmV, full0 + 8 * st, 0, (s0 + i) * kDecKeys, 0, g, b);
+  };
+  const int n = s1 - s0;
+  if (threadIdx.x == 0)
+    for (int i = 0; i < kDecStages && i < n; ++i) load_stage(i);
+
+  // Q as A operand: rows = query heads of the group (rows past it zero), 8 steps of 16 columns
+  uint32_t qa[8][4];
+  {
+    const int r0 = lane >> 2, c0 = (lane & 3) * 2;
+    const uint16_t* qg = q + b * p.qsb + static_cast<int64_t>(g) * p.group * p.qsh;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = r0 + 8 * (e & 1), c = c0 + 16 * k + 8 * (e >> 1);
+        qa[k][e] = r < p.group ? __ldg(reinterpret_cast<const uint32_t*>(qg + r * p.qsh + c)) : 0u;
+      }
+  }
+  float o[16][4];
+#pragma unroll
+  for (int t = 0; t < 16; ++t)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[t][e] = 0.f;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // rows lane / 4 and lane / 4 + 8
+  // ldmatrix addresses: lane's row inside the warp's 16 keys; chunk c of 16 bytes of row r sits at chunk c ^ (r & 7)
+  const int krow = warp * 16 + (lane & 7) + ((lane >> 4) << 3), kchunk = (lane >> 3) & 1;   // K: keys 0-7 | 8-15, columns 0-7 | 8-15
+  const int vrow = warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), vchunk = lane >> 4;   // V: the same, transposed on load
+  bool ok = true;
+  for (int i = 0; i < n; ++i) {
+    const int st = i % kDecStages;
+    if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * st, (i / kDecStages) & 1, abort_flag))) { ok = false; break; }
+    const uint32_t kt = smem_u32(smem) + st * 2 * kDecTile, vt = kt + kDecTile;
+    float s[2][4] = {};                                    // keys 0-7, 8-15 of the warp
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      uint32_t kb[4];
+      ldsm_x4(kt + (k >> 2) * (kDecTile / 2) + krow * 128 + (((((k & 3) << 1) | kchunk) ^ (krow & 7)) << 4), kb);
+      warp_mma<kBf16>(s[0], qa[k], kb[0], kb[1]);
+      warp_mma<kBf16>(s[1], qa[k], kb[2], kb[3]);
+    }
+    const int key0 = (s0 + i) * kDecKeys + warp * 16 + (lane & 3) * 2;
+    if ((s0 + i + 1) * kDecKeys > p.k_len) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (key0 + 8 * t + (e & 1) >= p.k_len) s[t][e] = -INFINITY;
+    }
+    float mx[2];
+    bool grow = false;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      mx[h] = fmaxf(fmaxf(s[0][2 * h], s[0][2 * h + 1]), fmaxf(s[1][2 * h], s[1][2 * h + 1]));
+      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2)) * p.scale_log2;
+      grow |= mx[h] > m[h] + kDecRescale;                  // (-inf + 8 is -inf: the first finite maximum counts)
+    }
+    if (__any_sync(0xffffffffu, grow)) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float mn = fmaxf(m[h], mx[h]);
+        const float alpha = m[h] == -INFINITY ? 0.f : fast_exp2(m[h] - mn);
+        m[h] = mn;
+        l[h] *= alpha;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+          o[t][2 * h] *= alpha;
+          o[t][2 * h + 1] *= alpha;
+        }
+      }
+    }
+    uint32_t pa[4];
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float mr = m[h] == -INFINITY ? 0.f : m[h];
+        const float p0 = fast_exp2(fmaf(s[t][2 * h], p.scale_log2, -mr)), p1 = fast_exp2(fmaf(s[t][2 * h + 1], p.scale_log2, -mr));
+        l[h] += p0 + p1;
+        pa[2 * t + h] = pack16t<kBf16>(p0, p1);
+      }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      uint32_t vb[4];
+      ldsm_x4_trans(vt + (c >> 2) * (kDecTile / 2) + vrow * 128 + (((((c & 3) << 1) | vchunk) ^ (vrow & 7)) << 4), vb);
+      warp_mma<kBf16>(o[2 * c], pa, vb[0], vb[1]);
+      warp_mma<kBf16>(o[2 * c + 1], pa, vb[2], vb[3]);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty0 + 8 * st);
+    if (threadIdx.x == 0 && i > 0 && i - 1 + kDecStages < n) {
+      // the stage before this one is refilled: by now every warp is done with it, or nearly
+      if (mbar_wait(empty0 + 8 * ((i - 1) % kDecStages), ((i - 1) / kDecStages) & 1, abort_flag)) load_stage(i - 1 + kDecStages);
+      else ok = false;
+    }
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    if (!ok) break;
+  }
+  // row sums over the four lanes of a row
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+  }
+  __syncthreads();                       // every stage has been read: the ring becomes the exchange buffer
+  if (*abort_flag) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000) { __nanosleep(1000); }      // let copies in flight land
+    if (threadIdx.x == 0 && status) atomicExch(status, static_cast<int>(kDevWaitTimeout));
+    return;
+  }
+  float* xo = reinterpret_cast<float*>(smem);                                    // [warp][16 rows][128]
+  float2* xml = reinterpret_cast<float2*>(smem + kDecWarps * kDecMaxRows * 128 * 4);     // [warp][16 rows]
+  {
+    const int r0 = lane >> 2, c0 = (lane & 3) * 2;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = r0 + 8 * h;
+      if (r < p.group) {
+#pragma unroll
+        for (int t = 0; t < 16; ++t)
+          *reinterpret_cast<float2*>(xo + (warp * kDecMaxRows + r) * 128 + t * 8 + c0) = make_float2(o[t][2 * h], o[t][2 * h + 1]);
+        if ((lane & 3) == 0) xml[warp * kDecMaxRows + r] = make_float2(m[h], l[h]);
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < p.group * 64; e += kDecThreads) {                // two columns of a row
+    const int r = e >> 6, c = (e & 63) * 2;
+    float mm = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kDecWarps; ++w) mm = fmaxf(mm, xml[w * kDecMaxRows + r].x);
+    float a0 = 0.f, a1 = 0.f, ll = 0.f;
+#pragma unroll
+    for (int w = 0; w < kDecWarps; ++w) {
+      const float2 ml = xml[w * kDecMaxRows + r];
+      const float f = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - mm);
+      const float2 v = *reinterpret_cast<const float2*>(xo + (w * kDecMaxRows + r) * 128 + c);
+      a0 += v.x * f;
+      a1 += v.y * f;
+      ll += ml.y * f;
+    }
+    if (p.splits == 1) {
+      const float inv = ll > 0.f ? 1.f / ll : 0.f;
+      *reinterpret_cast<uint32_t*>(out + b * p.osb + static_cast<int64_t>(g * p.group + r) * p.osh + c) =
+          pack16t<kBf16>(a0 * inv, a1 * inv);
+    } else {
+      const size_t row = (static_cast<size_t>(b * p.hkv + g) * p.splits + split) * p.group + r;
+      *reinterpret_cast<float2*>(part + row * 128 + c) = make_float2(a0, a1);
+      if (c == 0) part_ml[row] = make_float2(mm, ll);
+    }
+  }
+}
+
+// One CTA per (batch, query head), a thread per column: the splits' parts into the output.
+template <bool kBf16>
+__global__ void __launch_bounds__(128)
+decode_merge_kernel(const DecodeParams p, const float* __restrict__ part, const float2* __restrict__ part_ml,
+                    uint16_t* __restrict__ out) {
+  pdl_wait();
+  const int hq = p.hkv * p.group;
+  const int b = blockIdx.x / hq, h = blockIdx.x - b * hq;
+  const int g = h / p.group, r = h - g * p.group;
+  const size_t row0 = static_cast<size_t>(b * p.hkv + g) * p.splits * p.group + r;
+  float mm = -INFINITY;
+  for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, part_ml[row0 + static_cast<size_t>(s) * p.group].x);
+  float a = 0.f, ll = 0.f;
+#pragma unroll 8
+  for (int s = 0; s < p.splits; ++s) {
+    const size_t row = row0 + static_cast<size_t>(s) * p.group;
+    const float2 ml = part_ml[row];
+    const float f = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - mm);
+    a += part[row * 128 + threadIdx.x] * f;
+    ll += ml.y * f;
+  }
+  const float v = ll > 0.f ? a / ll : 0.f;
+  uint16_t* o = out + b * p.osb + h * p.osh + threadIdx.x;
+  *o = static_cast<uint16_t>(pack16t<kBf16>(v, 0.f));
+}
+
+// Number of splits: two CTAs per SM over all (batch, kv head) pairs, at least two stages each (a split costs a CTA's start
+// and its row of the merge, about what two stages take).
+static int decode_splits(int batch, int hkv, int k_len) {
+  const int stages = (k_len + kDecKeys - 1) / kDecKeys;
+  const long long heads = static_cast<long long>(batch) * hkv;
+  long long s = 2LL * sm_count() / heads;
+  if (s > stages / 2) s = stages / 2;
+  return s < 1 ? 1 : static_cast<int>(s);
+}
+
+size_t decode_workspace_bytes(int batch, int hq, int hkv, int k_len) {
+  if (batch < 1 || hq < 1 || hkv < 1 || hq % hkv != 0 || hq / hkv > kDecMaxRows || k_len < 1) return 0;
+  return static_cast<size_t>(batch) * hq * decode_splits(batch, hkv, k_len) * (128 * sizeof(float) + sizeof(float2));
+}
+
+int decode_launch(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv, int k_len,
+                  int head_dim, int64_t qsb, int64_t qsh, int64_t ksb, int64_t ksh, int64_t ksl, int64_t vsb, int64_t vsh,
+                  int64_t vsl, float scale, void* out, int64_t osb, int64_t osh, void* workspace, size_t workspace_bytes,
+                  int* status, cudaStream_t stream) {
+  if (!q || !k || !v || !out) return XATTN_B200_ERR_ARG;
+  if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16) return XATTN_B200_ERR_ARG;
+  if (head_dim != 128 || batch < 1 || hq < 1 || hkv < 1 || hq % hkv != 0 || k_len < 1 || !(scale > 0.f)) return XATTN_B200_ERR_ARG;
+  if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 3) || ((qsb | qsh | osb | osh) & 1)) return XATTN_B200_ERR_ARG;
+  if (hq / hkv > kDecMaxRows || hkv > 65535 || batch > 65535) return XATTN_B200_ERR_LIMIT;
+  int rc;
+  if ((rc = check_sm100())) return rc;
+  DecodeParams p;
+  p.batch = batch; p.hkv = hkv; p.group = hq / hkv; p.k_len = k_len;
+  p.stages = (k_len + kDecKeys - 1) / kDecKeys;
+  p.splits = decode_splits(batch, hkv, k_len);
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.qsb = qsb; p.qsh = qsh; p.osb = osb; p.osh = osh;
+  if (!workspace || workspace_bytes < decode_workspace_bytes(batch, hq, hkv, k_len)) return XATTN_B200_ERR_WORKSPACE;
+  if (reinterpret_cast<uintptr_t>(workspace) & 15) return XATTN_B200_ERR_ARG;
+  float* part = static_cast<float*>(workspace);
+  float2* part_ml = reinterpret_cast<float2*>(part + static_cast<size_t>(batch) * hq * p.splits * 128);
+  CUtensorMap tmK, tmV;
+  if ((rc = make_qkv_map(&tmK, k, k_len, hkv, batch, ksb, ksh, ksl, kDecKeys))) return rc;
+  if ((rc = make_qkv_map(&tmV, v, k_len, hkv, batch, vsb, vsh, vsl, kDecKeys))) return rc;
+  auto launch = [&](auto kern, auto merge) -> int {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem) != cudaSuccess)
+      return XATTN_B200_ERR_CUDA;
+    kern<<<dim3(p.splits, hkv, batch), kDecThreads, kDecSmem, stream>>>(tmK, tmV, static_cast<const uint16_t*>(q), p, part, part_ml,
+                                                                        static_cast<uint16_t*>(out), status);
+    int r = launch_status();
+    if (r || p.splits == 1) return r;
+    return launch_dependent(merge, dim3(batch * hq), dim3(128), 0, stream, p, static_cast<const float*>(part),
+                            static_cast<const float2*>(part_ml), static_cast<uint16_t*>(out));
+  };
+  return dtype == XATTN_B200_BF16 ? launch(decode_attn_kernel<true>, decode_merge_kernel<true>)
+                                  : launch(decode_attn_kernel<false>, decode_merge_kernel<false>);
+}
+
+}  // namespace xb

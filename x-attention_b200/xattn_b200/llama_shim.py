@@ -5,8 +5,8 @@ RoPE and the cache update (which stay the model's business) its core is: repeat 
 (:158-160), then prefill -> `Xattention_prefill` with the layer's per-head threshold row (:173-177), decode
 (q_len == 1 against a longer cache) -> a dense single-query attention from a third-party package (:188-197).
 `attention_core` is that core for callers that hold q/k/v after RoPE: K/V are NOT repeated (the kernels read
-kv head h // (Hq/Hkv)), prefill goes to the sm_100a XAttention path, decode and the "full" metric run dense
-through the same attention kernel without block lists.
+kv head h // (Hq/Hkv)), prefill goes to the sm_100a XAttention path, decode runs through a kernel of its own that
+splits the cache over the SMs, the "full" metric dense through the same attention kernel without block lists.
 
 `llama_attention_forward` / `patch_llama_attention` are the whole patch for Hugging Face's `LlamaAttention`
 (projections, in-place RoPE on the projection outputs, cache update, prefill or decode core, `o_proj` fed
@@ -65,7 +65,9 @@ def attention_core(query_states: torch.Tensor, key_states: torch.Tensor, value_s
         thr = config.threshold[layer_idx] if config.threshold.dim() == 2 else config.threshold
         return Xattention_prefill(query_states, key_states, value_states, config.stride, norm=1, threshold=thr,
                                   use_triton=True)
-    # decode, or dense prefill: every key block that a row may see (token-level causal inside the kernel)
+    if decoding:
+        return ops.decode_attention(query_states, key_states, value_states)
+    # dense prefill: every key block that a row may see (token-level causal inside the kernel)
     return ops.block_sparse_attention(query_states, key_states, value_states, None, None, causal=True)
 
 

@@ -314,3 +314,26 @@ def block_sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bl
         out_view.stride(0), out_view.stride(1), out_view.stride(2), ws.data_ptr() if ws is not None else 0, ws_bytes,
         _status(q.device).data_ptr(), _stream(q)), "block_sparse_attn")
     return out_view.to(in_dtype) if (in_dtype == torch.float32 and out is None) else out_view
+
+
+def decode_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Optional[float] = None) -> torch.Tensor:
+    """Dense attention of one query token per sequence: q [B,Hq,1,128] against the whole cache k/v [B,Hkv,Lk,128]
+    (bf16/fp16; fp32 is computed in bf16) -> [B,Hq,1,128], a transposed view of [B,1,Hq,128] storage."""
+    B, Hq, Lq, D = q.shape
+    Hkv, Lk = k.shape[1], k.shape[2]
+    if Lq != 1 or D != 128 or q.dtype not in _DT or Hq % Hkv or Hq // Hkv > 16:
+        return block_sparse_attention(q, k, v, None, None, True, scale)
+    _require_cuda(q, k, v)
+    if k.dtype != q.dtype or v.dtype != q.dtype:
+        raise TypeError("q/k/v must share one of bf16, fp16, fp32")
+    lib = _lib.load()
+    q, k, v = _aligned16(q), _aligned16(k), _aligned16(v)
+    ws_bytes = lib.xattn_b200_decode_workspace_bytes(B, Hq, Hkv, Lk)
+    out = torch.empty(B, 1, Hq, D, dtype=q.dtype, device=q.device)
+    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
+    ks, vs = k.stride(), v.stride()
+    _lib.check(lib.xattn_b200_decode_attn(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), _DT[q.dtype], B, Hq, Hkv, Lk, D, q.stride(0), q.stride(1), *ks[:3], *vs[:3],
+        1.0 / math.sqrt(D) if scale is None else float(scale), out.data_ptr(), Hq * D, D, ws.data_ptr(), ws_bytes,
+        _status(q.device).data_ptr(), _stream(q)), "decode_attn")
+    return out.transpose(1, 2)
