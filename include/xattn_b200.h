@@ -35,6 +35,8 @@ extern "C" {
 /* element types */
 #define XATTN_B200_BF16 0
 #define XATTN_B200_F16 1
+#define XATTN_B200_F32_TERMS 2   /* xattn_b200_estimate: rows of 3 * head_dim bf16 terms of fp32 values (xattn_b200_split_f32) */
+#define XATTN_B200_BF16_OUT_F32 3   /* xattn_b200_block_sparse_attn[_ws]: bf16 inputs, fp32 output */
 
 /* estimate semantics: which of the reference's two code paths to reproduce */
 #define XATTN_B200_SEMANTICS_TORCH 0  /* torch branch, xattn/src/Xattention.py:174-252 (what the reference runs on a B200) */
@@ -96,9 +98,9 @@ size_t xattn_b200_estimate_workspace_bytes_ex(int batch, int hq, int q_len, int 
  * q_len / k_len need not be multiples of `stride`: the tokens a ragged last stride group lacks count as the
  * zeros the reference pads with (xattn/src/Xattention.py:42-51); the library stages a zero-padded copy of the
  * one 128-row tile of Q (128- or 256-row tile of K) that holds that group in `workspace` -- a few MB instead
- * of a padded copy of the tensors (workspace sizes assume head_dim 128 for it).  head_dim is the
- * length of a row in elements, a multiple of 64 (it may exceed the model's head dimension when
- * rows carry split-precision terms, see xattn_b200_split_f32);  `scale` = 1/(sqrt(D)*stride*norm).
+ * of a padded copy of the tensors (workspace sizes assume head_dim 128 for it).  head_dim is a
+ * multiple of 64 (XATTN_B200_F32_TERMS: a row holds three times as many elements, and q_len and k_len are multiples of
+ * the stride);  `scale` = 1/(sqrt(D)*stride*norm).
  * attn_sums: float32 [batch, hq, q_blocks_pad, k_blocks_pad] (fully written).
  */
 int xattn_b200_estimate(const void* q, const void* k, int dtype, int batch, int hq, int hkv, int q_len, int k_len,
@@ -137,16 +139,16 @@ int xattn_b200_estimate_static(const void* q, const void* k, int dtype, int batc
                                float* attn_sums, int* status, void* cuda_stream);
 
 /*
- * Split fp32 rows into three bf16 terms (x = hi + mid + lo) laid out as rows of 6*head_dim so that
- * a bf16 GEMM over the widened rows reproduces the fp32 product to ~2^-24:
- *   role 0 (query side): [hi, hi, mid, hi, lo, mid]     role 1 (key side): [hi, mid, hi, lo, hi, mid]
- * x is [batch, heads, len_valid, head_dim] fp32 with element strides; out is contiguous
- * [batch, heads, len, 6*head_dim] bf16 with len >= len_valid, the rows past len_valid zero (the reference's
- * zero padding, xattn/src/Xattention.py:42-51).  No counterpart in the reference (its torch branch multiplies
+ * Split fp32 rows into three bf16 terms, x = hi + mid + lo to 2^-24, stored as rows [hi | mid | lo] of 3*head_dim
+ * (terms 3: what xattn_b200_estimate takes as XATTN_B200_F32_TERMS, its GEMM then adds the six products of terms that
+ * reach 2^-24), or hi alone (terms 1: the values rounded to bf16).
+ * x is [batch, heads, len_valid, head_dim] fp32 with element strides, head_dim a multiple of 8; out is contiguous
+ * [batch, heads, len, terms*head_dim] bf16 with len >= len_valid, 16-byte aligned, the rows past len_valid zero (the
+ * reference's zero padding, xattn/src/Xattention.py:42-51).  No counterpart in the reference (its torch branch multiplies
  * fp32 directly, xattn/src/Xattention.py:183).
  */
 int xattn_b200_split_f32(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t stride_b,
-                         int64_t stride_h, int64_t stride_l, int role, void* out, void* cuda_stream);
+                         int64_t stride_h, int64_t stride_l, int terms, void* out, void* cuda_stream);
 
 /*
  * Rotary position embedding, applied in place to the query and key projections in one launch.
@@ -221,7 +223,7 @@ int xattn_b200_mask_to_lists(const uint8_t* mask, int batch, int heads, int mask
  * out[b,h,i,:] = softmax_j(scale * q_i.k_j) v_j over keys j in kept blocks, and j <= i + (k_len-q_len)
  * when causal.  head_dim must be 128.  Rows with no visible key give zeros.
  * out has element strides (o_stride_b, o_stride_h, o_stride_l), unit stride along head_dim, same
- * dtype as the inputs.  block_idx and block_cnt NULL: a dense call, every block that holds a visible key is listed.
+ * dtype as the inputs, or fp32 when dtype is XATTN_B200_BF16_OUT_F32.  block_idx and block_cnt NULL: a dense call, every block that holds a visible key is listed.
  */
 int xattn_b200_block_sparse_attn(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv,
                                  int q_len, int k_len, int head_dim, int64_t q_stride_b, int64_t q_stride_h,

@@ -47,15 +47,9 @@ def xattn_estimate(
     always runs; which of the reference's two estimate variants it reproduces is set by
     ops.set_estimate_semantics.  K/V with fewer heads than Q (GQA) are accepted."""
     _check_modes(softmax, select_mode, kdb)
-    B, Hq, Lq, D = query_states.shape
-    Lk = key_states.shape[2]
-    assert Hq % key_states.shape[1] == 0
-    g = ops.geometry(Lq, Lk, chunk_size, stride, block_size)
-    sums = ops.estimate_block_sums(query_states, key_states, stride, block_size, chunk_size, float(norm),
-                                   bool(causal))
-    mask, _, _ = ops.select_blocks(sums, g["bpc"], g["block_offset"], threshold, bool(causal), True,
-                                   bool(keep_sink), bool(keep_recent))
-    return sums.to(query_states.dtype), mask
+    assert query_states.shape[1] % key_states.shape[1] == 0
+    return ops.estimate_and_select(query_states, key_states, stride, float(norm), threshold, block_size, bool(causal),
+                                   chunk_size, bool(keep_sink), bool(keep_recent))
 
 
 def find_blocks_chunked(input_tensor, current_index, threshold, num_to_choose, decoding: bool,
@@ -112,23 +106,7 @@ def Xattention_prefill(
     """Estimate -> select -> block-sparse attention (Xattention.py:302-402).  Returns [B, H, Lq, D] in the
     input dtype (a transposed view of [B, Lq, H, D] storage, as in the reference)."""
     _check_modes(True, "inverse", kdb)
-    B, Hq, Lq, D = query_states.shape
-    Lk = key_states.shape[2]
     assert block_size == 128
-    assert B == 1
-    if chunk_size is None:
-        chunk_size = ops.default_chunk_size(Lk)
-    dev = query_states.device
-    if key_states.device != dev:
-        key_states = key_states.to(dev)
-    if value_states.device != dev:
-        value_states = value_states.to(dev)
-    g = ops.geometry(Lq, Lk, chunk_size, stride, block_size)
-    # un-padded causal keys under the torch branch: the sums outside a row's own chunk are zero and are not kept
-    band = ops.band_applies(Lk, chunk_size, bool(causal))
-    sums = ops.estimate_block_sums(query_states, key_states, stride, block_size, chunk_size, float(norm),
-                                   bool(causal), band=band)
-    _, idx, cnt = ops.select_blocks(sums, g["bpc"], g["block_offset"], threshold, bool(causal), True,
-                                    bool(keep_sink), bool(keep_recent), list_shape=(Lq, Lk), want_mask=False,
-                                    band_k_blocks=g["kb"] if band else None)
-    return ops.block_sparse_attention(query_states, key_states, value_states, idx, cnt, bool(causal))
+    assert query_states.shape[0] == 1
+    return ops.prefill(query_states, key_states, value_states, stride, float(norm), threshold, block_size, bool(causal),
+                       chunk_size, bool(keep_sink), bool(keep_recent))

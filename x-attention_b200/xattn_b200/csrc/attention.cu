@@ -162,7 +162,8 @@ struct Units {
 };
 
 // kBf16: bf16 or fp16 (a template parameter: as a run-time switch every packed pair cost both conversions and a select).
-template <bool kBf16>
+// kOutF32: the output is written as fp32.
+template <bool kBf16, bool kOutF32>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -713,41 +714,76 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         const float l = s_l[(s * 2 + m) * 128 + r];
         inv = l > 0.f ? 1.f / l : 0.f;
       }
-      if (lane == 0) tma_store_wait_read();             // the staging tile's previous stores have read it
-      __syncwarp();
       const uint32_t tmem_o = tmem_base + 256 + s * 128 + lane_bits;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t pk[16];
-        if (n > 0) {
-          uint32_t v[32];
-          tmem_ld32(tmem_o + c * 32, v);
-          tc_wait_ld();
-#pragma unroll
-          for (int k = 0; k < 16; ++k)
-            pk[k] = pack16t<kBf16>(__uint_as_float(v[2 * k]) * inv, __uint_as_float(v[2 * k + 1]) * inv);
-        } else {                                        // an empty list: zeros
-#pragma unroll
-          for (int k = 0; k < 16; ++k) pk[k] = 0u;
-        }
-        uint8_t* row = stg + (c >> 1) * (32 * 128) + lane * 128;
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4)
-          *reinterpret_cast<uint4*>(row + (((((c & 1) << 2) | q4) ^ (lane & 7)) << 4)) =
-              make_uint4(pk[4 * q4], pk[4 * q4 + 1], pk[4 * q4 + 2], pk[4 * q4 + 3]);
-      }
-      if (n > 0) {
-        tc_fence_before();
-        mbar_arrive(bar(s, O_EMPTY));
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
+      if constexpr (kOutF32) {
         const int q_row0 = t.qb * 128 + quad * 32;      // first row of this warp
-        if (q_row0 < p.q_len) {
-          tma_store_5d(&tmO, smem_u32(stg), 0, q_row0, 0, t.h, t.b);
-          tma_store_5d(&tmO, smem_u32(stg + 32 * 128), 0, q_row0, 1, t.h, t.b);
-          tma_store_commit();
+        // 32 columns at a time through the two halves of the staging tile in turn
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v[32];
+          if (n > 0) {
+            tmem_ld32(tmem_o + c * 32, v);
+            tc_wait_ld();
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * inv);
+          } else {                                      // an empty list: zeros
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = 0u;
+          }
+          if (lane == 0) tma_store_wait_read_1();       // the half's previous store has read it
+          __syncwarp();
+          uint8_t* half = stg + (c & 1) * (32 * 128);
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4)
+            *reinterpret_cast<uint4*>(half + lane * 128 + ((q4 ^ (lane & 7)) << 4)) =
+                make_uint4(v[4 * q4], v[4 * q4 + 1], v[4 * q4 + 2], v[4 * q4 + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (q_row0 < p.q_len) tma_store_5d(&tmO, smem_u32(half), 0, q_row0, c, t.h, t.b);
+            tma_store_commit();
+          }
+        }
+        if (n > 0) {
+          tc_fence_before();
+          mbar_arrive(bar(s, O_EMPTY));
+        }
+      } else {
+        if (lane == 0) tma_store_wait_read();           // the staging tile's previous stores have read it
+        __syncwarp();
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
+          if (n > 0) {
+            uint32_t v[32];
+            tmem_ld32(tmem_o + c * 32, v);
+            tc_wait_ld();
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+              pk[k] = pack16t<kBf16>(__uint_as_float(v[2 * k]) * inv, __uint_as_float(v[2 * k + 1]) * inv);
+          } else {                                      // an empty list: zeros
+#pragma unroll
+            for (int k = 0; k < 16; ++k) pk[k] = 0u;
+          }
+          uint8_t* row = stg + (c >> 1) * (32 * 128) + lane * 128;
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4)
+            *reinterpret_cast<uint4*>(row + (((((c & 1) << 2) | q4) ^ (lane & 7)) << 4)) =
+                make_uint4(pk[4 * q4], pk[4 * q4 + 1], pk[4 * q4 + 2], pk[4 * q4 + 3]);
+        }
+        if (n > 0) {
+          tc_fence_before();
+          mbar_arrive(bar(s, O_EMPTY));
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          const int q_row0 = t.qb * 128 + quad * 32;    // first row of this warp
+          if (q_row0 < p.q_len) {
+            tma_store_5d(&tmO, smem_u32(stg), 0, q_row0, 0, t.h, t.b);
+            tma_store_5d(&tmO, smem_u32(stg + 32 * 128), 0, q_row0, 1, t.h, t.b);
+            tma_store_commit();
+          }
         }
       }
       if (threadIdx.x == 256) XB_TRACE_EV(0x44 + s, 0);
@@ -899,11 +935,12 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
                              int* status, cudaStream_t stream) {
   if (!q || !k || !v || !out || (block_idx == nullptr) != (block_cnt == nullptr)) return XATTN_B200_ERR_ARG;
   const bool dense = block_idx == nullptr;
-  if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16) return XATTN_B200_ERR_ARG;
+  if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16 && dtype != XATTN_B200_BF16_OUT_F32) return XATTN_B200_ERR_ARG;
+  const bool out_f32 = dtype == XATTN_B200_BF16_OUT_F32;
   if (head_dim != 128 || batch < 1 || hq < 1 || hkv < 1 || hq % hkv != 0 || q_len < 1 || k_len < 1)
     return XATTN_B200_ERR_ARG;
   if (causal && k_len < q_len) return XATTN_B200_ERR_ARG;
-  if ((reinterpret_cast<uintptr_t>(out) & 15) || (osl % 8) || (osh % 8) || (osb % 8)) return XATTN_B200_ERR_ARG;
+  if ((reinterpret_cast<uintptr_t>(out) & 15) || (osl % (out_f32 ? 4 : 8)) || (osh % (out_f32 ? 4 : 8)) || (osb % (out_f32 ? 4 : 8))) return XATTN_B200_ERR_ARG;
   if (!(scale > 0.f)) return XATTN_B200_ERR_ARG;
   int rc;
   if ((rc = check_sm100())) return rc;
@@ -911,12 +948,12 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
   if ((rc = make_qkv_map(&tmQ, q, q_len, hq, batch, qsb, qsh, qsl, 128))) return rc;
   if ((rc = make_qkv_map(&tmK, k, k_len, hkv, batch, ksb, ksh, ksl, 128))) return rc;
   if ((rc = make_qkv_map(&tmV, v, k_len, hkv, batch, vsb, vsh, vsl, 128))) return rc;
-  // the output: a store box is 32 rows of one 64-column half
-  if ((rc = make_qkv_map(&tmO, out, q_len, hq, batch, osb, osh, osl, 32, 1))) return rc;
+  // the output: a store box is 32 rows of 128 bytes, one of two (fp32: four) column parts
+  if ((rc = make_rows_map(&tmO, out, q_len, hq, batch, osb, osh, osl, 32, 1, out_f32 ? 4 : 2))) return rc;
   AttnParams p;
   p.batch = batch; p.hq = hq; p.hkv = hkv; p.q_len = q_len; p.k_len = k_len;
   p.q_blocks = (q_len + 127) / 128; p.list_k_blocks = (k_len + 127) / 128;
-  p.causal = causal ? 1 : 0; p.is_bf16 = dtype == XATTN_B200_BF16 ? 1 : 0;
+  p.causal = causal ? 1 : 0; p.is_bf16 = dtype != XATTN_B200_F16 ? 1 : 0;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.osb = osb; p.osh = osh; p.osl = osl;
   p.tile_list = nullptr;
@@ -940,7 +977,7 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
     if ((rc = launch_status())) return rc;
     p.tile_list = sorted;
     p.list_tiles = static_cast<int>(2 * units);
-  } else if (workspace && !dense && pair_path_applies(hq, hkv, k_len)) {
+  } else if (workspace && !dense && !out_f32 && pair_path_applies(hq, hkv, k_len)) {
     if ((rc = block_sparse_attn_pair_launch(tmQ, tmK, tmV, p, block_idx, block_cnt, out, workspace, workspace_bytes,
                                             &rest, &pair_header, min_share, status, stream)))
       return rc;
@@ -949,12 +986,13 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
   const long long sms = sm_count();
   const unsigned grid = static_cast<unsigned>(rest && units > sms ? sms : units);
   auto launch = [&](auto kern) -> int {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem) != cudaSuccess)
+    if (!allow_smem(kern, kAttnSmem))
       return XATTN_B200_ERR_CUDA;
     return launch_dependent(kern, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tmQ, tmK,
                             tmV, tmO, p, block_idx, block_cnt, rest, pair_header, min_share, status);
   };
-  return p.is_bf16 ? launch(block_sparse_attn_kernel<true>) : launch(block_sparse_attn_kernel<false>);
+  if (out_f32) return launch(block_sparse_attn_kernel<true, true>);
+  return p.is_bf16 ? launch(block_sparse_attn_kernel<true, false>) : launch(block_sparse_attn_kernel<false, false>);
 }
 
 }  // namespace xb

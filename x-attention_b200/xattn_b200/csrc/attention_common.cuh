@@ -77,19 +77,23 @@ template <int N, int kLaunchRegs> __device__ __forceinline__ void reg_set_from()
   if constexpr (N < kLaunchRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// [64 columns, rows, 2 column halves, heads, batch]: one box {64, rows, 2, 1, 1} brings `rows` x 128 columns
-// with a single TMA instruction, laid out as two 64-column swizzled halves one after the other (Q: 128 rows,
-// K/V: 64-key half tiles).
+// [128 bytes of columns, rows, column parts, heads, batch] of rows of 128 elements of `elem` bytes (2 or 4): one box
+// {128 bytes, `rows`, `parts`, 1, 1} moves `rows` rows of `parts` parts with a single TMA instruction, the parts one after
+// the other in shared memory (Q, K, V: both 64-column halves of 16-bit rows).
+static inline int make_rows_map(CUtensorMap* m, const void* base, int len, int heads, int batch, int64_t sb, int64_t sh,
+                                int64_t sl, uint32_t box_rows, uint32_t box_parts, int elem) {
+  const uint64_t cols = 128 / elem;
+  const uint64_t dims[5] = {cols, (uint64_t)len, (uint64_t)elem, (uint64_t)heads, (uint64_t)batch};
+  // a dimension of extent 1 never moves: give it a harmless valid stride
+  const uint64_t s_h = heads > 1 ? (uint64_t)sh * elem : 256, s_b = batch > 1 ? (uint64_t)sb * elem : 256;
+  const uint64_t str[4] = {(uint64_t)sl * elem, 128, s_h, s_b};
+  const uint32_t box[5] = {(uint32_t)cols, box_rows, box_parts, 1, 1};
+  return make_tmap(m, base, elem == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, box);
+}
 static inline int make_qkv_map(CUtensorMap* m, const void* base, int len, int heads, int batch, int64_t sb, int64_t sh,
                                int64_t sl, uint32_t box_rows, uint32_t box_halves = 2) {
-  const uint64_t dims[5] = {64, (uint64_t)len, 2, (uint64_t)heads, (uint64_t)batch};
-  // a dimension of extent 1 never moves: give it a harmless valid stride
-  const uint64_t s_h = heads > 1 ? (uint64_t)sh * 2 : 256, s_b = batch > 1 ? (uint64_t)sb * 2 : 256;
-  const uint64_t str[4] = {(uint64_t)sl * 2, 128, s_h, s_b};
-  const uint32_t box[5] = {64, box_rows, box_halves, 1, 1};
-  return make_tmap_16bit(m, base, 5, dims, str, box);
+  return make_rows_map(m, base, len, heads, batch, sb, sh, sl, box_rows, box_halves, 2);
 }
-
 
 // ---------------------------------------------------------------- split between the pair and the general kernel
 // Workspace header, in 32-bit words: [0] length of the pair list, [1] length of the list of items left to the

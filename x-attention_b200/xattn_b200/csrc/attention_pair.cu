@@ -580,8 +580,7 @@ int block_sparse_attn_pair_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK
   pair_classify_kernel<<<(units + 255) / 256, 256, 0, stream>>>(block_idx, block_cnt, p.batch, p.hq, p.hkv, p.q_blocks,
                                                                p.list_k_blocks, list, counter, rest);
   if ((rc = launch_status())) return rc;
-  if (cudaFuncSetAttribute(block_sparse_attn_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) !=
-      cudaSuccess)
+  if (!allow_smem(block_sparse_attn_pair_kernel, kPairSmem))
     return XATTN_B200_ERR_CUDA;
   const int sms = sm_count();
   const int grid = units < sms ? units : sms;

@@ -306,7 +306,7 @@ int decode_launch(const void* q, const void* k, const void* v, int dtype, int ba
   if ((rc = make_qkv_map(&tmK, k, k_len, hkv, batch, ksb, ksh, ksl, kDecKeys))) return rc;
   if ((rc = make_qkv_map(&tmV, v, k_len, hkv, batch, vsb, vsh, vsl, kDecKeys))) return rc;
   auto launch = [&](auto kern, auto merge) -> int {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem) != cudaSuccess)
+    if (!allow_smem(kern, kDecSmem))
       return XATTN_B200_ERR_CUDA;
     kern<<<dim3(p.splits, hkv, batch), kDecThreads, kDecSmem, stream>>>(tmK, tmV, static_cast<const uint16_t*>(q), p, part, part_ml,
                                                                         static_cast<uint16_t*>(out), status);

@@ -39,6 +39,7 @@ constexpr int kGemmSmem = kStages * kStageBytes + 1024 /*barriers*/ + 1024 /*ali
 struct EstGeom {
   int batch, hq, hkv;
   int S, d_chunks;             // K loop: S * d_chunks steps of 64 elements
+  int term_chunks;             // split fp32 rows: steps per term (0: plain rows); see k_columns
   int rows_total, cols_total;  // padded lengths / S
   int rows_valid, cols_valid;  // rows past rows_valid give zeros; causal: columns past cols_valid are hidden
   int rcs;                     // chunk_size / S
@@ -82,6 +83,20 @@ __host__ __device__ inline void row_bounds(const EstGeom& g, int i, int& lo, int
   lo = g.left_blank ? chunk_start : 0;
   hi = g.row_off + i;
   if (hi > g.cols_valid - 1) hi = g.cols_valid - 1;
+}
+
+// Columns of the A (query) and B (key) operands of step dc of a token.  Plain rows: the same 64-column chunk of both.
+// fp32 rows split into three bf16 terms [hi | mid | lo]: the six products hh, hm, mh, hl, lh, mm one after the other (the
+// three left out are below 2^-24 of the first), two bits per product naming the term of either side.
+__device__ __forceinline__ void k_columns(const EstGeom& g, int dc, int& a_col, int& b_col) {
+  if (g.term_chunks == 0) {
+    a_col = b_col = dc * kTileK;
+    return;
+  }
+  constexpr uint32_t kTermA = 0 | 0 << 2 | 1 << 4 | 0 << 6 | 2 << 8 | 1 << 10, kTermB = 0 | 1 << 2 | 0 << 4 | 2 << 6 | 0 << 8 | 1 << 10;
+  const int pair = dc / g.term_chunks, c = dc - pair * g.term_chunks;
+  a_col = ((kTermA >> (2 * pair) & 3) * g.term_chunks + c) * kTileK;
+  b_col = ((kTermB >> (2 * pair) & 3) * g.term_chunks + c) * kTileK;
 }
 
 // first column tile / first key block a row tile's scratch rows are indexed from
@@ -430,8 +445,10 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           mbar_expect_tx(full0 + 8 * s, stage_bytes);
           // (the tile that holds a ragged last stride group comes from its zero-padded staging copy)
           const bool qt = mt == g.q_tail_mt, kt = nt == g.k_tail_nt;
-          tma_load_5d(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, dc * kTileK, g.S - 1 - t, qt ? 0 : mt * kTileM, h, b);
-          tma_load_5d(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, dc * kTileK, t, kt ? 0 : nt * g.tile_n,
+          int ac, bc;
+          k_columns(g, dc, ac, bc);
+          tma_load_5d(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, ac, g.S - 1 - t, qt ? 0 : mt * kTileM, h, b);
+          tma_load_5d(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, bc, t, kt ? 0 : nt * g.tile_n,
                       h / group, b);
         }
       }
@@ -620,8 +637,10 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           const uint32_t full_even = mapa_shared(full0 + 8 * s, 0);
           if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * kPairStageBytes);
           const bool qt = mt == g.q_tail_mt, kt = nt == g.k_tail_nt;
-          tma_load_5d_pair(dstA, qt ? &tmQt : &tmQ, full_even, dc * kTileK, g.S - 1 - t, qt ? 0 : mt * kTileM, h, b);
-          tma_load_5d_pair(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, dc * kTileK, t,
+          int ac, bc;
+          k_columns(g, dc, ac, bc);
+          tma_load_5d_pair(dstA, qt ? &tmQt : &tmQ, full_even, ac, g.S - 1 - t, qt ? 0 : mt * kTileM, h, b);
+          tma_load_5d_pair(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, bc, t,
                            (kt ? 0 : nt * kTileN) + static_cast<int>(rank) * 128, h / group, b);
         }
       }
@@ -812,28 +831,49 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
   else out[0] = acc[0];
 }
 
-// x = hi + mid + lo in bf16; rows widened to 6*D (see the header).
-// Rows l >= len_valid are written as zeros (a length rounded up to the stride).
-__global__ void split_f32_kernel(const float* __restrict__ x, int heads, int len, int len_valid, int D, int64_t sb,
-                                 int64_t sh, int64_t sl, int role, __nv_bfloat16* __restrict__ out, size_t total) {
+// x = hi + mid + lo in bf16 (each the rounding of what the ones before it leave), stored as rows [hi | mid | lo] of
+// 3 * D, or hi alone (terms == 1: the plain rounding to bf16).  Rows l >= len_valid are written as zeros (a length
+// rounded up to the stride).  Eight elements per thread: two 16-byte loads, a 16-byte store per term.  HBM-bound: 4 bytes
+// read and 6 written per element; the GEMM picks the term of each K step by a tensor-map coordinate, where rows widened to
+// the six products' operands took 12 bytes per element (32 x 4096 x 128 q and k together: 198 -> 53 us).
+template <int kTerms>
+__global__ void __launch_bounds__(256)
+split_f32_kernel(const float* __restrict__ x, int heads, int len, int len_valid, int vecs, int64_t sb, int64_t sh, int64_t sl,
+                 uint4* __restrict__ out, size_t total) {
   for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < total;
        e += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const int d = static_cast<int>(e % D);
-    size_t rest = e / D;
+    const int d = static_cast<int>(e % vecs);
+    size_t rest = e / vecs;
     const int l = static_cast<int>(rest % len);
     rest /= len;
     const int h = static_cast<int>(rest % heads);
     const int b = static_cast<int>(rest / heads);
-    const float v = l < len_valid ? x[b * sb + h * sh + l * sl + d] : 0.f;
-    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-    const float r1 = v - __bfloat162float(hi);
-    const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
-    const __nv_bfloat16 lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
-    __nv_bfloat16* o = out + (e / D) * (6 * static_cast<size_t>(D)) + d;
-    if (role == 0) {
-      o[0] = hi; o[D] = hi; o[2 * D] = mid; o[3 * D] = hi; o[4 * D] = lo; o[5 * D] = mid;
+    float v[8];
+    if (l < len_valid) {
+      const float* row = x + b * sb + h * sh + l * sl + d * 8;
+      if (((reinterpret_cast<uintptr_t>(row) & 15) == 0)) {
+        const float4 a = __ldcs(reinterpret_cast<const float4*>(row)), c = __ldcs(reinterpret_cast<const float4*>(row) + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = row[k];
+      }
     } else {
-      o[0] = hi; o[D] = mid; o[2 * D] = hi; o[3 * D] = lo; o[4 * D] = hi; o[5 * D] = mid;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = 0.f;
+    }
+    uint4* o = out + (e / vecs) * (static_cast<size_t>(kTerms) * vecs) + d;
+#pragma unroll
+    for (int t = 0; t < kTerms; ++t) {
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const __nv_bfloat162 p = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+        w[k] = *reinterpret_cast<const uint32_t*>(&p);
+        v[2 * k] -= __low2float(p);
+        v[2 * k + 1] -= __high2float(p);
+      }
+      o[static_cast<size_t>(t) * vecs] = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
 }
@@ -897,6 +937,7 @@ static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int h
   g.scale_log2 = scale * 1.4426950408889634f;
   g.head_dim = head_dim;
   g.tab_n = 0;
+  g.term_chunks = 0;
   g.q_tail_mt = q_len % stride ? (q_len / stride) / kTileM : -1;
   g.k_tail_nt = k_len % stride ? (k_len / stride) / g.tile_n : -1;
   g.compact = g.left_blank;
@@ -963,7 +1004,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
                     int stride, int block_size, int chunk_size, float scale, int causal, int semantics,
                     float* attn_sums, void* workspace, size_t workspace_bytes, int* status, cudaStream_t stream) {
   if (!q || !k || !attn_sums) return XATTN_B200_ERR_ARG;
-  if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16) return XATTN_B200_ERR_ARG;
+  if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16 && dtype != XATTN_B200_F32_TERMS) return XATTN_B200_ERR_ARG;
   if (semantics != XATTN_B200_SEMANTICS_TORCH && semantics != XATTN_B200_SEMANTICS_TRITON &&
       semantics != XATTN_B200_SEMANTICS_TORCH_BAND)
     return XATTN_B200_ERR_ARG;
@@ -972,6 +1013,13 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   int rc = fill_geometry(batch, hq, hkv, q_len, k_len, head_dim, stride, block_size, chunk_size, scale, causal,
                          semantics, g);
   if (rc) return rc;
+  const bool split = dtype == XATTN_B200_F32_TERMS;
+  const uint64_t row_len = split ? 3 * (uint64_t)head_dim : (uint64_t)head_dim;
+  if (split) {
+    if (q_len % stride || k_len % stride) return XATTN_B200_ERR_ARG;       // (the split writes whole stride groups)
+    g.term_chunks = g.d_chunks;
+    g.d_chunks *= 6;
+  }
   const EstWorkspace w = workspace_layout(g);
   if (!workspace || workspace_bytes < w.total) return XATTN_B200_ERR_WORKSPACE;
   if ((rc = check_sm100())) return rc;
@@ -993,14 +1041,14 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // 5-D views [head_dim, S, len/S, heads, batch] whose second coordinate picks the token inside a stride group
   CUtensorMap tmQ, tmK;
   {
-    const uint64_t dims[5] = {(uint64_t)head_dim, (uint64_t)stride, (uint64_t)(q_len / stride), (uint64_t)hq,
+    const uint64_t dims[5] = {row_len, (uint64_t)stride, (uint64_t)(q_len / stride), (uint64_t)hq,
                               (uint64_t)batch};
     const uint64_t str[4] = {(uint64_t)qsl * 2, (uint64_t)qsl * 2 * stride, (uint64_t)qsh * 2, (uint64_t)qsb * 2};
     const uint32_t box[5] = {kTileK, 1, kTileM, 1, 1};
     if ((rc = make_tmap_16bit(&tmQ, q, 5, dims, str, box))) return rc;
   }
   {
-    const uint64_t dims[5] = {(uint64_t)head_dim, (uint64_t)stride, (uint64_t)(k_len / stride), (uint64_t)hkv,
+    const uint64_t dims[5] = {row_len, (uint64_t)stride, (uint64_t)(k_len / stride), (uint64_t)hkv,
                               (uint64_t)batch};
     const uint64_t str[4] = {(uint64_t)ksl * 2, (uint64_t)ksl * 2 * stride, (uint64_t)ksh * 2, (uint64_t)ksb * 2};
     const uint32_t box[5] = {kTileK, 1, (uint32_t)g.tile_n, 1, 1};
@@ -1008,8 +1056,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   }
 
   // up to 64 KiB of dynamic shared memory (8192 row tiles): above the 48 KiB a kernel gets without asking
-  if (cudaFuncSetAttribute(est_setup_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * sizeof(int) * 8192) !=
-      cudaSuccess)
+  if (!allow_smem(est_setup_kernel, 2 * sizeof(int) * 8192))
     return XATTN_B200_ERR_CUDA;
   // CTA pairs (256x256 tiles) when tiles are 256 columns wide and the two row tiles of a pair see about the
   // same columns (always, except when a 128-row chunk of the torch branch blanks everything left of it)
@@ -1095,15 +1142,15 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   if (use_pairs) {
     CUtensorMap tmKh;                     // K with a box of 128 rows: one CTA's half of a 256-column tile
     {
-      const uint64_t dims[5] = {(uint64_t)head_dim, (uint64_t)stride, (uint64_t)(k_len / stride), (uint64_t)hkv,
+      const uint64_t dims[5] = {row_len, (uint64_t)stride, (uint64_t)(k_len / stride), (uint64_t)hkv,
                                 (uint64_t)batch};
       const uint64_t str[4] = {(uint64_t)ksl * 2, (uint64_t)ksl * 2 * stride, (uint64_t)ksh * 2, (uint64_t)ksb * 2};
       const uint32_t box[5] = {kTileK, 1, 128, 1, 1};
       if ((rc = make_tmap_16bit(&tmKh, k, 5, dims, str, box))) return rc;
     }
-    const uint32_t idesc2 = make_idesc_f16(2 * kTileM, kTileN, dtype == XATTN_B200_BF16, false, false);
+    const uint32_t idesc2 = make_idesc_f16(2 * kTileM, kTileN, dtype != XATTN_B200_F16, false, false);
     auto launch_pair = [&](auto kern) -> int {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) != cudaSuccess)
+      if (!allow_smem(kern, kPairSmem))
         return XATTN_B200_ERR_CUDA;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1), 1, 1);
@@ -1118,9 +1165,11 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       // every pair must be resident at once (persistent kernel): shrink the grid to what the device can hold
-      int max_clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg) != cudaSuccess || max_clusters < 1)
-        return XATTN_B200_ERR_CUDA;
+      const int max_clusters = once_per_device(reinterpret_cast<const void*>(kern), [&]() {
+        int m = 0;
+        return cudaOccupancyMaxActiveClusters(&m, kern, &cfg) == cudaSuccess ? m : 0;
+      });
+      if (max_clusters < 1) return XATTN_B200_ERR_CUDA;
       if (static_cast<unsigned>(2 * max_clusters) < cfg.gridDim.x) cfg.gridDim.x = 2 * max_clusters;
       if (cudaLaunchKernelEx(&cfg, kern, tmQ, tmKh, tmQt, tmKt, g, (const int*)pair_lo, (const int*)pair_prefix,
                              partial, mtile, idesc2, status) != cudaSuccess)
@@ -1136,10 +1185,10 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     }
     if (rc) return rc;
   } else {
-  const uint32_t idesc = make_idesc_f16(kTileM, g.tile_n, dtype == XATTN_B200_BF16, false, false);
+  const uint32_t idesc = make_idesc_f16(kTileM, g.tile_n, dtype != XATTN_B200_F16, false, false);
   const int grid = sms;
   auto launch = [&](auto kern) -> int {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem) != cudaSuccess)
+    if (!allow_smem(kern, kGemmSmem))
       return XATTN_B200_ERR_CUDA;
     kern<<<grid, kGemmThreads, kGemmSmem, stream>>>(tmQ, tmK, tmQt, tmKt, g, tile_lo, tile_prefix, partial, mtile,
                                                     attn_sums, idesc, status);
@@ -1195,17 +1244,19 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
 }
 
 int split_f32_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
-                     int64_t sl, int role, void* out, cudaStream_t stream) {
-  if (!x || !out || batch < 1 || heads < 1 || len < 1 || len_valid < 1 || len_valid > len || head_dim < 1 ||
-      (role != 0 && role != 1))
+                     int64_t sl, int terms, void* out, cudaStream_t stream) {
+  if (!x || !out || batch < 1 || heads < 1 || len < 1 || len_valid < 1 || len_valid > len || head_dim < 8 || head_dim % 8 ||
+      (terms != 1 && terms != 3) || (reinterpret_cast<uintptr_t>(out) & 15))
     return XATTN_B200_ERR_ARG;
-  const size_t total = static_cast<size_t>(batch) * heads * len * head_dim;
+  const size_t total = static_cast<size_t>(batch) * heads * len * (head_dim / 8);
   const int block = 256;
   size_t blocks = (total + block - 1) / block;
   if (blocks > 148 * 32) blocks = 148 * 32;
-  split_f32_kernel<<<static_cast<int>(blocks), block, 0, stream>>>(x, heads, len, len_valid, head_dim, sb, sh, sl, role,
-                                                                    static_cast<__nv_bfloat16*>(out), total);
-  return launch_status();
+  auto launch = [&](auto kern) -> int {
+    kern<<<static_cast<int>(blocks), block, 0, stream>>>(x, heads, len, len_valid, head_dim / 8, sb, sh, sl, static_cast<uint4*>(out), total);
+    return launch_status();
+  };
+  return terms == 3 ? launch(split_f32_kernel<3>) : launch(split_f32_kernel<1>);
 }
 
 }  // namespace xb

@@ -28,10 +28,10 @@ inline EncodeTiledFn get_encode_tiled() {
   return fn;
 }
 
-// 16-bit tensor seen as up to 5 dimensions, innermost first.  `strides_bytes` has rank-1 entries
+// Tensor seen as up to 5 dimensions, innermost first.  `strides_bytes` has rank-1 entries
 // (the innermost stride is one element).  128-byte swizzle, zero fill outside the tensor.
-inline int make_tmap_16bit(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
-                           const uint64_t* strides_bytes, const uint32_t* box) {
+inline int make_tmap(CUtensorMap* map, const void* base, CUtensorMapDataType type, int rank, const uint64_t* dims,
+                     const uint64_t* strides_bytes, const uint32_t* box) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return XATTN_B200_ERR_CUDA;
   if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return XATTN_B200_ERR_ARG;
@@ -48,25 +48,66 @@ inline int make_tmap_16bit(CUtensorMap* map, const void* base, int rank, const u
       gstr[i - 1] = strides_bytes[i - 1];
     }
   }
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, static_cast<cuuint32_t>(rank), const_cast<void*>(base),
+  CUresult r = enc(map, type, static_cast<cuuint32_t>(rank), const_cast<void*>(base),
                    gdim, gstr, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? XATTN_B200_OK : XATTN_B200_ERR_CUDA;
 }
 
-inline int check_sm100() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return XATTN_B200_ERR_CUDA;
-  int major = 0;
-  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return XATTN_B200_ERR_CUDA;
-  return major == 10 ? XATTN_B200_OK : XATTN_B200_ERR_ARCH;
+inline int make_tmap_16bit(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
+                           const uint32_t* box) {
+  return make_tmap(map, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, dims, strides_bytes, box);
 }
 
+// What has to be set up or asked once per kernel and device, and costs microseconds of every call otherwise: `ask` runs at
+// the first use (its positive answer is kept; a failure is not).  A few dozen kernels and up to 16 devices; safe to use
+// from several threads (two may ask at once, and get the same answer).
+template <typename F>
+inline int once_per_device(const void* kernel, F&& ask) {
+  struct Slot {
+    std::atomic<const void*> key{nullptr};
+    std::atomic<int> answer[16] = {};
+  };
+  static Slot slots[128];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 0;
+  if (dev >= 16) return ask();
+  for (size_t i = (reinterpret_cast<uintptr_t>(kernel) >> 4) % 128, n = 0; n < 128; ++n, i = (i + 1) % 128) {
+    const void* k = slots[i].key.load(std::memory_order_acquire);
+    if (k == nullptr && slots[i].key.compare_exchange_strong(k, kernel)) k = kernel;
+    if (k != kernel) continue;
+    int a = slots[i].answer[dev].load(std::memory_order_acquire);
+    if (a <= 0) {
+      a = ask();
+      if (a > 0) slots[i].answer[dev].store(a, std::memory_order_release);
+    }
+    return a;
+  }
+  return ask();
+}
+inline int check_sm100() {
+  static const char key = 0;
+  const int major = once_per_device(&key, [] {
+    int dev = 0, m = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    return cudaDeviceGetAttribute(&m, cudaDevAttrComputeCapabilityMajor, dev) == cudaSuccess ? m : 0;
+  });
+  return major == 10 ? XATTN_B200_OK : (major > 0 ? XATTN_B200_ERR_ARCH : XATTN_B200_ERR_CUDA);
+}
 inline int sm_count() {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  static const char key = 0;
+  const int n = once_per_device(&key, [] {
+    int dev = 0, m = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? m : 0;
+  });
   return n > 0 ? n : 148;
+}
+// lets `kernel` take `bytes` of dynamic shared memory on the current device
+template <typename K>
+inline bool allow_smem(K kernel, size_t bytes) {
+  return once_per_device(reinterpret_cast<const void*>(kernel), [&]() {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) == cudaSuccess ? 1 : 0;
+  }) > 0;
 }
 
 // Kernel launches issued by this library in this process (every launcher calls launch_status() right after its

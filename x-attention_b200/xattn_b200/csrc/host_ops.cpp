@@ -1,0 +1,455 @@
+// Tensor plumbing of the Python layer, in C++: argument checks, device memory, streams, and the calls of the C ABI.
+//
+// A short call (a decode step, the prefill of a chat prompt) is bound by the host: in Python its plumbing took 40 to 100 us,
+// against 8 to 60 us of kernels.  These functions do the same work in a few microseconds.  They are plain CPython functions
+// on torch tensors, no operator registration and no dispatch; all of them enqueue on torch's current stream and return.
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <cmath>
+#include <cstdlib>
+#include <optional>
+
+#include "../../../include/xattn_b200.h"
+
+namespace {
+
+using at::Tensor;
+
+PyObject* g_error = nullptr;        // XattnB200Error
+PyObject* g_status_of = nullptr;    // device index -> address of the device's status word
+int* g_status[64] = {};
+
+[[noreturn]] void fail(PyObject* type, const char* text) {
+  PyErr_SetString(type, text);
+  throw python_error();
+}
+void check(int code, const char* what) {
+  if (code == 0) return;
+  PyErr_Format(g_error, "%s: %s (status %d)", what, xattn_b200_error_string(code), code);
+  throw python_error();
+}
+
+// ---------------------------------------------------------------------------------------------- arguments
+struct Args {
+  PyObject* const* v;
+  Py_ssize_t n;
+  const char* name;
+  void count(Py_ssize_t want) const {
+    if (n != want) {
+      PyErr_Format(PyExc_TypeError, "%s: %zd arguments, %zd wanted", name, n, want);
+      throw python_error();
+    }
+  }
+  const Tensor& tensor(int i) const {
+    if (!THPVariable_Check(v[i])) fail(PyExc_TypeError, "a tensor is wanted");
+    return THPVariable_Unpack(v[i]);
+  }
+  bool none(int i) const { return v[i] == Py_None; }
+  long long integer(int i) const {
+    const long long x = PyLong_AsLongLong(v[i]);
+    if (x == -1 && PyErr_Occurred()) throw python_error();
+    return x;
+  }
+  double real(int i) const {
+    const double x = PyFloat_AsDouble(v[i]);
+    if (x == -1.0 && PyErr_Occurred()) throw python_error();
+    return x;
+  }
+  bool flag(int i) const {
+    const int x = PyObject_IsTrue(v[i]);
+    if (x < 0) throw python_error();
+    return x != 0;
+  }
+};
+
+void need_cuda(const Tensor& t) {
+  if (!t.is_cuda()) fail(g_error, "xattn_b200 ops need CUDA tensors: there is no CPU path");
+}
+void need_4d(const Tensor& t) {
+  if (t.dim() != 4) fail(PyExc_ValueError, "tensors of four dimensions [batch, heads, length, head_dim] are wanted");
+}
+// unit inner stride, 16-byte aligned rows; otherwise a contiguous copy
+Tensor aligned16(const Tensor& x) {
+  const int64_t e = x.element_size();
+  const bool ok = x.stride(3) == 1 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 &&
+                  (x.stride(0) * e) % 16 == 0 && (x.stride(1) * e) % 16 == 0 && (x.stride(2) * e) % 16 == 0;
+  return ok ? x : x.contiguous();
+}
+Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Device& dev) {
+  return at::detail::empty_cuda(sizes, type, dev, std::nullopt);
+}
+
+// Where a call runs: the tensors' device, torch's current stream of it, the device's status word.
+struct Place {
+  c10::cuda::CUDAGuard guard;
+  at::Device dev;
+  void* stream;
+  int* status;
+  explicit Place(const Tensor& t) : guard(t.device()), dev(t.device()) {
+    const int i = dev.index();
+    stream = c10::cuda::getCurrentCUDAStream(i).stream();
+    if (i < 0 || i >= 64) fail(g_error, "device index out of range");
+    if (!g_status[i]) {
+      PyObject* r = PyObject_CallFunction(g_status_of, "i", i);
+      if (!r) throw python_error();
+      g_status[i] = static_cast<int*>(PyLong_AsVoidPtr(r));
+      Py_DECREF(r);
+      if (!g_status[i]) throw python_error();
+    }
+    status = g_status[i];
+  }
+};
+
+int dtype_code(at::ScalarType t) {
+  return t == at::kBFloat16 ? XATTN_B200_BF16 : (t == at::kHalf ? XATTN_B200_F16 : -1);
+}
+
+// ---------------------------------------------------------------------------------------------- phases
+struct Geometry {
+  int lq, lk, qb, kb, q_chunks, k_chunks, bpc, block_offset;
+};
+Geometry geometry(int64_t q_len, int64_t k_len, int chunk, int stride, int block) {
+  Geometry g;
+  check(xattn_b200_estimate_geometry(static_cast<int>(q_len), static_cast<int>(k_len), chunk, stride, block,
+                                     reinterpret_cast<int*>(&g)),
+        "estimate_geometry");
+  return g;
+}
+
+// An operand of the estimate: 16-bit rows, or fp32 rows split into three bf16 terms each.
+struct Operand {
+  Tensor t;               // [B, H, len, D] (fp32: [B, H, len rounded up to the stride, 3 D] terms)
+  int64_t len;
+  int dtype;
+};
+Operand split_f32(const Tensor& x, int stride, const Place& at_) {
+  const Tensor r = x.stride(3) == 1 ? x : x.contiguous();
+  const int64_t len = (x.size(2) + stride - 1) / stride * stride, D = x.size(3);
+  Operand o;
+  o.t = empty({x.size(0), x.size(1), len, 3 * D}, at::kBFloat16, at_.dev);
+  o.len = len;
+  o.dtype = XATTN_B200_F32_TERMS;
+  check(xattn_b200_split_f32(static_cast<const float*>(r.data_ptr()), x.size(0), x.size(1), len, x.size(2), D, r.stride(0),
+                             r.stride(1), r.stride(2), 3, o.t.data_ptr(), at_.stream),
+        "split_f32");
+  return o;
+}
+Operand operand(const Tensor& x, int stride, bool f32, const Place& at_) {
+  if (f32) return split_f32(x.scalar_type() == at::kFloat ? x : x.to(at::kFloat), stride, at_);
+  Operand o;
+  o.dtype = dtype_code(x.scalar_type());
+  o.len = x.size(2);
+  o.t = aligned16(x);
+  return o;
+}
+
+struct EstimateArgs {
+  int stride, block, chunk, semantics;
+  double norm;
+  bool causal, band;
+};
+// fp32 block sums [B, Hq, q_blocks_pad, k_blocks_pad or blocks_per_chunk]
+Tensor estimate(Operand& q, Operand& k, int64_t D, const Geometry& g, const EstimateArgs& a, const Place& at_) {
+  const int64_t B = q.t.size(0), Hq = q.t.size(1), Hkv = k.t.size(1);
+  // (the staging tiles of ragged lengths are sized for head_dim 128)
+  if (q.dtype != XATTN_B200_F32_TERMS && D != 128)
+    for (Operand* o : {&q, &k})
+      if (o->len % a.stride) {
+        o->t = at::constant_pad_nd(o->t, {0, 0, 0, a.stride - o->len % a.stride});
+        o->len = o->t.size(2);
+      }
+  const int sem = a.band ? XATTN_B200_SEMANTICS_TORCH_BAND : a.semantics;
+  const size_t bytes = xattn_b200_estimate_workspace_bytes_ex(B, Hq, q.len, k.len, a.stride, a.block, a.chunk, a.causal, sem);
+  if (bytes == 0)
+    fail(PyExc_ValueError, "unsupported estimate geometry (stride must be 4/8/16/32, block_size 128, chunk_size a multiple of 128)");
+  const Tensor ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
+  Tensor sums = empty({B, Hq, g.qb, a.band ? g.bpc : g.kb}, at::kFloat, at_.dev);
+  const double scale = 1.0 / std::sqrt(static_cast<double>(D)) / a.stride / a.norm;
+  check(xattn_b200_estimate(q.t.data_ptr(), k.t.data_ptr(), q.dtype, B, Hq, Hkv, q.len, k.len, D, q.t.stride(0), q.t.stride(1),
+                            q.t.stride(2), k.t.stride(0), k.t.stride(1), k.t.stride(2), a.stride, a.block, a.chunk,
+                            static_cast<float>(scale), a.causal, sem, static_cast<float*>(sums.data_ptr()), ws.data_ptr(), bytes,
+                            at_.status, at_.stream),
+        "estimate");
+  return sums;
+}
+
+struct Selection {
+  Tensor mask, idx, cnt;
+};
+struct SelectArgs {
+  int bpc, block_offset;
+  bool causal, cleanup, sink, recent, want_mask;
+  int64_t list_q, list_k;       // 0: no lists
+  int64_t band_kb;              // > 0: the sums are the chunk band of rows of that many key blocks
+};
+Selection select(const Tensor& sums, PyObject* threshold, const SelectArgs& a, const Place& at_) {
+  const int64_t B = sums.size(0), H = sums.size(1), QB = sums.size(2), KB = a.band_kb > 0 ? a.band_kb : sums.size(3);
+  if (a.band_kb > 0 && sums.size(3) != a.bpc) fail(PyExc_ValueError, "band sums must have blocks_per_chunk columns");
+  Tensor thr;
+  double value = 0.0;
+  if (THPVariable_Check(threshold)) {
+    thr = THPVariable_Unpack(threshold).detach();
+    if (thr.device() != at_.dev || thr.scalar_type() != at::kFloat) thr = thr.to(at_.dev, at::kFloat);
+    thr = thr.reshape({-1}).contiguous();
+    if (thr.numel() != H) fail(PyExc_ValueError, "per-head threshold needs one entry per head");
+  } else {
+    value = PyFloat_AsDouble(threshold);
+    if (value == -1.0 && PyErr_Occurred()) throw python_error();
+  }
+  Selection r;
+  if (a.want_mask) r.mask = empty({B, H, QB, KB}, at::kBool, at_.dev);
+  const int64_t lqb = (a.list_q + 127) / 128, lkb = (a.list_k + 127) / 128;
+  if (a.list_q > 0) {
+    r.idx = empty({B, H, lqb, lkb}, at::kInt, at_.dev);
+    r.cnt = empty({B, H, lqb}, at::kInt, at_.dev);
+  }
+  auto fn = a.band_kb > 0 ? xattn_b200_select_band : xattn_b200_select;
+  check(fn(static_cast<const float*>(sums.data_ptr()), B, H, QB, KB, a.bpc, a.block_offset, a.causal, a.cleanup, value,
+           thr.defined() ? static_cast<const float*>(thr.data_ptr()) : nullptr, a.sink, a.recent,
+           r.mask.defined() ? static_cast<uint8_t*>(r.mask.data_ptr()) : nullptr,
+           r.idx.defined() ? static_cast<int32_t*>(r.idx.data_ptr()) : nullptr,
+           r.cnt.defined() ? static_cast<int32_t*>(r.cnt.data_ptr()) : nullptr, lqb, lkb, a.list_q, a.list_k, at_.status, at_.stream),
+        "select");
+  return r;
+}
+
+// Attention over block lists (undefined: dense).  q, k, v 16 bit.  `out`: undefined, or [B, Hq, Lq, 128] with unit inner
+// stride.  out_f32: write fp32 (bf16 inputs only).  Returns a transposed view of [B, Lq, Hq, D] storage, or `out`.
+Tensor attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& idx, const Tensor& cnt, bool causal, double scale,
+                 Tensor out, bool out_f32, bool use_workspace, const Place& at_) {
+  const Tensor q = aligned16(q_), k = aligned16(k_), v = aligned16(v_);
+  const int64_t B = q.size(0), Hq = q.size(1), Lq = q.size(2), D = q.size(3), Hkv = k.size(1), Lk = k.size(2);
+  if (!out.defined()) out = empty({B, Lq, Hq, D}, out_f32 ? at::kFloat : q.scalar_type(), at_.dev).transpose(1, 2);
+  const size_t bytes = use_workspace ? xattn_b200_block_sparse_attn_workspace_bytes(B, Hq, Hkv, Lq, Lk) : 0;
+  Tensor ws;
+  if (bytes) ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
+  check(xattn_b200_block_sparse_attn_ws(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), out_f32 ? XATTN_B200_BF16_OUT_F32 : dtype_code(q.scalar_type()), B, Hq, Hkv, Lq, Lk,
+            D, q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
+            idx.defined() ? static_cast<const int32_t*>(idx.data_ptr()) : nullptr,
+            cnt.defined() ? static_cast<const int32_t*>(cnt.data_ptr()) : nullptr, causal, static_cast<float>(scale), out.data_ptr(),
+            out.stride(0), out.stride(1), out.stride(2), bytes ? ws.data_ptr() : nullptr, bytes, at_.status, at_.stream),
+        "block_sparse_attn");
+  return out;
+}
+// Non-causal calls: sorting the units by list length is one launch of a few microseconds; with only a few units per SM there
+// is nothing to balance.
+constexpr int64_t kOrderMinItems = 16 * 148;
+bool default_workspace(bool causal, bool dense, const Tensor& q) {
+  if (dense) return false;
+  const char* forced = std::getenv("XATTN_B200_ATTN_WORKSPACE");       // "0" / "1": overrides the rule (for measurements)
+  if (forced && (forced[0] == '0' || forced[0] == '1') && forced[1] == 0) return forced[0] == '1';
+  return !causal && q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) >= kOrderMinItems;
+}
+
+void need_16bit_or_f32(const Tensor& q, const Tensor& k, const char* text) {
+  if ((dtype_code(q.scalar_type()) < 0 && q.scalar_type() != at::kFloat) || (q.scalar_type() != at::kFloat && k.scalar_type() != q.scalar_type()))
+    fail(PyExc_TypeError, text);
+}
+bool band_applies(int64_t k_len, int chunk, bool causal, int semantics) {
+  return causal && semantics == XATTN_B200_SEMANTICS_TORCH && k_len % chunk == 0 && (chunk / 128) % 4 == 0;
+}
+
+// ---------------------------------------------------------------------------------------------- Python functions
+PyObject* wrap(Tensor t) { return t.defined() ? THPVariable_Wrap(std::move(t)) : Py_NewRef(Py_None); }
+
+// estimate(q, k, stride, block, chunk, norm, causal, semantics, band) -> sums
+PyObject* py_estimate(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Args a{v, n, "estimate"};
+  a.count(9);
+  const Tensor &q = a.tensor(0), &k = a.tensor(1);
+  need_cuda(q); need_cuda(k); need_4d(q); need_4d(k);
+  need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
+  const Place at_(q);
+  EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), a.flag(8)};
+  const Geometry g = geometry(q.size(2), k.size(2), e.chunk, e.stride, e.block);
+  const bool f32 = q.scalar_type() == at::kFloat;
+  Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
+  return wrap(estimate(qo, ko, q.size(3), g, e, at_));
+  END_HANDLE_TH_ERRORS
+}
+
+// select(sums, bpc, block_offset, threshold, causal, cleanup, sink, recent, want_mask, list_q, list_k, band_kb) -> (mask, idx, cnt)
+PyObject* py_select(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Args a{v, n, "select"};
+  a.count(12);
+  Tensor sums = a.tensor(0);
+  need_cuda(sums); need_4d(sums);
+  if (sums.scalar_type() != at::kFloat) sums = sums.to(at::kFloat);
+  sums = sums.contiguous();
+  const Place at_(sums);
+  Selection r = select(sums, v[3], {(int)a.integer(1), (int)a.integer(2), a.flag(4), a.flag(5), a.flag(6), a.flag(7), a.flag(8), a.integer(9),
+                                    a.integer(10), a.integer(11)}, at_);
+  PyObject* t = PyTuple_New(3);
+  if (!t) throw python_error();
+  PyTuple_SET_ITEM(t, 0, wrap(r.mask));
+  PyTuple_SET_ITEM(t, 1, wrap(r.idx));
+  PyTuple_SET_ITEM(t, 2, wrap(r.cnt));
+  return t;
+  END_HANDLE_TH_ERRORS
+}
+
+Tensor attention_any(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx, const Tensor& cnt, bool causal, double scale,
+                     Tensor out, std::optional<bool> use_workspace, const Place& at_) {
+  const int64_t D = q.size(3);
+  if (D != 128) fail(PyExc_ValueError, "head_dim must be 128");
+  const bool f32 = q.scalar_type() == at::kFloat, dense = !idx.defined();
+  Tensor q16 = q, k16 = k, v16 = v;
+  if (f32) { q16 = q.to(at::kBFloat16); k16 = k.to(at::kBFloat16); v16 = v.to(at::kBFloat16); }
+  if (dtype_code(q16.scalar_type()) < 0 || k16.scalar_type() != q16.scalar_type() || v16.scalar_type() != q16.scalar_type())
+    fail(PyExc_TypeError, "q/k/v must share one of bf16, fp16, fp32");
+  if (out.defined() && (out.sizes() != q.sizes() || out.scalar_type() != q16.scalar_type() || out.stride(3) != 1 || !out.is_cuda()))
+    fail(PyExc_ValueError, "out must be a CUDA tensor [B,Hq,Lq,D] of the compute dtype with unit inner stride");
+  const int64_t lqb = (q.size(2) + 127) / 128, lkb = (k.size(2) + 127) / 128;
+  if (!dense && (idx.sizes() != at::IntArrayRef({q.size(0), q.size(1), lqb, lkb}) || cnt.sizes() != at::IntArrayRef({q.size(0), q.size(1), lqb})))
+    fail(PyExc_ValueError, "block lists have the wrong shape");
+  const bool ws = dense ? false : use_workspace.value_or(default_workspace(causal, dense, q));
+  return attention(q16, k16, v16, dense ? idx : idx.contiguous(), dense ? cnt : cnt.contiguous(), causal, scale, out, f32 && !out.defined(), ws, at_);
+}
+
+// attention(q, k, v, idx, cnt, causal, scale, out, use_workspace) -> out
+PyObject* py_attention(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Args a{v, n, "attention"};
+  a.count(9);
+  const Tensor &q = a.tensor(0), &k = a.tensor(1), &vv = a.tensor(2);
+  Tensor idx, cnt, out;
+  if (!a.none(3)) idx = a.tensor(3);
+  if (!a.none(4)) cnt = a.tensor(4);
+  if (idx.defined() != cnt.defined()) fail(PyExc_ValueError, "block lists have the wrong shape");
+  if (!a.none(7)) out = a.tensor(7);
+  need_cuda(q); need_cuda(k); need_cuda(vv); need_4d(q); need_4d(k); need_4d(vv);
+  if (idx.defined()) { need_cuda(idx); need_cuda(cnt); }
+  const Place at_(q);
+  const double scale = a.none(6) ? 1.0 / std::sqrt(static_cast<double>(q.size(3))) : a.real(6);
+  std::optional<bool> ws;
+  if (!a.none(8)) ws = a.flag(8);
+  return wrap(attention_any(q, k, vv, idx, cnt, a.flag(5), scale, out, ws, at_));
+  END_HANDLE_TH_ERRORS
+}
+
+// decode(q, k, v, scale) -> out: one query token per sequence against its whole cache
+PyObject* py_decode(PyObject*, PyObject* const* pv, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Args a{pv, n, "decode"};
+  a.count(4);
+  const Tensor &q_ = a.tensor(0), &k_ = a.tensor(1), &v_ = a.tensor(2);
+  need_cuda(q_); need_cuda(k_); need_cuda(v_); need_4d(q_); need_4d(k_); need_4d(v_);
+  const Place at_(q_);
+  const int64_t B = q_.size(0), Hq = q_.size(1), D = q_.size(3), Hkv = k_.size(1), Lk = k_.size(2);
+  const double scale = a.none(3) ? 1.0 / std::sqrt(static_cast<double>(D)) : a.real(3);
+  const int code = dtype_code(q_.scalar_type());
+  if (q_.size(2) != 1 || D != 128 || code < 0 || Hq % Hkv || Hq / Hkv > 16)      // what the decode kernel does not cover
+    return wrap(attention_any(q_, k_, v_, Tensor(), Tensor(), true, scale, Tensor(), false, at_));
+  if (k_.scalar_type() != q_.scalar_type() || v_.scalar_type() != q_.scalar_type())
+    fail(PyExc_TypeError, "q/k/v must share one of bf16, fp16, fp32");
+  const Tensor q = aligned16(q_), k = aligned16(k_), v = aligned16(v_);
+  const size_t bytes = xattn_b200_decode_workspace_bytes(B, Hq, Hkv, Lk);
+  const Tensor ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
+  Tensor out = empty({B, 1, Hq, D}, q.scalar_type(), at_.dev);
+  check(xattn_b200_decode_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), code, B, Hq, Hkv, Lk, D, q.stride(0), q.stride(1), k.stride(0),
+                               k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2), static_cast<float>(scale), out.data_ptr(),
+                               Hq * D, D, ws.data_ptr(), bytes, at_.status, at_.stream),
+        "decode_attn");
+  return wrap(out.transpose(1, 2));
+  END_HANDLE_TH_ERRORS
+}
+
+// prefill(q, k, v, stride, norm, threshold, block, causal, chunk, sink, recent, semantics, out) -> out: all three phases
+PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Args a{pv, n, "prefill"};
+  a.count(13);
+  const Tensor& q = a.tensor(0);
+  Tensor k = a.tensor(1), v = a.tensor(2);
+  need_cuda(q); need_4d(q); need_4d(k); need_4d(v);
+  if (k.device() != q.device()) k = k.to(q.device());
+  if (v.device() != q.device()) v = v.to(q.device());
+  need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
+  const Place at_(q);
+  const int64_t Lq = q.size(2), Lk = k.size(2), D = q.size(3);
+  EstimateArgs e{(int)a.integer(3), (int)a.integer(6), a.none(8) ? xattn_b200_default_chunk_size(Lk) : (int)a.integer(8), (int)a.integer(11),
+                 a.real(4), a.flag(7), false};
+  // un-padded causal keys under the torch branch: the sums outside a row's own chunk are zero and are not kept
+  e.band = band_applies(Lk, e.chunk, e.causal, e.semantics);
+  const Geometry g = geometry(Lq, Lk, e.chunk, e.stride, e.block);
+  Tensor out;
+  if (!a.none(12)) out = a.tensor(12);
+  const bool f32 = q.scalar_type() == at::kFloat;
+  Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
+  Selection s;
+  {
+    const Tensor sums = estimate(qo, ko, D, g, e, at_);
+    s = select(sums, pv[5], {g.bpc, g.block_offset, e.causal, true, a.flag(9), a.flag(10), false, Lq, Lk, e.band ? g.kb : 0}, at_);
+  }
+  const double scale = 1.0 / std::sqrt(static_cast<double>(D));
+  if (f32 && D == 128 && !out.defined() && v.scalar_type() == at::kFloat) {
+    // the first terms of q and k ARE their bf16 roundings, which the attention phase computes with
+    const Tensor vc = v.stride(3) == 1 ? v : v.contiguous();
+    const Tensor v16 = empty(v.sizes(), at::kBFloat16, at_.dev);
+    check(xattn_b200_split_f32(static_cast<const float*>(vc.data_ptr()), v.size(0), v.size(1), Lk, Lk, D, vc.stride(0), vc.stride(1),
+                               vc.stride(2), 1, v16.data_ptr(), at_.stream),
+          "split_f32");
+    return wrap(attention(qo.t.narrow(3, 0, D).narrow(2, 0, Lq), ko.t.narrow(3, 0, D).narrow(2, 0, Lk), v16, s.idx, s.cnt, e.causal, scale,
+                          out, true, default_workspace(e.causal, false, q), at_));
+  }
+  return wrap(attention_any(q, k, v, s.idx, s.cnt, e.causal, scale, out, std::nullopt, at_));
+  END_HANDLE_TH_ERRORS
+}
+
+// estimate_and_select(q, k, stride, block, chunk, norm, causal, semantics, threshold, sink, recent) -> (sums in q's type, mask)
+PyObject* py_estimate_and_select(PyObject*, PyObject* const* pv, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Args a{pv, n, "estimate_and_select"};
+  a.count(11);
+  const Tensor &q = a.tensor(0), &k = a.tensor(1);
+  need_cuda(q); need_cuda(k); need_4d(q); need_4d(k);
+  need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
+  const Place at_(q);
+  const EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), false};
+  const Geometry g = geometry(q.size(2), k.size(2), e.chunk, e.stride, e.block);
+  const bool f32 = q.scalar_type() == at::kFloat;
+  Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
+  const Tensor sums = estimate(qo, ko, q.size(3), g, e, at_);
+  const Selection s = select(sums, pv[8], {g.bpc, g.block_offset, e.causal, true, a.flag(9), a.flag(10), true, 0, 0, 0}, at_);
+  PyObject* t = PyTuple_New(2);
+  if (!t) throw python_error();
+  PyTuple_SET_ITEM(t, 0, wrap(f32 ? sums : sums.to(q.scalar_type())));
+  PyTuple_SET_ITEM(t, 1, wrap(s.mask));
+  return t;
+  END_HANDLE_TH_ERRORS
+}
+
+// init(error class, status word callback)
+PyObject* py_init(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Args a{v, n, "init"};
+  a.count(2);
+  g_error = Py_NewRef(v[0]);
+  g_status_of = Py_NewRef(v[1]);
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"init", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_init)), METH_FASTCALL, nullptr},
+    {"estimate", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_estimate)), METH_FASTCALL, nullptr},
+    {"estimate_and_select", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_estimate_and_select)), METH_FASTCALL, nullptr},
+    {"select", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_select)), METH_FASTCALL, nullptr},
+    {"attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_attention)), METH_FASTCALL, nullptr},
+    {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_decode)), METH_FASTCALL, nullptr},
+    {"prefill", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_prefill)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Tensor plumbing of xattn_b200", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }

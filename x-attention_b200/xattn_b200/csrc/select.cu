@@ -504,7 +504,7 @@ int select_launch(const float* attn_sums, int batch, int heads, int q_blocks, in
   const int grid = static_cast<int>((rows + wpc - 1) / wpc);
   auto launch = [&](auto kern) -> int {
     if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
+        !allow_smem(kern, 160 * 1024))
       return XATTN_B200_ERR_CUDA;
     kern<<<grid, wpc * 32, smem, stream>>>(attn_sums, p, thr_per_head, mask, block_idx, block_cnt, status);
     return launch_status();

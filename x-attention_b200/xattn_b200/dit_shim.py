@@ -20,13 +20,7 @@ def _dense(q, k, v, out):
 
 def _xattn(q, k, v, out, threshold, stride):
     """Non-causal Xattention_prefill (xattn/src/Xattention.py:302-402) writing into `out`."""
-    Lq, Lk = q.shape[2], k.shape[2]
-    chunk = ops.default_chunk_size(Lk)
-    g = ops.geometry(Lq, Lk, chunk, stride, 128)
-    sums = ops.estimate_block_sums(q, k, stride, 128, chunk, 1.0, False)
-    _, idx, cnt = ops.select_blocks(sums, g["bpc"], g["block_offset"], threshold, False, True, list_shape=(Lq, Lk),
-                                    want_mask=False)
-    ops.block_sparse_attention(q, k, v, idx, cnt, causal=False, out=out)
+    ops.prefill(q, k, v, stride, 1.0, threshold, 128, False, None, False, False, out)
 
 
 def xattn_varlen_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens_q, cu_seqlens_kv,
