@@ -96,9 +96,7 @@ size_t xattn_b200_estimate_workspace_bytes_ex(int batch, int hq, int q_len, int 
  * normalises into `attn_sums`.
  *
  * q_len / k_len need not be multiples of `stride`: the tokens a ragged last stride group lacks count as the
- * zeros the reference pads with (xattn/src/Xattention.py:42-51); the library stages a zero-padded copy of the
- * one 128-row tile of Q (128- or 256-row tile of K) that holds that group in `workspace` -- a few MB instead
- * of a padded copy of the tensors (workspace sizes assume head_dim 128 for it).  head_dim is a
+ * zeros the reference pads with (xattn/src/Xattention.py:42-51); no copy is made for them.  head_dim is a
  * multiple of 64 (XATTN_B200_F32_TERMS: a row holds three times as many elements, and q_len and k_len are multiples of
  * the stride);  `scale` = 1/(sqrt(D)*stride*norm).
  * attn_sums: float32 [batch, hq, q_blocks_pad, k_blocks_pad] (fully written).

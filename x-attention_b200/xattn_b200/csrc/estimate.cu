@@ -39,7 +39,7 @@ constexpr int kGemmSmem = kStages * kStageBytes + 1024 /*barriers*/ + 1024 /*ali
 struct EstGeom {
   int batch, hq, hkv;
   int S, d_chunks;             // K loop: S * d_chunks steps of 64 elements
-  int term_chunks;             // split fp32 rows: steps per term (0: plain rows); see k_columns
+  int term_chunks;             // split fp32 rows: 64-column chunks per term (0: plain rows); see k_column
   int rows_total, cols_total;  // padded lengths / S
   int rows_valid, cols_valid;  // rows past rows_valid give zeros; causal: columns past cols_valid are hidden
   int rcs;                     // chunk_size / S
@@ -55,15 +55,17 @@ struct EstGeom {
   // chunk): the column tiles [tile_lo, tile_lo + m_pitch) of its row tile, i.e. key blocks from tile_lo * (tile_n /
   // rbs) on -- 16 floats per row instead of 1024 at 128K tokens.
   int compact, m_pitch, p_pitch;
-  // lengths that are no multiple of the stride: the row tile of Q' / column tile of K' that holds the ragged last
-  // stride group is read from a zero-padded staging copy of just that tile (-1: none)
-  int q_tail_mt, k_tail_nt;
+  // Lengths that are no multiple of the stride: the last stride group lacks the tokens of offset >= len % stride, which
+  // count as zeros.  Two tensor maps of each operand: token offsets below the remainder go through one that has that group,
+  // the others through one that ends before it (no group at all: the coordinate is moved past the only one).
+  int q_rem, k_rem, q_none, k_none;
   int head_dim;
   float scale_log2;
   // Tile tables of est_setup_kernel computed on the host and carried in the kernel parameters when they are small
   // (tab_n = n_mtiles <= kTabTiles, e.g. 32 row tiles at 32K tokens, 64 at 128K): every kernel copies them into
   // shared memory and est_setup_kernel is not launched.  Layout: tile_lo[kTabTiles], tile_prefix[kTabTiles + 1],
   // pair_lo[kTabTiles / 2], pair_prefix[kTabTiles / 2 + 1].
+  int direct;                  // the epilogue finishes the block sums: every row tile is computed, even one that sees nothing
   int tab_n;
   int tab[64 + 65 + 32 + 33];
 };
@@ -85,18 +87,12 @@ __host__ __device__ inline void row_bounds(const EstGeom& g, int i, int& lo, int
   if (hi > g.cols_valid - 1) hi = g.cols_valid - 1;
 }
 
-// Columns of the A (query) and B (key) operands of step dc of a token.  Plain rows: the same 64-column chunk of both.
-// fp32 rows split into three bf16 terms [hi | mid | lo]: the six products hh, hm, mh, hl, lh, mm one after the other (the
-// three left out are below 2^-24 of the first), two bits per product naming the term of either side.
-__device__ __forceinline__ void k_columns(const EstGeom& g, int dc, int& a_col, int& b_col) {
-  if (g.term_chunks == 0) {
-    a_col = b_col = dc * kTileK;
-    return;
-  }
-  constexpr uint32_t kTermA = 0 | 0 << 2 | 1 << 4 | 0 << 6 | 2 << 8 | 1 << 10, kTermB = 0 | 1 << 2 | 0 << 4 | 2 << 6 | 0 << 8 | 1 << 10;
-  const int pair = dc / g.term_chunks, c = dc - pair * g.term_chunks;
-  a_col = ((kTermA >> (2 * pair) & 3) * g.term_chunks + c) * kTileK;
-  b_col = ((kTermB >> (2 * pair) & 3) * g.term_chunks + c) * kTileK;
+// Columns of both operands of step dc of a token.  Plain rows: one 64-column chunk after the other.  fp32 rows split into
+// three bf16 terms [hi | mid | lo]: of one chunk after the other the three terms, three stages the MMA issuer treats as one.
+__device__ __forceinline__ int k_column(const EstGeom& g, int dc) {
+  if (g.term_chunks == 0) return dc * kTileK;
+  const int c = dc / 3, term = dc - 3 * c;
+  return (term * g.term_chunks + c) * kTileK;
 }
 
 // first column tile / first key block a row tile's scratch rows are indexed from
@@ -120,7 +116,7 @@ __host__ __device__ inline void row_tile_range(const EstGeom& g, int mt, int& fi
   }
   if (hi_max < lo_min) {
     first = 0;
-    count = 0;
+    count = g.direct;
   } else {
     first = lo_min / g.tile_n;
     count = hi_max / g.tile_n - lo_min / g.tile_n + 1;
@@ -285,7 +281,7 @@ __device__ __forceinline__ void est_epilogue_row(const EstGeom& g, uint32_t tadd
 // it are needed.  `out` is the 128 / RBS floats of this row's query block (written by its first row's lane).
 template <int RBS, typename Release>
 __device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, uint32_t taddr, int clo, int chi,
-                                                        float* __restrict__ out, bool write, Release release) {
+                                                        float* __restrict__ out, int out_cols, bool write, Release release) {
   constexpr int kChunks = 4, kPer = 32 / RBS;               // 128 columns; key blocks per 32-column chunk
   auto fully_visible = [&](int c8) { return __all_sync(0xffffffffu, clo <= c8 * 32 && chi >= c8 * 32 + 31); };
   float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -362,10 +358,17 @@ __device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, uint32
     for (int o = 1; o < RBS; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     blk[q] = v;
   }
-  if (write) {
+  if (!write) return;
+  if (g.band) {
 #pragma unroll
     for (int q = 0; q < kChunks * kPer; q += 4)
       *reinterpret_cast<float4*>(out + q) = make_float4(blk[q], blk[q + 1], blk[q + 2], blk[q + 3]);
+  } else {
+    // dense rows of a few blocks more or less than the tile holds
+#pragma unroll
+    for (int q = 0; q < kChunks * kPer; ++q)
+      if (q < out_cols) out[q] = blk[q];
+    for (int q = kChunks * kPer; q < out_cols; ++q) out[q] = 0.f;
   }
 }
 
@@ -385,7 +388,8 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // 128-column tiles (every operand tile is used once: the kernel streams Q and K from HBM) take six 32 KiB
   // stages, 256-column tiles four 48 KiB ones: 192 KiB in flight either way
-  const int n_stages = g.tile_n == 128 ? kMaxStages : kStages;
+  // (split fp32 rows use them in threes)
+  const int n_stages = g.tile_n == 128 ? kMaxStages : (g.term_chunks ? 3 : kStages);
   const int stage_bytes = kABytes + g.tile_n * kTileK * 2;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
   const uint32_t full0 = smem_u32(bars);                       // [kMaxStages]
@@ -395,7 +399,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);     // (uniform for the compiler too)
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -430,57 +434,78 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one thread)
     if (lane == 0) {
-      uint32_t it = 0;
+      int s = 0;
+      uint32_t ph = 0;
       for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x) {
         int bh, mt, nt;
         decode_tile(g.n_mtiles, tile_lo, tile_prefix, tiles_per_head, tile, bh, mt, nt, interleave);
         const int b = bh / g.hq, h = bh - b * g.hq;
-        for (int ks = 0; ks < k_steps; ++ks, ++it) {
-          const int s = it % n_stages;
-          const uint32_t ph = (it / n_stages) & 1;
+        int t = 0, dc = 0;
+        for (int ks = 0; ks < k_steps; ++ks) {
           if (!mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag)) break;
-          const int t = ks / g.d_chunks;
-          const int dc = ks - t * g.d_chunks;
           const uint32_t dstA = smem_u32(smem + s * stage_bytes);
           mbar_expect_tx(full0 + 8 * s, stage_bytes);
-          // (the tile that holds a ragged last stride group comes from its zero-padded staging copy)
-          const bool qt = mt == g.q_tail_mt, kt = nt == g.k_tail_nt;
-          int ac, bc;
-          k_columns(g, dc, ac, bc);
-          tma_load_5d(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, ac, g.S - 1 - t, qt ? 0 : mt * kTileM, h, b);
-          tma_load_5d(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, bc, t, kt ? 0 : nt * g.tile_n,
-                      h / group, b);
+          const bool qt = g.S - 1 - t < g.q_rem, kt = t < g.k_rem;
+          const int col = k_column(g, dc);
+          tma_load_5d(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b);
+          tma_load_5d(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, col, t, nt * g.tile_n + (kt ? 0 : g.k_none), h / group, b);
+          if (++dc == g.d_chunks) { dc = 0; ++t; }
+          if (++s == n_stages) { s = 0; ph ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (one thread)
-    if (lane == 0) {
-      uint32_t it = 0, local_tile = 0;
+    // ------------------------------------------------------------ MMA issuer (converged warp, one thread issues: see mma_ss_lead)
+    {
+      const uint32_t lead = elect_one() ? 1u : 0u;
+      auto wait = [&](uint32_t bar, uint32_t ph) { return __all_sync(0xffffffffu, mbar_wait(bar, ph, abort_flag)); };
+      int st = 0;
+      uint32_t ph = 0, local_tile = 0;
       const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
       const uint64_t b_desc0 = smem_desc_sw128(smem_u32(smem) + kABytes, 16, 1024);
       for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++local_tile) {
         const uint32_t acc = local_tile & 1;
         const uint32_t acc_ph = (local_tile >> 1) & 1;
-        if (!mbar_wait(tempty0 + 8 * acc, acc_ph ^ 1, abort_flag)) break;
+        if (!wait(tempty0 + 8 * acc, acc_ph ^ 1)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kTileN;
         bool ok = true;
-        for (int ks = 0; ks < k_steps; ++ks, ++it) {
-          const int s = it % n_stages;
-          const uint32_t ph = (it / n_stages) & 1;
-          if (!mbar_wait(full0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+        int term = g.term_chunks ? 0 : -1;
+        for (int ks = 0; ks < k_steps; ++ks) {
+          if (!wait(full0 + 8 * st, ph)) { ok = false; break; }
           tc_fence_after();
-          // descriptors differ from the stage-0 ones only in the start-address field (units of 16 bytes)
-          const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(s * (stage_bytes >> 4));
-          const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(s * (stage_bytes >> 4));
+          // D += A of stage sa * B of stage sb; descriptors differ from the stage-0 ones only in the start-address field
+          // (units of 16 bytes)
+          auto product = [&](int sa, int sb, uint32_t accumulate) {
+            const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(sa * (stage_bytes >> 4));
+            const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(sb * (stage_bytes >> 4));
 #pragma unroll
-          for (int k4 = 0; k4 < kTileK / 16; ++k4)
-            mma_ss(d_tmem, a_desc + k4 * 2, b_desc + k4 * 2, idesc, (ks > 0 || k4 > 0) ? 1u : 0u);
-          mma_commit(empty0 + 8 * s);          // stage reusable once these MMAs have read it
+            for (int k4 = 0; k4 < kTileK / 16; ++k4)
+              mma_ss_lead(d_tmem, a_desc + k4 * 2, b_desc + k4 * 2, idesc, k4 > 0 ? 1u : accumulate, lead);
+          };
+          if (term < 0) {
+            product(st, st, ks > 0 ? 1u : 0u);
+            mma_commit_lead(empty0 + 8 * st, lead);       // stage reusable once these MMAs have read it
+          } else {
+            // three stages hold the terms [hi, mid, lo] of one chunk: the products hh; hm, mh, mm; hl, lh (the three left out
+            // are below 2^-24 of the first).  Each term is loaded once for the products it enters.
+            if (term == 0) {
+              product(st, st, ks > 0 ? 1u : 0u);
+            } else if (term == 1) {
+              product(st - 1, st, 1u);
+              product(st, st - 1, 1u);
+              product(st, st, 1u);
+            } else {
+              product(st - 2, st, 1u);
+              product(st, st - 2, 1u);
+              for (int k = 2; k >= 0; --k) mma_commit_lead(empty0 + 8 * (st - k), lead);
+            }
+            term = term == 2 ? 0 : term + 1;
+          }
+          if (++st == n_stages) { st = 0; ph ^= 1; }
         }
         if (!ok) break;
-        mma_commit(tfull0 + 8 * acc);          // accumulator complete
+        mma_commit_lead(tfull0 + 8 * acc, lead);          // accumulator complete
       }
     }
   } else {
@@ -517,8 +542,9 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if constexpr (DIRECT) {
         // the query block of this row, and its first row's lane as the writer (RBS divides 32)
         const int qb = i / RBS;
+        const int out_cols = g.band ? g.bpc : g.kb_total;
         est_epilogue_row_direct<RBS>(g, taddr, clo, chi,
-                                     sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * g.bpc,
+                                     sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, out_cols,
                                      (lane % RBS) == 0 && qb < g.qb_total, release);
       } else {
         est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, row_ok,
@@ -583,7 +609,7 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kPairStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);     // (uniform for the compiler too)
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();                  // 0: issues the MMAs
   const int pair = blockIdx.x >> 1, n_pairs_grid = gridDim.x >> 1;
@@ -620,58 +646,82 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one thread per CTA)
     if (lane == 0) {
-      uint32_t it = 0;
+      int s = 0;
+      uint32_t ph = 0;
       for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs_grid) {
         int bh, pm, nt;
         decode_tile(n_groups, pair_lo, pair_prefix, tiles_per_head, tile, bh, pm, nt);
         const int b = bh / g.hq, h = bh - b * g.hq;
         const int mt = 2 * pm + static_cast<int>(rank);
-        for (int ks = 0; ks < k_steps; ++ks, ++it) {
-          const int s = it % kPairStages;
-          const uint32_t ph = (it / kPairStages) & 1;
+        int t = 0, dc = 0;
+        for (int ks = 0; ks < k_steps; ++ks) {
           if (!mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag)) break;
-          const int t = ks / g.d_chunks;
-          const int dc = ks - t * g.d_chunks;
           const uint32_t dstA = smem_u32(smem + s * kPairStageBytes);
           // all four loads of a stage are counted on the even CTA's barrier
           const uint32_t full_even = mapa_shared(full0 + 8 * s, 0);
           if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * kPairStageBytes);
-          const bool qt = mt == g.q_tail_mt, kt = nt == g.k_tail_nt;
-          int ac, bc;
-          k_columns(g, dc, ac, bc);
-          tma_load_5d_pair(dstA, qt ? &tmQt : &tmQ, full_even, ac, g.S - 1 - t, qt ? 0 : mt * kTileM, h, b);
-          tma_load_5d_pair(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, bc, t,
-                           (kt ? 0 : nt * kTileN) + static_cast<int>(rank) * 128, h / group, b);
+          const bool qt = g.S - 1 - t < g.q_rem, kt = t < g.k_rem;
+          const int col = k_column(g, dc);
+          tma_load_5d_pair(dstA, qt ? &tmQt : &tmQ, full_even, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b);
+          tma_load_5d_pair(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, col, t,
+                           nt * kTileN + static_cast<int>(rank) * 128 + (kt ? 0 : g.k_none), h / group, b);
+          if (++dc == g.d_chunks) { dc = 0; ++t; }
+          if (++s == kPairStages) { s = 0; ph ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (one thread of the even CTA)
-    if (lane == 0 && rank == 0) {
-      uint32_t it = 0, local_tile = 0;
+    // ------------------------------------------------------------ MMA issuer (even CTA; converged warp, one thread issues)
+    if (rank == 0) {
+      const uint32_t lead = elect_one() ? 1u : 0u;
+      auto wait = [&](uint32_t bar, uint32_t ph) { return __all_sync(0xffffffffu, mbar_wait(bar, ph, abort_flag)); };
+      int st = 0;
+      uint32_t ph = 0, local_tile = 0;
       const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
       const uint64_t b_desc0 = smem_desc_sw128(smem_u32(smem) + kABytes, 16, 1024);
       for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs_grid, ++local_tile) {
         const uint32_t acc = local_tile & 1;
         const uint32_t acc_ph = (local_tile >> 1) & 1;
-        if (!mbar_wait(tempty0 + 8 * acc, acc_ph ^ 1, abort_flag)) break;
+        if (!wait(tempty0 + 8 * acc, acc_ph ^ 1)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kTileN;
         bool ok = true;
-        for (int ks = 0; ks < k_steps; ++ks, ++it) {
-          const int s = it % kPairStages;
-          const uint32_t ph = (it / kPairStages) & 1;
-          if (!mbar_wait(full0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+        int term = g.term_chunks ? 0 : -1;
+        for (int ks = 0; ks < k_steps; ++ks) {
+          if (!wait(full0 + 8 * st, ph)) { ok = false; break; }
           tc_fence_after();
-          const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(s * (kPairStageBytes >> 4));
-          const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(s * (kPairStageBytes >> 4));
+          // D += A of stage sa * B of stage sb; descriptors differ from the stage-0 ones only in the start-address field
+          // (units of 16 bytes)
+          auto product = [&](int sa, int sb, uint32_t accumulate) {
+            const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(sa * (kPairStageBytes >> 4));
+            const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(sb * (kPairStageBytes >> 4));
 #pragma unroll
-          for (int k4 = 0; k4 < kTileK / 16; ++k4)
-            mma_ss_pair(d_tmem, a_desc + k4 * 2, b_desc + k4 * 2, idesc, (ks > 0 || k4 > 0) ? 1u : 0u);
-          mma_commit_pair(empty0 + 8 * s, 3);  // stage reusable in both CTAs once these MMAs have read it
+            for (int k4 = 0; k4 < kTileK / 16; ++k4)
+              mma_ss_pair_lead(d_tmem, a_desc + k4 * 2, b_desc + k4 * 2, idesc, k4 > 0 ? 1u : accumulate, lead);
+          };
+          if (term < 0) {
+            product(st, st, ks > 0 ? 1u : 0u);
+            mma_commit_pair_lead(empty0 + 8 * st, 3, lead);       // stage reusable once these MMAs have read it
+          } else {
+            // three stages hold the terms [hi, mid, lo] of one chunk: the products hh; hm, mh, mm; hl, lh (the three left out
+            // are below 2^-24 of the first).  Each term is loaded once for the products it enters.
+            if (term == 0) {
+              product(st, st, ks > 0 ? 1u : 0u);
+            } else if (term == 1) {
+              product(st - 1, st, 1u);
+              product(st, st - 1, 1u);
+              product(st, st, 1u);
+            } else {
+              product(st - 2, st, 1u);
+              product(st, st - 2, 1u);
+              for (int k = 2; k >= 0; --k) mma_commit_pair_lead(empty0 + 8 * (st - k), 3, lead);
+            }
+            term = term == 2 ? 0 : term + 1;
+          }
+          if (++st == kPairStages) { st = 0; ph ^= 1; }
         }
         if (!ok) break;
-        mma_commit_pair(tfull0 + 8 * acc, 3);  // accumulator complete in both CTAs
+        mma_commit_pair_lead(tfull0 + 8 * acc, 3, lead);  // accumulator complete in both CTAs
       }
     }
   } else {
@@ -878,31 +928,10 @@ split_f32_kernel(const float* __restrict__ x, int heads, int len, int len_valid,
   }
 }
 
-// Zero-padded copy of `n_tokens` tokens starting at `first_token` of every head ([batch, heads, n_tokens, D] 16-bit,
-// contiguous): the tile that holds the ragged last stride group, so that the tokens past the end read as the zeros
-// the reference pads with (xattn/src/Xattention.py:42-51) instead of the next head's data.  16 bytes per thread.
-__global__ void est_tail_kernel(const uint4* __restrict__ src, int64_t sb, int64_t sh, int64_t sl, int heads, int len,
-                                int D, int first_token, int n_tokens, uint4* __restrict__ dst, size_t total_vec) {
-  const int vec_per_row = D / 8;
-  for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < total_vec;
-       e += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const int c = static_cast<int>(e % vec_per_row);
-    size_t rest = e / vec_per_row;
-    const int tok = static_cast<int>(rest % n_tokens);
-    rest /= n_tokens;
-    const int h = static_cast<int>(rest % heads);
-    const int b = static_cast<int>(rest / heads);
-    const int t = first_token + tok;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (t < len) v = src[(b * sb + h * sh + static_cast<int64_t>(t) * sl) / 8 + c];
-    dst[e] = v;
-  }
-}
-
 // ------------------------------------------------------------------------------------ host side
 struct EstWorkspace {
   size_t off_tile_lo, off_tile_prefix, off_pair_lo, off_pair_prefix, off_rowstat, off_mtile, off_partial;
-  size_t off_qtail, off_ktail, total;
+  size_t total;
 };
 
 static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int head_dim, int stride, int block_size,
@@ -932,14 +961,18 @@ static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int h
   g.n_mtiles = (g.rows_total + kTileM - 1) / kTileM;
   // narrow tiles when every row sees at most one 128-column span (torch branch with chunk_size <= 128*stride):
   // a 256-wide tile would spend half of its MMA work on hidden columns
-  g.tile_n = (g.left_blank && g.rcs <= 128) ? 128 : kTileN;
+  // (and when the keys have no more than 128 columns at all)
+  g.tile_n = ((g.left_blank && g.rcs <= 128) || (g.causal ? g.cols_valid : g.cols_total) <= 128) ? 128 : kTileN;
   g.n_ntiles = (g.cols_total + g.tile_n - 1) / g.tile_n;
   g.scale_log2 = scale * 1.4426950408889634f;
   g.head_dim = head_dim;
   g.tab_n = 0;
   g.term_chunks = 0;
-  g.q_tail_mt = q_len % stride ? (q_len / stride) / kTileM : -1;
-  g.k_tail_nt = k_len % stride ? (k_len / stride) / g.tile_n : -1;
+  g.q_rem = q_len % stride;
+  g.k_rem = k_len % stride;
+  g.q_none = q_len < stride ? 1 : 0;
+  g.k_none = k_len < stride ? 1 : 0;
+  g.direct = 0;
   g.compact = g.left_blank;
   g.m_pitch = g.n_ntiles;
   g.p_pitch = g.kb_total;
@@ -968,11 +1001,6 @@ static EstWorkspace workspace_layout(const EstGeom& g) {
   w.off_rowstat = o; o = up(o + sizeof(float2) * rows);
   w.off_mtile = o; o = up(o + sizeof(float2) * rows * g.m_pitch);
   w.off_partial = o; o = up(o + sizeof(float) * rows * g.p_pitch);
-  // staging tiles [batch, heads, tile * S tokens, head_dim], 16 bit
-  w.off_qtail = o;
-  if (g.q_tail_mt >= 0) o = up(o + static_cast<size_t>(g.batch) * g.hq * kTileM * g.S * g.head_dim * 2);
-  w.off_ktail = o;
-  if (g.k_tail_nt >= 0) o = up(o + static_cast<size_t>(g.batch) * g.hkv * g.tile_n * g.S * g.head_dim * 2);
   w.total = o;
   return w;
 }
@@ -1018,7 +1046,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   if (split) {
     if (q_len % stride || k_len % stride) return XATTN_B200_ERR_ARG;       // (the split writes whole stride groups)
     g.term_chunks = g.d_chunks;
-    g.d_chunks *= 6;
+    g.d_chunks *= 3;
   }
   const EstWorkspace w = workspace_layout(g);
   if (!workspace || workspace_bytes < w.total) return XATTN_B200_ERR_WORKSPACE;
@@ -1038,22 +1066,16 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   float2* rowstat = reinterpret_cast<float2*>(ws + w.off_rowstat);
   float* partial = reinterpret_cast<float*>(ws + w.off_partial);
 
-  // 5-D views [head_dim, S, len/S, heads, batch] whose second coordinate picks the token inside a stride group
-  CUtensorMap tmQ, tmK;
-  {
-    const uint64_t dims[5] = {row_len, (uint64_t)stride, (uint64_t)(q_len / stride), (uint64_t)hq,
-                              (uint64_t)batch};
-    const uint64_t str[4] = {(uint64_t)qsl * 2, (uint64_t)qsl * 2 * stride, (uint64_t)qsh * 2, (uint64_t)qsb * 2};
-    const uint32_t box[5] = {kTileK, 1, kTileM, 1, 1};
-    if ((rc = make_tmap_16bit(&tmQ, q, 5, dims, str, box))) return rc;
-  }
-  {
-    const uint64_t dims[5] = {row_len, (uint64_t)stride, (uint64_t)(k_len / stride), (uint64_t)hkv,
-                              (uint64_t)batch};
-    const uint64_t str[4] = {(uint64_t)ksl * 2, (uint64_t)ksl * 2 * stride, (uint64_t)ksh * 2, (uint64_t)ksb * 2};
-    const uint32_t box[5] = {kTileK, 1, (uint32_t)g.tile_n, 1, 1};
-    if ((rc = make_tmap_16bit(&tmK, k, 5, dims, str, box))) return rc;
-  }
+  // 5-D views [head_dim, S, len/S, heads, batch] whose second coordinate picks the token inside a stride group; `up`: with
+  // the ragged last group (see EstGeom::q_rem)
+  auto make_map = [&](CUtensorMap* m, const void* x, int len, int heads, int64_t sb, int64_t sh, int64_t sl, uint32_t box_rows, bool up) -> int {
+    const int groups = len / stride > 0 && !up ? len / stride : (len + stride - 1) / stride;
+    const uint64_t dims[5] = {row_len, (uint64_t)stride, (uint64_t)groups, (uint64_t)heads, (uint64_t)batch};
+    // a dimension of extent 1 never moves: give it a harmless valid stride
+    const uint64_t str[4] = {(uint64_t)sl * 2, (uint64_t)sl * 2 * stride, heads > 1 ? (uint64_t)sh * 2 : 256, batch > 1 ? (uint64_t)sb * 2 : 256};
+    const uint32_t box[5] = {kTileK, 1, box_rows, 1, 1};
+    return make_tmap_16bit(m, x, 5, dims, str, box);
+  };
 
   // up to 64 KiB of dynamic shared memory (8192 row tiles): above the 48 KiB a kernel gets without asking
   if (!allow_smem(est_setup_kernel, 2 * sizeof(int) * 8192))
@@ -1064,48 +1086,30 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
 #ifdef XB_EST_NO_PAIRS
   use_pairs = false;
 #endif
-  // Chunks of exactly one 128-row, 128-column tile under the torch branch (128K tokens at stride 16): a row's only
-  // tile holds exactly the key blocks of its chunk-band output, so the GEMM's epilogue finishes the block sums
-  // itself and neither the scratch arrays nor est_rowstat_kernel / est_blocksum_kernel are needed.
-  bool direct = !use_pairs && g.band && g.left_blank && g.compact && g.m_pitch == 1 && g.tile_n == 128 &&
-                g.rcs == kTileM && g.row_off % 128 == 0 && g.rbs <= 32 && 32 % g.rbs == 0 &&
-                g.bpc == 128 / g.rbs && g.bpc % 4 == 0 && (reinterpret_cast<uintptr_t>(attn_sums) & 15) == 0;
+  // Every row sees a single 128-column tile and that tile's block sums are (nearly) a whole row of the output: chunks of
+  // exactly one 128-row, 128-column tile in the chunk-band layout (128K tokens at stride 16), or keys of at most 128 columns
+  // altogether (prompts of up to 2048 tokens at stride 16).  The GEMM's epilogue then finishes the block sums itself, and
+  // neither the scratch arrays nor est_rowstat_kernel / est_blocksum_kernel are needed.
+  bool direct = !use_pairs && g.tile_n == 128 && g.rbs <= 32 && 32 % g.rbs == 0;
+  if (g.band)
+    direct = direct && g.compact && g.m_pitch == 1 && g.rcs == kTileM && g.row_off % 128 == 0 && g.bpc == 128 / g.rbs &&
+             g.bpc % 4 == 0 && (reinterpret_cast<uintptr_t>(attn_sums) & 15) == 0;
+  else
+    direct = direct && g.kb_total <= 256 / g.rbs;
   for (int mt = 0; direct && mt < g.n_mtiles; ++mt) {
     int first, count;
     row_tile_range(g, mt, first, count);
-    direct = count == 1 && first * 128 == (mt * kTileM / g.rcs) * g.rcs + g.row_off;
+    direct = g.band ? count == 1 && first * 128 == (mt * kTileM / g.rcs) * g.rcs + g.row_off : count <= 1 && first == 0;
   }
-#ifdef XB_EST_NO_DIRECT
-  direct = false;
-#endif
-  // ragged lengths: stage the tile with the last (partial) stride group and map it like the tensor itself
-  CUtensorMap tmQt = tmQ, tmKt = tmK;
-  auto stage_tail = [&](const void* src, int64_t sb, int64_t sh, int64_t sl, int heads, int len, int tile_rows,
-                        int tail_tile, size_t off, uint32_t box_rows, CUtensorMap* map) -> int {
-    if ((sb % 8) || (sh % 8) || (sl % 8) || (head_dim % 8)) return XATTN_B200_ERR_ARG;
-    const int n_tokens = tile_rows * stride;
-    const size_t total_vec = static_cast<size_t>(batch) * heads * n_tokens * (head_dim / 8);
-    size_t blocks = (total_vec + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    est_tail_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(
-        static_cast<const uint4*>(src), sb, sh, sl, heads, len, head_dim, tail_tile * n_tokens, n_tokens,
-        reinterpret_cast<uint4*>(ws + off), total_vec);
-    int r = launch_status();
-    if (r) return r;
-    const uint64_t dims[5] = {(uint64_t)head_dim, (uint64_t)stride, (uint64_t)tile_rows, (uint64_t)heads,
-                              (uint64_t)batch};
-    const uint64_t tok = (uint64_t)head_dim * 2;
-    const uint64_t s_h = heads > 1 ? tok * n_tokens : 256, s_b = batch > 1 ? tok * n_tokens * heads : 256;
-    const uint64_t str[4] = {tok, tok * stride, s_h, s_b};
-    const uint32_t box[5] = {kTileK, 1, box_rows, 1, 1};
-    return make_tmap_16bit(map, ws + off, 5, dims, str, box);
-  };
-  if (g.q_tail_mt >= 0 &&
-      (rc = stage_tail(q, qsb, qsh, qsl, hq, q_len, kTileM, g.q_tail_mt, w.off_qtail, kTileM, &tmQt)))
-    return rc;
-  if (g.k_tail_nt >= 0 && (rc = stage_tail(k, ksb, ksh, ksl, hkv, k_len, g.tile_n, g.k_tail_nt, w.off_ktail,
-                                           use_pairs ? 128 : static_cast<uint32_t>(g.tile_n), &tmKt)))
-    return rc;
+  g.direct = direct ? 1 : 0;
+  CUtensorMap tmQ, tmK, tmQt, tmKt;
+  const uint32_t k_box = use_pairs ? 128 : static_cast<uint32_t>(g.tile_n);     // pairs: one CTA's half of a 256-column tile
+  if ((rc = make_map(&tmQ, q, q_len, hq, qsb, qsh, qsl, kTileM, false))) return rc;
+  if ((rc = make_map(&tmK, k, k_len, hkv, ksb, ksh, ksl, k_box, false))) return rc;
+  tmQt = tmQ;
+  tmKt = tmK;
+  if (g.q_rem && (rc = make_map(&tmQt, q, q_len, hq, qsb, qsh, qsl, kTileM, true))) return rc;
+  if (g.k_rem && (rc = make_map(&tmKt, k, k_len, hkv, ksb, ksh, ksl, k_box, true))) return rc;
 
   if (g.n_mtiles <= kTabTiles) {
     // few row tiles: the tables travel in the kernel parameters (the arithmetic of est_setup_kernel, on the host)
@@ -1140,14 +1144,6 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
 
   const int sms = sm_count();
   if (use_pairs) {
-    CUtensorMap tmKh;                     // K with a box of 128 rows: one CTA's half of a 256-column tile
-    {
-      const uint64_t dims[5] = {row_len, (uint64_t)stride, (uint64_t)(k_len / stride), (uint64_t)hkv,
-                                (uint64_t)batch};
-      const uint64_t str[4] = {(uint64_t)ksl * 2, (uint64_t)ksl * 2 * stride, (uint64_t)ksh * 2, (uint64_t)ksb * 2};
-      const uint32_t box[5] = {kTileK, 1, 128, 1, 1};
-      if ((rc = make_tmap_16bit(&tmKh, k, 5, dims, str, box))) return rc;
-    }
     const uint32_t idesc2 = make_idesc_f16(2 * kTileM, kTileN, dtype != XATTN_B200_F16, false, false);
     auto launch_pair = [&](auto kern) -> int {
       if (!allow_smem(kern, kPairSmem))
@@ -1171,7 +1167,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       });
       if (max_clusters < 1) return XATTN_B200_ERR_CUDA;
       if (static_cast<unsigned>(2 * max_clusters) < cfg.gridDim.x) cfg.gridDim.x = 2 * max_clusters;
-      if (cudaLaunchKernelEx(&cfg, kern, tmQ, tmKh, tmQt, tmKt, g, (const int*)pair_lo, (const int*)pair_prefix,
+      if (cudaLaunchKernelEx(&cfg, kern, tmQ, tmK, tmQt, tmKt, g, (const int*)pair_lo, (const int*)pair_prefix,
                              partial, mtile, idesc2, status) != cudaSuccess)
         return XATTN_B200_ERR_CUDA;
       return launch_status();

@@ -155,15 +155,8 @@ struct EstimateArgs {
   bool causal, band;
 };
 // fp32 block sums [B, Hq, q_blocks_pad, k_blocks_pad or blocks_per_chunk]
-Tensor estimate(Operand& q, Operand& k, int64_t D, const Geometry& g, const EstimateArgs& a, const Place& at_) {
+Tensor estimate(const Operand& q, const Operand& k, int64_t D, const Geometry& g, const EstimateArgs& a, const Place& at_) {
   const int64_t B = q.t.size(0), Hq = q.t.size(1), Hkv = k.t.size(1);
-  // (the staging tiles of ragged lengths are sized for head_dim 128)
-  if (q.dtype != XATTN_B200_F32_TERMS && D != 128)
-    for (Operand* o : {&q, &k})
-      if (o->len % a.stride) {
-        o->t = at::constant_pad_nd(o->t, {0, 0, 0, a.stride - o->len % a.stride});
-        o->len = o->t.size(2);
-      }
   const int sem = a.band ? XATTN_B200_SEMANTICS_TORCH_BAND : a.semantics;
   const size_t bytes = xattn_b200_estimate_workspace_bytes_ex(B, Hq, q.len, k.len, a.stride, a.block, a.chunk, a.causal, sem);
   if (bytes == 0)
@@ -271,7 +264,7 @@ PyObject* py_estimate(PyObject*, PyObject* const* v, Py_ssize_t n) {
   EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), a.flag(8)};
   const Geometry g = geometry(q.size(2), k.size(2), e.chunk, e.stride, e.block);
   const bool f32 = q.scalar_type() == at::kFloat;
-  Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
+  const Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
   return wrap(estimate(qo, ko, q.size(3), g, e, at_));
   END_HANDLE_TH_ERRORS
 }
@@ -384,7 +377,7 @@ PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   Tensor out;
   if (!a.none(12)) out = a.tensor(12);
   const bool f32 = q.scalar_type() == at::kFloat;
-  Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
+  const Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
   Selection s;
   {
     const Tensor sums = estimate(qo, ko, D, g, e, at_);
@@ -417,7 +410,7 @@ PyObject* py_estimate_and_select(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   const EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), false};
   const Geometry g = geometry(q.size(2), k.size(2), e.chunk, e.stride, e.block);
   const bool f32 = q.scalar_type() == at::kFloat;
-  Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
+  const Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
   const Tensor sums = estimate(qo, ko, q.size(3), g, e, at_);
   const Selection s = select(sums, pv[8], {g.bpc, g.block_offset, e.causal, true, a.flag(9), a.flag(10), true, 0, 0, 0}, at_);
   PyObject* t = PyTuple_New(2);
