@@ -4,12 +4,16 @@
 // xattn_estimate (xattn/src/Xattention.py:255-263), and the post-processing at
 // xattn/src/Xattention.py:275-297.  The reference sorts every row twice in fp64 with torch.sort,
 // builds cumulative sums with cat/cumsum and scatters, once per chunk with two host syncs.  Here one
-// launch covers all chunks and one WARP owns one (head, query-block) row, staged in shared memory.
-// Attention rows are peaked, so the kept set is small: the warp extracts the largest remaining score
-// (lowest index on ties) one at a time, accumulating the prefix in fp64 exactly as the rule is
-// stated, and stops at the first rank that is not taken.  Rows that are still going after
-// kPeelMax extractions (flat score rows) switch to a warp-level bitonic sort of what is left (every warp
-// has its own sort buffer) plus an fp64 prefix scan.  Both routes apply the same rule, so the result does not depend on the route.
+// launch covers all chunks and one WARP owns one (head, query-block) row.  The kept set is the first K of the ranked
+// scores, and K needs no ranking: it follows from the value at which the sum of the larger scores reaches what is wanted.
+//   * Rows of up to 1024 key blocks (select_reg_kernel): the row sits in the warp's registers.  The first few ranks of short
+//     rows are taken one by one (attention rows are peaked: most rows of a text keep two to four blocks); otherwise the cut
+//     value is found by bisection on the bit patterns of the scores, summing in fp64.  The bitmaps are a word per lane.
+//   * Longer rows (select_kernel): staged in shared memory; the largest remaining score is extracted one at a time, and
+//     rows that are still going after kPeelMax of them are sorted.
+// Both accumulate in fp64 exactly as the rule is stated.
+// Latency and instructions bound it, not bytes: 24 heads x 931 rows of 944 flat scores (video diffusion) took 1128 us with the
+// sort, 149 us with the bisection; 32 x 1024 rows of 16 scores (128K tokens) 27 -> 19 us.
 //
 // Rule per row R (chunk c = R / bpc, current_index cur = block_offset + c*bpc, diagonal d = cur + R%bpc),
 // scores x[0..N) taken as fp64, req = sum(x) * threshold:
@@ -114,9 +118,6 @@ __device__ __forceinline__ void warp_sort_desc(unsigned long long* __restrict__ 
 // Zero-score columns are not stored: all of them rank after the positive ones, in column order, and the rule
 // can only take the first of them or all of them (see below).  Taken columns are a bitmap, so the mask row and
 // the ascending block list are produced word by word.
-// kMaxSeg: the longest row the register sort is compiled for, in keys per lane (4 / 16 / 32: rows of up to 128 /
-// 512 / 1024 key blocks; the kernel's register count, and with it the warps per SM, follows the largest one).
-template <int kMaxSeg>
 __global__ void __launch_bounds__(256) select_kernel(const float* __restrict__ sums, const SelParams p,
                               const float* __restrict__ thr_per_head, uint8_t* __restrict__ mask_out,
                               int32_t* __restrict__ idx_out, int32_t* __restrict__ cnt_out, int* status) {
@@ -267,17 +268,13 @@ __global__ void __launch_bounds__(256) select_kernel(const float* __restrict__ s
       {
         int np2 = 32;
         while (np2 < M) np2 <<= 1;
-        if (np2 <= 32 * kMaxSeg) {
+        if (np2 <= 1024) {
           if (np2 == 32) warp_sort_desc<1>(keys, cval, cidx, M, lane);
           else if (np2 == 64) warp_sort_desc<2>(keys, cval, cidx, M, lane);
           else if (np2 == 128) warp_sort_desc<4>(keys, cval, cidx, M, lane);
-          if constexpr (kMaxSeg >= 16) {
-            if (np2 == 256) warp_sort_desc<8>(keys, cval, cidx, M, lane);
-            else if (np2 == 512) warp_sort_desc<16>(keys, cval, cidx, M, lane);
-          }
-          if constexpr (kMaxSeg >= 32) {
-            if (np2 == 1024) warp_sort_desc<32>(keys, cval, cidx, M, lane);
-          }
+          else if (np2 == 256) warp_sort_desc<8>(keys, cval, cidx, M, lane);
+          else if (np2 == 512) warp_sort_desc<16>(keys, cval, cidx, M, lane);
+          else warp_sort_desc<32>(keys, cval, cidx, M, lane);
         } else {
           // longer rows: the same network on the shared-memory array
           for (int t = lane; t < np2; t += 32) {
@@ -429,6 +426,289 @@ __global__ void __launch_bounds__(256) select_kernel(const float* __restrict__ s
   if (want_list && lane == 0) cnt_out[static_cast<size_t>(bh) * p.list_q_blocks + R] = base;
 }
 
+// Post-processing and outputs of one row: `word` is the lane's 32-column word of the taken columns (k_blocks <= 1024).
+struct RowOut {
+  uint8_t* mask;        // the row of the mask, or null
+  int32_t* list;        // the row's list, or null
+  int32_t* cnt;
+};
+__device__ __forceinline__ void finish_row(const SelParams& p, int R, int cur, uint32_t word, int lane, const RowOut& o) {
+  const int N = p.k_blocks;
+  const uint32_t valid = bits_le(N - 1, lane);
+  int hi_keep = N - 1;                             // causal clean-up: columns above are cleared
+  if (p.causal) {
+    hi_keep = cur + p.bpc - 1;
+    if (p.diagonal_cleanup && p.block_offset + R < hi_keep) hi_keep = p.block_offset + R;
+  }
+  const int recent = p.block_offset + R;
+  word &= valid & bits_le(hi_keep, lane);
+  if (p.keep_sink && R == 0) word = valid;
+  if (p.keep_recent && recent < N && (recent >> 5) == lane) word |= 1u << (recent & 31);
+  if (o.mask && 32 * lane < N) {
+    uint8_t* mo = o.mask + 32 * lane;
+    if (p.vec_mask && 32 * lane + 32 <= N) {
+      uint32_t b[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) b[q] = (((word >> (4 * q)) & 15u) * 0x00204081u) & 0x01010101u;
+      reinterpret_cast<uint4*>(mo)[0] = make_uint4(b[0], b[1], b[2], b[3]);
+      reinterpret_cast<uint4*>(mo)[1] = make_uint4(b[4], b[5], b[6], b[7]);
+    } else {
+      for (int q = 0; q < 32 && 32 * lane + q < N; ++q) mo[q] = static_cast<uint8_t>((word >> q) & 1u);
+    }
+  }
+  if (o.list) {
+    int hi_list = p.list_k_blocks - 1;             // columns the block list may hold
+    if (p.causal) {
+      // last token of query block R sees keys up to this position (query end aligned to key end)
+      int last_q = R * 128 + 127;
+      if (last_q > p.list_q_len - 1) last_q = p.list_q_len - 1;
+      const long long lim = static_cast<long long>(last_q) + (p.list_k_len - p.list_q_len);
+      const int jm = lim < 0 ? -1 : static_cast<int>(lim / 128);
+      if (jm < hi_list) hi_list = jm;
+    }
+    uint32_t lw = word & bits_le(hi_list, lane);
+    int incl = __popc(lw);
+    const int own = incl;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, s);
+      if (lane >= s) incl += up;
+    }
+    int pos = incl - own;
+    while (lw) {
+      o.list[pos++] = 32 * lane + __ffs(lw) - 1;
+      lw &= lw - 1;
+    }
+    if (lane == 31) *o.cnt = incl;
+  }
+}
+
+// Rows of up to 128 * kVec stored scores and up to 1024 key blocks, in registers: lane l holds the columns
+// 128 u + 4 l + e of the stored part (u < kVec, e < 4).
+template <int kVec>
+__global__ void __launch_bounds__(256) select_reg_kernel(const float* __restrict__ sums, const SelParams p,
+                                                         const float* __restrict__ thr_per_head, uint8_t* __restrict__ mask_out,
+                                                         int32_t* __restrict__ idx_out, int32_t* __restrict__ cnt_out) {
+  const int lane = threadIdx.x & 31;
+  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (w >= p.rows_total) return;                   // whole warps leave
+  constexpr unsigned kAll = 0xffffffffu;
+  const int bh = w / p.q_blocks;
+  const int R = w - bh * p.q_blocks;
+  const int N = p.k_blocks;
+  const int cur = p.block_offset + (R / p.bpc) * p.bpc;
+  const int d = cur + R % p.bpc;
+  const bool f0 = p.causal && cur != 0;            // block 0 forced
+  const int n_forced = p.causal ? (f0 ? 2 : 1) : 0;
+  const bool lag = n_forced == 1;
+  const int n_read = p.band ? p.bpc : N;
+  const int col0 = p.band ? cur : 0;
+  const float* x = sums + static_cast<size_t>(w) * n_read;
+  const double thr = thr_per_head ? static_cast<double>(__ldg(thr_per_head + bh % p.heads)) : p.threshold;
+
+  // ---- the row, once; scores as bit patterns (positive floats order like integers), forced and non-positive ones as 0
+  uint32_t v[4 * kVec];
+#pragma unroll
+  for (int u = 0; u < kVec; ++u) {
+    const int j = u * 128 + 4 * lane;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.vec_in) {
+      if (j < n_read) q = __ldg(reinterpret_cast<const float4*>(x + j));
+    } else {
+      if (j < n_read) q.x = __ldg(x + j);
+      if (j + 1 < n_read) q.y = __ldg(x + j + 1);
+      if (j + 2 < n_read) q.z = __ldg(x + j + 2);
+      if (j + 3 < n_read) q.w = __ldg(x + j + 3);
+    }
+    v[4 * u] = __float_as_uint(q.x); v[4 * u + 1] = __float_as_uint(q.y);
+    v[4 * u + 2] = __float_as_uint(q.z); v[4 * u + 3] = __float_as_uint(q.w);
+  }
+  double part = 0.0, fpart = 0.0;
+  int m = 0;
+#pragma unroll
+  for (int k = 0; k < 4 * kVec; ++k) {
+    const int jj = col0 + (k >> 2) * 128 + 4 * lane + (k & 3);
+    const float f = __uint_as_float(v[k]);
+    const double df = static_cast<double>(f);
+    part += df;
+    const bool forced = p.causal && (jj == d || (f0 && jj == 0));
+    if (forced) fpart += df;
+    if (forced || !(f > 0.f)) v[k] = 0u;
+    m += v[k] != 0u;
+  }
+  const double total = warp_sum(part), fsum = warp_sum(fpart);
+  const int M = __reduce_add_sync(kAll, m);
+  const double req = total * thr;
+
+  uint32_t word = 0u;                              // taken columns, 32 per lane
+  auto take = [&](int col) { if (lane == (col >> 5)) word |= 1u << (col & 31); };
+  if (p.causal) {
+    take(d);
+    if (f0) take(0);
+  }
+  bool untaken = !(req > 0.0);                     // the leading slots of the reference compare 0 < req too
+  if (req > 0.0) {
+    // Ranks r = 1, 2, ... of the positive scores; prefix[r] = sum of the first r.  K = number of ranks with
+    // fsum + prefix[r - 1] < req; without lag the first K ranks are taken, with it the first K + 1.
+    int K = 0;
+    double above = 0.0;                            // prefix[K]
+    bool cut = !(fsum < req);                      // the rank after the first K is refused (without lag)
+    // lowest column that holds the bit pattern `best`
+    auto column_of = [&](uint32_t best) {
+      int c = 0x7fffffff;
+#pragma unroll
+      for (int k = 4 * kVec - 1; k >= 0; --k)
+        if (v[k] == best) c = (k >> 2) * 128 + 4 * lane + (k & 3);
+      return __reduce_min_sync(kAll, c);
+    };
+    auto remove = [&](int c) {                     // (stored column)
+#pragma unroll
+      for (int k = 0; k < 4 * kVec; ++k)
+        if (c == (k >> 2) * 128 + 4 * lane + (k & 3)) v[k] = 0u;
+    };
+    auto largest = [&]() {
+      uint32_t b = 0u;
+#pragma unroll
+      for (int k = 0; k < 4 * kVec; ++k) b = v[k] > b ? v[k] : b;
+      return __reduce_max_sync(kAll, b);
+    };
+    auto take_next = [&]() {                       // the largest remaining score, lowest column on ties
+      const uint32_t b = largest();
+      const int c = column_of(b);
+      remove(c);
+      take(col0 + c);
+      return b;
+    };
+    if (kVec <= 2) {
+      // short rows: the first ranks one at a time
+#pragma unroll 1
+      for (int n = 0; n < kPeelProbe && K < M && !cut; ++n) {
+        above += static_cast<double>(__uint_as_float(take_next()));
+        ++K;
+        cut = !(fsum + above < req);
+      }
+    }
+    if (!cut && K < M) {
+      // Bisection for the cut value: scores with pattern > hi are taken (their sum keeps fsum + above below req), the scores
+      // in (lo, hi] are undecided.
+      uint32_t hi = largest(), lo = 0u;
+      int inside = M - K;
+#pragma unroll 1
+      while (inside > 1 && hi - lo > 1u) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        double s = 0.0;
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < 4 * kVec; ++k)
+          if (v[k] > mid && v[k] <= hi) {
+            s += static_cast<double>(__uint_as_float(v[k]));
+            ++n;
+          }
+        s = warp_sum(s);
+        n = __reduce_add_sync(kAll, n);
+        if (fsum + (above + s) < req) {
+          above += s;
+          K += n;
+          inside -= n;
+          hi = mid;
+        } else {
+          lo = mid;
+          inside = n;
+        }
+      }
+      // the scores in (lo, hi] are equal: in column order until the sum reaches req
+      uint32_t tie = 0u;
+#pragma unroll
+      for (int k = 0; k < 4 * kVec; ++k)
+        if (v[k] > lo && v[k] <= hi) tie = v[k];
+      tie = __reduce_max_sync(kAll, tie);
+      int e = 0;
+      const double step = static_cast<double>(__uint_as_float(tie)), base = above;
+#pragma unroll 1
+      while (e < inside && fsum + above < req) {
+        ++e;
+        above = base + step * e;
+      }
+      K += e;
+      cut = !(fsum + above < req);
+      if (e == inside) {                           // (the usual case: one score, and it is taken)
+        hi = lo;
+        e = 0;
+      }
+      // taken so far: every score above hi.  Four ballots hold 128 columns, bit l of ballot e being column 4 l + e; lane
+      // 4 u + q builds the word of columns 128 u + 32 q ...
+      uint32_t stored = 0u;
+#pragma unroll
+      for (int u = 0; u < kVec; ++u) {
+        uint32_t wd = 0u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint32_t t = (__ballot_sync(kAll, v[4 * u + q] > hi) >> (8 * (lane & 3))) & 0xffu;
+          t = (t | (t << 12)) & 0x000f000fu;
+          t = (t | (t << 6)) & 0x03030303u;
+          t = (t | (t << 3)) & 0x11111111u;
+          wd |= t << q;
+        }
+        if ((lane >> 2) == u) stored = wd;
+      }
+#pragma unroll
+      for (int k = 0; k < 4 * kVec; ++k)
+        if (v[k] > hi) v[k] = 0u;
+      // from stored columns to key blocks: shifted by col0
+      {
+        const int t = lane - (col0 >> 5), sh = col0 & 31;
+        const uint32_t a = __shfl_sync(kAll, stored, t & 31), b = __shfl_sync(kAll, stored, (t - 1) & 31);
+        uint32_t wd = 0u;
+        if (t >= 0 && t < 4 * kVec) wd = a << sh;
+        if (sh && t >= 1 && t <= 4 * kVec) wd |= b >> (32 - sh);
+        word |= wd;
+      }
+#pragma unroll 1
+      for (; e > 0; --e) {                         // some of several equal scores
+        const int c = column_of(tie);
+        remove(c);
+        take(col0 + c);
+      }
+    }
+    int n_taken = K;
+    if (lag && K < M) {
+      take_next();
+      n_taken = K + 1;
+    }
+    const int n_others = N - n_forced;
+    if (n_taken < M) {
+      untaken = true;
+    } else if (M < n_others) {
+      // ranks that hold a zero score (column order): all of them, the first (lag), or none
+      const bool first = lag ? K == M : total < req;
+      if (!first) {
+        untaken = true;
+      } else {
+        // zero-score columns are the valid ones not taken so far: every positive score is
+        const uint32_t zero = ~word & bits_le(N - 1, lane);
+        if (total < req) {
+          word |= zero;
+        } else {
+          const int best = __reduce_min_sync(kAll, zero ? 32 * lane + __ffs(zero) - 1 : 0x7fffffff);
+          if (best != 0x7fffffff) take(best);
+          if (M + 1 < n_others) untaken = true;
+        }
+      }
+    }
+  }
+  if (untaken) take(0);
+  RowOut o;
+  o.mask = mask_out ? mask_out + static_cast<size_t>(w) * N : nullptr;
+  o.list = nullptr;
+  o.cnt = nullptr;
+  if (idx_out && cnt_out && R < p.list_q_blocks) {
+    const size_t row = static_cast<size_t>(bh) * p.list_q_blocks + R;
+    o.list = idx_out + row * p.list_k_blocks;
+    o.cnt = cnt_out + row;
+  }
+  finish_row(p, R, cur, word, lane, o);
+}
+
 __device__ __forceinline__ bool list_keeps(int causal, int R, int j, int list_q_len, int list_k_len) {
   if (!causal) return true;
   // last token of query block R sees keys up to this position (query end aligned to key end)
@@ -494,23 +774,28 @@ int select_launch(const float* attn_sums, int batch, int heads, int q_blocks, in
   // 16-byte accesses to the rows of the scores and of the mask
   p.vec_in = (n_read % 4 == 0 && (reinterpret_cast<uintptr_t>(attn_sums) & 15) == 0) ? 1 : 0;
   p.vec_mask = (k_blocks % 16 == 0 && mask != nullptr && (reinterpret_cast<uintptr_t>(mask) & 15) == 0) ? 1 : 0;
-  int wpc = (72 * 1024) / p.per_warp_bytes;        // three CTAs per SM when rows are long
-  wpc = wpc < 1 ? 1 : (wpc > 8 ? 8 : wpc);
-  p.warps_per_cta = wpc;
   const long long rows = static_cast<long long>(batch) * heads * q_blocks;
   if (rows > 0x7fffffffLL) return XATTN_B200_ERR_LIMIT;
   p.rows_total = static_cast<int>(rows);
+  if (k_blocks <= 1024) {
+    // rows that fit the warp's registers: the instantiation with just enough of them for the stored scores
+    auto launch_reg = [&](auto kern) -> int {
+      kern<<<static_cast<int>((rows + 7) / 8), 256, 0, stream>>>(attn_sums, p, thr_per_head, mask, block_idx, block_cnt);
+      return launch_status();
+    };
+    if (n_read <= 128) return launch_reg(select_reg_kernel<1>);
+    if (n_read <= 256) return launch_reg(select_reg_kernel<2>);
+    if (n_read <= 512) return launch_reg(select_reg_kernel<4>);
+    return launch_reg(select_reg_kernel<8>);
+  }
+  int wpc = (72 * 1024) / p.per_warp_bytes;        // three CTAs per SM when rows are long
+  wpc = wpc < 1 ? 1 : (wpc > 8 ? 8 : wpc);
+  p.warps_per_cta = wpc;
   const size_t smem = static_cast<size_t>(wpc) * p.per_warp_bytes;
   const int grid = static_cast<int>((rows + wpc - 1) / wpc);
-  auto launch = [&](auto kern) -> int {
-    if (smem > 48 * 1024 &&
-        !allow_smem(kern, 160 * 1024))
-      return XATTN_B200_ERR_CUDA;
-    kern<<<grid, wpc * 32, smem, stream>>>(attn_sums, p, thr_per_head, mask, block_idx, block_cnt, status);
-    return launch_status();
-  };
-  // the instantiation whose flat-row sort holds just enough keys per lane in registers for this row length
-  return np2 > 512 ? launch(select_kernel<32>) : (np2 > 128 ? launch(select_kernel<16>) : launch(select_kernel<4>));
+  if (smem > 48 * 1024 && !allow_smem(select_kernel, 160 * 1024)) return XATTN_B200_ERR_CUDA;
+  select_kernel<<<grid, wpc * 32, smem, stream>>>(attn_sums, p, thr_per_head, mask, block_idx, block_cnt, status);
+  return launch_status();
 }
 
 int mask_to_lists_launch(const uint8_t* mask, int batch, int heads, int mask_q_blocks, int mask_k_blocks, int q_len,
