@@ -432,8 +432,9 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int interleave = g.tile_n == 128 ? group : 1;      // streaming case only: see decode_tile
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (one thread)
-    if (lane == 0) {
+    // ------------------------------------------------------------ TMA producer (converged warp, one thread issues)
+    {
+      const uint32_t lead = elect_one() ? 1u : 0u;
       int s = 0;
       uint32_t ph = 0;
       for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x) {
@@ -442,13 +443,13 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int b = bh / g.hq, h = bh - b * g.hq;
         int t = 0, dc = 0;
         for (int ks = 0; ks < k_steps; ++ks) {
-          if (!mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag)) break;
+          if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag))) break;
           const uint32_t dstA = smem_u32(smem + s * stage_bytes);
-          mbar_expect_tx(full0 + 8 * s, stage_bytes);
+          mbar_expect_tx_lead(full0 + 8 * s, stage_bytes, lead);
           const bool qt = g.S - 1 - t < g.q_rem, kt = t < g.k_rem;
           const int col = k_column(g, dc);
-          tma_load_5d(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b);
-          tma_load_5d(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, col, t, nt * g.tile_n + (kt ? 0 : g.k_none), h / group, b);
+          tma_load_5d_lead(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
+          tma_load_5d_lead(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, col, t, nt * g.tile_n + (kt ? 0 : g.k_none), h / group, b, lead);
           if (++dc == g.d_chunks) { dc = 0; ++t; }
           if (++s == n_stages) { s = 0; ph ^= 1; }
         }
@@ -644,8 +645,9 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int group = g.hq / g.hkv;
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (one thread per CTA)
-    if (lane == 0) {
+    // ------------------------------------------------------------ TMA producer (converged warp, one thread issues)
+    {
+      const uint32_t lead = elect_one() ? 1u : 0u;
       int s = 0;
       uint32_t ph = 0;
       for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs_grid) {
@@ -655,16 +657,16 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const int mt = 2 * pm + static_cast<int>(rank);
         int t = 0, dc = 0;
         for (int ks = 0; ks < k_steps; ++ks) {
-          if (!mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag)) break;
+          if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag))) break;
           const uint32_t dstA = smem_u32(smem + s * kPairStageBytes);
           // all four loads of a stage are counted on the even CTA's barrier
           const uint32_t full_even = mapa_shared(full0 + 8 * s, 0);
-          if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * kPairStageBytes);
+          mbar_expect_tx_lead(full0 + 8 * s, 2 * kPairStageBytes, rank == 0 ? lead : 0u);
           const bool qt = g.S - 1 - t < g.q_rem, kt = t < g.k_rem;
           const int col = k_column(g, dc);
-          tma_load_5d_pair(dstA, qt ? &tmQt : &tmQ, full_even, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b);
-          tma_load_5d_pair(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, col, t,
-                           nt * kTileN + static_cast<int>(rank) * 128 + (kt ? 0 : g.k_none), h / group, b);
+          tma_load_5d_pair_lead(dstA, qt ? &tmQt : &tmQ, full_even, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
+          tma_load_5d_pair_lead(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, col, t,
+                           nt * kTileN + static_cast<int>(rank) * 128 + (kt ? 0 : g.k_none), h / group, b, lead);
           if (++dc == g.d_chunks) { dc = 0; ++t; }
           if (++s == kPairStages) { s = 0; ph ^= 1; }
         }
