@@ -13,12 +13,23 @@ import torch
 
 from . import _lib
 
-try:
-    from . import _host
-except ImportError as e:
-    raise _lib.XattnB200Error(f"_host.so is missing or does not load ({e}): build it with `python -m xattn_b200.build` "
-                              "(there is no fallback for this path)") from e
 
+class _Host:
+    """The functions of the CPython module _host, which is loaded at the first use of one: the package has to be
+    importable before anything is built (the build itself is part of it)."""
+
+    def __getattr__(self, name):
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise _lib.XattnB200Error(f"_host.so is missing or does not load ({e}): build it with `python -m "
+                                      "xattn_b200.build` (there is no fallback for this path)") from e
+        module.init(_lib.XattnB200Error, lambda index: _status(torch.device("cuda", index)).data_ptr())
+        self.__dict__.update({k: v for k, v in vars(module).items() if not k.startswith("_")})
+        return self.__dict__[name]
+
+
+_host = _Host()
 _DT = {torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
 _SEM = {"torch": _lib.SEMANTICS_TORCH, "triton": _lib.SEMANTICS_TRITON}
 
@@ -53,9 +64,6 @@ def _status(device: torch.device) -> torch.Tensor:
         w = torch.zeros(1, dtype=torch.int32).pin_memory()
         _status_words[key] = w
     return w
-
-
-_host.init(_lib.XattnB200Error, lambda index: _status(torch.device("cuda", index)).data_ptr())
 
 
 def check_device_status(device: Optional[torch.device] = None, synchronize: bool = True) -> None:
