@@ -71,39 +71,33 @@ struct Tile {
 __device__ __forceinline__ size_t tile_row(const AttnParams& p, const Tile& t) {
   return (static_cast<size_t>(t.b) * p.hq + t.h) * p.q_blocks + t.qb;
 }
-// The tiles of unit u.  With a tile list: its entries 2u and 2u+1 (-1: none), tile i being (b, h, qb) with qb from the last
-// to the first.  Otherwise a "super row" is two query blocks hi, hi-1; its hq units per batch entry are, for each kv head,
-// the pairs of query heads at hi, then those at hi-1, and for an odd group first one unit that takes the last head at hi
-// and hi-1.  Causal: super row by super row, the heaviest (last) first.  Non-causal: kv head by kv head, so that the CTAs
-// work on one head's K and V at a time.
-__device__ __forceinline__ void unit_tiles(const AttnParams& p, int u, Tile& t0, Tile& t1) {
-  if (p.tile_list) {
-    auto decode = [&](int i, Tile& t) {
-      t.b = t.h = 0;
-      t.qb = -1;
-      if (i < 0) return;
-      const int rest = fast_div(i, p.by_hq, t.h);
-      t.qb = p.q_blocks - 1 - fast_div(rest, p.by_batch, t.b);
-    };
-    int i0 = -1, i1 = -1;
-    if (2 * u < p.list_tiles) i0 = __ldg(p.tile_list + 2 * u);
-    if (2 * u + 1 < p.list_tiles) i1 = __ldg(p.tile_list + 2 * u + 1);
-    decode(i0, t0);
-    decode(i1, t1);
+// Tile s of unit u.  With a tile list (kList, and one given): its entries 2u and 2u+1 (-1: none), tile i being (b, h, qb)
+// with qb from the last to the first.  Otherwise a "super row" is two query blocks hi, hi-1; its hq units per batch entry
+// are, for each kv head, the pairs of query heads at hi, then those at hi-1, and for an odd group first one unit that takes
+// the last head at hi and hi-1.  Causal: super row by super row, the heaviest (last) first.  Non-causal: kv head by kv
+// head, so that the CTAs work on one head's K and V at a time.
+template <bool kList>
+__device__ __forceinline__ Tile unit_tile(const AttnParams& p, int u, int s) {
+  Tile t;
+  if (kList && p.tile_list) {
+    t.b = t.h = 0;
+    t.qb = -1;
+    const int i = 2 * u + s < p.list_tiles ? __ldg(p.tile_list + 2 * u + s) : -1;
+    if (i < 0) return t;
+    const int rest = fast_div(i, p.by_hq, t.h);
+    t.qb = p.q_blocks - 1 - fast_div(rest, p.by_batch, t.b);
   } else {
     int x, j, g;
     const int hi = fast_div(u, p.by_units, x), lo = fast_div(x, p.by_group, j);
     const int r = p.causal ? hi : lo, bg = p.causal ? lo : hi;
-    t0.b = fast_div(bg, p.by_hkv, g);
+    t.b = fast_div(bg, p.by_hkv, g);
     const int group = static_cast<int>(p.by_group.d), odd = group & 1, pairs = group >> 1;
     const int lower = j - odd >= pairs ? 1 : 0;
     const int across = odd && j == 0 ? 1 : 0;
-    t0.qb = p.q_blocks - 1 - 2 * r - (across ? 0 : lower);
-    t0.h = g * group + (across ? group - 1 : 2 * (j - odd - lower * pairs));
-    t1.b = t0.b;
-    t1.qb = t0.qb - across;
-    t1.h = t0.h + 1 - across;
+    t.qb = p.q_blocks - 1 - 2 * r - (across ? s : lower);
+    t.h = g * group + (across ? group - 1 : 2 * (j - odd - lower * pairs) + s);
   }
+  return t;
 }
 // number of listed blocks; a dense call lists every block that holds a key the tile's last row may see
 __device__ __forceinline__ int tile_count(const AttnParams& p, const int32_t* __restrict__ block_cnt, const Tile& t) {
@@ -126,9 +120,8 @@ __device__ __forceinline__ List tile_list(const AttnParams& p, const int32_t* __
   l.n = n;
   return l;
 }
-// the lane's entry of the 32-wide window at walk position j0
-__device__ __forceinline__ int list_window(const List& l, int j0, int lane) {
-  const int j = j0 + lane;
+// entry j of the list, walking order
+__device__ __forceinline__ int list_entry(const List& l, int j) {
   if (j >= l.n) return 0;
   if (!l.last) return l.n - 1 - j;
   // volatile asm pins the issue point: a plain read-only load would be sunk by the compiler to its first use,
@@ -162,8 +155,8 @@ struct Units {
 };
 
 // kBf16: bf16 or fp16 (a template parameter: as a run-time switch every packed pair cost both conversions and a select).
-// kOutF32: the output is written as fp32.
-template <bool kBf16, bool kOutF32>
+// kOutF32: the output is written as fp32.  kList: the units may come from a list.
+template <bool kBf16, bool kOutF32, bool kList>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -234,7 +227,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   // it declined.
   pdl_wait();
   AttnParams p = p_in;
-  if (rest_list && pair_path_chosen(pair_header, pair_min_share)) {
+  if (kList && rest_list && pair_path_chosen(pair_header, pair_min_share)) {
     p.tile_list = rest_list;
     p.list_tiles = *reinterpret_cast<const volatile int*>(pair_header + kPairRestCount);
   }
@@ -251,109 +244,85 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     reg_set_from<kRegLoadMma, 128>();
     if (warp == 12) {
       // ------------------------------------------------------------ K/V loader: the union of the two lists
+      // Lanes 0-15 walk the list of stream 0, lanes 16-31 that of stream 1, with a window of 16 entries each.
+      const int s = lane >> 4, wl = lane & 15;
       uint32_t step = 0;
-      int ok = 1;
-      Tile t, tn;                                       // (tile of stream 0: both read the same kv head)
-      List l0, l1, l0n, l1n;
-      int w0n, w1n, unit = blockIdx.x;
-      // unit u, the CTA's k-th: published, its lists on their way
-      auto fetch = [&](int u, uint32_t k) {
-        l0n.n = l1n.n = -1;
-        Tile t1;
-        if (u >= 0) {
-          unit_tiles(p, u, tn, t1);
-          l0n = tile_list(p, block_idx, tn, tile_count(p, block_cnt, tn));
-          l1n = tile_list(p, block_idx, t1, tile_count(p, block_cnt, t1));
-          w0n = list_window(l0n, 0, lane);
-          w1n = list_window(l1n, 0, lane);
-        }
-        if (lane == 0) {
-          if (mbar_wait(unit_empty + 8 * (k % kUnitSlots), (k / kUnitSlots & 1) ^ 1, abort_flag)) {
-            int4* out = reinterpret_cast<int4*>(unit_ring + 2 * (k % kUnitSlots));
-            out[0] = make_int4(tn.b, tn.h, tn.qb, l0n.n);
-            out[1] = make_int4(t1.b, t1.h, t1.qb, l1n.n);
-            mbar_arrive(unit_full + 8 * (k % kUnitSlots));
-          } else {
-            ok = 0;
-          }
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-      };
+      bool ok = true;
+      auto wait = [&](uint32_t b, uint32_t ph) -> bool { return __all_sync(0xffffffffu, mbar_wait(b, ph, abort_flag)); };
+      Tile tn;
+      List ln;                                          // the next unit's, with the first window
+      int wn = 0, unit = blockIdx.x;
       // the first turn of the loop has no lists to load, it only fetches those of the CTA's own unit; turn k works on the
       // CTA's unit k - 1 and requests and fetches unit k
-      l0n.n = l1n.n = 0;
-      l0n.last = l1n.last = nullptr;
-      w0n = w1n = 0;
+      ln.n = 0;
+      ln.last = nullptr;
       tn.b = tn.h = 0;
 #pragma unroll 1
       for (uint32_t k = 0; unit >= 0 && ok; ++k) {
-        t = tn; l0 = l0n; l1 = l1n;
-        int w0 = w0n, w1 = w1n;
-        if (k > 0 && lane == 0 && !rest_list) {
+        const List l = ln;
+        int i = 0, w = wn, g_;
+        const int kvh = __shfl_sync(0xffffffffu, fast_div(tn.h, p.by_group, g_), 0), b = __shfl_sync(0xffffffffu, tn.b, 0);
+        if (k > 0 && lane == 0 && !(kList && rest_list)) {
           mbar_expect_tx(answer_full, 16);
           clc_try_cancel(smem_u32(answer), answer_full);
         }
         __syncwarp();
-        int g_;
-        const int kvh = fast_div(t.h, p.by_group, g_);
-        int i0 = 0, i1 = 0;
-        int w0x = list_window(l0, 32, lane), w1x = list_window(l1, 32, lane);
+        int wx = list_entry(l, 16 + wl);
         bool fetched = false;
 #pragma unroll 1
-        while (ok) {
-          if (i0 < l0.n || i1 < l1.n) {
-            const int c0 = i0 < l0.n ? __shfl_sync(0xffffffffu, w0, i0 & 31) : -1;
-            const int c1 = i1 < l1.n ? __shfl_sync(0xffffffffu, w1, i1 & 31) : -1;
-            const int blk = c0 > c1 ? c0 : c1;
-            const bool f0 = i0 < l0.n && c0 == blk, f1 = i1 < l1.n && c1 == blk;
+        while (true) {
+          const bool have = i < l.n;
+          if (__any_sync(0xffffffffu, have)) {
+            const int c = __shfl_sync(0xffffffffu, w, (lane & 16) | (i & 15)), own = have ? c : -1;
+            const int other = __shfl_xor_sync(0xffffffffu, own, 16), blk = own > other ? own : other;
+            const bool f = have && own == blk;
+            int e = f ? (kStepUses | (i == 0 ? kStepFirst : 0) | (i == l.n - 1 ? kStepLast : 0)) << s : 0;
+            e |= __shfl_xor_sync(0xffffffffu, e, 16);
+            const int sl = step & 1;
+            const uint32_t ph = ((step >> 1) & 1) ^ 1, dst = smem_u32(smem + (2 + 2 * sl) * kTile16);
+            if (!wait(bar(sl, K_EMPTY), ph)) { ok = false; break; }
             if (lane == 0) {
-              const int sl = step & 1;
-              const uint32_t ph = ((step >> 1) & 1) ^ 1;
-              const uint32_t dst = smem_u32(smem + (2 + 2 * sl) * kTile16);
-              if (mbar_wait(bar(sl, K_EMPTY), ph, abort_flag)) {
-                XB_TRACE_EV(0x12, step);
-                ring[step & (kRingEntries - 1)] =
-                    (f0 ? kStepUses | (i0 == 0 ? kStepFirst : 0) | (i0 == l0.n - 1 ? kStepLast : 0) : 0) |
-                    (f1 ? kStepUses | (i1 == 0 ? kStepFirst : 0) | (i1 == l1.n - 1 ? kStepLast : 0) : 0) << 1;
-                mbar_expect_tx(bar(sl, K_FULL), kTile16);
-                tma_load_5d(dst, &tmK, bar(sl, K_FULL), 0, blk * 128, 0, kvh, t.b);
-              } else {
-                ok = 0;
-              }
-              if (ok && mbar_wait(bar(sl, V_EMPTY), ph, abort_flag)) {
-                XB_TRACE_EV(0x13, step);
-                mbar_expect_tx(bar(sl, V_FULL), kTile16);
-                tma_load_5d(dst + kTile16, &tmV, bar(sl, V_FULL), 0, blk * 128, 0, kvh, t.b);
-              } else {
-                ok = 0;
-              }
+              XB_TRACE_EV(0x12, step);
+              ring[step & (kRingEntries - 1)] = e;
+              mbar_expect_tx(bar(sl, K_FULL), kTile16);
+              tma_load_5d(dst, &tmK, bar(sl, K_FULL), 0, blk * 128, 0, kvh, b);
             }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (f0 && (++i0 & 31) == 0) {
-              w0 = w0x;
-              w0x = list_window(l0, i0 + 32, lane);
-            }
-            if (f1 && (++i1 & 31) == 0) {
-              w1 = w1x;
-              w1x = list_window(l1, i1 + 32, lane);
+            if (!wait(bar(sl, V_EMPTY), ph)) { ok = false; break; }
+            if (lane == 0) {
+              XB_TRACE_EV(0x13, step);
+              mbar_expect_tx(bar(sl, V_FULL), kTile16);
+              tma_load_5d(dst + kTile16, &tmV, bar(sl, V_FULL), 0, blk * 128, 0, kvh, b);
             }
             ++step;
+            if (f && (++i & 15) == 0) {
+              w = wx;
+              wx = list_entry(l, i + 16 + wl);
+            }
+            __syncwarp();
           } else if (fetched) {
             break;
           }
           if (!fetched) {
-            // the next unit's lists, on their way while this unit's blocks are loaded
+            // the next unit: published, its lists on their way while this unit's blocks are loaded
             fetched = true;
-            if (rest_list) {
+            if (kList && rest_list) {
               if (k > 0) unit += gridDim.x;
               if (unit >= rest_units) unit = -1;
             } else if (k > 0) {
-              if (!__all_sync(0xffffffffu, mbar_wait(answer_full, (k - 1) & 1, abort_flag))) { ok = 0; break; }
+              if (!wait(answer_full, (k - 1) & 1)) { ok = false; break; }
               unit = clc_answer(smem_u32(answer));
               fence_proxy_async_smem();                 // read before the next answer is written
-              __syncwarp();
             }
-            fetch(unit, k);
+            ln.n = -1;
+            if (unit >= 0) {
+              tn = unit_tile<kList>(p, unit, s);
+              ln = tile_list(p, block_idx, tn, tile_count(p, block_cnt, tn));
+              wn = list_entry(ln, wl);
+            }
+            if (!wait(unit_empty + 8 * (k % kUnitSlots), (k / kUnitSlots & 1) ^ 1)) { ok = false; break; }
+            if (wl == 0) reinterpret_cast<int4*>(unit_ring)[2 * (k % kUnitSlots) + s] = make_int4(tn.b, tn.h, tn.qb, ln.n);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(unit_full + 8 * (k % kUnitSlots));
           }
         }
       }
@@ -534,7 +503,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       }
       nt = units.tile(s);
       units.release(lane);
-      if (nt.n > 0) nwin = list_window(list_of(nt), 0, lane);
+      if (nt.n > 0) nwin = list_entry(list_of(nt), lane);
     };
     int m = 0;
     nt.n = 0;
@@ -554,12 +523,12 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       int row_last_lo = p.k_len - 1;                    // the same for the first row of the warp
       if (p.causal && t.qb * 128 + quad * 32 + k_off < row_last_lo) row_last_lo = t.qb * 128 + quad * 32 + k_off;
       float m_used = -INFINITY, l = 0.f;
-      int w = nwin, w_next = list_window(list, 32, lane);
+      int w = nwin, w_next = list_entry(list, 32 + lane);
 #pragma unroll 1
       for (int j = 0; j < n; ++j, ++bc) {
         if (j > 0 && (j & 31) == 0) {
           w = w_next;
-          w_next = list_window(list, j + 32, lane);
+          w_next = list_entry(list, j + 32 + lane);
         }
         const int k0 = __shfl_sync(0xffffffffu, w, j & 31) * 128;
         if (lane == 0) XB_TRACE_EV(0x30, bc);
@@ -842,8 +811,7 @@ attn_order_kernel(const AttnParams p, const int32_t* __restrict__ block_cnt, int
   unsigned long long lim64 = s_blocks / (8ull * sms);
   const int limit = lim64 < 64 ? 64 : (lim64 > kOrderBuckets - 2 ? kOrderBuckets - 2 : static_cast<int>(lim64));
   auto length = [&](int u) {
-    Tile t0, t1;
-    unit_tiles(p, u, t0, t1);
+    const Tile t0 = unit_tile<false>(p, u, 0), t1 = unit_tile<false>(p, u, 1);
     const int c = tile_count(p, block_cnt, t0) + tile_count(p, block_cnt, t1);
     return c < 0 ? 0 : (c > kOrderBuckets - 1 ? kOrderBuckets - 1 : c);
   };
@@ -888,8 +856,7 @@ attn_order_kernel(const AttnParams p, const int32_t* __restrict__ block_cnt, int
   for (int u = first + tid; u < first + n_seg; u += kOrderThreads) {
     const int rank = atomicAdd(&hist[kOrderBuckets - 1 - length(u)], 1);
     const int at = rank < own_long ? before + rank : all_long + first - before + (rank - own_long);
-    Tile t0, t1;
-    unit_tiles(p, u, t0, t1);
+    const Tile t0 = unit_tile<false>(p, u, 0), t1 = unit_tile<false>(p, u, 1);
     // the numbering of the tile list: ((q_blocks - 1 - qb) * batch + b) * hq + h
     auto item = [&](const Tile& t) { return t.qb < 0 ? -1 : ((p.q_blocks - 1 - t.qb) * p.batch + t.b) * p.hq + t.h; };
     sorted[2 * at] = item(t0);
@@ -991,8 +958,11 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
     return launch_dependent(kern, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tmQ, tmK,
                             tmV, tmO, p, block_idx, block_cnt, rest, pair_header, min_share, status);
   };
-  if (out_f32) return launch(block_sparse_attn_kernel<true, true>);
-  return p.is_bf16 ? launch(block_sparse_attn_kernel<true, false>) : launch(block_sparse_attn_kernel<false, false>);
+  if (p.tile_list || rest)
+    return out_f32 ? launch(block_sparse_attn_kernel<true, true, true>)
+                   : (p.is_bf16 ? launch(block_sparse_attn_kernel<true, false, true>) : launch(block_sparse_attn_kernel<false, false, true>));
+  return out_f32 ? launch(block_sparse_attn_kernel<true, true, false>)
+                 : (p.is_bf16 ? launch(block_sparse_attn_kernel<true, false, false>) : launch(block_sparse_attn_kernel<false, false, false>));
 }
 
 }  // namespace xb

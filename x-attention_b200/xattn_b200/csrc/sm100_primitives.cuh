@@ -92,11 +92,12 @@ __device__ __forceinline__ uint32_t clock32() {
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   static_assert(kWaitCycleLimit > 0 && kWaitCycleLimit < (1LL << 32), "wait limit");
   if (mbar_try_wait(bar, parity)) return true;
-  const uint32_t t0 = clock32();
+  uint32_t t0 = 0;
 #pragma unroll 1
   while (!mbar_try_wait_hint(bar, parity, 20000u)) {
-    if (*abort_flag) return false;
-    if (clock32() - t0 > static_cast<uint32_t>(kWaitCycleLimit)) {
+    const uint32_t t = clock32() | 1u;
+    if (t0 == 0) t0 = t;
+    if (*abort_flag || t - t0 > static_cast<uint32_t>(kWaitCycleLimit)) {
       *abort_flag = 1;
       return false;
     }
