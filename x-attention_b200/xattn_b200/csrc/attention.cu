@@ -795,6 +795,7 @@ attn_order_kernel(const AttnParams p, const int32_t* __restrict__ block_cnt, int
   __shared__ unsigned long long s_blocks;
   __shared__ int s_long[3];           // very long units: of all heads, of the heads before this one, of this one
   pdl_launch_dependents();            // the attention kernel may take its place; it waits for this grid to end
+  pdl_wait();
   const int tid = threadIdx.x;
   const int n_seg = static_cast<int>(p.by_units.d);                      // units of a (batch, kv head)
   const int n_heads = gridDim.x, first = blockIdx.x * n_seg;
@@ -940,8 +941,8 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
     if (workspace_bytes < order_workspace_bytes(batch, hq, q_len)) return XATTN_B200_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace) & 15) != 0) return XATTN_B200_ERR_ARG;
     int32_t* sorted = static_cast<int32_t*>(workspace);
-    attn_order_kernel<<<batch * hkv, kOrderThreads, 0, stream>>>(p, block_cnt, sm_count(), sorted);
-    if ((rc = launch_status())) return rc;
+    if ((rc = launch_dependent(attn_order_kernel, dim3(batch * hkv), dim3(kOrderThreads), 0, stream, p, block_cnt, sm_count(), sorted)))
+      return rc;
     p.tile_list = sorted;
     p.list_tiles = static_cast<int>(2 * units);
   } else if (workspace && !dense && !out_f32 && pair_path_applies(hq, hkv, k_len)) {

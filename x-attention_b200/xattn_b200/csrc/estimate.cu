@@ -127,6 +127,8 @@ __host__ __device__ inline void row_tile_range(const EstGeom& g, int mt, int& fi
 __global__ void est_setup_kernel(EstGeom g, int* __restrict__ tile_lo, int* __restrict__ tile_prefix,
                                  int* __restrict__ pair_lo, int* __restrict__ pair_prefix) {
   extern __shared__ int s_cnt[];                  // [n_mtiles] tile counts, then [n_mtiles] first tiles
+  pdl_launch_dependents();
+  pdl_wait();
   int* s_lo = s_cnt + g.n_mtiles;
   for (int mt = threadIdx.x; mt < g.n_mtiles; mt += blockDim.x) {
     row_tile_range(g, mt, s_lo[mt], s_cnt[mt]);
@@ -423,6 +425,8 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_launch_dependents();
+  pdl_wait();                       // up to here nothing was touched that an earlier kernel writes
   const uint32_t tmem_base = *tmem_slot;
 
   const int tiles_per_head = tile_prefix[g.n_mtiles];
@@ -636,6 +640,8 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before();
   cluster_sync_all();               // barriers of both CTAs are initialised before any remote arrival or copy
   tc_fence_after();
+  pdl_launch_dependents();
+  pdl_wait();                       // up to here nothing was touched that an earlier kernel writes
   const uint32_t tmem_base = *tmem_slot;
 
   const int n_groups = (g.n_mtiles + 1) / 2;
@@ -790,6 +796,8 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 __global__ void __launch_bounds__(256)
 est_rowstat_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
                    const float2* __restrict__ mtile, float2* __restrict__ rowstat, int total_rows) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total_rows) return;
   const int i = idx % g.rows_total;
@@ -820,6 +828,8 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
                     const float* __restrict__ partial, const float2* __restrict__ mtile,
                     const float2* __restrict__ rowstat, float* __restrict__ sums) {
   __shared__ float2 s_stat[32];                            // FUSED: (m_i, 1/l_i) of the query block's rows (rbs <= 32)
+  pdl_launch_dependents();
+  pdl_wait();
   const int qb = blockIdx.y, bh = blockIdx.z;
   const int i0 = qb * g.rbs;
   if (FUSED) {
@@ -892,6 +902,8 @@ template <int kTerms>
 __global__ void __launch_bounds__(256)
 split_f32_kernel(const float* __restrict__ x, int heads, int len, int len_valid, int vecs, int64_t sb, int64_t sh, int64_t sl,
                  uint4* __restrict__ out, size_t total) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < total;
        e += static_cast<size_t>(gridDim.x) * blockDim.x) {
     const int d = static_cast<int>(e % vecs);
@@ -1140,8 +1152,9 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     p_prefix[n_pairs] = acc;
     g.tab_n = g.n_mtiles;
   } else {
-    est_setup_kernel<<<1, 256, 2 * sizeof(int) * g.n_mtiles, stream>>>(g, tile_lo, tile_prefix, pair_lo, pair_prefix);
-    if ((rc = launch_status())) return rc;
+    if ((rc = launch_dependent(est_setup_kernel, dim3(1), dim3(256), 2 * sizeof(int) * g.n_mtiles, stream, g, tile_lo, tile_prefix,
+                               pair_lo, pair_prefix)))
+      return rc;
   }
 
   const int sms = sm_count();
@@ -1169,10 +1182,8 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       });
       if (max_clusters < 1) return XATTN_B200_ERR_CUDA;
       if (static_cast<unsigned>(2 * max_clusters) < cfg.gridDim.x) cfg.gridDim.x = 2 * max_clusters;
-      if (cudaLaunchKernelEx(&cfg, kern, tmQ, tmK, tmQt, tmKt, g, (const int*)pair_lo, (const int*)pair_prefix,
-                             partial, mtile, idesc2, status) != cudaSuccess)
-        return XATTN_B200_ERR_CUDA;
-      return launch_status();
+      return launch_dependent_clusters(kern, 2, cfg.gridDim, cfg.blockDim, kPairSmem, stream, tmQ, tmK, tmQt, tmKt, g,
+                                       (const int*)pair_lo, (const int*)pair_prefix, partial, mtile, idesc2, status);
     };
     switch (g.rbs) {
       case 4: rc = launch_pair(est_gemm_pair_kernel<4>); break;
@@ -1188,9 +1199,8 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   auto launch = [&](auto kern) -> int {
     if (!allow_smem(kern, kGemmSmem))
       return XATTN_B200_ERR_CUDA;
-    kern<<<grid, kGemmThreads, kGemmSmem, stream>>>(tmQ, tmK, tmQt, tmKt, g, tile_lo, tile_prefix, partial, mtile,
-                                                    attn_sums, idesc, status);
-    return launch_status();
+    return launch_dependent(kern, dim3(grid), dim3(kGemmThreads), kGemmSmem, stream, tmQ, tmK, tmQt, tmKt, g,
+                            (const int*)tile_lo, (const int*)tile_prefix, partial, mtile, attn_sums, idesc, status);
   };
   if (direct) {
     switch (g.rbs) {
@@ -1224,21 +1234,19 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
 #endif
   const bool fused = max_tiles_per_row <= 8 && per_row >= XB_FUSE_MIN;
   if (!fused) {
-    est_rowstat_kernel<<<static_cast<int>((total_rows + 255) / 256), 256, 0, stream>>>(
-        g, tile_lo, tile_prefix, mtile, rowstat, static_cast<int>(total_rows));
-    if ((rc = launch_status())) return rc;
+    if ((rc = launch_dependent(est_rowstat_kernel, dim3(static_cast<unsigned>((total_rows + 255) / 256)), dim3(256), 0, stream, g,
+                               (const int*)tile_lo, (const int*)tile_prefix, (const float2*)mtile, rowstat, static_cast<int>(total_rows))))
+      return rc;
   }
   int bt = per_row >= 256 ? 256 : ((per_row + 31) / 32) * 32;
   if (fused && bt < 8 * g.rbs) bt = 8 * g.rbs;           // eight threads per row for the statistics (rbs <= 32)
   const dim3 fgrid((per_row + bt - 1) / bt, g.qb_total, batch * hq);
-  if (vec4) {
-    if (fused) est_blocksum_kernel<4, true><<<fgrid, bt, 0, stream>>>(g, tile_lo, tile_prefix, partial, mtile, rowstat, attn_sums);
-    else est_blocksum_kernel<4, false><<<fgrid, bt, 0, stream>>>(g, tile_lo, tile_prefix, partial, mtile, rowstat, attn_sums);
-  } else {
-    if (fused) est_blocksum_kernel<1, true><<<fgrid, bt, 0, stream>>>(g, tile_lo, tile_prefix, partial, mtile, rowstat, attn_sums);
-    else est_blocksum_kernel<1, false><<<fgrid, bt, 0, stream>>>(g, tile_lo, tile_prefix, partial, mtile, rowstat, attn_sums);
-  }
-  return launch_status();
+  auto launch_sums = [&](auto kern) -> int {
+    return launch_dependent(kern, fgrid, dim3(bt), 0, stream, g, (const int*)tile_lo, (const int*)tile_prefix, (const float*)partial,
+                            (const float2*)mtile, (const float2*)rowstat, attn_sums);
+  };
+  if (vec4) return fused ? launch_sums(est_blocksum_kernel<4, true>) : launch_sums(est_blocksum_kernel<4, false>);
+  return fused ? launch_sums(est_blocksum_kernel<1, true>) : launch_sums(est_blocksum_kernel<1, false>);
 }
 
 int split_f32_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
@@ -1251,8 +1259,8 @@ int split_f32_launch(const float* x, int batch, int heads, int len, int len_vali
   size_t blocks = (total + block - 1) / block;
   if (blocks > 148 * 32) blocks = 148 * 32;
   auto launch = [&](auto kern) -> int {
-    kern<<<static_cast<int>(blocks), block, 0, stream>>>(x, heads, len, len_valid, head_dim / 8, sb, sh, sl, static_cast<uint4*>(out), total);
-    return launch_status();
+    return launch_dependent(kern, dim3(static_cast<unsigned>(blocks)), dim3(block), 0, stream, x, heads, len, len_valid, head_dim / 8, sb,
+                            sh, sl, static_cast<uint4*>(out), total);
   };
   return terms == 3 ? launch(split_f32_kernel<3>) : launch(split_f32_kernel<1>);
 }

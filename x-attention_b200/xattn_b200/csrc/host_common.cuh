@@ -122,24 +122,35 @@ inline int launch_status() {
   return cudaGetLastError() == cudaSuccess ? XATTN_B200_OK : XATTN_B200_ERR_CUDA;
 }
 
-// Launches `kernel` so that it may start while the kernel before it in the stream is still running (programmatic
+// Launches `kernel`, in clusters of `cluster` CTAs, so that it may start while the kernel before it in the stream is still running (programmatic
 // stream serialization): the kernel must execute pdl_wait() before it touches anything that kernel writes.
+// (Every kernel of a call is launched like this, and lets the next one start early: a prefill is three to six short
+// kernels in a row, and the launch of one then runs under the one before it.)
 template <typename... KArgs, typename... Args>
-inline int launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream,
-                            Args&&... args) {
+inline int launch_dependent_clusters(void (*kernel)(KArgs...), unsigned cluster, dim3 grid, dim3 block, size_t smem_bytes,
+                                     cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem_bytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
   launch_counter().fetch_add(1, std::memory_order_relaxed);
   return (e == cudaSuccess && cudaGetLastError() == cudaSuccess) ? XATTN_B200_OK : XATTN_B200_ERR_CUDA;
+}
+template <typename... KArgs, typename... Args>
+inline int launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream,
+                            Args&&... args) {
+  return launch_dependent_clusters(kernel, 1, grid, block, smem_bytes, stream, std::forward<Args>(args)...);
 }
 
 }  // namespace xb

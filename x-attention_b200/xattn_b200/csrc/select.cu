@@ -25,6 +25,7 @@
 //   block 0 is set when at least one rank position was not taken; causal clears columns >= cur + bpc
 //   and columns right of the diagonal; keep_sink sets query-block row 0; keep_recent sets the diagonal.
 #include "host_common.cuh"
+#include "sm100_primitives.cuh"
 
 namespace xb {
 
@@ -122,6 +123,8 @@ __global__ void __launch_bounds__(256) select_kernel(const float* __restrict__ s
                               const float* __restrict__ thr_per_head, uint8_t* __restrict__ mask_out,
                               int32_t* __restrict__ idx_out, int32_t* __restrict__ cnt_out, int* status) {
   extern __shared__ __align__(16) uint8_t sel_smem[];
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int w = blockIdx.x * p.warps_per_cta + wib;
@@ -489,6 +492,8 @@ template <int kVec>
 __global__ void __launch_bounds__(256) select_reg_kernel(const float* __restrict__ sums, const SelParams p,
                                                          const float* __restrict__ thr_per_head, uint8_t* __restrict__ mask_out,
                                                          int32_t* __restrict__ idx_out, int32_t* __restrict__ cnt_out) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= p.rows_total) return;                   // whole warps leave
@@ -721,6 +726,8 @@ __device__ __forceinline__ bool list_keeps(int causal, int R, int j, int list_q_
 __global__ void mask_to_lists_kernel(const uint8_t* __restrict__ mask, int rows_total, int mask_q_blocks,
                                      int mask_k_blocks, int list_q_blocks, int list_k_blocks, int q_len, int k_len,
                                      int causal, int32_t* __restrict__ idx_out, int32_t* __restrict__ cnt_out) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= rows_total) return;
@@ -780,8 +787,8 @@ int select_launch(const float* attn_sums, int batch, int heads, int q_blocks, in
   if (k_blocks <= 1024) {
     // rows that fit the warp's registers: the instantiation with just enough of them for the stored scores
     auto launch_reg = [&](auto kern) -> int {
-      kern<<<static_cast<int>((rows + 7) / 8), 256, 0, stream>>>(attn_sums, p, thr_per_head, mask, block_idx, block_cnt);
-      return launch_status();
+      return launch_dependent(kern, dim3(static_cast<unsigned>((rows + 7) / 8)), dim3(256), 0, stream, attn_sums, p, thr_per_head, mask,
+                              block_idx, block_cnt);
     };
     if (n_read <= 128) return launch_reg(select_reg_kernel<1>);
     if (n_read <= 256) return launch_reg(select_reg_kernel<2>);
@@ -794,8 +801,8 @@ int select_launch(const float* attn_sums, int batch, int heads, int q_blocks, in
   const size_t smem = static_cast<size_t>(wpc) * p.per_warp_bytes;
   const int grid = static_cast<int>((rows + wpc - 1) / wpc);
   if (smem > 48 * 1024 && !allow_smem(select_kernel, 160 * 1024)) return XATTN_B200_ERR_CUDA;
-  select_kernel<<<grid, wpc * 32, smem, stream>>>(attn_sums, p, thr_per_head, mask, block_idx, block_cnt, status);
-  return launch_status();
+  return launch_dependent(select_kernel, dim3(grid), dim3(wpc * 32), smem, stream, attn_sums, p, thr_per_head, mask, block_idx, block_cnt,
+                          status);
 }
 
 int mask_to_lists_launch(const uint8_t* mask, int batch, int heads, int mask_q_blocks, int mask_k_blocks, int q_len,
@@ -805,10 +812,8 @@ int mask_to_lists_launch(const uint8_t* mask, int batch, int heads, int mask_q_b
   if (mask_q_blocks < lq || mask_k_blocks < lk) return XATTN_B200_ERR_ARG;
   const int rows = batch * heads * lq;
   const int wpb = 8;
-  mask_to_lists_kernel<<<(rows + wpb - 1) / wpb, wpb * 32, 0, stream>>>(mask, rows, mask_q_blocks, mask_k_blocks, lq,
-                                                                        lk, q_len, k_len, causal ? 1 : 0, block_idx,
-                                                                        block_cnt);
-  return launch_status();
+  return launch_dependent(mask_to_lists_kernel, dim3((rows + wpb - 1) / wpb), dim3(wpb * 32), 0, stream, mask, rows, mask_q_blocks,
+                          mask_k_blocks, lq, lk, q_len, k_len, causal ? 1 : 0, block_idx, block_cnt);
 }
 
 }  // namespace xb
