@@ -261,7 +261,8 @@ int xattn_b200_block_sparse_attn_ws(const void* q, const void* k, const void* v,
  * see completely.  Replaces the third-party single-query attention of the reference's Llama patch
  * (xattn/src/load_llama.py:188-197); the same result as the general kernel up to the summation order.  hq / hkv <= 16
  * (XATTN_B200_ERR_LIMIT otherwise: use xattn_b200_block_sparse_attn without lists).  The cache is split over the SMs; the
- * parts are merged through `workspace` (device memory, 16-byte aligned, contents irrelevant on entry).
+ * parts are merged through `workspace` (device memory, 16-byte aligned, contents irrelevant on entry; may be null where
+ * xattn_b200_decode_workspace_bytes is 0).
  */
 size_t xattn_b200_decode_workspace_bytes(int batch, int hq, int hkv, int k_len);
 int xattn_b200_decode_attn(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv, int k_len,

@@ -94,3 +94,15 @@ def test_more_units_than_sms(causal, ordered, hq, hkv, L):
         p = torch.where(keep, torch.softmax(p, -1), torch.zeros(()))
         want = p @ v.float().repeat_interleave(rep, 1)
         _close(out[:, :, r0:r1], want)
+
+
+@pytest.mark.parametrize("batch,hkv,k_len", [(1, 8, 300), (1, 8, 4096), (1, 8, 4097), (4, 8, 9000), (8, 8, 3001), (3, 16, 700), (6, 8, 5000)])
+def test_decode_step_merges(batch, hkv, k_len):
+    """Caches that one CTA, a cluster of two, four or eight, or more CTAs than a cluster share; fully checked in batch."""
+    from xattn_b200 import ops
+    q, k, v = _qkv(k_len + batch, batch, 2 * hkv, hkv, 1, k_len)
+    k[:, :, -1] *= 3.0
+    out = ops.decode_attention(q.to(DEV), k.to(DEV), v.to(DEV))
+    want = torch.nn.functional.scaled_dot_product_attention(q.float(), k.float().repeat_interleave(2, 1),
+                                                            v.float().repeat_interleave(2, 1))
+    _close(out, want)

@@ -13,8 +13,10 @@
 //     MMAs on purpose: with at most 16 useful rows a 128-row tcgen05 tile would be seven eighths padding, and the products
 //     take under a tenth of the time the bytes do;
 //   * every warp takes 16 keys of a stage and keeps a running softmax of its own; the four warps of a CTA are merged
-//     through shared memory at the end, the CTAs of a (batch, kv head) by a small second kernel (launched as a dependent
-//     one, so its launch latency runs under the first), or not at all when the cache needs no split.
+//     through shared memory at the end.  The CTAs of a (batch, kv head) are merged through distributed shared memory where
+//     they are a cluster (up to eight: caches of up to 4096 keys, or many heads), and by a small second kernel, launched as a
+//     dependent one, where there are more.  The second launch costs the host 2.5 us, which a step on a short cache would pay
+//     in full (2011 keys, 8 kv heads: 10.2 us a call with it, 6.0 without); a long cache hides it.
 #include "attention_common.cuh"
 
 namespace xb {
@@ -30,6 +32,7 @@ constexpr float kDecRescale = 8.0f;                       // log2 units: the run
 
 struct DecodeParams {
   int batch, hkv, group, k_len, splits, stages;           // stages: 64-key stages of the whole cache
+  int cluster;                                            // the splits are a cluster
   float scale_log2;
   int64_t qsb, qsh, osb, osh;
 };
@@ -79,7 +82,8 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     fence_mbar_init();
   }
   __syncthreads();
-  pdl_launch_dependents();              // the merging kernel may take its place; it waits for this grid to end
+  pdl_launch_dependents();              // the next kernel may take its place; it waits for this grid to end
+  pdl_wait();
   auto load_stage = [&](int i) {        // one thread: the CTA's i-th stage
     const int st = i % kDecStages;
     const uint32_t dst = smem_u32(smem) + st * 2 * kDecTile;
@@ -191,14 +195,17 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
   }
   __syncthreads();                       // every stage has been read: the ring becomes the exchange buffer
-  if (*abort_flag) {
+  const bool aborted = *abort_flag != 0;
+  if (aborted) {
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000) { __nanosleep(1000); }      // let copies in flight land
     if (threadIdx.x == 0 && status) atomicExch(status, static_cast<int>(kDevWaitTimeout));
-    return;
+    __syncthreads();
   }
   float* xo = reinterpret_cast<float*>(smem);                                    // [warp][16 rows][128]
   float2* xml = reinterpret_cast<float2*>(smem + kDecWarps * kDecMaxRows * 128 * 4);     // [warp][16 rows]
+  float* res = xo + kDecWarps * kDecMaxRows * 128 + 2 * kDecWarps * kDecMaxRows;          // [16 rows][128], the CTA's part
+  float2* res_ml = reinterpret_cast<float2*>(res + kDecMaxRows * 128);                    // [16 rows]
   {
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
 #pragma unroll
@@ -232,11 +239,45 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       const float inv = ll > 0.f ? 1.f / ll : 0.f;
       *reinterpret_cast<uint32_t*>(out + b * p.osb + static_cast<int64_t>(g * p.group + r) * p.osh + c) =
           pack16t<kBf16>(a0 * inv, a1 * inv);
+    } else if (p.cluster) {
+      *reinterpret_cast<float2*>(res + r * 128 + c) = make_float2(a0, a1);
+      if (c == 0) res_ml[r] = make_float2(mm, ll);
     } else {
       const size_t row = (static_cast<size_t>(b * p.hkv + g) * p.splits + split) * p.group + r;
       *reinterpret_cast<float2*>(part + row * 128 + c) = make_float2(a0, a1);
       if (c == 0) part_ml[row] = make_float2(mm, ll);
     }
+  }
+  if (p.cluster) {
+    // every CTA merges its share of the outputs, two columns of a row at a time
+    cluster_sync_all();
+    for (int e = split * kDecThreads + threadIdx.x; e < p.group * 64; e += p.splits * kDecThreads) {
+      const int r = e >> 6, c = (e & 63) * 2;
+      float2 ml[8], v[8];
+      float mm = -INFINITY;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        ml[s] = make_float2(-INFINITY, 0.f);
+        v[s] = make_float2(0.f, 0.f);
+        if (s < p.splits) {
+          ml[s] = ld_shared_cluster_f2(mapa_shared(smem_u32(res_ml + r), s));
+          v[s] = ld_shared_cluster_f2(mapa_shared(smem_u32(res + r * 128 + c), s));
+        }
+        mm = fmaxf(mm, ml[s].x);
+      }
+      float a0 = 0.f, a1 = 0.f, ll = 0.f;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const float f = ml[s].x == -INFINITY ? 0.f : fast_exp2(ml[s].x - mm);
+        a0 += v[s].x * f;
+        a1 += v[s].y * f;
+        ll += ml[s].y * f;
+      }
+      const float inv = ll > 0.f ? 1.f / ll : 0.f;
+      *reinterpret_cast<uint32_t*>(out + b * p.osb + static_cast<int64_t>(g * p.group + r) * p.osh + c) =
+          pack16t<kBf16>(a0 * inv, a1 * inv);
+    }
+    cluster_sync_all();                  // nobody leaves while its part may still be read
   }
 }
 
@@ -245,6 +286,7 @@ template <bool kBf16>
 __global__ void __launch_bounds__(128)
 decode_merge_kernel(const DecodeParams p, const float* __restrict__ part, const float2* __restrict__ part_ml,
                     uint16_t* __restrict__ out) {
+  pdl_launch_dependents();
   pdl_wait();
   const int hq = p.hkv * p.group;
   const int b = blockIdx.x / hq, h = blockIdx.x - b * hq;
@@ -267,18 +309,27 @@ decode_merge_kernel(const DecodeParams p, const float* __restrict__ part, const 
 }
 
 // Number of splits: two CTAs per SM over all (batch, kv head) pairs, at least two stages each (a split costs a CTA's start
-// and its row of the merge, about what two stages take).
-static int decode_splits(int batch, int hkv, int k_len) {
+// and its row of the merge, about what two stages take).  Up to eight of them are a cluster, whose size is a power of two;
+// so are those of caches of up to 4096 keys, where eight CTAs of eight stages take about as long as the second kernel.
+constexpr int kDecClusterMax = 8, kDecClusterStages = 64;
+static int decode_splits(int batch, int hkv, int k_len, int& cluster) {
   const int stages = (k_len + kDecKeys - 1) / kDecKeys;
   const long long heads = static_cast<long long>(batch) * hkv;
   long long s = 2LL * sm_count() / heads;
   if (s > stages / 2) s = stages / 2;
+  if (s > kDecClusterMax && (stages <= kDecClusterStages || s < kDecClusterMax * 3 / 2)) s = kDecClusterMax;
+  cluster = s > 1 && s <= kDecClusterMax ? 1 : 0;
+  if (cluster)
+    while (s & (s - 1)) s &= s - 1;
   return s < 1 ? 1 : static_cast<int>(s);
 }
 
 size_t decode_workspace_bytes(int batch, int hq, int hkv, int k_len) {
   if (batch < 1 || hq < 1 || hkv < 1 || hq % hkv != 0 || hq / hkv > kDecMaxRows || k_len < 1) return 0;
-  return static_cast<size_t>(batch) * hq * decode_splits(batch, hkv, k_len) * (128 * sizeof(float) + sizeof(float2));
+  int cluster = 0;
+  const int splits = decode_splits(batch, hkv, k_len, cluster);
+  if (cluster || splits == 1) return 0;
+  return static_cast<size_t>(batch) * hq * splits * (128 * sizeof(float) + sizeof(float2));
 }
 
 int decode_launch(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv, int k_len,
@@ -295,10 +346,11 @@ int decode_launch(const void* q, const void* k, const void* v, int dtype, int ba
   DecodeParams p;
   p.batch = batch; p.hkv = hkv; p.group = hq / hkv; p.k_len = k_len;
   p.stages = (k_len + kDecKeys - 1) / kDecKeys;
-  p.splits = decode_splits(batch, hkv, k_len);
+  p.splits = decode_splits(batch, hkv, k_len, p.cluster);
   p.scale_log2 = scale * 1.4426950408889634f;
   p.qsb = qsb; p.qsh = qsh; p.osb = osb; p.osh = osh;
-  if (!workspace || workspace_bytes < decode_workspace_bytes(batch, hq, hkv, k_len)) return XATTN_B200_ERR_WORKSPACE;
+  const size_t need = decode_workspace_bytes(batch, hq, hkv, k_len);
+  if (need && (!workspace || workspace_bytes < need)) return XATTN_B200_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return XATTN_B200_ERR_ARG;
   float* part = static_cast<float*>(workspace);
   float2* part_ml = reinterpret_cast<float2*>(part + static_cast<size_t>(batch) * hq * p.splits * 128);
@@ -308,10 +360,9 @@ int decode_launch(const void* q, const void* k, const void* v, int dtype, int ba
   auto launch = [&](auto kern, auto merge) -> int {
     if (!allow_smem(kern, kDecSmem))
       return XATTN_B200_ERR_CUDA;
-    kern<<<dim3(p.splits, hkv, batch), kDecThreads, kDecSmem, stream>>>(tmK, tmV, static_cast<const uint16_t*>(q), p, part, part_ml,
-                                                                        static_cast<uint16_t*>(out), status);
-    int r = launch_status();
-    if (r || p.splits == 1) return r;
+    const int r = launch_dependent_clusters(kern, p.cluster ? p.splits : 1, dim3(p.splits, hkv, batch), dim3(kDecThreads), kDecSmem, stream,
+                                            tmK, tmV, static_cast<const uint16_t*>(q), p, part, part_ml, static_cast<uint16_t*>(out), status);
+    if (r || p.cluster || p.splits == 1) return r;
     return launch_dependent(merge, dim3(batch * hq), dim3(128), 0, stream, p, static_cast<const float*>(part),
                             static_cast<const float2*>(part_ml), static_cast<uint16_t*>(out));
   };

@@ -346,11 +346,12 @@ PyObject* py_decode(PyObject*, PyObject* const* pv, Py_ssize_t n) {
     fail(PyExc_TypeError, "q/k/v must share one of bf16, fp16, fp32");
   const Tensor q = aligned16(q_), k = aligned16(k_), v = aligned16(v_);
   const size_t bytes = xattn_b200_decode_workspace_bytes(B, Hq, Hkv, Lk);
-  const Tensor ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
+  Tensor ws;
+  if (bytes) ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
   Tensor out = empty({B, 1, Hq, D}, q.scalar_type(), at_.dev);
   check(xattn_b200_decode_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), code, B, Hq, Hkv, Lk, D, q.stride(0), q.stride(1), k.stride(0),
                                k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2), static_cast<float>(scale), out.data_ptr(),
-                               Hq * D, D, ws.data_ptr(), bytes, at_.status, at_.stream),
+                               Hq * D, D, bytes ? ws.data_ptr() : nullptr, bytes, at_.status, at_.stream),
         "decode_attn");
   return wrap(out.transpose(1, 2));
   END_HANDLE_TH_ERRORS

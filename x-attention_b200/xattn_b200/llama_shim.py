@@ -58,15 +58,12 @@ def default_threshold_table(stride: int) -> torch.Tensor:
 def attention_core(query_states: torch.Tensor, key_states: torch.Tensor, value_states: torch.Tensor,
                    layer_idx: int, config: FastPrefillConfig) -> torch.Tensor:
     """q [B,Hq,q_len,D], k/v [B,Hkv,k_len,D] (after RoPE and the cache update) -> [B,Hq,q_len,D]."""
-    B, Hq, q_len, D = query_states.shape
-    k_len = key_states.shape[2]
-    decoding = q_len != k_len and q_len == 1                       # load_llama.py:156
-    if not decoding and config.metric == "xattn":
+    if query_states.size(2) == 1 and key_states.size(2) != 1:      # load_llama.py:156
+        return ops.decode_attention(query_states, key_states, value_states)
+    if config.metric == "xattn":
         thr = config.threshold[layer_idx] if config.threshold.dim() == 2 else config.threshold
         return Xattention_prefill(query_states, key_states, value_states, config.stride, norm=1, threshold=thr,
                                   use_triton=True)
-    if decoding:
-        return ops.decode_attention(query_states, key_states, value_states)
     # dense prefill: every key block that a row may see (token-level causal inside the kernel)
     return ops.block_sparse_attention(query_states, key_states, value_states, None, None, causal=True)
 
