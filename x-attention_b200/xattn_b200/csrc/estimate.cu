@@ -65,6 +65,8 @@ struct EstGeom {
   // (tab_n = n_mtiles <= kTabTiles, e.g. 32 row tiles at 32K tokens, 64 at 128K): every kernel copies them into
   // shared memory and est_setup_kernel is not launched.  Layout: tile_lo[kTabTiles], tile_prefix[kTabTiles + 1],
   // pair_lo[kTabTiles / 2], pair_prefix[kTabTiles / 2 + 1].
+  // few tiles: the K loop of each is split over a cluster of `split` CTAs (1: persistent CTAs, a tile each at a time)
+  int split;
   int direct;                  // the epilogue finishes the block sums: every row tile is computed, even one that sees nothing
   int tab_n;
   int tab[64 + 65 + 32 + 33];
@@ -431,7 +433,11 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   const int tiles_per_head = tile_prefix[g.n_mtiles];
   const int total_tiles = tiles_per_head * g.batch * g.hq;
-  const int k_steps = g.S * g.d_chunks;
+  // this CTA's tiles and its part of their K loop (split fp32 rows: whole triples of terms)
+  const int split = g.split, rank = split > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int tile0 = blockIdx.x / split, tile_step = gridDim.x / split;
+  const int k_unit = g.term_chunks ? 3 : 1, k_units = g.S * g.d_chunks / k_unit;
+  const int ks0 = k_units * rank / split * k_unit, ks1 = k_units * (rank + 1) / split * k_unit;
   const int group = g.hq / g.hkv;
   const int interleave = g.tile_n == 128 ? group : 1;      // streaming case only: see decode_tile
 
@@ -441,12 +447,12 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t lead = elect_one() ? 1u : 0u;
       int s = 0;
       uint32_t ph = 0;
-      for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x) {
+      for (int tile = tile0; tile < total_tiles && !*abort_flag; tile += tile_step) {
         int bh, mt, nt;
         decode_tile(g.n_mtiles, tile_lo, tile_prefix, tiles_per_head, tile, bh, mt, nt, interleave);
         const int b = bh / g.hq, h = bh - b * g.hq;
-        int t = 0, dc = 0;
-        for (int ks = 0; ks < k_steps; ++ks) {
+        int t = ks0 / g.d_chunks, dc = ks0 - t * g.d_chunks;
+        for (int ks = ks0; ks < ks1; ++ks) {
           if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag))) break;
           const uint32_t dstA = smem_u32(smem + s * stage_bytes);
           mbar_expect_tx_lead(full0 + 8 * s, stage_bytes, lead);
@@ -459,6 +465,10 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
     }
+    if (split > 1) {
+      cluster_sync_all();
+      cluster_sync_all();
+    }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (converged warp, one thread issues: see mma_ss_lead)
     {
@@ -468,7 +478,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       uint32_t ph = 0, local_tile = 0;
       const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
       const uint64_t b_desc0 = smem_desc_sw128(smem_u32(smem) + kABytes, 16, 1024);
-      for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++local_tile) {
+      for (int tile = tile0; tile < total_tiles && !*abort_flag; tile += tile_step, ++local_tile) {
         const uint32_t acc = local_tile & 1;
         const uint32_t acc_ph = (local_tile >> 1) & 1;
         if (!wait(tempty0 + 8 * acc, acc_ph ^ 1)) break;
@@ -476,7 +486,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint32_t d_tmem = tmem_base + acc * kTileN;
         bool ok = true;
         int term = g.term_chunks ? 0 : -1;
-        for (int ks = 0; ks < k_steps; ++ks) {
+        for (int ks = ks0; ks < ks1; ++ks) {
           if (!wait(full0 + 8 * st, ph)) { ok = false; break; }
           tc_fence_after();
           // D += A of stage sa * B of stage sb; descriptors differ from the stage-0 ones only in the start-address field
@@ -489,13 +499,13 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               mma_ss_lead(d_tmem, a_desc + k4 * 2, b_desc + k4 * 2, idesc, k4 > 0 ? 1u : accumulate, lead);
           };
           if (term < 0) {
-            product(st, st, ks > 0 ? 1u : 0u);
+            product(st, st, ks > ks0 ? 1u : 0u);
             mma_commit_lead(empty0 + 8 * st, lead);       // stage reusable once these MMAs have read it
           } else {
             // three stages hold the terms [hi, mid, lo] of one chunk: the products hh; hm, mh, mm; hl, lh (the three left out
             // are below 2^-24 of the first).  Each term is loaded once for the products it enters.
             if (term == 0) {
-              product(st, st, ks > 0 ? 1u : 0u);
+              product(st, st, ks > ks0 ? 1u : 0u);
             } else if (term == 1) {
               product(st - 1, st, 1u);
               product(st, st - 1, 1u);
@@ -513,6 +523,10 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         mma_commit_lead(tfull0 + 8 * acc, lead);          // accumulator complete
       }
     }
+    if (split > 1) {
+      cluster_sync_all();
+      cluster_sync_all();
+    }
   } else {
     // ------------------------------------------------------------ epilogue (4 warps, thread = tile row)
     const int quad = warp & 3;                  // TMEM lane quarter this warp may access
@@ -520,7 +534,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int kGroups = g.tile_n / RBS;         // key blocks per tile
     const int n_chunks = g.tile_n / 32;
     uint32_t local_tile = 0;
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++local_tile) {
+    for (int tile = tile0; tile < total_tiles; tile += tile_step, ++local_tile) {
       int bh, mt, nt;
       decode_tile(g.n_mtiles, tile_lo, tile_prefix, tiles_per_head, tile, bh, mt, nt, interleave);
       const uint32_t acc = local_tile & 1;
@@ -532,9 +546,51 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int clo = lo - n0 > 0 ? lo - n0 : 0;
       const int chi = hi - n0 < g.tile_n - 1 ? hi - n0 : g.tile_n - 1;
       // warp-uniform: the tensor-memory loads below are warp-collective
-      if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, acc_ph, abort_flag))) break;
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, acc_ph, abort_flag));
+      if (!ok && split == 1) break;                   // (a cluster's barriers are passed in any case)
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * kTileN + (static_cast<uint32_t>(quad * 32) << 16);
+      if (split > 1) {
+        // The cluster's accumulators are added up, every CTA finishing 128 / split rows: the others' parts of them come
+        // through its shared memory ([source][32-row quarter][4 columns][lane] of 16 bytes; the operand stages, which no CTA
+        // reads any more) and go back to tensor memory added to its own.  (The loader and issuer warps keep the barriers
+        // company below.)
+        const int own = 4 / split, dest = quad / own;              // quarters a CTA finishes; the CTA of this warp's
+        cluster_sync_all();
+        if (dest != rank) {
+          const int slot = rank < dest ? rank : rank - 1;
+          const uint32_t base = mapa_shared(smem_u32(smem) + (slot * own + quad % own) * g.tile_n * 128 + lane * 16, dest);
+#pragma unroll 1
+          for (int c = 0; c < n_chunks; ++c) {
+            uint32_t v[32];
+            tmem_ld32(taddr + c * 32, v);
+            tc_wait_ld();
+#pragma unroll
+            for (int q4 = 0; q4 < 8; ++q4) st_shared_cluster_v4(base + (c * 8 + q4) * 512, v[4 * q4], v[4 * q4 + 1], v[4 * q4 + 2], v[4 * q4 + 3]);
+          }
+        }
+        cluster_sync_all();
+        if (dest != rank || !ok) break;
+#pragma unroll 1
+        for (int c = 0; c < n_chunks; ++c) {
+          uint32_t v[32];
+          tmem_ld32(taddr + c * 32, v);
+          tc_wait_ld();
+          for (int src = 0; src < split - 1; ++src) {
+            const uint8_t* from = smem + (src * own + quad % own) * g.tile_n * 128 + c * 8 * 512 + lane * 16;
+#pragma unroll
+            for (int q4 = 0; q4 < 8; ++q4) {
+              const float4 x = *reinterpret_cast<const float4*>(from + q4 * 512);
+              v[4 * q4] = __float_as_uint(__uint_as_float(v[4 * q4]) + x.x);
+              v[4 * q4 + 1] = __float_as_uint(__uint_as_float(v[4 * q4 + 1]) + x.y);
+              v[4 * q4 + 2] = __float_as_uint(__uint_as_float(v[4 * q4 + 2]) + x.z);
+              v[4 * q4 + 3] = __float_as_uint(__uint_as_float(v[4 * q4 + 3]) + x.w);
+            }
+          }
+          tmem_st32(taddr + c * 32, v);
+        }
+        tc_wait_st();
+      }
       const bool row_ok = i < g.rows_total;
       const size_t rrow = static_cast<size_t>(bh) * g.rows_total + (row_ok ? i : 0);
       const int nlo = tile_lo[mt];
@@ -987,6 +1043,7 @@ static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int h
   g.q_none = q_len < stride ? 1 : 0;
   g.k_none = k_len < stride ? 1 : 0;
   g.direct = 0;
+  g.split = 1;
   g.compact = g.left_blank;
   g.m_pitch = g.n_ntiles;
   g.p_pitch = g.kb_total;
@@ -1097,9 +1154,19 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // CTA pairs (256x256 tiles) when tiles are 256 columns wide and the two row tiles of a pair see about the
   // same columns (always, except when a 128-row chunk of the torch branch blanks everything left of it)
   bool use_pairs = g.tile_n == kTileN && g.n_mtiles >= 2 && (!g.left_blank || g.rcs % (2 * kTileM) == 0);
-#ifdef XB_EST_NO_PAIRS
-  use_pairs = false;
-#endif
+  // Few tiles (short prompts: 32 heads of up to 2048 tokens at stride 16 are 32 tiles for 148 SMs): the K loop of each, which is
+  // a stream of operands through one SM, is split over a cluster of two or four CTAs instead.
+  {
+    long long tiles = 0;
+    for (int mt = 0; mt < g.n_mtiles && tiles <= sm_count(); ++mt) {
+      int first, count;
+      row_tile_range(g, mt, first, count);
+      tiles += static_cast<long long>(count > 0 ? count : 1) * batch * hq;
+    }
+    const bool long_k = g.S * g.d_chunks >= 32;          // (the exchange costs about what eight steps take)
+    g.split = !long_k ? 1 : (4 * tiles <= sm_count() ? 4 : (2 * tiles <= sm_count() ? 2 : 1));
+    if (g.split > 1) use_pairs = false;
+  }
   // Every row sees a single 128-column tile and that tile's block sums are (nearly) a whole row of the output: chunks of
   // exactly one 128-row, 128-column tile in the chunk-band layout (128K tokens at stride 16), or keys of at most 128 columns
   // altogether (prompts of up to 2048 tokens at stride 16).  The GEMM's epilogue then finishes the block sums itself, and
@@ -1195,11 +1262,20 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     if (rc) return rc;
   } else {
   const uint32_t idesc = make_idesc_f16(kTileM, g.tile_n, dtype != XATTN_B200_F16, false, false);
-  const int grid = sms;
+  // persistent CTAs, or exactly the tiles' clusters
+  long long tiles = 0;
+  if (g.split > 1)
+    for (int mt = 0; mt < g.n_mtiles; ++mt) {
+      int first, count;
+      row_tile_range(g, mt, first, count);
+      tiles += static_cast<long long>(count) * batch * hq;
+    }
+  if (tiles == 0) g.split = 1;
+  const int grid = g.split > 1 ? static_cast<int>(tiles) * g.split : sms;
   auto launch = [&](auto kern) -> int {
     if (!allow_smem(kern, kGemmSmem))
       return XATTN_B200_ERR_CUDA;
-    return launch_dependent(kern, dim3(grid), dim3(kGemmThreads), kGemmSmem, stream, tmQ, tmK, tmQt, tmKt, g,
+    return launch_dependent_clusters(kern, g.split, dim3(grid), dim3(kGemmThreads), kGemmSmem, stream, tmQ, tmK, tmQt, tmKt, g,
                             (const int*)tile_lo, (const int*)tile_prefix, partial, mtile, attn_sums, idesc, status);
   };
   if (direct) {
