@@ -11,25 +11,6 @@ namespace xb {
 constexpr int kTile16 = 128 * 128 * 2;     // one 128x128 16-bit tile = two 64-column TMA boxes
 constexpr int kHalf16 = kTile16 / 2;
 
-// Division of numbers below 2^31 by a divisor known on the host: a multiplication and a shift instead of the ~25
-// instructions of an integer division, which add up in code that every role of a kernel has to decode its work with.
-struct FastDiv {
-  uint32_t d, mul, shift;
-};
-static inline FastDiv make_fast_div(uint32_t d) {
-  FastDiv f;
-  f.d = d;
-  f.shift = 0;
-  while ((1ull << f.shift) < d) ++f.shift;
-  f.mul = static_cast<uint32_t>((((1ull << f.shift) - d) << 32) / d + 1);
-  return f;
-}
-__device__ __forceinline__ int fast_div(int n, const FastDiv& f, int& rem) {
-  const uint32_t q = (__umulhi(static_cast<uint32_t>(n), f.mul) + static_cast<uint32_t>(n)) >> f.shift;
-  rem = n - static_cast<int>(q * f.d);
-  return static_cast<int>(q);
-}
-
 struct AttnParams {
   int batch, hq, hkv, q_len, k_len;
   int q_blocks, list_k_blocks;

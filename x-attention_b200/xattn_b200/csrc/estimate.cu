@@ -65,6 +65,7 @@ struct EstGeom {
   // (tab_n = n_mtiles <= kTabTiles, e.g. 32 row tiles at 32K tokens, 64 at 128K): every kernel copies them into
   // shared memory and est_setup_kernel is not launched.  Layout: tile_lo[kTabTiles], tile_prefix[kTabTiles + 1],
   // pair_lo[kTabTiles / 2], pair_prefix[kTabTiles / 2 + 1].
+  FastDiv by_tiles, by_group, by_hq;     // tiles per head (of the kernel that runs), query heads per kv head, query heads
   // few tiles: the K loop of each is split over a cluster of `split` CTAs (1: persistent CTAs, a tile each at a time)
   int split;
   int direct;                  // the epilogue finishes the block sums: every row tile is computed, even one that sees nothing
@@ -172,20 +173,13 @@ __device__ __forceinline__ void load_tables(const EstGeom& g, int* s_tab) {
 // the heads of a kv group take the same (row, column) tile one after the other, so that the K tile they share is
 // read from DRAM once and found in L2 by the other heads: it matters when the kernel streams its operands from
 // HBM (128-column tiles), where K otherwise came from DRAM about twice.
-__device__ __forceinline__ void decode_tile(int n_groups, const int* __restrict__ tile_lo,
-                                            const int* __restrict__ tile_prefix, int tiles_per_head, int tile,
-                                            int& bh, int& mt, int& nt, int interleave = 1) {
-  int rem;
-  if (interleave > 1) {
-    const int hg = tile % interleave;                  // head inside its kv group
-    const int t2 = tile / interleave;
-    const int bkv = t2 / tiles_per_head;               // batch * kv heads + kv head
-    rem = t2 - bkv * tiles_per_head;
-    bh = bkv * interleave + hg;
-  } else {
-    bh = tile / tiles_per_head;
-    rem = tile - bh * tiles_per_head;
-  }
+__device__ __forceinline__ void decode_tile(const EstGeom& g, int n_groups, const int* __restrict__ tile_lo,
+                                            const int* __restrict__ tile_prefix, int tile, int& bh, int& mt, int& nt,
+                                            bool interleave = false) {
+  int rem, hg = 0;
+  if (interleave) tile = fast_div(tile, g.by_group, hg);     // hg: head inside its kv group
+  bh = fast_div(tile, g.by_tiles, rem);
+  if (interleave) bh = bh * static_cast<int>(g.by_group.d) + hg;
   int lo = 0, hi = n_groups;     // find mt with prefix[mt] <= rem < prefix[mt+1]
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -283,96 +277,79 @@ __device__ __forceinline__ void est_epilogue_row(const EstGeom& g, uint32_t tadd
 // registers, division by the row sum, and the sum over the RBS rows of a query block taken across lanes -- and
 // written to the chunk-band block sums directly.  Neither the per-row scratch nor the two kernels that would read
 // it are needed.  `out` is the 128 / RBS floats of this row's query block (written by its first row's lane).
-template <int RBS, typename Release>
-__device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, uint32_t taddr, int clo, int chi,
-                                                        float* __restrict__ out, int out_cols, bool write, Release release) {
-  constexpr int kChunks = 4, kPer = 32 / RBS;               // 128 columns; key blocks per 32-column chunk
-  auto fully_visible = [&](int c8) { return __all_sync(0xffffffffu, clo <= c8 * 32 && chi >= c8 * 32 + 31); };
-  float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  {
-    uint32_t va[32], vb[32];
-    tmem_ld32(taddr, va);
+//
+// The row's 128 scores are in registers (`v`, 32-column chunks from `nvis` on hidden from the whole warp): one tensor-memory
+// round trip, all of it at once.  The block sums of the RBS rows of a query block are added by halves: a lane gives away
+// half of its sums and receives the other lane's part of the half it keeps, 14 shuffles for 8 rows instead of 48.
+template <int RBS>
+__device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, uint32_t (&v)[4][32], int nvis, int clo, int chi,
+                                                        float* __restrict__ out, int out_cols, bool write, int lane) {
+  constexpr int kBlocks = 128 / RBS;
+  float mx8[8];
 #pragma unroll
-    for (int c8 = 0; c8 < kChunks; c8 += 2) {
-      tc_wait_ld();
-      tmem_ld32(taddr + (c8 + 1) * 32, vb);
-      auto max_chunk = [&](const uint32_t (&v)[32], int c) {
-        if (fully_visible(c)) {
+  for (int q = 0; q < 8; ++q) mx8[q] = -INFINITY;
 #pragma unroll
-          for (int k = 0; k < 32; ++k) mx4[k & 3] = fmaxf(mx4[k & 3], __uint_as_float(v[k]));
-        } else {
+  for (int c = 0; c < 4; ++c) {
+    if (c >= nvis) continue;
+    if (!__all_sync(0xffffffffu, clo <= c * 32 && chi >= c * 32 + 31)) {
 #pragma unroll
-          for (int k = 0; k < 32; ++k) {
-            const int col = c * 32 + k;
-            if (col >= clo && col <= chi) mx4[k & 3] = fmaxf(mx4[k & 3], __uint_as_float(v[k]));
-          }
-        }
-      };
-      max_chunk(va, c8);
-      tc_wait_ld();
-      if (c8 + 2 < kChunks) tmem_ld32(taddr + (c8 + 2) * 32, va);
-      max_chunk(vb, c8 + 1);
+      for (int k = 0; k < 32; ++k) v[c][k] = c * 32 + k >= clo && c * 32 + k <= chi ? v[c][k] : 0xff800000u;
     }
+#pragma unroll
+    for (int k = 0; k < 16; ++k)
+      mx8[k & 7] = max3(mx8[k & 7], __uint_as_float(v[c][2 * k]), __uint_as_float(v[c][2 * k + 1]));
   }
-  const float m_scaled = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * g.scale_log2;     // scale > 0
-  float blk[kChunks * kPer];
+  const float mx = fmaxf(max3(mx8[0], mx8[1], mx8[2]), max3(max3(mx8[3], mx8[4], mx8[5]), mx8[6], mx8[7]));
+  const float m = mx == -INFINITY ? 0.f : mx * g.scale_log2;           // scale > 0
+  const unsigned long long scale2 = pack_f32x2(g.scale_log2, g.scale_log2), nm2 = pack_f32x2(-m, -m);
+  float blk[kBlocks];
   float row_sum = 0.f;
-  {
-    uint32_t va[32], vb[32];
-    tmem_ld32(taddr, va);
 #pragma unroll
-    for (int c8 = 0; c8 < kChunks; c8 += 2) {
-      tc_wait_ld();
-      tmem_ld32(taddr + (c8 + 1) * 32, vb);
-      auto sum_chunk = [&](const uint32_t (&v)[32], int c) {
-        float gs[kPer];
+  for (int c = 0; c < 4; ++c) {
+    constexpr int kPer = 32 / RBS;
 #pragma unroll
-        for (int q = 0; q < kPer; ++q) gs[q] = 0.f;
-        if (fully_visible(c)) {
+    for (int q = 0; q < kPer; ++q) blk[c * kPer + q] = 0.f;
+    if (c >= nvis) continue;
 #pragma unroll
-          for (int k = 0; k < 32; ++k) gs[k / RBS] += fast_exp2(fmaf(__uint_as_float(v[k]), g.scale_log2, -m_scaled));
-        } else {
+    for (int q = 0; q < kPer; ++q) {
+      unsigned long long s2 = 0ull;
 #pragma unroll
-          for (int k = 0; k < 32; ++k) {
-            const int col = c * 32 + k;
-            const float x = fmaf(__uint_as_float(v[k]), g.scale_log2, -m_scaled);
-            gs[k / RBS] += (col >= clo && col <= chi) ? fast_exp2(x) : 0.f;
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-          row_sum += gs[q];
-          blk[c * kPer + q] = gs[q];
-        }
-      };
-      sum_chunk(va, c8);
-      tc_wait_ld();
-      if (c8 + 2 < kChunks) tmem_ld32(taddr + (c8 + 2) * 32, va);
-      else release();                                   // the tile's last load has completed
-      sum_chunk(vb, c8 + 1);
+      for (int k = q * RBS / 2; k < (q + 1) * RBS / 2; ++k) {
+        float y0, y1;
+        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c][2 * k]), __uint_as_float(v[c][2 * k + 1])), scale2, nm2), y0, y1);
+        s2 = add_f32x2(s2, pack_f32x2(fast_exp2(y0), fast_exp2(y1)));
+      }
+      float a, b;
+      unpack_f32x2(s2, a, b);
+      blk[c * kPer + q] = a + b;
+      row_sum += a + b;
     }
   }
-  // normalise (a row that sees nothing contributes nothing), then add the RBS rows of the query block: they are RBS
-  // consecutive lanes
+  // normalise (a row that sees nothing contributes nothing), then add the RBS rows of the query block, RBS lanes
   const float inv = row_sum > 0.f ? 1.f / row_sum : 0.f;
 #pragma unroll
-  for (int q = 0; q < kChunks * kPer; ++q) {
-    float v = blk[q] * inv;
+  for (int q = 0; q < kBlocks; ++q) blk[q] *= inv;
+  int n = kBlocks, base = 0;
 #pragma unroll
-    for (int o = 1; o < RBS; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    blk[q] = v;
+  for (int o = 1; o < RBS; o <<= 1) {
+    if (n > 1) {
+      n >>= 1;
+      const bool upper = (lane & o) != 0;
+      if (upper) base += n;
+#pragma unroll
+      for (int j = 0; j < kBlocks / 2; ++j)
+        if (j < n) blk[j] = (upper ? blk[j + n] : blk[j]) + __shfl_xor_sync(0xffffffffu, upper ? blk[j] : blk[j + n], o);
+    } else {
+      write = write && (lane & o) == 0;                                // (more lanes than sums)
+      blk[0] += __shfl_xor_sync(0xffffffffu, blk[0], o);
+    }
   }
   if (!write) return;
-  if (g.band) {
+  constexpr int kLeft = kBlocks > RBS ? kBlocks / RBS : 1;
 #pragma unroll
-    for (int q = 0; q < kChunks * kPer; q += 4)
-      *reinterpret_cast<float4*>(out + q) = make_float4(blk[q], blk[q + 1], blk[q + 2], blk[q + 3]);
-  } else {
-    // dense rows of a few blocks more or less than the tile holds
-#pragma unroll
-    for (int q = 0; q < kChunks * kPer; ++q)
-      if (q < out_cols) out[q] = blk[q];
-    for (int q = kChunks * kPer; q < out_cols; ++q) out[q] = 0.f;
+  for (int q = 0; q < kLeft; ++q) {
+    if (base + q < out_cols) out[base + q] = blk[q];
+    if (kBlocks + base + q < out_cols) out[kBlocks + base + q] = 0.f;  // (dense rows of more blocks than the tile holds)
   }
 }
 
@@ -438,8 +415,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int tile0 = blockIdx.x / split, tile_step = gridDim.x / split;
   const int k_unit = g.term_chunks ? 3 : 1, k_units = g.S * g.d_chunks / k_unit;
   const int ks0 = k_units * rank / split * k_unit, ks1 = k_units * (rank + 1) / split * k_unit;
-  const int group = g.hq / g.hkv;
-  const int interleave = g.tile_n == 128 ? group : 1;      // streaming case only: see decode_tile
+  const bool interleave = g.tile_n == 128 && g.hq > g.hkv;      // streaming case only: see decode_tile
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (converged warp, one thread issues)
@@ -449,8 +425,9 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       uint32_t ph = 0;
       for (int tile = tile0; tile < total_tiles && !*abort_flag; tile += tile_step) {
         int bh, mt, nt;
-        decode_tile(g.n_mtiles, tile_lo, tile_prefix, tiles_per_head, tile, bh, mt, nt, interleave);
-        const int b = bh / g.hq, h = bh - b * g.hq;
+        decode_tile(g, g.n_mtiles, tile_lo, tile_prefix, tile, bh, mt, nt, interleave);
+        int h, hg_;
+        const int b = fast_div(bh, g.by_hq, h), hkv = fast_div(h, g.by_group, hg_);
         int t = ks0 / g.d_chunks, dc = ks0 - t * g.d_chunks;
         for (int ks = ks0; ks < ks1; ++ks) {
           if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag))) break;
@@ -459,7 +436,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const bool qt = g.S - 1 - t < g.q_rem, kt = t < g.k_rem;
           const int col = k_column(g, dc);
           tma_load_5d_lead(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
-          tma_load_5d_lead(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, col, t, nt * g.tile_n + (kt ? 0 : g.k_none), h / group, b, lead);
+          tma_load_5d_lead(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, col, t, nt * g.tile_n + (kt ? 0 : g.k_none), hkv, b, lead);
           if (++dc == g.d_chunks) { dc = 0; ++t; }
           if (++s == n_stages) { s = 0; ph ^= 1; }
         }
@@ -536,7 +513,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     uint32_t local_tile = 0;
     for (int tile = tile0; tile < total_tiles; tile += tile_step, ++local_tile) {
       int bh, mt, nt;
-      decode_tile(g.n_mtiles, tile_lo, tile_prefix, tiles_per_head, tile, bh, mt, nt, interleave);
+      decode_tile(g, g.n_mtiles, tile_lo, tile_prefix, tile, bh, mt, nt, interleave);
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
       const int i = mt * kTileM + r;
@@ -550,18 +527,34 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (!ok && split == 1) break;                   // (a cluster's barriers are passed in any case)
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * kTileN + (static_cast<uint32_t>(quad * 32) << 16);
+      // 32-column chunks that some row of the warp sees
+      const int nvis = min((__reduce_max_sync(0xffffffffu, chi >= clo ? chi : -1) + 32) >> 5, n_chunks);
+      // of this warp's quarter of the rows: the chunk in the parts that the other CTAs of the cluster sent
+      const int own = 4 / split;                      // quarters a CTA finishes
+      auto add_parts = [&](uint32_t (&v)[32], int c) {
+        for (int src = 0; src < split - 1; ++src) {
+          const uint8_t* from = smem + (src * own + quad % own) * g.tile_n * 128 + c * 8 * 512 + lane * 16;
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4) {
+            const float4 x = *reinterpret_cast<const float4*>(from + q4 * 512);
+            v[4 * q4] = __float_as_uint(__uint_as_float(v[4 * q4]) + x.x);
+            v[4 * q4 + 1] = __float_as_uint(__uint_as_float(v[4 * q4 + 1]) + x.y);
+            v[4 * q4 + 2] = __float_as_uint(__uint_as_float(v[4 * q4 + 2]) + x.z);
+            v[4 * q4 + 3] = __float_as_uint(__uint_as_float(v[4 * q4 + 3]) + x.w);
+          }
+        }
+      };
       if (split > 1) {
         // The cluster's accumulators are added up, every CTA finishing 128 / split rows: the others' parts of them come
         // through its shared memory ([source][32-row quarter][4 columns][lane] of 16 bytes; the operand stages, which no CTA
-        // reads any more) and go back to tensor memory added to its own.  (The loader and issuer warps keep the barriers
-        // company below.)
-        const int own = 4 / split, dest = quad / own;              // quarters a CTA finishes; the CTA of this warp's
+        // reads any more).  (The loader and issuer warps keep the barriers company below.)
+        const int dest = quad / own;                  // the CTA that finishes this warp's rows
         cluster_sync_all();
         if (dest != rank) {
           const int slot = rank < dest ? rank : rank - 1;
           const uint32_t base = mapa_shared(smem_u32(smem) + (slot * own + quad % own) * g.tile_n * 128 + lane * 16, dest);
 #pragma unroll 1
-          for (int c = 0; c < n_chunks; ++c) {
+          for (int c = 0; c < nvis; ++c) {
             uint32_t v[32];
             tmem_ld32(taddr + c * 32, v);
             tc_wait_ld();
@@ -571,25 +564,17 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         cluster_sync_all();
         if (dest != rank || !ok) break;
+        if (!DIRECT) {
 #pragma unroll 1
-        for (int c = 0; c < n_chunks; ++c) {
-          uint32_t v[32];
-          tmem_ld32(taddr + c * 32, v);
-          tc_wait_ld();
-          for (int src = 0; src < split - 1; ++src) {
-            const uint8_t* from = smem + (src * own + quad % own) * g.tile_n * 128 + c * 8 * 512 + lane * 16;
-#pragma unroll
-            for (int q4 = 0; q4 < 8; ++q4) {
-              const float4 x = *reinterpret_cast<const float4*>(from + q4 * 512);
-              v[4 * q4] = __float_as_uint(__uint_as_float(v[4 * q4]) + x.x);
-              v[4 * q4 + 1] = __float_as_uint(__uint_as_float(v[4 * q4 + 1]) + x.y);
-              v[4 * q4 + 2] = __float_as_uint(__uint_as_float(v[4 * q4 + 2]) + x.z);
-              v[4 * q4 + 3] = __float_as_uint(__uint_as_float(v[4 * q4 + 3]) + x.w);
-            }
+          for (int c = 0; c < nvis; ++c) {
+            uint32_t v[32];
+            tmem_ld32(taddr + c * 32, v);
+            tc_wait_ld();
+            add_parts(v, c);
+            tmem_st32(taddr + c * 32, v);
           }
-          tmem_st32(taddr + c * 32, v);
+          tc_wait_st();
         }
-        tc_wait_st();
       }
       const bool row_ok = i < g.rows_total;
       const size_t rrow = static_cast<size_t>(bh) * g.rows_total + (row_ok ? i : 0);
@@ -604,9 +589,18 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // the query block of this row, and its first row's lane as the writer (RBS divides 32)
         const int qb = i / RBS;
         const int out_cols = g.band ? g.bpc : g.kb_total;
-        est_epilogue_row_direct<RBS>(g, taddr, clo, chi,
-                                     sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, out_cols,
-                                     (lane % RBS) == 0 && qb < g.qb_total, release);
+        uint32_t v[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld32(taddr + c * 32, v[c]);
+        tc_wait_ld();
+        release();
+        if (split > 1) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (c < nvis) add_parts(v[c], c);
+        }
+        est_epilogue_row_direct<RBS>(g, v, nvis, clo, chi, sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols,
+                                     out_cols, qb < g.qb_total, lane);
       } else {
         est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, row_ok,
                               partial + rrow * g.p_pitch - scratch_block0(g, nlo), nt * kGroups,
@@ -704,7 +698,6 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int tiles_per_head = pair_prefix[n_groups];
   const int total_tiles = tiles_per_head * g.batch * g.hq;
   const int k_steps = g.S * g.d_chunks;
-  const int group = g.hq / g.hkv;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (converged warp, one thread issues)
@@ -714,8 +707,9 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       uint32_t ph = 0;
       for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs_grid) {
         int bh, pm, nt;
-        decode_tile(n_groups, pair_lo, pair_prefix, tiles_per_head, tile, bh, pm, nt);
-        const int b = bh / g.hq, h = bh - b * g.hq;
+        decode_tile(g, n_groups, pair_lo, pair_prefix, tile, bh, pm, nt);
+        int h, hg_;
+        const int b = fast_div(bh, g.by_hq, h), hkv = fast_div(h, g.by_group, hg_);
         const int mt = 2 * pm + static_cast<int>(rank);
         int t = 0, dc = 0;
         for (int ks = 0; ks < k_steps; ++ks) {
@@ -728,7 +722,7 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           const int col = k_column(g, dc);
           tma_load_5d_pair_lead(dstA, qt ? &tmQt : &tmQ, full_even, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
           tma_load_5d_pair_lead(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, col, t,
-                           nt * kTileN + static_cast<int>(rank) * 128 + (kt ? 0 : g.k_none), h / group, b, lead);
+                           nt * kTileN + static_cast<int>(rank) * 128 + (kt ? 0 : g.k_none), hkv, b, lead);
           if (++dc == g.d_chunks) { dc = 0; ++t; }
           if (++s == kPairStages) { s = 0; ph ^= 1; }
         }
@@ -797,7 +791,7 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint32_t local_tile = 0;
     for (int tile = pair; tile < total_tiles; tile += n_pairs_grid, ++local_tile) {
       int bh, pm, nt;
-      decode_tile(n_groups, pair_lo, pair_prefix, tiles_per_head, tile, bh, pm, nt);
+      decode_tile(g, n_groups, pair_lo, pair_prefix, tile, bh, pm, nt);
       const int mt = 2 * pm + static_cast<int>(rank);
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
@@ -1015,6 +1009,9 @@ static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int h
   const int lq = q_len + q_pad, lk = k_len + k_pad;
   if (lk / chunk_size < lq / chunk_size) return XATTN_B200_ERR_ARG;   // Xattention.py:39
   g.batch = batch; g.hq = hq; g.hkv = hkv;
+  g.by_tiles = make_fast_div(1);
+  g.by_group = make_fast_div(hq / hkv);
+  g.by_hq = make_fast_div(hq);
   g.S = stride; g.d_chunks = head_dim / kTileK;
   g.rows_total = lq / stride; g.cols_total = lk / stride;
   g.rows_valid = g.rows_total - q_pad / stride;
@@ -1192,36 +1189,39 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   if (g.q_rem && (rc = make_map(&tmQt, q, q_len, hq, qsb, qsh, qsl, kTileM, true))) return rc;
   if (g.k_rem && (rc = make_map(&tmKt, k, k_len, hkv, ksb, ksh, ksl, k_box, true))) return rc;
 
-  if (g.n_mtiles <= kTabTiles) {
-    // few row tiles: the tables travel in the kernel parameters (the arithmetic of est_setup_kernel, on the host)
-    int* t_lo = g.tab, *t_prefix = g.tab + kTabPrefix, *p_lo = g.tab + kTabPairLo, *p_prefix = g.tab + kTabPairPrefix;
-    int cnt[kTabTiles];
-    int acc = 0;
-    for (int mt = 0; mt < g.n_mtiles; ++mt) {
-      row_tile_range(g, mt, t_lo[mt], cnt[mt]);
-      t_prefix[mt] = acc;
-      acc += cnt[mt];
+  // The tile tables (the arithmetic of est_setup_kernel): their totals, and, for few row tiles, the tables themselves, which
+  // then travel in the kernel parameters.
+  const bool in_params = g.n_mtiles <= kTabTiles;
+  int tiles_per_head = 0, pairs_per_head = 0;
+  for (int mt = 0, lo = 0, hi = -1; mt < g.n_mtiles; ++mt) {
+    int first, cnt;
+    row_tile_range(g, mt, first, cnt);
+    if (mt % 2 == 0) {
+      lo = 0x7fffffff;
+      hi = -1;
     }
-    t_prefix[g.n_mtiles] = acc;
-    const int n_pairs = (g.n_mtiles + 1) / 2;
-    acc = 0;
-    for (int pm = 0; pm < n_pairs; ++pm) {
-      int lo = 0x7fffffff, hi = -1;
-      for (int mt = 2 * pm; mt < 2 * pm + 2 && mt < g.n_mtiles; ++mt)
-        if (cnt[mt] > 0) {
-          lo = t_lo[mt] < lo ? t_lo[mt] : lo;
-          hi = t_lo[mt] + cnt[mt] - 1 > hi ? t_lo[mt] + cnt[mt] - 1 : hi;
-        }
-      p_lo[pm] = hi < 0 ? 0 : lo;
-      p_prefix[pm] = acc;
-      acc += hi < 0 ? 0 : hi - lo + 1;
+    if (cnt > 0) {
+      lo = first < lo ? first : lo;
+      hi = first + cnt - 1 > hi ? first + cnt - 1 : hi;
     }
-    p_prefix[n_pairs] = acc;
+    if (in_params) {
+      g.tab[mt] = first;
+      g.tab[kTabPrefix + mt] = tiles_per_head;
+      g.tab[kTabPairLo + mt / 2] = hi < 0 ? 0 : lo;
+      g.tab[kTabPairPrefix + mt / 2] = pairs_per_head;
+    }
+    tiles_per_head += cnt;
+    if (mt % 2 == 1 || mt == g.n_mtiles - 1) pairs_per_head += hi < 0 ? 0 : hi - lo + 1;
+  }
+  g.by_tiles = make_fast_div(static_cast<uint32_t>((use_pairs ? pairs_per_head : tiles_per_head) > 0 ? (use_pairs ? pairs_per_head : tiles_per_head) : 1));
+  if (static_cast<long long>(tiles_per_head) * batch * hq > 0x7fffffffLL) return XATTN_B200_ERR_LIMIT;
+  if (in_params) {
+    g.tab[kTabPrefix + g.n_mtiles] = tiles_per_head;
+    g.tab[kTabPairPrefix + (g.n_mtiles + 1) / 2] = pairs_per_head;
     g.tab_n = g.n_mtiles;
-  } else {
-    if ((rc = launch_dependent(est_setup_kernel, dim3(1), dim3(256), 2 * sizeof(int) * g.n_mtiles, stream, g, tile_lo, tile_prefix,
-                               pair_lo, pair_prefix)))
-      return rc;
+  } else if ((rc = launch_dependent(est_setup_kernel, dim3(1), dim3(256), 2 * sizeof(int) * g.n_mtiles, stream, g, tile_lo, tile_prefix,
+                                    pair_lo, pair_prefix))) {
+    return rc;
   }
 
   const int sms = sm_count();
@@ -1263,13 +1263,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   } else {
   const uint32_t idesc = make_idesc_f16(kTileM, g.tile_n, dtype != XATTN_B200_F16, false, false);
   // persistent CTAs, or exactly the tiles' clusters
-  long long tiles = 0;
-  if (g.split > 1)
-    for (int mt = 0; mt < g.n_mtiles; ++mt) {
-      int first, count;
-      row_tile_range(g, mt, first, count);
-      tiles += static_cast<long long>(count) * batch * hq;
-    }
+  const long long tiles = static_cast<long long>(tiles_per_head) * batch * hq;
   if (tiles == 0) g.split = 1;
   const int grid = g.split > 1 ? static_cast<int>(tiles) * g.split : sms;
   auto launch = [&](auto kern) -> int {

@@ -153,4 +153,23 @@ inline int launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
   return launch_dependent_clusters(kernel, 1, grid, block, smem_bytes, stream, std::forward<Args>(args)...);
 }
 
+// Division of numbers below 2^31 by a divisor known on the host: a multiplication and a shift instead of the ~25
+// instructions of an integer division, which add up in code that every role of a kernel has to decode its work with.
+struct FastDiv {
+  uint32_t d, mul, shift;
+};
+static inline FastDiv make_fast_div(uint32_t d) {
+  FastDiv f;
+  f.d = d;
+  f.shift = 0;
+  while ((1ull << f.shift) < d) ++f.shift;
+  f.mul = static_cast<uint32_t>((((1ull << f.shift) - d) << 32) / d + 1);
+  return f;
+}
+__device__ __forceinline__ int fast_div(int n, const FastDiv& f, int& rem) {
+  const uint32_t q = (__umulhi(static_cast<uint32_t>(n), f.mul) + static_cast<uint32_t>(n)) >> f.shift;
+  rem = n - static_cast<int>(q * f.d);
+  return static_cast<int>(q);
+}
+
 }  // namespace xb
