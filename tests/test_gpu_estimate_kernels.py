@@ -48,3 +48,10 @@ def test_query_shorter_than_the_keys(lq, lk, chunk, semantics):
 def test_split_fp32_terms(L, stride, chunk, causal):
     """fp32 inputs as three bf16 terms: through the single-CTA kernel with 128- and 256-column tiles and the CTA pairs."""
     _check(3, 3, L, L, stride, chunk, causal, torch.float32)
+
+
+@pytest.mark.parametrize("lq,lk,stride,chunk", [(2304, 2304, 8, 256), (1152, 1664, 4, 128), (5120, 5120, 16, 2560), (768, 3840, 4, 768), (1280, 1280, 32, 640)])
+def test_dense_rows_of_a_few_chunks(lq, lk, stride, chunk):
+    """Un-padded causal keys whose chunks are a tile or less each: the epilogue writes whole rows, zeros included; chunks that
+    are not a multiple of a tile leave tiles that hang over the row's end."""
+    _check(2, 2, lq, lk, stride, chunk, True, torch.bfloat16)

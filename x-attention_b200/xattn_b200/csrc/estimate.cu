@@ -20,6 +20,8 @@
 //                        spans at most eight tiles, compute the row statistics itself: no est_rowstat launch).
 #include <math.h>
 
+#include <type_traits>
+
 #include "host_common.cuh"
 #include "sm100_primitives.cuh"
 
@@ -271,58 +273,80 @@ __device__ __forceinline__ void est_epilogue_row(const EstGeom& g, uint32_t tadd
   if (row_ok) *mslot = make_float2(m_scaled, tile_sum);
 }
 
-// Epilogue for geometries in which a reshaped row sees a single 128-column tile (the torch branch with chunks of
-// 128 reshaped rows, e.g. 128K tokens at stride 16): the tile's row maximum and row sum ARE the row's, so the
-// normalised block sums are finished here -- exp2 against the row maximum, sums over groups of RBS columns kept in
-// registers, division by the row sum, and the sum over the RBS rows of a query block taken across lanes -- and
-// written to the chunk-band block sums directly.  Neither the per-row scratch nor the two kernels that would read
-// it are needed.  `out` is the 128 / RBS floats of this row's query block (written by its first row's lane).
+// Epilogue for geometries in which a reshaped row sees a single column tile (the torch branch with chunks of 128 or 256
+// reshaped rows, e.g. 128K or 64K tokens at stride 16; prompts of that many columns altogether): the tile's row maximum and
+// row sum ARE the row's, so the normalised block sums are finished here -- exp2 against the row maximum, sums over groups of
+// RBS columns kept in registers, division by the row sum, and the sum over the RBS rows of a query block taken across lanes
+// -- and written to the block sums directly.  Neither the per-row scratch nor the two kernels that would read it are needed.
+// `out`: the query block's row of out_cols sums, the tile's first one at col0; the others are zero.
 //
-// The row's 128 scores are in registers (`v`, 32-column chunks from `nvis` on hidden from the whole warp): one tensor-memory
-// round trip, all of it at once.  The block sums of the RBS rows of a query block are added by halves: a lane gives away
-// half of its sums and receives the other lane's part of the half it keeps, 14 shuffles for 8 rows instead of 48.
-template <int RBS>
-__device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, uint32_t (&v)[4][32], int nvis, int clo, int chi,
-                                                        float* __restrict__ out, int out_cols, bool write, int lane) {
-  constexpr int kBlocks = 128 / RBS;
+// The row's scores come in halves of 128 columns (`load(half, v)`; chunks of 32 columns from `nvis` on are hidden from the
+// whole warp), each in registers as a whole: one tensor-memory round trip for 128 columns, and the lower half once more for
+// 256.  The block sums of the RBS rows of a query block are added by halves: a lane gives away half of its sums and receives
+// the other lane's part of the half it keeps, 14 shuffles for 8 rows of 16 sums instead of 48.
+template <int RBS, int kHalves, typename Load>
+__device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, Load load, int nvis, int clo, int chi,
+                                                        float* __restrict__ out, int col0, int out_cols, bool write, int lane) {
+  constexpr int kBlocks = kHalves * 128 / RBS, kPer = 32 / RBS;
+  uint32_t v[4][32];
   float mx8[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) mx8[q] = -INFINITY;
+  auto hide = [&](int half) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    if (c >= nvis) continue;
-    if (!__all_sync(0xffffffffu, clo <= c * 32 && chi >= c * 32 + 31)) {
+    for (int c = 0; c < 4; ++c) {
+      const int c0 = half * 128 + c * 32;
+      if (half * 4 + c < nvis && !__all_sync(0xffffffffu, clo <= c0 && chi >= c0 + 31)) {
 #pragma unroll
-      for (int k = 0; k < 32; ++k) v[c][k] = c * 32 + k >= clo && c * 32 + k <= chi ? v[c][k] : 0xff800000u;
+        for (int k = 0; k < 32; ++k) v[c][k] = c0 + k >= clo && c0 + k <= chi ? v[c][k] : 0xff800000u;
+      }
     }
+  };
 #pragma unroll
-    for (int k = 0; k < 16; ++k)
-      mx8[k & 7] = max3(mx8[k & 7], __uint_as_float(v[c][2 * k]), __uint_as_float(v[c][2 * k + 1]));
+  for (int half = 0; half < kHalves; ++half) {
+    if (half * 4 >= nvis && half > 0) continue;
+    load(half, v);
+    hide(half);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (half * 4 + c >= nvis) continue;
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        mx8[k & 7] = max3(mx8[k & 7], __uint_as_float(v[c][2 * k]), __uint_as_float(v[c][2 * k + 1]));
+    }
   }
   const float mx = fmaxf(max3(mx8[0], mx8[1], mx8[2]), max3(max3(mx8[3], mx8[4], mx8[5]), mx8[6], mx8[7]));
   const float m = mx == -INFINITY ? 0.f : mx * g.scale_log2;           // scale > 0
   const unsigned long long scale2 = pack_f32x2(g.scale_log2, g.scale_log2), nm2 = pack_f32x2(-m, -m);
   float blk[kBlocks];
   float row_sum = 0.f;
+  // the upper half is still in registers; the lower one of two is loaded again
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    constexpr int kPer = 32 / RBS;
+  for (int half = kHalves - 1; half >= 0; --half) {
+    if (kHalves == 2 && half == 0 && nvis > 4) {
+      load(0, v);
+      hide(0);
+    }
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) blk[c * kPer + q] = 0.f;
-    if (c >= nvis) continue;
+    for (int c = 0; c < 4; ++c) {
+      const int b0 = (half * 4 + c) * kPer;
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      unsigned long long s2 = 0ull;
+      for (int q = 0; q < kPer; ++q) blk[b0 + q] = 0.f;
+      if (half * 4 + c >= nvis) continue;
 #pragma unroll
-      for (int k = q * RBS / 2; k < (q + 1) * RBS / 2; ++k) {
-        float y0, y1;
-        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c][2 * k]), __uint_as_float(v[c][2 * k + 1])), scale2, nm2), y0, y1);
-        s2 = add_f32x2(s2, pack_f32x2(fast_exp2(y0), fast_exp2(y1)));
+      for (int q = 0; q < kPer; ++q) {
+        unsigned long long s2 = 0ull;
+#pragma unroll
+        for (int k = q * RBS / 2; k < (q + 1) * RBS / 2; ++k) {
+          float y0, y1;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c][2 * k]), __uint_as_float(v[c][2 * k + 1])), scale2, nm2), y0, y1);
+          s2 = add_f32x2(s2, pack_f32x2(fast_exp2(y0), fast_exp2(y1)));
+        }
+        float a, b;
+        unpack_f32x2(s2, a, b);
+        blk[b0 + q] = a + b;
+        row_sum += a + b;
       }
-      float a, b;
-      unpack_f32x2(s2, a, b);
-      blk[c * kPer + q] = a + b;
-      row_sum += a + b;
     }
   }
   // normalise (a row that sees nothing contributes nothing), then add the RBS rows of the query block, RBS lanes
@@ -347,13 +371,17 @@ __device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, uint32
   if (!write) return;
   constexpr int kLeft = kBlocks > RBS ? kBlocks / RBS : 1;
 #pragma unroll
-  for (int q = 0; q < kLeft; ++q) {
-    if (base + q < out_cols) out[base + q] = blk[q];
-    if (kBlocks + base + q < out_cols) out[kBlocks + base + q] = 0.f;  // (dense rows of more blocks than the tile holds)
-  }
+  for (int q = 0; q < kLeft; ++q)
+    if (col0 + base + q < out_cols) out[col0 + base + q] = blk[q];
+  // (dense rows of more blocks than the tile holds)
+  constexpr int kWriters = kBlocks > RBS ? RBS : kBlocks;
+  const int outside = out_cols - (out_cols - col0 < kBlocks ? out_cols - col0 : kBlocks);
+#pragma unroll 1
+  for (int c = base / kLeft; c < outside; c += kWriters) out[c < col0 ? c : c + kBlocks] = 0.f;
 }
 
-template <int RBS, bool DIRECT>
+// kDirect: 128-column halves per row of the epilogue above, 0: the general one
+template <int RBS, int kDirect>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt, const EstGeom g,
@@ -564,7 +592,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         cluster_sync_all();
         if (dest != rank || !ok) break;
-        if (!DIRECT) {
+        if (kDirect == 0) {
 #pragma unroll 1
           for (int c = 0; c < nvis; ++c) {
             uint32_t v[32];
@@ -585,22 +613,26 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(tempty0 + 8 * acc);
       };
-      if constexpr (DIRECT) {
+      if constexpr (kDirect > 0) {
         // the query block of this row, and its first row's lane as the writer (RBS divides 32)
         const int qb = i / RBS;
-        const int out_cols = g.band ? g.bpc : g.kb_total;
-        uint32_t v[4][32];
+        const int out_cols = g.band ? g.bpc : g.kb_total, col0 = g.band ? 0 : nt * kGroups;
+        // (the accumulator goes back to the MMA thread with the last read: the second one of the lower half, if it is read again)
+        int reads = kDirect == 2 && nvis > 4 ? 3 : 1;
+        auto load = [&](int half, uint32_t (&v)[4][32]) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32(taddr + c * 32, v[c]);
-        tc_wait_ld();
-        release();
-        if (split > 1) {
+          for (int c = 0; c < 4; ++c) tmem_ld32(taddr + half * 128 + c * 32, v[c]);
+          tc_wait_ld();
+          if (--reads == 0) release();
+          if (split > 1) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (c < nvis) add_parts(v[c], c);
-        }
-        est_epilogue_row_direct<RBS>(g, v, nvis, clo, chi, sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols,
-                                     out_cols, qb < g.qb_total, lane);
+            for (int c = 0; c < 4; ++c)
+              if (half * 4 + c < nvis) add_parts(v[c], half * 4 + c);
+          }
+        };
+        est_epilogue_row_direct<RBS, kDirect>(g, load, nvis, clo, chi,
+                                              sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, col0, out_cols,
+                                              qb < g.qb_total, lane);
       } else {
         est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, row_ok,
                               partial + rrow * g.p_pitch - scratch_block0(g, nlo), nt * kGroups,
@@ -640,12 +672,13 @@ constexpr int kPairBBytes = 128 * kTileK * 2;                // this CTA's half 
 constexpr int kPairStageBytes = kABytes + kPairBBytes;       // 32 KiB
 constexpr int kPairSmem = kPairStages * kPairStageBytes + 1024 /*barriers*/ + 1024 /*alignment slack*/;
 
-template <int RBS>
+template <int RBS, bool kDirect>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKh,
                      const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt,
                      const EstGeom g, const int* pair_lo, const int* pair_prefix,
-                     float* __restrict__ partial, float2* __restrict__ mtile, const uint32_t idesc, int* status) {
+                     float* __restrict__ partial, float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc,
+                     int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_tab[kTabInts];
   if (g.tab_n) {                                  // (made visible by the __syncthreads() that ends the prologue)
@@ -807,17 +840,33 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint32_t taddr = tmem_base + acc * kTileN + (static_cast<uint32_t>(quad * 32) << 16);
       const bool row_ok = i < g.rows_total;
       const size_t rrow = static_cast<size_t>(bh) * g.rows_total + (row_ok ? i : 0);
-      // (compact scratch: both row tiles of a pair lie in one chunk and start at the pair's first column tile)
-      const int nlo = pair_lo[pm];
-      est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, row_ok,
-                            partial + rrow * g.p_pitch - scratch_block0(g, nlo), nt * kGroups,
-                            mtile + rrow * g.m_pitch + nt - scratch_tile0(g, nlo), [&]() {
-                              // all TMEM reads of this accumulator are done: hand it back to the MMA thread of
-                              // the even CTA
-                              tc_fence_before();
-                              __syncwarp();
-                              if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty0 + 8 * acc, 0));
-                            });
+      // all TMEM reads of this accumulator are done: hand it back to the MMA thread of the even CTA
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty0 + 8 * acc, 0));
+      };
+      if constexpr (kDirect) {
+        const int qb = i / RBS;
+        const int out_cols = g.band ? g.bpc : g.kb_total, col0 = g.band ? 0 : nt * kGroups;
+        const int nvis = (__reduce_max_sync(0xffffffffu, chi >= clo ? chi : -1) + 32) >> 5;
+        int reads = nvis > 4 ? 3 : 1;
+        auto load = [&](int half, uint32_t (&v)[4][32]) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld32(taddr + half * 128 + c * 32, v[c]);
+          tc_wait_ld();
+          if (--reads == 0) release();
+        };
+        est_epilogue_row_direct<RBS, 2>(g, load, nvis, clo, chi,
+                                        sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, col0, out_cols,
+                                        qb < g.qb_total, lane);
+      } else {
+        // (compact scratch: both row tiles of a pair lie in one chunk and start at the pair's first column tile)
+        const int nlo = pair_lo[pm];
+        est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, row_ok,
+                              partial + rrow * g.p_pitch - scratch_block0(g, nlo), nt * kGroups,
+                              mtile + rrow * g.m_pitch + nt - scratch_tile0(g, nlo), release);
+      }
     }
   }
 
@@ -1164,20 +1213,19 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     g.split = !long_k ? 1 : (4 * tiles <= sm_count() ? 4 : (2 * tiles <= sm_count() ? 2 : 1));
     if (g.split > 1) use_pairs = false;
   }
-  // Every row sees a single 128-column tile and that tile's block sums are (nearly) a whole row of the output: chunks of
-  // exactly one 128-row, 128-column tile in the chunk-band layout (128K tokens at stride 16), or keys of at most 128 columns
-  // altogether (prompts of up to 2048 tokens at stride 16).  The GEMM's epilogue then finishes the block sums itself, and
+  // Every row sees a single column tile, and that tile's block sums are (nearly) a whole row of the output: chunks of exactly
+  // 128 or 256 reshaped rows in the chunk-band layout (128K or 64K tokens at stride 16), or keys of at most 256 columns
+  // altogether (prompts of up to 4096 tokens at stride 16) or of a few such chunks.  The GEMM's epilogue then finishes the block sums itself, and
   // neither the scratch arrays nor est_rowstat_kernel / est_blocksum_kernel are needed.
-  bool direct = !use_pairs && g.tile_n == 128 && g.rbs <= 32 && 32 % g.rbs == 0;
+  bool direct = g.rbs <= 32 && 32 % g.rbs == 0;
   if (g.band)
-    direct = direct && g.compact && g.m_pitch == 1 && g.rcs == kTileM && g.row_off % 128 == 0 && g.bpc == 128 / g.rbs &&
-             g.bpc % 4 == 0 && (reinterpret_cast<uintptr_t>(attn_sums) & 15) == 0;
+    direct = direct && g.compact && g.m_pitch == 1 && g.rcs == g.tile_n && g.row_off % g.tile_n == 0 && g.bpc == g.tile_n / g.rbs;
   else
-    direct = direct && g.kb_total <= 256 / g.rbs;
+    direct = direct && g.kb_total <= 8 * g.tile_n / g.rbs;             // (the epilogue writes the zeros, a few at a time)
   for (int mt = 0; direct && mt < g.n_mtiles; ++mt) {
     int first, count;
     row_tile_range(g, mt, first, count);
-    direct = g.band ? count == 1 && first * 128 == (mt * kTileM / g.rcs) * g.rcs + g.row_off : count <= 1 && first == 0;
+    direct = g.band ? count == 1 && first * g.tile_n == (mt * kTileM / g.rcs) * g.rcs + g.row_off : count <= 1;
   }
   g.direct = direct ? 1 : 0;
   CUtensorMap tmQ, tmK, tmQt, tmKt;
@@ -1250,16 +1298,16 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       if (max_clusters < 1) return XATTN_B200_ERR_CUDA;
       if (static_cast<unsigned>(2 * max_clusters) < cfg.gridDim.x) cfg.gridDim.x = 2 * max_clusters;
       return launch_dependent_clusters(kern, 2, cfg.gridDim, cfg.blockDim, kPairSmem, stream, tmQ, tmK, tmQt, tmKt, g,
-                                       (const int*)pair_lo, (const int*)pair_prefix, partial, mtile, idesc2, status);
+                                       (const int*)pair_lo, (const int*)pair_prefix, partial, mtile, attn_sums, idesc2, status);
     };
     switch (g.rbs) {
-      case 4: rc = launch_pair(est_gemm_pair_kernel<4>); break;
-      case 8: rc = launch_pair(est_gemm_pair_kernel<8>); break;
-      case 16: rc = launch_pair(est_gemm_pair_kernel<16>); break;
-      case 32: rc = launch_pair(est_gemm_pair_kernel<32>); break;
+      case 4: rc = direct ? launch_pair(est_gemm_pair_kernel<4, true>) : launch_pair(est_gemm_pair_kernel<4, false>); break;
+      case 8: rc = direct ? launch_pair(est_gemm_pair_kernel<8, true>) : launch_pair(est_gemm_pair_kernel<8, false>); break;
+      case 16: rc = direct ? launch_pair(est_gemm_pair_kernel<16, true>) : launch_pair(est_gemm_pair_kernel<16, false>); break;
+      case 32: rc = direct ? launch_pair(est_gemm_pair_kernel<32, true>) : launch_pair(est_gemm_pair_kernel<32, false>); break;
       default: rc = XATTN_B200_ERR_ARG;
     }
-    if (rc) return rc;
+    if (rc || direct) return rc;                       // (direct: the block sums are complete)
   } else {
   const uint32_t idesc = make_idesc_f16(kTileM, g.tile_n, dtype != XATTN_B200_F16, false, false);
   // persistent CTAs, or exactly the tiles' clusters
@@ -1272,23 +1320,19 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     return launch_dependent_clusters(kern, g.split, dim3(grid), dim3(kGemmThreads), kGemmSmem, stream, tmQ, tmK, tmQt, tmKt, g,
                             (const int*)tile_lo, (const int*)tile_prefix, partial, mtile, attn_sums, idesc, status);
   };
-  if (direct) {
-    switch (g.rbs) {
-      case 4: rc = launch(est_gemm_kernel<4, true>); break;
-      case 8: rc = launch(est_gemm_kernel<8, true>); break;
-      case 16: rc = launch(est_gemm_kernel<16, true>); break;
-      case 32: rc = launch(est_gemm_kernel<32, true>); break;
-      default: rc = XATTN_B200_ERR_ARG;
-    }
-    return rc;                                         // the block sums are complete
-  }
+  auto launch_rbs = [&](auto rbs) -> int {
+    constexpr int kRbs = decltype(rbs)::value;
+    if (!direct) return launch(est_gemm_kernel<kRbs, 0>);
+    return g.tile_n == 128 ? launch(est_gemm_kernel<kRbs, 1>) : launch(est_gemm_kernel<kRbs, 2>);
+  };
   switch (g.rbs) {
-    case 4: rc = launch(est_gemm_kernel<4, false>); break;
-    case 8: rc = launch(est_gemm_kernel<8, false>); break;
-    case 16: rc = launch(est_gemm_kernel<16, false>); break;
-    case 32: rc = launch(est_gemm_kernel<32, false>); break;
+    case 4: rc = launch_rbs(std::integral_constant<int, 4>()); break;
+    case 8: rc = launch_rbs(std::integral_constant<int, 8>()); break;
+    case 16: rc = launch_rbs(std::integral_constant<int, 16>()); break;
+    case 32: rc = launch_rbs(std::integral_constant<int, 32>()); break;
     default: rc = XATTN_B200_ERR_ARG;
   }
+  if (direct) return rc;                               // the block sums are complete
   if (rc) return rc;
   }
 
