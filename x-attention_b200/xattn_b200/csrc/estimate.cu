@@ -15,9 +15,8 @@
 //                        warps run the epilogue: per row, max over the tile's visible columns, exp2,
 //                        sums over groups of block/S columns.  Output per (row, key block): an
 //                        un-normalised partial sum, plus the max it was taken against per (row, tile).
-//   est_rowstat_kernel   per row: combine the tiles' maxima and sums into the row's max and 1/sum
-//   est_blocksum_kernel  per (query block, key block): normalise and add the block/S rows (and, when a row
-//                        spans at most eight tiles, compute the row statistics itself: no est_rowstat launch).
+//   est_blocksum_kernel  per query block: the rows' maxima and sums over their tiles, then per key block: normalise and
+//                        add the block/S rows.  (Rows of a single tile need neither, see est_epilogue_row_direct.)
 #include <math.h>
 
 #include <type_traits>
@@ -52,11 +51,11 @@ struct EstGeom {
   int tile_n;                  // columns per tile: 256, or 128 when no row sees more than 128 columns
   int band;                    // attn_sums holds only the chunk's own key blocks (left_blank only): row stride bpc
   int bpc;                     // key blocks per chunk
-  // scratch layout: a reshaped row keeps m_pitch (max, sum) pairs and p_pitch partial block sums.  Dense: one per
-  // column tile / key block of the whole row.  Compact (left_blank: a row only ever touches the tiles of its own
-  // chunk): the column tiles [tile_lo, tile_lo + m_pitch) of its row tile, i.e. key blocks from tile_lo * (tile_n /
-  // rbs) on -- 16 floats per row instead of 1024 at 128K tokens.
-  int compact, m_pitch, p_pitch;
+  // Scratch layout: tile by tile, m_pitch tiles per row tile; a tile holds tile_n / rbs partial block sums and one (max, sum)
+  // pair of each of its 128 rows, the rows of a block sum next to one another (the epilogue's lanes are rows, and
+  // est_blocksum_kernel reads the rows of a query block).  Dense: every column tile.  Compact (left_blank: a row only ever
+  // touches the tiles of its own chunk): the column tiles [tile_lo, tile_lo + m_pitch) of the row tile.
+  int compact, m_pitch;
   // Lengths that are no multiple of the stride: the last stride group lacks the tokens of offset >= len % stride, which
   // count as zeros.  Two tensor maps of each operand: token offsets below the remainder go through one that has that group,
   // the others through one that ends before it (no group at all: the coordinate is moved past the only one).
@@ -100,10 +99,10 @@ __device__ __forceinline__ int k_column(const EstGeom& g, int dc) {
   return (term * g.term_chunks + c) * kTileK;
 }
 
-// first column tile / first key block a row tile's scratch rows are indexed from
+// first column tile of a row tile's scratch, and the number of its tile (bh, mt, nt)
 __host__ __device__ inline int scratch_tile0(const EstGeom& g, int nlo) { return g.compact ? nlo : 0; }
-__host__ __device__ inline int scratch_block0(const EstGeom& g, int nlo) {
-  return g.compact ? nlo * (g.tile_n / g.rbs) : 0;
+__device__ __forceinline__ size_t scratch_tile(const EstGeom& g, int bh, int mt, int nt, int nlo) {
+  return (static_cast<size_t>(bh) * g.n_mtiles + mt) * g.m_pitch + nt - scratch_tile0(g, nlo);
 }
 // column-tile range of row tile mt: first tile and count (the formula of est_setup_kernel, also used by the host
 // to size the compact scratch)
@@ -194,27 +193,27 @@ __device__ __forceinline__ void decode_tile(const EstGeom& g, int n_groups, cons
 // Epilogue of one accumulator tile for one row (thread): softmax statistics and un-normalised block sums of the
 // tile's visible columns [clo, chi].  Two passes over the row in tensor memory (maximum, then exp2 and sums over
 // groups of RBS columns), the load of the next 32 columns in flight while the current ones are processed; chunks
-// that every lane of the warp sees completely skip the per-element range test.  `release` is called once all
+// that every lane of the warp sees completely skip the per-element range test.  `part`: this row's first partial sum, the
+// next key block's is kTileM floats on (a warp stores 128 contiguous bytes).  `release` is called once all
 // tensor-memory reads of the tile are done.
 template <int RBS, typename Release>
 __device__ __forceinline__ void est_epilogue_row(const EstGeom& g, uint32_t taddr, int n_chunks, int clo, int chi,
-                                                 bool row_ok, float* __restrict__ prow, int kb0,
-                                                 float2* __restrict__ mslot, Release release) {
-  auto fully_visible = [&](int c8) { return __all_sync(0xffffffffu, clo <= c8 * 32 && chi >= c8 * 32 + 31); };
+                                                 bool write, float* __restrict__ part, float2* __restrict__ mslot,
+                                                 Release release) {
+  // columns hidden from this row become -inf, in chunks that some row of the warp sees only in part
+  auto hide = [&](uint32_t (&v)[32], int c8) {
+    if (!__all_sync(0xffffffffu, clo <= c8 * 32 && chi >= c8 * 32 + 31)) {
+#pragma unroll
+      for (int k = 0; k < 32; ++k) v[k] = c8 * 32 + k >= clo && c8 * 32 + k <= chi ? v[k] : 0xff800000u;
+    }
+  };
   // pass 1: row maximum over the visible columns
   float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
   {
-    auto max_chunk = [&](const uint32_t (&v)[32], int c8) {
-      if (fully_visible(c8)) {
+    auto max_chunk = [&](uint32_t (&v)[32], int c8) {
+      hide(v, c8);
 #pragma unroll
-        for (int k = 0; k < 32; ++k) mx4[k & 3] = fmaxf(mx4[k & 3], __uint_as_float(v[k]));
-      } else {
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          const int c = c8 * 32 + k;
-          if (c >= clo && c <= chi) mx4[k & 3] = fmaxf(mx4[k & 3], __uint_as_float(v[k]));
-        }
-      }
+      for (int k = 0; k < 16; ++k) mx4[k & 3] = max3(mx4[k & 3], __uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
     };
     uint32_t va[32], vb[32];
     tmem_ld32(taddr, va);
@@ -230,31 +229,31 @@ __device__ __forceinline__ void est_epilogue_row(const EstGeom& g, uint32_t tadd
   }
   const float m_scaled = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * g.scale_log2;     // scale > 0
   // pass 2: exp2 and sums over groups of RBS columns
+  const float m_ref = m_scaled == -INFINITY ? 0.f : m_scaled;
+  const unsigned long long scale2 = pack_f32x2(g.scale_log2, g.scale_log2), nm2 = pack_f32x2(-m_ref, -m_ref);
   float tile_sum = 0.f;
   {
-    auto sum_chunk = [&](const uint32_t (&v)[32], int c8) {
+    auto sum_chunk = [&](uint32_t (&v)[32], int c8) {
+      hide(v, c8);
       float gs[32 / RBS];
 #pragma unroll
-      for (int q = 0; q < 32 / RBS; ++q) gs[q] = 0.f;
-      if (fully_visible(c8)) {
+      for (int q = 0; q < 32 / RBS; ++q) {
+        unsigned long long s2 = 0ull;
 #pragma unroll
-        for (int k = 0; k < 32; ++k) gs[k / RBS] += fast_exp2(fmaf(__uint_as_float(v[k]), g.scale_log2, -m_scaled));
-      } else {
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          const int c = c8 * 32 + k;
-          const float x = fmaf(__uint_as_float(v[k]), g.scale_log2, -m_scaled);
-          gs[k / RBS] += (c >= clo && c <= chi) ? fast_exp2(x) : 0.f;
+        for (int k = q * RBS / 2; k < (q + 1) * RBS / 2; ++k) {
+          float y0, y1;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1])), scale2, nm2), y0, y1);
+          s2 = add_f32x2(s2, pack_f32x2(fast_exp2(y0), fast_exp2(y1)));
         }
+        float a, b;
+        unpack_f32x2(s2, a, b);
+        gs[q] = a + b;
       }
 #pragma unroll
       for (int q = 0; q < 32 / RBS; ++q) tile_sum += gs[q];
-      if (row_ok) {
+      if (write) {
 #pragma unroll
-        for (int q = 0; q < 32 / RBS; ++q) {
-          const int kb = kb0 + c8 * (32 / RBS) + q;
-          if (kb < g.kb_total) prow[kb] = gs[q];
-        }
+        for (int q = 0; q < 32 / RBS; ++q) part[(c8 * (32 / RBS) + q) * kTileM] = gs[q];
       }
     };
     uint32_t va[32], vb[32];
@@ -270,7 +269,7 @@ __device__ __forceinline__ void est_epilogue_row(const EstGeom& g, uint32_t tadd
       sum_chunk(vb, c8 + 1);
     }
   }
-  if (row_ok) *mslot = make_float2(m_scaled, tile_sum);
+  if (write) *mslot = make_float2(m_scaled, tile_sum);
 }
 
 // Epilogue for geometries in which a reshaped row sees a single column tile (the torch branch with chunks of 128 or 256
@@ -604,9 +603,6 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tc_wait_st();
         }
       }
-      const bool row_ok = i < g.rows_total;
-      const size_t rrow = static_cast<size_t>(bh) * g.rows_total + (row_ok ? i : 0);
-      const int nlo = tile_lo[mt];
       auto release = [&]() {
         // all TMEM reads of this accumulator are done: hand it back to the MMA thread
         tc_fence_before();
@@ -634,9 +630,8 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                                               sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, col0, out_cols,
                                               qb < g.qb_total, lane);
       } else {
-        est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, row_ok,
-                              partial + rrow * g.p_pitch - scratch_block0(g, nlo), nt * kGroups,
-                              mtile + rrow * g.m_pitch + nt - scratch_tile0(g, nlo), release);
+        const size_t tile_at = scratch_tile(g, bh, mt, nt, tile_lo[mt]) * kTileM;
+        est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, true, partial + tile_at * kGroups + r, mtile + tile_at + r, release);
       }
     }
   }
@@ -838,8 +833,6 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, acc_ph, abort_flag))) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * kTileN + (static_cast<uint32_t>(quad * 32) << 16);
-      const bool row_ok = i < g.rows_total;
-      const size_t rrow = static_cast<size_t>(bh) * g.rows_total + (row_ok ? i : 0);
       // all TMEM reads of this accumulator are done: hand it back to the MMA thread of the even CTA
       auto release = [&]() {
         tc_fence_before();
@@ -862,10 +855,9 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                                         qb < g.qb_total, lane);
       } else {
         // (compact scratch: both row tiles of a pair lie in one chunk and start at the pair's first column tile)
-        const int nlo = pair_lo[pm];
-        est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, row_ok,
-                              partial + rrow * g.p_pitch - scratch_block0(g, nlo), nt * kGroups,
-                              mtile + rrow * g.m_pitch + nt - scratch_tile0(g, nlo), release);
+        const bool write = mt < g.n_mtiles;
+        const size_t tile_at = scratch_tile(g, bh, write ? mt : 0, nt, pair_lo[pm]) * kTileM;
+        est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, write, partial + tile_at * kGroups + r, mtile + tile_at + r, release);
       }
     }
   }
@@ -887,109 +879,98 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
 }
 
-// Normalisation of the partial sums, as two streaming kernels.
-//   est_rowstat_kernel  one thread per reshaped row i:  m_i = max_t m_{i,t},
-//                       1/l_i with l_i = sum_t s_{i,t} 2^(m_{i,t} - m_i)      (m, s = per-tile max and sum)
-//   est_blocksum_kernel one thread per (query block, key block):
-//                       out[qb][kb] = sum_{i in qb} partial[i][kb] * 2^(m_{i,t(kb)} - m_i) / l_i
-__global__ void __launch_bounds__(256)
-est_rowstat_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
-                   const float2* __restrict__ mtile, float2* __restrict__ rowstat, int total_rows) {
+// Normalisation of the partial sums, one CTA per query block:
+//   row i:  m_i = max_t m_{i,t},  l_i = sum_t s_{i,t} 2^(m_{i,t} - m_i)                (m, s = per-tile max and sum)
+//   out[kb] = sum_i partial[i][kb] * f_{i,t(kb)},  f_{i,t} = 2^(m_{i,t} - m_i) / l_i
+// A stream over the partial sums: a thread per key block reads its RBS rows as 16-byte vectors (64 contiguous bytes for
+// RBS = 16), the factors come from shared memory.  The first key block's rows are on their way while the statistics are
+// computed.  (32K tokens, stride 8: the estimate phase 267 us with rows apart in the scratch and the factors recomputed by every thread,
+// 238 us like this.)
+constexpr int kSumThreads = 128;
+template <int RBS>
+__global__ void __launch_bounds__(kSumThreads)
+est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix, const float* __restrict__ partial,
+                    const float2* __restrict__ mtile, float* __restrict__ sums, int seg_tiles) {
+  extern __shared__ float s_f[];                           // [tile][row] factors, seg_tiles tiles at a time
+  __shared__ float2 s_part[kSumThreads];                   // [part][row] (max, sum)
+  constexpr int kParts = kSumThreads / RBS;
   pdl_launch_dependents();
   pdl_wait();
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= total_rows) return;
-  const int i = idx % g.rows_total;
-  const int mt = i / kTileM;
-  // (the three table entries a row needs come straight from the kernel parameters when the tables are there)
+  const int qb = blockIdx.x, bh = blockIdx.y;
+  const int i0 = qb * RBS, mt = i0 / kTileM, r0 = i0 % kTileM;
   const int nlo = g.tab_n ? g.tab[mt] : tile_lo[mt];
   const int ncnt = g.tab_n ? g.tab[kTabPrefix + mt + 1] - g.tab[kTabPrefix + mt] : tile_prefix[mt + 1] - tile_prefix[mt];
-  const float2* mrow = mtile + static_cast<size_t>(idx) * g.m_pitch + nlo - scratch_tile0(g, nlo);
-  float m = -INFINITY, l = 0.f;
-  if (i < g.rows_valid) {
-    for (int t = 0; t < ncnt; ++t) m = fmaxf(m, mrow[t].x);
-    if (m > -INFINITY)
-      for (int t = 0; t < ncnt; ++t) {
-        const float2 ms = mrow[t];
-        if (ms.x > -INFINITY) l += ms.y * exp2f(ms.x - m);
-      }
-  }
-  rowstat[idx] = make_float2(m, l > 0.f ? 1.f / l : 0.f);
-}
-
-// VEC consecutive key blocks per thread (4 when kb_total is a multiple of 4: one 16-byte store; they share a tile)
-// FUSED: the query block's row statistics are computed here (eight threads per row, one (max, sum) pair each, so
-// a row costs one memory round trip) instead of being read from est_rowstat_kernel's output; for geometries whose
-// rows span at most eight column tiles.
-template <int VEC, bool FUSED>
-__global__ void __launch_bounds__(256)
-est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
-                    const float* __restrict__ partial, const float2* __restrict__ mtile,
-                    const float2* __restrict__ rowstat, float* __restrict__ sums) {
-  __shared__ float2 s_stat[32];                            // FUSED: (m_i, 1/l_i) of the query block's rows (rbs <= 32)
-  pdl_launch_dependents();
-  pdl_wait();
-  const int qb = blockIdx.y, bh = blockIdx.z;
-  const int i0 = qb * g.rbs;
-  if (FUSED) {
-    const int mt_ = i0 / kTileM;
-    const int nlo_ = g.tab_n ? g.tab[mt_] : tile_lo[mt_];
-    const int ncnt_ = g.tab_n ? g.tab[kTabPrefix + mt_ + 1] - g.tab[kTabPrefix + mt_]
-                              : tile_prefix[mt_ + 1] - tile_prefix[mt_];
-    int rows_ = g.rows_valid - i0;
-    rows_ = rows_ > g.rbs ? g.rbs : rows_;
-    const int row = threadIdx.x >> 3, slot = threadIdx.x & 7;
-    if (row < g.rbs) {                                     // whole 8-lane groups take the branch together
-      float2 ms = make_float2(-INFINITY, 0.f);
-      if (row < rows_ && slot < ncnt_)
-        ms = mtile[(static_cast<size_t>(bh) * g.rows_total + i0 + row) * g.m_pitch + nlo_ - scratch_tile0(g, nlo_) + slot];
-      const unsigned grp = 0xffu << (threadIdx.x & 24);    // the eight lanes of this row
-      float m = ms.x;
-      m = fmaxf(m, __shfl_xor_sync(grp, m, 1));
-      m = fmaxf(m, __shfl_xor_sync(grp, m, 2));
-      m = fmaxf(m, __shfl_xor_sync(grp, m, 4));
-      const float term = (m > -INFINITY && ms.x > -INFINITY) ? ms.y * exp2f(ms.x - m) : 0.f;
-      float l = 0.f;                                       // summed in tile order, as est_rowstat_kernel does
+  const int gpt = g.tile_n / RBS;                          // key blocks per tile
+  const size_t tile0 = scratch_tile(g, bh, mt, nlo, nlo);
+  const float2* ms = mtile + tile0 * kTileM + r0;
+  const float* pp = partial + tile0 * gpt * kTileM + r0;   // key block nlo * gpt + k: at k * kTileM
+  // band layout: only the key blocks of the query block's own chunk, [cur, cur + bpc)
+  const int cur = g.band ? (g.row_off + (i0 / g.rcs) * g.rcs) / RBS : 0, n_out = g.band ? g.bpc : g.kb_total;
+  float4 p4[RBS / 4];
+  auto fetch = [&](int kl) {                               // the rows of output kl; zeros outside the tiles
+    const int k = cur + kl - nlo * gpt;
+    const bool in = kl < n_out && k >= 0 && k < ncnt * gpt;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) l += __shfl_sync(grp, term, (threadIdx.x & 24) + k);
-      if (slot == 0) s_stat[row] = make_float2(m, l > 0.f ? 1.f / l : 0.f);
+    for (int j = 0; j < RBS / 4; ++j)
+      p4[j] = in ? __ldcs(reinterpret_cast<const float4*>(pp + static_cast<size_t>(k) * kTileM) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  fetch(threadIdx.x);
+  float row_m, row_inv;                                    // of row threadIdx.x % RBS
+  {
+    const int row = threadIdx.x % RBS, part = threadIdx.x / RBS;
+    const bool valid = i0 + row < g.rows_valid;
+    float m = -INFINITY, l = 0.f;
+    for (int t = part; t < ncnt; t += kParts) {
+      const float2 x = ms[t * kTileM + row];
+      if (valid && x.x > -INFINITY) {
+        const float mn = fmaxf(m, x.x);
+        l = l * exp2f(m - mn) + x.y * exp2f(x.x - mn);
+        m = mn;
+      }
+    }
+    s_part[threadIdx.x] = make_float2(m, l);
+    __syncthreads();
+    float mm = -INFINITY, ll = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < kParts; ++k) mm = fmaxf(mm, s_part[k * RBS + row].x);
+#pragma unroll 4
+    for (int k = 0; k < kParts; ++k) {
+      const float2 x = s_part[k * RBS + row];
+      if (x.x > -INFINITY) ll += x.y * exp2f(x.x - mm);
+    }
+    row_m = mm;
+    row_inv = ll > 0.f ? 1.f / ll : 0.f;
+  }
+  float* out = sums + (static_cast<size_t>(bh) * g.qb_total + qb) * n_out;
+#pragma unroll 1
+  for (int t0 = 0; t0 == 0 || t0 < ncnt; t0 += seg_tiles) {
+    const int t1 = t0 + seg_tiles < ncnt ? t0 + seg_tiles : ncnt;
+    if (t0 > 0) {
+      __syncthreads();
+      fetch(threadIdx.x);
+    }
+    for (int t = t0 + threadIdx.x / RBS; t < t1; t += kParts) {
+      const float x = ms[t * kTileM + threadIdx.x % RBS].x;
+      s_f[(t - t0) * RBS + threadIdx.x % RBS] = row_inv > 0.f && x > -INFINITY ? exp2f(x - row_m) * row_inv : 0.f;
     }
     __syncthreads();
-  }
-  // band layout: only the key blocks of the query block's own chunk, [cur, cur + bpc)
-  const int cur = g.band ? (g.row_off + (i0 / g.rcs) * g.rcs) / g.rbs : 0;
-  const int kb_local = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
-  if (kb_local >= (g.band ? g.bpc : g.kb_total)) return;
-  const int kb = cur + kb_local;
-  const int mt = i0 / kTileM;
-  const int nlo = g.tab_n ? g.tab[mt] : tile_lo[mt];
-  const int ncnt = g.tab_n ? g.tab[kTabPrefix + mt + 1] - g.tab[kTabPrefix + mt] : tile_prefix[mt + 1] - tile_prefix[mt];
-  const int gpt = g.tile_n / g.rbs;                       // key blocks per tile (a multiple of 4)
-  const int t = kb / gpt;
-  float acc[VEC];
+    for (int kl = threadIdx.x; kl < n_out; kl += kSumThreads) {
+      const int k = cur + kl - nlo * gpt, t = k >= 0 ? k / gpt : -1;
+      if (t >= t0 && t < t1) {
+        const float4* f4 = reinterpret_cast<const float4*>(s_f + (t - t0) * RBS);
+        float acc = 0.f;
 #pragma unroll
-  for (int q = 0; q < VEC; ++q) acc[q] = 0.f;
-  if (t >= nlo && t < nlo + ncnt) {
-    const size_t r0 = static_cast<size_t>(bh) * g.rows_total + i0;
-    int rows = g.rows_valid - i0;                         // rows past rows_valid contribute nothing
-    rows = rows > g.rbs ? g.rbs : rows;
-#pragma unroll 2
-    for (int row = 0; row < rows; ++row) {
-      const float2 st = FUSED ? s_stat[row] : rowstat[r0 + row];
-      const float mx = mtile[(r0 + row) * g.m_pitch + t - scratch_tile0(g, nlo)].x;
-      const float f = (st.y > 0.f && mx > -INFINITY) ? exp2f(mx - st.x) * st.y : 0.f;
-      const float* pp = partial + (r0 + row) * g.p_pitch + kb - scratch_block0(g, nlo);
-      if (VEC == 4) {
-        const float4 pv = *reinterpret_cast<const float4*>(pp);
-        if (f != 0.f) { acc[0] += pv.x * f; acc[1 % VEC] += pv.y * f; acc[2 % VEC] += pv.z * f; acc[3 % VEC] += pv.w * f; }
-      } else {
-        if (f != 0.f) acc[0] += pp[0] * f;
+        for (int j = 0; j < RBS / 4; ++j) {
+          const float4 f = f4[j];
+          acc += p4[j].x * f.x + p4[j].y * f.y + p4[j].z * f.z + p4[j].w * f.w;
+        }
+        out[kl] = acc;
+      } else if (t0 == 0 && (t < 0 || t >= ncnt)) {
+        out[kl] = 0.f;
       }
+      if (kl + kSumThreads < n_out) fetch(kl + kSumThreads);
     }
   }
-  float* out = sums + (static_cast<size_t>(bh) * g.qb_total + qb) * (g.band ? g.bpc : g.kb_total) + kb_local;
-  if (VEC == 4) *reinterpret_cast<float4*>(out) = make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]);
-  else out[0] = acc[0];
 }
 
 // x = hi + mid + lo in bf16 (each the rounding of what the ones before it leave), stored as rows [hi | mid | lo] of
@@ -1043,7 +1024,7 @@ split_f32_kernel(const float* __restrict__ x, int heads, int len, int len_valid,
 
 // ------------------------------------------------------------------------------------ host side
 struct EstWorkspace {
-  size_t off_tile_lo, off_tile_prefix, off_pair_lo, off_pair_prefix, off_rowstat, off_mtile, off_partial;
+  size_t off_tile_lo, off_tile_prefix, off_pair_lo, off_pair_prefix, off_mtile, off_partial;
   size_t total;
 };
 
@@ -1092,7 +1073,6 @@ static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int h
   g.split = 1;
   g.compact = g.left_blank;
   g.m_pitch = g.n_ntiles;
-  g.p_pitch = g.kb_total;
   if (g.compact) {
     int max_cnt = 1;
     for (int mt = 0; mt < g.n_mtiles; ++mt) {
@@ -1101,7 +1081,6 @@ static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int h
       max_cnt = cnt > max_cnt ? cnt : max_cnt;
     }
     g.m_pitch = max_cnt;
-    g.p_pitch = max_cnt * (g.tile_n / g.rbs);
   }
   return XATTN_B200_OK;
 }
@@ -1114,10 +1093,9 @@ static EstWorkspace workspace_layout(const EstGeom& g) {
   w.off_tile_prefix = o; o = up(o + sizeof(int) * (g.n_mtiles + 1));
   w.off_pair_lo = o; o = up(o + sizeof(int) * ((g.n_mtiles + 1) / 2));
   w.off_pair_prefix = o; o = up(o + sizeof(int) * ((g.n_mtiles + 1) / 2 + 1));
-  const size_t rows = static_cast<size_t>(g.batch) * g.hq * g.rows_total;
-  w.off_rowstat = o; o = up(o + sizeof(float2) * rows);
+  const size_t rows = static_cast<size_t>(g.batch) * g.hq * g.n_mtiles * kTileM;
   w.off_mtile = o; o = up(o + sizeof(float2) * rows * g.m_pitch);
-  w.off_partial = o; o = up(o + sizeof(float) * rows * g.p_pitch);
+  w.off_partial = o; o = up(o + sizeof(float) * rows * g.m_pitch * (g.tile_n / g.rbs));
   w.total = o;
   return w;
 }
@@ -1180,7 +1158,6 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   int* pair_lo = reinterpret_cast<int*>(ws + w.off_pair_lo);
   int* pair_prefix = reinterpret_cast<int*>(ws + w.off_pair_prefix);
   float2* mtile = reinterpret_cast<float2*>(ws + w.off_mtile);
-  float2* rowstat = reinterpret_cast<float2*>(ws + w.off_rowstat);
   float* partial = reinterpret_cast<float*>(ws + w.off_partial);
 
   // 5-D views [head_dim, S, len/S, heads, batch] whose second coordinate picks the token inside a stride group; `up`: with
@@ -1216,7 +1193,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // Every row sees a single column tile, and that tile's block sums are (nearly) a whole row of the output: chunks of exactly
   // 128 or 256 reshaped rows in the chunk-band layout (128K or 64K tokens at stride 16), or keys of at most 256 columns
   // altogether (prompts of up to 4096 tokens at stride 16) or of a few such chunks.  The GEMM's epilogue then finishes the block sums itself, and
-  // neither the scratch arrays nor est_rowstat_kernel / est_blocksum_kernel are needed.
+  // neither the scratch arrays nor est_blocksum_kernel are needed.
   bool direct = g.rbs <= 32 && 32 % g.rbs == 0;
   if (g.band)
     direct = direct && g.compact && g.m_pitch == 1 && g.rcs == g.tile_n && g.row_off % g.tile_n == 0 && g.bpc == g.tile_n / g.rbs;
@@ -1336,31 +1313,19 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   if (rc) return rc;
   }
 
-  // rows that span at most eight column tiles: their statistics are computed inside est_blocksum_kernel
-  const int max_tiles_per_row = g.m_pitch;             // (dense scratch: every column tile of the row)
-  const int out_cols = g.band ? g.bpc : g.kb_total;
-  const bool vec4 = g.kb_total % 4 == 0 && out_cols % 4 == 0 && (reinterpret_cast<uintptr_t>(attn_sums) & 15) == 0;
-  const int per_row = vec4 ? out_cols / 4 : out_cols;
-  // (and a query block with enough key blocks to amortise the extra round trip: measured -11 us at 32K, where a
-  // CTA sums 128 key blocks, and +10 us at 128K, where it sums 16)
-#ifndef XB_FUSE_MIN
-#define XB_FUSE_MIN 32
-#endif
-  const bool fused = max_tiles_per_row <= 8 && per_row >= XB_FUSE_MIN;
-  if (!fused) {
-    if ((rc = launch_dependent(est_rowstat_kernel, dim3(static_cast<unsigned>((total_rows + 255) / 256)), dim3(256), 0, stream, g,
-                               (const int*)tile_lo, (const int*)tile_prefix, (const float2*)mtile, rowstat, static_cast<int>(total_rows))))
-      return rc;
-  }
-  int bt = per_row >= 256 ? 256 : ((per_row + 31) / 32) * 32;
-  if (fused && bt < 8 * g.rbs) bt = 8 * g.rbs;           // eight threads per row for the statistics (rbs <= 32)
-  const dim3 fgrid((per_row + bt - 1) / bt, g.qb_total, batch * hq);
+  const int seg_tiles = g.m_pitch < 32 * 1024 / (4 * g.rbs) ? g.m_pitch : 32 * 1024 / (4 * g.rbs);     // 32 KiB of factors at most
   auto launch_sums = [&](auto kern) -> int {
-    return launch_dependent(kern, fgrid, dim3(bt), 0, stream, g, (const int*)tile_lo, (const int*)tile_prefix, (const float*)partial,
-                            (const float2*)mtile, (const float2*)rowstat, attn_sums);
+    return launch_dependent(kern, dim3(g.qb_total, batch * hq), dim3(kSumThreads), static_cast<size_t>(seg_tiles) * g.rbs * sizeof(float),
+                            stream, g, (const int*)tile_lo, (const int*)tile_prefix, (const float*)partial, (const float2*)mtile,
+                            attn_sums, seg_tiles);
   };
-  if (vec4) return fused ? launch_sums(est_blocksum_kernel<4, true>) : launch_sums(est_blocksum_kernel<4, false>);
-  return fused ? launch_sums(est_blocksum_kernel<1, true>) : launch_sums(est_blocksum_kernel<1, false>);
+  switch (g.rbs) {
+    case 4: return launch_sums(est_blocksum_kernel<4>);
+    case 8: return launch_sums(est_blocksum_kernel<8>);
+    case 16: return launch_sums(est_blocksum_kernel<16>);
+    case 32: return launch_sums(est_blocksum_kernel<32>);
+    default: return XATTN_B200_ERR_ARG;
+  }
 }
 
 int split_f32_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
