@@ -69,6 +69,8 @@ struct EstGeom {
   FastDiv by_tiles, by_group, by_hq;     // tiles per head (of the kernel that runs), query heads per kv head, query heads
   // few tiles: the K loop of each is split over a cluster of `split` CTAs (1: persistent CTAs, a tile each at a time)
   int split;
+  // CTA pairs: the two are query heads 2p, 2p + 1 of a kv group at the same rows (otherwise neighbouring row tiles of a head)
+  int pair_heads;
   int direct;                  // the epilogue finishes the block sums: every row tile is computed, even one that sees nothing
   int tab_n;
   int tab[64 + 65 + 32 + 33];
@@ -658,6 +660,11 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // its own 128 rows in its own tensor memory, where its four epilogue warps work exactly as in the single-CTA
 // kernel.  The single-CTA kernel is bound by operand bytes in flight per SM (L2 latency x shared-memory
 // capacity); the pair moves a third fewer bytes per FLOP and has six 32 KiB stages in flight.
+// The pair's rows are the same 128 of two query heads that share a kv head, if there are such (pair_heads): both see the
+// same columns, so that a tile of which they see only the first 128 (every other one on the diagonal) is computed 128
+// columns wide (32K tokens at stride 16: a tenth of the MMAs, the estimate 147 -> 140 us at the power cap).  Otherwise they
+// are neighbouring row tiles of one head.  (128-column tiles, which stream their operands from HBM, do not gain: 205 -> 202
+// us for the estimate of 128K tokens, 960 -> 973 us for the prefill.)
 //   full[s]   (even CTA)  1 arrival (its producer's expect_tx of both CTAs' bytes) + the bytes of four TMA loads
 //   empty[s]  (each CTA)  1 arrival: the commit of the MMAs that read stage s, delivered to both CTAs
 //   tfull[a]  (each CTA)  1 arrival: the commit of a tile's last MMA, delivered to both CTAs
@@ -667,19 +674,20 @@ constexpr int kPairBBytes = 128 * kTileK * 2;                // this CTA's half 
 constexpr int kPairStageBytes = kABytes + kPairBBytes;       // 32 KiB
 constexpr int kPairSmem = kPairStages * kPairStageBytes + 1024 /*barriers*/ + 1024 /*alignment slack*/;
 
-template <int RBS, bool kDirect>
+// kDirect: see est_gemm_kernel (0 or 2)
+template <int RBS, int kDirect>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKh,
                      const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt,
-                     const EstGeom g, const int* pair_lo, const int* pair_prefix,
-                     float* __restrict__ partial, float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc,
+                     const EstGeom g, const int* group_lo, const int* group_prefix,
+                     float* __restrict__ partial, float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc_wide, const uint32_t idesc_narrow,
                      int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_tab[kTabInts];
   if (g.tab_n) {                                  // (made visible by the __syncthreads() that ends the prologue)
     load_tables(g, s_tab);
-    pair_lo = s_tab + kTabPairLo;
-    pair_prefix = s_tab + kTabPairPrefix;
+    group_lo = s_tab + (g.pair_heads ? 0 : kTabPairLo);
+    group_prefix = s_tab + (g.pair_heads ? kTabPrefix : kTabPairPrefix);
   }
   // the same offset in both CTAs of the pair (the dynamic shared memory of a kernel starts at the same address
   // in every CTA), which the MMA descriptors rely on
@@ -722,10 +730,25 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   pdl_wait();                       // up to here nothing was touched that an earlier kernel writes
   const uint32_t tmem_base = *tmem_slot;
 
-  const int n_groups = (g.n_mtiles + 1) / 2;
-  const int tiles_per_head = pair_prefix[n_groups];
-  const int total_tiles = tiles_per_head * g.batch * g.hq;
+  // row groups of a pair: row tiles of two heads, or pairs of row tiles of one
+  const int n_groups = g.pair_heads ? g.n_mtiles : (g.n_mtiles + 1) / 2;
+  const int total_tiles = group_prefix[n_groups] * (g.pair_heads ? g.batch * g.hq / 2 : g.batch * g.hq);
   const int k_steps = g.S * g.d_chunks;
+  // tile -> this CTA's (batch * head), row tile and column tile; whether the tile is 128 columns wide
+  auto decode = [&](int tile, int& bh, int& mt, int& nt) -> bool {
+    int grp;
+    decode_tile(g, n_groups, group_lo, group_prefix, tile, bh, grp, nt);
+    if (!g.pair_heads) {
+      mt = 2 * grp + static_cast<int>(rank);
+      return false;
+    }
+    bh = 2 * bh + static_cast<int>(rank);
+    mt = grp;
+    const int last = mt * kTileM + kTileM - 1 < g.rows_valid - 1 ? mt * kTileM + kTileM - 1 : g.rows_valid - 1;
+    int lo, hi;
+    row_bounds(g, last, lo, hi);
+    return hi - nt * kTileN < 128;
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (converged warp, one thread issues)
@@ -734,23 +757,25 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       int s = 0;
       uint32_t ph = 0;
       for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs_grid) {
-        int bh, pm, nt;
-        decode_tile(g, n_groups, pair_lo, pair_prefix, tile, bh, pm, nt);
-        int h, hg_;
+        int bh, mt, nt, h, hg_;
+        const bool narrow = decode(tile, bh, mt, nt);
         const int b = fast_div(bh, g.by_hq, h), hkv = fast_div(h, g.by_group, hg_);
-        const int mt = 2 * pm + static_cast<int>(rank);
+        const int col0 = nt * g.tile_n + static_cast<int>(rank) * (narrow ? 64 : 128);      // this CTA's columns of B
+        const uint32_t stage_bytes = 2 * (kABytes + (narrow ? kPairBBytes / 2 : kPairBBytes));
         int t = 0, dc = 0;
         for (int ks = 0; ks < k_steps; ++ks) {
           if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag))) break;
           const uint32_t dstA = smem_u32(smem + s * kPairStageBytes);
-          // all four loads of a stage are counted on the even CTA's barrier
+          // all loads of a stage are counted on the even CTA's barrier
           const uint32_t full_even = mapa_shared(full0 + 8 * s, 0);
-          mbar_expect_tx_lead(full0 + 8 * s, 2 * kPairStageBytes, rank == 0 ? lead : 0u);
+          mbar_expect_tx_lead(full0 + 8 * s, stage_bytes, rank == 0 ? lead : 0u);
           const bool qt = g.S - 1 - t < g.q_rem, kt = t < g.k_rem;
           const int col = k_column(g, dc);
           tma_load_5d_pair_lead(dstA, qt ? &tmQt : &tmQ, full_even, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
-          tma_load_5d_pair_lead(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, col, t,
-                           nt * kTileN + static_cast<int>(rank) * 128 + (kt ? 0 : g.k_none), hkv, b, lead);
+          const int k_col = col0 + (kt ? 0 : g.k_none);                        // (B in boxes of 64 columns)
+          tma_load_5d_pair_lead(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, col, t, k_col, hkv, b, lead);
+          tma_load_5d_pair_lead(dstA + kABytes + kPairBBytes / 2, kt ? &tmKt : &tmKh, full_even, col, t, k_col + 64, hkv, b,
+                                narrow ? 0u : lead);
           if (++dc == g.d_chunks) { dc = 0; ++t; }
           if (++s == kPairStages) { s = 0; ph ^= 1; }
         }
@@ -766,6 +791,8 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
       const uint64_t b_desc0 = smem_desc_sw128(smem_u32(smem) + kABytes, 16, 1024);
       for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs_grid, ++local_tile) {
+        int bh_, mt_, nt_;
+        const uint32_t idesc = decode(tile, bh_, mt_, nt_) ? idesc_narrow : idesc_wide;
         const uint32_t acc = local_tile & 1;
         const uint32_t acc_ph = (local_tile >> 1) & 1;
         if (!wait(tempty0 + 8 * acc, acc_ph ^ 1)) break;
@@ -814,21 +841,19 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // ------------------------------------------------------------ epilogue (4 warps, thread = tile row)
     const int quad = warp & 3;                  // TMEM lane quarter this warp may access
     const int r = quad * 32 + lane;
-    constexpr int kGroups = kTileN / RBS;       // key blocks per tile
-    constexpr int n_chunks = kTileN / 32;
+    const int kGroups = g.tile_n / RBS;         // key blocks per tile
     uint32_t local_tile = 0;
     for (int tile = pair; tile < total_tiles; tile += n_pairs_grid, ++local_tile) {
-      int bh, pm, nt;
-      decode_tile(g, n_groups, pair_lo, pair_prefix, tile, bh, pm, nt);
-      const int mt = 2 * pm + static_cast<int>(rank);
+      int bh, mt, nt;
+      const int n_chunks = decode(tile, bh, mt, nt) ? 4 : 8;
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
       const int i = mt * kTileM + r;
       int lo, hi;
       row_bounds(g, i < g.rows_total ? i : g.rows_total, lo, hi);   // rows past the end see nothing
-      const int n0 = nt * kTileN;
+      const int n0 = nt * g.tile_n;
       const int clo = lo - n0 > 0 ? lo - n0 : 0;
-      const int chi = hi - n0 < kTileN - 1 ? hi - n0 : kTileN - 1;
+      const int chi = hi - n0 < g.tile_n - 1 ? hi - n0 : g.tile_n - 1;
       // warp-uniform: the tensor-memory loads below are warp-collective
       if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, acc_ph, abort_flag))) break;
       tc_fence_after();
@@ -839,24 +864,24 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty0 + 8 * acc, 0));
       };
-      if constexpr (kDirect) {
+      if constexpr (kDirect > 0) {
         const int qb = i / RBS;
         const int out_cols = g.band ? g.bpc : g.kb_total, col0 = g.band ? 0 : nt * kGroups;
         const int nvis = (__reduce_max_sync(0xffffffffu, chi >= clo ? chi : -1) + 32) >> 5;
-        int reads = nvis > 4 ? 3 : 1;
+        int reads = kDirect == 2 && nvis > 4 ? 3 : 1;
         auto load = [&](int half, uint32_t (&v)[4][32]) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) tmem_ld32(taddr + half * 128 + c * 32, v[c]);
           tc_wait_ld();
           if (--reads == 0) release();
         };
-        est_epilogue_row_direct<RBS, 2>(g, load, nvis, clo, chi,
+        est_epilogue_row_direct<RBS, kDirect>(g, load, nvis, clo, chi,
                                         sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, col0, out_cols,
                                         qb < g.qb_total, lane);
       } else {
         // (compact scratch: both row tiles of a pair lie in one chunk and start at the pair's first column tile)
         const bool write = mt < g.n_mtiles;
-        const size_t tile_at = scratch_tile(g, bh, write ? mt : 0, nt, pair_lo[pm]) * kTileM;
+        const size_t tile_at = scratch_tile(g, bh, write ? mt : 0, nt, group_lo[g.pair_heads ? mt : mt / 2]) * kTileM;
         est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, write, partial + tile_at * kGroups + r, mtile + tile_at + r, release);
       }
     }
@@ -906,10 +931,19 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
   const float* pp = partial + tile0 * gpt * kTileM + r0;   // key block nlo * gpt + k: at k * kTileM
   // band layout: only the key blocks of the query block's own chunk, [cur, cur + bpc)
   const int cur = g.band ? (g.row_off + (i0 / g.rcs) * g.rcs) / RBS : 0, n_out = g.band ? g.bpc : g.kb_total;
+  int k_end = ncnt * gpt;                                  // blocks past the last one that any of the rows sees are zero
+  {
+    const int last = i0 + RBS - 1 < g.rows_valid - 1 ? i0 + RBS - 1 : g.rows_valid - 1;
+    int lo, hi;
+    row_bounds(g, last, lo, hi);
+    const int vis = hi / RBS + 1 - nlo * gpt;
+    if (i0 >= g.rows_valid) k_end = 0;
+    else if (vis < k_end) k_end = vis;
+  }
   float4 p4[RBS / 4];
   auto fetch = [&](int kl) {                               // the rows of output kl; zeros outside the tiles
     const int k = cur + kl - nlo * gpt;
-    const bool in = kl < n_out && k >= 0 && k < ncnt * gpt;
+    const bool in = kl < n_out && k >= 0 && k < k_end;
 #pragma unroll
     for (int j = 0; j < RBS / 4; ++j)
       p4[j] = in ? __ldcs(reinterpret_cast<const float4*>(pp + static_cast<size_t>(k) * kTileM) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -955,7 +989,7 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
     }
     __syncthreads();
     for (int kl = threadIdx.x; kl < n_out; kl += kSumThreads) {
-      const int k = cur + kl - nlo * gpt, t = k >= 0 ? k / gpt : -1;
+      const int k = cur + kl - nlo * gpt, t = k >= 0 && k < k_end ? k / gpt : -1;
       if (t >= t0 && t < t1) {
         const float4* f4 = reinterpret_cast<const float4*>(s_f + (t - t0) * RBS);
         float acc = 0.f;
@@ -965,7 +999,7 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
           acc += p4[j].x * f.x + p4[j].y * f.y + p4[j].z * f.z + p4[j].w * f.w;
         }
         out[kl] = acc;
-      } else if (t0 == 0 && (t < 0 || t >= ncnt)) {
+      } else if (t0 == 0 && t < 0) {
         out[kl] = 0.f;
       }
       if (kl + kSumThreads < n_out) fetch(kl + kSumThreads);
@@ -1071,6 +1105,7 @@ static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int h
   g.k_none = k_len < stride ? 1 : 0;
   g.direct = 0;
   g.split = 1;
+  g.pair_heads = 0;
   g.compact = g.left_blank;
   g.m_pitch = g.n_ntiles;
   if (g.compact) {
@@ -1177,6 +1212,8 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // CTA pairs (256x256 tiles) when tiles are 256 columns wide and the two row tiles of a pair see about the
   // same columns (always, except when a 128-row chunk of the torch branch blanks everything left of it)
   bool use_pairs = g.tile_n == kTileN && g.n_mtiles >= 2 && (!g.left_blank || g.rcs % (2 * kTileM) == 0);
+  g.pair_heads = g.tile_n == kTileN && (hq / hkv) % 2 == 0 ? 1 : 0;
+  if (g.pair_heads) use_pairs = true;
   // Few tiles (short prompts: 32 heads of up to 2048 tokens at stride 16 are 32 tiles for 148 SMs): the K loop of each, which is
   // a stream of operands through one SM, is split over a cluster of two or four CTAs instead.
   {
@@ -1189,6 +1226,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     const bool long_k = g.S * g.d_chunks >= 32;          // (the exchange costs about what eight steps take)
     g.split = !long_k ? 1 : (4 * tiles <= sm_count() ? 4 : (2 * tiles <= sm_count() ? 2 : 1));
     if (g.split > 1) use_pairs = false;
+    if (!use_pairs) g.pair_heads = 0;
   }
   // Every row sees a single column tile, and that tile's block sums are (nearly) a whole row of the output: chunks of exactly
   // 128 or 256 reshaped rows in the chunk-band layout (128K or 64K tokens at stride 16), or keys of at most 256 columns
@@ -1206,7 +1244,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   }
   g.direct = direct ? 1 : 0;
   CUtensorMap tmQ, tmK, tmQt, tmKt;
-  const uint32_t k_box = use_pairs ? 128 : static_cast<uint32_t>(g.tile_n);     // pairs: one CTA's half of a 256-column tile
+  const uint32_t k_box = use_pairs ? 64 : static_cast<uint32_t>(g.tile_n);
   if ((rc = make_map(&tmQ, q, q_len, hq, qsb, qsh, qsl, kTileM, false))) return rc;
   if ((rc = make_map(&tmK, k, k_len, hkv, ksb, ksh, ksl, k_box, false))) return rc;
   tmQt = tmQ;
@@ -1238,7 +1276,8 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     tiles_per_head += cnt;
     if (mt % 2 == 1 || mt == g.n_mtiles - 1) pairs_per_head += hi < 0 ? 0 : hi - lo + 1;
   }
-  g.by_tiles = make_fast_div(static_cast<uint32_t>((use_pairs ? pairs_per_head : tiles_per_head) > 0 ? (use_pairs ? pairs_per_head : tiles_per_head) : 1));
+  const int per_head = use_pairs && !g.pair_heads ? pairs_per_head : tiles_per_head;
+  g.by_tiles = make_fast_div(static_cast<uint32_t>(per_head > 0 ? per_head : 1));
   if (static_cast<long long>(tiles_per_head) * batch * hq > 0x7fffffffLL) return XATTN_B200_ERR_LIMIT;
   if (in_params) {
     g.tab[kTabPrefix + g.n_mtiles] = tiles_per_head;
@@ -1252,6 +1291,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   const int sms = sm_count();
   if (use_pairs) {
     const uint32_t idesc2 = make_idesc_f16(2 * kTileM, kTileN, dtype != XATTN_B200_F16, false, false);
+    const uint32_t idesc2n = make_idesc_f16(2 * kTileM, 128, dtype != XATTN_B200_F16, false, false);
     auto launch_pair = [&](auto kern) -> int {
       if (!allow_smem(kern, kPairSmem))
         return XATTN_B200_ERR_CUDA;
@@ -1275,13 +1315,19 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       if (max_clusters < 1) return XATTN_B200_ERR_CUDA;
       if (static_cast<unsigned>(2 * max_clusters) < cfg.gridDim.x) cfg.gridDim.x = 2 * max_clusters;
       return launch_dependent_clusters(kern, 2, cfg.gridDim, cfg.blockDim, kPairSmem, stream, tmQ, tmK, tmQt, tmKt, g,
-                                       (const int*)pair_lo, (const int*)pair_prefix, partial, mtile, attn_sums, idesc2, status);
+                                       (const int*)(g.pair_heads ? tile_lo : pair_lo), (const int*)(g.pair_heads ? tile_prefix : pair_prefix),
+                                       partial, mtile, attn_sums, idesc2, idesc2n, status);
+    };
+    auto launch_pair_rbs = [&](auto rbs) -> int {
+      constexpr int kRbs = decltype(rbs)::value;
+      if (!direct) return launch_pair(est_gemm_pair_kernel<kRbs, 0>);
+      return launch_pair(est_gemm_pair_kernel<kRbs, 2>);
     };
     switch (g.rbs) {
-      case 4: rc = direct ? launch_pair(est_gemm_pair_kernel<4, true>) : launch_pair(est_gemm_pair_kernel<4, false>); break;
-      case 8: rc = direct ? launch_pair(est_gemm_pair_kernel<8, true>) : launch_pair(est_gemm_pair_kernel<8, false>); break;
-      case 16: rc = direct ? launch_pair(est_gemm_pair_kernel<16, true>) : launch_pair(est_gemm_pair_kernel<16, false>); break;
-      case 32: rc = direct ? launch_pair(est_gemm_pair_kernel<32, true>) : launch_pair(est_gemm_pair_kernel<32, false>); break;
+      case 4: rc = launch_pair_rbs(std::integral_constant<int, 4>()); break;
+      case 8: rc = launch_pair_rbs(std::integral_constant<int, 8>()); break;
+      case 16: rc = launch_pair_rbs(std::integral_constant<int, 16>()); break;
+      case 32: rc = launch_pair_rbs(std::integral_constant<int, 32>()); break;
       default: rc = XATTN_B200_ERR_ARG;
     }
     if (rc || direct) return rc;                       // (direct: the block sums are complete)
