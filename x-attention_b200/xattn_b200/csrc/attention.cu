@@ -611,6 +611,8 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           }
           tc_wait_st();
         }
+        // (the diagonal block for its first 64 rows: no row of the warp sees keys 64-127)
+        const bool upper_hidden = lim_lo < 33 && __shfl_sync(0xffffffffu, row_last - k0, 31) < 64;
         uint32_t v[4][32];
         tmem_ld32(ts, v[0]);
         tmem_ld32(ts + 32, v[1]);
@@ -624,13 +626,25 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         chunk_max(v[3]);
         rescale();
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 2; ++c) {
           uint32_t pk[16];
           chunk_exp(v[c], pk);
           tmem_st16(ts + c * 16, pk);
-          if (c == 1) {
-            half_ready(0);
-            if (lane == 0) XB_TRACE_EV(0x34, bc);
+        }
+        half_ready(0);
+        if (lane == 0) XB_TRACE_EV(0x34, bc);
+        if (upper_hidden) {
+          uint32_t z[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) z[k] = 0u;
+          tmem_st16(ts + 32, z);
+          tmem_st16(ts + 48, z);
+        } else {
+#pragma unroll
+          for (int c = 2; c < 4; ++c) {
+            uint32_t pk[16];
+            chunk_exp(v[c], pk);
+            tmem_st16(ts + c * 16, pk);
           }
         }
         {
