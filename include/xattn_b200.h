@@ -35,7 +35,8 @@ extern "C" {
 /* element types */
 #define XATTN_B200_BF16 0
 #define XATTN_B200_F16 1
-#define XATTN_B200_F32_TERMS 2   /* xattn_b200_estimate: rows of 3 * head_dim bf16 terms of fp32 values (xattn_b200_split_f32) */
+#define XATTN_B200_F32_TERMS 2    /* xattn_b200_estimate: rows of 3 * head_dim bf16 terms of fp32 values (xattn_b200_split_f32) */
+#define XATTN_B200_F32 4          /* xattn_b200_estimate */
 #define XATTN_B200_BF16_OUT_F32 3   /* xattn_b200_block_sparse_attn[_ws]: bf16 inputs, fp32 output */
 
 /* estimate semantics: which of the reference's two code paths to reproduce */
@@ -97,8 +98,11 @@ size_t xattn_b200_estimate_workspace_bytes_ex(int batch, int hq, int q_len, int 
  *
  * q_len / k_len need not be multiples of `stride`: the tokens a ragged last stride group lacks count as the
  * zeros the reference pads with (xattn/src/Xattention.py:42-51); no copy is made for them.  head_dim is a
- * multiple of 64 (XATTN_B200_F32_TERMS: a row holds three times as many elements, and q_len and k_len are multiples of
- * the stride);  `scale` = 1/(sqrt(D)*stride*norm).
+ * multiple of 64;  `scale` = 1/(sqrt(D)*stride*norm).
+ * XATTN_B200_F32: every value is split on the way into three bf16 terms, x = hi + mid + lo to 2^-24, and the six products of
+ * terms that reach 2^-24 are added (the reference's torch branch multiplies fp32 directly, xattn/src/Xattention.py:183).
+ * XATTN_B200_F32_TERMS: the same from rows split before; only where xattn_b200_estimate_f32_terms says that this is the faster
+ * way, q_len and k_len multiples of the stride.
  * attn_sums: float32 [batch, hq, q_blocks_pad, k_blocks_pad] (fully written).
  */
 int xattn_b200_estimate(const void* q, const void* k, int dtype, int batch, int hq, int hkv, int q_len, int k_len,
@@ -106,6 +110,30 @@ int xattn_b200_estimate(const void* q, const void* k, int dtype, int batch, int 
                         int64_t k_stride_h, int64_t k_stride_l, int stride, int block_size, int chunk_size,
                         float scale, int causal, int semantics, float* attn_sums, void* workspace,
                         size_t workspace_bytes, int* status, void* cuda_stream);
+
+/*
+ * The estimate of fp32 q and k, with q and k rounded to bf16 (what the attention phase of fp32 inputs computes with) written on
+ * the way: contiguous [batch, heads, len, head_dim], 16-byte aligned, both or neither (NULL).
+ */
+int xattn_b200_estimate_f32(const float* q, const float* k, int batch, int hq, int hkv, int q_len, int k_len, int head_dim,
+                            int64_t q_stride_b, int64_t q_stride_h, int64_t q_stride_l, int64_t k_stride_b, int64_t k_stride_h,
+                            int64_t k_stride_l, int stride, int block_size, int chunk_size, float scale, int causal,
+                            int semantics, float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16,
+                            int* status, void* cuda_stream);
+
+/* 1: the estimate of fp32 q and k of that shape is faster from rows split into terms first (many tiles use each value). */
+int xattn_b200_estimate_f32_terms(int hq, int hkv, int q_len, int k_len, int stride, int block_size, int chunk_size, int causal,
+                                  int semantics);
+
+/*
+ * Split fp32 rows into three bf16 terms, x = hi + mid + lo to 2^-24, stored as rows [hi | mid | lo] of 3*head_dim
+ * (terms 3), or hi alone (terms 1: the values rounded to bf16).
+ * x is [batch, heads, len_valid, head_dim] fp32 with element strides, head_dim a multiple of 8; out is contiguous
+ * [batch, heads, len, terms*head_dim] bf16 with len >= len_valid, 16-byte aligned, the rows past len_valid zero (the
+ * reference's zero padding, xattn/src/Xattention.py:42-51).
+ */
+int xattn_b200_split_f32(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t stride_b,
+                         int64_t stride_h, int64_t stride_l, int terms, void* out, void* cuda_stream);
 
 /*
  * The estimate without a caller-supplied workspace.  No counterpart in the reference.
@@ -135,18 +163,6 @@ int xattn_b200_estimate_static(const void* q, const void* k, int dtype, int batc
                                int64_t k_stride_b, int64_t k_stride_h, int64_t k_stride_l, int stride,
                                int block_size, int chunk_size, float scale, int causal, int semantics,
                                float* attn_sums, int* status, void* cuda_stream);
-
-/*
- * Split fp32 rows into three bf16 terms, x = hi + mid + lo to 2^-24, stored as rows [hi | mid | lo] of 3*head_dim
- * (terms 3: what xattn_b200_estimate takes as XATTN_B200_F32_TERMS, its GEMM then adds the six products of terms that
- * reach 2^-24), or hi alone (terms 1: the values rounded to bf16).
- * x is [batch, heads, len_valid, head_dim] fp32 with element strides, head_dim a multiple of 8; out is contiguous
- * [batch, heads, len, terms*head_dim] bf16 with len >= len_valid, 16-byte aligned, the rows past len_valid zero (the
- * reference's zero padding, xattn/src/Xattention.py:42-51).  No counterpart in the reference (its torch branch multiplies
- * fp32 directly, xattn/src/Xattention.py:183).
- */
-int xattn_b200_split_f32(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t stride_b,
-                         int64_t stride_h, int64_t stride_l, int terms, void* out, void* cuda_stream);
 
 /*
  * Rotary position embedding, applied in place to the query and key projections in one launch.

@@ -43,11 +43,34 @@ def test_query_shorter_than_the_keys(lq, lk, chunk, semantics):
     _check(4, 2, lq, lk, 16, chunk, True, torch.float16, semantics)
 
 
+@pytest.mark.parametrize("hkv", [3, 1])
 @pytest.mark.parametrize("L,stride,chunk,causal", [(300, 16, 2048, True), (2048, 16, 2048, True), (2500, 8, 2048, False), (1900, 8, 2048, True),
-                                                   (4096, 8, 4096, True), (5000, 16, 4096, True)])
-def test_split_fp32_terms(L, stride, chunk, causal):
-    """fp32 inputs as three bf16 terms: through the single-CTA kernel with 128- and 256-column tiles and the CTA pairs."""
-    _check(3, 3, L, L, stride, chunk, causal, torch.float32)
+                                                   (4096, 8, 4096, True), (5000, 16, 4096, True), (9001, 8, 16384, True), (8192, 4, 8192, True)])
+def test_split_fp32_terms(L, stride, chunk, causal, hkv):
+    """fp32 inputs as three bf16 terms: split as the tiles are loaded (128- and 256-column tiles, one per row and several) and,
+    for the longest, before."""
+    _check(3, hkv, L, L, stride, chunk, causal, torch.float32)
+
+
+@pytest.mark.parametrize("lq,lk,stride,chunk,causal,semantics", [
+    (1003, 1003, 16, 2048, True, 0), (4096, 4096, 16, 2048, True, 2), (3000, 3000, 8, 4096, True, 1), (2000, 2500, 8, 2048, False, 0),
+    (2048, 6144, 16, 2048, True, 2), (3, 5, 16, 2048, True, 0)])       # the last but one: keys that no tile reads
+def test_bf16_roundings_of_fp32_operands(lq, lk, stride, chunk, causal, semantics):
+    """The roundings written along with the estimate are those of every token, bit by bit."""
+    from xattn_b200 import _lib, ops
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k = (torch.randn(2, h, n, 128, device="cuda", generator=g) for h, n in ((4, lq), (2, lk)))
+    q16, k16 = (torch.full(x.shape, float("nan"), device="cuda", dtype=torch.bfloat16) for x in (q, k))
+    gm = ops.geometry(lq, lk, chunk, stride)
+    sums = torch.empty(2, 4, gm["qb"], gm["bpc"] if semantics == 2 else gm["kb"], device="cuda")
+    ws = torch.empty(lib.xattn_b200_estimate_workspace_bytes(2, 4, lq, lk, stride, 128, chunk), dtype=torch.uint8, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.check(lib.xattn_b200_estimate_f32(q.data_ptr(), k.data_ptr(), 2, 4, 2, lq, lk, 128, *q.stride()[:3], *k.stride()[:3], stride, 128,
+                                           chunk, 0.01, int(causal), semantics, sums.data_ptr(), ws.data_ptr(), ws.numel(), q16.data_ptr(),
+                                           k16.data_ptr(), status.data_ptr(), torch.cuda.current_stream().cuda_stream), "estimate_f32")
+    assert int(status) == 0 and bool(torch.isfinite(sums).all())
+    assert torch.equal(q16, q.to(torch.bfloat16)) and torch.equal(k16, k.to(torch.bfloat16))
 
 
 @pytest.mark.parametrize("lq,lk,stride,chunk", [(2304, 2304, 8, 256), (1152, 1664, 4, 128), (5120, 5120, 16, 2560), (768, 3840, 4, 768), (1280, 1280, 32, 640)])

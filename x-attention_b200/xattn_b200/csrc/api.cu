@@ -7,9 +7,10 @@ size_t estimate_workspace_bytes(int batch, int hq, int q_len, int k_len, int str
 int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, int hkv, int q_len, int k_len,
                     int head_dim, int64_t qsb, int64_t qsh, int64_t qsl, int64_t ksb, int64_t ksh, int64_t ksl,
                     int stride, int block_size, int chunk_size, float scale, int causal, int semantics,
-                    float* attn_sums, void* workspace, size_t workspace_bytes, int* status, cudaStream_t stream);
+                    float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16, int* status, cudaStream_t stream);
 int split_f32_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
                      int64_t sl, int terms, void* out, cudaStream_t stream);
+int estimate_f32_terms(int hq, int hkv, int q_len, int k_len, int stride, int block_size, int chunk_size, int causal, int semantics);
 int rope_qk_launch(void* q, void* k, int dtype, int batch, int hq, int hkv, int len, int head_dim, int64_t qsb,
                    int64_t qsh, int64_t qsl, int64_t ksb, int64_t ksh, int64_t ksl, const void* cos, const void* sin,
                    int64_t cs_stride_b, int64_t cs_stride_l, cudaStream_t stream);
@@ -93,8 +94,23 @@ int xattn_b200_estimate(const void* q, const void* k, int dtype, int batch, int 
                         size_t workspace_bytes, int* status, void* cuda_stream) {
   return xb::estimate_launch(q, k, dtype, batch, hq, hkv, q_len, k_len, head_dim, q_stride_b, q_stride_h, q_stride_l,
                              k_stride_b, k_stride_h, k_stride_l, stride, block_size, chunk_size, scale, causal,
-                             semantics, attn_sums, workspace, workspace_bytes, status,
+                             semantics, attn_sums, workspace, workspace_bytes, nullptr, nullptr, status,
                              static_cast<cudaStream_t>(cuda_stream));
+}
+
+int xattn_b200_estimate_f32(const float* q, const float* k, int batch, int hq, int hkv, int q_len, int k_len, int head_dim,
+                            int64_t q_stride_b, int64_t q_stride_h, int64_t q_stride_l, int64_t k_stride_b, int64_t k_stride_h,
+                            int64_t k_stride_l, int stride, int block_size, int chunk_size, float scale, int causal,
+                            int semantics, float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16,
+                            int* status, void* cuda_stream) {
+  return xb::estimate_launch(q, k, XATTN_B200_F32, batch, hq, hkv, q_len, k_len, head_dim, q_stride_b, q_stride_h, q_stride_l,
+                             k_stride_b, k_stride_h, k_stride_l, stride, block_size, chunk_size, scale, causal, semantics,
+                             attn_sums, workspace, workspace_bytes, q_bf16, k_bf16, status, static_cast<cudaStream_t>(cuda_stream));
+}
+
+int xattn_b200_estimate_f32_terms(int hq, int hkv, int q_len, int k_len, int stride, int block_size, int chunk_size, int causal,
+                                  int semantics) {
+  return xb::estimate_f32_terms(hq, hkv, q_len, k_len, stride, block_size, chunk_size, causal ? 1 : 0, semantics);
 }
 
 int xattn_b200_split_f32(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t stride_b,

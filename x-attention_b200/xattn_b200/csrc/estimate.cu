@@ -37,10 +37,26 @@ constexpr int kStageBytes = kABytes + kBBytes;               // 48 KiB
 constexpr int kGemmThreads = 192;                            // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
 constexpr int kGemmSmem = kStages * kStageBytes + 1024 /*barriers*/ + 1024 /*alignment slack*/;
 
+// fp32 operands: units of 128 rows x 32 columns go through a ring, four warps split them into three bf16 terms that are kept
+// the way a stage of 16-bit operands is, for 64 columns (half of them worked on by the MMAs, half written)
+constexpr int kF32Cols = 32;
+constexpr int kF32Unit = kTileM * kF32Cols * 4;              // 16 KiB
+constexpr int kF32Smem = 224 * 1024;                         // terms and ring: 3 x 32 KiB and 8 units, or 3 x 48 KiB and 5
+constexpr int kMaxUnits = 8;
+// Warps that split the units, every warp some rows of each: sixteen, or eight where the epilogue needs the registers.
+__host__ __device__ constexpr int convert_warps(int direct) { return direct ? 8 : 16; }
+__host__ __device__ constexpr int f32_threads(int direct) { return kGemmThreads + 32 * convert_warps(direct); }
+
+// bf16 roundings of fp32 operands, [batch, heads, len, head_dim] contiguous, written on the way (null: not wanted)
+struct EstRounded {
+  uint4 *q, *k;
+  int q_len, k_len;
+};
+
 struct EstGeom {
   int batch, hq, hkv;
-  int S, d_chunks;             // K loop: S * d_chunks steps of 64 elements
-  int term_chunks;             // split fp32 rows: 64-column chunks per term (0: plain rows); see k_column
+  int S, d_chunks;             // K loop: S * d_chunks steps of 64 elements (fp32: of 32)
+  int term_chunks;             // rows of bf16 terms of fp32 values: 64-column chunks per term (0: plain rows); see k_column
   int rows_total, cols_total;  // padded lengths / S
   int rows_valid, cols_valid;  // rows past rows_valid give zeros; causal: columns past cols_valid are hidden
   int rcs;                     // chunk_size / S
@@ -93,8 +109,8 @@ __host__ __device__ inline void row_bounds(const EstGeom& g, int i, int& lo, int
   if (hi > g.cols_valid - 1) hi = g.cols_valid - 1;
 }
 
-// Columns of both operands of step dc of a token.  Plain rows: one 64-column chunk after the other.  fp32 rows split into
-// three bf16 terms [hi | mid | lo]: of one chunk after the other the three terms, three stages the MMA issuer treats as one.
+// Columns of both operands of step dc of a token.  Plain rows: one 64-column chunk after the other.  Rows of three bf16 terms
+// [hi | mid | lo]: of one chunk after the other the three terms, three stages the MMA issuer treats as one.
 __device__ __forceinline__ int k_column(const EstGeom& g, int dc) {
   if (g.term_chunks == 0) return dc * kTileK;
   const int c = dc / 3, term = dc - 3 * c;
@@ -381,13 +397,35 @@ __device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, Load l
   for (int c = base / kLeft; c < outside; c += kWriters) out[c < col0 ? c : c + kBlocks] = 0.f;
 }
 
+// Eight fp32 values, in pairs: the next term of each, the rounding of what the terms before leave.
+__device__ __forceinline__ uint4 next_term(unsigned long long (&v)[4]) {
+  uint32_t w[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float x, y;
+    unpack_f32x2(v[k], x, y);
+    const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+    w[k] = *reinterpret_cast<const uint32_t*>(&p);
+    v[k] = fma_f32x2(pack_f32x2(__low2float(p), __high2float(p)), pack_f32x2(-1.f, -1.f), v[k]);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // kDirect: 128-column halves per row of the epilogue above, 0: the general one
-template <int RBS, int kDirect>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+// kF32: fp32 operands.  x = hi + mid + lo in bf16 (each the rounding of what the ones before it leave), and the six products
+// of terms that reach 2^-24 of the first: hh; hm, mh, mm; hl, lh.  The split happens here, between the loads and the MMAs:
+// more warps take the fp32 units from shared memory and write the terms to shared memory, half of a 64-column stage while the
+// MMAs read the other.  Terms written to HBM first cost 10 bytes per element, and the GEMM then found HBM busy with writing
+// them back (32 heads of 4096 tokens, chunks of 2048: split 56 us + GEMM 46 -> 44; the prefill, whose attention phase takes the
+// bf16 roundings written here, 151 -> 107 us).  Bound by the latency of a converter's step (waits, shared-memory traffic
+// next to the MMAs', three dependent roundings); with loads alone it runs in 30 us.  Eight converter warps took 5 to 10 % less
+// than four.
+template <int RBS, int kDirect, bool kF32>
+__global__ void __launch_bounds__(kF32 ? f32_threads(kDirect) : kGemmThreads, 1)
 est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt, const EstGeom g,
                 const int* tile_lo, const int* tile_prefix, float* __restrict__ partial,
-                float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc, int* status) {
+                float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc, const EstRounded rounded, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_tab[kTabInts];
   if (g.tab_n) {                                  // (made visible by the __syncthreads() that ends the prologue)
@@ -398,28 +436,33 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // 128-column tiles (every operand tile is used once: the kernel streams Q and K from HBM) take six 32 KiB
   // stages, 256-column tiles four 48 KiB ones: 192 KiB in flight either way
-  // (split fp32 rows use them in threes)
-  const int n_stages = g.tile_n == 128 ? kMaxStages : (g.term_chunks ? 3 : kStages);
+  // (fp32: three stages' space for the terms, the rest the ring of units)
   const int stage_bytes = kABytes + g.tile_n * kTileK * 2;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
-  const uint32_t full0 = smem_u32(bars);                       // [kMaxStages]
-  const uint32_t empty0 = smem_u32(bars + kMaxStages);         // [kMaxStages]
-  const uint32_t tfull0 = smem_u32(bars + 2 * kMaxStages);     // [2]
-  const uint32_t tempty0 = smem_u32(bars + 2 * kMaxStages + 2);// [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
+  const int n_stages = kF32 ? (kF32Smem - 3 * stage_bytes) / kF32Unit : (g.tile_n == 128 ? kMaxStages : kStages);
+  constexpr int kBars = kF32 ? kMaxUnits : kMaxStages;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (kF32 ? kF32Smem : kStages * kStageBytes));
+  const uint32_t full0 = smem_u32(bars);                       // [kBars]
+  const uint32_t empty0 = smem_u32(bars + kBars);              // [kBars]
+  const uint32_t tfull0 = smem_u32(bars + 2 * kBars);          // [2]
+  const uint32_t tempty0 = smem_u32(bars + 2 * kBars + 2);     // [2]
+  const uint32_t terms_full0 = smem_u32(bars + 2 * kBars + 4); // [2] (fp32) terms of 32 columns written / read
+  const uint32_t terms_empty0 = smem_u32(bars + 2 * kBars + 6);// [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kBars + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);     // (uniform for the compiler too)
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kMaxStages; ++s) {
+    for (int s = 0; s < kBars; ++s) {
       mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, kF32 ? convert_warps(kDirect) : 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull0 + 8 * a, 1);
       mbar_init(tempty0 + 8 * a, 4);
+      mbar_init(terms_full0 + 8 * a, convert_warps(kDirect));
+      mbar_init(terms_empty0 + 8 * a, 1);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -439,11 +482,10 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   const int tiles_per_head = tile_prefix[g.n_mtiles];
   const int total_tiles = tiles_per_head * g.batch * g.hq;
-  // this CTA's tiles and its part of their K loop (split fp32 rows: whole triples of terms)
+  // this CTA's tiles and its part of their K loop
   const int split = g.split, rank = split > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   const int tile0 = blockIdx.x / split, tile_step = gridDim.x / split;
-  const int k_unit = g.term_chunks ? 3 : 1, k_units = g.S * g.d_chunks / k_unit;
-  const int ks0 = k_units * rank / split * k_unit, ks1 = k_units * (rank + 1) / split * k_unit;
+  const int k_steps = g.S * g.d_chunks, ks0 = k_steps * rank / split, ks1 = k_steps * (rank + 1) / split;
   const bool interleave = g.tile_n == 128 && g.hq > g.hkv;      // streaming case only: see decode_tile
 
   if (warp == 0) {
@@ -459,15 +501,30 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int b = fast_div(bh, g.by_hq, h), hkv = fast_div(h, g.by_group, hg_);
         int t = ks0 / g.d_chunks, dc = ks0 - t * g.d_chunks;
         for (int ks = ks0; ks < ks1; ++ks) {
-          if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag))) break;
-          const uint32_t dstA = smem_u32(smem + s * stage_bytes);
-          mbar_expect_tx_lead(full0 + 8 * s, stage_bytes, lead);
           const bool qt = g.S - 1 - t < g.q_rem, kt = t < g.k_rem;
-          const int col = k_column(g, dc);
-          tma_load_5d_lead(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
-          tma_load_5d_lead(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, col, t, nt * g.tile_n + (kt ? 0 : g.k_none), hkv, b, lead);
+          if constexpr (kF32) {
+            bool ok = true;
+            for (int n = -kTileM; n < g.tile_n && ok; n += kTileM) {         // A, then 128 rows of B at a time
+              ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag));
+              if (!ok) break;
+              const uint32_t dst = smem_u32(smem + 3 * stage_bytes + s * kF32Unit);
+              mbar_expect_tx_lead(full0 + 8 * s, kF32Unit, lead);
+              if (n < 0)
+                tma_load_5d_lead(dst, qt ? &tmQt : &tmQ, full0 + 8 * s, dc * kF32Cols, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
+              else
+                tma_load_5d_lead(dst, kt ? &tmKt : &tmK, full0 + 8 * s, dc * kF32Cols, t, nt * g.tile_n + n + (kt ? 0 : g.k_none), hkv, b, lead);
+              if (++s == n_stages) { s = 0; ph ^= 1; }
+            }
+            if (!ok) break;
+          } else {
+            if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag))) break;
+            const uint32_t dstA = smem_u32(smem + s * stage_bytes);
+            mbar_expect_tx_lead(full0 + 8 * s, stage_bytes, lead);
+            tma_load_5d_lead(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, dc * kTileK, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
+            tma_load_5d_lead(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, dc * kTileK, t, nt * g.tile_n + (kt ? 0 : g.k_none), hkv, b, lead);
+            if (++s == n_stages) { s = 0; ph ^= 1; }
+          }
           if (++dc == g.d_chunks) { dc = 0; ++t; }
-          if (++s == n_stages) { s = 0; ph ^= 1; }
         }
       }
     }
@@ -491,42 +548,104 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kTileN;
         bool ok = true;
-        int term = g.term_chunks ? 0 : -1;
         for (int ks = ks0; ks < ks1; ++ks) {
-          if (!wait(full0 + 8 * st, ph)) { ok = false; break; }
+          if (!wait(kF32 ? terms_full0 + 8 * st : full0 + 8 * st, ph)) { ok = false; break; }
           tc_fence_after();
-          // D += A of stage sa * B of stage sb; descriptors differ from the stage-0 ones only in the start-address field
-          // (units of 16 bytes)
-          auto product = [&](int sa, int sb, uint32_t accumulate) {
-            const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(sa * (stage_bytes >> 4));
-            const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(sb * (stage_bytes >> 4));
+          // D += A of stage sa * B of stage sb, 16-column steps [k0, k1); descriptors differ from the stage-0 ones only in the
+          // start-address field (units of 16 bytes)
+          auto product = [&](int sa, int sb, int k0, int n, uint32_t accumulate) {
+            const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(sa * (stage_bytes >> 4) + 2 * k0);
+            const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(sb * (stage_bytes >> 4) + 2 * k0);
 #pragma unroll
-            for (int k4 = 0; k4 < kTileK / 16; ++k4)
-              mma_ss_lead(d_tmem, a_desc + k4 * 2, b_desc + k4 * 2, idesc, k4 > 0 ? 1u : accumulate, lead);
+            for (int k = 0; k < n; ++k) mma_ss_lead(d_tmem, a_desc + k * 2, b_desc + k * 2, idesc, k > 0 ? 1u : accumulate, lead);
           };
-          if (term < 0) {
-            product(st, st, ks > ks0 ? 1u : 0u);
-            mma_commit_lead(empty0 + 8 * st, lead);       // stage reusable once these MMAs have read it
+          if constexpr (kF32) {
+            const int k0 = st * (kF32Cols / 16);
+            product(0, 0, k0, kF32Cols / 16, ks > ks0 ? 1u : 0u);
+            product(0, 1, k0, kF32Cols / 16, 1u);
+            product(1, 0, k0, kF32Cols / 16, 1u);
+            product(1, 1, k0, kF32Cols / 16, 1u);
+            product(0, 2, k0, kF32Cols / 16, 1u);
+            product(2, 0, k0, kF32Cols / 16, 1u);
+            mma_commit_lead(terms_empty0 + 8 * st, lead);
+            if (++st == 2) { st = 0; ph ^= 1; }
           } else {
-            // three stages hold the terms [hi, mid, lo] of one chunk: the products hh; hm, mh, mm; hl, lh (the three left out
-            // are below 2^-24 of the first).  Each term is loaded once for the products it enters.
-            if (term == 0) {
-              product(st, st, ks > ks0 ? 1u : 0u);
-            } else if (term == 1) {
-              product(st - 1, st, 1u);
-              product(st, st - 1, 1u);
-              product(st, st, 1u);
-            } else {
-              product(st - 2, st, 1u);
-              product(st, st - 2, 1u);
-              for (int k = 2; k >= 0; --k) mma_commit_lead(empty0 + 8 * (st - k), lead);
-            }
-            term = term == 2 ? 0 : term + 1;
+            product(st, st, 0, kTileK / 16, ks > ks0 ? 1u : 0u);
+            mma_commit_lead(empty0 + 8 * st, lead);       // stage reusable once these MMAs have read it
+            if (++st == n_stages) { st = 0; ph ^= 1; }
           }
-          if (++st == n_stages) { st = 0; ph ^= 1; }
         }
         if (!ok) break;
         mma_commit_lead(tfull0 + 8 * acc, lead);          // accumulator complete
+      }
+    }
+    if (split > 1) {
+      cluster_sync_all();
+      cluster_sync_all();
+    }
+  } else if (kF32 && warp >= kGemmThreads / 32) {
+    // ------------------------------------------------------------ converters (fp32): some rows of each unit per warp
+    // A lane takes eight columns (two 16-byte chunks) of one row of each group of eight.  Rows p and p ^ 5 next to one another:
+    // neither the fp32 reads (chunks 2 col, 2 col + 1 of a swizzled row) nor the term writes (chunk col of a half) of a
+    // quarter-warp then share a bank.
+    constexpr int kGroups = kTileM / 8 / convert_warps(kDirect);
+    const int col = lane & 3, r7 = (lane >> 3) ^ ((lane >> 2 & 1) * 5), row0 = (warp - kGemmThreads / 32) * 8 * kGroups + r7;
+    const uint32_t src0 = smem_u32(smem) + 3 * stage_bytes + row0 * 128, ch0 = ((2 * col) ^ r7) * 16, ch1 = ((2 * col + 1) ^ r7) * 16;
+    const int row_vecs = g.head_dim / 8;
+    int s = 0, half = 0;
+    uint32_t ph = 0, half_ph = 0;
+    bool ok = true;
+    auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)); };
+    for (int tile = tile0; tile < total_tiles && ok; tile += tile_step) {
+      int bh, mt, nt, h, hg;
+      decode_tile(g, g.n_mtiles, tile_lo, tile_prefix, tile, bh, mt, nt, interleave);
+      const int b = fast_div(bh, g.by_hq, h), hkv = fast_div(h, g.by_group, hg);
+      // the roundings are written by the first tile of a row tile, and by the first one that has the column tile
+      uint4* q_out = nt == tile_lo[mt] ? rounded.q : nullptr;
+      uint4* k_out = hg == 0 && (mt == 0 || nt >= tile_lo[mt - 1] + tile_prefix[mt] - tile_prefix[mt - 1]) ? rounded.k : nullptr;
+      if (q_out) q_out += static_cast<size_t>(bh) * rounded.q_len * row_vecs + col;
+      if (k_out) k_out += static_cast<size_t>(b * g.hkv + hkv) * rounded.k_len * row_vecs + col;
+      int t = ks0 / g.d_chunks, dc = ks0 - t * g.d_chunks;
+#pragma unroll 1
+      for (int ks = ks0; ks < ks1 && ok; ++ks) {
+        if (!wait(terms_empty0 + 8 * half, half_ph ^ 1)) { ok = false; break; }
+#pragma unroll 1
+        for (int n = -kTileM; n < g.tile_n; n += kTileM) {                   // A, then 128 rows of B at a time
+          if (!wait(full0 + 8 * s, ph)) { ok = false; break; }
+          unsigned long long v[kGroups][4];
+#pragma unroll
+          for (int i = 0; i < kGroups; ++i) {
+            const uint32_t src = src0 + s * kF32Unit + i * 8 * 128;
+            ld_shared_2b64(src + ch0, v[i][0], v[i][1]);
+            ld_shared_2b64(src + ch1, v[i][2], v[i][3]);
+          }
+          uint4 term[3][kGroups];                        // (all groups term by term: their chains of conversions overlap)
+#pragma unroll
+          for (int e = 0; e < 3; ++e)
+#pragma unroll
+            for (int i = 0; i < kGroups; ++i) term[e][i] = next_term(v[i]);
+          const uint32_t dst = smem_u32(smem) + (n < 0 ? 0 : kABytes + n * 128) + row0 * 128 + (((4 * half + col) ^ r7) * 16);
+          uint4* out = n < 0 ? q_out : k_out;
+          const int out_len = out ? (n < 0 ? rounded.q_len : rounded.k_len) : 0;
+          const int token = ((n < 0 ? mt * kTileM : nt * g.tile_n + n) + row0) * g.S + (n < 0 ? g.S - 1 - t : t);
+#pragma unroll
+          for (int i = 0; i < kGroups; ++i) {
+#pragma unroll
+            for (int e = 0; e < 3; ++e) st_shared_v4(dst + i * 8 * 128 + e * stage_bytes, term[e][i]);
+            if (token + i * 8 * g.S < out_len) out[static_cast<size_t>(token + i * 8 * g.S) * row_vecs + dc * 4] = term[0][i];
+          }
+          // The unit goes back after the stores of its terms, which need what was read: an arrival right behind the reads has been
+          // seen to overtake a part of one (the MMAs take shared memory first), and the next unit to land in between.
+          __syncwarp();
+          if (lane == 0) mbar_arrive(empty0 + 8 * s);
+          if (++s == n_stages) { s = 0; ph ^= 1; }
+        }
+        if (!ok) break;
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(terms_full0 + 8 * half);
+        if (++half == 2) { half = 0; half_ph ^= 1; }
+        if (++dc == g.d_chunks) { dc = 0; ++t; }
       }
     }
     if (split > 1) {
@@ -816,8 +935,7 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             product(st, st, ks > 0 ? 1u : 0u);
             mma_commit_pair_lead(empty0 + 8 * st, 3, lead);       // stage reusable once these MMAs have read it
           } else {
-            // three stages hold the terms [hi, mid, lo] of one chunk: the products hh; hm, mh, mm; hl, lh (the three left out
-            // are below 2^-24 of the first).  Each term is loaded once for the products it enters.
+            // three stages hold the terms of one chunk: the products of est_gemm_kernel's fp32 form, each as its terms arrive
             if (term == 0) {
               product(st, st, ks > 0 ? 1u : 0u);
             } else if (term == 1) {
@@ -1007,11 +1125,9 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
   }
 }
 
-// x = hi + mid + lo in bf16 (each the rounding of what the ones before it leave), stored as rows [hi | mid | lo] of
-// 3 * D, or hi alone (terms == 1: the plain rounding to bf16).  Rows l >= len_valid are written as zeros (a length
-// rounded up to the stride).  Eight elements per thread: two 16-byte loads, a 16-byte store per term.  HBM-bound: 4 bytes
-// read and 6 written per element; the GEMM picks the term of each K step by a tensor-map coordinate, where rows widened to
-// the six products' operands took 12 bytes per element (32 x 4096 x 128 q and k together: 198 -> 53 us).
+// fp32 values as rows [hi | mid | lo] of 3 * D bf16 terms, or rounded to bf16 (kTerms == 1).  Rows l >= len_valid are written
+// as zeros (a length rounded up to the stride).  Eight elements per thread: two 16-byte loads, a 16-byte store per term.
+// HBM-bound: 4 bytes read and 2 or 6 written per element.
 template <int kTerms>
 __global__ void __launch_bounds__(256)
 split_f32_kernel(const float* __restrict__ x, int heads, int len, int len_valid, int vecs, int64_t sb, int64_t sh, int64_t sl,
@@ -1026,33 +1142,20 @@ split_f32_kernel(const float* __restrict__ x, int heads, int len, int len_valid,
     rest /= len;
     const int h = static_cast<int>(rest % heads);
     const int b = static_cast<int>(rest / heads);
-    float v[8];
+    unsigned long long v[4] = {};
     if (l < len_valid) {
       const float* row = x + b * sb + h * sh + l * sl + d * 8;
-      if (((reinterpret_cast<uintptr_t>(row) & 15) == 0)) {
+      if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
         const float4 a = __ldcs(reinterpret_cast<const float4*>(row)), c = __ldcs(reinterpret_cast<const float4*>(row) + 1);
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+        v[0] = pack_f32x2(a.x, a.y); v[1] = pack_f32x2(a.z, a.w); v[2] = pack_f32x2(c.x, c.y); v[3] = pack_f32x2(c.z, c.w);
       } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = row[k];
+        for (int k = 0; k < 4; ++k) v[k] = pack_f32x2(row[2 * k], row[2 * k + 1]);
       }
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = 0.f;
     }
     uint4* o = out + (e / vecs) * (static_cast<size_t>(kTerms) * vecs) + d;
 #pragma unroll
-    for (int t = 0; t < kTerms; ++t) {
-      uint32_t w[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const __nv_bfloat162 p = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-        w[k] = *reinterpret_cast<const uint32_t*>(&p);
-        v[2 * k] -= __low2float(p);
-        v[2 * k + 1] -= __high2float(p);
-      }
-      o[static_cast<size_t>(t) * vecs] = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    for (int t = 0; t < kTerms; ++t) o[static_cast<size_t>(t) * vecs] = next_term(v);
   }
 }
 
@@ -1157,12 +1260,40 @@ size_t estimate_workspace_bytes(int batch, int hq, int q_len, int k_len, int str
   return need;
 }
 
+int split_f32_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
+                     int64_t sl, int terms, void* out, cudaStream_t stream);
+
+// CTA pairs (256x256 tiles) when tiles are 256 columns wide and the two row tiles of a pair see about the
+// same columns (always, except when a 128-row chunk of the torch branch blanks everything left of it)
+static bool pairs_fit(const EstGeom& g) { return g.tile_n == kTileN && g.n_mtiles >= 2 && (!g.left_blank || g.rcs % (2 * kTileM) == 0); }
+
+// Whether the estimate of fp32 inputs is better done from rows of bf16 terms, written once, than by splitting the values as each
+// tile is loaded.  The terms cost a pass over HBM of 10 bytes per element, and the GEMM of a tile then takes half the time (CTA
+// pairs; the split is bound by shared memory and the latency of its steps): with T tiles of 128 x 256 per head that half is about
+// T * stride * 0.026 us, the pass 0.00023 us per token and head.  Measured (32 heads; estimate alone; terms, split in the GEMM):
+// 4096 tokens at stride 16 134, 81 us; 8192 at 16 288, 243; 8192 at 8 334, 317, with 8 kv heads 274, 317.
+int estimate_f32_terms(int hq, int hkv, int q_len, int k_len, int stride, int block_size, int chunk_size, int causal, int semantics) {
+  EstGeom g;
+  if (fill_geometry(1, hq, hkv, q_len, k_len, 128, stride, block_size, chunk_size, 1.f, causal, semantics, g) || !pairs_fit(g)) return 0;
+  long long tiles = 0;
+  for (int mt = 0; mt < g.n_mtiles; ++mt) {
+    int first, count;
+    row_tile_range(g, mt, first, count);
+    tiles += count;
+  }
+  return tiles * stride * 105 > q_len + static_cast<long long>(k_len) * hkv / hq;
+}
+
 int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, int hkv, int q_len, int k_len,
                     int head_dim, int64_t qsb, int64_t qsh, int64_t qsl, int64_t ksb, int64_t ksh, int64_t ksl,
                     int stride, int block_size, int chunk_size, float scale, int causal, int semantics,
-                    float* attn_sums, void* workspace, size_t workspace_bytes, int* status, cudaStream_t stream) {
+                    float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16, int* status,
+                    cudaStream_t stream) {
+  const bool f32 = dtype == XATTN_B200_F32, terms = dtype == XATTN_B200_F32_TERMS;
   if (!q || !k || !attn_sums) return XATTN_B200_ERR_ARG;
-  if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16 && dtype != XATTN_B200_F32_TERMS) return XATTN_B200_ERR_ARG;
+  if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16 && !f32 && !terms) return XATTN_B200_ERR_ARG;
+  if ((q_bf16 || k_bf16) && (!f32 || !q_bf16 || !k_bf16 || ((reinterpret_cast<uintptr_t>(q_bf16) | reinterpret_cast<uintptr_t>(k_bf16)) & 15)))
+    return XATTN_B200_ERR_ARG;
   if (semantics != XATTN_B200_SEMANTICS_TORCH && semantics != XATTN_B200_SEMANTICS_TRITON &&
       semantics != XATTN_B200_SEMANTICS_TORCH_BAND)
     return XATTN_B200_ERR_ARG;
@@ -1171,10 +1302,10 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   int rc = fill_geometry(batch, hq, hkv, q_len, k_len, head_dim, stride, block_size, chunk_size, scale, causal,
                          semantics, g);
   if (rc) return rc;
-  const bool split = dtype == XATTN_B200_F32_TERMS;
-  const uint64_t row_len = split ? 3 * (uint64_t)head_dim : (uint64_t)head_dim;
-  if (split) {
-    if (q_len % stride || k_len % stride) return XATTN_B200_ERR_ARG;       // (the split writes whole stride groups)
+  if (f32) g.d_chunks = head_dim / kF32Cols;
+  if (terms) {
+    // (the terms are written for whole stride groups; geometries without CTA pairs take fp32 rows)
+    if (q_len % stride || k_len % stride || !pairs_fit(g)) return XATTN_B200_ERR_ARG;
     g.term_chunks = g.d_chunks;
     g.d_chunks *= 3;
   }
@@ -1199,21 +1330,21 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // the ragged last group (see EstGeom::q_rem)
   auto make_map = [&](CUtensorMap* m, const void* x, int len, int heads, int64_t sb, int64_t sh, int64_t sl, uint32_t box_rows, bool up) -> int {
     const int groups = len / stride > 0 && !up ? len / stride : (len + stride - 1) / stride;
-    const uint64_t dims[5] = {row_len, (uint64_t)stride, (uint64_t)groups, (uint64_t)heads, (uint64_t)batch};
+    const uint64_t dims[5] = {(uint64_t)head_dim * (terms ? 3 : 1), (uint64_t)stride, (uint64_t)groups, (uint64_t)heads, (uint64_t)batch};
     // a dimension of extent 1 never moves: give it a harmless valid stride
-    const uint64_t str[4] = {(uint64_t)sl * 2, (uint64_t)sl * 2 * stride, heads > 1 ? (uint64_t)sh * 2 : 256, batch > 1 ? (uint64_t)sb * 2 : 256};
-    const uint32_t box[5] = {kTileK, 1, box_rows, 1, 1};
-    return make_tmap_16bit(m, x, 5, dims, str, box);
+    const uint64_t e = f32 ? 4 : 2;
+    const uint64_t str[4] = {(uint64_t)sl * e, (uint64_t)sl * e * stride, heads > 1 ? (uint64_t)sh * e : 256, batch > 1 ? (uint64_t)sb * e : 256};
+    const uint32_t box[5] = {static_cast<uint32_t>(f32 ? kF32Cols : kTileK), 1, box_rows, 1, 1};
+    return make_tmap(m, x, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, box);
   };
 
   // up to 64 KiB of dynamic shared memory (8192 row tiles): above the 48 KiB a kernel gets without asking
   if (!allow_smem(est_setup_kernel, 2 * sizeof(int) * 8192))
     return XATTN_B200_ERR_CUDA;
-  // CTA pairs (256x256 tiles) when tiles are 256 columns wide and the two row tiles of a pair see about the
-  // same columns (always, except when a 128-row chunk of the torch branch blanks everything left of it)
-  bool use_pairs = g.tile_n == kTileN && g.n_mtiles >= 2 && (!g.left_blank || g.rcs % (2 * kTileM) == 0);
+  bool use_pairs = pairs_fit(g);
   g.pair_heads = g.tile_n == kTileN && (hq / hkv) % 2 == 0 ? 1 : 0;
   if (g.pair_heads) use_pairs = true;
+  if (f32) use_pairs = false;
   // Few tiles (short prompts: 32 heads of up to 2048 tokens at stride 16 are 32 tiles for 148 SMs): the K loop of each, which is
   // a stream of operands through one SM, is split over a cluster of two or four CTAs instead.
   {
@@ -1223,7 +1354,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       row_tile_range(g, mt, first, count);
       tiles += static_cast<long long>(count > 0 ? count : 1) * batch * hq;
     }
-    const bool long_k = g.S * g.d_chunks >= 32;          // (the exchange costs about what eight steps take)
+    const bool long_k = g.S * g.d_chunks >= 32 && !terms;          // (the exchange costs about what eight steps take)
     g.split = !long_k ? 1 : (4 * tiles <= sm_count() ? 4 : (2 * tiles <= sm_count() ? 2 : 1));
     if (g.split > 1) use_pairs = false;
     if (!use_pairs) g.pair_heads = 0;
@@ -1244,7 +1375,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   }
   g.direct = direct ? 1 : 0;
   CUtensorMap tmQ, tmK, tmQt, tmKt;
-  const uint32_t k_box = use_pairs ? 64 : static_cast<uint32_t>(g.tile_n);
+  const uint32_t k_box = use_pairs ? 64 : (f32 ? static_cast<uint32_t>(kTileM) : static_cast<uint32_t>(g.tile_n));
   if ((rc = make_map(&tmQ, q, q_len, hq, qsb, qsh, qsl, kTileM, false))) return rc;
   if ((rc = make_map(&tmK, k, k_len, hkv, ksb, ksh, ksl, k_box, false))) return rc;
   tmQt = tmQ;
@@ -1337,16 +1468,40 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   const long long tiles = static_cast<long long>(tiles_per_head) * batch * hq;
   if (tiles == 0) g.split = 1;
   const int grid = g.split > 1 ? static_cast<int>(tiles) * g.split : sms;
-  auto launch = [&](auto kern) -> int {
-    if (!allow_smem(kern, kGemmSmem))
-      return XATTN_B200_ERR_CUDA;
-    return launch_dependent_clusters(kern, g.split, dim3(grid), dim3(kGemmThreads), kGemmSmem, stream, tmQ, tmK, tmQt, tmKt, g,
-                            (const int*)tile_lo, (const int*)tile_prefix, partial, mtile, attn_sums, idesc, status);
+  // The roundings of fp32 operands come with the tiles: a row tile's with its first, a column tile's with the first row tile that
+  // has it.  Where that leaves tokens out (keys that no query of the call may see), they are written by a pass of their own.
+  EstRounded rounded = {static_cast<uint4*>(q_bf16), static_cast<uint4*>(k_bf16), q_len, k_len};
+  if (q_bf16) {
+    int q_tokens = 0, k_tokens = 0, last = 0;            // the tokens before these are covered
+    for (int mt = 0; mt < g.n_mtiles; ++mt) {
+      int first, cnt;
+      row_tile_range(g, mt, first, cnt);
+      if (cnt > 0 && q_tokens == mt * kTileM * g.S) q_tokens += kTileM * g.S;
+      if (cnt > 0 && first <= last) last = first + cnt > last ? first + cnt : last;
+    }
+    k_tokens = last * g.tile_n * g.S;
+    if (q_tokens < q_len) {
+      if ((rc = split_f32_launch(static_cast<const float*>(q), batch, hq, q_len, q_len, head_dim, qsb, qsh, qsl, 1, q_bf16, stream))) return rc;
+      rounded.q = nullptr;
+    }
+    if (k_tokens < k_len) {
+      if ((rc = split_f32_launch(static_cast<const float*>(k), batch, hkv, k_len, k_len, head_dim, ksb, ksh, ksl, 1, k_bf16, stream))) return rc;
+      rounded.k = nullptr;
+    }
+  }
+  auto launch = [&](auto kern, int threads, int smem) -> int {
+    if (!allow_smem(kern, smem)) return XATTN_B200_ERR_CUDA;
+    return launch_dependent_clusters(kern, g.split, dim3(grid), dim3(threads), smem, stream, tmQ, tmK, tmQt, tmKt, g, (const int*)tile_lo,
+                                     (const int*)tile_prefix, partial, mtile, attn_sums, idesc, rounded, status);
+  };
+  auto launch_type = [&](auto rbs, auto halves) -> int {
+    constexpr int kRbs = decltype(rbs)::value, kDirect = decltype(halves)::value;
+    return f32 ? launch(est_gemm_kernel<kRbs, kDirect, true>, f32_threads(kDirect), kF32Smem + 2048)
+               : launch(est_gemm_kernel<kRbs, kDirect, false>, kGemmThreads, kGemmSmem);
   };
   auto launch_rbs = [&](auto rbs) -> int {
-    constexpr int kRbs = decltype(rbs)::value;
-    if (!direct) return launch(est_gemm_kernel<kRbs, 0>);
-    return g.tile_n == 128 ? launch(est_gemm_kernel<kRbs, 1>) : launch(est_gemm_kernel<kRbs, 2>);
+    if (!direct) return launch_type(rbs, std::integral_constant<int, 0>());
+    return g.tile_n == 128 ? launch_type(rbs, std::integral_constant<int, 1>()) : launch_type(rbs, std::integral_constant<int, 2>());
   };
   switch (g.rbs) {
     case 4: rc = launch_rbs(std::integral_constant<int, 4>()); break;

@@ -20,7 +20,7 @@ size_t estimate_workspace_bytes(int batch, int hq, int q_len, int k_len, int str
 int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, int hkv, int q_len, int k_len,
                     int head_dim, int64_t qsb, int64_t qsh, int64_t qsl, int64_t ksb, int64_t ksh, int64_t ksl,
                     int stride, int block_size, int chunk_size, float scale, int causal, int semantics,
-                    float* attn_sums, void* workspace, size_t workspace_bytes, int* status, cudaStream_t stream);
+                    float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16, int* status, cudaStream_t stream);
 }  // namespace xb
 
 // The scratch itself.  In host code this name is only a handle for the runtime's symbol table, not an
@@ -69,5 +69,5 @@ extern "C" int xattn_b200_estimate_static(const void* q, const void* k, int dtyp
   return xb::estimate_launch(q, k, dtype, batch, hq, hkv, q_len, k_len, head_dim, q_stride_b, q_stride_h,
                              q_stride_l, k_stride_b, k_stride_h, k_stride_l, stride, block_size, chunk_size, scale,
                              causal, semantics, attn_sums, scratch, static_cast<size_t>(XATTN_B200_STATIC_SCRATCH_BYTES),
-                             status, static_cast<cudaStream_t>(cuda_stream));
+                             nullptr, nullptr, status, static_cast<cudaStream_t>(cuda_stream));
 }

@@ -122,53 +122,57 @@ Geometry geometry(int64_t q_len, int64_t k_len, int chunk, int stride, int block
   return g;
 }
 
-// An operand of the estimate: 16-bit rows, or fp32 rows split into three bf16 terms each.
-struct Operand {
-  Tensor t;               // [B, H, len, D] (fp32: [B, H, len rounded up to the stride, 3 D] terms)
-  int64_t len;
-  int dtype;
-};
-Operand split_f32(const Tensor& x, int stride, const Place& at_) {
-  const Tensor r = x.stride(3) == 1 ? x : x.contiguous();
-  const int64_t len = (x.size(2) + stride - 1) / stride * stride, D = x.size(3);
-  Operand o;
-  o.t = empty({x.size(0), x.size(1), len, 3 * D}, at::kBFloat16, at_.dev);
-  o.len = len;
-  o.dtype = XATTN_B200_F32_TERMS;
-  check(xattn_b200_split_f32(static_cast<const float*>(r.data_ptr()), x.size(0), x.size(1), len, x.size(2), D, r.stride(0),
-                             r.stride(1), r.stride(2), 3, o.t.data_ptr(), at_.stream),
-        "split_f32");
-  return o;
-}
-Operand operand(const Tensor& x, int stride, bool f32, const Place& at_) {
-  if (f32) return split_f32(x.scalar_type() == at::kFloat ? x : x.to(at::kFloat), stride, at_);
-  Operand o;
-  o.dtype = dtype_code(x.scalar_type());
-  o.len = x.size(2);
-  o.t = aligned16(x);
-  return o;
-}
-
 struct EstimateArgs {
   int stride, block, chunk, semantics;
   double norm;
   bool causal, band;
 };
 // fp32 block sums [B, Hq, q_blocks_pad, k_blocks_pad or blocks_per_chunk]
-Tensor estimate(const Operand& q, const Operand& k, int64_t D, const Geometry& g, const EstimateArgs& a, const Place& at_) {
-  const int64_t B = q.t.size(0), Hq = q.t.size(1), Hkv = k.t.size(1);
+// q16, k16 (fp32 inputs, null: not wanted): set to the bf16 roundings of q and k.
+Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const EstimateArgs& a, Tensor* q16, Tensor* k16, const Place& at_) {
+  int dtype = q_.scalar_type() == at::kFloat ? XATTN_B200_F32 : dtype_code(q_.scalar_type());
+  Tensor q = aligned16(q_), k = aligned16(dtype == XATTN_B200_F32 && k_.scalar_type() != at::kFloat ? k_.to(at::kFloat) : k_);
+  const int64_t B = q.size(0), Hq = q.size(1), Hkv = k.size(1), D = q.size(3);
+  int64_t Lq = q.size(2), Lk = k.size(2);
   const int sem = a.band ? XATTN_B200_SEMANTICS_TORCH_BAND : a.semantics;
-  const size_t bytes = xattn_b200_estimate_workspace_bytes_ex(B, Hq, q.len, k.len, a.stride, a.block, a.chunk, a.causal, sem);
+  if (dtype == XATTN_B200_F32 && xattn_b200_estimate_f32_terms(Hq, Hkv, Lq, Lk, a.stride, a.block, a.chunk, a.causal, sem)) {
+    dtype = XATTN_B200_F32_TERMS;
+    const auto split = [&](const Tensor& x) {
+      const int64_t len = (x.size(2) + a.stride - 1) / a.stride * a.stride;
+      Tensor t = empty({B, x.size(1), len, 3 * D}, at::kBFloat16, at_.dev);
+      check(xattn_b200_split_f32(static_cast<const float*>(x.data_ptr()), B, x.size(1), len, x.size(2), D, x.stride(0), x.stride(1),
+                                 x.stride(2), 3, t.data_ptr(), at_.stream),
+            "split_f32");
+      return t;
+    };
+    q = split(q);
+    k = split(k);
+    // (the first terms ARE the roundings)
+    if (q16) *q16 = q.narrow(3, 0, D).narrow(2, 0, Lq);
+    if (k16) *k16 = k.narrow(3, 0, D).narrow(2, 0, Lk);
+    Lq = q.size(2);
+    Lk = k.size(2);
+  } else if (dtype == XATTN_B200_F32 && q16) {
+    *q16 = empty(q.sizes(), at::kBFloat16, at_.dev);
+    *k16 = empty(k.sizes(), at::kBFloat16, at_.dev);
+  }
+  const size_t bytes = xattn_b200_estimate_workspace_bytes_ex(B, Hq, Lq, Lk, a.stride, a.block, a.chunk, a.causal, sem);
   if (bytes == 0)
     fail(PyExc_ValueError, "unsupported estimate geometry (stride must be 4/8/16/32, block_size 128, chunk_size a multiple of 128)");
   const Tensor ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
   Tensor sums = empty({B, Hq, g.qb, a.band ? g.bpc : g.kb}, at::kFloat, at_.dev);
   const double scale = 1.0 / std::sqrt(static_cast<double>(D)) / a.stride / a.norm;
-  check(xattn_b200_estimate(q.t.data_ptr(), k.t.data_ptr(), q.dtype, B, Hq, Hkv, q.len, k.len, D, q.t.stride(0), q.t.stride(1),
-                            q.t.stride(2), k.t.stride(0), k.t.stride(1), k.t.stride(2), a.stride, a.block, a.chunk,
-                            static_cast<float>(scale), a.causal, sem, static_cast<float*>(sums.data_ptr()), ws.data_ptr(), bytes,
-                            at_.status, at_.stream),
-        "estimate");
+  if (dtype == XATTN_B200_F32)
+    check(xattn_b200_estimate_f32(static_cast<const float*>(q.data_ptr()), static_cast<const float*>(k.data_ptr()), B, Hq, Hkv, Lq, Lk, D,
+                                  q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), a.stride, a.block, a.chunk,
+                                  static_cast<float>(scale), a.causal, sem, static_cast<float*>(sums.data_ptr()), ws.data_ptr(), bytes,
+                                  q16 ? q16->data_ptr() : nullptr, k16 ? k16->data_ptr() : nullptr, at_.status, at_.stream),
+          "estimate_f32");
+  else
+    check(xattn_b200_estimate(q.data_ptr(), k.data_ptr(), dtype, B, Hq, Hkv, Lq, Lk, D, q.stride(0), q.stride(1), q.stride(2), k.stride(0),
+                              k.stride(1), k.stride(2), a.stride, a.block, a.chunk, static_cast<float>(scale), a.causal, sem,
+                              static_cast<float*>(sums.data_ptr()), ws.data_ptr(), bytes, at_.status, at_.stream),
+          "estimate");
   return sums;
 }
 
@@ -263,9 +267,7 @@ PyObject* py_estimate(PyObject*, PyObject* const* v, Py_ssize_t n) {
   const Place at_(q);
   EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), a.flag(8)};
   const Geometry g = geometry(q.size(2), k.size(2), e.chunk, e.stride, e.block);
-  const bool f32 = q.scalar_type() == at::kFloat;
-  const Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
-  return wrap(estimate(qo, ko, q.size(3), g, e, at_));
+  return wrap(estimate(q, k, g, e, nullptr, nullptr, at_));
   END_HANDLE_TH_ERRORS
 }
 
@@ -377,23 +379,22 @@ PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   const Geometry g = geometry(Lq, Lk, e.chunk, e.stride, e.block);
   Tensor out;
   if (!a.none(12)) out = a.tensor(12);
-  const bool f32 = q.scalar_type() == at::kFloat;
-  const Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
+  // fp32: the attention phase computes with the bf16 roundings, those of q and k come from the estimate
+  const bool f32 = q.scalar_type() == at::kFloat && D == 128 && !out.defined() && v.scalar_type() == at::kFloat;
+  Tensor q16, k16;
   Selection s;
   {
-    const Tensor sums = estimate(qo, ko, D, g, e, at_);
+    const Tensor sums = estimate(q, k, g, e, f32 ? &q16 : nullptr, f32 ? &k16 : nullptr, at_);
     s = select(sums, pv[5], {g.bpc, g.block_offset, e.causal, true, a.flag(9), a.flag(10), false, Lq, Lk, e.band ? g.kb : 0}, at_);
   }
   const double scale = 1.0 / std::sqrt(static_cast<double>(D));
-  if (f32 && D == 128 && !out.defined() && v.scalar_type() == at::kFloat) {
-    // the first terms of q and k ARE their bf16 roundings, which the attention phase computes with
+  if (f32) {
     const Tensor vc = v.stride(3) == 1 ? v : v.contiguous();
     const Tensor v16 = empty(v.sizes(), at::kBFloat16, at_.dev);
     check(xattn_b200_split_f32(static_cast<const float*>(vc.data_ptr()), v.size(0), v.size(1), Lk, Lk, D, vc.stride(0), vc.stride(1),
                                vc.stride(2), 1, v16.data_ptr(), at_.stream),
           "split_f32");
-    return wrap(attention(qo.t.narrow(3, 0, D).narrow(2, 0, Lq), ko.t.narrow(3, 0, D).narrow(2, 0, Lk), v16, s.idx, s.cnt, e.causal, scale,
-                          out, true, default_workspace(e.causal, false, q), at_));
+    return wrap(attention(q16, k16, v16, s.idx, s.cnt, e.causal, scale, out, true, default_workspace(e.causal, false, q), at_));
   }
   return wrap(attention_any(q, k, v, s.idx, s.cnt, e.causal, scale, out, std::nullopt, at_));
   END_HANDLE_TH_ERRORS
@@ -411,8 +412,7 @@ PyObject* py_estimate_and_select(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   const EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), false};
   const Geometry g = geometry(q.size(2), k.size(2), e.chunk, e.stride, e.block);
   const bool f32 = q.scalar_type() == at::kFloat;
-  const Operand qo = operand(q, e.stride, f32, at_), ko = operand(k, e.stride, f32, at_);
-  const Tensor sums = estimate(qo, ko, q.size(3), g, e, at_);
+  const Tensor sums = estimate(q, k, g, e, nullptr, nullptr, at_);
   const Selection s = select(sums, pv[8], {g.bpc, g.block_offset, e.causal, true, a.flag(9), a.flag(10), true, 0, 0, 0}, at_);
   PyObject* t = PyTuple_New(2);
   if (!t) throw python_error();
