@@ -1025,21 +1025,30 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // Normalisation of the partial sums, one CTA per query block:
 //   row i:  m_i = max_t m_{i,t},  l_i = sum_t s_{i,t} 2^(m_{i,t} - m_i)                (m, s = per-tile max and sum)
 //   out[kb] = sum_i partial[i][kb] * f_{i,t(kb)},  f_{i,t} = 2^(m_{i,t} - m_i) / l_i
-// A stream over the partial sums: a thread per key block reads its RBS rows as 16-byte vectors (64 contiguous bytes for
-// RBS = 16), the factors come from shared memory.  The first key block's rows are on their way while the statistics are
-// computed.  (32K tokens, stride 8: the estimate phase 267 us with rows apart in the scratch and the factors recomputed by every thread,
-// 238 us like this.)
+// A stream over the partial sums, bound by the latency of each query block's chain (statistics, factors, sums): a warp per query
+// block, a lane per key block, whose RBS rows it reads as 16-byte vectors (64 contiguous bytes for RBS = 16), a few key blocks in
+// flight at a time and the first ones while the statistics are computed; the factors come from shared memory.  The longest query
+// blocks go first.  Calls of few query blocks (a short prompt's last chunk against a long cache) have four warps per query block.
+// (32 heads, 32768 tokens: at stride 16 20.5 us with a CTA per query block, 12.7 like this; at stride 8 21.8 and 14.8.)
 constexpr int kSumThreads = 128;
-template <int RBS>
+template <int RBS, int kTeam>
 __global__ void __launch_bounds__(kSumThreads)
 est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix, const float* __restrict__ partial,
                     const float2* __restrict__ mtile, float* __restrict__ sums, int seg_tiles) {
-  extern __shared__ float s_f[];                           // [tile][row] factors, seg_tiles tiles at a time
-  __shared__ float2 s_part[kSumThreads];                   // [part][row] (max, sum)
-  constexpr int kParts = kSumThreads / RBS;
+  extern __shared__ float s_factors[];                     // [team][tile][row] factors, seg_tiles tiles at a time
+  __shared__ float2 s_part[4][RBS];                        // (teams of four warps) [warp][row] (max, sum)
+  constexpr int kParts = kTeam / RBS, kTeams = kSumThreads / kTeam;
+  constexpr int kAhead = kTeam > 32 || RBS > 16 ? 1 : 16 / RBS;          // key blocks per lane in flight (32 / RBS: 10 % slower)
   pdl_launch_dependents();
   pdl_wait();
-  const int qb = blockIdx.x, bh = blockIdx.y;
+  const int team = threadIdx.x / kTeam, tid = threadIdx.x % kTeam, heads = g.batch * g.hq;
+  const int item = blockIdx.x * kTeams + team;
+  if (item >= heads * g.qb_total) return;                  // (a whole team, and teams of the whole CTA have none left over)
+  const int qb = g.qb_total - 1 - item / heads, bh = item % heads;
+  auto sync = [&]() {
+    if constexpr (kTeam == 32) __syncwarp(); else __syncthreads();
+  };
+  float* s_f = s_factors + team * seg_tiles * RBS;
   const int i0 = qb * RBS, mt = i0 / kTileM, r0 = i0 % kTileM;
   const int nlo = g.tab_n ? g.tab[mt] : tile_lo[mt];
   const int ncnt = g.tab_n ? g.tab[kTabPrefix + mt + 1] - g.tab[kTabPrefix + mt] : tile_prefix[mt + 1] - tile_prefix[mt];
@@ -1058,69 +1067,86 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
     if (i0 >= g.rows_valid) k_end = 0;
     else if (vis < k_end) k_end = vis;
   }
-  float4 p4[RBS / 4];
-  auto fetch = [&](int kl) {                               // the rows of output kl; zeros outside the tiles
-    const int k = cur + kl - nlo * gpt;
-    const bool in = kl < n_out && k >= 0 && k < k_end;
+  float4 p4[kAhead][RBS / 4];
+  auto fetch = [&](int kl0) {                              // the rows of outputs kl0 + u * kTeam; zeros outside the tiles
 #pragma unroll
-    for (int j = 0; j < RBS / 4; ++j)
-      p4[j] = in ? __ldcs(reinterpret_cast<const float4*>(pp + static_cast<size_t>(k) * kTileM) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < kAhead; ++u) {
+      const int kl = kl0 + u * kTeam, k = cur + kl - nlo * gpt;
+      const bool in = kl < n_out && k >= 0 && k < k_end;
+#pragma unroll
+      for (int j = 0; j < RBS / 4; ++j)
+        p4[u][j] = in ? __ldcs(reinterpret_cast<const float4*>(pp + static_cast<size_t>(k) * kTileM) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   };
-  fetch(threadIdx.x);
-  float row_m, row_inv;                                    // of row threadIdx.x % RBS
+  fetch(tid);
+  float row_m, row_inv;                                    // of row tid % RBS
   {
-    const int row = threadIdx.x % RBS, part = threadIdx.x / RBS;
+    const int row = tid % RBS, part = tid / RBS;
     const bool valid = i0 + row < g.rows_valid;
     float m = -INFINITY, l = 0.f;
-    for (int t = part; t < ncnt; t += kParts) {
-      const float2 x = ms[t * kTileM + row];
-      if (valid && x.x > -INFINITY) {
-        const float mn = fmaxf(m, x.x);
-        l = l * exp2f(m - mn) + x.y * exp2f(x.x - mn);
+    auto add = [&](float xm, float xl) {
+      if (xm > -INFINITY) {
+        const float mn = fmaxf(m, xm);
+        l = l * exp2f(m - mn) + xl * exp2f(xm - mn);
         m = mn;
       }
-    }
-    s_part[threadIdx.x] = make_float2(m, l);
-    __syncthreads();
-    float mm = -INFINITY, ll = 0.f;
+    };
+    if (valid) {
 #pragma unroll 4
-    for (int k = 0; k < kParts; ++k) mm = fmaxf(mm, s_part[k * RBS + row].x);
-#pragma unroll 4
-    for (int k = 0; k < kParts; ++k) {
-      const float2 x = s_part[k * RBS + row];
-      if (x.x > -INFINITY) ll += x.y * exp2f(x.x - mm);
+      for (int t = part; t < ncnt; t += kParts) {
+        const float2 x = ms[t * kTileM + row];
+        add(x.x, x.y);
+      }
     }
-    row_m = mm;
-    row_inv = ll > 0.f ? 1.f / ll : 0.f;
+#pragma unroll
+    for (int o = RBS; o < 32; o <<= 1) add(__shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, l, o));
+    if constexpr (kTeam > 32) {
+      if ((threadIdx.x & 31) < RBS) s_part[threadIdx.x >> 5][row] = make_float2(m, l);
+      __syncthreads();
+      m = -INFINITY;
+      l = 0.f;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) add(s_part[w][row].x, s_part[w][row].y);
+    }
+    row_m = m;
+    row_inv = l > 0.f ? 1.f / l : 0.f;
   }
   float* out = sums + (static_cast<size_t>(bh) * g.qb_total + qb) * n_out;
 #pragma unroll 1
   for (int t0 = 0; t0 == 0 || t0 < ncnt; t0 += seg_tiles) {
     const int t1 = t0 + seg_tiles < ncnt ? t0 + seg_tiles : ncnt;
     if (t0 > 0) {
-      __syncthreads();
-      fetch(threadIdx.x);
+      sync();
+      fetch(tid);
     }
-    for (int t = t0 + threadIdx.x / RBS; t < t1; t += kParts) {
-      const float x = ms[t * kTileM + threadIdx.x % RBS].x;
-      s_f[(t - t0) * RBS + threadIdx.x % RBS] = row_inv > 0.f && x > -INFINITY ? exp2f(x - row_m) * row_inv : 0.f;
+    for (int t = t0 + tid / RBS; t < t1; t += kParts) {
+      const float x = ms[t * kTileM + tid % RBS].x;
+      s_f[(t - t0) * RBS + tid % RBS] = row_inv > 0.f && x > -INFINITY ? exp2f(x - row_m) * row_inv : 0.f;
     }
-    __syncthreads();
-    for (int kl = threadIdx.x; kl < n_out; kl += kSumThreads) {
-      const int k = cur + kl - nlo * gpt, t = k >= 0 && k < k_end ? k / gpt : -1;
-      if (t >= t0 && t < t1) {
-        const float4* f4 = reinterpret_cast<const float4*>(s_f + (t - t0) * RBS);
-        float acc = 0.f;
+    sync();
+#pragma unroll 1
+    for (int kl0 = tid; kl0 < n_out; kl0 += kAhead * kTeam) {
+      float acc[kAhead];
 #pragma unroll
-        for (int j = 0; j < RBS / 4; ++j) {
-          const float4 f = f4[j];
-          acc += p4[j].x * f.x + p4[j].y * f.y + p4[j].z * f.z + p4[j].w * f.w;
+      for (int u = 0; u < kAhead; ++u) {
+        const int k = cur + kl0 + u * kTeam - nlo * gpt, t = k >= 0 && k < k_end ? k / gpt : -1;
+        acc[u] = 0.f;
+        if (t >= t0 && t < t1) {
+          const float4* f4 = reinterpret_cast<const float4*>(s_f + (t - t0) * RBS);
+#pragma unroll
+          for (int j = 0; j < RBS / 4; ++j) {
+            const float4 f = f4[j];
+            acc[u] += p4[u][j].x * f.x + p4[u][j].y * f.y + p4[u][j].z * f.z + p4[u][j].w * f.w;
+          }
         }
-        out[kl] = acc;
-      } else if (t0 == 0 && t < 0) {
-        out[kl] = 0.f;
       }
-      if (kl + kSumThreads < n_out) fetch(kl + kSumThreads);
+      const int here = kl0;
+      if (kl0 + kAhead * kTeam < n_out) fetch(kl0 + kAhead * kTeam);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int kl = here + u * kTeam, k = cur + kl - nlo * gpt, t = k >= 0 && k < k_end ? k / gpt : -1;
+        if (kl < n_out && ((t >= t0 && t < t1) || (t0 == 0 && t < 0))) out[kl] = acc[u];
+      }
     }
   }
 }
@@ -1514,17 +1540,21 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   if (rc) return rc;
   }
 
-  const int seg_tiles = g.m_pitch < 32 * 1024 / (4 * g.rbs) ? g.m_pitch : 32 * 1024 / (4 * g.rbs);     // 32 KiB of factors at most
+  // A warp per query block where that fills the chip (16 warps per SM), otherwise four.  32 KiB of factors per CTA at most.
+  const long long items = static_cast<long long>(batch) * hq * g.qb_total;
+  const bool wide = items < 16 * 148;
+  const int teams = wide ? 1 : kSumThreads / 32, seg_max = 32 * 1024 / (4 * g.rbs * teams);
+  const int seg_tiles = g.m_pitch < seg_max ? g.m_pitch : seg_max;
   auto launch_sums = [&](auto kern) -> int {
-    return launch_dependent(kern, dim3(g.qb_total, batch * hq), dim3(kSumThreads), static_cast<size_t>(seg_tiles) * g.rbs * sizeof(float),
-                            stream, g, (const int*)tile_lo, (const int*)tile_prefix, (const float*)partial, (const float2*)mtile,
-                            attn_sums, seg_tiles);
+    return launch_dependent(kern, dim3(static_cast<unsigned>((items + teams - 1) / teams)), dim3(kSumThreads),
+                            static_cast<size_t>(teams) * seg_tiles * g.rbs * sizeof(float), stream, g, (const int*)tile_lo,
+                            (const int*)tile_prefix, (const float*)partial, (const float2*)mtile, attn_sums, seg_tiles);
   };
   switch (g.rbs) {
-    case 4: return launch_sums(est_blocksum_kernel<4>);
-    case 8: return launch_sums(est_blocksum_kernel<8>);
-    case 16: return launch_sums(est_blocksum_kernel<16>);
-    case 32: return launch_sums(est_blocksum_kernel<32>);
+    case 4: return wide ? launch_sums(est_blocksum_kernel<4, 128>) : launch_sums(est_blocksum_kernel<4, 32>);
+    case 8: return wide ? launch_sums(est_blocksum_kernel<8, 128>) : launch_sums(est_blocksum_kernel<8, 32>);
+    case 16: return wide ? launch_sums(est_blocksum_kernel<16, 128>) : launch_sums(est_blocksum_kernel<16, 32>);
+    case 32: return wide ? launch_sums(est_blocksum_kernel<32, 128>) : launch_sums(est_blocksum_kernel<32, 32>);
     default: return XATTN_B200_ERR_ARG;
   }
 }
