@@ -1540,9 +1540,10 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   if (rc) return rc;
   }
 
-  // A warp per query block where that fills the chip (16 warps per SM), otherwise four.  32 KiB of factors per CTA at most.
+  // A warp per query block where that fills the chip (32 warps per SM; 2528 query blocks: the estimate 58.6 us by one warp each, 57.5
+  // by four), otherwise four.  32 KiB of factors per CTA at most.
   const long long items = static_cast<long long>(batch) * hq * g.qb_total;
-  const bool wide = items < 16 * 148;
+  const bool wide = items < 32 * 148;
   const int teams = wide ? 1 : kSumThreads / 32, seg_max = 32 * 1024 / (4 * g.rbs * teams);
   const int seg_tiles = g.m_pitch < seg_max ? g.m_pitch : seg_max;
   auto launch_sums = [&](auto kern) -> int {
