@@ -54,11 +54,6 @@ inline int make_tmap(CUtensorMap* map, const void* base, CUtensorMapDataType typ
   return r == CUDA_SUCCESS ? XATTN_B200_OK : XATTN_B200_ERR_CUDA;
 }
 
-inline int make_tmap_16bit(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
-                           const uint32_t* box) {
-  return make_tmap(map, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, dims, strides_bytes, box);
-}
-
 // What has to be set up or asked once per kernel and device, and costs microseconds of every call otherwise: `ask` runs at
 // the first use (its positive answer is kept; a failure is not).  A few dozen kernels and up to 16 devices; safe to use
 // from several threads (two may ask at once, and get the same answer).

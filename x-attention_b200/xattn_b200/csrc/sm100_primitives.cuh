@@ -105,24 +105,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return true;
 }
 
-// Bounded wait that polls without ever suspending the thread: for the single-thread roles (TMA issue, MMA
-// issue) whose reaction time is on the critical path; a suspended thread was measured to resume ~1000 cycles
-// after the phase completed.
-__device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  const long long t0 = clock64();
-#pragma unroll 1
-  while (true) {
-#pragma unroll 1
-    for (int i = 0; i < 512; ++i)
-      if (mbar_test(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() - t0 > kWaitCycleLimit) {
-      *abort_flag = 1;
-      return false;
-    }
-  }
-}
-
 // ------------------------------------------------------------------ programmatic dependent launch
 // A kernel launched with the programmatic-stream-serialization attribute may start once every CTA of the kernel
 // before it in the stream has executed pdl_launch_dependents() or exited; what that kernel wrote is visible only
@@ -141,14 +123,6 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* m, 
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1,
-                                            int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
 
@@ -190,12 +164,6 @@ __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bu
 
 // Bring a tile into L2 only (no shared memory, no barrier): used to hide HBM latency for tiles whose
 // shared-memory slot is not free yet.
-__device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* m, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
-               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-               : "memory");
-}
-
 __device__ __forceinline__ void tma_prefetch_l2_5d(const CUtensorMap* m, int c0, int c1, int c2, int c3, int c4) {
   asm volatile("cp.async.bulk.prefetch.tensor.5d.L2.global.tile [%0, {%1, %2, %3, %4, %5}];"
                ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
@@ -379,23 +347,9 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// issued by the even CTA only; descriptors are offsets valid in both CTAs' shared memory
-__device__ __forceinline__ void mma_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// one arrival, once the pair's MMAs issued so far are complete, on the barrier at this offset in every CTA of
-// `cta_mask` (no data moves: this is the commit's own multicast of the arrival)
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint16_t cta_mask) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"(cta_mask)
-               : "memory");
-}
-// the same two for a converged warp of which the thread with `lead` issues (see mma_ss_lead)
+// Issued by the even CTA only (the thread with `lead` of a converged warp, see mma_ss_lead); descriptors are offsets valid in
+// both CTAs' shared memory.  The commit: one arrival, once the pair's MMAs issued so far are complete, on the barrier at this
+// offset in every CTA of `cta_mask` (no data moves: this is the commit's own multicast of the arrival).
 __device__ __forceinline__ void mma_ss_pair_lead(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                  uint32_t accumulate, uint32_t lead) {
   asm volatile(
@@ -413,15 +367,6 @@ __device__ __forceinline__ void mma_commit_pair_lead(uint32_t bar, uint16_t cta_
 }
 // TMA load into this CTA's shared memory whose completion is counted on a barrier that may live in the peer CTA
 // (`bar_cluster` is a shared::cluster address)
-__device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster, int c0,
-                                                 int c1, int c2, int c3, int c4) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
-      : "memory");
-}
-
 __device__ __forceinline__ void tma_load_5d_pair_lead(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster, int c0, int c1,
                                                       int c2, int c3, int c4, uint32_t lead) {
   asm volatile(
