@@ -42,12 +42,9 @@ import torch  # noqa: E402
 
 METRIC = "prefill_attention_effective_tflops"
 UNIT = "TFLOP/s (dense-equivalent, 4*Lq*Lk*D*Hq/2 causal)"
-# dram__bytes_read.sum + dram__bytes_write.sum of ONE launch of the attention kernel that does the bulk of the call,
-# from ncu captures of this benchmark's own command line.  32K: block_sparse_attn_kernel on the full workload
-# (405.4 MB read + 234.1 MB written).  128K: block_sparse_attn_pair_kernel, captured on two of the eight kv-head
-# groups (--heads-limit 2: 421.3 MB + 219.8 MB) and multiplied by four -- every kv group reads and writes its own
-# Q, K, V and O, so the traffic grows in proportion.
-NCU_ATTENTION_TRAFFIC_BYTES = {"llama3_8b_32k": 639_545_088, "llama3_8b_128k": 4 * 641_088_000}
+# dram__bytes_read.sum + dram__bytes_write.sum of ONE launch of block_sparse_attn_kernel at the workload's shapes, from ncu
+# captures (32K: 404.7 MB read + 226.3 MB written; 128K: 1615.7 MB + 1032.4 MB).
+NCU_ATTENTION_TRAFFIC_BYTES = {"llama3_8b_32k": 404_710_912 + 226_263_296, "llama3_8b_128k": 1_615_714_304 + 1_032_417_792}
 DEFAULT_WORKLOAD = "llama3_8b_32k"
 LONG_WORKLOAD = "llama3_8b_128k"
 
