@@ -78,3 +78,19 @@ def test_dense_rows_of_a_few_chunks(lq, lk, stride, chunk):
     """Un-padded causal keys whose chunks are a tile or less each: the epilogue writes whole rows, zeros included; chunks that
     are not a multiple of a tile leave tiles that hang over the row's end."""
     _check(2, 2, lq, lk, stride, chunk, True, torch.bfloat16)
+
+
+@pytest.mark.parametrize("stride,hkv,chunk,causal,semantics", [(4, 20, 16384, True, "torch"), (8, 8, 16384, True, "triton"),
+                                                               (16, 20, 8192, True, "torch"), (32, 8, 16384, False, "torch")])
+def test_many_query_blocks(stride, hkv, chunk, causal, semantics):
+    """Block sums by a warp per query block, which calls of many query blocks get: the first and the last head."""
+    from xattn_b200 import ops
+    hq, L = 40, 15400                                    # 40 * 128 (padded) query blocks; several column tiles per row
+    g = torch.Generator().manual_seed(stride)
+    k = torch.randn(1, hkv, L, 128, generator=g).bfloat16()
+    q = torch.randn(1, hq, L, 128, generator=g).bfloat16()
+    got = ops.estimate_block_sums(q.to(DEV), k.to(DEV), stride, 128, chunk, 1.0, causal, semantics=semantics).cpu()
+    for h in (0, hq - 1):
+        want = orc.estimate_block_sums(q[:, h:h + 1].float(), k[:, h * hkv // hq:h * hkv // hq + 1].float(), 128, stride, 1.0, chunk, causal,
+                                       semantics)
+        assert torch.allclose(got[:, h:h + 1], want, rtol=RTOL, atol=ATOL), float((got[:, h:h + 1] - want).abs().max())
