@@ -206,6 +206,15 @@ int xattn_b200_select(const float* attn_sums, int batch, int heads, int q_blocks
                       int list_k_len, int* status, void* cuda_stream);
 
 /*
+ * xattn_b200_select without lists that also writes attn_sums rounded to XATTN_B200_BF16 or _F16 (same shape, 8-byte aligned):
+ * what xattn_estimate returns (xattn/src/Xattention.py:299).  k_blocks <= 1024.
+ */
+int xattn_b200_select_rounded(const float* attn_sums, int batch, int heads, int q_blocks, int k_blocks, int blocks_per_chunk,
+                              int block_offset, int causal, int diagonal_cleanup, double threshold,
+                              const float* threshold_per_head, int keep_sink, int keep_recent, uint8_t* mask, void* rounded,
+                              int rounded_dtype, int* status, void* cuda_stream);
+
+/*
  * xattn_b200_select for attn_sums in chunk-band layout (XATTN_B200_SEMANTICS_TORCH_BAND): attn_sums is
  * [batch, heads, q_blocks, blocks_per_chunk]; entry c of row R is the score of key block current_index + c, every
  * other key block has score zero.  Same rule, same outputs (mask and lists are over all k_blocks columns), but a

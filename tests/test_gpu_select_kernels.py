@@ -53,3 +53,16 @@ def test_against_the_oracle(N, bpc, causal, kind):
                 for h in range(2):
                     for r in range(R):
                         assert idx[0, h, r, :cnt[0, h, r]].tolist() == mask[0, h, r].nonzero().flatten().tolist()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("L,chunk", [(100, 128), (1003, 384), (8192, 8192), (65536 + 640, 2048 + 128), (131200, 128)])   # 1 to 1025 key blocks
+def test_returned_sums_are_the_selections_own_rounded(L, chunk, dtype):
+    """The sums in the inputs' type, which the selection kernel writes for rows of up to 1024 blocks, bit by bit."""
+    from xattn_b200 import api, ops
+    g = torch.Generator(device=DEV).manual_seed(L)
+    q, k = (torch.randn(1, h, L, 128, device=DEV, generator=g).to(dtype) for h in (2, 1))
+    sums, mask = api.xattn_estimate(q, k, 128, 16, threshold=0.8, chunk_size=chunk, causal=True)
+    want = ops.estimate_block_sums(q, k, 16, 128, chunk, 1.0, True)
+    assert sums.dtype == dtype and mask.shape == sums.shape
+    assert torch.equal(sums, want.to(dtype))

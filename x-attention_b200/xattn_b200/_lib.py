@@ -36,6 +36,7 @@ SIGNATURES = {
     "xattn_b200_rope_qk": (_i, [_p, _p, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64, _i64, _p, _p, _i64, _i64, _p]),
     "xattn_b200_select": (_i, [_p, _i, _i, _i, _i, _i, _i, _i, _i, _d, _p, _i, _i, _p, _p, _p,
                                _i, _i, _i, _i, _p, _p]),
+    "xattn_b200_select_rounded": (_i, [_p, _i, _i, _i, _i, _i, _i, _i, _i, _d, _p, _i, _i, _p, _p, _i, _p, _p]),
     "xattn_b200_select_band": (_i, [_p, _i, _i, _i, _i, _i, _i, _i, _i, _d, _p, _i, _i, _p, _p, _p,
                                     _i, _i, _i, _i, _p, _p]),
     "xattn_b200_mask_to_lists": (_i, [_p, _i, _i, _i, _i, _i, _i, _i, _p, _p, _p]),

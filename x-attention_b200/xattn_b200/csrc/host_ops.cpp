@@ -185,7 +185,8 @@ struct SelectArgs {
   int64_t list_q, list_k;       // 0: no lists
   int64_t band_kb;              // > 0: the sums are the chunk band of rows of that many key blocks
 };
-Selection select(const Tensor& sums, PyObject* threshold, const SelectArgs& a, const Place& at_) {
+// rounded (mask only, 16-bit types): set to the sums in that type, written by the same kernel.
+Selection select(const Tensor& sums, PyObject* threshold, const SelectArgs& a, const Place& at_, Tensor* rounded = nullptr) {
   const int64_t B = sums.size(0), H = sums.size(1), QB = sums.size(2), KB = a.band_kb > 0 ? a.band_kb : sums.size(3);
   if (a.band_kb > 0 && sums.size(3) != a.bpc) fail(PyExc_ValueError, "band sums must have blocks_per_chunk columns");
   Tensor thr;
@@ -205,6 +206,14 @@ Selection select(const Tensor& sums, PyObject* threshold, const SelectArgs& a, c
   if (a.list_q > 0) {
     r.idx = empty({B, H, lqb, lkb}, at::kInt, at_.dev);
     r.cnt = empty({B, H, lqb}, at::kInt, at_.dev);
+  }
+  if (rounded) {
+    check(xattn_b200_select_rounded(static_cast<const float*>(sums.data_ptr()), B, H, QB, KB, a.bpc, a.block_offset, a.causal, a.cleanup,
+                                    value, thr.defined() ? static_cast<const float*>(thr.data_ptr()) : nullptr, a.sink, a.recent,
+                                    static_cast<uint8_t*>(r.mask.data_ptr()), rounded->data_ptr(), dtype_code(rounded->scalar_type()),
+                                    at_.status, at_.stream),
+          "select_rounded");
+    return r;
   }
   auto fn = a.band_kb > 0 ? xattn_b200_select_band : xattn_b200_select;
   check(fn(static_cast<const float*>(sums.data_ptr()), B, H, QB, KB, a.bpc, a.block_offset, a.causal, a.cleanup, value,
@@ -413,10 +422,16 @@ PyObject* py_estimate_and_select(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   const Geometry g = geometry(q.size(2), k.size(2), e.chunk, e.stride, e.block);
   const bool f32 = q.scalar_type() == at::kFloat;
   const Tensor sums = estimate(q, k, g, e, nullptr, nullptr, at_);
-  const Selection s = select(sums, pv[8], {g.bpc, g.block_offset, e.causal, true, a.flag(9), a.flag(10), true, 0, 0, 0}, at_);
+  // the sums in q's type: rounded by the selection kernel where it holds a row in registers (up to 1024 key blocks)
+  Tensor result = sums;
+  const bool in_select = !f32 && sums.size(3) <= 1024;
+  if (in_select) result = empty(sums.sizes(), q.scalar_type(), at_.dev);
+  const Selection s = select(sums, pv[8], {g.bpc, g.block_offset, e.causal, true, a.flag(9), a.flag(10), true, 0, 0, 0}, at_,
+                             in_select ? &result : nullptr);
+  if (!f32 && !in_select) result = sums.to(q.scalar_type());
   PyObject* t = PyTuple_New(2);
   if (!t) throw python_error();
-  PyTuple_SET_ITEM(t, 0, wrap(f32 ? sums : sums.to(q.scalar_type())));
+  PyTuple_SET_ITEM(t, 0, wrap(result));
   PyTuple_SET_ITEM(t, 1, wrap(s.mask));
   return t;
   END_HANDLE_TH_ERRORS
