@@ -43,6 +43,14 @@ def test_query_shorter_than_the_keys(lq, lk, chunk, semantics):
     _check(4, 2, lq, lk, 16, chunk, True, torch.float16, semantics)
 
 
+@pytest.mark.parametrize("hq,hkv,lq,lk,stride,chunk", [(1, 1, 2600, 4096, 8, 2048), (28, 4, 5596, 8192, 16, 4096), (3, 1, 2100, 6144, 8, 2048),
+                                                       (7, 1, 413, 16384, 8, 8192)])
+def test_pair_of_a_row_tile_and_one_that_sees_nothing(hq, hkv, lq, lk, stride, chunk):
+    """Un-padded keys, chunks of 256 columns, an odd group: a CTA pair whose second row tile lies past the queries computes its
+    first one's column tile only, whose epilogue writes whole rows of the output."""
+    _check(hq, hkv, lq, lk, stride, chunk, True, torch.bfloat16)
+
+
 @pytest.mark.parametrize("hkv", [3, 1])
 @pytest.mark.parametrize("L,stride,chunk,causal", [(300, 16, 2048, True), (2048, 16, 2048, True), (2500, 8, 2048, False), (1900, 8, 2048, True),
                                                    (4096, 8, 4096, True), (5000, 16, 4096, True), (9001, 8, 16384, True), (8192, 4, 8192, True)])

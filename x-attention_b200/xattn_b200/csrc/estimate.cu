@@ -144,6 +144,11 @@ __host__ __device__ inline void row_tile_range(const EstGeom& g, int mt, int& fi
     count = hi_max / g.tile_n - lo_min / g.tile_n + 1;
   }
 }
+// Whether row tile mt counts in the column-tile range of its pair (2p, 2p + 1), the union of the two: the second one does not
+// if it sees nothing.  Its own range is then made up (the one tile that has its rows of the output zeroed, see EstGeom::direct)
+// and would add column tiles that the first one does not see, for each of which the epilogue would write the first one's rows
+// as zeros beside the sums of the right tile.  The first one's tile zeroes them as well.
+__host__ __device__ inline bool counts_in_pair(const EstGeom& g, int mt) { return mt % 2 == 0 || mt * kTileM < g.rows_valid; }
 
 // tile_lo[mt], tile_prefix[mt] (exclusive prefix of tile counts, n_mtiles+1 entries)
 __global__ void est_setup_kernel(EstGeom g, int* __restrict__ tile_lo, int* __restrict__ tile_prefix,
@@ -170,7 +175,7 @@ __global__ void est_setup_kernel(EstGeom g, int* __restrict__ tile_lo, int* __re
     for (int pm = 0; pm < n_pairs; ++pm) {
       int lo = 0x7fffffff, hi = -1;
       for (int mt = 2 * pm; mt < 2 * pm + 2 && mt < g.n_mtiles; ++mt)
-        if (s_cnt[mt] > 0) {
+        if (s_cnt[mt] > 0 && counts_in_pair(g, mt)) {
           lo = s_lo[mt] < lo ? s_lo[mt] : lo;
           hi = s_lo[mt] + s_cnt[mt] - 1 > hi ? s_lo[mt] + s_cnt[mt] - 1 : hi;
         }
@@ -1420,7 +1425,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       lo = 0x7fffffff;
       hi = -1;
     }
-    if (cnt > 0) {
+    if (cnt > 0 && counts_in_pair(g, mt)) {
       lo = first < lo ? first : lo;
       hi = first + cnt - 1 > hi ? first + cnt - 1 : hi;
     }
