@@ -1,0 +1,57 @@
+"""What the operators refuse on the host, before anything is launched, and odd forms of tensors that they take."""
+import pytest
+import torch
+
+import xattn_b200
+from xattn_b200 import api, llama_shim, ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(autouse=True)
+def _status_clean():
+    yield
+    xattn_b200.check_device_status()
+
+
+def _qkv(lq, lk, hq=4, hkv=2, batch=1, dtype=torch.bfloat16):
+    g = torch.Generator(device=DEV).manual_seed(lq + lk)
+    return [torch.randn(batch, h, n, 128, generator=g, device=DEV).to(dtype) for h, n in ((hq, lq), (hkv, lk), (hkv, lk))]
+
+
+def _calls(q, k, v):
+    """Every operator that makes its tensor maps from q's and k's sizes."""
+    cfg = llama_shim.FastPrefillConfig(0.9, num_heads=q.shape[1])
+    calls = [lambda: llama_shim.attention_core(q, k, v, 0, cfg)] if q.shape[2] == 1 else [
+        lambda: ops.block_sparse_attention(q, k, v, None, None, True), lambda: api.Xattention_prefill(q, k, v, 16)]
+    return calls
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("lq,which,dim,size", [(1, 1, 0, 1), (1, 2, 0, 1), *[(n, w, d, s) for n in (1, 300) for w, d, s in (
+    (2, 1, 0), (2, 1, 1), (2, 2, 200), (1, 3, 64), (2, 3, 64))]])
+def test_smaller_keys_or_values_are_refused(lq, which, dim, size, dtype):
+    """Keys or values (tensor 1, 2) whose batch, heads, length or head_dim is below what the call reads."""
+    t = _qkv(lq, 300, batch=2 if dim == 0 else 1, dtype=dtype)
+    t[which] = t[which].narrow(dim, 0, size)
+    for call in _calls(*t):
+        with pytest.raises(ValueError):
+            call()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("lq", [1, 300])
+def test_of_larger_values_the_leading_part_counts(lq, dtype):
+    q, k, v = _qkv(lq, 300, dtype=dtype)
+    longer = torch.full((2, 3, 345, 128), float("nan"), device=DEV, dtype=dtype)
+    longer[:1, :2, :300] = v
+    for call, want in zip(_calls(q, k, longer), _calls(q, k, v)):
+        assert torch.equal(call(), want())
+
+
+def test_lists_of_another_type_are_refused():
+    q, k, v = _qkv(300, 300)
+    idx, cnt = ops.mask_to_lists(torch.ones(1, 4, 3, 3, dtype=torch.bool, device=DEV), 300, 300, True)
+    with pytest.raises(ValueError):
+        ops.block_sparse_attention(q, k, v, idx.long(), cnt.long(), True)

@@ -74,6 +74,26 @@ void need_cuda(const Tensor& t) {
 void need_4d(const Tensor& t) {
   if (t.dim() != 4) fail(PyExc_ValueError, "tensors of four dimensions [batch, heads, length, head_dim] are wanted");
 }
+// `x` as the kernels read it: [batch, heads, len, dim] of the sizes that the call takes from q and k, on q's device.  What is
+// smaller would be read past its end; of what is larger the leading part counts.
+Tensor fit(const Tensor& x, int64_t batch, int64_t heads, int64_t len, int64_t dim, const Tensor& q, const char* name) {
+  if (x.device() != q.device()) {
+    PyErr_Format(PyExc_ValueError, "%s must be on the device of the query tensor", name);
+    throw python_error();
+  }
+  if (x.size(0) == batch && x.size(1) == heads && x.size(2) == len && x.size(3) == dim) return x;
+  if (x.size(0) < batch || x.size(1) < heads || x.size(2) < len || x.size(3) < dim) {
+    PyErr_Format(PyExc_ValueError, "%s is [%lld, %lld, %lld, %lld], at least [%lld, %lld, %lld, %lld] is wanted", name, (long long)x.size(0),
+                 (long long)x.size(1), (long long)x.size(2), (long long)x.size(3), (long long)batch, (long long)heads, (long long)len,
+                 (long long)dim);
+    throw python_error();
+  }
+  return x.narrow(0, 0, batch).narrow(1, 0, heads).narrow(2, 0, len).narrow(3, 0, dim);
+}
+Tensor fit_k(const Tensor& k, const Tensor& q) { return fit(k, q.size(0), k.size(1), k.size(2), q.size(3), q, "the key tensor"); }
+Tensor fit_v(const Tensor& v, const Tensor& k, const Tensor& q) {
+  return fit(v, q.size(0), k.size(1), k.size(2), q.size(3), q, "the value tensor");
+}
 // unit inner stride, 16-byte aligned rows; otherwise a contiguous copy
 Tensor aligned16(const Tensor& x) {
   const int64_t e = x.element_size();
@@ -270,8 +290,9 @@ PyObject* py_estimate(PyObject*, PyObject* const* v, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const Args a{v, n, "estimate"};
   a.count(9);
-  const Tensor &q = a.tensor(0), &k = a.tensor(1);
-  need_cuda(q); need_cuda(k); need_4d(q); need_4d(k);
+  const Tensor& q = a.tensor(0);
+  need_cuda(q); need_cuda(a.tensor(1)); need_4d(q); need_4d(a.tensor(1));
+  const Tensor k = fit_k(a.tensor(1), q);
   need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
   const Place at_(q);
   EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), a.flag(8)};
@@ -310,7 +331,7 @@ Tensor attention_any(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   if (f32) { q16 = q.to(at::kBFloat16); k16 = k.to(at::kBFloat16); v16 = v.to(at::kBFloat16); }
   if (dtype_code(q16.scalar_type()) < 0 || k16.scalar_type() != q16.scalar_type() || v16.scalar_type() != q16.scalar_type())
     fail(PyExc_TypeError, "q/k/v must share one of bf16, fp16, fp32");
-  if (out.defined() && (out.sizes() != q.sizes() || out.scalar_type() != q16.scalar_type() || out.stride(3) != 1 || !out.is_cuda()))
+  if (out.defined() && (out.sizes() != q.sizes() || out.scalar_type() != q16.scalar_type() || out.stride(3) != 1 || out.device() != q.device()))
     fail(PyExc_ValueError, "out must be a CUDA tensor [B,Hq,Lq,D] of the compute dtype with unit inner stride");
   const int64_t lqb = (q.size(2) + 127) / 128, lkb = (k.size(2) + 127) / 128;
   if (!dense && (idx.sizes() != at::IntArrayRef({q.size(0), q.size(1), lqb, lkb}) || cnt.sizes() != at::IntArrayRef({q.size(0), q.size(1), lqb})))
@@ -324,14 +345,19 @@ PyObject* py_attention(PyObject*, PyObject* const* v, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const Args a{v, n, "attention"};
   a.count(9);
-  const Tensor &q = a.tensor(0), &k = a.tensor(1), &vv = a.tensor(2);
+  const Tensor &q = a.tensor(0), &k_ = a.tensor(1), &v_ = a.tensor(2);
   Tensor idx, cnt, out;
   if (!a.none(3)) idx = a.tensor(3);
   if (!a.none(4)) cnt = a.tensor(4);
   if (idx.defined() != cnt.defined()) fail(PyExc_ValueError, "block lists have the wrong shape");
   if (!a.none(7)) out = a.tensor(7);
-  need_cuda(q); need_cuda(k); need_cuda(vv); need_4d(q); need_4d(k); need_4d(vv);
-  if (idx.defined()) { need_cuda(idx); need_cuda(cnt); }
+  need_cuda(q); need_cuda(k_); need_cuda(v_); need_4d(q); need_4d(k_); need_4d(v_);
+  const Tensor k = fit_k(k_, q), vv = fit_v(v_, k_, q);
+  if (idx.defined()) {
+    need_cuda(idx); need_cuda(cnt);
+    if (idx.device() != q.device() || cnt.device() != q.device() || idx.element_size() != 4 || cnt.element_size() != 4)
+      fail(PyExc_ValueError, "block lists are 32-bit integers on the device of the query tensor");
+  }
   const Place at_(q);
   const double scale = a.none(6) ? 1.0 / std::sqrt(static_cast<double>(q.size(3))) : a.real(6);
   std::optional<bool> ws;
@@ -345,8 +371,9 @@ PyObject* py_decode(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const Args a{pv, n, "decode"};
   a.count(4);
-  const Tensor &q_ = a.tensor(0), &k_ = a.tensor(1), &v_ = a.tensor(2);
-  need_cuda(q_); need_cuda(k_); need_cuda(v_); need_4d(q_); need_4d(k_); need_4d(v_);
+  const Tensor& q_ = a.tensor(0);
+  need_cuda(q_); need_cuda(a.tensor(1)); need_cuda(a.tensor(2)); need_4d(q_); need_4d(a.tensor(1)); need_4d(a.tensor(2));
+  const Tensor k_ = fit_k(a.tensor(1), q_), v_ = fit_v(a.tensor(2), k_, q_);
   const Place at_(q_);
   const int64_t B = q_.size(0), Hq = q_.size(1), D = q_.size(3), Hkv = k_.size(1), Lk = k_.size(2);
   const double scale = a.none(3) ? 1.0 / std::sqrt(static_cast<double>(D)) : a.real(3);
@@ -378,6 +405,8 @@ PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   need_cuda(q); need_4d(q); need_4d(k); need_4d(v);
   if (k.device() != q.device()) k = k.to(q.device());
   if (v.device() != q.device()) v = v.to(q.device());
+  v = fit_v(v, k, q);
+  k = fit_k(k, q);
   need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
   const Place at_(q);
   const int64_t Lq = q.size(2), Lk = k.size(2), D = q.size(3);
@@ -414,8 +443,9 @@ PyObject* py_estimate_and_select(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const Args a{pv, n, "estimate_and_select"};
   a.count(11);
-  const Tensor &q = a.tensor(0), &k = a.tensor(1);
-  need_cuda(q); need_cuda(k); need_4d(q); need_4d(k);
+  const Tensor& q = a.tensor(0);
+  need_cuda(q); need_cuda(a.tensor(1)); need_4d(q); need_4d(a.tensor(1));
+  const Tensor k = fit_k(a.tensor(1), q);
   need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
   const Place at_(q);
   const EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), false};
