@@ -4,6 +4,7 @@ import torch
 
 import xattn_b200
 from xattn_b200 import api, llama_shim, ops
+from xattn_b200._lib import XattnB200Error
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -55,3 +56,24 @@ def test_lists_of_another_type_are_refused():
     idx, cnt = ops.mask_to_lists(torch.ones(1, 4, 3, 3, dtype=torch.bool, device=DEV), 300, 300, True)
     with pytest.raises(ValueError):
         ops.block_sparse_attention(q, k, v, idx.long(), cnt.long(), True)
+
+
+def test_divisors_of_zero_raise():
+    """No key heads, a chunk of no tokens, a norm of zero: errors of Python, not of the process."""
+    q, k, v = _qkv(1, 300)
+    for kk, vv in ((k[:, :0], v[:, :0]), (k[:, :0], v)):
+        with pytest.raises(XattnB200Error):
+            ops.decode_attention(q, kk, vv)
+    q, k, v = _qkv(300, 300)
+    for chunk in (0, -128, 100):
+        with pytest.raises(XattnB200Error):
+            api.Xattention_prefill(q, k, v, 16, chunk_size=chunk)
+        with pytest.raises(XattnB200Error):
+            api.xattn_estimate(q, k, 128, 16, chunk_size=chunk)
+    with pytest.raises(XattnB200Error):
+        api.Xattention_prefill(q, k, v, 0)
+    for x in (q, q.float()):
+        with pytest.raises(ZeroDivisionError):
+            api.Xattention_prefill(x, k.to(x.dtype), v.to(x.dtype), 16, norm=0)
+        with pytest.raises(ZeroDivisionError):
+            api.xattn_estimate(x, k.to(x.dtype), 128, 16, norm=0)

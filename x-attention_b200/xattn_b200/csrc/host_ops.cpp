@@ -181,6 +181,7 @@ Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const Est
     fail(PyExc_ValueError, "unsupported estimate geometry (stride must be 4/8/16/32, block_size 128, chunk_size a multiple of 128)");
   const Tensor ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
   Tensor sums = empty({B, Hq, g.qb, a.band ? g.bpc : g.kb}, at::kFloat, at_.dev);
+  if (D == 0 || a.norm == 0.0) fail(PyExc_ZeroDivisionError, "the scale of the scores is 1 / (sqrt(head_dim) * stride * norm)");
   const double scale = 1.0 / std::sqrt(static_cast<double>(D)) / a.stride / a.norm;
   if (dtype == XATTN_B200_F32)
     check(xattn_b200_estimate_f32(static_cast<const float*>(q.data_ptr()), static_cast<const float*>(k.data_ptr()), B, Hq, Hkv, Lq, Lk, D,
@@ -378,7 +379,7 @@ PyObject* py_decode(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   const int64_t B = q_.size(0), Hq = q_.size(1), D = q_.size(3), Hkv = k_.size(1), Lk = k_.size(2);
   const double scale = a.none(3) ? 1.0 / std::sqrt(static_cast<double>(D)) : a.real(3);
   const int code = dtype_code(q_.scalar_type());
-  if (q_.size(2) != 1 || D != 128 || code < 0 || Hq % Hkv || Hq / Hkv > 16)      // what the decode kernel does not cover
+  if (q_.size(2) != 1 || D != 128 || code < 0 || Hkv == 0 || Hq % Hkv || Hq / Hkv > 16)      // what the decode kernel does not cover
     return wrap(attention_any(q_, k_, v_, Tensor(), Tensor(), true, scale, Tensor(), false, at_));
   if (k_.scalar_type() != q_.scalar_type() || v_.scalar_type() != q_.scalar_type())
     fail(PyExc_TypeError, "q/k/v must share one of bf16, fp16, fp32");
@@ -412,9 +413,9 @@ PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   const int64_t Lq = q.size(2), Lk = k.size(2), D = q.size(3);
   EstimateArgs e{(int)a.integer(3), (int)a.integer(6), a.none(8) ? xattn_b200_default_chunk_size(Lk) : (int)a.integer(8), (int)a.integer(11),
                  a.real(4), a.flag(7), false};
+  const Geometry g = geometry(Lq, Lk, e.chunk, e.stride, e.block);       // (refuses a chunk of no blocks)
   // un-padded causal keys under the torch branch: the sums outside a row's own chunk are zero and are not kept
   e.band = band_applies(Lk, e.chunk, e.causal, e.semantics);
-  const Geometry g = geometry(Lq, Lk, e.chunk, e.stride, e.block);
   Tensor out;
   if (!a.none(12)) out = a.tensor(12);
   // fp32: the attention phase computes with the bf16 roundings, those of q and k come from the estimate
