@@ -98,7 +98,7 @@ size_t xattn_b200_estimate_workspace_bytes_ex(int batch, int hq, int q_len, int 
  *
  * q_len / k_len need not be multiples of `stride`: the tokens a ragged last stride group lacks count as the
  * zeros the reference pads with (xattn/src/Xattention.py:42-51); no copy is made for them.  head_dim is a
- * multiple of 64;  `scale` = 1/(sqrt(D)*stride*norm).
+ * multiple of 64 (XATTN_B200_F32: of 32);  `scale` = 1/(sqrt(D)*stride*norm).
  * XATTN_B200_F32: every value is split on the way into three bf16 terms, x = hi + mid + lo to 2^-24, and the six products of
  * terms that reach 2^-24 are added (the reference's torch branch multiplies fp32 directly, xattn/src/Xattention.py:183).
  * XATTN_B200_F32_TERMS: the same from rows split before; only where xattn_b200_estimate_f32_terms says that this is the faster

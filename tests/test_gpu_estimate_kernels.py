@@ -60,6 +60,22 @@ def test_split_fp32_terms(L, stride, chunk, causal, hkv):
     _check(3, hkv, L, L, stride, chunk, causal, torch.float32)
 
 
+@pytest.mark.parametrize("D,dtype", [(32, torch.float32), (96, torch.float32), (192, torch.float32), (64, torch.bfloat16), (192, torch.float16)])
+@pytest.mark.parametrize("lq,lk,stride,chunk,causal", [(300, 300, 16, 2048, True), (1900, 2500, 8, 2048, True), (3000, 3000, 4, 1024, False),
+                                                       (8192, 8192, 8, 4096, True)])
+def test_other_head_dims(lq, lk, stride, chunk, causal, D, dtype):
+    """16-bit rows of any multiple of 64, fp32 rows of any multiple of 32: an odd number of 32-column steps per token."""
+    from xattn_b200 import ops
+    g = torch.Generator().manual_seed(D + lq)
+    q, k = torch.randn(1, 2, lq, D, generator=g).to(dtype), torch.randn(1, 1, lk, D, generator=g).to(dtype)
+    got = ops.estimate_block_sums(q.to(DEV), k.to(DEV), stride, 128, chunk, 1.0, causal).cpu()
+    want = orc.estimate_block_sums(q.float(), k.float().repeat_interleave(2, 1), 128, stride, 1.0, chunk, causal, "torch")
+    assert torch.allclose(got, want, rtol=RTOL, atol=ATOL), float((got - want).abs().max())
+    if dtype == torch.float32:
+        with pytest.raises(Exception, match="argument"):
+            ops.estimate_block_sums(q.to(DEV)[..., :24], k.to(DEV)[..., :24], stride, 128, chunk, 1.0, causal)
+
+
 @pytest.mark.parametrize("lq,lk,stride,chunk,causal,semantics", [
     (1003, 1003, 16, 2048, True, 0), (4096, 4096, 16, 2048, True, 2), (3000, 3000, 8, 4096, True, 1), (2000, 2500, 8, 2048, False, 0),
     (2048, 6144, 16, 2048, True, 2), (3, 5, 16, 2048, True, 0)])       # the last but one: keys that no tile reads

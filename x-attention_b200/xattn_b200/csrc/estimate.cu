@@ -1197,11 +1197,11 @@ struct EstWorkspace {
 };
 
 static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int head_dim, int stride, int block_size,
-                         int chunk_size, float scale, int causal, int semantics, EstGeom& g) {
+                         int chunk_size, float scale, int causal, int semantics, EstGeom& g, int step_cols = kTileK) {
   if (batch < 1 || hq < 1 || hkv < 1 || hq % hkv != 0 || q_len < 1 || k_len < 1) return XATTN_B200_ERR_ARG;
   if (stride != 4 && stride != 8 && stride != 16 && stride != 32) return XATTN_B200_ERR_ARG;
   if (block_size != 128 || chunk_size < block_size || chunk_size % block_size != 0) return XATTN_B200_ERR_ARG;
-  if (head_dim < kTileK || head_dim % kTileK != 0) return XATTN_B200_ERR_ARG;
+  if (head_dim < step_cols || head_dim % step_cols != 0) return XATTN_B200_ERR_ARG;
   const int k_pad = (chunk_size - k_len % chunk_size) % chunk_size;
   const int q_pad = (chunk_size - q_len % chunk_size) % chunk_size;
   const int lq = q_len + q_pad, lk = k_len + k_pad;
@@ -1210,7 +1210,7 @@ static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int h
   g.by_tiles = make_fast_div(1);
   g.by_group = make_fast_div(hq / hkv);
   g.by_hq = make_fast_div(hq);
-  g.S = stride; g.d_chunks = head_dim / kTileK;
+  g.S = stride; g.d_chunks = head_dim / step_cols;
   g.rows_total = lq / stride; g.cols_total = lk / stride;
   g.rows_valid = g.rows_total - q_pad / stride;
   g.cols_valid = g.cols_total - k_pad / stride;
@@ -1331,9 +1331,8 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   if (!(scale > 0.f)) return XATTN_B200_ERR_ARG;
   EstGeom g;
   int rc = fill_geometry(batch, hq, hkv, q_len, k_len, head_dim, stride, block_size, chunk_size, scale, causal,
-                         semantics, g);
+                         semantics, g, f32 ? kF32Cols : kTileK);
   if (rc) return rc;
-  if (f32) g.d_chunks = head_dim / kF32Cols;
   if (terms) {
     // (the terms are written for whole stride groups; geometries without CTA pairs take fp32 rows)
     if (q_len % stride || k_len % stride || !pairs_fit(g)) return XATTN_B200_ERR_ARG;

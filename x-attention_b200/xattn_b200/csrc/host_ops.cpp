@@ -95,12 +95,12 @@ Tensor fit_v(const Tensor& v, const Tensor& k, const Tensor& q) {
   return fit(v, q.size(0), k.size(1), k.size(2), q.size(3), q, "the value tensor");
 }
 // unit inner stride, 16-byte aligned rows; otherwise a contiguous copy
-Tensor aligned16(const Tensor& x) {
+bool is_aligned16(const Tensor& x) {
   const int64_t e = x.element_size();
-  const bool ok = x.stride(3) == 1 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 &&
-                  (x.stride(0) * e) % 16 == 0 && (x.stride(1) * e) % 16 == 0 && (x.stride(2) * e) % 16 == 0;
-  return ok ? x : x.contiguous();
+  return x.stride(3) == 1 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 && (x.stride(0) * e) % 16 == 0 &&
+         (x.stride(1) * e) % 16 == 0 && (x.stride(2) * e) % 16 == 0;
 }
+Tensor aligned16(const Tensor& x) { return is_aligned16(x) ? x : x.contiguous(); }
 Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Device& dev) {
   return at::detail::empty_cuda(sizes, type, dev, std::nullopt);
 }
@@ -151,11 +151,12 @@ struct EstimateArgs {
 // q16, k16 (fp32 inputs, null: not wanted): set to the bf16 roundings of q and k.
 Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const EstimateArgs& a, Tensor* q16, Tensor* k16, const Place& at_) {
   int dtype = q_.scalar_type() == at::kFloat ? XATTN_B200_F32 : dtype_code(q_.scalar_type());
-  Tensor q = aligned16(q_), k = aligned16(dtype == XATTN_B200_F32 && k_.scalar_type() != at::kFloat ? k_.to(at::kFloat) : k_);
+  const bool f32 = dtype == XATTN_B200_F32;
+  Tensor q = aligned16(q_), k = aligned16(f32 && k_.scalar_type() != at::kFloat ? k_.to(at::kFloat) : k_);
   const int64_t B = q.size(0), Hq = q.size(1), Hkv = k.size(1), D = q.size(3);
   int64_t Lq = q.size(2), Lk = k.size(2);
   const int sem = a.band ? XATTN_B200_SEMANTICS_TORCH_BAND : a.semantics;
-  if (dtype == XATTN_B200_F32 && xattn_b200_estimate_f32_terms(Hq, Hkv, Lq, Lk, a.stride, a.block, a.chunk, a.causal, sem)) {
+  if (f32 && D % 64 == 0 && xattn_b200_estimate_f32_terms(Hq, Hkv, Lq, Lk, a.stride, a.block, a.chunk, a.causal, sem)) {
     dtype = XATTN_B200_F32_TERMS;
     const auto split = [&](const Tensor& x) {
       const int64_t len = (x.size(2) + a.stride - 1) / a.stride * a.stride;
@@ -172,7 +173,7 @@ Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const Est
     if (k16) *k16 = k.narrow(3, 0, D).narrow(2, 0, Lk);
     Lq = q.size(2);
     Lk = k.size(2);
-  } else if (dtype == XATTN_B200_F32 && q16) {
+  } else if (f32 && q16) {
     *q16 = empty(q.sizes(), at::kBFloat16, at_.dev);
     *k16 = empty(k.sizes(), at::kBFloat16, at_.dev);
   }
