@@ -76,6 +76,27 @@ def test_other_head_dims(lq, lk, stride, chunk, causal, D, dtype):
             ops.estimate_block_sums(q.to(DEV)[..., :24], k.to(DEV)[..., :24], stride, 128, chunk, 1.0, causal)
 
 
+@pytest.mark.parametrize("L,chunk", [(900, 2048), (8192, 8192)])          # split in the GEMM, split before
+def test_fp32_operands_in_any_memory(L, chunk):
+    """fp32 tensors off a 16-byte boundary, of odd row strides, expanded or transposed: the results of contiguous copies, bit by
+    bit."""
+    from xattn_b200 import api, ops
+    g = torch.Generator(device=DEV).manual_seed(L)
+    flat = torch.randn(4 * L * 131 + 1, device=DEV, generator=g)
+    forms = [flat[1:1 + 4 * L * 128].view(1, 4, L, 128), flat[:4 * L * 131].view(1, 4, L, 131)[..., :128],
+             flat[:L * 128].view(1, 1, L, 128).expand(1, 4, L, 128), flat[:128].view(1, 1, 1, 128).expand(1, 4, L, 128),
+             flat[:4 * L * 128].view(1, 4, 128, L).transpose(2, 3)]
+    k = torch.randn(1, 4, L, 128, device=DEV, generator=g)
+    for x in forms:
+        for a, b in ((x, k), (k, x)):
+            got = ops.estimate_block_sums(a, b, 16, 128, chunk)
+            assert torch.equal(got, ops.estimate_block_sums(a.clone(memory_format=torch.contiguous_format),
+                                                            b.clone(memory_format=torch.contiguous_format), 16, 128, chunk))
+        out = api.Xattention_prefill(k, x, x, 16, chunk_size=chunk)
+        c = x.clone(memory_format=torch.contiguous_format)
+        assert torch.equal(out, api.Xattention_prefill(k, c, c, 16, chunk_size=chunk))
+
+
 @pytest.mark.parametrize("lq,lk,stride,chunk,causal,semantics", [
     (1003, 1003, 16, 2048, True, 0), (4096, 4096, 16, 2048, True, 2), (3000, 3000, 8, 4096, True, 1), (2000, 2500, 8, 2048, False, 0),
     (2048, 6144, 16, 2048, True, 2), (3, 5, 16, 2048, True, 0)])       # the last but one: keys that no tile reads

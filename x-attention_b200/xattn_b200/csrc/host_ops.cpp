@@ -101,6 +101,13 @@ bool is_aligned16(const Tensor& x) {
          (x.stride(1) * e) % 16 == 0 && (x.stride(2) * e) % 16 == 0;
 }
 Tensor aligned16(const Tensor& x) { return is_aligned16(x) ? x : x.contiguous(); }
+// The same for fp32 tensors, which any strides and any alignment will do for: what the tensor maps cannot express (rows of a
+// contiguous tensor that starts off a 16-byte boundary, expanded dimensions) is copied.
+Tensor aligned16_f32(const Tensor& x) {
+  bool ok = is_aligned16(x);
+  for (int i = 0; i < 3; ++i) ok = ok && (x.size(i) == 1 || x.stride(i) > 0);
+  return ok ? x : x.clone(at::MemoryFormat::Contiguous);
+}
 Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Device& dev) {
   return at::detail::empty_cuda(sizes, type, dev, std::nullopt);
 }
@@ -152,7 +159,7 @@ struct EstimateArgs {
 Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const EstimateArgs& a, Tensor* q16, Tensor* k16, const Place& at_) {
   int dtype = q_.scalar_type() == at::kFloat ? XATTN_B200_F32 : dtype_code(q_.scalar_type());
   const bool f32 = dtype == XATTN_B200_F32;
-  Tensor q = aligned16(q_), k = aligned16(f32 && k_.scalar_type() != at::kFloat ? k_.to(at::kFloat) : k_);
+  Tensor q = f32 ? aligned16_f32(q_) : aligned16(q_), k = f32 ? aligned16_f32(k_.scalar_type() != at::kFloat ? k_.to(at::kFloat) : k_) : aligned16(k_);
   const int64_t B = q.size(0), Hq = q.size(1), Hkv = k.size(1), D = q.size(3);
   int64_t Lq = q.size(2), Lk = k.size(2);
   const int sem = a.band ? XATTN_B200_SEMANTICS_TORCH_BAND : a.semantics;
