@@ -77,3 +77,12 @@ def test_divisors_of_zero_raise():
             api.Xattention_prefill(x, k.to(x.dtype), v.to(x.dtype), 16, norm=0)
         with pytest.raises(ZeroDivisionError):
             api.xattn_estimate(x, k.to(x.dtype), 128, 16, norm=0)
+
+
+@pytest.mark.parametrize("hq", [1, 4])
+def test_decode_step_of_odd_batch_and_head_strides(hq):
+    """A query whose strides of extent 1 are odd: a view of a longer row, contiguous as far as torch is concerned."""
+    q, k, v = _qkv(1, 300, hq=hq, hkv=1)
+    row = torch.randn(1, hq * 128 + 1, device=DEV).bfloat16()
+    odd = row.as_strided(q.shape, (hq * 128 + 1, 128 if hq > 1 else 129, 128, 1))
+    assert torch.equal(ops.decode_attention(odd, k, v), ops.decode_attention(odd.clone(), k, v))

@@ -339,6 +339,9 @@ int decode_launch(const void* q, const void* k, const void* v, int dtype, int ba
   if (!q || !k || !v || !out) return XATTN_B200_ERR_ARG;
   if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16) return XATTN_B200_ERR_ARG;
   if (head_dim != 128 || batch < 1 || hq < 1 || hkv < 1 || hq % hkv != 0 || k_len < 1 || !(scale > 0.f)) return XATTN_B200_ERR_ARG;
+  // a dimension of extent 1 never moves: its stride is no matter
+  if (batch == 1) qsb = osb = 0;
+  if (hq == 1) qsh = osh = 0;
   if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 3) || ((qsb | qsh | osb | osh) & 1)) return XATTN_B200_ERR_ARG;
   if (hq / hkv > kDecMaxRows || hkv > 65535 || batch > 65535) return XATTN_B200_ERR_LIMIT;
   int rc;
