@@ -284,8 +284,8 @@ int xattn_b200_block_sparse_attn_ws(const void* q, const void* k, const void* v,
 /*
  * Decode step: dense attention of one query token per sequence (q [batch, hq, 1, 128]) against its key cache, which it may
  * see completely.  Replaces the third-party single-query attention of the reference's Llama patch
- * (xattn/src/load_llama.py:188-197); the same result as the general kernel up to the summation order.  hq / hkv <= 16
- * (XATTN_B200_ERR_LIMIT otherwise: use xattn_b200_block_sparse_attn without lists).  The cache is split over the SMs; the
+ * (xattn/src/load_llama.py:188-197); the same result as the general kernel up to the summation order.  hq / hkv <= 16,
+ * batch and hkv <= 65535 (XATTN_B200_ERR_LIMIT otherwise: use xattn_b200_block_sparse_attn without lists).  The cache is split over the SMs; the
  * parts are merged through `workspace` (device memory, 16-byte aligned, contents irrelevant on entry; may be null where
  * xattn_b200_decode_workspace_bytes is 0).
  */

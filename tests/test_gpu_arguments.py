@@ -86,3 +86,11 @@ def test_decode_step_of_odd_batch_and_head_strides(hq):
     row = torch.randn(1, hq * 128 + 1, device=DEV).bfloat16()
     odd = row.as_strided(q.shape, (hq * 128 + 1, 128 if hq > 1 else 129, 128, 1))
     assert torch.equal(ops.decode_attention(odd, k, v), ops.decode_attention(odd.clone(), k, v))
+
+
+def test_decode_step_of_more_sequences_than_a_grid_dimension_holds():
+    q, k, v = _qkv(1, 2, hq=1, hkv=1, batch=65537)
+    out = ops.decode_attention(q, k, v)
+    want = torch.nn.functional.scaled_dot_product_attention(q[-5:].float(), k[-5:].float(), v[-5:].float())
+    # probabilities and outputs are rounded to bf16, 2^-9 relative each, of values up to about 5
+    assert (out[-5:].float() - want).abs().max() < 2e-2 and bool(torch.isfinite(out.float()).all())

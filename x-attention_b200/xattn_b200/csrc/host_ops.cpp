@@ -387,7 +387,8 @@ PyObject* py_decode(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   const int64_t B = q_.size(0), Hq = q_.size(1), D = q_.size(3), Hkv = k_.size(1), Lk = k_.size(2);
   const double scale = a.none(3) ? 1.0 / std::sqrt(static_cast<double>(D)) : a.real(3);
   const int code = dtype_code(q_.scalar_type());
-  if (q_.size(2) != 1 || D != 128 || code < 0 || Hkv == 0 || Hq % Hkv || Hq / Hkv > 16)      // what the decode kernel does not cover
+  // what the decode kernel does not cover (batch and kv heads are dimensions of its grid)
+  if (q_.size(2) != 1 || D != 128 || code < 0 || Hkv == 0 || Hq % Hkv || Hq / Hkv > 16 || B > 65535 || Hkv > 65535)
     return wrap(attention_any(q_, k_, v_, Tensor(), Tensor(), true, scale, Tensor(), false, at_));
   if (k_.scalar_type() != q_.scalar_type() || v_.scalar_type() != q_.scalar_type())
     fail(PyExc_TypeError, "q/k/v must share one of bf16, fp16, fp32");
