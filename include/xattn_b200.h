@@ -35,7 +35,7 @@ extern "C" {
 /* element types */
 #define XATTN_B200_BF16 0
 #define XATTN_B200_F16 1
-#define XATTN_B200_F32_TERMS 2    /* xattn_b200_estimate: rows of 3 * head_dim bf16 terms of fp32 values (xattn_b200_split_f32) */
+#define XATTN_B200_F32_TERMS 2    /* xattn_b200_estimate: rows of 3 * head_dim bf16 terms of fp32 values (xattn_b200_split_f32_terms) */
 #define XATTN_B200_F32 4          /* xattn_b200_estimate */
 #define XATTN_B200_BF16_OUT_F32 3   /* xattn_b200_block_sparse_attn[_ws]: bf16 inputs, fp32 output */
 
@@ -132,8 +132,18 @@ int xattn_b200_estimate_f32_terms(int hq, int hkv, int q_len, int k_len, int str
  * [batch, heads, len, terms*head_dim] bf16 with len >= len_valid, 16-byte aligned, the rows past len_valid zero (the
  * reference's zero padding, xattn/src/Xattention.py:42-51).
  */
+int xattn_b200_split_f32_terms(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t stride_b,
+                               int64_t stride_h, int64_t stride_l, int terms, void* out, void* cuda_stream);
+
+/*
+ * The same three terms laid out as rows of 6*head_dim, for a bf16 product over the widened rows by any GEMM
+ * (xattn_b200_estimate with XATTN_B200_BF16 and that head_dim included), which then reproduces the fp32 product to ~2^-24:
+ *   role 0 (query side): [hi, hi, mid, hi, lo, mid]     role 1 (key side): [hi, mid, hi, lo, hi, mid]
+ * Any head_dim; out contiguous [batch, heads, len, 6*head_dim] bf16.  No counterpart in the reference, and slower than
+ * XATTN_B200_F32, which writes no terms to memory.
+ */
 int xattn_b200_split_f32(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t stride_b,
-                         int64_t stride_h, int64_t stride_l, int terms, void* out, void* cuda_stream);
+                         int64_t stride_h, int64_t stride_l, int role, void* out, void* cuda_stream);
 
 /*
  * The estimate without a caller-supplied workspace.  No counterpart in the reference.

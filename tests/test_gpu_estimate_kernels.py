@@ -118,6 +118,31 @@ def test_bf16_roundings_of_fp32_operands(lq, lk, stride, chunk, causal, semantic
     assert torch.equal(q16, q.to(torch.bfloat16)) and torch.equal(k16, k.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("D", [5, 64, 128])
+def test_rows_of_six_terms(D):
+    """The widened rows of either side, bit by bit, and (head dimensions that the estimate takes) the product over them."""
+    from xattn_b200 import _lib, ops
+    lib = _lib.load()
+    B, H, L, padded, stream = 2, 3, 133, 136, torch.cuda.current_stream().cuda_stream
+    g = torch.Generator().manual_seed(D)
+    x = [torch.randn(B, H, L, D + 3, generator=g)[..., :D] for _ in range(2)]
+    wide = []
+    for role, order in ((0, (0, 0, 1, 0, 2, 1)), (1, (0, 1, 0, 2, 0, 1))):
+        d = x[role].to(DEV)
+        out = torch.full((B, H, padded, 6 * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+        _lib.check(lib.xattn_b200_split_f32(d.data_ptr(), B, H, padded, L, D, *d.stride()[:3], role, out.data_ptr(), stream), "split_f32")
+        hi = x[role].bfloat16()
+        mid = (x[role] - hi.float()).bfloat16()
+        terms = (hi, mid, (x[role] - hi.float() - mid.float()).bfloat16())
+        assert torch.equal(out[:, :, :L].cpu(), torch.cat([terms[t] for t in order], -1)) and not out[:, :, L:].any()
+        wide.append(out)
+    assert lib.xattn_b200_split_f32(d.data_ptr(), B, H, padded, L, D, *d.stride()[:3], 3, out.data_ptr(), stream) != 0
+    if D % 64 == 0:
+        got = ops.estimate_block_sums(wide[0], wide[1], 8, 128, 256, norm=(6 * D) ** -0.5 * D ** 0.5).cpu()
+        pad = [torch.nn.functional.pad(t, (0, 0, 0, padded - L)) for t in x]
+        assert torch.allclose(got, orc.estimate_block_sums(pad[0], pad[1], 128, 8, 1.0, 256, True, "torch"), rtol=RTOL, atol=ATOL)
+
+
 @pytest.mark.parametrize("lq,lk,stride,chunk", [(2304, 2304, 8, 256), (1152, 1664, 4, 128), (5120, 5120, 16, 2560), (768, 3840, 4, 768), (1280, 1280, 32, 640)])
 def test_dense_rows_of_a_few_chunks(lq, lk, stride, chunk):
     """Un-padded causal keys whose chunks are a tile or less each: the epilogue writes whole rows, zeros included; chunks that

@@ -1190,6 +1190,35 @@ split_f32_kernel(const float* __restrict__ x, int heads, int len, int len_valid,
   }
 }
 
+// The same terms as rows of 6 * D for a product over the widened rows, an element per thread (HBM-bound: 4 bytes read and 12
+// written).  role 0: [hi, hi, mid, hi, lo, mid], 1: [hi, mid, hi, lo, hi, mid].
+__global__ void __launch_bounds__(256)
+split_f32_role_kernel(const float* __restrict__ x, int heads, int len, int len_valid, int D, int64_t sb, int64_t sh, int64_t sl, int role,
+                      __nv_bfloat16* __restrict__ out, size_t total) {
+  pdl_launch_dependents();
+  pdl_wait();
+  for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < total;
+       e += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    const int d = static_cast<int>(e % D);
+    size_t rest = e / D;
+    const int l = static_cast<int>(rest % len);
+    rest /= len;
+    const int h = static_cast<int>(rest % heads);
+    const int b = static_cast<int>(rest / heads);
+    const float v = l < len_valid ? x[b * sb + h * sh + l * sl + d] : 0.f;
+    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+    const float left = v - __bfloat162float(hi);
+    const __nv_bfloat16 mid = __float2bfloat16_rn(left), lo = __float2bfloat16_rn(left - __bfloat162float(mid));
+    __nv_bfloat16* o = out + (e / D) * (6 * static_cast<size_t>(D)) + d;
+    o[0] = hi;
+    o[D] = role ? mid : hi;
+    o[2 * D] = role ? hi : mid;
+    o[3 * D] = role ? lo : hi;
+    o[4 * D] = role ? hi : lo;
+    o[5 * D] = mid;
+  }
+}
+
 // ------------------------------------------------------------------------------------ host side
 struct EstWorkspace {
   size_t off_tile_lo, off_tile_prefix, off_pair_lo, off_pair_prefix, off_mtile, off_partial;
@@ -1578,6 +1607,16 @@ int split_f32_launch(const float* x, int batch, int heads, int len, int len_vali
                             sh, sl, static_cast<uint4*>(out), total);
   };
   return terms == 3 ? launch(split_f32_kernel<3>) : launch(split_f32_kernel<1>);
+}
+
+int split_f32_role_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
+                          int64_t sl, int role, void* out, cudaStream_t stream) {
+  if (!x || !out || batch < 1 || heads < 1 || len < 1 || len_valid < 1 || len_valid > len || head_dim < 1 || (role != 0 && role != 1))
+    return XATTN_B200_ERR_ARG;
+  const size_t total = static_cast<size_t>(batch) * heads * len * head_dim, cap = 32 * static_cast<size_t>(sm_count());
+  const size_t blocks = (total + 255) / 256;
+  return launch_dependent(split_f32_role_kernel, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), dim3(256), 0, stream, x, heads, len,
+                          len_valid, head_dim, sb, sh, sl, role, static_cast<__nv_bfloat16*>(out), total);
 }
 
 }  // namespace xb

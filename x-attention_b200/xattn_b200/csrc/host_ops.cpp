@@ -168,9 +168,9 @@ Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const Est
     const auto split = [&](const Tensor& x) {
       const int64_t len = (x.size(2) + a.stride - 1) / a.stride * a.stride;
       Tensor t = empty({B, x.size(1), len, 3 * D}, at::kBFloat16, at_.dev);
-      check(xattn_b200_split_f32(static_cast<const float*>(x.data_ptr()), B, x.size(1), len, x.size(2), D, x.stride(0), x.stride(1),
+      check(xattn_b200_split_f32_terms(static_cast<const float*>(x.data_ptr()), B, x.size(1), len, x.size(2), D, x.stride(0), x.stride(1),
                                  x.stride(2), 3, t.data_ptr(), at_.stream),
-            "split_f32");
+            "split_f32_terms");
       return t;
     };
     q = split(q);
@@ -439,9 +439,9 @@ PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   if (f32) {
     const Tensor vc = v.stride(3) == 1 ? v : v.contiguous();
     const Tensor v16 = empty(v.sizes(), at::kBFloat16, at_.dev);
-    check(xattn_b200_split_f32(static_cast<const float*>(vc.data_ptr()), v.size(0), v.size(1), Lk, Lk, D, vc.stride(0), vc.stride(1),
+    check(xattn_b200_split_f32_terms(static_cast<const float*>(vc.data_ptr()), v.size(0), v.size(1), Lk, Lk, D, vc.stride(0), vc.stride(1),
                                vc.stride(2), 1, v16.data_ptr(), at_.stream),
-          "split_f32");
+          "split_f32_terms");
     return wrap(attention(q16, k16, v16, s.idx, s.cnt, e.causal, scale, out, true, default_workspace(e.causal, false, q), at_));
   }
   return wrap(attention_any(q, k, v, s.idx, s.cnt, e.causal, scale, out, std::nullopt, at_));
