@@ -3,6 +3,8 @@
 // A short call (a decode step, the prefill of a chat prompt) is bound by the host: in Python its plumbing took 40 to 100 us,
 // against 8 to 60 us of kernels.  These functions do the same work in a few microseconds.  They are plain CPython functions
 // on torch tensors, no operator registration and no dispatch; all of them enqueue on torch's current stream and return.
+// Once the arguments are read the interpreter lock is given back (without_gil): an allocation may wait for the device, and a
+// launch does while its queue is full; other Python threads run on meanwhile.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -12,8 +14,11 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <cmath>
+#include <cstdarg>
+#include <cstdio>
 #include <cstdlib>
 #include <optional>
+#include <string>
 
 #include "../../../include/xattn_b200.h"
 
@@ -25,14 +30,39 @@ PyObject* g_error = nullptr;        // XattnB200Error
 PyObject* g_status_of = nullptr;    // device index -> address of the device's status word
 int* g_status[64] = {};
 
-[[noreturn]] void fail(PyObject* type, const char* text) {
-  PyErr_SetString(type, text);
-  throw python_error();
+// An error on its way to Python, thrown with or without the interpreter lock (see END_PY).
+struct Refused {
+  PyObject* type;
+  std::string text;
+};
+[[noreturn]] void fail(PyObject* type, const char* format, ...) {
+  char text[256];
+  va_list args;
+  va_start(args, format);
+  std::vsnprintf(text, sizeof text, format, args);
+  va_end(args);
+  throw Refused{type, text};
 }
 void check(int code, const char* what) {
-  if (code == 0) return;
-  PyErr_Format(g_error, "%s: %s (status %d)", what, xattn_b200_error_string(code), code);
-  throw python_error();
+  if (code != 0) fail(g_error, "%s: %s (status %d)", what, xattn_b200_error_string(code), code);
+}
+#define BEGIN_PY HANDLE_TH_ERRORS try {
+#define END_PY                                      \
+  }                                                 \
+  catch (const Refused& r) {                        \
+    PyErr_SetString(r.type, r.text.c_str());        \
+    return nullptr;                                 \
+  }                                                 \
+  END_HANDLE_TH_ERRORS
+
+// f() without the interpreter lock: no Python object is touched in it (torch takes the lock itself where a tensor needs it)
+template <typename F>
+auto without_gil(F&& f) {
+  struct Release {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Release() { PyEval_RestoreThread(state); }
+  } release;
+  return f();
 }
 
 // ---------------------------------------------------------------------------------------------- arguments
@@ -41,10 +71,7 @@ struct Args {
   Py_ssize_t n;
   const char* name;
   void count(Py_ssize_t want) const {
-    if (n != want) {
-      PyErr_Format(PyExc_TypeError, "%s: %zd arguments, %zd wanted", name, n, want);
-      throw python_error();
-    }
+    if (n != want) fail(PyExc_TypeError, "%s: %zd arguments, %zd wanted", name, n, want);
   }
   const Tensor& tensor(int i) const {
     if (!THPVariable_Check(v[i])) fail(PyExc_TypeError, "a tensor is wanted");
@@ -77,17 +104,11 @@ void need_4d(const Tensor& t) {
 // `x` as the kernels read it: [batch, heads, len, dim] of the sizes that the call takes from q and k, on q's device.  What is
 // smaller would be read past its end; of what is larger the leading part counts.
 Tensor fit(const Tensor& x, int64_t batch, int64_t heads, int64_t len, int64_t dim, const Tensor& q, const char* name) {
-  if (x.device() != q.device()) {
-    PyErr_Format(PyExc_ValueError, "%s must be on the device of the query tensor", name);
-    throw python_error();
-  }
+  if (x.device() != q.device()) fail(PyExc_ValueError, "%s must be on the device of the query tensor", name);
   if (x.size(0) == batch && x.size(1) == heads && x.size(2) == len && x.size(3) == dim) return x;
-  if (x.size(0) < batch || x.size(1) < heads || x.size(2) < len || x.size(3) < dim) {
-    PyErr_Format(PyExc_ValueError, "%s is [%lld, %lld, %lld, %lld], at least [%lld, %lld, %lld, %lld] is wanted", name, (long long)x.size(0),
-                 (long long)x.size(1), (long long)x.size(2), (long long)x.size(3), (long long)batch, (long long)heads, (long long)len,
-                 (long long)dim);
-    throw python_error();
-  }
+  if (x.size(0) < batch || x.size(1) < heads || x.size(2) < len || x.size(3) < dim)
+    fail(PyExc_ValueError, "%s is [%lld, %lld, %lld, %lld], at least [%lld, %lld, %lld, %lld] is wanted", name, (long long)x.size(0),
+         (long long)x.size(1), (long long)x.size(2), (long long)x.size(3), (long long)batch, (long long)heads, (long long)len, (long long)dim);
   return x.narrow(0, 0, batch).narrow(1, 0, heads).narrow(2, 0, len).narrow(3, 0, dim);
 }
 Tensor fit_k(const Tensor& k, const Tensor& q) { return fit(k, q.size(0), k.size(1), k.size(2), q.size(3), q, "the key tensor"); }
@@ -205,6 +226,14 @@ Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const Est
   return sums;
 }
 
+struct Threshold {
+  Tensor per_head;              // undefined: `value` for all
+  double value;
+};
+Threshold threshold_of(const Args& a, int i) {
+  if (THPVariable_Check(a.v[i])) return {a.tensor(i), 0.0};
+  return {Tensor(), a.real(i)};
+}
 struct Selection {
   Tensor mask, idx, cnt;
 };
@@ -215,19 +244,16 @@ struct SelectArgs {
   int64_t band_kb;              // > 0: the sums are the chunk band of rows of that many key blocks
 };
 // rounded (mask only, 16-bit types): set to the sums in that type, written by the same kernel.
-Selection select(const Tensor& sums, PyObject* threshold, const SelectArgs& a, const Place& at_, Tensor* rounded = nullptr) {
+Selection select(const Tensor& sums, const Threshold& threshold, const SelectArgs& a, const Place& at_, Tensor* rounded = nullptr) {
   const int64_t B = sums.size(0), H = sums.size(1), QB = sums.size(2), KB = a.band_kb > 0 ? a.band_kb : sums.size(3);
   if (a.band_kb > 0 && sums.size(3) != a.bpc) fail(PyExc_ValueError, "band sums must have blocks_per_chunk columns");
   Tensor thr;
-  double value = 0.0;
-  if (THPVariable_Check(threshold)) {
-    thr = THPVariable_Unpack(threshold).detach();
+  const double value = threshold.value;
+  if (threshold.per_head.defined()) {
+    thr = threshold.per_head.detach();
     if (thr.device() != at_.dev || thr.scalar_type() != at::kFloat) thr = thr.to(at_.dev, at::kFloat);
     thr = thr.reshape({-1}).contiguous();
     if (thr.numel() != H) fail(PyExc_ValueError, "per-head threshold needs one entry per head");
-  } else {
-    value = PyFloat_AsDouble(threshold);
-    if (value == -1.0 && PyErr_Occurred()) throw python_error();
   }
   Selection r;
   if (a.want_mask) r.mask = empty({B, H, QB, KB}, at::kBool, at_.dev);
@@ -296,39 +322,43 @@ PyObject* wrap(Tensor t) { return t.defined() ? THPVariable_Wrap(std::move(t)) :
 
 // estimate(q, k, stride, block, chunk, norm, causal, semantics, band) -> sums
 PyObject* py_estimate(PyObject*, PyObject* const* v, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
+  BEGIN_PY
   const Args a{v, n, "estimate"};
   a.count(9);
-  const Tensor& q = a.tensor(0);
+  const Tensor q = a.tensor(0);
   need_cuda(q); need_cuda(a.tensor(1)); need_4d(q); need_4d(a.tensor(1));
   const Tensor k = fit_k(a.tensor(1), q);
   need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
   const Place at_(q);
-  EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), a.flag(8)};
+  const EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), a.flag(8)};
   const Geometry g = geometry(q.size(2), k.size(2), e.chunk, e.stride, e.block);
-  return wrap(estimate(q, k, g, e, nullptr, nullptr, at_));
-  END_HANDLE_TH_ERRORS
+  return wrap(without_gil([&] { return estimate(q, k, g, e, nullptr, nullptr, at_); }));
+  END_PY
 }
 
 // select(sums, bpc, block_offset, threshold, causal, cleanup, sink, recent, want_mask, list_q, list_k, band_kb) -> (mask, idx, cnt)
 PyObject* py_select(PyObject*, PyObject* const* v, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
+  BEGIN_PY
   const Args a{v, n, "select"};
   a.count(12);
   Tensor sums = a.tensor(0);
   need_cuda(sums); need_4d(sums);
-  if (sums.scalar_type() != at::kFloat) sums = sums.to(at::kFloat);
-  sums = sums.contiguous();
   const Place at_(sums);
-  Selection r = select(sums, v[3], {(int)a.integer(1), (int)a.integer(2), a.flag(4), a.flag(5), a.flag(6), a.flag(7), a.flag(8), a.integer(9),
-                                    a.integer(10), a.integer(11)}, at_);
+  const Threshold threshold = threshold_of(a, 3);
+  const SelectArgs sel{(int)a.integer(1), (int)a.integer(2), a.flag(4), a.flag(5), a.flag(6), a.flag(7), a.flag(8), a.integer(9), a.integer(10),
+                       a.integer(11)};
+  Selection r = without_gil([&] {
+    if (sums.scalar_type() != at::kFloat) sums = sums.to(at::kFloat);
+    sums = sums.contiguous();
+    return select(sums, threshold, sel, at_);
+  });
   PyObject* t = PyTuple_New(3);
   if (!t) throw python_error();
   PyTuple_SET_ITEM(t, 0, wrap(r.mask));
   PyTuple_SET_ITEM(t, 1, wrap(r.idx));
   PyTuple_SET_ITEM(t, 2, wrap(r.cnt));
   return t;
-  END_HANDLE_TH_ERRORS
+  END_PY
 }
 
 Tensor attention_any(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx, const Tensor& cnt, bool causal, double scale,
@@ -351,10 +381,10 @@ Tensor attention_any(const Tensor& q, const Tensor& k, const Tensor& v, const Te
 
 // attention(q, k, v, idx, cnt, causal, scale, out, use_workspace) -> out
 PyObject* py_attention(PyObject*, PyObject* const* v, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
+  BEGIN_PY
   const Args a{v, n, "attention"};
   a.count(9);
-  const Tensor &q = a.tensor(0), &k_ = a.tensor(1), &v_ = a.tensor(2);
+  const Tensor q = a.tensor(0), k_ = a.tensor(1), v_ = a.tensor(2);
   Tensor idx, cnt, out;
   if (!a.none(3)) idx = a.tensor(3);
   if (!a.none(4)) cnt = a.tensor(4);
@@ -371,16 +401,17 @@ PyObject* py_attention(PyObject*, PyObject* const* v, Py_ssize_t n) {
   const double scale = a.none(6) ? 1.0 / std::sqrt(static_cast<double>(q.size(3))) : a.real(6);
   std::optional<bool> ws;
   if (!a.none(8)) ws = a.flag(8);
-  return wrap(attention_any(q, k, vv, idx, cnt, a.flag(5), scale, out, ws, at_));
-  END_HANDLE_TH_ERRORS
+  const bool causal = a.flag(5);
+  return wrap(without_gil([&] { return attention_any(q, k, vv, idx, cnt, causal, scale, out, ws, at_); }));
+  END_PY
 }
 
 // decode(q, k, v, scale) -> out: one query token per sequence against its whole cache
 PyObject* py_decode(PyObject*, PyObject* const* pv, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
+  BEGIN_PY
   const Args a{pv, n, "decode"};
   a.count(4);
-  const Tensor& q_ = a.tensor(0);
+  const Tensor q_ = a.tensor(0);
   need_cuda(q_); need_cuda(a.tensor(1)); need_cuda(a.tensor(2)); need_4d(q_); need_4d(a.tensor(1)); need_4d(a.tensor(2));
   const Tensor k_ = fit_k(a.tensor(1), q_), v_ = fit_v(a.tensor(2), k_, q_);
   const Place at_(q_);
@@ -389,103 +420,110 @@ PyObject* py_decode(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   const int code = dtype_code(q_.scalar_type());
   // what the decode kernel does not cover (batch and kv heads are dimensions of its grid)
   if (q_.size(2) != 1 || D != 128 || code < 0 || Hkv == 0 || Hq % Hkv || Hq / Hkv > 16 || B > 65535 || Hkv > 65535)
-    return wrap(attention_any(q_, k_, v_, Tensor(), Tensor(), true, scale, Tensor(), false, at_));
+    return wrap(without_gil([&] { return attention_any(q_, k_, v_, Tensor(), Tensor(), true, scale, Tensor(), false, at_); }));
   if (k_.scalar_type() != q_.scalar_type() || v_.scalar_type() != q_.scalar_type())
     fail(PyExc_TypeError, "q/k/v must share one of bf16, fp16, fp32");
-  const Tensor q = aligned16(q_), k = aligned16(k_), v = aligned16(v_);
-  const size_t bytes = xattn_b200_decode_workspace_bytes(B, Hq, Hkv, Lk);
-  Tensor ws;
-  if (bytes) ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
-  Tensor out = empty({B, 1, Hq, D}, q.scalar_type(), at_.dev);
-  check(xattn_b200_decode_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), code, B, Hq, Hkv, Lk, D, q.stride(0), q.stride(1), k.stride(0),
-                               k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2), static_cast<float>(scale), out.data_ptr(),
-                               Hq * D, D, bytes ? ws.data_ptr() : nullptr, bytes, at_.status, at_.stream),
-        "decode_attn");
-  return wrap(out.transpose(1, 2));
-  END_HANDLE_TH_ERRORS
+  return wrap(without_gil([&] {
+    const Tensor q = aligned16(q_), k = aligned16(k_), v = aligned16(v_);
+    const size_t bytes = xattn_b200_decode_workspace_bytes(B, Hq, Hkv, Lk);
+    Tensor ws;
+    if (bytes) ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
+    Tensor out = empty({B, 1, Hq, D}, q.scalar_type(), at_.dev);
+    check(xattn_b200_decode_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), code, B, Hq, Hkv, Lk, D, q.stride(0), q.stride(1), k.stride(0),
+                                 k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2), static_cast<float>(scale), out.data_ptr(),
+                                 Hq * D, D, bytes ? ws.data_ptr() : nullptr, bytes, at_.status, at_.stream),
+          "decode_attn");
+    return out.transpose(1, 2);
+  }));
+  END_PY
 }
 
 // prefill(q, k, v, stride, norm, threshold, block, causal, chunk, sink, recent, semantics, out) -> out: all three phases
 PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
+  BEGIN_PY
   const Args a{pv, n, "prefill"};
   a.count(13);
-  const Tensor& q = a.tensor(0);
-  Tensor k = a.tensor(1), v = a.tensor(2);
+  const Tensor q = a.tensor(0);
+  Tensor k = a.tensor(1), v = a.tensor(2), out;
   need_cuda(q); need_4d(q); need_4d(k); need_4d(v);
-  if (k.device() != q.device()) k = k.to(q.device());
-  if (v.device() != q.device()) v = v.to(q.device());
-  v = fit_v(v, k, q);
-  k = fit_k(k, q);
-  need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
   const Place at_(q);
   const int64_t Lq = q.size(2), Lk = k.size(2), D = q.size(3);
   EstimateArgs e{(int)a.integer(3), (int)a.integer(6), a.none(8) ? xattn_b200_default_chunk_size(Lk) : (int)a.integer(8), (int)a.integer(11),
                  a.real(4), a.flag(7), false};
-  const Geometry g = geometry(Lq, Lk, e.chunk, e.stride, e.block);       // (refuses a chunk of no blocks)
-  // un-padded causal keys under the torch branch: the sums outside a row's own chunk are zero and are not kept
-  e.band = band_applies(Lk, e.chunk, e.causal, e.semantics);
-  Tensor out;
+  const Threshold threshold = threshold_of(a, 5);
+  const bool sink = a.flag(9), recent = a.flag(10);
   if (!a.none(12)) out = a.tensor(12);
-  // fp32: the attention phase computes with the bf16 roundings, those of q and k come from the estimate
-  const bool f32 = q.scalar_type() == at::kFloat && D == 128 && !out.defined() && v.scalar_type() == at::kFloat;
-  Tensor q16, k16;
-  Selection s;
-  {
-    const Tensor sums = estimate(q, k, g, e, f32 ? &q16 : nullptr, f32 ? &k16 : nullptr, at_);
-    s = select(sums, pv[5], {g.bpc, g.block_offset, e.causal, true, a.flag(9), a.flag(10), false, Lq, Lk, e.band ? g.kb : 0}, at_);
-  }
-  const double scale = 1.0 / std::sqrt(static_cast<double>(D));
-  if (f32) {
+  return wrap(without_gil([&] {
+    if (k.device() != q.device()) k = k.to(q.device());
+    if (v.device() != q.device()) v = v.to(q.device());
+    v = fit_v(v, k, q);
+    k = fit_k(k, q);
+    need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
+    const Geometry g = geometry(Lq, Lk, e.chunk, e.stride, e.block);       // (refuses a chunk of no blocks)
+    // un-padded causal keys under the torch branch: the sums outside a row's own chunk are zero and are not kept
+    e.band = band_applies(Lk, e.chunk, e.causal, e.semantics);
+    // fp32: the attention phase computes with the bf16 roundings, those of q and k come from the estimate
+    const bool f32 = q.scalar_type() == at::kFloat && D == 128 && !out.defined() && v.scalar_type() == at::kFloat;
+    Tensor q16, k16;
+    Selection s;
+    {
+      const Tensor sums = estimate(q, k, g, e, f32 ? &q16 : nullptr, f32 ? &k16 : nullptr, at_);
+      s = select(sums, threshold, {g.bpc, g.block_offset, e.causal, true, sink, recent, false, Lq, Lk, e.band ? g.kb : 0}, at_);
+    }
+    const double scale = 1.0 / std::sqrt(static_cast<double>(D));
+    if (!f32) return attention_any(q, k, v, s.idx, s.cnt, e.causal, scale, out, std::nullopt, at_);
     const Tensor vc = v.stride(3) == 1 ? v : v.contiguous();
     const Tensor v16 = empty(v.sizes(), at::kBFloat16, at_.dev);
     check(xattn_b200_split_f32_terms(static_cast<const float*>(vc.data_ptr()), v.size(0), v.size(1), Lk, Lk, D, vc.stride(0), vc.stride(1),
-                               vc.stride(2), 1, v16.data_ptr(), at_.stream),
+                                     vc.stride(2), 1, v16.data_ptr(), at_.stream),
           "split_f32_terms");
-    return wrap(attention(q16, k16, v16, s.idx, s.cnt, e.causal, scale, out, true, default_workspace(e.causal, false, q), at_));
-  }
-  return wrap(attention_any(q, k, v, s.idx, s.cnt, e.causal, scale, out, std::nullopt, at_));
-  END_HANDLE_TH_ERRORS
+    return attention(q16, k16, v16, s.idx, s.cnt, e.causal, scale, out, true, default_workspace(e.causal, false, q), at_);
+  }));
+  END_PY
 }
 
 // estimate_and_select(q, k, stride, block, chunk, norm, causal, semantics, threshold, sink, recent) -> (sums in q's type, mask)
 PyObject* py_estimate_and_select(PyObject*, PyObject* const* pv, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
+  BEGIN_PY
   const Args a{pv, n, "estimate_and_select"};
   a.count(11);
-  const Tensor& q = a.tensor(0);
+  const Tensor q = a.tensor(0);
   need_cuda(q); need_cuda(a.tensor(1)); need_4d(q); need_4d(a.tensor(1));
   const Tensor k = fit_k(a.tensor(1), q);
   need_16bit_or_f32(q, k, "q/k must both be bf16, fp16 or fp32");
   const Place at_(q);
   const EstimateArgs e{(int)a.integer(2), (int)a.integer(3), (int)a.integer(4), (int)a.integer(7), a.real(5), a.flag(6), false};
   const Geometry g = geometry(q.size(2), k.size(2), e.chunk, e.stride, e.block);
-  const bool f32 = q.scalar_type() == at::kFloat;
-  const Tensor sums = estimate(q, k, g, e, nullptr, nullptr, at_);
-  // the sums in q's type: rounded by the selection kernel where it holds a row in registers (up to 1024 key blocks)
-  Tensor result = sums;
-  const bool in_select = !f32 && sums.size(3) <= 1024;
-  if (in_select) result = empty(sums.sizes(), q.scalar_type(), at_.dev);
-  const Selection s = select(sums, pv[8], {g.bpc, g.block_offset, e.causal, true, a.flag(9), a.flag(10), true, 0, 0, 0}, at_,
-                             in_select ? &result : nullptr);
-  if (!f32 && !in_select) result = sums.to(q.scalar_type());
+  const Threshold threshold = threshold_of(a, 8);
+  const bool sink = a.flag(9), recent = a.flag(10);
+  Tensor result;
+  Selection s = without_gil([&] {
+    const bool f32 = q.scalar_type() == at::kFloat;
+    const Tensor sums = estimate(q, k, g, e, nullptr, nullptr, at_);
+    // the sums in q's type: rounded by the selection kernel where it holds a row in registers (up to 1024 key blocks)
+    const bool in_select = !f32 && sums.size(3) <= 1024;
+    result = in_select ? empty(sums.sizes(), q.scalar_type(), at_.dev) : sums;
+    Selection r = select(sums, threshold, {g.bpc, g.block_offset, e.causal, true, sink, recent, true, 0, 0, 0}, at_, in_select ? &result : nullptr);
+    if (!f32 && !in_select) result = sums.to(q.scalar_type());
+    return r;
+  });
   PyObject* t = PyTuple_New(2);
   if (!t) throw python_error();
   PyTuple_SET_ITEM(t, 0, wrap(result));
   PyTuple_SET_ITEM(t, 1, wrap(s.mask));
   return t;
-  END_HANDLE_TH_ERRORS
+  END_PY
 }
 
 // init(error class, status word callback)
 PyObject* py_init(PyObject*, PyObject* const* v, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
+  BEGIN_PY
   const Args a{v, n, "init"};
   a.count(2);
   g_error = Py_NewRef(v[0]);
   g_status_of = Py_NewRef(v[1]);
   Py_RETURN_NONE;
-  END_HANDLE_TH_ERRORS
+  END_PY
 }
 
 PyMethodDef methods[] = {
