@@ -97,6 +97,15 @@ def test_fp32_operands_in_any_memory(L, chunk):
         assert torch.equal(out, api.Xattention_prefill(k, c, c, 16, chunk_size=chunk))
 
 
+def test_ring_of_fp32_units_under_load():
+    """Units go from the converters back to TMA thousands of times per call: repeated calls agree bit by bit."""
+    from xattn_b200 import ops
+    q, k = (torch.randn(1, 16, 4096, 128, device=DEV, generator=torch.Generator(device=DEV).manual_seed(s)) for s in (1, 2))
+    first = ops.estimate_block_sums(q, k, 16, 128, 2048)
+    for _ in range(100):
+        assert torch.equal(ops.estimate_block_sums(q, k, 16, 128, 2048), first)
+
+
 @pytest.mark.parametrize("lq,lk,stride,chunk,causal,semantics", [
     (1003, 1003, 16, 2048, True, 0), (4096, 4096, 16, 2048, True, 2), (3000, 3000, 8, 4096, True, 1), (2000, 2500, 8, 2048, False, 0),
     (2048, 6144, 16, 2048, True, 2), (3, 5, 16, 2048, True, 0)])       # the last but one: keys that no tile reads

@@ -178,6 +178,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       warp_mma<kBf16>(o[2 * c], pa, vb[0], vb[1]);
       warp_mma<kBf16>(o[2 * c + 1], pa, vb[2], vb[3]);
     }
+    if (i + kDecStages < n) fence_proxy_async_smem();      // every lane's reads of the stage come before the TMA writes that refill it
     __syncwarp();
     if (lane == 0) mbar_arrive(empty0 + 8 * st);
     if (threadIdx.x == 0 && i > 0 && i - 1 + kDecStages < n) {

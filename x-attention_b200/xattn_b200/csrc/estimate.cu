@@ -634,20 +634,21 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const int out_len = out ? (n < 0 ? rounded.q_len : rounded.k_len) : 0;
           const int token = ((n < 0 ? mt * kTileM : nt * g.tile_n + n) + row0) * g.S + (n < 0 ? g.S - 1 - t : t);
 #pragma unroll
-          for (int i = 0; i < kGroups; ++i) {
+          for (int i = 0; i < kGroups; ++i)
 #pragma unroll
             for (int e = 0; e < 3; ++e) st_shared_v4(dst + i * 8 * 128 + e * stage_bytes, term[e][i]);
-            if (token + i * 8 * g.S < out_len) out[static_cast<size_t>(token + i * 8 * g.S) * row_vecs + dc * 4] = term[0][i];
-          }
-          // The unit goes back after the stores of its terms, which need what was read: an arrival right behind the reads has been
-          // seen to overtake a part of one (the MMAs take shared memory first), and the next unit to land in between.
+          // The unit goes back to TMA, which writes through the async proxy: a proxy fence of every lane orders its reads before
+          // that.  (Without one, an arrival right behind the reads gave wrong terms.)  It orders the lane's stores of terms before
+          // the MMAs' reads, too, the last unit's those of the whole step.
+          fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(empty0 + 8 * s);
           if (++s == n_stages) { s = 0; ph ^= 1; }
+#pragma unroll
+          for (int i = 0; i < kGroups; ++i)
+            if (token + i * 8 * g.S < out_len) out[static_cast<size_t>(token + i * 8 * g.S) * row_vecs + dc * 4] = term[0][i];
         }
         if (!ok) break;
-        fence_proxy_async_smem();
-        __syncwarp();
         if (lane == 0) mbar_arrive(terms_full0 + 8 * half);
         if (++half == 2) { half = 0; half_ph ^= 1; }
         if (++dc == g.d_chunks) { dc = 0; ++t; }
