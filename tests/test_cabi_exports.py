@@ -44,6 +44,17 @@ def test_host_only_entry_points(lib):
     assert lib.xattn_b200_estimate_workspace_bytes(1, 32, 4096, 4096, 3, 128, 2048) == 0       # bad stride
 
 
+def test_workspace_bytes_cover_every_mask_and_semantics(lib):
+    for stride in (4, 8, 16, 32):
+        for chunk in (128, 256, 384, 640, 1024, 1152, 2048, 4096):
+            for nq, extra, ragged in ((1, 0, 0), (1, 1, 0), (2, 0, 5), (3, 0, 0), (3, 2, 100), (8, 0, 0)):
+                q, k = nq * chunk - ragged, (nq + extra) * chunk - ragged
+                most = lib.xattn_b200_estimate_workspace_bytes(1, 8, q, k, stride, 128, chunk)
+                for causal, semantics in ((0, 0), (0, 1), (1, 0), (1, 1), (1, 2)):
+                    need = lib.xattn_b200_estimate_workspace_bytes_ex(1, 8, q, k, stride, 128, chunk, causal, semantics)
+                    assert need <= most, (stride, chunk, q, k, causal, semantics)
+
+
 def test_ops_refuse_cpu_tensors():
     import torch
     from xattn_b200 import Xattention_prefill

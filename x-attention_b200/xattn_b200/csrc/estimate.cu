@@ -1302,23 +1302,17 @@ static EstWorkspace workspace_layout(const EstGeom& g) {
 // Scratch of one estimate call: exact for the given mask and semantics, or (causal < 0) enough for any.
 size_t estimate_workspace_bytes(int batch, int hq, int q_len, int k_len, int stride, int block_size, int chunk_size,
                                 int causal, int semantics) {
-  EstGeom g;
-  const int ql = q_len, kl = k_len;      // (head_dim 128 and hkv = hq assumed for the staging tiles of ragged lengths)
-  if (causal >= 0) {
-    if (fill_geometry(batch, hq, hq, ql, kl, 128, stride, block_size, chunk_size, 1.f, causal, semantics, g) !=
-        XATTN_B200_OK)
-      return 0;
-    return workspace_layout(g).total;
-  }
-  size_t need = 0;
-  for (int c = 0; c < 2; ++c) {
-    if (fill_geometry(batch, hq, hq, ql, kl, 128, stride, block_size, chunk_size, 1.f, c, c ? XATTN_B200_SEMANTICS_TRITON : 0, g) !=
-        XATTN_B200_OK)
-      return 0;
-    const size_t t = workspace_layout(g).total;
-    need = t > need ? t : need;
-  }
-  return need;
+  auto bytes = [&](int c, int sem) -> size_t {           // (neither head_dim nor hkv changes the layout)
+    EstGeom g;
+    const int rc = fill_geometry(batch, hq, hq, q_len, k_len, 128, stride, block_size, chunk_size, 1.f, c, sem, g);
+    return rc == XATTN_B200_OK ? workspace_layout(g).total : 0;
+  };
+  if (causal >= 0) return bytes(causal, semantics);
+  // The causal torch layout is the compact one, and not always the smaller: chunks of one and a half 128-column tiles make row
+  // tiles span two of them where the other layouts have a single 256-column tile.
+  const size_t need[] = {bytes(0, XATTN_B200_SEMANTICS_TORCH), bytes(1, XATTN_B200_SEMANTICS_TRITON), bytes(1, XATTN_B200_SEMANTICS_TORCH)};
+  const size_t most = need[0] > need[1] ? need[0] : need[1];
+  return most > need[2] ? most : need[2];
 }
 
 int split_f32_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
