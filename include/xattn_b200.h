@@ -152,13 +152,14 @@ int xattn_b200_split_f32(const float* x, int batch, int heads, int len, int len_
  * GPU memory was handed out at start-up to a pool that this caller does not own, a plugin host that
  * forbids allocation after initialisation, or a latency-critical section where an allocation (and the
  * device synchronisation it can imply) is not acceptable.  The scratch that xattn_b200_estimate takes
- * from the caller lives here in a fixed array inside the library image, XATTN_B200_STATIC_SCRATCH_BYTES
- * large, resident on every GPU that loads the library until the process exits.  The call itself
+ * from the caller lives here in a fixed array inside the library image (36 MiB), resident on every GPU that loads the library until the process exits.  The call itself
  * allocates and frees nothing; the caller still provides q, k and attn_sums.
  *
  * Arguments and results are those of xattn_b200_estimate (minus workspace/workspace_bytes).
- * Returns XATTN_B200_ERR_LIMIT when xattn_b200_estimate_workspace_bytes_ex(...) for the call exceeds
- * XATTN_B200_STATIC_SCRATCH_BYTES -- use xattn_b200_estimate with your own workspace then.
+ * Returns XATTN_B200_ERR_LIMIT when the partial results of the call's rows (a row is `stride` tokens of a head) exceed
+ * XATTN_B200_STATIC_SCRATCH_BYTES, at 4 bytes per key block and 8 per 256 columns -- use xattn_b200_estimate with your
+ * own workspace then.  Rows are padded to whole tiles; a call that fits without its padding only goes in slices of heads,
+ * one after the other on the stream.
  *
  * The first call on each device looks up the array's device address (the device must be current, as
  * for every call); make that first call outside any CUDA stream capture.  All calls on a device share

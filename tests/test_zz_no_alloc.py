@@ -16,10 +16,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _call_static(lib, q, k, stride, chunk, causal, sums, status):
+def _call_static(lib, q, k, stride, chunk, causal, sums, status, dtype=0):
     B, H, L, D = q.shape
     return lib.xattn_b200_estimate_static(
-        q.data_ptr(), k.data_ptr(), 0, B, H, k.shape[1], L, k.shape[2], D,
+        q.data_ptr(), k.data_ptr(), dtype, B, H, k.shape[1], L, k.shape[2], D,
         q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2),
         stride, 128, chunk, 1.0 / math.sqrt(D) / stride, int(causal), 0,
         sums.data_ptr(), status.data_ptr(), torch.cuda.current_stream().cuda_stream)
@@ -44,6 +44,28 @@ def test_static_scratch_estimate_matches_regular_estimate_twice():
         assert int(status[0]) == 0
         # same kernels, same inputs, different scratch memory: identical within the sums tolerance
         assert torch.allclose(got, want, rtol=2e-4, atol=2e-5), (got - want).abs().max()
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,L,stride,chunk,causal,dtype", [
+    (8, 48, 6, 8160, 32, 640, True, torch.bfloat16),        # 74 MiB with the padding, 26 without: a batch entry at a time
+    (1, 36, 1, 20608, 16, 128, False, torch.bfloat16),      # 39 and 31 MiB: one kv group in two parts
+    (1, 36, 6, 20608, 16, 128, False, torch.float32)])      # the same in two slices of whole groups
+def test_static_scratch_estimate_in_slices_of_heads(B, Hq, Hkv, L, stride, chunk, causal, dtype):
+    """Calls that fit the scratch without their padding only: heads in slices, into their rows of the one output."""
+    from xattn_b200 import _lib, ops
+    lib = _lib.load()
+    dev = torch.device("cuda", 0)
+    assert lib.xattn_b200_estimate_workspace_bytes_ex(B, Hq, L, L, stride, 128, chunk, int(causal), 0) > (36 << 20)
+    g = torch.Generator(device=dev).manual_seed(L)
+    q, k = (torch.randn(B, L, h, 128, generator=g, device=dev, dtype=dtype).transpose(1, 2) for h in (Hq, Hkv))
+    want = ops.estimate_block_sums(q, k, stride, 128, chunk, 1.0, causal, semantics="torch")
+    got = torch.full_like(want, float("nan"))
+    status = torch.zeros(1, dtype=torch.int32).pin_memory()
+    rc = _call_static(lib, q, k, stride, chunk, causal, got, status, 4 if dtype == torch.float32 else 0)
+    assert rc == 0, lib.xattn_b200_error_string(rc)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    assert torch.allclose(got, want, rtol=2e-4, atol=2e-5), (got - want).abs().max()
 
 
 def test_static_scratch_estimate_refuses_oversized_problems():

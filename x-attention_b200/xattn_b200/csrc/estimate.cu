@@ -1315,6 +1315,15 @@ size_t estimate_workspace_bytes(int batch, int hq, int q_len, int k_len, int str
   return most > need[2] ? most : need[2];
 }
 
+// Of that, what the rows of the call take without their padding to whole tiles (0: refused arguments).
+size_t estimate_row_bytes(int batch, int hq, int q_len, int k_len, int stride, int block_size, int chunk_size, int causal, int semantics) {
+  EstGeom g;
+  if (fill_geometry(batch, hq, hq, q_len, k_len, 128, stride, block_size, chunk_size, 1.f, causal, semantics, g) != XATTN_B200_OK) return 0;
+  const size_t pairs = g.compact ? g.m_pitch : (g.cols_total + kTileN - 1) / kTileN;
+  const size_t sums = g.compact ? pairs * (g.tile_n / g.rbs) : g.kb_total;
+  return static_cast<size_t>(batch) * hq * g.rows_total * (sizeof(float2) * pairs + sizeof(float) * sums);
+}
+
 int split_f32_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
                      int64_t sl, int terms, void* out, cudaStream_t stream);
 
