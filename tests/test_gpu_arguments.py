@@ -1,4 +1,8 @@
 """What the operators refuse on the host, before anything is launched, and odd forms of tensors that they take."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -94,3 +98,35 @@ def test_decode_step_of_more_sequences_than_a_grid_dimension_holds():
     want = torch.nn.functional.scaled_dot_product_attention(q[-5:].float(), k[-5:].float(), v[-5:].float())
     # probabilities and outputs are rounded to bf16, 2^-9 relative each, of values up to about 5
     assert (out[-5:].float() - want).abs().max() < 2e-2 and bool(torch.isfinite(out.float()).all())
+
+
+def test_a_failed_launch_is_not_reported_twice():
+    """A launch refused by the runtime (into a stream capture that a synchronisation has invalidated) fails its own call and
+    no later one.  In a process of its own: an abandoned capture is not for other tests to inherit."""
+    code = """
+import torch
+from xattn_b200 import _lib, ops
+lib = _lib.load()
+mask = torch.ones(1, 2, 3, 3, dtype=torch.uint8, device="cuda")
+idx, cnt = ops.mask_to_lists(mask, 300, 300, True)
+def call():
+    return lib.xattn_b200_mask_to_lists(mask.data_ptr(), 1, 2, 3, 3, 300, 300, 1, idx.data_ptr(), cnt.data_ptr(),
+                                        torch.cuda.current_stream().cuda_stream)
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.stream(torch.cuda.Stream()):
+    graph.capture_begin(capture_error_mode="global")
+    try:
+        torch.cuda.synchronize()
+    except RuntimeError:
+        pass
+    refused = call()
+    try:
+        graph.capture_end()
+    except RuntimeError:
+        pass
+print("codes", refused, call())
+"""
+    path = os.pathsep.join(p for p in sys.path if p)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120, env=dict(os.environ, PYTHONPATH=path))
+    assert "codes 3 0" in r.stdout, r.stdout + r.stderr

@@ -139,8 +139,8 @@ inline int launch_dependent_clusters(void (*kernel)(KArgs...), unsigned cluster,
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-  launch_counter().fetch_add(1, std::memory_order_relaxed);
-  return (e == cudaSuccess && cudaGetLastError() == cudaSuccess) ? XATTN_B200_OK : XATTN_B200_ERR_CUDA;
+  const int rc = launch_status();         // (in every case: it also clears the error, which the next launch would report as its own)
+  return e == cudaSuccess ? rc : XATTN_B200_ERR_CUDA;
 }
 template <typename... KArgs, typename... Args>
 inline int launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream,
