@@ -100,6 +100,17 @@ def test_decode_step_of_more_sequences_than_a_grid_dimension_holds():
     assert (out[-5:].float() - want).abs().max() < 2e-2 and bool(torch.isfinite(out.float()).all())
 
 
+def test_thresholds_are_what_float_takes():
+    q, k, v = _qkv(300, 300)
+    want = api.Xattention_prefill(q, k, v, 16, threshold=0.75)
+    for threshold in ("0.75", torch.full((4,), 0.75), torch.full((1, 4, 1), 0.75, device=DEV, dtype=torch.float64)):
+        assert torch.equal(api.Xattention_prefill(q, k, v, 16, threshold=threshold), want)
+    with pytest.raises(ValueError):
+        api.Xattention_prefill(q, k, v, 16, threshold="high")
+    with pytest.raises(TypeError):
+        api.Xattention_prefill(q, k, v, 16, threshold=None)
+
+
 def test_a_failed_launch_is_not_reported_twice():
     """A launch refused by the runtime (into a stream capture that a synchronisation has invalidated) fails its own call and
     no later one.  In a process of its own: an abandoned capture is not for other tests to inherit."""

@@ -84,8 +84,10 @@ struct Args {
     return x;
   }
   double real(int i) const {
-    const double x = PyFloat_AsDouble(v[i]);
-    if (x == -1.0 && PyErr_Occurred()) throw python_error();
+    PyObject* f = PyNumber_Float(v[i]);            // what float() takes
+    if (!f) throw python_error();
+    const double x = PyFloat_AS_DOUBLE(f);
+    Py_DECREF(f);
     return x;
   }
   bool flag(int i) const {
