@@ -106,6 +106,19 @@ def test_ring_of_fp32_units_under_load():
         assert torch.equal(ops.estimate_block_sums(q, k, 16, 128, 2048), first)
 
 
+@pytest.mark.parametrize("lq,lk", [(862, 1024), (1024, 1030), (12, 12)])
+def test_ragged_operands_of_other_head_dims_in_any_memory(lq, lk):
+    """16-bit rows of 64 or 192: off a 16-byte boundary, or with expanded heads."""
+    from xattn_b200 import ops
+    for D in (64, 192):
+        g = torch.Generator(device=DEV).manual_seed(D)
+        flat = torch.randn(2 * 1030 * D + 1, device=DEV, generator=g).bfloat16()
+        for q, k in ((flat[1:1 + 2 * lq * D].view(1, 2, lq, D), flat[:lk * D].view(1, 1, lk, D).expand(1, 2, lk, D)),
+                     (flat[:lq * D].view(1, 1, lq, D).expand(1, 2, lq, D), flat[1:1 + lk * D].view(1, 1, lk, D))):
+            want = ops.estimate_block_sums(q.clone(memory_format=torch.contiguous_format), k.clone(memory_format=torch.contiguous_format), 16, 128, 1024)
+            assert torch.equal(ops.estimate_block_sums(q, k, 16, 128, 1024), want)
+
+
 @pytest.mark.parametrize("lq,lk,stride,chunk,causal,semantics", [
     (1003, 1003, 16, 2048, True, 0), (4096, 4096, 16, 2048, True, 2), (3000, 3000, 8, 4096, True, 1), (2000, 2500, 8, 2048, False, 0),
     (2048, 6144, 16, 2048, True, 2), (3, 5, 16, 2048, True, 0)])       # the last but one: keys that no tile reads

@@ -124,9 +124,9 @@ bool is_aligned16(const Tensor& x) {
          (x.stride(1) * e) % 16 == 0 && (x.stride(2) * e) % 16 == 0;
 }
 Tensor aligned16(const Tensor& x) { return is_aligned16(x) ? x : x.contiguous(); }
-// The same for fp32 tensors, which any strides and any alignment will do for: what the tensor maps cannot express (rows of a
-// contiguous tensor that starts off a 16-byte boundary, expanded dimensions) is copied.
-Tensor aligned16_f32(const Tensor& x) {
+// The same for tensors which any strides and any alignment will do for: what the tensor maps cannot express (rows of a
+// contiguous tensor that starts off a 16-byte boundary, expanded dimensions) is copied, too.
+Tensor aligned16_any(const Tensor& x) {
   bool ok = is_aligned16(x);
   for (int i = 0; i < 3; ++i) ok = ok && (x.size(i) == 1 || x.stride(i) > 0);
   return ok ? x : x.clone(at::MemoryFormat::Contiguous);
@@ -182,7 +182,10 @@ struct EstimateArgs {
 Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const EstimateArgs& a, Tensor* q16, Tensor* k16, const Place& at_) {
   int dtype = q_.scalar_type() == at::kFloat ? XATTN_B200_F32 : dtype_code(q_.scalar_type());
   const bool f32 = dtype == XATTN_B200_F32;
-  Tensor q = f32 ? aligned16_f32(q_) : aligned16(q_), k = f32 ? aligned16_f32(k_.scalar_type() != at::kFloat ? k_.to(at::kFloat) : k_) : aligned16(k_);
+  // any memory: fp32, and 16-bit rows of another head_dim than 128 whose length is no multiple of the stride
+  const bool any = f32 || (q_.size(3) != 128 && (q_.size(2) % a.stride || k_.size(2) % a.stride));
+  auto operand = [&](const Tensor& x) { return any ? aligned16_any(x) : aligned16(x); };
+  Tensor q = operand(q_), k = operand(f32 && k_.scalar_type() != at::kFloat ? k_.to(at::kFloat) : k_);
   const int64_t B = q.size(0), Hq = q.size(1), Hkv = k.size(1), D = q.size(3);
   int64_t Lq = q.size(2), Lk = k.size(2);
   const int sem = a.band ? XATTN_B200_SEMANTICS_TORCH_BAND : a.semantics;
