@@ -115,3 +115,33 @@ def test_decode_ring_under_load():
     first = ops.decode_attention(q, k, v)
     for _ in range(100):
         assert torch.equal(ops.decode_attention(q, k, v), first)
+
+
+def test_calls_in_a_row_without_a_pause():
+    """The kernels of a call start before the ones in front of them have ended, and the lists lie where the estimate's scratch
+    has just been: calls of several shapes in a row give what each gives alone."""
+    from xattn_b200 import api
+    inputs = []
+    for i, (L, dtype) in enumerate([(1500, torch.bfloat16), (3000, torch.float16), (700, torch.float32), (5000, torch.bfloat16)]):
+        q, k, v = (x.to(DEV) for x in _qkv(i, 1, 4, 2, L, L, dtype))
+        inputs.append((q, k, v, 8, 1, 0.6, 128, True, i != 1, 1, 1024 if i < 2 else 2048))
+    want = []
+    for x in inputs:
+        want.append(api.Xattention_prefill(*x))
+        torch.cuda.synchronize()
+    for _ in range(100):
+        got = [api.Xattention_prefill(*x) for x in inputs]
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("count", [2 ** 30, -5, 4])
+def test_counts_beyond_a_row_of_the_lists(count):
+    """A count that no list can have is cut to the row of the lists (three blocks here), or to none."""
+    from xattn_b200 import ops
+    q, k, v = (x.to(DEV) for x in _qkv(7, 1, 4, 2, 300, 384))
+    idx, cnt = ops.mask_to_lists(torch.ones(1, 4, 3, 3, dtype=torch.bool, device=DEV), 300, 384, False)
+    want = ops.block_sparse_attention(q, k, v, idx, cnt, False)
+    for workspace in (False, True):
+        got = ops.block_sparse_attention(q, k, v, idx, torch.full_like(cnt, count), False, use_workspace=workspace)
+        assert torch.equal(got, want if count > 0 else torch.zeros_like(want))

@@ -82,7 +82,7 @@ __device__ __forceinline__ Tile unit_tile(const AttnParams& p, int u, int s) {
   if (kList && p.tile_list) {
     t.b = t.h = 0;
     t.qb = -1;
-    const int i = 2 * u + s < p.list_tiles ? __ldg(p.tile_list + 2 * u + s) : -1;
+    const int i = 2 * u + s < p.list_tiles ? ld_written(p.tile_list + 2 * u + s) : -1;
     if (i < 0) return t;
     const int rest = fast_div(i, p.by_hq, t.h);
     t.qb = p.q_blocks - 1 - fast_div(rest, p.by_batch, t.b);
@@ -102,7 +102,10 @@ __device__ __forceinline__ Tile unit_tile(const AttnParams& p, int u, int s) {
 // number of listed blocks; a dense call lists every block that holds a key the tile's last row may see
 __device__ __forceinline__ int tile_count(const AttnParams& p, const int32_t* __restrict__ block_cnt, const Tile& t) {
   if (t.qb < 0) return 0;
-  if (block_cnt) return __ldg(block_cnt + tile_row(p, t));
+  if (block_cnt) {
+    const int n = ld_written(block_cnt + tile_row(p, t));
+    return n < 0 ? 0 : (n < p.list_k_blocks ? n : p.list_k_blocks);      // (a list is read from its end: never past its row)
+  }
   if (!p.causal) return p.list_k_blocks;
   int last = t.qb * 128 + 127;
   last = (last < p.q_len - 1 ? last : p.q_len - 1) + p.k_len - p.q_len;
@@ -124,11 +127,9 @@ __device__ __forceinline__ List tile_list(const AttnParams& p, const int32_t* __
 __device__ __forceinline__ int list_entry(const List& l, int j) {
   if (j >= l.n) return 0;
   if (!l.last) return l.n - 1 - j;
-  // volatile asm pins the issue point: a plain read-only load would be sunk by the compiler to its first use,
-  // which turns the intended prefetch into an exposed memory latency
-  int v;
-  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(l.last - j));
-  return v;
+  // (its volatile asm also pins the issue point: a plain load would be sunk by the compiler to its first use, which turns
+  // the intended prefetch into an exposed memory latency)
+  return ld_written(l.last - j);
 }
 
 // Reader of the published units.
@@ -820,7 +821,7 @@ attn_order_kernel(const AttnParams p, const int32_t* __restrict__ block_cnt, int
   // blocks listed by the whole call; a unit with more than an eighth of one SM's share of them is a very long one
   const int rows = p.batch * p.hq * p.q_blocks;
   unsigned long long sum = 0;
-  for (int i = tid; i < rows; i += kOrderThreads) sum += static_cast<unsigned>(__ldg(block_cnt + i));
+  for (int i = tid; i < rows; i += kOrderThreads) sum += static_cast<unsigned>(ld_written(block_cnt + i));
   atomicAdd(&s_blocks, sum);
   __syncthreads();
   unsigned long long lim64 = s_blocks / (8ull * sms);

@@ -174,7 +174,7 @@ block_sparse_attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __g
 #endif
 
   // this launch's share of the list: entries list_offset + blockIdx.x + i * gridDim.x, at most kPairSchedCap
-  const int total = __ldg(counter);
+  const int total = ld_written(counter);
   const int G = gridDim.x;
   int n_local = 0;
   {
@@ -184,7 +184,11 @@ block_sparse_attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __g
       n_local = static_cast<int>(avail < kPairSchedCap ? avail : kPairSchedCap);
     }
   }
-  for (int i = threadIdx.x; i < n_local; i += kPairThreads) sch[i] = list[list_offset + blockIdx.x + i * G];
+  for (int i = threadIdx.x; i < n_local; i += kPairThreads) {
+    const int32_t* e = reinterpret_cast<const int32_t*>(list + list_offset + blockIdx.x + i * G);
+    sch[i].unit = ld_written(e);
+    sch[i].blocks = static_cast<uint32_t>(ld_written(e + 1));
+  }
   if (threadIdx.x == 0) {
     mbar_init(gbar(K_FULL), 1);
     mbar_init(gbar(K_EMPTY), 2);

@@ -105,7 +105,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int r = r0 + 8 * (e & 1), c = c0 + 16 * k + 8 * (e >> 1);
-        qa[k][e] = r < p.group ? __ldg(reinterpret_cast<const uint32_t*>(qg + r * p.qsh + c)) : 0u;
+        qa[k][e] = r < p.group ? ld_written(reinterpret_cast<const uint32_t*>(qg + r * p.qsh + c)) : 0u;
       }
   }
   float o[16][4];
@@ -294,14 +294,14 @@ decode_merge_kernel(const DecodeParams p, const float* __restrict__ part, const 
   const int g = h / p.group, r = h - g * p.group;
   const size_t row0 = static_cast<size_t>(b * p.hkv + g) * p.splits * p.group + r;
   float mm = -INFINITY;
-  for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, part_ml[row0 + static_cast<size_t>(s) * p.group].x);
+  for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, ld_written(part_ml + row0 + static_cast<size_t>(s) * p.group).x);
   float a = 0.f, ll = 0.f;
 #pragma unroll 8
   for (int s = 0; s < p.splits; ++s) {
     const size_t row = row0 + static_cast<size_t>(s) * p.group;
-    const float2 ml = part_ml[row];
+    const float2 ml = ld_written(part_ml + row);
     const float f = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - mm);
-    a += part[row * 128 + threadIdx.x] * f;
+    a += ld_written(part + row * 128 + threadIdx.x) * f;
     ll += ml.y * f;
   }
   const float v = ll > 0.f ? a / ll : 0.f;

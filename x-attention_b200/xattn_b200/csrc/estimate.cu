@@ -1081,7 +1081,7 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
       const bool in = kl < n_out && k >= 0 && k < k_end;
 #pragma unroll
       for (int j = 0; j < RBS / 4; ++j)
-        p4[u][j] = in ? __ldcs(reinterpret_cast<const float4*>(pp + static_cast<size_t>(k) * kTileM) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        p4[u][j] = in ? ld_written_once(reinterpret_cast<const float4*>(pp + static_cast<size_t>(k) * kTileM) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
   fetch(tid);
@@ -1100,7 +1100,7 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
     if (valid) {
 #pragma unroll 4
       for (int t = part; t < ncnt; t += kParts) {
-        const float2 x = ms[t * kTileM + row];
+        const float2 x = ld_written(ms + t * kTileM + row);
         add(x.x, x.y);
       }
     }
@@ -1126,7 +1126,7 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
       fetch(tid);
     }
     for (int t = t0 + tid / RBS; t < t1; t += kParts) {
-      const float x = ms[t * kTileM + tid % RBS].x;
+      const float x = ld_written(ms + t * kTileM + tid % RBS).x;
       s_f[(t - t0) * RBS + tid % RBS] = row_inv > 0.f && x > -INFINITY ? exp2f(x - row_m) * row_inv : 0.f;
     }
     sync();
@@ -1178,11 +1178,11 @@ split_f32_kernel(const float* __restrict__ x, int heads, int len, int len_valid,
     if (l < len_valid) {
       const float* row = x + b * sb + h * sh + l * sl + d * 8;
       if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
-        const float4 a = __ldcs(reinterpret_cast<const float4*>(row)), c = __ldcs(reinterpret_cast<const float4*>(row) + 1);
+        const float4 a = ld_written_once(reinterpret_cast<const float4*>(row)), c = ld_written_once(reinterpret_cast<const float4*>(row) + 1);
         v[0] = pack_f32x2(a.x, a.y); v[1] = pack_f32x2(a.z, a.w); v[2] = pack_f32x2(c.x, c.y); v[3] = pack_f32x2(c.z, c.w);
       } else {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = pack_f32x2(row[2 * k], row[2 * k + 1]);
+        for (int k = 0; k < 4; ++k) v[k] = pack_f32x2(ld_written(row + 2 * k), ld_written(row + 2 * k + 1));
       }
     }
     uint4* o = out + (e / vecs) * (static_cast<size_t>(kTerms) * vecs) + d;
@@ -1206,7 +1206,7 @@ split_f32_role_kernel(const float* __restrict__ x, int heads, int len, int len_v
     rest /= len;
     const int h = static_cast<int>(rest % heads);
     const int b = static_cast<int>(rest / heads);
-    const float v = l < len_valid ? x[b * sb + h * sh + l * sl + d] : 0.f;
+    const float v = l < len_valid ? ld_written(x + b * sb + h * sh + l * sl + d) : 0.f;
     const __nv_bfloat16 hi = __float2bfloat16_rn(v);
     const float left = v - __bfloat162float(hi);
     const __nv_bfloat16 mid = __float2bfloat16_rn(left), lo = __float2bfloat16_rn(left - __bfloat162float(mid));

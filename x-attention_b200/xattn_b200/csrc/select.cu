@@ -173,13 +173,13 @@ __global__ void __launch_bounds__(256) select_kernel(const float* __restrict__ s
       for (int e = 0; e < 4; ++e) vv[u][e] = 0.f;
       if (p.vec_in) {
         if (j < n_read) {
-          const float4 q = __ldg(reinterpret_cast<const float4*>(x + j));
+          const float4 q = ld_written(reinterpret_cast<const float4*>(x + j));
           vv[u][0] = q.x; vv[u][1] = q.y; vv[u][2] = q.z; vv[u][3] = q.w;
         }
       } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (j + e < n_read) vv[u][e] = __ldg(x + j + e);
+          if (j + e < n_read) vv[u][e] = ld_written(x + j + e);
       }
     }
 #pragma unroll
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(256) select_reg_kernel(const float* __restrict
   const int n_read = p.band ? p.bpc : N;
   const int col0 = p.band ? cur : 0;
   const float* x = sums + static_cast<size_t>(w) * n_read;
-  const double thr = thr_per_head ? static_cast<double>(__ldg(thr_per_head + bh % p.heads)) : p.threshold;
+  const double thr = thr_per_head ? static_cast<double>(ld_written(thr_per_head + bh % p.heads)) : p.threshold;
 
   // ---- the row, once; scores as bit patterns (positive floats order like integers), forced and non-positive ones as 0
   uint32_t v[4 * kVec];
@@ -520,12 +520,12 @@ __global__ void __launch_bounds__(256) select_reg_kernel(const float* __restrict
     const int j = u * 128 + 4 * lane;
     float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
     if (p.vec_in) {
-      if (j < n_read) q = __ldg(reinterpret_cast<const float4*>(x + j));
+      if (j < n_read) q = ld_written(reinterpret_cast<const float4*>(x + j));
     } else {
-      if (j < n_read) q.x = __ldg(x + j);
-      if (j + 1 < n_read) q.y = __ldg(x + j + 1);
-      if (j + 2 < n_read) q.z = __ldg(x + j + 2);
-      if (j + 3 < n_read) q.w = __ldg(x + j + 3);
+      if (j < n_read) q.x = ld_written(x + j);
+      if (j + 1 < n_read) q.y = ld_written(x + j + 1);
+      if (j + 2 < n_read) q.z = ld_written(x + j + 2);
+      if (j + 3 < n_read) q.w = ld_written(x + j + 3);
     }
     v[4 * u] = __float_as_uint(q.x); v[4 * u + 1] = __float_as_uint(q.y);
     v[4 * u + 2] = __float_as_uint(q.z); v[4 * u + 3] = __float_as_uint(q.w);
@@ -762,7 +762,7 @@ __global__ void mask_to_lists_kernel(const uint8_t* __restrict__ mask, int rows_
   int base = 0;
   for (int j0 = 0; j0 < list_k_blocks; j0 += 32) {
     const int j = j0 + lane;
-    const int keep = (j < list_k_blocks && mrow[j] && list_keeps(causal, R, j, q_len, k_len)) ? 1 : 0;
+    const int keep = (j < list_k_blocks && ld_written(mrow + j) && list_keeps(causal, R, j, q_len, k_len)) ? 1 : 0;
     const unsigned bal = __ballot_sync(0xffffffffu, keep);
     if (keep) lrow[base + __popc(bal & ((1u << lane) - 1u))] = j;
     base += __popc(bal);
