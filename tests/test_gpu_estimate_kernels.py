@@ -186,3 +186,21 @@ def test_many_query_blocks(stride, hkv, chunk, causal, semantics):
         want = orc.estimate_block_sums(q[:, h:h + 1].float(), k[:, h * hkv // hq:h * hkv // hq + 1].float(), 128, stride, 1.0, chunk, causal,
                                        semantics)
         assert torch.allclose(got[:, h:h + 1], want, rtol=RTOL, atol=ATOL), float((got[:, h:h + 1] - want).abs().max())
+
+
+@pytest.mark.parametrize("lq,lk,stride,chunk,causal", [(3, 3, 32, 2048, True), (1, 5, 16, 16384, False), (413, 4096, 8, 2048, True),
+                                                       (2500, 2500, 4, 8192, False), (1000, 1000, 16, 2048, True)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_operands_at_the_end_of_their_memory(dtype, lq, lk, stride, chunk, causal):
+    """Nothing past the end of q and k is named by a load: both end where an allocation of their own does (its size a multiple
+    of what the allocator maps), stored as a projection leaves them.  Lengths below the stride, row and column tiles past the
+    end, a ragged last group."""
+    from xattn_b200 import ops
+    hq, hkv = 9, 3
+    ends = []
+    for h, n in ((hq, lq), (hkv, lk)):
+        memory = torch.zeros((64 << 20) // torch.finfo(dtype).bits * 8, dtype=dtype, device=DEV)
+        ends.append(memory[-n * h * 128:].view(1, n, h, 128).transpose(1, 2))
+        ends[-1].copy_(torch.randn(1, h, n, 128, generator=torch.Generator().manual_seed(n)).to(dtype))
+    got = ops.estimate_block_sums(*ends, stride, 128, chunk, 1.0, causal)
+    assert torch.equal(got, ops.estimate_block_sums(*(x.clone() for x in ends), stride, 128, chunk, 1.0, causal))

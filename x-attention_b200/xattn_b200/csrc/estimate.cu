@@ -73,9 +73,11 @@ struct EstGeom {
   // touches the tiles of its own chunk): the column tiles [tile_lo, tile_lo + m_pitch) of the row tile.
   int compact, m_pitch;
   // Lengths that are no multiple of the stride: the last stride group lacks the tokens of offset >= len % stride, which
-  // count as zeros.  Two tensor maps of each operand: token offsets below the remainder go through one that has that group,
-  // the others through one that ends before it (no group at all: the coordinate is moved past the only one).
-  int q_rem, k_rem, q_none, k_none;
+  // count as zeros.  Two tensor maps of each operand: token offsets below the remainder go through one that has that group (and
+  // no other offsets), the others through one of the whole groups (see load_tile).
+  int q_rem, k_rem;
+  int q_groups, k_groups;      // whole stride groups
+  int row_cols;                // columns of the maps
   int head_dim;
   float scale_log2;
   // Tile tables of est_setup_kernel computed on the host and carried in the kernel parameters when they are small
@@ -115,6 +117,23 @@ __device__ __forceinline__ int k_column(const EstGeom& g, int dc) {
   if (g.term_chunks == 0) return dc * kTileK;
   const int c = dc / 3, term = dc - 3 * c;
   return (term * g.term_chunks + c) * kTileK;
+}
+
+// Loads a box of rows [row, row + box) of one token offset; `n_rows`: those that the map has of that offset.  A box without any
+// of them is zeros, and is taken from past the columns of the tensor's first row: its own coordinates are out of bounds all the
+// same, but name an address that can be far behind the tensor (3 tokens of 9 fp32 heads at stride 32: up to 290 KiB), and such
+// loads have raised memory faults where nothing is mapped there.
+template <bool kPair>
+__device__ __forceinline__ void load_tile(const EstGeom& g, uint32_t dst, const CUtensorMap* m, uint32_t bar, int col, int offset, int row, int h,
+                                          int b, int n_rows, uint32_t lead) {
+  const bool in = row < n_rows;
+  col = in ? col : g.row_cols;
+  offset = in ? offset : 0;
+  row = in ? row : 0;
+  h = in ? h : 0;
+  b = in ? b : 0;
+  if constexpr (kPair) tma_load_5d_pair_lead(dst, m, bar, col, offset, row, h, b, lead);
+  else tma_load_5d_lead(dst, m, bar, col, offset, row, h, b, lead);
 }
 
 // first column tile of a row tile's scratch, and the number of its tile (bh, mt, nt)
@@ -515,9 +534,9 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               const uint32_t dst = smem_u32(smem + 3 * stage_bytes + s * kF32Unit);
               mbar_expect_tx_lead(full0 + 8 * s, kF32Unit, lead);
               if (n < 0)
-                tma_load_5d_lead(dst, qt ? &tmQt : &tmQ, full0 + 8 * s, dc * kF32Cols, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
+                load_tile<false>(g, dst, qt ? &tmQt : &tmQ, full0 + 8 * s, dc * kF32Cols, g.S - 1 - t, mt * kTileM, h, b, g.q_groups + qt, lead);
               else
-                tma_load_5d_lead(dst, kt ? &tmKt : &tmK, full0 + 8 * s, dc * kF32Cols, t, nt * g.tile_n + n + (kt ? 0 : g.k_none), hkv, b, lead);
+                load_tile<false>(g, dst, kt ? &tmKt : &tmK, full0 + 8 * s, dc * kF32Cols, t, nt * g.tile_n + n, hkv, b, g.k_groups + kt, lead);
               if (++s == n_stages) { s = 0; ph ^= 1; }
             }
             if (!ok) break;
@@ -525,8 +544,8 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag))) break;
             const uint32_t dstA = smem_u32(smem + s * stage_bytes);
             mbar_expect_tx_lead(full0 + 8 * s, stage_bytes, lead);
-            tma_load_5d_lead(dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, dc * kTileK, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
-            tma_load_5d_lead(dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, dc * kTileK, t, nt * g.tile_n + (kt ? 0 : g.k_none), hkv, b, lead);
+            load_tile<false>(g, dstA, qt ? &tmQt : &tmQ, full0 + 8 * s, dc * kTileK, g.S - 1 - t, mt * kTileM, h, b, g.q_groups + qt, lead);
+            load_tile<false>(g, dstA + kABytes, kt ? &tmKt : &tmK, full0 + 8 * s, dc * kTileK, t, nt * g.tile_n, hkv, b, g.k_groups + kt, lead);
             if (++s == n_stages) { s = 0; ph ^= 1; }
           }
           if (++dc == g.d_chunks) { dc = 0; ++t; }
@@ -896,11 +915,11 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           mbar_expect_tx_lead(full0 + 8 * s, stage_bytes, rank == 0 ? lead : 0u);
           const bool qt = g.S - 1 - t < g.q_rem, kt = t < g.k_rem;
           const int col = k_column(g, dc);
-          tma_load_5d_pair_lead(dstA, qt ? &tmQt : &tmQ, full_even, col, g.S - 1 - t, mt * kTileM + (qt ? 0 : g.q_none), h, b, lead);
-          const int k_col = col0 + (kt ? 0 : g.k_none);                        // (B in boxes of 64 columns)
-          tma_load_5d_pair_lead(dstA + kABytes, kt ? &tmKt : &tmKh, full_even, col, t, k_col, hkv, b, lead);
-          tma_load_5d_pair_lead(dstA + kABytes + kPairBBytes / 2, kt ? &tmKt : &tmKh, full_even, col, t, k_col + 64, hkv, b,
-                                narrow ? 0u : lead);
+          load_tile<true>(g, dstA, qt ? &tmQt : &tmQ, full_even, col, g.S - 1 - t, mt * kTileM, h, b, g.q_groups + qt, lead);
+          // (B in boxes of 64 columns)
+          load_tile<true>(g, dstA + kABytes, kt ? &tmKt : &tmKh, full_even, col, t, col0, hkv, b, g.k_groups + kt, lead);
+          load_tile<true>(g, dstA + kABytes + kPairBBytes / 2, kt ? &tmKt : &tmKh, full_even, col, t, col0 + 64, hkv, b, g.k_groups + kt,
+                          narrow ? 0u : lead);
           if (++dc == g.d_chunks) { dc = 0; ++t; }
           if (++s == kPairStages) { s = 0; ph ^= 1; }
         }
@@ -1265,8 +1284,9 @@ static int fill_geometry(int batch, int hq, int hkv, int q_len, int k_len, int h
   g.term_chunks = 0;
   g.q_rem = q_len % stride;
   g.k_rem = k_len % stride;
-  g.q_none = q_len < stride ? 1 : 0;
-  g.k_none = k_len < stride ? 1 : 0;
+  g.q_groups = q_len / stride;
+  g.k_groups = k_len / stride;
+  g.row_cols = head_dim;
   g.direct = 0;
   g.split = 1;
   g.pair_heads = 0;
@@ -1369,6 +1389,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   if (terms) {
     // (the terms are written for whole stride groups; geometries without CTA pairs take fp32 rows)
     if (q_len % stride || k_len % stride || !pairs_fit(g)) return XATTN_B200_ERR_ARG;
+    g.row_cols = 3 * head_dim;
     g.term_chunks = g.d_chunks;
     g.d_chunks *= 3;
   }
@@ -1389,11 +1410,12 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   float2* mtile = reinterpret_cast<float2*>(ws + w.off_mtile);
   float* partial = reinterpret_cast<float*>(ws + w.off_partial);
 
-  // 5-D views [head_dim, S, len/S, heads, batch] whose second coordinate picks the token inside a stride group; `up`: with
-  // the ragged last group (see EstGeom::q_rem)
-  auto make_map = [&](CUtensorMap* m, const void* x, int len, int heads, int64_t sb, int64_t sh, int64_t sl, uint32_t box_rows, bool up) -> int {
-    const int groups = len / stride > 0 && !up ? len / stride : (len + stride - 1) / stride;
-    const uint64_t dims[5] = {(uint64_t)head_dim * (terms ? 3 : 1), (uint64_t)stride, (uint64_t)groups, (uint64_t)heads, (uint64_t)batch};
+  // 5-D views [head_dim, S, len/S, heads, batch] whose second coordinate picks the token inside a stride group; `tail`: with
+  // the ragged last group and the token offsets it has (see EstGeom::q_rem).  No map describes a token that does not exist.
+  auto make_map = [&](CUtensorMap* m, const void* x, int len, int heads, int64_t sb, int64_t sh, int64_t sl, uint32_t box_rows, bool tail) -> int {
+    if (len < stride) tail = true;                       // (no whole group: the map is never loaded from in its bounds)
+    const int offsets = tail ? len % stride : stride, groups = len / stride + (tail ? 1 : 0);
+    const uint64_t dims[5] = {(uint64_t)g.row_cols, (uint64_t)offsets, (uint64_t)groups, (uint64_t)heads, (uint64_t)batch};
     // a dimension of extent 1 never moves: give it a harmless valid stride
     const uint64_t e = f32 ? 4 : 2;
     const uint64_t str[4] = {(uint64_t)sl * e, (uint64_t)sl * e * stride, heads > 1 ? (uint64_t)sh * e : 256, batch > 1 ? (uint64_t)sb * e : 256};
