@@ -101,12 +101,18 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
     const uint16_t* qg = q + b * p.qsb + static_cast<int64_t>(g) * p.group * p.qsh;
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
+    for (int h = 0; h < 2; ++h) {
+      const int r = r0 + 8 * h;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = r0 + 8 * (e & 1), c = c0 + 16 * k + 8 * (e >> 1);
-        qa[k][e] = r < p.group ? ld_written(reinterpret_cast<const uint32_t*>(qg + r * p.qsh + c)) : 0u;
+      for (int k = 0; k < 8; ++k) qa[k][h] = qa[k][2 + h] = 0u;
+      if (r < p.group) {
+        const uint16_t* row = qg + r * p.qsh + c0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) qa[k][2 * e + h] = ld_written(reinterpret_cast<const uint32_t*>(row + 16 * k + 8 * e));
       }
+    }
   }
   float o[16][4];
 #pragma unroll
@@ -293,16 +299,34 @@ decode_merge_kernel(const DecodeParams p, const float* __restrict__ part, const 
   const int b = blockIdx.x / hq, h = blockIdx.x - b * hq;
   const int g = h / p.group, r = h - g * p.group;
   const size_t row0 = static_cast<size_t>(b * p.hkv + g) * p.splits * p.group + r;
+  constexpr int kAhead = 8;               // loads in flight: a split's part waits for its factor otherwise (128K tokens: 90 us)
   float mm = -INFINITY;
-  for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, ld_written(part_ml + row0 + static_cast<size_t>(s) * p.group).x);
+#pragma unroll 1
+  for (int s0 = 0; s0 < p.splits; s0 += kAhead) {
+    float2 ml[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j)
+      ml[j] = s0 + j < p.splits ? ld_written(part_ml + row0 + static_cast<size_t>(s0 + j) * p.group) : make_float2(-INFINITY, 0.f);
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) mm = fmaxf(mm, ml[j].x);
+  }
   float a = 0.f, ll = 0.f;
-#pragma unroll 8
-  for (int s = 0; s < p.splits; ++s) {
-    const size_t row = row0 + static_cast<size_t>(s) * p.group;
-    const float2 ml = ld_written(part_ml + row);
-    const float f = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - mm);
-    a += ld_written(part + row * 128 + threadIdx.x) * f;
-    ll += ml.y * f;
+#pragma unroll 1
+  for (int s0 = 0; s0 < p.splits; s0 += kAhead) {
+    float2 ml[kAhead];
+    float x[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const size_t row = row0 + static_cast<size_t>(s0 + j) * p.group;
+      ml[j] = s0 + j < p.splits ? ld_written(part_ml + row) : make_float2(-INFINITY, 0.f);
+      x[j] = s0 + j < p.splits ? ld_written(part + row * 128 + threadIdx.x) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const float f = ml[j].x == -INFINITY ? 0.f : fast_exp2(ml[j].x - mm);
+      a += x[j] * f;
+      ll += ml[j].y * f;
+    }
   }
   const float v = ll > 0.f ? a / ll : 0.f;
   uint16_t* o = out + b * p.osb + h * p.osh + threadIdx.x;

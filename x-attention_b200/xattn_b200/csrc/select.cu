@@ -520,7 +520,8 @@ __global__ void __launch_bounds__(256) select_reg_kernel(const float* __restrict
     const int j = u * 128 + 4 * lane;
     float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
     if (p.vec_in) {
-      if (j < n_read) q = ld_written(reinterpret_cast<const float4*>(x + j));
+      const float4 in = ld_written(reinterpret_cast<const float4*>(x + (j < n_read ? j : 0)));      // (no branch per load)
+      if (j < n_read) q = in;
     } else {
       if (j < n_read) q.x = ld_written(x + j);
       if (j + 1 < n_read) q.y = ld_written(x + j + 1);
