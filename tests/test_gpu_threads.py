@@ -75,3 +75,40 @@ def test_calls_from_several_threads():
     for a, b in zip(got, want):
         for x, y in zip(a, b):
             assert torch.equal(x, y)
+
+
+def test_calls_under_stream_capture():
+    """Every kind of call in one CUDA graph, behind a fill, a copy and a join with another stream: replays give the results of
+    the calls made directly, on new inputs in the same memory."""
+    from xattn_b200 import api, check_device_status, ops
+    g = torch.Generator(device=DEV).manual_seed(3)
+    q, k, v = (torch.randn(1, h, 2500, 128, device=DEV, generator=g).bfloat16() for h in (4, 2, 2))
+    new = [torch.randn(x.shape, device=DEV, generator=g).bfloat16() for x in (q, k, v)]
+    f = [x.float() for x in (q, k, v)]
+
+    def calls():
+        idx, cnt = ops.mask_to_lists(torch.ones(1, 4, 20, 20, dtype=torch.bool, device=DEV), 2500, 2500, True)
+        return (api.Xattention_prefill(q, k, v, 16), *api.xattn_estimate(q, k, 128, 8), ops.decode_attention(q[:, :, -1:], k, v),
+                api.Xattention_prefill(*f, 8), ops.block_sparse_attention(q, k, v, idx, cnt, True, use_workspace=True),
+                ops.block_sparse_attention(q, k, v, idx, cnt, False, use_workspace=True), ops.block_sparse_attention(q, k, v, None, None))
+
+    calls()                                          # (everything that is asked once per kernel and device)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph):
+        zero = torch.zeros(1000, device=DEV)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            aside = ops.decode_attention(q[:, :, :1], k, v)
+        for x, y in zip(f, (q, k, v)):
+            x.copy_(y)
+        torch.cuda.current_stream().wait_stream(side)
+        got = calls()
+    for _ in range(3):
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip((aside, *got), (ops.decode_attention(q[:, :, :1], k, v), *calls())):
+            assert torch.equal(a, b)
+        for x, y in zip((q, k, v), new):
+            x.copy_(y)
+    assert not zero.any()
+    check_device_status()
