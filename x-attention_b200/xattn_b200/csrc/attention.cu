@@ -22,7 +22,7 @@
 //   warp  14    loader of Q
 //
 // What bounds it, and what follows from that (dense causal mask, 32 heads x 16384 tokens: 1110 -> 1372 TFLOP/s; 32768
-// tokens with 2.5 listed blocks per row: 254 -> 185 us):
+// tokens with 2.5 listed blocks per row: 254 -> 166 us in short runs):
 //   * A 128x128 block is 1024 cycles of MMA and 1024 cycles of ex2 (16 per cycle and SM), so the two streams have to be
 //     half a period apart.  One warp issues the MMAs of both in fixed alternation: a stream's batch then goes through
 //     the tensor pipe in one piece.  Two issuing warps' batches interleave, both streams' scores are complete at the

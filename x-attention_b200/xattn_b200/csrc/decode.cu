@@ -5,7 +5,7 @@
 // cache on as many SMs as there are pairs of heads (128K tokens, 32 / 8 heads: 1.8 ms).
 //
 // The step reads K and V once and does next to nothing with them, so it is HBM-bound (128K tokens, 8 kv heads: 537 MB, 83 us
-// at the measured copy bandwidth; measured 95 us) or, for short caches, pure latency.  Therefore:
+// at the measured copy bandwidth; measured 87 us) or, for short caches, pure latency.  Therefore:
 //   * the cache is split along its length so that every SM has two CTAs' worth of it; a CTA streams its keys through a ring
 //     of TMA stages (64 keys of K and V, 32 KiB each), three stages per CTA = 192 KiB in flight per SM, which covers the
 //     HBM latency (6.5 TB/s x 1 us / 148 SMs = 44 KiB) several times over;

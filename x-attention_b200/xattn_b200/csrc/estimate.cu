@@ -80,16 +80,16 @@ struct EstGeom {
   int row_cols;                // columns of the maps
   int head_dim;
   float scale_log2;
-  // Tile tables of est_setup_kernel computed on the host and carried in the kernel parameters when they are small
-  // (tab_n = n_mtiles <= kTabTiles, e.g. 32 row tiles at 32K tokens, 64 at 128K): every kernel copies them into
-  // shared memory and est_setup_kernel is not launched.  Layout: tile_lo[kTabTiles], tile_prefix[kTabTiles + 1],
-  // pair_lo[kTabTiles / 2], pair_prefix[kTabTiles / 2 + 1].
   FastDiv by_tiles, by_group, by_hq;     // tiles per head (of the kernel that runs), query heads per kv head, query heads
   // few tiles: the K loop of each is split over a cluster of `split` CTAs (1: persistent CTAs, a tile each at a time)
   int split;
   // CTA pairs: the two are query heads 2p, 2p + 1 of a kv group at the same rows (otherwise neighbouring row tiles of a head)
   int pair_heads;
   int direct;                  // the epilogue finishes the block sums: every row tile is computed, even one that sees nothing
+  // Tile tables of est_setup_kernel computed on the host and carried in the kernel parameters when they are small
+  // (tab_n = n_mtiles <= kTabTiles, e.g. 32 row tiles at 32K tokens, 64 at 128K): every kernel copies them into
+  // shared memory and est_setup_kernel is not launched.  Layout: tile_lo[kTabTiles], tile_prefix[kTabTiles + 1],
+  // pair_lo[kTabTiles / 2], pair_prefix[kTabTiles / 2 + 1].
   int tab_n;
   int tab[64 + 65 + 32 + 33];
 };
@@ -441,9 +441,9 @@ __device__ __forceinline__ uint4 next_term(unsigned long long (&v)[4]) {
 // more warps take the fp32 units from shared memory and write the terms to shared memory, half of a 64-column stage while the
 // MMAs read the other.  Terms written to HBM first cost 10 bytes per element, and the GEMM then found HBM busy with writing
 // them back (32 heads of 4096 tokens, chunks of 2048: split 56 us + GEMM 46 -> 44; the prefill, whose attention phase takes the
-// bf16 roundings written here, 151 -> 107 us).  Bound by the latency of a converter's step (waits, shared-memory traffic
-// next to the MMAs', three dependent roundings); with loads alone it runs in 30 us.  Eight converter warps took 5 to 10 % less
-// than four.
+// bf16 roundings written here, 151 -> 114 us, 2 us of them for the proxy fence of every unit).  Bound by the latency of a
+// converter's step (waits, shared-memory traffic next to the MMAs', three dependent roundings); with loads alone it runs in 30
+// us.  Sixteen converter warps, or eight where the epilogue of a single tile needs the registers.
 template <int RBS, int kDirect, bool kF32>
 __global__ void __launch_bounds__(kF32 ? f32_threads(kDirect) : kGemmThreads, 1)
 est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -1423,9 +1423,6 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     return make_tmap(m, x, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, box);
   };
 
-  // up to 64 KiB of dynamic shared memory (8192 row tiles): above the 48 KiB a kernel gets without asking
-  if (!allow_smem(est_setup_kernel, 2 * sizeof(int) * 8192))
-    return XATTN_B200_ERR_CUDA;
   bool use_pairs = pairs_fit(g);
   g.pair_heads = g.tile_n == kTileN && (hq / hkv) % 2 == 0 ? 1 : 0;
   if (g.pair_heads) use_pairs = true;
@@ -1471,6 +1468,8 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // The tile tables (the arithmetic of est_setup_kernel): their totals, and, for few row tiles, the tables themselves, which
   // then travel in the kernel parameters.
   const bool in_params = g.n_mtiles <= kTabTiles;
+  // up to 64 KiB of dynamic shared memory (8192 row tiles): above the 48 KiB a kernel gets without asking
+  if (!in_params && !allow_smem(est_setup_kernel, 2 * sizeof(int) * 8192)) return XATTN_B200_ERR_CUDA;
   int tiles_per_head = 0, pairs_per_head = 0;
   for (int mt = 0, lo = 0, hi = -1; mt < g.n_mtiles; ++mt) {
     int first, cnt;
@@ -1602,7 +1601,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // A warp per query block where that fills the chip (32 warps per SM; 2528 query blocks: the estimate 58.6 us by one warp each, 57.5
   // by four), otherwise four.  32 KiB of factors per CTA at most.
   const long long items = static_cast<long long>(batch) * hq * g.qb_total;
-  const bool wide = items < 32 * 148;
+  const bool wide = items < 32LL * sm_count();
   const int teams = wide ? 1 : kSumThreads / 32, seg_max = 32 * 1024 / (4 * g.rbs * teams);
   const int seg_tiles = g.m_pitch < seg_max ? g.m_pitch : seg_max;
   auto launch_sums = [&](auto kern) -> int {
@@ -1626,8 +1625,9 @@ int split_f32_launch(const float* x, int batch, int heads, int len, int len_vali
     return XATTN_B200_ERR_ARG;
   const size_t total = static_cast<size_t>(batch) * heads * len * (head_dim / 8);
   const int block = 256;
+  const size_t most = 32 * static_cast<size_t>(sm_count());
   size_t blocks = (total + block - 1) / block;
-  if (blocks > 148 * 32) blocks = 148 * 32;
+  if (blocks > most) blocks = most;
   auto launch = [&](auto kern) -> int {
     return launch_dependent(kern, dim3(static_cast<unsigned>(blocks)), dim3(block), 0, stream, x, heads, len, len_valid, head_dim / 8, sb,
                             sh, sl, static_cast<uint4*>(out), total);

@@ -148,7 +148,8 @@ inline int launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
   return launch_dependent_clusters(kernel, 1, grid, block, smem_bytes, stream, std::forward<Args>(args)...);
 }
 
-// Division of numbers below 2^31 by a divisor known on the host: a multiplication and a shift instead of the ~25
+// Division of numbers below 2^31 by a divisor known on the host (the round-up method of Granlund and Montgomery, "Division by
+// invariant integers using multiplication"): a multiplication and a shift instead of the ~25
 // instructions of an integer division, which add up in code that every role of a kernel has to decode its work with.
 struct FastDiv {
   uint32_t d, mul, shift;

@@ -9,6 +9,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -306,12 +307,12 @@ Tensor attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Ten
 }
 // Non-causal calls: sorting the units by list length is one launch of a few microseconds; with only a few units per SM there
 // is nothing to balance.
-constexpr int64_t kOrderMinItems = 16 * 148;
+constexpr int64_t kOrderMinItemsPerSm = 16;
 bool default_workspace(bool causal, bool dense, const Tensor& q) {
   if (dense) return false;
   const char* forced = std::getenv("XATTN_B200_ATTN_WORKSPACE");       // "0" / "1": overrides the rule (for measurements)
   if (forced && (forced[0] == '0' || forced[0] == '1') && forced[1] == 0) return forced[0] == '1';
-  return !causal && q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) >= kOrderMinItems;
+  return !causal && q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) >= kOrderMinItemsPerSm * at::cuda::getDeviceProperties(q.get_device())->multiProcessorCount;
 }
 
 void need_16bit_or_f32(const Tensor& q, const Tensor& k, const char* text) {

@@ -11,7 +11,8 @@
 //     value is found by bisection on the bit patterns of the scores, summing in fp64.  The bitmaps are a word per lane.
 //   * Longer rows (select_kernel): staged in shared memory; the largest remaining score is extracted one at a time, and
 //     rows that are still going after kPeelMax of them are sorted.
-// Both accumulate in fp64 exactly as the rule is stated.
+// Both accumulate in fp64, in different orders (the first in groups of scores, the second rank by rank), so that a rank whose
+// prefix equals what is wanted to within the rounding of fp64 may go either way, as it may in the reference with its own order.
 // Latency and instructions bound it, not bytes: 24 heads x 931 rows of 944 flat scores (video diffusion) took 1128 us with the
 // sort, 149 us with the bisection; 32 x 1024 rows of 16 scores (128K tokens) 27 -> 19 us.
 //

@@ -28,7 +28,7 @@ def xattn_varlen_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu
     """q, k, v [1, heads, total, D] (16 bit, any strides with unit stride on D); cu_seqlens_* = [0, valid, total].
     Returns [1, heads, total, D] (a view of [1, total, heads, D] storage).  The two segments are read through
     strided views and written straight into their rows of the result: no copy of q, k, v or of the outputs,
-    whatever the segment lengths (the estimate stages only the tile that holds a ragged last stride group)."""
+    whatever the segment lengths."""
     v0q, v1q = int(cu_seqlens_q[1]), int(cu_seqlens_q[2])
     v0k, v1k = int(cu_seqlens_kv[1]), int(cu_seqlens_kv[2])
     B, H, _, D = q.shape

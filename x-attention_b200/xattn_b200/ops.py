@@ -185,7 +185,7 @@ def mask_to_lists(mask: torch.Tensor, q_len: int, k_len: int, causal: bool):
 # ------------------------------------------------------------------------------ phase 3
 # Causal calls are not offered scratch memory by default: the general kernel now loads K/V once for two query heads of a
 # kv group itself, and the split into two kernels no longer gains (Llama-3.1-8B at 128K tokens, where 95 % of the blocks
-# qualify for the pair kernel: 700 us with the split, 610 us without).
+# qualify for the pair kernel: 700 us with the split, 596 us without).
 def pair_split_share(percent: Optional[int] = None) -> int:
     """Share (per cent) of a call's listed blocks that must qualify for the pair kernel before the library splits
     the call between the two attention kernels (process-wide; 0: whenever anything qualifies, 101: never).
