@@ -20,6 +20,7 @@ struct AttnParams {
   FastDiv by_units, by_hq, by_batch, by_group, by_hkv;          // (general kernel: see unit_tile) hq, batch, hq / hkv, hkv
   const int32_t* tile_list;     // general kernel: its tiles, two per unit (null: all, in their natural order)
   int list_tiles;               // entries of that list
+  int early_next;               // the kernel after this one may start under the tail
 };
 
 __device__ __forceinline__ uint32_t pack16(float lo, float hi, int is_bf16) {
