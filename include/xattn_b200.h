@@ -121,6 +121,36 @@ int xattn_b200_estimate_f32(const float* q, const float* k, int batch, int hq, i
                             int semantics, float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16,
                             int* status, void* cuda_stream);
 
+/*
+ * Phases 1 and 2 in one call (xattn/src/Xattention.py:13-299): the estimate (dtype XATTN_B200_F32: with q_bf16 and k_bf16 as in
+ * xattn_b200_estimate_f32), then xattn_b200_select, _select_band (semantics XATTN_B200_SEMANTICS_TORCH_BAND) or _select_rounded
+ * (`rounded` not NULL) on its sums, with the diagonal cleaned up.  Where every row of the estimate sees a single column tile the
+ * selection happens inside its kernel.
+ * Fields have the meaning of the arguments of those functions; list_q_len and list_k_len are the lengths of the lists.
+ */
+typedef struct {
+  const void *q, *k;
+  int dtype, batch, hq, hkv, q_len, k_len, head_dim;
+  int64_t q_stride_b, q_stride_h, q_stride_l, k_stride_b, k_stride_h, k_stride_l;
+  int stride, block_size, chunk_size;
+  float scale;
+  int causal, semantics;
+  float* attn_sums;
+  void* workspace;
+  size_t workspace_bytes;
+  void *q_bf16, *k_bf16;
+  double threshold;
+  const float* threshold_per_head;
+  int keep_sink, keep_recent;
+  uint8_t* mask;
+  void* rounded;
+  int rounded_dtype;
+  int32_t *block_idx, *block_cnt;
+  int list_q_len, list_k_len;
+  int* status;
+} xattn_b200_estimate_select_args;
+int xattn_b200_estimate_select(const xattn_b200_estimate_select_args* args, void* cuda_stream);
+
 /* 1: the estimate of fp32 q and k of that shape is faster from rows split into terms first (many tiles use each value). */
 int xattn_b200_estimate_f32_terms(int hq, int hkv, int q_len, int k_len, int stride, int block_size, int chunk_size, int causal,
                                   int semantics);

@@ -31,6 +31,7 @@ SIGNATURES = {
                                         _i, _i, _i, _f, _i, _i, _p, _p, _p]),
     "xattn_b200_estimate_f32": (_i, [_p, _p, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64, _i64,
                                      _i, _i, _i, _f, _i, _i, _p, _p, _sz, _p, _p, _p, _p]),
+    "xattn_b200_estimate_select": (_i, [_p, _p]),
     "xattn_b200_estimate_f32_terms": (_i, [_i, _i, _i, _i, _i, _i, _i, _i, _i]),
     "xattn_b200_split_f32": (_i, [_p, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i, _p, _p]),
     "xattn_b200_split_f32_terms": (_i, [_p, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i, _p, _p]),

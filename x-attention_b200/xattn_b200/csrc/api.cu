@@ -1,5 +1,5 @@
 // extern "C" surface of libxattn_b200.so (declared in include/xattn_b200.h): argument plumbing only.
-#include "host_common.cuh"
+#include "select_row.cuh"
 
 namespace xb {
 size_t estimate_workspace_bytes(int batch, int hq, int q_len, int k_len, int stride, int block_size, int chunk_size,
@@ -7,7 +7,8 @@ size_t estimate_workspace_bytes(int batch, int hq, int q_len, int k_len, int str
 int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, int hkv, int q_len, int k_len,
                     int head_dim, int64_t qsb, int64_t qsh, int64_t qsl, int64_t ksb, int64_t ksh, int64_t ksl,
                     int stride, int block_size, int chunk_size, float scale, int causal, int semantics,
-                    float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16, int* status, cudaStream_t stream);
+                    float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16, int* status, cudaStream_t stream,
+                    const SelCall* select = nullptr, bool* selected = nullptr);
 int split_f32_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
                      int64_t sl, int terms, void* out, cudaStream_t stream);
 int split_f32_role_launch(const float* x, int batch, int heads, int len, int len_valid, int head_dim, int64_t sb, int64_t sh,
@@ -16,11 +17,6 @@ int estimate_f32_terms(int hq, int hkv, int q_len, int k_len, int stride, int bl
 int rope_qk_launch(void* q, void* k, int dtype, int batch, int hq, int hkv, int len, int head_dim, int64_t qsb,
                    int64_t qsh, int64_t qsl, int64_t ksb, int64_t ksh, int64_t ksl, const void* cos, const void* sin,
                    int64_t cs_stride_b, int64_t cs_stride_l, cudaStream_t stream);
-int select_launch(const float* attn_sums, int batch, int heads, int q_blocks, int k_blocks, int bpc, int block_offset,
-                  int causal, int diagonal_cleanup, double threshold, const float* thr_per_head, int keep_sink,
-                  int keep_recent, uint8_t* mask, int32_t* block_idx, int32_t* block_cnt, int list_q_blocks,
-                  int list_k_blocks, int list_q_len, int list_k_len, int band, void* rounded, int rounded_dtype, int* status,
-                  cudaStream_t stream);
 int mask_to_lists_launch(const uint8_t* mask, int batch, int heads, int mask_q_blocks, int mask_k_blocks, int q_len,
                          int k_len, int causal, int32_t* block_idx, int32_t* block_cnt, cudaStream_t stream);
 int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv,
@@ -111,6 +107,27 @@ int xattn_b200_estimate_f32(const float* q, const float* k, int batch, int hq, i
                              attn_sums, workspace, workspace_bytes, q_bf16, k_bf16, status, static_cast<cudaStream_t>(cuda_stream));
 }
 
+int xattn_b200_estimate_select(const xattn_b200_estimate_select_args* a, void* cuda_stream) {
+  if (!a) return XATTN_B200_ERR_ARG;
+  int geo[8];
+  int rc = xattn_b200_estimate_geometry(a->q_len, a->k_len, a->chunk_size, a->stride, a->block_size, geo);
+  if (rc) return rc;
+  const bool band = a->semantics == XATTN_B200_SEMANTICS_TORCH_BAND, lists = a->block_idx != nullptr;
+  const xb::SelCall call = {a->attn_sums, a->batch, a->hq, geo[2], geo[3], geo[6], geo[7], a->causal, 1, a->threshold, a->threshold_per_head,
+                            a->keep_sink, a->keep_recent, a->mask, a->block_idx, a->block_cnt, lists ? (a->list_q_len + 127) / 128 : 0,
+                            lists ? (a->list_k_len + 127) / 128 : 0, a->list_q_len, a->list_k_len, band ? 1 : 0, a->rounded, a->rounded_dtype};
+  xb::SelParams p;
+  if ((rc = xb::select_params(call, p))) return rc;          // (a refusal leaves no work in flight)
+  bool selected = false;
+  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+  if ((rc = xb::estimate_launch(a->q, a->k, a->dtype, a->batch, a->hq, a->hkv, a->q_len, a->k_len, a->head_dim, a->q_stride_b, a->q_stride_h,
+                                a->q_stride_l, a->k_stride_b, a->k_stride_h, a->k_stride_l, a->stride, a->block_size, a->chunk_size, a->scale,
+                                a->causal, a->semantics, a->attn_sums, a->workspace, a->workspace_bytes, a->q_bf16, a->k_bf16, a->status,
+                                stream, &call, &selected)))
+    return rc;
+  return selected ? XATTN_B200_OK : xb::select_launch(call, a->status, stream);
+}
+
 int xattn_b200_estimate_f32_terms(int hq, int hkv, int q_len, int k_len, int stride, int block_size, int chunk_size, int causal,
                                   int semantics) {
   return xb::estimate_f32_terms(hq, hkv, q_len, k_len, stride, block_size, chunk_size, causal ? 1 : 0, semantics);
@@ -142,9 +159,9 @@ int xattn_b200_select(const float* attn_sums, int batch, int heads, int q_blocks
                       const float* threshold_per_head, int keep_sink, int keep_recent, uint8_t* mask,
                       int32_t* block_idx, int32_t* block_cnt, int list_q_blocks, int list_k_blocks, int list_q_len,
                       int list_k_len, int* status, void* cuda_stream) {
-  return xb::select_launch(attn_sums, batch, heads, q_blocks, k_blocks, blocks_per_chunk, block_offset, causal,
-                           diagonal_cleanup, threshold, threshold_per_head, keep_sink, keep_recent, mask, block_idx,
-                           block_cnt, list_q_blocks, list_k_blocks, list_q_len, list_k_len, 0, nullptr, 0, status,
+  return xb::select_launch({attn_sums, batch, heads, q_blocks, k_blocks, blocks_per_chunk, block_offset, causal,
+                            diagonal_cleanup, threshold, threshold_per_head, keep_sink, keep_recent, mask, block_idx,
+                            block_cnt, list_q_blocks, list_k_blocks, list_q_len, list_k_len, 0, nullptr, 0}, status,
                            static_cast<cudaStream_t>(cuda_stream));
 }
 
@@ -153,9 +170,9 @@ int xattn_b200_select_band(const float* attn_sums, int batch, int heads, int q_b
                            const float* threshold_per_head, int keep_sink, int keep_recent, uint8_t* mask,
                            int32_t* block_idx, int32_t* block_cnt, int list_q_blocks, int list_k_blocks,
                            int list_q_len, int list_k_len, int* status, void* cuda_stream) {
-  return xb::select_launch(attn_sums, batch, heads, q_blocks, k_blocks, blocks_per_chunk, block_offset, causal,
-                           diagonal_cleanup, threshold, threshold_per_head, keep_sink, keep_recent, mask, block_idx,
-                           block_cnt, list_q_blocks, list_k_blocks, list_q_len, list_k_len, 1, nullptr, 0, status,
+  return xb::select_launch({attn_sums, batch, heads, q_blocks, k_blocks, blocks_per_chunk, block_offset, causal,
+                            diagonal_cleanup, threshold, threshold_per_head, keep_sink, keep_recent, mask, block_idx,
+                            block_cnt, list_q_blocks, list_k_blocks, list_q_len, list_k_len, 1, nullptr, 0}, status,
                            static_cast<cudaStream_t>(cuda_stream));
 }
 
@@ -163,9 +180,9 @@ int xattn_b200_select_rounded(const float* attn_sums, int batch, int heads, int 
                               int block_offset, int causal, int diagonal_cleanup, double threshold,
                               const float* threshold_per_head, int keep_sink, int keep_recent, uint8_t* mask, void* rounded,
                               int rounded_dtype, int* status, void* cuda_stream) {
-  return xb::select_launch(attn_sums, batch, heads, q_blocks, k_blocks, blocks_per_chunk, block_offset, causal,
-                           diagonal_cleanup, threshold, threshold_per_head, keep_sink, keep_recent, mask, nullptr, nullptr, 0, 0, 0, 0, 0,
-                           rounded, rounded_dtype, status, static_cast<cudaStream_t>(cuda_stream));
+  return xb::select_launch({attn_sums, batch, heads, q_blocks, k_blocks, blocks_per_chunk, block_offset, causal,
+                            diagonal_cleanup, threshold, threshold_per_head, keep_sink, keep_recent, mask, nullptr, nullptr, 0, 0, 0, 0, 0,
+                            rounded, rounded_dtype}, status, static_cast<cudaStream_t>(cuda_stream));
 }
 
 int xattn_b200_mask_to_lists(const uint8_t* mask, int batch, int heads, int mask_q_blocks, int mask_k_blocks,

@@ -21,8 +21,7 @@
 
 #include <type_traits>
 
-#include "host_common.cuh"
-#include "sm100_primitives.cuh"
+#include "select_row.cuh"
 
 namespace xb {
 
@@ -51,6 +50,20 @@ __host__ __device__ constexpr int f32_threads(int direct) { return kGemmThreads 
 struct EstRounded {
   uint4 *q, *k;
   int q_len, k_len;
+};
+
+// The selection on rows that the epilogue has finished (EstGeom::direct): a chain of a microsecond per row, which runs under the
+// next tiles' products, or, where a cluster of four has a single tile, on a warp per row.  As a kernel of its own it was a launch and a
+// hand-over between two kernels more (1003 tokens: the prefill 26.2 -> 24.2 us; 128K tokens 773 -> 765 in short runs).
+// Single CTAs with 128-column tiles of 16-bit operands, and CTA pairs, do it: the other kernels' epilogues have no registers left
+// for it (spills: 4096 tokens against 65536 51.9 -> 52.5 us a call although nothing was selected there).
+__host__ __device__ constexpr bool selects(int direct, bool f32) { return direct == 1 && !f32; }
+struct EstSelect {
+  int on;
+  SelParams p;
+  const float* thr_per_head;
+  uint8_t* mask;
+  int32_t *idx, *cnt;
 };
 
 struct EstGeom {
@@ -421,6 +434,24 @@ __device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, Load l
   for (int c = base / kLeft; c < outside; c += kWriters) out[c < col0 ? c : c + kBlocks] = 0.f;
 }
 
+// Selects query blocks [qb0, qb0 + n) of a head, whose sums this warp (or, behind a barrier, its CTA) has written: every
+// `step`-th of them from the `first` on.
+template <int RBS>
+__device__ __forceinline__ void est_select_rows(const EstGeom& g, const EstSelect& sel, const float* sums, int bh, int qb0, int n, int first,
+                                                int step, int lane) {
+  __syncwarp();
+#pragma unroll 1
+  for (int r = first; r < n && qb0 + r < g.qb_total; r += step)
+    select_row<1>(sums, sel.p, sel.thr_per_head, sel.mask, sel.idx, sel.cnt, bh * g.qb_total + qb0 + r, lane);
+}
+
+// After a wait that ran out: the rows of a tile list nothing, so that nobody reads a list that was never written.
+template <int RBS>
+__device__ __forceinline__ void est_forget_rows(const EstGeom& g, const EstSelect& sel, int bh, int mt) {
+  const int r = static_cast<int>(threadIdx.x), qb = mt * kTileM / RBS + r;
+  if (sel.cnt && r < kTileM / RBS && qb < sel.p.list_q_blocks && qb < g.qb_total) sel.cnt[static_cast<size_t>(bh) * sel.p.list_q_blocks + qb] = 0;
+}
+
 // Eight fp32 values, in pairs: the next term of each, the rounding of what the terms before leave.
 __device__ __forceinline__ uint4 next_term(unsigned long long (&v)[4]) {
   uint32_t w[4];
@@ -449,7 +480,7 @@ __global__ void __launch_bounds__(kF32 ? f32_threads(kDirect) : kGemmThreads, 1)
 est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt, const EstGeom g,
                 const int* tile_lo, const int* tile_prefix, float* __restrict__ partial,
-                float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc, const EstRounded rounded, int* status) {
+                float2* __restrict__ mtile, float* sums, const uint32_t idesc, const EstRounded rounded, const EstSelect sel, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_tab[kTabInts];
   if (g.tab_n) {                                  // (made visible by the __syncthreads() that ends the prologue)
@@ -775,6 +806,9 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         est_epilogue_row_direct<RBS, kDirect>(g, load, nvis, clo, chi,
                                               sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, col0, out_cols,
                                               qb < g.qb_total, lane);
+        if constexpr (selects(kDirect, kF32)) {
+          if (sel.on && split == 1) est_select_rows<RBS>(g, sel, sums, bh, (mt * kTileM + quad * 32) / RBS, 32 / RBS, 0, 1, lane);
+        }
       } else {
         const size_t tile_at = scratch_tile(g, bh, mt, nt, tile_lo[mt]) * kTileM;
         est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, true, partial + tile_at * kGroups + r, mtile + tile_at + r, release);
@@ -790,7 +824,19 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000) { __nanosleep(1000); }
     if (threadIdx.x == 0 && status) atomicExch(status, static_cast<int>(kDevWaitTimeout));
+    if (selects(kDirect, kF32) && sel.on)
+      for (int tile = tile0; tile < total_tiles; tile += tile_step) {
+        int bh, mt, nt;
+        decode_tile(g, g.n_mtiles, tile_lo, tile_prefix, tile, bh, mt, nt, interleave);
+        est_forget_rows<RBS>(g, sel, bh, mt);
+      }
     __syncthreads();
+  } else if (selects(kDirect, kF32) && sel.on && split > 1) {
+    // a cluster's CTA has finished 128 / split rows, few query blocks: a warp each
+    int bh, mt, nt;
+    decode_tile(g, g.n_mtiles, tile_lo, tile_prefix, tile0, bh, mt, nt, interleave);
+    est_select_rows<RBS>(g, sel, sums, bh, (mt * kTileM + rank * (kTileM / split)) / RBS, kTileM / split / RBS, warp,
+                         static_cast<int>(blockDim.x >> 5), lane);
   }
   if (warp == 1) {
     tc_fence_after();
@@ -824,8 +870,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKh,
                      const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt,
                      const EstGeom g, const int* group_lo, const int* group_prefix,
-                     float* __restrict__ partial, float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc_wide, const uint32_t idesc_narrow,
-                     int* status) {
+                     float* __restrict__ partial, float2* __restrict__ mtile, float* sums, const uint32_t idesc_wide, const uint32_t idesc_narrow,
+                     const EstSelect sel, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_tab[kTabInts];
   if (g.tab_n) {                                  // (made visible by the __syncthreads() that ends the prologue)
@@ -1021,6 +1067,7 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         est_epilogue_row_direct<RBS, kDirect>(g, load, nvis, clo, chi,
                                         sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, col0, out_cols,
                                         qb < g.qb_total, lane);
+        if (sel.on) est_select_rows<RBS>(g, sel, sums, bh, (mt * kTileM + quad * 32) / RBS, 32 / RBS, 0, 1, lane);
       } else {
         // (compact scratch: both row tiles of a pair lie in one chunk and start at the pair's first column tile)
         const bool write = mt < g.n_mtiles;
@@ -1038,6 +1085,12 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000) { __nanosleep(1000); }
     if (threadIdx.x == 0 && status) atomicExch(status, static_cast<int>(kDevWaitTimeout));
+    if (kDirect > 0 && sel.on)
+      for (int tile = pair; tile < total_tiles; tile += n_pairs_grid) {
+        int bh, mt, nt;
+        decode(tile, bh, mt, nt);
+        if (mt < g.n_mtiles) est_forget_rows<RBS>(g, sel, bh, mt);
+      }
   }
   // neither CTA may release tensor memory, or leave while the other can still signal its barriers
   cluster_sync_all();
@@ -1372,7 +1425,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
                     int head_dim, int64_t qsb, int64_t qsh, int64_t qsl, int64_t ksb, int64_t ksh, int64_t ksl,
                     int stride, int block_size, int chunk_size, float scale, int causal, int semantics,
                     float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16, int* status,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, const SelCall* select, bool* selected) {
   const bool f32 = dtype == XATTN_B200_F32, terms = dtype == XATTN_B200_F32_TERMS;
   if (!q || !k || !attn_sums) return XATTN_B200_ERR_ARG;
   if (dtype != XATTN_B200_BF16 && dtype != XATTN_B200_F16 && !f32 && !terms) return XATTN_B200_ERR_ARG;
@@ -1456,6 +1509,25 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     direct = g.band ? count == 1 && first * g.tile_n == (mt * kTileM / g.rcs) * g.rcs + g.row_off : count <= 1;
   }
   g.direct = direct ? 1 : 0;
+  // The block sums finished there can be selected on there, too: rows of up to 128 stored sums (four per lane).  Clusters of two do
+  // not gain: a CTA has the rows of eight query blocks at stride 16, two rounds for its six warps (2100 tokens 35.4 us a call
+  // with it, 35.2 without).
+  EstSelect sel;
+  sel.on = 0;
+  if (select) {
+    const SelCall& c = *select;
+    const int cols = g.band ? g.bpc : g.kb_total;
+    if (direct && (use_pairs || selects(g.tile_n / 128, f32)) && g.split != 2 && cols <= 128 && c.k_blocks <= 1024 && c.attn_sums == attn_sums && c.batch == batch && c.heads == hq &&
+        c.q_blocks == g.qb_total && c.k_blocks == g.kb_total && c.bpc == g.bpc && (c.band ? 1 : 0) == g.band) {
+      if ((rc = select_params(c, sel.p))) return rc;
+      sel.on = 1;
+      sel.thr_per_head = c.thr_per_head;
+      sel.mask = c.mask;
+      sel.idx = c.block_idx;
+      sel.cnt = c.block_cnt;
+      *selected = true;
+    }
+  }
   CUtensorMap tmQ, tmK, tmQt, tmKt;
   const uint32_t k_box = use_pairs ? 64 : (f32 ? static_cast<uint32_t>(kTileM) : static_cast<uint32_t>(g.tile_n));
   if ((rc = make_map(&tmQ, q, q_len, hq, qsb, qsh, qsl, kTileM, false))) return rc;
@@ -1531,7 +1603,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       if (static_cast<unsigned>(2 * max_clusters) < cfg.gridDim.x) cfg.gridDim.x = 2 * max_clusters;
       return launch_dependent_clusters(kern, 2, cfg.gridDim, cfg.blockDim, kPairSmem, stream, tmQ, tmK, tmQt, tmKt, g,
                                        (const int*)(g.pair_heads ? tile_lo : pair_lo), (const int*)(g.pair_heads ? tile_prefix : pair_prefix),
-                                       partial, mtile, attn_sums, idesc2, idesc2n, status);
+                                       partial, mtile, attn_sums, idesc2, idesc2n, sel, status);
     };
     auto launch_pair_rbs = [&](auto rbs) -> int {
       constexpr int kRbs = decltype(rbs)::value;
@@ -1576,7 +1648,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   auto launch = [&](auto kern, int threads, int smem) -> int {
     if (!allow_smem(kern, smem)) return XATTN_B200_ERR_CUDA;
     return launch_dependent_clusters(kern, g.split, dim3(grid), dim3(threads), smem, stream, tmQ, tmK, tmQt, tmKt, g, (const int*)tile_lo,
-                                     (const int*)tile_prefix, partial, mtile, attn_sums, idesc, rounded, status);
+                                     (const int*)tile_prefix, partial, mtile, attn_sums, idesc, rounded, sel, status);
   };
   auto launch_type = [&](auto rbs, auto halves) -> int {
     constexpr int kRbs = decltype(rbs)::value, kDirect = decltype(halves)::value;

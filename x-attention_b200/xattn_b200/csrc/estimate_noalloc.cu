@@ -19,10 +19,12 @@ size_t estimate_workspace_bytes(int batch, int hq, int q_len, int k_len, int str
                                 int causal, int semantics);
 size_t estimate_row_bytes(int batch, int hq, int q_len, int k_len, int stride, int block_size, int chunk_size, int causal,
                           int semantics);
+struct SelCall;
 int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, int hkv, int q_len, int k_len,
                     int head_dim, int64_t qsb, int64_t qsh, int64_t qsl, int64_t ksb, int64_t ksh, int64_t ksl,
                     int stride, int block_size, int chunk_size, float scale, int causal, int semantics,
-                    float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16, int* status, cudaStream_t stream);
+                    float* attn_sums, void* workspace, size_t workspace_bytes, void* q_bf16, void* k_bf16, int* status, cudaStream_t stream,
+                    const SelCall* select, bool* selected);
 }  // namespace xb
 
 // The scratch itself.  In host code this name is only a handle for the runtime's symbol table, not an
@@ -77,7 +79,7 @@ extern "C" int xattn_b200_estimate_static(const void* q, const void* k, int dtyp
   auto launch = [&](const void* q0, const void* k0, int b, int h, int g, float* sums) {
     return xb::estimate_launch(q0, k0, dtype, b, h, g, q_len, k_len, head_dim, q_stride_b, q_stride_h, q_stride_l, k_stride_b,
                                k_stride_h, k_stride_l, stride, block_size, chunk_size, scale, causal, semantics, sums, scratch,
-                               kScratch, nullptr, nullptr, status, static_cast<cudaStream_t>(cuda_stream));
+                               kScratch, nullptr, nullptr, status, static_cast<cudaStream_t>(cuda_stream), nullptr, nullptr);
   };
   if (whole) return launch(q, k, batch, hq, hkv, attn_sums);
   // Slices of heads, one after the other on the stream: the rows of a head are padded to whole tiles, which for many heads of

@@ -180,7 +180,9 @@ struct EstimateArgs {
 };
 // fp32 block sums [B, Hq, q_blocks_pad, k_blocks_pad or blocks_per_chunk]
 // q16, k16 (fp32 inputs, null: not wanted): set to the bf16 roundings of q and k.
-Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const EstimateArgs& a, Tensor* q16, Tensor* k16, const Place& at_) {
+// then: null, or what follows the estimate in the same call of the library: the fields of the selection, the others are set here.
+Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const EstimateArgs& a, Tensor* q16, Tensor* k16, const Place& at_,
+                xattn_b200_estimate_select_args* then = nullptr) {
   int dtype = q_.scalar_type() == at::kFloat ? XATTN_B200_F32 : dtype_code(q_.scalar_type());
   const bool f32 = dtype == XATTN_B200_F32;
   // any memory: fp32, and 16-bit rows of another head_dim than 128 whose length is no multiple of the stride
@@ -218,6 +220,23 @@ Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const Est
   Tensor sums = empty({B, Hq, g.qb, a.band ? g.bpc : g.kb}, at::kFloat, at_.dev);
   if (D == 0 || a.norm == 0.0) fail(PyExc_ZeroDivisionError, "the scale of the scores is 1 / (sqrt(head_dim) * stride * norm)");
   const double scale = 1.0 / std::sqrt(static_cast<double>(D)) / a.stride / a.norm;
+  if (then) {
+    xattn_b200_estimate_select_args& t = *then;
+    t.q = q.data_ptr(); t.k = k.data_ptr();
+    t.dtype = dtype; t.batch = B; t.hq = Hq; t.hkv = Hkv; t.q_len = Lq; t.k_len = Lk; t.head_dim = D;
+    t.q_stride_b = q.stride(0); t.q_stride_h = q.stride(1); t.q_stride_l = q.stride(2);
+    t.k_stride_b = k.stride(0); t.k_stride_h = k.stride(1); t.k_stride_l = k.stride(2);
+    t.stride = a.stride; t.block_size = a.block; t.chunk_size = a.chunk;
+    t.scale = static_cast<float>(scale);
+    t.causal = a.causal; t.semantics = sem;
+    t.attn_sums = static_cast<float*>(sums.data_ptr());
+    t.workspace = ws.data_ptr(); t.workspace_bytes = bytes;
+    t.q_bf16 = dtype == XATTN_B200_F32 && q16 ? q16->data_ptr() : nullptr;
+    t.k_bf16 = dtype == XATTN_B200_F32 && k16 ? k16->data_ptr() : nullptr;
+    t.status = at_.status;
+    check(xattn_b200_estimate_select(then, at_.stream), "estimate_select");
+    return sums;
+  }
   if (dtype == XATTN_B200_F32)
     check(xattn_b200_estimate_f32(static_cast<const float*>(q.data_ptr()), static_cast<const float*>(k.data_ptr()), B, Hq, Hkv, Lq, Lk, D,
                                   q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), a.stride, a.block, a.chunk,
@@ -249,12 +268,8 @@ struct SelectArgs {
   int64_t list_q, list_k;       // 0: no lists
   int64_t band_kb;              // > 0: the sums are the chunk band of rows of that many key blocks
 };
-// rounded (mask only, 16-bit types): set to the sums in that type, written by the same kernel.
-Selection select(const Tensor& sums, const Threshold& threshold, const SelectArgs& a, const Place& at_, Tensor* rounded = nullptr) {
-  const int64_t B = sums.size(0), H = sums.size(1), QB = sums.size(2), KB = a.band_kb > 0 ? a.band_kb : sums.size(3);
-  if (a.band_kb > 0 && sums.size(3) != a.bpc) fail(PyExc_ValueError, "band sums must have blocks_per_chunk columns");
-  Tensor thr;
-  const double value = threshold.value;
+// What a selection writes, allocated, and its threshold per head as the kernels read it (undefined: `value` for all).
+Selection new_selection(const SelectArgs& a, int64_t B, int64_t H, int64_t QB, int64_t KB, const Threshold& threshold, Tensor& thr, const Place& at_) {
   if (threshold.per_head.defined()) {
     thr = threshold.per_head.detach();
     if (thr.device() != at_.dev || thr.scalar_type() != at::kFloat) thr = thr.to(at_.dev, at::kFloat);
@@ -263,26 +278,50 @@ Selection select(const Tensor& sums, const Threshold& threshold, const SelectArg
   }
   Selection r;
   if (a.want_mask) r.mask = empty({B, H, QB, KB}, at::kBool, at_.dev);
-  const int64_t lqb = (a.list_q + 127) / 128, lkb = (a.list_k + 127) / 128;
   if (a.list_q > 0) {
+    const int64_t lqb = (a.list_q + 127) / 128, lkb = (a.list_k + 127) / 128;
     r.idx = empty({B, H, lqb, lkb}, at::kInt, at_.dev);
     r.cnt = empty({B, H, lqb}, at::kInt, at_.dev);
   }
-  if (rounded) {
-    check(xattn_b200_select_rounded(static_cast<const float*>(sums.data_ptr()), B, H, QB, KB, a.bpc, a.block_offset, a.causal, a.cleanup,
-                                    value, thr.defined() ? static_cast<const float*>(thr.data_ptr()) : nullptr, a.sink, a.recent,
-                                    static_cast<uint8_t*>(r.mask.data_ptr()), rounded->data_ptr(), dtype_code(rounded->scalar_type()),
-                                    at_.status, at_.stream),
-          "select_rounded");
-    return r;
-  }
+  return r;
+}
+template <typename T>
+T* data(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
+
+Selection select(const Tensor& sums, const Threshold& threshold, const SelectArgs& a, const Place& at_) {
+  const int64_t B = sums.size(0), H = sums.size(1), QB = sums.size(2), KB = a.band_kb > 0 ? a.band_kb : sums.size(3);
+  if (a.band_kb > 0 && sums.size(3) != a.bpc) fail(PyExc_ValueError, "band sums must have blocks_per_chunk columns");
+  Tensor thr;
+  Selection r = new_selection(a, B, H, QB, KB, threshold, thr, at_);
   auto fn = a.band_kb > 0 ? xattn_b200_select_band : xattn_b200_select;
-  check(fn(static_cast<const float*>(sums.data_ptr()), B, H, QB, KB, a.bpc, a.block_offset, a.causal, a.cleanup, value,
-           thr.defined() ? static_cast<const float*>(thr.data_ptr()) : nullptr, a.sink, a.recent,
-           r.mask.defined() ? static_cast<uint8_t*>(r.mask.data_ptr()) : nullptr,
-           r.idx.defined() ? static_cast<int32_t*>(r.idx.data_ptr()) : nullptr,
-           r.cnt.defined() ? static_cast<int32_t*>(r.cnt.data_ptr()) : nullptr, lqb, lkb, a.list_q, a.list_k, at_.status, at_.stream),
+  check(fn(static_cast<const float*>(sums.data_ptr()), B, H, QB, KB, a.bpc, a.block_offset, a.causal, a.cleanup, threshold.value,
+           data<float>(thr), a.sink, a.recent, data<uint8_t>(r.mask), data<int32_t>(r.idx), data<int32_t>(r.cnt), (a.list_q + 127) / 128,
+           (a.list_k + 127) / 128, a.list_q, a.list_k, at_.status, at_.stream),
         "select");
+  return r;
+}
+
+// The estimate and the selection on it.  rounded (mask only): the sums in that tensor's type, null: not wanted.
+struct Estimated {
+  Tensor sums;
+  Selection s;
+};
+Estimated estimate_and_select(const Tensor& q, const Tensor& k, const Geometry& g, const EstimateArgs& e, const Threshold& threshold,
+                              const SelectArgs& a, Tensor* q16, Tensor* k16, const Tensor* rounded, const Place& at_) {
+  Tensor thr;
+  Estimated r;
+  r.s = new_selection(a, q.size(0), q.size(1), g.qb, g.kb, threshold, thr, at_);
+  xattn_b200_estimate_select_args t = {};
+  t.threshold = threshold.value;
+  t.threshold_per_head = data<float>(thr);
+  t.keep_sink = a.sink; t.keep_recent = a.recent;
+  t.mask = data<uint8_t>(r.s.mask); t.block_idx = data<int32_t>(r.s.idx); t.block_cnt = data<int32_t>(r.s.cnt);
+  t.list_q_len = a.list_q; t.list_k_len = a.list_k;
+  if (rounded) {
+    t.rounded = rounded->data_ptr();
+    t.rounded_dtype = dtype_code(rounded->scalar_type());
+  }
+  r.sums = estimate(q, k, g, e, q16, k16, at_, &t);
   return r;
 }
 
@@ -471,11 +510,8 @@ PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
     // fp32: the attention phase computes with the bf16 roundings, those of q and k come from the estimate
     const bool f32 = q.scalar_type() == at::kFloat && D == 128 && !out.defined() && v.scalar_type() == at::kFloat;
     Tensor q16, k16;
-    Selection s;
-    {
-      const Tensor sums = estimate(q, k, g, e, f32 ? &q16 : nullptr, f32 ? &k16 : nullptr, at_);
-      s = select(sums, threshold, {g.bpc, g.block_offset, e.causal, true, sink, recent, false, Lq, Lk, e.band ? g.kb : 0}, at_);
-    }
+    const Selection s = estimate_and_select(q, k, g, e, threshold, {g.bpc, g.block_offset, e.causal, true, sink, recent, false, Lq, Lk, 0},
+                                            f32 ? &q16 : nullptr, f32 ? &k16 : nullptr, nullptr, at_).s;
     const double scale = 1.0 / std::sqrt(static_cast<double>(D));
     if (!f32) return attention_any(q, k, v, s.idx, s.cnt, e.causal, scale, out, std::nullopt, at_);
     const Tensor vc = v.stride(3) == 1 ? v : v.contiguous();
@@ -505,13 +541,13 @@ PyObject* py_estimate_and_select(PyObject*, PyObject* const* pv, Py_ssize_t n) {
   Tensor result;
   Selection s = without_gil([&] {
     const bool f32 = q.scalar_type() == at::kFloat;
-    const Tensor sums = estimate(q, k, g, e, nullptr, nullptr, at_);
-    // the sums in q's type: rounded by the selection kernel where it holds a row in registers (up to 1024 key blocks)
-    const bool in_select = !f32 && sums.size(3) <= 1024;
-    result = in_select ? empty(sums.sizes(), q.scalar_type(), at_.dev) : sums;
-    Selection r = select(sums, threshold, {g.bpc, g.block_offset, e.causal, true, sink, recent, true, 0, 0, 0}, at_, in_select ? &result : nullptr);
-    if (!f32 && !in_select) result = sums.to(q.scalar_type());
-    return r;
+    // the sums in q's type: rounded by the selection where it holds a row in registers (up to 1024 key blocks)
+    const bool in_select = !f32 && g.kb <= 1024;
+    if (in_select) result = empty({q.size(0), q.size(1), g.qb, g.kb}, q.scalar_type(), at_.dev);
+    Estimated r = estimate_and_select(q, k, g, e, threshold, {g.bpc, g.block_offset, e.causal, true, sink, recent, true, 0, 0, 0}, nullptr,
+                                      nullptr, in_select ? &result : nullptr, at_);
+    if (!in_select) result = f32 ? r.sums : r.sums.to(q.scalar_type());
+    return r.s;
   });
   PyObject* t = PyTuple_New(2);
   if (!t) throw python_error();
