@@ -1108,11 +1108,14 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // flight at a time and the first ones while the statistics are computed; the factors come from shared memory.  The longest query
 // blocks go first.  Calls of few query blocks (a short prompt's last chunk against a long cache) have four warps per query block.
 // (32 heads, 32768 tokens: at stride 16 20.5 us with a CTA per query block, 12.7 like this; at stride 8 21.8 and 14.8.)
+// kVec > 0: the query block's warp (of four: the first) then selects on its row of sums, of up to 128 * kVec, see select_row: as a
+// kernel of its own that was a launch and a hand-over between two kernels more (stride 8: 2500 tokens 47.0 -> 44.2 us a call, 3000
+// 51.4 -> 48.6, 1024 against 70000 103 -> 93; video diffusion 15100 -> 15000; at the power cap, from 8000 tokens on, nothing).
 constexpr int kSumThreads = 128;
-template <int RBS, int kTeam>
+template <int RBS, int kTeam, int kVec>
 __global__ void __launch_bounds__(kSumThreads)
 est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix, const float* __restrict__ partial,
-                    const float2* __restrict__ mtile, float* __restrict__ sums, int seg_tiles) {
+                    const float2* __restrict__ mtile, float* sums, int seg_tiles, const EstSelect sel) {
   extern __shared__ float s_factors[];                     // [team][tile][row] factors, seg_tiles tiles at a time
   __shared__ float2 s_part[4][RBS];                        // (teams of four warps) [warp][row] (max, sum)
   constexpr int kParts = kTeam / RBS, kTeams = kSumThreads / kTeam;
@@ -1226,6 +1229,10 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
         if (kl < n_out && ((t >= t0 && t < t1) || (t0 == 0 && t < 0))) out[kl] = acc[u];
       }
     }
+  }
+  if constexpr (kVec > 0) {
+    sync();
+    if (tid < 32) select_row<kVec>(sums, sel.p, sel.thr_per_head, sel.mask, sel.idx, sel.cnt, bh * g.qb_total + qb, threadIdx.x & 31);
   }
 }
 
@@ -1509,16 +1516,17 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     direct = g.band ? count == 1 && first * g.tile_n == (mt * kTileM / g.rcs) * g.rcs + g.row_off : count <= 1;
   }
   g.direct = direct ? 1 : 0;
-  // The block sums finished there can be selected on there, too: rows of up to 128 stored sums (four per lane).  Clusters of two do
+  // Block sums finished there can be selected on there, too: rows of up to 128 stored sums (four per lane).  Clusters of two do
   // not gain: a CTA has the rows of eight query blocks at stride 16, two rounds for its six warps (2100 tokens 35.4 us a call
-  // with it, 35.2 without).
+  // with it, 35.2 without).  Otherwise est_blocksum_kernel selects, rows of up to 1024.
   EstSelect sel;
   sel.on = 0;
   if (select) {
     const SelCall& c = *select;
     const int cols = g.band ? g.bpc : g.kb_total;
-    if (direct && (use_pairs || selects(g.tile_n / 128, f32)) && g.split != 2 && cols <= 128 && c.k_blocks <= 1024 && c.attn_sums == attn_sums && c.batch == batch && c.heads == hq &&
-        c.q_blocks == g.qb_total && c.k_blocks == g.kb_total && c.bpc == g.bpc && (c.band ? 1 : 0) == g.band) {
+    const bool here = direct ? (use_pairs || selects(g.tile_n / 128, f32)) && g.split != 2 && cols <= 128 : true;
+    if (here && c.k_blocks <= 1024 && c.attn_sums == attn_sums && c.batch == batch && c.heads == hq && c.q_blocks == g.qb_total &&
+        c.k_blocks == g.kb_total && c.bpc == g.bpc && (c.band ? 1 : 0) == g.band) {
       if ((rc = select_params(c, sel.p))) return rc;
       sel.on = 1;
       sel.thr_per_head = c.thr_per_head;
@@ -1679,13 +1687,26 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   auto launch_sums = [&](auto kern) -> int {
     return launch_dependent(kern, dim3(static_cast<unsigned>((items + teams - 1) / teams)), dim3(kSumThreads),
                             static_cast<size_t>(teams) * seg_tiles * g.rbs * sizeof(float), stream, g, (const int*)tile_lo,
-                            (const int*)tile_prefix, (const float*)partial, (const float2*)mtile, attn_sums, seg_tiles);
+                            (const int*)tile_prefix, (const float*)partial, (const float2*)mtile, attn_sums, seg_tiles, sel);
+  };
+  // with the selection: the instantiation with just enough registers for a row of sums
+  auto launch_vec = [&](auto rbs, auto team) -> int {
+    constexpr int kRbs = decltype(rbs)::value, kTeam = decltype(team)::value;
+    const int cols = g.band ? g.bpc : g.kb_total;
+    if (!sel.on) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 0>);
+    if (cols <= 128) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 1>);
+    if (cols <= 256) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 2>);
+    if (cols <= 512) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 4>);
+    return launch_sums(est_blocksum_kernel<kRbs, kTeam, 8>);
+  };
+  auto launch_team = [&](auto rbs) -> int {
+    return wide ? launch_vec(rbs, std::integral_constant<int, 128>()) : launch_vec(rbs, std::integral_constant<int, 32>());
   };
   switch (g.rbs) {
-    case 4: return wide ? launch_sums(est_blocksum_kernel<4, 128>) : launch_sums(est_blocksum_kernel<4, 32>);
-    case 8: return wide ? launch_sums(est_blocksum_kernel<8, 128>) : launch_sums(est_blocksum_kernel<8, 32>);
-    case 16: return wide ? launch_sums(est_blocksum_kernel<16, 128>) : launch_sums(est_blocksum_kernel<16, 32>);
-    case 32: return wide ? launch_sums(est_blocksum_kernel<32, 128>) : launch_sums(est_blocksum_kernel<32, 32>);
+    case 4: return launch_team(std::integral_constant<int, 4>());
+    case 8: return launch_team(std::integral_constant<int, 8>());
+    case 16: return launch_team(std::integral_constant<int, 16>());
+    case 32: return launch_team(std::integral_constant<int, 32>());
     default: return XATTN_B200_ERR_ARG;
   }
 }
