@@ -323,6 +323,18 @@ int xattn_b200_block_sparse_attn_ws(const void* q, const void* k, const void* v,
                                     void* workspace, size_t workspace_bytes, int* status, void* cuda_stream);
 
 /*
+ * The same for a caller who knows that no list has more than max_blocks blocks (0: unknown; the chunk-band estimate: those of a chunk
+ * and one): a hint at how to hand the work to the SMs, longer lists give the same results.
+ */
+int xattn_b200_block_sparse_attn_bounded(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv,
+                                    int q_len, int k_len, int head_dim, int64_t q_stride_b, int64_t q_stride_h,
+                                    int64_t q_stride_l, int64_t k_stride_b, int64_t k_stride_h, int64_t k_stride_l,
+                                    int64_t v_stride_b, int64_t v_stride_h, int64_t v_stride_l,
+                                    const int32_t* block_idx, const int32_t* block_cnt, int causal, float scale,
+                                    void* out, int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_l,
+                                    void* workspace, size_t workspace_bytes, int max_blocks, int* status, void* cuda_stream);
+
+/*
  * Decode step: dense attention of one query token per sequence (q [batch, hq, 1, 128]) against its key cache, which it may
  * see completely.  Replaces the third-party single-query attention of the reference's Llama patch
  * (xattn/src/load_llama.py:188-197); the same result as the general kernel up to the summation order.  hq / hkv <= 16,

@@ -145,3 +145,47 @@ def test_counts_beyond_a_row_of_the_lists(count):
     for workspace in (False, True):
         got = ops.block_sparse_attention(q, k, v, idx, torch.full_like(cnt, count), False, use_workspace=workspace)
         assert torch.equal(got, want if count > 0 else torch.zeros_like(want))
+
+
+@pytest.mark.parametrize("hq,hkv", [(7, 1), (32, 8), (6, 3)])
+def test_two_units_at_a_time(hq, hkv):
+    """Causal calls of many units with short lists take them in twos and keep K/V tiles in their slots from one to the next: against the same call
+    head by head, whose units are too few for that.  Lists as the selection leaves them and worse: the same in all heads, the same in
+    some, of 0 to 12 blocks, with and without the diagonal; odd groups, and (7 heads) an odd number of units."""
+    from xattn_b200 import _lib, ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = -(-24 * sms // hq) | 1                     # pairs of query blocks
+    L = 256 * rows - 131                              # ragged; an even number of query blocks
+    g = torch.Generator(device=DEV).manual_seed(hq)
+    q = torch.randn(1, hq, L, 128, device=DEV, generator=g).bfloat16()
+    k, v = (torch.randn(1, hkv, L, 128, device=DEV, generator=g).bfloat16() for _ in range(2))
+    n = (L + 127) // 128
+    cnt = torch.randint(0, 4, (1, 1, n), device=DEV, generator=g)
+    cnt = torch.where(torch.rand(1, 1, n, device=DEV, generator=g) < 0.1, torch.randint(5, 13, (1, 1, n), device=DEV, generator=g), cnt).expand(1, hq, n)
+    r = torch.arange(n, device=DEV)
+    # per head and row: block 0, the diagonal, then blocks in between, sorted, without repeats
+    mid = torch.rand(1, 1, n, 12, device=DEV, generator=g).expand(1, hq, n, 12).clone()
+    own = torch.rand(1, hq, n, 1, device=DEV, generator=g) < 0.3            # lists of their own
+    mid = torch.where(own, torch.rand(1, hq, n, 12, device=DEV, generator=g), mid)
+    cand = (mid * (r + 1)[:, None]).long()
+    cand[..., 0] = r
+    cand[..., 1] = 0
+    cand = torch.where(torch.arange(12, device=DEV) < cnt[..., None], cand, n)
+    cand = cand.sort(-1).values
+    keep = (cand < n) & torch.cat([torch.ones_like(cand[..., :1], dtype=torch.bool), cand[..., 1:] != cand[..., :-1]], -1)
+    order = (~keep).long().sort(dim=-1, stable=True).indices
+    idx = torch.zeros(1, hq, n, n, dtype=torch.int32, device=DEV)
+    idx[..., :12] = cand.gather(-1, order).clamp(max=n - 1)
+    cnt = keep.sum(-1).to(torch.int32)
+    out = torch.empty(1, L, hq, 128, dtype=q.dtype, device=DEV).transpose(1, 2)
+    lib = _lib.load()
+    _lib.check(lib.xattn_b200_block_sparse_attn_bounded(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.BF16, 1, hq, hkv, L, L, 128, *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
+        idx.data_ptr(), cnt.data_ptr(), 1, 128 ** -0.5, out.data_ptr(), *out.stride()[:3], None, 0, 13, None,
+        torch.cuda.current_stream().cuda_stream), "block_sparse_attn_bounded")
+    assert torch.equal(out, ops.block_sparse_attention(q, k, v, idx, cnt, True))
+    for h in range(hq):
+        kv = h // (hq // hkv)
+        one = ops.block_sparse_attention(q[:, h:h + 1], k[:, kv:kv + 1], v[:, kv:kv + 1], idx[:, h:h + 1], cnt[:, h:h + 1], True)
+        assert torch.equal(out[:, h], one[:, 0]), h
+    ops.check_device_status()

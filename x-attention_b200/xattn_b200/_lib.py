@@ -49,6 +49,9 @@ SIGNATURES = {
     "xattn_b200_block_sparse_attn_ws": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, _i,
                                              _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64,
                                              _p, _p, _i, _f, _p, _i64, _i64, _i64, _p, _sz, _p, _p]),
+    "xattn_b200_block_sparse_attn_bounded": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, _i,
+                                             _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64,
+                                             _p, _p, _i, _f, _p, _i64, _i64, _i64, _p, _sz, _i, _p, _p]),
     "xattn_b200_decode_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "xattn_b200_decode_attn": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64,
                                     _f, _p, _i64, _i64, _p, _sz, _p, _p]),

@@ -43,6 +43,7 @@
 #include <math.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "attention_common.cuh"
 
@@ -63,6 +64,7 @@ constexpr int kUnitSlots = 4;
 constexpr int kUnitReaders = 13;                              // warps that read it
 constexpr int kAttnSmem = kAttnSmemTiles + kStageBytes + 2 * 2 * 128 * 4 /*row sums*/ + kRingEntries * 4 +
                           kUnitSlots * 2 * 16 + 16 + 512 /*barriers*/;
+constexpr int kReuseBlocks = 8;           // lists up to that length may find a K/V tile of the unit before in its slot (longer: not worth the look)
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 struct Tile {
@@ -157,7 +159,8 @@ struct Units {
 
 // kBf16: bf16 or fp16 (a template parameter: as a run-time switch every packed pair cost both conversions and a select).
 // kOutF32: the output is written as fp32.  kList: the units may come from a list.
-template <bool kBf16, bool kOutF32, bool kList>
+// kTwo: a CTA takes two units next to one another at a time (the causal numbering, no list of units), see the loader.
+template <bool kBf16, bool kOutF32, bool kList, bool kTwo>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -252,9 +255,14 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       auto wait = [&](uint32_t b, uint32_t ph) -> bool { return __all_sync(0xffffffffu, mbar_wait(b, ph, abort_flag)); };
       Tile tn;
       List ln;                                          // the next unit's, with the first window
-      int wn = 0, unit = blockIdx.x;
-      // the first turn of the loop has no lists to load, it only fetches those of the CTA's own unit; turn k works on the
-      // CTA's unit k - 1 and requests and fetches unit k
+      int wn = 0, unit = kTwo ? 2 * blockIdx.x : blockIdx.x;
+      bool second = false;                              // (kTwo) `unit` is the second one of its request
+      uint32_t requests = 0;
+      int held[2] = {-1, -1};                           // (kTwo) the K/V tiles in the two slots, numbered through batch and heads
+      // The first turn of the loop has no lists to load, it only fetches those of the CTA's own unit; turn k works on the
+      // CTA's unit k - 1 and requests and fetches unit k.  With two units per request (kTwo) the second one is the
+      // other pair of heads at the same rows, whose list is mostly the same: of two blocks (sink and diagonal), say, both are still
+      // in the slots where the second unit wants them, and are not loaded again.
       ln.n = 0;
       ln.last = nullptr;
       tn.b = tn.h = 0;
@@ -263,7 +271,10 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         const List l = ln;
         int i = 0, w = wn, g_;
         const int kvh = __shfl_sync(0xffffffffu, fast_div(tn.h, p.by_group, g_), 0), b = __shfl_sync(0xffffffffu, tn.b, 0);
-        if (k > 0 && lane == 0 && !(kList && rest_list)) {
+        const bool more = kTwo && k > 0 && !second && unit + 1 < rest_units, request = k > 0 && !more && !(kList && rest_list);
+        const int tile0 = (b * p.hkv + kvh) * p.list_k_blocks;
+        const bool reuse = kTwo && __all_sync(0xffffffffu, l.n <= kReuseBlocks);
+        if (request && lane == 0) {
           mbar_expect_tx(answer_full, 16);
           clc_try_cancel(smem_u32(answer), answer_full);
         }
@@ -281,18 +292,31 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
             e |= __shfl_xor_sync(0xffffffffu, e, 16);
             const int sl = step & 1;
             const uint32_t ph = ((step >> 1) & 1) ^ 1, dst = smem_u32(smem + (2 + 2 * sl) * kTile16);
+            bool there = false;
+            if constexpr (kTwo) {
+              if (reuse) there = (sl ? held[1] : held[0]) == tile0 + blk;
+              if (sl) held[1] = tile0 + blk; else held[0] = tile0 + blk;
+            }
             if (!wait(bar(sl, K_EMPTY), ph)) { ok = false; break; }
             if (lane == 0) {
               XB_TRACE_EV(0x12, step);
               ring[step & (kRingEntries - 1)] = e;
-              mbar_expect_tx(bar(sl, K_FULL), kTile16);
-              tma_load_5d(dst, &tmK, bar(sl, K_FULL), 0, blk * 128, 0, kvh, b);
+              if (kTwo && there) {
+                mbar_arrive(bar(sl, K_FULL));
+              } else {
+                mbar_expect_tx(bar(sl, K_FULL), kTile16);
+                tma_load_5d(dst, &tmK, bar(sl, K_FULL), 0, blk * 128, 0, kvh, b);
+              }
             }
             if (!wait(bar(sl, V_EMPTY), ph)) { ok = false; break; }
             if (lane == 0) {
               XB_TRACE_EV(0x13, step);
-              mbar_expect_tx(bar(sl, V_FULL), kTile16);
-              tma_load_5d(dst + kTile16, &tmV, bar(sl, V_FULL), 0, blk * 128, 0, kvh, b);
+              if (kTwo && there) {
+                mbar_arrive(bar(sl, V_FULL));
+              } else {
+                mbar_expect_tx(bar(sl, V_FULL), kTile16);
+                tma_load_5d(dst + kTile16, &tmV, bar(sl, V_FULL), 0, blk * 128, 0, kvh, b);
+              }
             }
             ++step;
             if (f && (++i & 15) == 0) {
@@ -309,9 +333,15 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
             if (kList && rest_list) {
               if (k > 0) unit += gridDim.x;
               if (unit >= rest_units) unit = -1;
-            } else if (k > 0) {
-              if (!wait(answer_full, (k - 1) & 1)) { ok = false; break; }
+            } else if (more) {
+              ++unit;
+              second = true;
+            } else if (request) {
+              if (!wait(answer_full, requests & 1)) { ok = false; break; }
+              ++requests;
               unit = clc_answer(smem_u32(answer));
+              if (kTwo && unit > 0) unit *= 2;
+              second = false;
               fence_proxy_async_smem();                 // read before the next answer is written
             }
             ln.n = -1;
@@ -916,7 +946,7 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
                              int q_len, int k_len, int head_dim, int64_t qsb, int64_t qsh, int64_t qsl, int64_t ksb,
                              int64_t ksh, int64_t ksl, int64_t vsb, int64_t vsh, int64_t vsl,
                              const int32_t* block_idx, const int32_t* block_cnt, int causal, float scale, void* out,
-                             int64_t osb, int64_t osh, int64_t osl, void* workspace, size_t workspace_bytes,
+                             int64_t osb, int64_t osh, int64_t osl, void* workspace, size_t workspace_bytes, int max_list,
                              int* status, cudaStream_t stream) {
   if (!q || !k || !v || !out || (block_idx == nullptr) != (block_cnt == nullptr)) return XATTN_B200_ERR_ARG;
   const bool dense = block_idx == nullptr;
@@ -973,18 +1003,27 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
   }
   // (a dependent launch in every case: after the pair kernel, or after whatever kernel produced the block lists)
   const long long sms = sm_count();
-  const unsigned grid = static_cast<unsigned>(rest && units > sms ? sms : units);
+  // Two units at a time where the caller knows the lists to be short and there are enough units to go round: at least as many per SM as
+  // a list has blocks, so that two of the longest are no more than the tail of the call (32 heads, this kernel: 128K tokens, 111 units
+  // per SM, lists of up to 17 blocks, mostly 2: 661 -> 647 us at the power cap and 556 -> 542 in short runs; 9973 tokens, 8 units
+  // per SM, 81 -> 84; 58695 tokens, whose few rows of hundreds of blocks then met on one SM, 400 -> 640).  The look at the slots
+  // stays out of the other calls: it cost dense ones 1 %.
+  const bool two = causal && !dense && !rest && max_list > 0 && units >= 24 * sms && units >= max_list * sms &&
+                   static_cast<long long>(batch) * hkv * p.list_k_blocks < 0x7fffffffLL;
+  const unsigned grid = static_cast<unsigned>(rest && units > sms ? sms : (two ? (units + 1) / 2 : units));
   auto launch = [&](auto kern) -> int {
     if (!allow_smem(kern, kAttnSmem))
       return XATTN_B200_ERR_CUDA;
     return launch_dependent(kern, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tmQ, tmK,
                             tmV, tmO, p, block_idx, block_cnt, rest, pair_header, min_share, status);
   };
-  if (p.tile_list || rest)
-    return out_f32 ? launch(block_sparse_attn_kernel<true, true, true>)
-                   : (p.is_bf16 ? launch(block_sparse_attn_kernel<true, false, true>) : launch(block_sparse_attn_kernel<false, false, true>));
-  return out_f32 ? launch(block_sparse_attn_kernel<true, true, false>)
-                 : (p.is_bf16 ? launch(block_sparse_attn_kernel<true, false, false>) : launch(block_sparse_attn_kernel<false, false, false>));
+  auto launch_type = [&](auto list, auto pairs) -> int {
+    constexpr bool kList = decltype(list)::value, kTwo = decltype(pairs)::value;
+    return out_f32 ? launch(block_sparse_attn_kernel<true, true, kList, kTwo>)
+                   : (p.is_bf16 ? launch(block_sparse_attn_kernel<true, false, kList, kTwo>) : launch(block_sparse_attn_kernel<false, false, kList, kTwo>));
+  };
+  if (p.tile_list || rest) return launch_type(std::true_type(), std::false_type());
+  return two ? launch_type(std::false_type(), std::true_type()) : launch_type(std::false_type(), std::false_type());
 }
 
 }  // namespace xb

@@ -328,19 +328,19 @@ Estimated estimate_and_select(const Tensor& q, const Tensor& k, const Geometry& 
 // Attention over block lists (undefined: dense).  q, k, v 16 bit.  `out`: undefined, or [B, Hq, Lq, 128] with unit inner
 // stride.  out_f32: write fp32 (bf16 inputs only).  Returns a transposed view of [B, Lq, Hq, D] storage, or `out`.
 Tensor attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& idx, const Tensor& cnt, bool causal, double scale,
-                 Tensor out, bool out_f32, bool use_workspace, const Place& at_) {
+                 Tensor out, bool out_f32, bool use_workspace, const Place& at_, int max_blocks = 0) {
   const Tensor q = aligned16(q_), k = aligned16(k_), v = aligned16(v_);
   const int64_t B = q.size(0), Hq = q.size(1), Lq = q.size(2), D = q.size(3), Hkv = k.size(1), Lk = k.size(2);
   if (!out.defined()) out = empty({B, Lq, Hq, D}, out_f32 ? at::kFloat : q.scalar_type(), at_.dev).transpose(1, 2);
   const size_t bytes = use_workspace ? xattn_b200_block_sparse_attn_workspace_bytes(B, Hq, Hkv, Lq, Lk) : 0;
   Tensor ws;
   if (bytes) ws = empty({static_cast<int64_t>(bytes)}, at::kByte, at_.dev);
-  check(xattn_b200_block_sparse_attn_ws(
+  check(xattn_b200_block_sparse_attn_bounded(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), out_f32 ? XATTN_B200_BF16_OUT_F32 : dtype_code(q.scalar_type()), B, Hq, Hkv, Lq, Lk,
             D, q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
             idx.defined() ? static_cast<const int32_t*>(idx.data_ptr()) : nullptr,
             cnt.defined() ? static_cast<const int32_t*>(cnt.data_ptr()) : nullptr, causal, static_cast<float>(scale), out.data_ptr(),
-            out.stride(0), out.stride(1), out.stride(2), bytes ? ws.data_ptr() : nullptr, bytes, at_.status, at_.stream),
+            out.stride(0), out.stride(1), out.stride(2), bytes ? ws.data_ptr() : nullptr, bytes, max_blocks, at_.status, at_.stream),
         "block_sparse_attn");
   return out;
 }
@@ -407,7 +407,7 @@ PyObject* py_select(PyObject*, PyObject* const* v, Py_ssize_t n) {
 }
 
 Tensor attention_any(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx, const Tensor& cnt, bool causal, double scale,
-                     Tensor out, std::optional<bool> use_workspace, const Place& at_) {
+                     Tensor out, std::optional<bool> use_workspace, const Place& at_, int max_blocks = 0) {
   const int64_t D = q.size(3);
   if (D != 128) fail(PyExc_ValueError, "head_dim must be 128");
   const bool f32 = q.scalar_type() == at::kFloat, dense = !idx.defined();
@@ -421,7 +421,7 @@ Tensor attention_any(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   if (!dense && (idx.sizes() != at::IntArrayRef({q.size(0), q.size(1), lqb, lkb}) || cnt.sizes() != at::IntArrayRef({q.size(0), q.size(1), lqb})))
     fail(PyExc_ValueError, "block lists have the wrong shape");
   const bool ws = dense ? false : use_workspace.value_or(default_workspace(causal, dense, q));
-  return attention(q16, k16, v16, dense ? idx : idx.contiguous(), dense ? cnt : cnt.contiguous(), causal, scale, out, f32 && !out.defined(), ws, at_);
+  return attention(q16, k16, v16, dense ? idx : idx.contiguous(), dense ? cnt : cnt.contiguous(), causal, scale, out, f32 && !out.defined(), ws, at_, max_blocks);
 }
 
 // attention(q, k, v, idx, cnt, causal, scale, out, use_workspace) -> out
@@ -513,13 +513,15 @@ PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
     const Selection s = estimate_and_select(q, k, g, e, threshold, {g.bpc, g.block_offset, e.causal, true, sink, recent, false, Lq, Lk, 0},
                                             f32 ? &q16 : nullptr, f32 ? &k16 : nullptr, nullptr, at_).s;
     const double scale = 1.0 / std::sqrt(static_cast<double>(D));
-    if (!f32) return attention_any(q, k, v, s.idx, s.cnt, e.causal, scale, out, std::nullopt, at_);
+    // (a row's own chunk and block 0; keep_sink sets a whole row, of the first block)
+    const int max_blocks = e.band && !sink ? g.bpc + 1 : 0;
+    if (!f32) return attention_any(q, k, v, s.idx, s.cnt, e.causal, scale, out, std::nullopt, at_, max_blocks);
     const Tensor vc = v.stride(3) == 1 ? v : v.contiguous();
     const Tensor v16 = empty(v.sizes(), at::kBFloat16, at_.dev);
     check(xattn_b200_split_f32_terms(static_cast<const float*>(vc.data_ptr()), v.size(0), v.size(1), Lk, Lk, D, vc.stride(0), vc.stride(1),
                                      vc.stride(2), 1, v16.data_ptr(), at_.stream),
           "split_f32_terms");
-    return attention(q16, k16, v16, s.idx, s.cnt, e.causal, scale, out, true, default_workspace(e.causal, false, q), at_);
+    return attention(q16, k16, v16, s.idx, s.cnt, e.causal, scale, out, true, default_workspace(e.causal, false, q), at_, max_blocks);
   }));
   END_PY
 }
