@@ -189,3 +189,28 @@ def test_two_units_at_a_time(hq, hkv):
         one = ops.block_sparse_attention(q[:, h:h + 1], k[:, kv:kv + 1], v[:, kv:kv + 1], idx[:, h:h + 1], cnt[:, h:h + 1], True)
         assert torch.equal(out[:, h], one[:, 0]), h
     ops.check_device_status()
+
+
+# (batch, query heads, kv heads, keys): clusters of eight and of sixteen and the second kernel, and the lines between them; deep
+# rings and not; ragged last stages, CTAs of unequal numbers of stages; 1 to 16 rows per kv head; strided caches
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,hq,hkv,n", [
+    (1, 32, 8, 4096), (1, 32, 8, 4097), (1, 32, 8, 4160), (1, 32, 8, 49152), (1, 32, 8, 49153), (1, 28, 4, 5000), (1, 28, 4, 102400),
+    (1, 28, 4, 102401), (1, 16, 1, 4111), (7, 1, 1, 6000), (2, 14, 7, 4500), (3, 5, 5, 4500), (2, 32, 8, 4500), (1, 12, 2, 20001), (3, 28, 4, 2500)])
+def test_decode_splits(B, hq, hkv, n, dtype):
+    from xattn_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(n + hq)
+    q = torch.randn(B, 1, hq, 128, device=DEV, generator=g).to(dtype).transpose(1, 2)
+    k = torch.randn(B, n, hkv, 128, device=DEV, generator=g).to(dtype).transpose(1, 2)
+    v = torch.randn(B, hkv, n, 128, device=DEV, generator=g).to(dtype)
+    out = ops.decode_attention(q, k, v)
+    rep = hq // hkv
+    for b in range(B):
+        for h in range(hkv):
+            s = q[b, h * rep:(h + 1) * rep, 0].double() @ k[b, h].double().T * 128 ** -0.5
+            want = s.softmax(-1) @ v[b, h].double()
+            # probabilities and results rounded to 8 or 11 bits: each at most half a unit in the last place, both together less than one
+            tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+            err = (out[b, h * rep:(h + 1) * rep, 0].double() - want).norm() / want.norm()
+            assert err < tol, (b, h, float(err))
+    ops.check_device_status()

@@ -17,22 +17,25 @@
 //     they are a cluster (up to eight: caches of up to 4096 keys, or many heads), and by a small second kernel, launched as a
 //     dependent one, where there are more.  The second launch costs the host 2.5 us, which a step on a short cache would pay
 //     in full (2011 keys, 8 kv heads: 10.2 us a call with it, 6.0 without); a long cache hides it.
+#include <type_traits>
+
 #include "attention_common.cuh"
 
 namespace xb {
 
 constexpr int kDecWarps = 4;
-constexpr int kDecThreads = kDecWarps * 32;
+__host__ __device__ constexpr int dec_threads(bool wide) { return kDecWarps * 32 + (wide ? 32 : 0); }   // (wide: and a warp that loads)
 constexpr int kDecKeys = 64;                              // keys per stage: 16 per warp
 constexpr int kDecTile = kDecKeys * 128 * 2;              // [2 column halves][64 keys][64 columns], 128-byte swizzle
-constexpr int kDecStages = 3;
+constexpr int kDecStages = 3, kDecMaxStages = 6;          // of the ring: three for two CTAs per SM, up to six for one
 constexpr int kDecMaxRows = 16;                           // query heads per kv head
-constexpr int kDecSmem = kDecStages * 2 * kDecTile + 1024 /*alignment slack*/ + 256 /*barriers*/;
+constexpr int dec_smem(int ring) { return ring * 2 * kDecTile + 1024 /*alignment slack*/ + 256 /*barriers*/; }
 constexpr float kDecRescale = 8.0f;                       // log2 units: the running maximum moves lazily
 
 struct DecodeParams {
   int batch, hkv, group, k_len, splits, stages;           // stages: 64-key stages of the whole cache
   int cluster;                                            // the splits are a cluster
+  int ring;                                               // stages of the ring
   float scale_log2;
   int64_t qsb, qsh, osb, osh;
 };
@@ -58,23 +61,28 @@ __device__ __forceinline__ void warp_mma(float (&c)[4], const uint32_t (&a)[4], 
 }
 
 // part: [batch * hkv][splits][group][128] un-normalised outputs, then [..][splits][group] (max, sum) pairs
-template <bool kBf16>
-__global__ void __launch_bounds__(kDecThreads, 2)
+// kWide: the kernel for clusters of sixteen, and for smaller ones that have an SM per CTA.  Its ring may be deeper, and it has a warp
+// of its own that refills a slot as soon as the four warps are done with it; one of them does it a stage later, which leaves a CTA
+// a stage less in flight (30000 keys, 4 kv heads: 17.8 us a call against 26.3).  The others, two CTAs per SM, have enough in flight,
+// and with that warp their merge kernel came 5 us later.
+template <bool kBf16, bool kWide>
+__global__ void __launch_bounds__(dec_threads(kWide), 2)
 decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const uint16_t* __restrict__ q, const DecodeParams p, float* __restrict__ part,
                    float2* __restrict__ part_ml, uint16_t* __restrict__ out, int* status) {
+  const int ring = kWide ? p.ring : kDecStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kDecStages * 2 * kDecTile);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kDecStages);
-  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kDecStages);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + ring * 2 * kDecTile);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kDecMaxStages);
+  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kDecMaxStages);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int split = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
   // stages [s0, s1) of the cache
   const int s0 = static_cast<int>(static_cast<long long>(p.stages) * split / p.splits);
   const int s1 = static_cast<int>(static_cast<long long>(p.stages) * (split + 1) / p.splits);
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kDecStages; ++s) {
+    for (int s = 0; s < ring; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, kDecWarps);
     }
@@ -84,17 +92,31 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   __syncthreads();
   pdl_launch_dependents();              // the next kernel may take its place; it waits for this grid to end
   pdl_wait();
-  auto load_stage = [&](int i) {        // one thread: the CTA's i-th stage
-    const int st = i % kDecStages;
+  auto load_stage = [&](int i, int st) {        // one thread: the CTA's i-th stage, into slot st
     const uint32_t dst = smem_u32(smem) + st * 2 * kDecTile;
     mbar_expect_tx(full0 + 8 * st, 2 * kDecTile);
     tma_load_5d(dst, &tmK, full0 + 8 * st, 0, (s0 + i) * kDecKeys, 0, g, b);
     tma_load_5d(dst + kDecTile, &tmV, full0 + 8 * st, 0, (s0 + i) * kDecKeys, 0, g, b);
   };
   const int n = s1 - s0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < kDecStages && i < n; ++i) load_stage(i);
-
+  constexpr int kDecThreads = dec_threads(kWide);
+  if (!kWide && threadIdx.x == 0)
+    for (int i = 0; i < ring && i < n; ++i) load_stage(i, i);
+  if (kWide && warp == kDecWarps) {
+    if (lane == 0) {
+      int st = 0;
+      uint32_t ph = 1;
+      for (int i = 0; i < n; ++i) {
+        if (i >= ring && !mbar_wait(empty0 + 8 * st, ph, abort_flag)) break;
+        load_stage(i, st);
+        if (++st == ring) { st = 0; ph ^= 1; }
+      }
+    }
+    __syncwarp();
+  }
+  float o[16][4];
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // rows lane / 4 and lane / 4 + 8
+  if (warp < kDecWarps) {
   // Q as A operand: rows = query heads of the group (rows past it zero), 8 steps of 16 columns
   uint32_t qa[8][4];
   {
@@ -114,19 +136,18 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       }
     }
   }
-  float o[16][4];
 #pragma unroll
   for (int t = 0; t < 16; ++t)
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[t][e] = 0.f;
-  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // rows lane / 4 and lane / 4 + 8
   // ldmatrix addresses: lane's row inside the warp's 16 keys; chunk c of 16 bytes of row r sits at chunk c ^ (r & 7)
   const int krow = warp * 16 + (lane & 7) + ((lane >> 4) << 3), kchunk = (lane >> 3) & 1;   // K: keys 0-7 | 8-15, columns 0-7 | 8-15
   const int vrow = warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), vchunk = lane >> 4;   // V: the same, transposed on load
   bool ok = true;
+  int st = 0, last = ring - 1;                           // this stage's slot, the slot of the one before
+  uint32_t ph = 0, last_ph = 1;                            // and the phases of their barriers
   for (int i = 0; i < n; ++i) {
-    const int st = i % kDecStages;
-    if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * st, (i / kDecStages) & 1, abort_flag))) { ok = false; break; }
+    if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * st, ph, abort_flag))) break;
     const uint32_t kt = smem_u32(smem) + st * 2 * kDecTile, vt = kt + kDecTile;
     float s[2][4] = {};                                    // keys 0-7, 8-15 of the warp
 #pragma unroll
@@ -184,22 +205,28 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       warp_mma<kBf16>(o[2 * c], pa, vb[0], vb[1]);
       warp_mma<kBf16>(o[2 * c + 1], pa, vb[2], vb[3]);
     }
-    if (i + kDecStages < n) fence_proxy_async_smem();      // every lane's reads of the stage come before the TMA writes that refill it
+    if (i + ring < n) fence_proxy_async_smem();      // every lane's reads of the stage come before the TMA writes that refill it
     __syncwarp();
     if (lane == 0) mbar_arrive(empty0 + 8 * st);
-    if (threadIdx.x == 0 && i > 0 && i - 1 + kDecStages < n) {
-      // the stage before this one is refilled: by now every warp is done with it, or nearly
-      if (mbar_wait(empty0 + 8 * ((i - 1) % kDecStages), ((i - 1) / kDecStages) & 1, abort_flag)) load_stage(i - 1 + kDecStages);
-      else ok = false;
+    if constexpr (!kWide) {
+      if (threadIdx.x == 0 && i > 0 && i - 1 + ring < n) {
+        // the stage before this one is refilled: by now every warp is done with it, or nearly
+        if (mbar_wait(empty0 + 8 * last, last_ph, abort_flag)) load_stage(i - 1 + ring, last);
+        else ok = false;
+      }
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      if (!ok) break;
+      last = st;
+      last_ph = ph;
     }
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    if (!ok) break;
+    if (++st == ring) { st = 0; ph ^= 1; }
   }
   // row sums over the four lanes of a row
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+  }
   }
   __syncthreads();                       // every stage has been read: the ring becomes the exchange buffer
   const bool aborted = *abort_flag != 0;
@@ -213,7 +240,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   float2* xml = reinterpret_cast<float2*>(smem + kDecWarps * kDecMaxRows * 128 * 4);     // [warp][16 rows]
   float* res = xo + kDecWarps * kDecMaxRows * 128 + 2 * kDecWarps * kDecMaxRows;          // [16 rows][128], the CTA's part
   float2* res_ml = reinterpret_cast<float2*>(res + kDecMaxRows * 128);                    // [16 rows]
-  {
+  if (warp < kDecWarps) {
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -260,26 +287,30 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     cluster_sync_all();
     for (int e = split * kDecThreads + threadIdx.x; e < p.group * 64; e += p.splits * kDecThreads) {
       const int r = e >> 6, c = (e & 63) * 2;
-      float2 ml[8], v[8];
-      float mm = -INFINITY;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        ml[s] = make_float2(-INFINITY, 0.f);
-        v[s] = make_float2(0.f, 0.f);
-        if (s < p.splits) {
-          ml[s] = ld_shared_cluster_f2(mapa_shared(smem_u32(res_ml + r), s));
-          v[s] = ld_shared_cluster_f2(mapa_shared(smem_u32(res + r * 128 + c), s));
-        }
-        mm = fmaxf(mm, ml[s].x);
-      }
       float a0 = 0.f, a1 = 0.f, ll = 0.f;
+      auto merge = [&](auto most) {                        // parts of up to `most` CTAs
+        constexpr int kParts = decltype(most)::value;
+        float2 ml[kParts], v[kParts];
+        float mm = -INFINITY;
 #pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        const float f = ml[s].x == -INFINITY ? 0.f : fast_exp2(ml[s].x - mm);
-        a0 += v[s].x * f;
-        a1 += v[s].y * f;
-        ll += ml[s].y * f;
-      }
+        for (int s = 0; s < kParts; ++s) {
+          ml[s] = make_float2(-INFINITY, 0.f);
+          v[s] = make_float2(0.f, 0.f);
+          if (s < p.splits) {
+            ml[s] = ld_shared_cluster_f2(mapa_shared(smem_u32(res_ml + r), s));
+            v[s] = ld_shared_cluster_f2(mapa_shared(smem_u32(res + r * 128 + c), s));
+          }
+          mm = fmaxf(mm, ml[s].x);
+        }
+#pragma unroll
+        for (int s = 0; s < kParts; ++s) {
+          const float f = ml[s].x == -INFINITY ? 0.f : fast_exp2(ml[s].x - mm);
+          a0 += v[s].x * f;
+          a1 += v[s].y * f;
+          ll += ml[s].y * f;
+        }
+      };
+      merge(std::integral_constant<int, kWide ? 16 : 8>());
       const float inv = ll > 0.f ? 1.f / ll : 0.f;
       *reinterpret_cast<uint32_t*>(out + b * p.osb + static_cast<int64_t>(g * p.group + r) * p.osh + c) =
           pack16t<kBf16>(a0 * inv, a1 * inv);
@@ -336,14 +367,25 @@ decode_merge_kernel(const DecodeParams p, const float* __restrict__ part, const 
 // Number of splits: two CTAs per SM over all (batch, kv head) pairs, at least two stages each (a split costs a CTA's start
 // and its row of the merge, about what two stages take).  Up to eight of them are a cluster, whose size is a power of two;
 // so are those of caches of up to 4096 keys, where eight CTAs of eight stages take about as long as the second kernel.
-constexpr int kDecClusterMax = 8, kDecClusterStages = 64;
+// Longer caches: clusters of sixteen, where all of them fit on the chip at the same time (14 on this one with two CTAs per SM, half as
+// many with one), rather than more CTAs and a second kernel, which starts when the first has ended and reads what it wrote.  us a
+// call, 1 sequence, 32 / 8 heads: 4200 keys 13.6 -> 8.1, 9000 16.2 -> 11.5, 30000 28.7 -> 25.8; 28 / 4 heads: 4200 11.7 -> 7.4, 30000
+// 27.6 -> 18.0, 60000 36.9 -> 30.2; 8 / 1 heads, 30000 keys: 45 -> 17.  Up to 128 of 148 SMs stream then, and with rings of three
+// 43 GB/s each (5.5 TB/s), so that from about 50 stages per CTA on the second kernel is the lesser cost (60000 keys: 47.3 and
+// 46.3); with deep rings 73 GB/s each, and the line lies at about 100 (100000 keys, 4 heads: 46.4 and 47.5, 2 heads: 45.6 and 45.0).
+constexpr int kDecClusterMax = 8, kDecClusterStages = 64, kDecClusterWide = 16;
+constexpr int kDecWideStages = 48, kDecWideStagesDeep = 100;      // stages per CTA up to which sixteen are the faster way (rings of 3, of 6)
+static int wide_clusters();                              // clusters of sixteen that can be on the device at a time
 static int decode_splits(int batch, int hkv, int k_len, int& cluster) {
   const int stages = (k_len + kDecKeys - 1) / kDecKeys;
   const long long heads = static_cast<long long>(batch) * hkv;
   long long s = 2LL * sm_count() / heads;
   if (s > stages / 2) s = stages / 2;
   if (s > kDecClusterMax && (stages <= kDecClusterStages || s < kDecClusterMax * 3 / 2)) s = kDecClusterMax;
-  cluster = s > 1 && s <= kDecClusterMax ? 1 : 0;
+  if (s > kDecClusterMax && s >= kDecClusterWide && heads <= wide_clusters() &&
+      stages <= kDecClusterWide * (2 * heads <= wide_clusters() ? kDecWideStagesDeep : kDecWideStages))
+    s = kDecClusterWide;
+  cluster = s > 1 && (s <= kDecClusterMax || s == kDecClusterWide) ? 1 : 0;
   if (cluster)
     while (s & (s - 1)) s &= s - 1;
   return s < 1 ? 1 : static_cast<int>(s);
@@ -355,6 +397,40 @@ size_t decode_workspace_bytes(int batch, int hq, int hkv, int k_len) {
   const int splits = decode_splits(batch, hkv, k_len, cluster);
   if (cluster || splits == 1) return 0;
   return static_cast<size_t>(batch) * hq * splits * (128 * sizeof(float) + sizeof(float2));
+}
+
+// once per kernel and device: its shared memory, and (wide) clusters of sixteen
+template <typename K>
+static bool dec_allow(K kern, bool wide) {
+  return once_per_device(reinterpret_cast<const void*>(kern), [&]() {
+    const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_smem(kDecMaxStages)) == cudaSuccess &&
+                    (!wide || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess);
+    if (!ok) cudaGetLastError();
+    return ok ? 1 : 0;
+  }) > 0;
+}
+static int wide_clusters() {
+  static const char key = 0;
+  return once_per_device(&key, []() {
+    const auto kern = decode_attn_kernel<true, true>;
+    if (!dec_allow(kern, true)) return 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kDecClusterWide, 64, 1);
+    cfg.blockDim = dim3(dec_threads(true), 1, 1);
+    cfg.dynamicSmemBytes = dec_smem(kDecStages);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kDecClusterWide;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int m = 0;
+    if (cudaOccupancyMaxActiveClusters(&m, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return m;
+  });
 }
 
 int decode_launch(const void* q, const void* k, const void* v, int dtype, int batch, int hq, int hkv, int k_len,
@@ -375,6 +451,13 @@ int decode_launch(const void* q, const void* k, const void* v, int dtype, int ba
   p.batch = batch; p.hkv = hkv; p.group = hq / hkv; p.k_len = k_len;
   p.stages = (k_len + kDecKeys - 1) / kDecKeys;
   p.splits = decode_splits(batch, hkv, k_len, p.cluster);
+  // where every CTA has an SM to itself its ring is deeper (of sixteen, whose clusters are counted for rings of three: half as many)
+  p.ring = kDecStages;
+  const long long heads = static_cast<long long>(batch) * hkv;
+  if (p.splits > kDecClusterMax ? p.cluster && 2 * heads <= wide_clusters() : 4 * p.splits * heads <= 3LL * sm_count()) {
+    const int most = (p.stages + p.splits - 1) / p.splits;
+    p.ring = most < kDecStages ? kDecStages : (most > kDecMaxStages ? kDecMaxStages : most);
+  }
   p.scale_log2 = scale * 1.4426950408889634f;
   p.qsb = qsb; p.qsh = qsh; p.osb = osb; p.osh = osh;
   const size_t need = decode_workspace_bytes(batch, hq, hkv, k_len);
@@ -385,17 +468,20 @@ int decode_launch(const void* q, const void* k, const void* v, int dtype, int ba
   CUtensorMap tmK, tmV;
   if ((rc = make_qkv_map(&tmK, k, k_len, hkv, batch, ksb, ksh, ksl, kDecKeys))) return rc;
   if ((rc = make_qkv_map(&tmV, v, k_len, hkv, batch, vsb, vsh, vsl, kDecKeys))) return rc;
+  const bool wide = p.cluster && (p.splits > kDecClusterMax || p.ring > kDecStages);
   auto launch = [&](auto kern, auto merge) -> int {
-    if (!allow_smem(kern, kDecSmem))
+    if (!dec_allow(kern, wide))
       return XATTN_B200_ERR_CUDA;
-    const int r = launch_dependent_clusters(kern, p.cluster ? p.splits : 1, dim3(p.splits, hkv, batch), dim3(kDecThreads), kDecSmem, stream,
+    const int r = launch_dependent_clusters(kern, p.cluster ? p.splits : 1, dim3(p.splits, hkv, batch), dim3(dec_threads(wide)), dec_smem(p.ring), stream,
                                             tmK, tmV, static_cast<const uint16_t*>(q), p, part, part_ml, static_cast<uint16_t*>(out), status);
     if (r || p.cluster || p.splits == 1) return r;
     return launch_dependent(merge, dim3(batch * hq), dim3(128), 0, stream, p, static_cast<const float*>(part),
                             static_cast<const float2*>(part_ml), static_cast<uint16_t*>(out));
   };
-  return dtype == XATTN_B200_BF16 ? launch(decode_attn_kernel<true>, decode_merge_kernel<true>)
-                                  : launch(decode_attn_kernel<false>, decode_merge_kernel<false>);
+  const bool bf16 = dtype == XATTN_B200_BF16;
+  if (wide)
+    return bf16 ? launch(decode_attn_kernel<true, true>, decode_merge_kernel<true>) : launch(decode_attn_kernel<false, true>, decode_merge_kernel<false>);
+  return bf16 ? launch(decode_attn_kernel<true, false>, decode_merge_kernel<true>) : launch(decode_attn_kernel<false, false>, decode_merge_kernel<false>);
 }
 
 }  // namespace xb
