@@ -1110,7 +1110,9 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // (32 heads, 32768 tokens: at stride 16 20.5 us with a CTA per query block, 12.7 like this; at stride 8 21.8 and 14.8.)
 // kVec > 0: the query block's warp (of four: the first) then selects on its row of sums, of up to 128 * kVec, see select_row: as a
 // kernel of its own that was a launch and a hand-over between two kernels more (stride 8: 2500 tokens 47.0 -> 44.2 us a call, 3000
-// 51.4 -> 48.6, 1024 against 70000 103 -> 93; video diffusion 15100 -> 15000; at the power cap, from 8000 tokens on, nothing).
+// 51.4 -> 48.6, 1024 against 70000 103 -> 93; at the power cap, from 8000 tokens on, nothing).  Rows of more than 512 sums go to the
+// selection kernel: with the registers that those take here the sums, which stream, are the slower for it (estimate and mask of 84758
+// tokens 3121 us apart, 3173 together).
 constexpr int kSumThreads = 128;
 template <int RBS, int kTeam, int kVec>
 __global__ void __launch_bounds__(kSumThreads)
@@ -1518,13 +1520,13 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   g.direct = direct ? 1 : 0;
   // Block sums finished there can be selected on there, too: rows of up to 128 stored sums (four per lane).  Clusters of two do
   // not gain: a CTA has the rows of eight query blocks at stride 16, two rounds for its six warps (2100 tokens 35.4 us a call
-  // with it, 35.2 without).  Otherwise est_blocksum_kernel selects, rows of up to 1024.
+  // with it, 35.2 without).  Otherwise est_blocksum_kernel selects, rows of up to 512.
   EstSelect sel;
   sel.on = 0;
   if (select) {
     const SelCall& c = *select;
     const int cols = g.band ? g.bpc : g.kb_total;
-    const bool here = direct ? (use_pairs || selects(g.tile_n / 128, f32)) && g.split != 2 && cols <= 128 : true;
+    const bool here = direct ? (use_pairs || selects(g.tile_n / 128, f32)) && g.split != 2 && cols <= 128 : cols <= 512;
     if (here && c.k_blocks <= 1024 && c.attn_sums == attn_sums && c.batch == batch && c.heads == hq && c.q_blocks == g.qb_total &&
         c.k_blocks == g.kb_total && c.bpc == g.bpc && (c.band ? 1 : 0) == g.band) {
       if ((rc = select_params(c, sel.p))) return rc;
@@ -1696,8 +1698,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     if (!sel.on) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 0>);
     if (cols <= 128) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 1>);
     if (cols <= 256) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 2>);
-    if (cols <= 512) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 4>);
-    return launch_sums(est_blocksum_kernel<kRbs, kTeam, 8>);
+    return launch_sums(est_blocksum_kernel<kRbs, kTeam, 4>);
   };
   auto launch_team = [&](auto rbs) -> int {
     return wide ? launch_vec(rbs, std::integral_constant<int, 128>()) : launch_vec(rbs, std::integral_constant<int, 32>());
