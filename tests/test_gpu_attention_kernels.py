@@ -195,8 +195,8 @@ def test_two_units_at_a_time(hq, hkv):
 # rings and not; ragged last stages, CTAs of unequal numbers of stages; 1 to 16 rows per kv head; strided caches
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,hq,hkv,n", [
-    (1, 32, 8, 4096), (1, 32, 8, 4097), (1, 32, 8, 4160), (1, 32, 8, 49152), (1, 32, 8, 49153), (1, 28, 4, 5000), (1, 28, 4, 102400),
-    (1, 28, 4, 102401), (1, 16, 1, 4111), (7, 1, 1, 6000), (2, 14, 7, 4500), (3, 5, 5, 4500), (2, 32, 8, 4500), (1, 12, 2, 20001), (3, 28, 4, 2500)])
+    (1, 32, 8, 4096), (1, 32, 8, 4097), (1, 32, 8, 4160), (1, 32, 8, 36864), (1, 32, 8, 36865), (1, 28, 4, 5000), (1, 28, 4, 65536),
+    (1, 28, 4, 65537), (1, 16, 1, 4111), (7, 1, 1, 6000), (2, 14, 7, 4500), (3, 5, 5, 4500), (2, 32, 8, 4500), (1, 12, 2, 20001), (3, 28, 4, 2500)])
 def test_decode_splits(B, hq, hkv, n, dtype):
     from xattn_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(n + hq)

@@ -60,11 +60,18 @@ __device__ __forceinline__ void warp_mma(float (&c)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+template <bool kBf16>
+__device__ __forceinline__ float2 unpack16t(uint32_t v) {
+  if constexpr (kBf16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
+  else return __half22float2(*reinterpret_cast<const __half2*>(&v));
+}
+
 // part: [batch * hkv][splits][group][128] un-normalised outputs, then [..][splits][group] (max, sum) pairs
 // kWide: the kernel for clusters of sixteen, and for smaller ones that have an SM per CTA.  Its ring may be deeper, and it has a warp
 // of its own that refills a slot as soon as the four warps are done with it; one of them does it a stage later, which leaves a CTA
-// a stage less in flight (30000 keys, 4 kv heads: 17.8 us a call against 26.3).  The others, two CTAs per SM, have enough in flight,
-// and with that warp their merge kernel came 5 us later.
+// a stage less in flight (30000 keys, 4 kv heads: 17.8 us a call against 26.3, before the second term below).  The others, two CTAs per SM, have enough in flight,
+// and with that warp their merge kernel came 5 us later.  Each part of the cache has a maximum of its own, whose exponential is exact,
+// so that fewer parts round a little more: here the probabilities are multiplied in two terms, which hides under the loads.
 template <bool kBf16, bool kWide>
 __global__ void __launch_bounds__(dec_threads(kWide), 2)
 decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -188,7 +195,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         }
       }
     }
-    uint32_t pa[4];
+    uint32_t pa[4], pl[4];                                 // (kWide) pl: what the rounding of pa leaves
 #pragma unroll
     for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -197,6 +204,10 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         const float p0 = fast_exp2(fmaf(s[t][2 * h], p.scale_log2, -mr)), p1 = fast_exp2(fmaf(s[t][2 * h + 1], p.scale_log2, -mr));
         l[h] += p0 + p1;
         pa[2 * t + h] = pack16t<kBf16>(p0, p1);
+        if constexpr (kWide) {
+          const float2 r = unpack16t<kBf16>(pa[2 * t + h]);
+          pl[2 * t + h] = pack16t<kBf16>(p0 - r.x, p1 - r.y);
+        }
       }
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -204,6 +215,10 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       ldsm_x4_trans(vt + (c >> 2) * (kDecTile / 2) + vrow * 128 + (((((c & 3) << 1) | vchunk) ^ (vrow & 7)) << 4), vb);
       warp_mma<kBf16>(o[2 * c], pa, vb[0], vb[1]);
       warp_mma<kBf16>(o[2 * c + 1], pa, vb[2], vb[3]);
+      if constexpr (kWide) {
+        warp_mma<kBf16>(o[2 * c], pl, vb[0], vb[1]);
+        warp_mma<kBf16>(o[2 * c + 1], pl, vb[2], vb[3]);
+      }
     }
     if (i + ring < n) fence_proxy_async_smem();      // every lane's reads of the stage come before the TMA writes that refill it
     __syncwarp();
@@ -369,12 +384,12 @@ decode_merge_kernel(const DecodeParams p, const float* __restrict__ part, const 
 // so are those of caches of up to 4096 keys, where eight CTAs of eight stages take about as long as the second kernel.
 // Longer caches: clusters of sixteen, where all of them fit on the chip at the same time (14 on this one with two CTAs per SM, half as
 // many with one), rather than more CTAs and a second kernel, which starts when the first has ended and reads what it wrote.  us a
-// call, 1 sequence, 32 / 8 heads: 4200 keys 13.6 -> 8.1, 9000 16.2 -> 11.5, 30000 28.7 -> 25.8; 28 / 4 heads: 4200 11.7 -> 7.4, 30000
-// 27.6 -> 18.0, 60000 36.9 -> 30.2; 8 / 1 heads, 30000 keys: 45 -> 17.  Up to 128 of 148 SMs stream then, and with rings of three
-// 43 GB/s each (5.5 TB/s), so that from about 50 stages per CTA on the second kernel is the lesser cost (60000 keys: 47.3 and
-// 46.3); with deep rings 73 GB/s each, and the line lies at about 100 (100000 keys, 4 heads: 46.4 and 47.5, 2 heads: 45.6 and 45.0).
+// call, 1 sequence, 32 / 8 heads: 4200 keys 13.6 -> 8.8, 12717 19.0 -> 15.1, 30000 29.4 -> 27.7; 28 / 4 heads: 4200 12.0 -> 7.1, 30000
+// 27.8 -> 20.2, 60000 37.0 -> 34.7; 8 / 1 heads, 30000 keys: 45 -> 19.  Up to 128 of 148 SMs stream then, and the time per key is a
+// third longer than with all of them (rings of three) or grows with the CTA's own share (deep rings, fewer heads): from about 40 and
+// 66 stages per CTA on the second kernel is the lesser cost.
 constexpr int kDecClusterMax = 8, kDecClusterStages = 64, kDecClusterWide = 16;
-constexpr int kDecWideStages = 48, kDecWideStagesDeep = 100;      // stages per CTA up to which sixteen are the faster way (rings of 3, of 6)
+constexpr int kDecWideStages = 36, kDecWideStagesDeep = 64;      // stages per CTA up to which sixteen are the faster way (rings of 3, of 6)
 static int wide_clusters();                              // clusters of sixteen that can be on the device at a time
 static int decode_splits(int batch, int hkv, int k_len, int& cluster) {
   const int stages = (k_len + kDecKeys - 1) / kDecKeys;
