@@ -271,10 +271,14 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         const List l = ln;
         int i = 0, w = wn, g_;
         const int kvh = __shfl_sync(0xffffffffu, fast_div(tn.h, p.by_group, g_), 0), b = __shfl_sync(0xffffffffu, tn.b, 0);
-        const bool more = kTwo && k > 0 && !second && unit + 1 < rest_units, request = k > 0 && !more && !(kList && rest_list);
-        const int tile0 = (b * p.hkv + kvh) * p.list_k_blocks;
-        const bool reuse = kTwo && __all_sync(0xffffffffu, l.n <= kReuseBlocks);
-        if (request && lane == 0) {
+        bool more = false, reuse = false;
+        int tile0 = 0;
+        if constexpr (kTwo) {
+          more = k > 0 && !second && unit + 1 < rest_units;
+          reuse = __all_sync(0xffffffffu, l.n <= kReuseBlocks);
+          tile0 = (b * p.hkv + kvh) * p.list_k_blocks;
+        }
+        if (k > 0 && !more && lane == 0 && !(kList && rest_list)) {
           mbar_expect_tx(answer_full, 16);
           clc_try_cancel(smem_u32(answer), answer_full);
         }
@@ -333,15 +337,17 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
             if (kList && rest_list) {
               if (k > 0) unit += gridDim.x;
               if (unit >= rest_units) unit = -1;
-            } else if (more) {
+            } else if (kTwo && more) {
               ++unit;
               second = true;
-            } else if (request) {
-              if (!wait(answer_full, requests & 1)) { ok = false; break; }
-              ++requests;
+            } else if (k > 0) {
+              if (!wait(answer_full, (kTwo ? requests : k - 1) & 1)) { ok = false; break; }
               unit = clc_answer(smem_u32(answer));
-              if (kTwo && unit > 0) unit *= 2;
-              second = false;
+              if constexpr (kTwo) {
+                if (unit > 0) unit *= 2;
+                second = false;
+                ++requests;
+              }
               fence_proxy_async_smem();                 // read before the next answer is written
             }
             ln.n = -1;
@@ -351,7 +357,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
               wn = list_entry(ln, wl);
             }
             // (no unit is left for this SM: the set-up of the kernel after this one may run under the tail)
-            if (unit < 0 && p.early_next) pdl_launch_dependents();
+            if (!kList && !kTwo && unit < 0 && p.early_next) pdl_launch_dependents();
             if (!wait(unit_empty + 8 * (k % kUnitSlots), (k / kUnitSlots & 1) ^ 1)) { ok = false; break; }
             if (wl == 0) reinterpret_cast<int4*>(unit_ring)[2 * (k % kUnitSlots) + s] = make_int4(tn.b, tn.h, tn.qb, ln.n);
             __syncwarp();

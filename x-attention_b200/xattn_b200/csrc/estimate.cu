@@ -55,8 +55,9 @@ struct EstRounded {
 // The selection on rows that the epilogue has finished (EstGeom::direct): a chain of a microsecond per row, which runs under the
 // next tiles' products, or, where a cluster of four has a single tile, on a warp per row.  As a kernel of its own it was a launch and a
 // hand-over between two kernels more (1003 tokens: the prefill 26.2 -> 24.2 us; 128K tokens 773 -> 765 in short runs).
-// Single CTAs with 128-column tiles of 16-bit operands, and CTA pairs, do it: the other kernels' epilogues have no registers left
-// for it (spills: 4096 tokens against 65536 51.9 -> 52.5 us a call although nothing was selected there).
+// Only the kernel of single CTAs with 128-column tiles of 16-bit operands does it: in the others the epilogue has no registers left for
+// it (spills: 4096 tokens against 65536 51.9 -> 52.5 us a call although nothing was selected there), or, CTA pairs with their few
+// steps per tile, no time (114688 tokens at stride 8 939 -> 967, 3590 tokens of a 16384-token chunk 34.5 -> 38.1).
 __host__ __device__ constexpr bool selects(int direct, bool f32) { return direct == 1 && !f32; }
 struct EstSelect {
   int on;
@@ -870,8 +871,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKh,
                      const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt,
                      const EstGeom g, const int* group_lo, const int* group_prefix,
-                     float* __restrict__ partial, float2* __restrict__ mtile, float* sums, const uint32_t idesc_wide, const uint32_t idesc_narrow,
-                     const EstSelect sel, int* status) {
+                     float* __restrict__ partial, float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc_wide, const uint32_t idesc_narrow,
+                     int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_tab[kTabInts];
   if (g.tab_n) {                                  // (made visible by the __syncthreads() that ends the prologue)
@@ -1067,7 +1068,6 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         est_epilogue_row_direct<RBS, kDirect>(g, load, nvis, clo, chi,
                                         sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, col0, out_cols,
                                         qb < g.qb_total, lane);
-        if (sel.on) est_select_rows<RBS>(g, sel, sums, bh, (mt * kTileM + quad * 32) / RBS, 32 / RBS, 0, 1, lane);
       } else {
         // (compact scratch: both row tiles of a pair lie in one chunk and start at the pair's first column tile)
         const bool write = mt < g.n_mtiles;
@@ -1085,12 +1085,6 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000) { __nanosleep(1000); }
     if (threadIdx.x == 0 && status) atomicExch(status, static_cast<int>(kDevWaitTimeout));
-    if (kDirect > 0 && sel.on)
-      for (int tile = pair; tile < total_tiles; tile += n_pairs_grid) {
-        int bh, mt, nt;
-        decode(tile, bh, mt, nt);
-        if (mt < g.n_mtiles) est_forget_rows<RBS>(g, sel, bh, mt);
-      }
   }
   // neither CTA may release tensor memory, or leave while the other can still signal its barriers
   cluster_sync_all();
@@ -1489,15 +1483,17 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   g.pair_heads = g.tile_n == kTileN && (hq / hkv) % 2 == 0 ? 1 : 0;
   if (g.pair_heads) use_pairs = true;
   if (f32) use_pairs = false;
+  bool many = false;                                       // more than four tiles per SM
   // Few tiles (short prompts: 32 heads of up to 2048 tokens at stride 16 are 32 tiles for 148 SMs): the K loop of each, which is
   // a stream of operands through one SM, is split over a cluster of two or four CTAs instead.
   {
     long long tiles = 0;
-    for (int mt = 0; mt < g.n_mtiles && tiles <= sm_count(); ++mt) {
+    for (int mt = 0; mt < g.n_mtiles && tiles <= 4LL * sm_count(); ++mt) {
       int first, count;
       row_tile_range(g, mt, first, count);
       tiles += static_cast<long long>(count > 0 ? count : 1) * batch * hq;
     }
+    many = tiles > 4LL * sm_count();
     const bool long_k = g.S * g.d_chunks >= 32 && !terms;          // (the exchange costs about what eight steps take)
     g.split = !long_k ? 1 : (4 * tiles <= sm_count() ? 4 : (2 * tiles <= sm_count() ? 2 : 1));
     if (g.split > 1) use_pairs = false;
@@ -1518,15 +1514,16 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     direct = g.band ? count == 1 && first * g.tile_n == (mt * kTileM / g.rcs) * g.rcs + g.row_off : count <= 1;
   }
   g.direct = direct ? 1 : 0;
-  // Block sums finished there can be selected on there, too: rows of up to 128 stored sums (four per lane).  Clusters of two do
-  // not gain: a CTA has the rows of eight query blocks at stride 16, two rounds for its six warps (2100 tokens 35.4 us a call
-  // with it, 35.2 without).  Otherwise est_blocksum_kernel selects, rows of up to 512.
+  // Block sums finished there can be selected on there, too: rows of up to 128 stored sums (four per lane), in clusters of four, or
+  // where a CTA has tiles enough that the selection on one runs under the next.  Clusters of two do not gain: a CTA has the rows of
+  // eight query blocks at stride 16, two rounds for its six warps (2100 tokens 35.4 us a call with it, 35.2 without).  Otherwise
+  // est_blocksum_kernel selects, rows of up to 512.
   EstSelect sel;
   sel.on = 0;
   if (select) {
     const SelCall& c = *select;
     const int cols = g.band ? g.bpc : g.kb_total;
-    const bool here = direct ? (use_pairs || selects(g.tile_n / 128, f32)) && g.split != 2 && cols <= 128 : cols <= 512;
+    const bool here = direct ? !use_pairs && selects(g.tile_n / 128, f32) && (g.split == 4 || (g.split == 1 && many)) && cols <= 128 : cols <= 512;
     if (here && c.k_blocks <= 1024 && c.attn_sums == attn_sums && c.batch == batch && c.heads == hq && c.q_blocks == g.qb_total &&
         c.k_blocks == g.kb_total && c.bpc == g.bpc && (c.band ? 1 : 0) == g.band) {
       if ((rc = select_params(c, sel.p))) return rc;
@@ -1613,7 +1610,7 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       if (static_cast<unsigned>(2 * max_clusters) < cfg.gridDim.x) cfg.gridDim.x = 2 * max_clusters;
       return launch_dependent_clusters(kern, 2, cfg.gridDim, cfg.blockDim, kPairSmem, stream, tmQ, tmK, tmQt, tmKt, g,
                                        (const int*)(g.pair_heads ? tile_lo : pair_lo), (const int*)(g.pair_heads ? tile_prefix : pair_prefix),
-                                       partial, mtile, attn_sums, idesc2, idesc2n, sel, status);
+                                       partial, mtile, attn_sums, idesc2, idesc2n, status);
     };
     auto launch_pair_rbs = [&](auto rbs) -> int {
       constexpr int kRbs = decltype(rbs)::value;
