@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kF32 ? f32_threads(kDirect) : kGemmThreads, 1)
 est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt, const EstGeom g,
                 const int* tile_lo, const int* tile_prefix, float* __restrict__ partial,
-                float2* __restrict__ mtile, float* sums, const uint32_t idesc, const EstRounded rounded, const EstSelect sel, int* status) {
+                float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc, const EstRounded rounded, const EstSelect sel, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_tab[kTabInts];
   if (g.tab_n) {                                  // (made visible by the __syncthreads() that ends the prologue)
@@ -917,7 +917,11 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before();
   cluster_sync_all();               // barriers of both CTAs are initialised before any remote arrival or copy
   tc_fence_after();
-  pdl_launch_dependents();
+  // In long calls the next kernel comes as the last tiles finish, not before: CTAs of it that sat beside this one for milliseconds then
+  // ran with this kernel's division of the SM's memory between cache and shared memory (video diffusion: block sums 575 us, 510 like
+  // this; short calls want it early: 1024 tokens against 70000 97.5 us a call like this, 93.5 early).
+  const bool late = g.tab_n == 0;                           // more than 64 row tiles
+  if (!late) pdl_launch_dependents();
   pdl_wait();                       // up to here nothing was touched that an earlier kernel writes
   const uint32_t tmem_base = *tmem_slot;
 
@@ -972,6 +976,7 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
       }
     }
+    if (late) pdl_launch_dependents();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (even CTA; converged warp, one thread issues)
     if (rank == 0) {
@@ -1111,7 +1116,7 @@ constexpr int kSumThreads = 128;
 template <int RBS, int kTeam, int kVec>
 __global__ void __launch_bounds__(kSumThreads)
 est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix, const float* __restrict__ partial,
-                    const float2* __restrict__ mtile, float* sums, int seg_tiles, const EstSelect sel) {
+                    const float2* __restrict__ mtile, float* __restrict__ sums, int seg_tiles, const EstSelect sel) {
   extern __shared__ float s_factors[];                     // [team][tile][row] factors, seg_tiles tiles at a time
   __shared__ float2 s_part[4][RBS];                        // (teams of four warps) [warp][row] (max, sum)
   constexpr int kParts = kTeam / RBS, kTeams = kSumThreads / kTeam;
