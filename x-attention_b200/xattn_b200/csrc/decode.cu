@@ -69,10 +69,13 @@ __device__ __forceinline__ float2 unpack16t(uint32_t v) {
 // part: [batch * hkv][splits][group][128] un-normalised outputs, then [..][splits][group] (max, sum) pairs
 // kWide: the kernel for clusters of sixteen, and for smaller ones that have an SM per CTA.  Its ring may be deeper, and it has a warp
 // of its own that refills a slot as soon as the four warps are done with it; one of them does it a stage later, which leaves a CTA
-// a stage less in flight (30000 keys, 4 kv heads: 17.8 us a call against 26.3, before the second term below).  The others, two CTAs per SM, have enough in flight,
-// and with that warp their merge kernel came 5 us later.  Each part of the cache has a maximum of its own, whose exponential is exact,
-// so that fewer parts round a little more: here the probabilities are multiplied in two terms, which hides under the loads.
-template <bool kBf16, bool kWide>
+// a stage less in flight (30000 keys, 4 kv heads: 17.8 us a call against 26.3, before the second term below).  The others, two CTAs
+// per SM, have enough in flight, and with that warp their merge kernel came 5 us later.
+// kSixteen: clusters of sixteen, up to eight otherwise.  Each part of the cache has a maximum of its own, whose exponential is exact, so
+// that these parts, fewer than those of two CTAs per SM, would round a little more: they multiply the probabilities in two 16-bit
+// terms.  Clusters of up to eight have the same parts in either kernel, and one term in both: a sequence's result does not depend on
+// the batch that it is in.
+template <bool kBf16, bool kWide, bool kSixteen>
 __global__ void __launch_bounds__(dec_threads(kWide), 2)
 decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const uint16_t* __restrict__ q, const DecodeParams p, float* __restrict__ part,
@@ -195,7 +198,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         }
       }
     }
-    uint32_t pa[4], pl[4];                                 // (kWide) pl: what the rounding of pa leaves
+    uint32_t pa[4], pl[4];                                 // (kSixteen) pl: what the rounding of pa leaves
 #pragma unroll
     for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -204,7 +207,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         const float p0 = fast_exp2(fmaf(s[t][2 * h], p.scale_log2, -mr)), p1 = fast_exp2(fmaf(s[t][2 * h + 1], p.scale_log2, -mr));
         l[h] += p0 + p1;
         pa[2 * t + h] = pack16t<kBf16>(p0, p1);
-        if constexpr (kWide) {
+        if constexpr (kSixteen) {
           const float2 r = unpack16t<kBf16>(pa[2 * t + h]);
           pl[2 * t + h] = pack16t<kBf16>(p0 - r.x, p1 - r.y);
         }
@@ -215,7 +218,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       ldsm_x4_trans(vt + (c >> 2) * (kDecTile / 2) + vrow * 128 + (((((c & 3) << 1) | vchunk) ^ (vrow & 7)) << 4), vb);
       warp_mma<kBf16>(o[2 * c], pa, vb[0], vb[1]);
       warp_mma<kBf16>(o[2 * c + 1], pa, vb[2], vb[3]);
-      if constexpr (kWide) {
+      if constexpr (kSixteen) {
         warp_mma<kBf16>(o[2 * c], pl, vb[0], vb[1]);
         warp_mma<kBf16>(o[2 * c + 1], pl, vb[2], vb[3]);
       }
@@ -325,7 +328,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
           ll += ml[s].y * f;
         }
       };
-      merge(std::integral_constant<int, kWide ? 16 : 8>());
+      merge(std::integral_constant<int, kSixteen ? 16 : 8>());
       const float inv = ll > 0.f ? 1.f / ll : 0.f;
       *reinterpret_cast<uint32_t*>(out + b * p.osb + static_cast<int64_t>(g * p.group + r) * p.osh + c) =
           pack16t<kBf16>(a0 * inv, a1 * inv);
@@ -427,7 +430,7 @@ static bool dec_allow(K kern, bool wide) {
 static int wide_clusters() {
   static const char key = 0;
   return once_per_device(&key, []() {
-    const auto kern = decode_attn_kernel<true, true>;
+    const auto kern = decode_attn_kernel<true, true, true>;
     if (!dec_allow(kern, true)) return 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kDecClusterWide, 64, 1);
@@ -493,10 +496,13 @@ int decode_launch(const void* q, const void* k, const void* v, int dtype, int ba
     return launch_dependent(merge, dim3(batch * hq), dim3(128), 0, stream, p, static_cast<const float*>(part),
                             static_cast<const float2*>(part_ml), static_cast<uint16_t*>(out));
   };
-  const bool bf16 = dtype == XATTN_B200_BF16;
-  if (wide)
-    return bf16 ? launch(decode_attn_kernel<true, true>, decode_merge_kernel<true>) : launch(decode_attn_kernel<false, true>, decode_merge_kernel<false>);
-  return bf16 ? launch(decode_attn_kernel<true, false>, decode_merge_kernel<true>) : launch(decode_attn_kernel<false, false>, decode_merge_kernel<false>);
+  auto launch_type = [&](auto bf16) -> int {
+    constexpr bool kBf16 = decltype(bf16)::value;
+    if (!wide) return launch(decode_attn_kernel<kBf16, false, false>, decode_merge_kernel<kBf16>);
+    return p.splits > kDecClusterMax ? launch(decode_attn_kernel<kBf16, true, true>, decode_merge_kernel<kBf16>)
+                                     : launch(decode_attn_kernel<kBf16, true, false>, decode_merge_kernel<kBf16>);
+  };
+  return dtype == XATTN_B200_BF16 ? launch_type(std::true_type()) : launch_type(std::false_type());
 }
 
 }  // namespace xb
