@@ -30,3 +30,31 @@ def test_a_sequence_alone_and_in_a_batch(hq, hkv, n, dtype):
     together = ops.decode_attention(q, k, v)
     for b in (0, batch - 1):
         assert torch.equal(ops.decode_attention(q[b:b + 1], k[b:b + 1], v[b:b + 1])[0], together[b])
+
+
+# every way to split a cache: one CTA, clusters of four, eight and sixteen, more CTAs and a second kernel
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch,hq,hkv,n", [(1, 8, 2, 100), (1, 32, 8, 500), (1, 32, 8, 2011), (4, 32, 8, 2011), (1, 32, 8, 5000), (1, 28, 4, 5000),
+                                            (1, 8, 8, 4097), (3, 28, 4, 9000), (4, 32, 8, 9000), (1, 32, 8, 40000)])
+def test_infinite_values(batch, hq, hkv, n, dtype):
+    """A value that is infinite makes its column of the head infinite, whatever its key's probability rounds to; the other columns
+    are what they are without it.  A NaN stays one."""
+    from xattn_b200 import ops
+    q, k, v = _step(n + hq, batch, hq, hkv, n, dtype)
+    q = q * 0.1                                       # (no probability vanishes)
+    want = ops.decode_attention(q, k, v)
+    bad = v.clone()
+    keys = torch.linspace(0, n - 1, 12, device=DEV).long().tolist()
+    for i, key in enumerate(keys):
+        bad[:, :, key, i] = float("inf")
+        bad[:, :, key, 32 + i] = float("-inf")
+    bad[:, :, keys[3], 64] = float("nan")
+    got = ops.decode_attention(q, k, bad)
+    assert (got[..., :12] == float("inf")).all()
+    assert (got[..., 32:44] == float("-inf")).all()
+    assert got[..., 64].isnan().all()
+    rest = [c for c in range(128) if c not in (*range(12), *range(32, 44), 64)]
+    # (the probabilities of such a call may be multiplied in one 16-bit term instead of two: at most half a unit in the last place
+    # of the values' type per probability and per result, on averages of values of at most 6)
+    tol = 6 * 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert (got[..., rest].float() - want[..., rest].float()).abs().max() <= tol

@@ -112,141 +112,166 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   constexpr int kDecThreads = dec_threads(kWide);
   if (!kWide && threadIdx.x == 0)
     for (int i = 0; i < ring && i < n; ++i) load_stage(i, i);
-  if (kWide && warp == kDecWarps) {
-    if (lane == 0) {
-      int st = 0;
-      uint32_t ph = 1;
+  float o[16][4];
+  float m[2], l[2];                                        // rows lane / 4 and lane / 4 + 8
+  int st = 0, last = ring - 1;                             // this stage's slot (of the loading warp: to load), the slot of the one before
+  uint32_t ph = kWide && warp == kDecWarps ? 1 : 0, last_ph = 1;       // and the phases of their barriers
+  int loads = 0;
+  auto pass = [&](auto two_terms) {                        // the CTA's part of the cache, with the probabilities in one or two terms
+    constexpr bool kTwo = decltype(two_terms)::value;
+    if (kWide && warp == kDecWarps) {
+      if (lane == 0) {
+        for (int i = 0; i < n; ++i, ++loads) {
+          if (loads >= ring && !mbar_wait(empty0 + 8 * st, ph, abort_flag)) break;
+          load_stage(i, st);
+          if (++st == ring) { st = 0; ph ^= 1; }
+        }
+      }
+      __syncwarp();
+    }
+    if (warp < kDecWarps) {
+      // Q as A operand: rows = query heads of the group (rows past it zero), 8 steps of 16 columns
+      uint32_t qa[8][4];
+      {
+        const int r0 = lane >> 2, c0 = (lane & 3) * 2;
+        const uint16_t* qg = q + b * p.qsb + static_cast<int64_t>(g) * p.group * p.qsh;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = r0 + 8 * h;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) qa[k][h] = qa[k][2 + h] = 0u;
+          if (r < p.group) {
+            const uint16_t* row = qg + r * p.qsh + c0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) qa[k][2 * e + h] = ld_written(reinterpret_cast<const uint32_t*>(row + 16 * k + 8 * e));
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 16; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[t][e] = 0.f;
+      m[0] = m[1] = -INFINITY;
+      l[0] = l[1] = 0.f;
+      // ldmatrix addresses: lane's row inside the warp's 16 keys; chunk c of 16 bytes of row r sits at chunk c ^ (r & 7)
+      const int krow = warp * 16 + (lane & 7) + ((lane >> 4) << 3), kchunk = (lane >> 3) & 1;   // K: keys 0-7 | 8-15, columns 0-7 | 8-15
+      const int vrow = warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), vchunk = lane >> 4;   // V: the same, transposed on load
+      bool ok = true;
       for (int i = 0; i < n; ++i) {
-        if (i >= ring && !mbar_wait(empty0 + 8 * st, ph, abort_flag)) break;
-        load_stage(i, st);
+        if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * st, ph, abort_flag))) break;
+        const uint32_t kt = smem_u32(smem) + st * 2 * kDecTile, vt = kt + kDecTile;
+        float s[2][4] = {};                                    // keys 0-7, 8-15 of the warp
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          uint32_t kb[4];
+          ldsm_x4(kt + (k >> 2) * (kDecTile / 2) + krow * 128 + (((((k & 3) << 1) | kchunk) ^ (krow & 7)) << 4), kb);
+          warp_mma<kBf16>(s[0], qa[k], kb[0], kb[1]);
+          warp_mma<kBf16>(s[1], qa[k], kb[2], kb[3]);
+        }
+        const int key0 = (s0 + i) * kDecKeys + warp * 16 + (lane & 3) * 2;
+        if ((s0 + i + 1) * kDecKeys > p.k_len) {
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (key0 + 8 * t + (e & 1) >= p.k_len) s[t][e] = -INFINITY;
+        }
+        float mx[2];
+        bool grow = false;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          mx[h] = fmaxf(fmaxf(s[0][2 * h], s[0][2 * h + 1]), fmaxf(s[1][2 * h], s[1][2 * h + 1]));
+          mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+          mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2)) * p.scale_log2;
+          grow |= mx[h] > m[h] + kDecRescale;                  // (-inf + 8 is -inf: the first finite maximum counts)
+        }
+        if (__any_sync(0xffffffffu, grow)) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float mn = fmaxf(m[h], mx[h]);
+            const float alpha = m[h] == -INFINITY ? 0.f : fast_exp2(m[h] - mn);
+            m[h] = mn;
+            l[h] *= alpha;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+              o[t][2 * h] *= alpha;
+              o[t][2 * h + 1] *= alpha;
+            }
+          }
+        }
+        uint32_t pa[4], pl[4];                                 // (kTwo) pl: what the rounding of pa leaves
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float mr = m[h] == -INFINITY ? 0.f : m[h];
+            const float p0 = fast_exp2(fmaf(s[t][2 * h], p.scale_log2, -mr)), p1 = fast_exp2(fmaf(s[t][2 * h + 1], p.scale_log2, -mr));
+            l[h] += p0 + p1;
+            pa[2 * t + h] = pack16t<kBf16>(p0, p1);
+            if constexpr (kTwo) {
+              const float2 r = unpack16t<kBf16>(pa[2 * t + h]);
+              pl[2 * t + h] = pack16t<kBf16>(p0 - r.x, p1 - r.y);
+            }
+          }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          uint32_t vb[4];
+          ldsm_x4_trans(vt + (c >> 2) * (kDecTile / 2) + vrow * 128 + (((((c & 3) << 1) | vchunk) ^ (vrow & 7)) << 4), vb);
+          warp_mma<kBf16>(o[2 * c], pa, vb[0], vb[1]);
+          warp_mma<kBf16>(o[2 * c + 1], pa, vb[2], vb[3]);
+          if constexpr (kTwo) {
+            warp_mma<kBf16>(o[2 * c], pl, vb[0], vb[1]);
+            warp_mma<kBf16>(o[2 * c + 1], pl, vb[2], vb[3]);
+          }
+        }
+        if (i + ring < n) fence_proxy_async_smem();      // every lane's reads of the stage come before the TMA writes that refill it
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty0 + 8 * st);
+        if constexpr (!kWide) {
+          if (threadIdx.x == 0 && i > 0 && i - 1 + ring < n) {
+            // the stage before this one is refilled: by now every warp is done with it, or nearly
+            if (mbar_wait(empty0 + 8 * last, last_ph, abort_flag)) load_stage(i - 1 + ring, last);
+            else ok = false;
+          }
+          ok = __shfl_sync(0xffffffffu, ok, 0);
+          if (!ok) break;
+          last = st;
+          last_ph = ph;
+        }
         if (++st == ring) { st = 0; ph ^= 1; }
       }
-    }
-    __syncwarp();
-  }
-  float o[16][4];
-  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // rows lane / 4 and lane / 4 + 8
-  if (warp < kDecWarps) {
-  // Q as A operand: rows = query heads of the group (rows past it zero), 8 steps of 16 columns
-  uint32_t qa[8][4];
-  {
-    const int r0 = lane >> 2, c0 = (lane & 3) * 2;
-    const uint16_t* qg = q + b * p.qsb + static_cast<int64_t>(g) * p.group * p.qsh;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = r0 + 8 * h;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) qa[k][h] = qa[k][2 + h] = 0u;
-      if (r < p.group) {
-        const uint16_t* row = qg + r * p.qsh + c0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) qa[k][2 * e + h] = ld_written(reinterpret_cast<const uint32_t*>(row + 16 * k + 8 * e));
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < 16; ++t)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[t][e] = 0.f;
-  // ldmatrix addresses: lane's row inside the warp's 16 keys; chunk c of 16 bytes of row r sits at chunk c ^ (r & 7)
-  const int krow = warp * 16 + (lane & 7) + ((lane >> 4) << 3), kchunk = (lane >> 3) & 1;   // K: keys 0-7 | 8-15, columns 0-7 | 8-15
-  const int vrow = warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), vchunk = lane >> 4;   // V: the same, transposed on load
-  bool ok = true;
-  int st = 0, last = ring - 1;                           // this stage's slot, the slot of the one before
-  uint32_t ph = 0, last_ph = 1;                            // and the phases of their barriers
-  for (int i = 0; i < n; ++i) {
-    if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * st, ph, abort_flag))) break;
-    const uint32_t kt = smem_u32(smem) + st * 2 * kDecTile, vt = kt + kDecTile;
-    float s[2][4] = {};                                    // keys 0-7, 8-15 of the warp
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      uint32_t kb[4];
-      ldsm_x4(kt + (k >> 2) * (kDecTile / 2) + krow * 128 + (((((k & 3) << 1) | kchunk) ^ (krow & 7)) << 4), kb);
-      warp_mma<kBf16>(s[0], qa[k], kb[0], kb[1]);
-      warp_mma<kBf16>(s[1], qa[k], kb[2], kb[3]);
-    }
-    const int key0 = (s0 + i) * kDecKeys + warp * 16 + (lane & 3) * 2;
-    if ((s0 + i + 1) * kDecKeys > p.k_len) {
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (key0 + 8 * t + (e & 1) >= p.k_len) s[t][e] = -INFINITY;
-    }
-    float mx[2];
-    bool grow = false;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      mx[h] = fmaxf(fmaxf(s[0][2 * h], s[0][2 * h + 1]), fmaxf(s[1][2 * h], s[1][2 * h + 1]));
-      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2)) * p.scale_log2;
-      grow |= mx[h] > m[h] + kDecRescale;                  // (-inf + 8 is -inf: the first finite maximum counts)
-    }
-    if (__any_sync(0xffffffffu, grow)) {
+      // row sums over the four lanes of a row
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const float mn = fmaxf(m[h], mx[h]);
-        const float alpha = m[h] == -INFINITY ? 0.f : fast_exp2(m[h] - mn);
-        m[h] = mn;
-        l[h] *= alpha;
-#pragma unroll
-        for (int t = 0; t < 16; ++t) {
-          o[t][2 * h] *= alpha;
-          o[t][2 * h + 1] *= alpha;
-        }
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
       }
     }
-    uint32_t pa[4], pl[4];                                 // (kSixteen) pl: what the rounding of pa leaves
+  };
+  pass(std::integral_constant<bool, kSixteen>());
+  // every stage has been read: the ring becomes the exchange buffer
+  if constexpr (kSixteen) {
+    // The products of an infinite value with the second terms, zero or of either sign, are NaN: where a result is not finite the cache is
+    // read again for the first terms alone.  (As a copy of the pass: a choice inside it made every call longer, 30000 keys, 4 kv heads,
+    // 20.2 -> 26.0 us around the products of a step, 23.4 around all of them.)
+    float check = 0.f;
+    if (warp < kDecWarps) {
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+      for (int t = 0; t < 16; ++t)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float mr = m[h] == -INFINITY ? 0.f : m[h];
-        const float p0 = fast_exp2(fmaf(s[t][2 * h], p.scale_log2, -mr)), p1 = fast_exp2(fmaf(s[t][2 * h + 1], p.scale_log2, -mr));
-        l[h] += p0 + p1;
-        pa[2 * t + h] = pack16t<kBf16>(p0, p1);
-        if constexpr (kSixteen) {
-          const float2 r = unpack16t<kBf16>(pa[2 * t + h]);
-          pl[2 * t + h] = pack16t<kBf16>(p0 - r.x, p1 - r.y);
-        }
-      }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      uint32_t vb[4];
-      ldsm_x4_trans(vt + (c >> 2) * (kDecTile / 2) + vrow * 128 + (((((c & 3) << 1) | vchunk) ^ (vrow & 7)) << 4), vb);
-      warp_mma<kBf16>(o[2 * c], pa, vb[0], vb[1]);
-      warp_mma<kBf16>(o[2 * c + 1], pa, vb[2], vb[3]);
-      if constexpr (kSixteen) {
-        warp_mma<kBf16>(o[2 * c], pl, vb[0], vb[1]);
-        warp_mma<kBf16>(o[2 * c + 1], pl, vb[2], vb[3]);
-      }
+        for (int e = 0; e < 4; ++e) check = fmaf(o[t][e], 0.f, check);
     }
-    if (i + ring < n) fence_proxy_async_smem();      // every lane's reads of the stage come before the TMA writes that refill it
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty0 + 8 * st);
-    if constexpr (!kWide) {
-      if (threadIdx.x == 0 && i > 0 && i - 1 + ring < n) {
-        // the stage before this one is refilled: by now every warp is done with it, or nearly
-        if (mbar_wait(empty0 + 8 * last, last_ph, abort_flag)) load_stage(i - 1 + ring, last);
-        else ok = false;
-      }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      last = st;
-      last_ph = ph;
+    if (__syncthreads_or(check != 0.f) && !*abort_flag) {
+      fence_proxy_async_smem();                            // (the reads of the last stages come before the TMA writes that follow)
+      __syncthreads();
+      pass(std::false_type());
+      __syncthreads();
     }
-    if (++st == ring) { st = 0; ph ^= 1; }
+  } else {
+    __syncthreads();
   }
-  // row sums over the four lanes of a row
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
-    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
-  }
-  }
-  __syncthreads();                       // every stage has been read: the ring becomes the exchange buffer
   const bool aborted = *abort_flag != 0;
   if (aborted) {
     const long long t0 = clock64();
