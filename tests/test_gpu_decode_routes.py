@@ -58,3 +58,23 @@ def test_infinite_values(batch, hq, hkv, n, dtype):
     # of the values' type per probability and per result, on averages of values of at most 6)
     tol = 6 * 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
     assert (got[..., rest].float() - want[..., rest].float()).abs().max() <= tol
+
+
+@pytest.mark.parametrize("n", [4097, 4500, 30000])
+def test_two_ctas_per_sm_make_sixteen_per_head(n):
+    """Heads for which two CTAs per SM come to sixteen each, but whose clusters of sixteen do not fit on the chip together: they take
+    the second kernel, with its scratch, as one head fewer and one more do."""
+    from xattn_b200 import _lib, ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    heads = 2 * sms // 16
+    assert 2 * sms // heads == 16
+    lib = _lib.load()
+    q, k, v = _step(n, heads, 4, 1, n, torch.bfloat16)
+    out = ops.decode_attention(q, k, v)
+    for b in (0, heads // 2, heads - 1):
+        s = q[b, :, 0].double() @ k[b, 0].double().T * 128 ** -0.5
+        want = s.softmax(-1) @ v[b, 0].double()
+        # probabilities and results rounded to 8 bits: each at most half a unit in the last place, both together less than one
+        assert (out[b, :, 0].double() - want).norm() / want.norm() < 2.0 ** -8
+    for h in (heads - 1, heads, heads + 1):
+        assert lib.xattn_b200_decode_workspace_bytes(h, 4, 1, n) > 0, h

@@ -425,10 +425,10 @@ static int decode_splits(int batch, int hkv, int k_len, int& cluster) {
   long long s = 2LL * sm_count() / heads;
   if (s > stages / 2) s = stages / 2;
   if (s > kDecClusterMax && (stages <= kDecClusterStages || s < kDecClusterMax * 3 / 2)) s = kDecClusterMax;
-  if (s > kDecClusterMax && s >= kDecClusterWide && heads <= wide_clusters() &&
-      stages <= kDecClusterWide * (2 * heads <= wide_clusters() ? kDecWideStagesDeep : kDecWideStages))
-    s = kDecClusterWide;
-  cluster = s > 1 && (s <= kDecClusterMax || s == kDecClusterWide) ? 1 : 0;
+  const bool sixteen = s >= kDecClusterWide && heads <= wide_clusters() &&
+                       stages <= kDecClusterWide * (2 * heads <= wide_clusters() ? kDecWideStagesDeep : kDecWideStages);
+  if (sixteen) s = kDecClusterWide;
+  cluster = s > 1 && (s <= kDecClusterMax || sixteen) ? 1 : 0;         // (sixteen splits that come out as such are not one)
   if (cluster)
     while (s & (s - 1)) s &= s - 1;
   return s < 1 ? 1 : static_cast<int>(s);
