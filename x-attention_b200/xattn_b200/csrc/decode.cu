@@ -410,23 +410,23 @@ decode_merge_kernel(const DecodeParams p, const float* __restrict__ part, const 
 // Number of splits: two CTAs per SM over all (batch, kv head) pairs, at least two stages each (a split costs a CTA's start
 // and its row of the merge, about what two stages take).  Up to eight of them are a cluster, whose size is a power of two;
 // so are those of caches of up to 4096 keys, where eight CTAs of eight stages take about as long as the second kernel.
-// Longer caches: clusters of sixteen, where all of them fit on the chip at the same time (14 on this one with two CTAs per SM, half as
-// many with one), rather than more CTAs and a second kernel, which starts when the first has ended and reads what it wrote.  us a
+// Longer caches: clusters of sixteen, where all of them fit on the chip at the same time (14 on this one with two CTAs per SM, seven
+// with one), rather than more CTAs and a second kernel, which starts when the first has ended and reads what it wrote.  us a
 // call, 1 sequence, 32 / 8 heads: 4200 keys 13.6 -> 8.8, 12717 19.0 -> 15.1, 30000 29.4 -> 27.7; 28 / 4 heads: 4200 12.0 -> 7.1, 30000
 // 27.8 -> 20.2, 60000 37.0 -> 34.7; 8 / 1 heads, 30000 keys: 45 -> 19.  Up to 128 of 148 SMs stream then, and the time per key is a
 // third longer than with all of them (rings of three) or grows with the CTA's own share (deep rings, fewer heads): from about 40 and
 // 66 stages per CTA on the second kernel is the lesser cost.
 constexpr int kDecClusterMax = 8, kDecClusterStages = 64, kDecClusterWide = 16;
 constexpr int kDecWideStages = 36, kDecWideStagesDeep = 64;      // stages per CTA up to which sixteen are the faster way (rings of 3, of 6)
-static int wide_clusters();                              // clusters of sixteen that can be on the device at a time
+static int wide_clusters(bool deep);                     // clusters of sixteen, with rings of three or six, that fit on the device at a time
 static int decode_splits(int batch, int hkv, int k_len, int& cluster) {
   const int stages = (k_len + kDecKeys - 1) / kDecKeys;
   const long long heads = static_cast<long long>(batch) * hkv;
   long long s = 2LL * sm_count() / heads;
   if (s > stages / 2) s = stages / 2;
   if (s > kDecClusterMax && (stages <= kDecClusterStages || s < kDecClusterMax * 3 / 2)) s = kDecClusterMax;
-  const bool sixteen = s >= kDecClusterWide && heads <= wide_clusters() &&
-                       stages <= kDecClusterWide * (2 * heads <= wide_clusters() ? kDecWideStagesDeep : kDecWideStages);
+  const bool sixteen = s >= kDecClusterWide && heads <= wide_clusters(false) &&
+                       stages <= kDecClusterWide * (heads <= wide_clusters(true) ? kDecWideStagesDeep : kDecWideStages);
   if (sixteen) s = kDecClusterWide;
   cluster = s > 1 && (s <= kDecClusterMax || sixteen) ? 1 : 0;         // (sixteen splits that come out as such are not one)
   if (cluster)
@@ -452,15 +452,15 @@ static bool dec_allow(K kern, bool wide) {
     return ok ? 1 : 0;
   }) > 0;
 }
-static int wide_clusters() {
-  static const char key = 0;
-  return once_per_device(&key, []() {
+static int wide_clusters(bool deep) {
+  static const char keys[2] = {};
+  return once_per_device(&keys[deep], [&]() {
     const auto kern = decode_attn_kernel<true, true, true>;
     if (!dec_allow(kern, true)) return 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kDecClusterWide, 64, 1);
     cfg.blockDim = dim3(dec_threads(true), 1, 1);
-    cfg.dynamicSmemBytes = dec_smem(kDecStages);
+    cfg.dynamicSmemBytes = dec_smem(deep ? kDecMaxStages : kDecStages);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = kDecClusterWide;
@@ -494,10 +494,10 @@ int decode_launch(const void* q, const void* k, const void* v, int dtype, int ba
   p.batch = batch; p.hkv = hkv; p.group = hq / hkv; p.k_len = k_len;
   p.stages = (k_len + kDecKeys - 1) / kDecKeys;
   p.splits = decode_splits(batch, hkv, k_len, p.cluster);
-  // where every CTA has an SM to itself its ring is deeper (of sixteen, whose clusters are counted for rings of three: half as many)
+  // where every CTA has an SM to itself its ring is deeper
   p.ring = kDecStages;
   const long long heads = static_cast<long long>(batch) * hkv;
-  if (p.splits > kDecClusterMax ? p.cluster && 2 * heads <= wide_clusters() : 4 * p.splits * heads <= 3LL * sm_count()) {
+  if (p.splits > kDecClusterMax ? p.cluster && heads <= wide_clusters(true) : 4 * p.splits * heads <= 3LL * sm_count()) {
     const int most = (p.stages + p.splits - 1) / p.splits;
     p.ring = most < kDecStages ? kDecStages : (most > kDecMaxStages ? kDecMaxStages : most);
   }
