@@ -127,6 +127,7 @@ int xattn_b200_estimate_f32(const float* q, const float* k, int batch, int hq, i
  * (`rounded` not NULL) on its sums, with the diagonal cleaned up.  Where every row of the estimate sees a single column tile the
  * selection happens inside its kernel.
  * Fields have the meaning of the arguments of those functions; list_q_len and list_k_len are the lengths of the lists.
+ * Where a device wait ran out (status word) the sums are undefined; every row of the mask and every list is written all the same.
  */
 typedef struct {
   const void *q, *k;

@@ -51,3 +51,23 @@ def test_a_wait_that_runs_out_reports_101_and_leaves_the_context_usable(tmp_path
     out = xattn_b200.Xattention_prefill(q, q, q, 16, threshold=0.9, chunk_size=2048)
     xattn_b200.check_device_status(dev)
     assert torch.isfinite(out.float()).all()
+
+
+@pytest.mark.parametrize("k_blocks", [5, 128, 300])
+def test_rows_without_a_selection_are_empty(tmp_path, k_blocks):
+    """Where a wait of the estimate ran out, the rows of the mask and the lists that its kernel would have selected are memory that
+    nobody wrote: its teardown empties them, those rows and no others."""
+    lib = _build(tmp_path)
+    lib.forget_probe.argtypes = [ctypes.c_int] * 3 + [ctypes.c_void_p] * 2 + [ctypes.c_int] * 3 + [ctypes.c_void_p]
+    heads, q_blocks, list_q_blocks = 3, 21, 19        # (the last two query blocks are padding without lists)
+    for bh, qb0, n in ((0, 0, 4), (1, 8, 8), (2, 16, 8), (2, 20, 1)):
+        mask = torch.full((heads, q_blocks, k_blocks), 7, dtype=torch.uint8, device="cuda")
+        cnt = torch.full((heads, list_q_blocks), 9, dtype=torch.int32, device="cuda")
+        want_mask, want_cnt = mask.clone(), cnt.clone()
+        want_mask[bh, qb0:qb0 + n] = 0
+        want_cnt[bh, qb0:qb0 + n] = 0
+        stream = torch.cuda.current_stream().cuda_stream
+        assert lib.forget_probe(q_blocks, k_blocks, list_q_blocks, mask.data_ptr(), cnt.data_ptr(), bh, qb0, n, stream) == 0
+        assert torch.equal(mask, want_mask) and torch.equal(cnt, want_cnt)
+        assert lib.forget_probe(q_blocks, k_blocks, list_q_blocks, None, None, bh, qb0, n, stream) == 0
+    torch.cuda.synchronize()

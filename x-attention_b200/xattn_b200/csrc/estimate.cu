@@ -446,13 +446,6 @@ __device__ __forceinline__ void est_select_rows(const EstGeom& g, const EstSelec
     select_row<1>(sums, sel.p, sel.thr_per_head, sel.mask, sel.idx, sel.cnt, bh * g.qb_total + qb0 + r, lane);
 }
 
-// After a wait that ran out: the rows of a tile list nothing, so that nobody reads a list that was never written.
-template <int RBS>
-__device__ __forceinline__ void est_forget_rows(const EstGeom& g, const EstSelect& sel, int bh, int mt) {
-  const int r = static_cast<int>(threadIdx.x), qb = mt * kTileM / RBS + r;
-  if (sel.cnt && r < kTileM / RBS && qb < sel.p.list_q_blocks && qb < g.qb_total) sel.cnt[static_cast<size_t>(bh) * sel.p.list_q_blocks + qb] = 0;
-}
-
 // Eight fp32 values, in pairs: the next term of each, the rounding of what the terms before leave.
 __device__ __forceinline__ uint4 next_term(unsigned long long (&v)[4]) {
   uint32_t w[4];
@@ -829,7 +822,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       for (int tile = tile0; tile < total_tiles; tile += tile_step) {
         int bh, mt, nt;
         decode_tile(g, g.n_mtiles, tile_lo, tile_prefix, tile, bh, mt, nt, interleave);
-        est_forget_rows<RBS>(g, sel, bh, mt);
+        forget_rows(sel.p, sel.mask, sel.cnt, bh, (mt * kTileM + rank * (kTileM / split)) / RBS, kTileM / split / RBS);
       }
     __syncthreads();
   } else if (selects(kDirect, kF32) && sel.on && split > 1) {

@@ -353,6 +353,18 @@ __device__ __forceinline__ void select_row(const float* sums, const SelParams& p
   finish_row(p, R, cur, word, lane, o);
 }
 
+// By a whole CTA, where sums were never finished (a device wait ran out): query blocks [qb0, qb0 + n) of a head select and list
+// nothing, so that nobody reads a row of the mask or a list that was never written.
+__device__ __forceinline__ void forget_rows(const SelParams& p, uint8_t* mask_out, int32_t* cnt_out, int bh, int qb0, int n) {
+  for (int qb = qb0; qb < qb0 + n && qb < p.q_blocks; ++qb) {
+    if (mask_out) {
+      uint8_t* row = mask_out + (static_cast<size_t>(bh) * p.q_blocks + qb) * p.k_blocks;
+      for (int c = threadIdx.x; c < p.k_blocks; c += blockDim.x) row[c] = 0;
+    }
+    if (cnt_out && threadIdx.x == 0 && qb < p.list_q_blocks) cnt_out[static_cast<size_t>(bh) * p.list_q_blocks + qb] = 0;
+  }
+}
+
 int select_params(const SelCall& c, SelParams& p);      // checks the call
 
 int select_launch(const SelCall& c, int* status, cudaStream_t stream);
