@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kF32 ? f32_threads(kDirect) : kGemmThreads, 1)
 est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt, const EstGeom g,
                 const int* tile_lo, const int* tile_prefix, float* __restrict__ partial,
-                float2* __restrict__ mtile, float* __restrict__ sums, const uint32_t idesc, const EstRounded rounded, const EstSelect sel, int* status) {
+                float2* __restrict__ mtile, float* sums, const uint32_t idesc, const EstRounded rounded, const EstSelect sel, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_tab[kTabInts];
   if (g.tab_n) {                                  // (made visible by the __syncthreads() that ends the prologue)
@@ -1109,7 +1109,7 @@ constexpr int kSumThreads = 128;
 template <int RBS, int kTeam, int kVec>
 __global__ void __launch_bounds__(kSumThreads)
 est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix, const float* __restrict__ partial,
-                    const float2* __restrict__ mtile, float* __restrict__ sums, int seg_tiles, const EstSelect sel) {
+                    const float2* __restrict__ mtile, float* sums, int seg_tiles, const EstSelect sel) {
   extern __shared__ float s_factors[];                     // [team][tile][row] factors, seg_tiles tiles at a time
   __shared__ float2 s_part[4][RBS];                        // (teams of four warps) [warp][row] (max, sum)
   constexpr int kParts = kTeam / RBS, kTeams = kSumThreads / kTeam;

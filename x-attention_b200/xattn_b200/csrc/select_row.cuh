@@ -126,6 +126,9 @@ __device__ __forceinline__ void select_row(const float* sums, const SelParams& p
   const float* x = sums + static_cast<size_t>(w) * n_read;
   const double thr = thr_per_head ? static_cast<double>(ld_written(thr_per_head + bh % p.heads)) : p.threshold;
 
+  // The row may be what this warp, or its CTA, has just stored: it is behind a barrier of theirs, and the compiler, which does not know
+  // what the loads read, keeps the stores in front of them.
+  asm volatile("" ::: "memory");
   // ---- the row, once; scores as bit patterns (positive floats order like integers), forced and non-positive ones as 0
   uint32_t v[4 * kVec];
 #pragma unroll
