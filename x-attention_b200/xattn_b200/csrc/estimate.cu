@@ -910,11 +910,6 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before();
   cluster_sync_all();               // barriers of both CTAs are initialised before any remote arrival or copy
   tc_fence_after();
-  // In long calls the next kernel comes as the last tiles finish, not before: CTAs of it that sat beside this one for milliseconds then
-  // ran with this kernel's division of the SM's memory between cache and shared memory (video diffusion: block sums 575 us, 510 like
-  // this; short calls want it early: 1024 tokens against 70000 97.5 us a call like this, 93.5 early).
-  const bool late = g.tab_n == 0;                           // more than 64 row tiles
-  if (!late) pdl_launch_dependents();
   pdl_wait();                       // up to here nothing was touched that an earlier kernel writes
   const uint32_t tmem_base = *tmem_slot;
 
@@ -969,7 +964,12 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
       }
     }
-    if (late) pdl_launch_dependents();
+    // The next kernel comes as the last tiles finish, not before: its CTAs would sit beside this one's for as long as those run, and the
+    // block sums are then slower (video diffusion 575 us, 510 like this; presumably as the SM's memory stays divided between cache and
+    // shared memory the way this kernel wants it).  us a call, early and like this: 1024 tokens against 70000 101.4 and 97.4, 5000 tokens
+    // (estimate and mask, stride 8) 31.25 and 31.10, 32768 tokens (the same, stride 16) 161.0 and 160.4, 20000 tokens 248.5 and 245.1,
+    // 60000 tokens at stride 8 1923 and 1911, video diffusion 15361 and 15338; in front of the attention 65536 tokens 494 and 496.
+    pdl_launch_dependents();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (even CTA; converged warp, one thread issues)
     if (rank == 0) {
