@@ -67,3 +67,17 @@ def test_ops_refuse_cpu_tensors():
 def test_reference_import_path():
     from xattn.src.Xattention import Xattention_prefill, xattn_estimate  # noqa: F401
     from xattn.src.utils import find_blocks_chunked  # noqa: F401
+
+
+def test_the_arguments_of_the_combined_call_are_bound_in_order():
+    from xattn_b200 import _lib
+    text = open(os.path.join(ROOT, "include", "xattn_b200.h")).read()
+    body = re.search(r"typedef struct \{([^}]*)\} xattn_b200_estimate_select_args;", text).group(1)
+    kinds = {"int": ctypes.c_int, "int64_t": ctypes.c_int64, "float": ctypes.c_float, "double": ctypes.c_double, "size_t": ctypes.c_size_t}
+    fields = []
+    for line in body.split(";"):
+        words = line.replace("const ", "").split(None, 1)
+        if words:
+            fields += [(n.strip(" *"), ctypes.c_void_p if "*" in n else kinds[words[0].strip("*")])
+                       for n in (words[1] if "*" not in words[0] else "*" + words[1]).split(",")]
+    assert fields == _lib.EstimateSelectArgs._fields_

@@ -15,6 +15,18 @@ SEMANTICS_TORCH, SEMANTICS_TRITON, SEMANTICS_TORCH_BAND = 0, 1, 2
 
 _i, _i64, _f, _d, _p, _sz = C.c_int, C.c_int64, C.c_float, C.c_double, C.c_void_p, C.c_size_t
 
+
+
+class EstimateSelectArgs(C.Structure):
+    """xattn_b200_estimate_select_args"""
+    _fields_ = [(n, t) for names, t in (
+        ("q k", _p), ("dtype batch hq hkv q_len k_len head_dim", _i),
+        ("q_stride_b q_stride_h q_stride_l k_stride_b k_stride_h k_stride_l", _i64), ("stride block_size chunk_size", _i), ("scale", _f),
+        ("causal semantics", _i), ("attn_sums workspace", _p), ("workspace_bytes", _sz), ("q_bf16 k_bf16", _p), ("threshold", _d),
+        ("threshold_per_head", _p), ("keep_sink keep_recent", _i), ("mask rounded", _p), ("rounded_dtype", _i), ("block_idx block_cnt", _p),
+        ("list_q_len list_k_len", _i), ("status", _p)) for n in names.split()]
+
+
 # name -> (restype, argtypes); must list every symbol the header declares
 SIGNATURES = {
     "xattn_b200_version": (_i, []),
@@ -31,7 +43,7 @@ SIGNATURES = {
                                         _i, _i, _i, _f, _i, _i, _p, _p, _p]),
     "xattn_b200_estimate_f32": (_i, [_p, _p, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64, _i64,
                                      _i, _i, _i, _f, _i, _i, _p, _p, _sz, _p, _p, _p, _p]),
-    "xattn_b200_estimate_select": (_i, [_p, _p]),
+    "xattn_b200_estimate_select": (_i, [C.POINTER(EstimateSelectArgs), _p]),
     "xattn_b200_estimate_f32_terms": (_i, [_i, _i, _i, _i, _i, _i, _i, _i, _i]),
     "xattn_b200_split_f32": (_i, [_p, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i, _p, _p]),
     "xattn_b200_split_f32_terms": (_i, [_p, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i, _p, _p]),
