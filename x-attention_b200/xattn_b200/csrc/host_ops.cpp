@@ -234,7 +234,7 @@ Tensor estimate(const Tensor& q_, const Tensor& k_, const Geometry& g, const Est
     t.q_bf16 = dtype == XATTN_B200_F32 && q16 ? q16->data_ptr() : nullptr;
     t.k_bf16 = dtype == XATTN_B200_F32 && k16 ? k16->data_ptr() : nullptr;
     t.status = at_.status;
-    check(xattn_b200_estimate_select(then, at_.stream), "estimate_select");
+    check(xattn_b200_estimate_select(then, at_.stream), "estimate");
     return sums;
   }
   if (dtype == XATTN_B200_F32)
