@@ -58,14 +58,19 @@ struct EstRounded {
 // Only the kernel of single CTAs with 128-column tiles of 16-bit operands does it: in the others the epilogue has no registers left for
 // it (spills: 4096 tokens against 65536 51.9 -> 52.5 us a call although nothing was selected there), or, CTA pairs with their few
 // steps per tile, no time (114688 tokens at stride 8 939 -> 967, 3590 tokens of a 16384-token chunk 34.5 -> 38.1).
-__host__ __device__ constexpr bool selects(int direct, bool f32) { return direct == 1 && !f32; }
+// And only calls that select there take the kernel that can: the others' epilogue is the faster without that code (1003 tokens at
+// stride 8 25.4 us a call with it, 24.5 without).
+__host__ __device__ constexpr bool can_select(int direct, bool f32) { return direct == 1 && !f32; }
 struct EstSelect {
-  int on;
   SelParams p;
   const float* thr_per_head;
   uint8_t* mask;
   int32_t *idx, *cnt;
 };
+
+struct EstNothing {};
+template <bool kSelect>
+using EstSelectIf = std::conditional_t<kSelect, EstSelect, EstNothing>;
 
 struct EstGeom {
   int batch, hq, hkv;
@@ -437,7 +442,6 @@ __device__ __forceinline__ void est_epilogue_row_direct(const EstGeom& g, Load l
 
 // Selects query blocks [qb0, qb0 + n) of a head, whose sums this warp (or, behind a barrier, its CTA) has written: every
 // `step`-th of them from the `first` on.
-template <int RBS>
 __device__ __forceinline__ void est_select_rows(const EstGeom& g, const EstSelect& sel, const float* sums, int bh, int qb0, int n, int first,
                                                 int step, int lane) {
   __syncwarp();
@@ -469,12 +473,13 @@ __device__ __forceinline__ uint4 next_term(unsigned long long (&v)[4]) {
 // bf16 roundings written here, 151 -> 114 us, 2 us of them for the proxy fence of every unit).  Bound by the latency of a
 // converter's step (waits, shared-memory traffic next to the MMAs', three dependent roundings); with loads alone it runs in 30
 // us.  Sixteen converter warps, or eight where the epilogue of a single tile needs the registers.
-template <int RBS, int kDirect, bool kF32>
+// kSelect: and selects on its rows (can_select)
+template <int RBS, int kDirect, bool kF32, bool kSelect>
 __global__ void __launch_bounds__(kF32 ? f32_threads(kDirect) : kGemmThreads, 1)
 est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmQt, const __grid_constant__ CUtensorMap tmKt, const EstGeom g,
                 const int* tile_lo, const int* tile_prefix, float* __restrict__ partial,
-                float2* __restrict__ mtile, float* sums, const uint32_t idesc, const EstRounded rounded, const EstSelect sel, int* status) {
+                float2* __restrict__ mtile, float* sums, const uint32_t idesc, const EstRounded rounded, const EstSelectIf<kSelect> sel, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_tab[kTabInts];
   if (g.tab_n) {                                  // (made visible by the __syncthreads() that ends the prologue)
@@ -800,8 +805,8 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         est_epilogue_row_direct<RBS, kDirect>(g, load, nvis, clo, chi,
                                               sums + (static_cast<size_t>(bh) * g.qb_total + (qb < g.qb_total ? qb : 0)) * out_cols, col0, out_cols,
                                               qb < g.qb_total, lane);
-        if constexpr (selects(kDirect, kF32)) {
-          if (sel.on && split == 1) est_select_rows<RBS>(g, sel, sums, bh, (mt * kTileM + quad * 32) / RBS, 32 / RBS, 0, 1, lane);
+        if constexpr (kSelect) {
+          if (split == 1) est_select_rows(g, sel, sums, bh, (mt * kTileM + quad * 32) / RBS, 32 / RBS, 0, 1, lane);
         }
       } else {
         const size_t tile_at = scratch_tile(g, bh, mt, nt, tile_lo[mt]) * kTileM;
@@ -818,19 +823,21 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000) { __nanosleep(1000); }
     if (threadIdx.x == 0 && status) atomicExch(status, static_cast<int>(kDevWaitTimeout));
-    if (selects(kDirect, kF32) && sel.on)
+    if constexpr (kSelect)
       for (int tile = tile0; tile < total_tiles; tile += tile_step) {
         int bh, mt, nt;
         decode_tile(g, g.n_mtiles, tile_lo, tile_prefix, tile, bh, mt, nt, interleave);
         forget_rows(sel.p, sel.mask, sel.cnt, bh, (mt * kTileM + rank * (kTileM / split)) / RBS, kTileM / split / RBS);
       }
     __syncthreads();
-  } else if (selects(kDirect, kF32) && sel.on && split > 1) {
-    // a cluster's CTA has finished 128 / split rows, few query blocks: a warp each
-    int bh, mt, nt;
-    decode_tile(g, g.n_mtiles, tile_lo, tile_prefix, tile0, bh, mt, nt, interleave);
-    est_select_rows<RBS>(g, sel, sums, bh, (mt * kTileM + rank * (kTileM / split)) / RBS, kTileM / split / RBS, warp,
-                         static_cast<int>(blockDim.x >> 5), lane);
+  } else if constexpr (kSelect) {
+    if (split > 1) {
+      // a cluster's CTA has finished 128 / split rows, few query blocks: a warp each
+      int bh, mt, nt;
+      decode_tile(g, g.n_mtiles, tile_lo, tile_prefix, tile0, bh, mt, nt, interleave);
+      est_select_rows(g, sel, sums, bh, (mt * kTileM + rank * (kTileM / split)) / RBS, kTileM / split / RBS, warp,
+                      static_cast<int>(blockDim.x >> 5), lane);
+    }
   }
   if (warp == 1) {
     tc_fence_after();
@@ -1109,7 +1116,7 @@ constexpr int kSumThreads = 128;
 template <int RBS, int kTeam, int kVec>
 __global__ void __launch_bounds__(kSumThreads)
 est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix, const float* __restrict__ partial,
-                    const float2* __restrict__ mtile, float* sums, int seg_tiles, const EstSelect sel) {
+                    const float2* __restrict__ mtile, float* sums, int seg_tiles, const EstSelectIf<(kVec > 0)> sel) {
   extern __shared__ float s_factors[];                     // [team][tile][row] factors, seg_tiles tiles at a time
   __shared__ float2 s_part[4][RBS];                        // (teams of four warps) [warp][row] (max, sum)
   constexpr int kParts = kTeam / RBS, kTeams = kSumThreads / kTeam;
@@ -1517,15 +1524,15 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // eight query blocks at stride 16, two rounds for its six warps (2100 tokens 35.4 us a call with it, 35.2 without).  Otherwise
   // est_blocksum_kernel selects, rows of up to 512.
   EstSelect sel;
-  sel.on = 0;
+  bool selecting = false;
   if (select) {
     const SelCall& c = *select;
     const int cols = g.band ? g.bpc : g.kb_total;
-    const bool here = direct ? !use_pairs && selects(g.tile_n / 128, f32) && (g.split == 4 || (g.split == 1 && many)) && cols <= 128 : cols <= 512;
+    const bool here = direct ? !use_pairs && can_select(g.tile_n / 128, f32) && (g.split == 4 || (g.split == 1 && many)) && cols <= 128 : cols <= 512;
     if (here && c.k_blocks <= 1024 && c.attn_sums == attn_sums && c.batch == batch && c.heads == hq && c.q_blocks == g.qb_total &&
         c.k_blocks == g.kb_total && c.bpc == g.bpc && (c.band ? 1 : 0) == g.band) {
       if ((rc = select_params(c, sel.p))) return rc;
-      sel.on = 1;
+      selecting = true;
       sel.thr_per_head = c.thr_per_head;
       sel.mask = c.mask;
       sel.idx = c.block_idx;
@@ -1650,15 +1657,18 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
       rounded.k = nullptr;
     }
   }
-  auto launch = [&](auto kern, int threads, int smem) -> int {
+  auto launch = [&](auto kern, int threads, int smem, auto what) -> int {
     if (!allow_smem(kern, smem)) return XATTN_B200_ERR_CUDA;
     return launch_dependent_clusters(kern, g.split, dim3(grid), dim3(threads), smem, stream, tmQ, tmK, tmQt, tmKt, g, (const int*)tile_lo,
-                                     (const int*)tile_prefix, partial, mtile, attn_sums, idesc, rounded, sel, status);
+                                     (const int*)tile_prefix, partial, mtile, attn_sums, idesc, rounded, what, status);
   };
   auto launch_type = [&](auto rbs, auto halves) -> int {
     constexpr int kRbs = decltype(rbs)::value, kDirect = decltype(halves)::value;
-    return f32 ? launch(est_gemm_kernel<kRbs, kDirect, true>, f32_threads(kDirect), kF32Smem + 2048)
-               : launch(est_gemm_kernel<kRbs, kDirect, false>, kGemmThreads, kGemmSmem);
+    if constexpr (can_select(kDirect, false)) {
+      if (selecting) return launch(est_gemm_kernel<kRbs, kDirect, false, true>, kGemmThreads, kGemmSmem, sel);
+    }
+    return f32 ? launch(est_gemm_kernel<kRbs, kDirect, true, false>, f32_threads(kDirect), kF32Smem + 2048, EstNothing())
+               : launch(est_gemm_kernel<kRbs, kDirect, false, false>, kGemmThreads, kGemmSmem, EstNothing());
   };
   auto launch_rbs = [&](auto rbs) -> int {
     if (!direct) return launch_type(rbs, std::integral_constant<int, 0>());
@@ -1681,19 +1691,19 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   const bool wide = items < 32LL * sm_count();
   const int teams = wide ? 1 : kSumThreads / 32, seg_max = 32 * 1024 / (4 * g.rbs * teams);
   const int seg_tiles = g.m_pitch < seg_max ? g.m_pitch : seg_max;
-  auto launch_sums = [&](auto kern) -> int {
+  auto launch_sums = [&](auto kern, auto what) -> int {
     return launch_dependent(kern, dim3(static_cast<unsigned>((items + teams - 1) / teams)), dim3(kSumThreads),
                             static_cast<size_t>(teams) * seg_tiles * g.rbs * sizeof(float), stream, g, (const int*)tile_lo,
-                            (const int*)tile_prefix, (const float*)partial, (const float2*)mtile, attn_sums, seg_tiles, sel);
+                            (const int*)tile_prefix, (const float*)partial, (const float2*)mtile, attn_sums, seg_tiles, what);
   };
   // with the selection: the instantiation with just enough registers for a row of sums
   auto launch_vec = [&](auto rbs, auto team) -> int {
     constexpr int kRbs = decltype(rbs)::value, kTeam = decltype(team)::value;
     const int cols = g.band ? g.bpc : g.kb_total;
-    if (!sel.on) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 0>);
-    if (cols <= 128) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 1>);
-    if (cols <= 256) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 2>);
-    return launch_sums(est_blocksum_kernel<kRbs, kTeam, 4>);
+    if (!selecting) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 0>, EstNothing());
+    if (cols <= 128) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 1>, sel);
+    if (cols <= 256) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 2>, sel);
+    return launch_sums(est_blocksum_kernel<kRbs, kTeam, 4>, sel);
   };
   auto launch_team = [&](auto rbs) -> int {
     return wide ? launch_vec(rbs, std::integral_constant<int, 128>()) : launch_vec(rbs, std::integral_constant<int, 32>());
