@@ -356,8 +356,6 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
               ln = tile_list(p, block_idx, tn, tile_count(p, block_cnt, tn));
               wn = list_entry(ln, wl);
             }
-            // (no unit is left for this SM: the set-up of the kernel after this one may run under the tail)
-            if (!kList && !kTwo && unit < 0 && p.early_next) pdl_launch_dependents();
             if (!wait(unit_empty + 8 * (k % kUnitSlots), (k / kUnitSlots & 1) ^ 1)) { ok = false; break; }
             if (wl == 0) reinterpret_cast<int4*>(unit_ring)[2 * (k % kUnitSlots) + s] = make_int4(tn.b, tn.h, tn.qb, ln.n);
             __syncwarp();
@@ -365,6 +363,8 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           }
         }
       }
+      // (no unit is left for this SM, and its last one's tiles are on their way: the set-up of the kernel after this one may run under the tail)
+      if (!kList && !kTwo && p.early_next) pdl_launch_dependents();
       // the end marker: a step that no stream uses
       if (lane == 0 && ok && mbar_wait(bar(step & 1, K_EMPTY), ((step >> 1) & 1) ^ 1, abort_flag)) {
         ring[step & (kRingEntries - 1)] = kStepEnd;
@@ -983,9 +983,12 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
   const int super_rows = (p.q_blocks + 1) / 2;
   const long long units = static_cast<long long>(super_rows) * batch * hq;
   if (units > 0x3fffffffLL || p.list_k_blocks > 65534) return XATTN_B200_ERR_LIMIT;
-  // Short calls let the next kernel set up under their tail (back to back: 1003 tokens 26.8 -> 26.2 us a call, 2100 tokens 36.6 ->
-  // 35.2); with more than two units per SM it gains nothing (4096 tokens against 65536 51.9 and 52.2, 32768 tokens 473 and 477).
-  p.early_next = units <= 2LL * sm_count() ? 1 : 0;
+  // Short calls let the next kernel set up under their tail (us a call, back to back, without and with it: 1003 tokens at stride 16 24.0 and
+  // 23.1, 2000 tokens at stride 8 36.7 and 36.0); with more than two units per SM it gains nothing (4096 tokens against 65536 51.9 and
+  // 52.2, 32768 tokens 473 and 477).  Dense calls only up to one unit per SM (300 tokens 12.2 and 11.0, 1003 tokens 21.0 and 19.7): beyond
+  // that other CTAs get hold of the units left over, and it goes either way (1100 tokens 23.0 and 22.6, 1400 28.3 and 28.9, 1530 31.4 and
+  // 31.9, 2000 45.6 and 45.4).
+  p.early_next = units <= (dense ? 1LL : 2LL) * sm_count() ? 1 : 0;
   p.by_units = make_fast_div(causal ? batch * hq : super_rows * (hq / hkv));
   p.by_hq = make_fast_div(hq);
   p.by_batch = make_fast_div(batch);
