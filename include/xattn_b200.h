@@ -124,8 +124,11 @@ int xattn_b200_estimate_f32(const float* q, const float* k, int batch, int hq, i
 /*
  * Phases 1 and 2 in one call (xattn/src/Xattention.py:13-299): the estimate (dtype XATTN_B200_F32: with q_bf16 and k_bf16 as in
  * xattn_b200_estimate_f32), then xattn_b200_select, _select_band (semantics XATTN_B200_SEMANTICS_TORCH_BAND) or _select_rounded
- * (`rounded` not NULL) on its sums, with the diagonal cleaned up.  Where every row of the estimate sees a single column tile the
- * selection happens inside its kernel.
+ * (`rounded` not NULL) on its sums, with the diagonal cleaned up.  The selection happens inside the estimate's last kernel where
+ *   - every row sees a single tile of 128 columns, the operands have 16 bits, there are few tiles (clusters of four CTAs share one) or
+ *     more than four per SM, and a row has up to 128 sums, in the GEMM; or
+ *   - rows see more than one tile and have up to 512 sums, in the kernel that adds them up (up to 1024 key blocks),
+ * and otherwise in a kernel of its own.  The results are the same.
  * Fields have the meaning of the arguments of those functions; list_q_len and list_k_len are the lengths of the lists.
  * Where a device wait ran out (status word) the sums are undefined; every row of the mask and every list is written all the same.
  */

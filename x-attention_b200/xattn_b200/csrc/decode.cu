@@ -6,17 +6,18 @@
 //
 // The step reads K and V once and does next to nothing with them, so it is HBM-bound (128K tokens, 8 kv heads: 537 MB, 83 us
 // at the measured copy bandwidth; measured 87 us) or, for short caches, pure latency.  Therefore:
-//   * the cache is split along its length so that every SM has two CTAs' worth of it; a CTA streams its keys through a ring
-//     of TMA stages (64 keys of K and V, 32 KiB each), three stages per CTA = 192 KiB in flight per SM, which covers the
-//     HBM latency (6.5 TB/s x 1 us / 148 SMs = 44 KiB) several times over;
+//   * the cache is split along its length over the SMs, two CTAs for each or one; a CTA streams its keys through a ring of TMA
+//     stages (64 keys of K and V, 32 KiB each): three stages where two CTAs share an SM, up to six where it has one to itself,
+//     192 KiB in flight per SM either way, which covers the HBM latency (6.5 TB/s x 1 us / 148 SMs = 44 KiB) several times over;
 //   * all query heads of a kv group are rows of one MMA (m16n8k16), so K and V are read once per kv head.  These are warp
 //     MMAs on purpose: with at most 16 useful rows a 128-row tcgen05 tile would be seven eighths padding, and the products
 //     take under a tenth of the time the bytes do;
 //   * every warp takes 16 keys of a stage and keeps a running softmax of its own; the four warps of a CTA are merged
 //     through shared memory at the end.  The CTAs of a (batch, kv head) are merged through distributed shared memory where
-//     they are a cluster (up to eight: caches of up to 4096 keys, or many heads), and by a small second kernel, launched as a
-//     dependent one, where there are more.  The second launch costs the host 2.5 us, which a step on a short cache would pay
-//     in full (2011 keys, 8 kv heads: 10.2 us a call with it, 6.0 without); a long cache hides it.
+//     they are a cluster (up to eight: caches of up to 4096 keys, or many heads; sixteen: see decode_splits), and by a small
+//     second kernel, launched as a dependent one, where there are more.  The second launch costs the host 2.5 us, which a step
+//     on a short cache would pay in full (2011 keys, 8 kv heads: 10.2 us a call with it, 6.0 without), and the second kernel
+//     starts when the first has ended; a long cache hides both.
 #include <type_traits>
 
 #include "attention_common.cuh"
@@ -412,8 +413,8 @@ decode_merge_kernel(const DecodeParams p, const float* __restrict__ part, const 
 // so are those of caches of up to 4096 keys, where eight CTAs of eight stages take about as long as the second kernel.
 // Longer caches: clusters of sixteen, where all of them fit on the chip at the same time (14 on this one with two CTAs per SM, seven
 // with one), rather than more CTAs and a second kernel, which starts when the first has ended and reads what it wrote.  us a
-// call, 1 sequence, 32 / 8 heads: 4200 keys 13.6 -> 8.8, 12717 19.0 -> 15.1, 30000 29.4 -> 27.7; 28 / 4 heads: 4200 12.0 -> 7.1, 30000
-// 27.8 -> 20.2, 60000 37.0 -> 34.7; 8 / 1 heads, 30000 keys: 45 -> 19.  Up to 128 of 148 SMs stream then, and the time per key is a
+// call, 1 sequence, 32 / 8 heads: 4200 keys 12.5 -> 8.3, 12717 18.8 -> 15.4, 30000 29.1 -> 27.8; 28 / 4 heads: 30000 27.4 -> 20.5, 60000
+// 36.6 -> 35.2; 8 / 1 heads, 30000 keys: 45 -> 19.  Up to 128 of 148 SMs stream then, and the time per key is a
 // third longer than with all of them (rings of three) or grows with the CTA's own share (deep rings, fewer heads): from about 40 and
 // 66 stages per CTA on the second kernel is the lesser cost.
 constexpr int kDecClusterMax = 8, kDecClusterStages = 64, kDecClusterWide = 16;
