@@ -175,7 +175,7 @@ def test_dense_rows_of_a_few_chunks(lq, lk, stride, chunk):
 @pytest.mark.parametrize("stride,hkv,chunk,causal,semantics", [(4, 20, 16384, True, "torch"), (8, 8, 16384, True, "triton"),
                                                                (16, 20, 8192, True, "torch"), (32, 8, 16384, False, "torch")])
 def test_many_query_blocks(stride, hkv, chunk, causal, semantics):
-    """Block sums by a warp per query block, which calls of many query blocks get: the first and the last head."""
+    """Calls of many row tiles, several column tiles per row: the first and the last head."""
     from xattn_b200 import ops
     hq, L = 40, 15400                                    # 40 * 128 (padded) query blocks; several column tiles per row
     g = torch.Generator().manual_seed(stride)
@@ -186,6 +186,47 @@ def test_many_query_blocks(stride, hkv, chunk, causal, semantics):
         want = orc.estimate_block_sums(q[:, h:h + 1].float(), k[:, h * hkv // hq:h * hkv // hq + 1].float(), 128, stride, 1.0, chunk, causal,
                                        semantics)
         assert torch.allclose(got[:, h:h + 1], want, rtol=RTOL, atol=ATOL), float((got[:, h:h + 1] - want).abs().max())
+
+
+@pytest.mark.parametrize("lq,lk,stride,chunk", [(1, 70000, 8, 16384), (300, 66001, 16, 2048), (2500, 40000, 4, 2048), (129, 70001, 32, 4096)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_key_blocks_over_several_ctas(lq, lk, stride, chunk, causal):
+    """Few row tiles against many key blocks: a row tile's are divided over CTAs, the last part being a short one."""
+    _check(2, 1, lq, lk, stride, chunk, causal, torch.bfloat16)
+
+
+@pytest.mark.parametrize("lq,lk,stride,chunk", [(8192, 8192, 16, 8192), (1024, 8192, 8, 2048), (3, 40000, 16, 16384)])
+def test_sums_off_a_16_byte_boundary(lq, lk, stride, chunk):
+    """Sums stored as vectors where their memory allows it: the same ones, and nothing beside them, where it does not."""
+    from xattn_b200 import _lib, ops
+    lib = _lib.load()
+    g = torch.Generator(device=DEV).manual_seed(lq)
+    q, k = torch.randn(1, 4, lq, 128, device=DEV, generator=g).bfloat16(), torch.randn(1, 2, lk, 128, device=DEV, generator=g).bfloat16()
+    want = ops.estimate_block_sums(q, k, stride, 128, chunk)
+    memory = torch.full((want.numel() + 8,), float("nan"), device=DEV)
+    sums = memory[1:1 + want.numel()]
+    ws = torch.empty(lib.xattn_b200_estimate_workspace_bytes(1, 4, lq, lk, stride, 128, chunk), dtype=torch.uint8, device=DEV)
+    _lib.check(lib.xattn_b200_estimate(q.data_ptr(), k.data_ptr(), _lib.BF16, 1, 4, 2, lq, lk, 128, *q.stride()[:3], *k.stride()[:3], stride, 128,
+                                       chunk, 128 ** -0.5 / stride, 1, 0, sums.data_ptr(), ws.data_ptr(), ws.numel(), None,
+                                       torch.cuda.current_stream().cuda_stream), "estimate")
+    assert torch.equal(sums.view(want.shape), want) and bool(memory[:1].isnan().all()) and bool(memory[1 + want.numel():].isnan().all())
+
+
+@pytest.mark.parametrize("stride,chunk,lq,lk", [(16, 512, 4096, 4096), (16, 1536, 4608, 9216), (8, 512, 1536, 3072), (4, 1024, 5120, 5120), (32, 2560, 5120, 5120)])
+def test_row_tiles_that_span_chunks(stride, chunk, lq, lk):
+    """The chunk band of row tiles of which every query block has a chunk of its own: the columns of it in the dense sums (which
+    another kernel may finish: sums of up to 128 x 32 probabilities in another order, 2^-24 each)."""
+    from xattn_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(chunk)
+    q, k = torch.randn(1, 4, lq, 128, device=DEV, generator=g).bfloat16(), torch.randn(1, 2, lk, 128, device=DEV, generator=g).bfloat16()
+    dense, band = (ops.estimate_block_sums(q, k, stride, 128, chunk, 1.0, True, band=b) for b in (False, True))
+    bpc, first = chunk // 128, (lk - lq) // 128
+    for c in range(lq // chunk):
+        rows = slice(c * bpc, (c + 1) * bpc)
+        assert torch.allclose(band[:, :, rows], dense[:, :, rows, first + c * bpc:first + (c + 1) * bpc], rtol=1e-5, atol=1e-6)
+    got = dense.cpu()
+    want = orc.estimate_block_sums(q.float().cpu(), k.float().cpu().repeat_interleave(2, 1), 128, stride, 1.0, chunk, True, "torch")
+    assert torch.allclose(got, want, rtol=RTOL, atol=ATOL), float((got - want).abs().max())
 
 
 @pytest.mark.parametrize("lq,lk,stride,chunk,causal", [(3, 3, 32, 2048, True), (1, 5, 16, 16384, False), (413, 4096, 8, 2048, True),

@@ -7,8 +7,8 @@ DEV = "cuda"
 
 
 # (tokens, stride, chunk): every way a row of sums is finished in the GEMM's epilogue -- clusters of four, which select there, and
-# those that leave it to a kernel behind them: clusters of two, single CTAs with a few tiles, tiles of 256 columns, CTA pairs -- and four
-# warps per query block behind it; ragged lengths, rows of padding, chunks of their own and all of the keys
+# those that leave it to a kernel behind them: clusters of two, single CTAs with a few tiles, tiles of 256 columns, CTA pairs -- and sixteen
+# warps per row tile behind it; ragged lengths, rows of padding, chunks of their own and all of the keys
 @pytest.mark.parametrize("hq,hkv", [(4, 2), (3, 3), (32, 8)])
 @pytest.mark.parametrize("q_len,k_len,stride,chunk", [
     (3, 3, 16, 2048), (200, 200, 4, 128), (1003, 1003, 16, 2048), (1003, 1003, 8, 2048), (1024, 1024, 8, 1024), (2000, 2000, 16, 4096),
@@ -76,7 +76,7 @@ def test_under_the_next_tiles(hq, hkv, L, stride, chunk, causal, dtype):
     _compare(hq, hkv, L, L, stride, chunk, dtype, causal, 0.93, launches=(mask, fused + 1 + extra))
 
 
-# Calls of at least 32 query blocks per SM: a warp per query block adds its sums and selects.  Bands of 128, 256 and 512 (the
+# Calls of at least 32 query blocks per SM: the kernel of the block sums selects on its row tiles.  Bands of 128, 256 and 512 (the
 # prefill) and dense rows of as many (the mask), every stride, ragged lengths.
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("hq,hkv,L,stride,chunk,causal", [

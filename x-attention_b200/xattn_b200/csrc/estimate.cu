@@ -15,7 +15,7 @@
 //                        warps run the epilogue: per row, max over the tile's visible columns, exp2,
 //                        sums over groups of block/S columns.  Output per (row, key block): an
 //                        un-normalised partial sum, plus the max it was taken against per (row, tile).
-//   est_blocksum_kernel  per query block: the rows' maxima and sums over their tiles, then per key block: normalise and
+//   est_blocksum_kernel  per row tile: the rows' maxima and sums over their column tiles, then per key block: normalise and
 //                        add the block/S rows.  (Rows of a single tile need neither, see est_epilogue_row_direct.)
 #include <math.h>
 
@@ -1099,141 +1099,203 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
 }
 
-// Normalisation of the partial sums, one CTA per query block:
+// Normalisation of the partial sums, a CTA per row tile:
 //   row i:  m_i = max_t m_{i,t},  l_i = sum_t s_{i,t} 2^(m_{i,t} - m_i)                (m, s = per-tile max and sum)
 //   out[kb] = sum_i partial[i][kb] * f_{i,t(kb)},  f_{i,t} = 2^(m_{i,t} - m_i) / l_i
-// A stream over the partial sums, bound by the latency of each query block's chain (statistics, factors, sums): a warp per query
-// block, a lane per key block, whose RBS rows it reads as 16-byte vectors (64 contiguous bytes for RBS = 16), a few key blocks in
-// flight at a time and the first ones while the statistics are computed; the factors come from shared memory.  The longest query
-// blocks go first.  Calls of few query blocks (a short prompt's last chunk against a long cache) have four warps per query block.
-// (32 heads, 32768 tokens: at stride 16 20.5 us with a CTA per query block, 12.7 like this; at stride 8 21.8 and 14.8.)
-// kVec > 0: the query block's warp (of four: the first) then selects on its row of sums, of up to 128 * kVec, see select_row: as a
-// kernel of its own that was a launch and a hand-over between two kernels more (stride 8: 2500 tokens 47.0 -> 44.2 us a call, 3000
-// 51.4 -> 48.6, 1024 against 70000 103 -> 93; at the power cap, from 8000 tokens on, nothing).  Rows of more than 512 sums go to the
-// selection kernel: with the registers that those take here the sums, which stream, are the slower for it (estimate and mask of 84758
-// tokens 3121 us apart, 3173 together).
-constexpr int kSumThreads = 128;
-template <int RBS, int kTeam, int kVec>
-__global__ void __launch_bounds__(kSumThreads)
+// A stream over the partial sums behind a short chain (statistics, factors): a key block's 128 rows are 512 contiguous bytes that a
+// warp reads as one vector per lane, kLines key blocks at a time, the first ones while the statistics are on their way; a lane's four
+// rows belong to one query block, whose lanes add by halves.  Bound by HBM where the partial sums do not stay in L2 (video diffusion,
+// 119K tokens: 1.33 GB), by latency otherwise.  A warp (or four) per query block read 64 bytes here and there of every key block and
+// loaded the next ones only when the ones before were added up.  us between the GEMM's end and the sums', before and now: 119K tokens
+// at stride 8 (24 heads) 521 and 284, 32768 at stride 8 17.1 and 12.1, 1024 tokens against 70000 16.5 and 7.0, 9973 9.4 and 5.7.
+// kVec > 0: and the selection on the tile's rows of sums, of up to 128 * kVec, from shared memory, a warp per row (select_values; as a
+// kernel of its own that is a launch and a hand-over between two kernels more): with the selection 32768 tokens at stride 16
+// 18.4 and 14.1, 9973 tokens at stride 8 13.6 and 8.1, 2500 tokens the call 24.8 and 21.0.
+// Rows of more than 512 sums go to the selection kernel, whose registers would leave too few warps here.
+constexpr size_t kSumSmem = 84 * 1024;                   // the tile's sums, for the selection: at most 32 rows of 512 and a few more
+
+template <int N>
+__device__ __forceinline__ void store_sums(float* p, const float* a) {
+  if constexpr (N == 1) *p = a[0];
+  else if constexpr (N == 2) *reinterpret_cast<float2*>(p) = make_float2(a[0], a[1]);
+  else {
+#pragma unroll
+    for (int j = 0; j < N; j += 4) *reinterpret_cast<float4*>(p + j) = make_float4(a[j], a[j + 1], a[j + 2], a[j + 3]);
+  }
+}
+
+template <int RBS, int kVec, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, kVec > 2 ? 24 / kWarps : 32 / kWarps)
 est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix, const float* __restrict__ partial,
-                    const float2* __restrict__ mtile, float* sums, int seg_tiles, const EstSelectIf<(kVec > 0)> sel) {
-  extern __shared__ float s_factors[];                     // [team][tile][row] factors, seg_tiles tiles at a time
-  __shared__ float2 s_part[4][RBS];                        // (teams of four warps) [warp][row] (max, sum)
-  constexpr int kParts = kTeam / RBS, kTeams = kSumThreads / kTeam;
-  constexpr int kAhead = kTeam > 32 || RBS > 16 ? 1 : 16 / RBS;          // key blocks per lane in flight (32 / RBS: 10 % slower)
+                    const float2* __restrict__ mtile, float* __restrict__ sums, int pitch, const EstSelectIf<(kVec > 0)> sel) {
+  extern __shared__ float s_rows[];                      // (kVec > 0) [query block][pitch]
+  __shared__ float4 s_max[kWarps][kTileM / 4], s_sum[kWarps][kTileM / 4];       // [warp][row] of the warp's tiles; [0]: of the whole row, and 1 / sum
+  constexpr int kLines = RBS == 32 ? 4 : 8;              // key blocks that a warp has in flight (a divisor of a tile's)
+  constexpr int kShare = RBS / 4, kLeft = kLines > kShare ? kLines / kShare : 1;      // lanes per query block; sums a lane ends up with
   pdl_launch_dependents();
   pdl_wait();
-  const int team = threadIdx.x / kTeam, tid = threadIdx.x % kTeam, heads = g.batch * g.hq;
-  const int item = blockIdx.x * kTeams + team;
-  if (item >= heads * g.qb_total) return;                  // (a whole team, and teams of the whole CTA have none left over)
-  const int qb = g.qb_total - 1 - item / heads, bh = item % heads;
-  auto sync = [&]() {
-    if constexpr (kTeam == 32) __syncwarp(); else __syncthreads();
-  };
-  float* s_f = s_factors + team * seg_tiles * RBS;
-  const int i0 = qb * RBS, mt = i0 / kTileM, r0 = i0 % kTileM;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int mt = g.n_mtiles - 1 - blockIdx.y, bh = blockIdx.x;
+  const int i0 = mt * kTileM;
   const int nlo = g.tab_n ? g.tab[mt] : tile_lo[mt];
   const int ncnt = g.tab_n ? g.tab[kTabPrefix + mt + 1] - g.tab[kTabPrefix + mt] : tile_prefix[mt + 1] - tile_prefix[mt];
-  const int gpt = g.tile_n / RBS;                          // key blocks per tile
+  const int gpt = g.tile_n / RBS, by_gpt = __ffs(gpt) - 1;               // key blocks per tile, a power of two
   const size_t tile0 = scratch_tile(g, bh, mt, nlo, nlo);
-  const float2* ms = mtile + tile0 * kTileM + r0;
-  const float* pp = partial + tile0 * gpt * kTileM + r0;   // key block nlo * gpt + k: at k * kTileM
-  // band layout: only the key blocks of the query block's own chunk, [cur, cur + bpc)
-  const int cur = g.band ? (g.row_off + (i0 / g.rcs) * g.rcs) / RBS : 0, n_out = g.band ? g.bpc : g.kb_total;
-  int k_end = ncnt * gpt;                                  // blocks past the last one that any of the rows sees are zero
-  {
-    const int last = i0 + RBS - 1 < g.rows_valid - 1 ? i0 + RBS - 1 : g.rows_valid - 1;
+  const float4* ms = reinterpret_cast<const float4*>(mtile + tile0 * kTileM) + 2 * lane;        // rows 4 lane .. 4 lane + 3
+  const float* pp = partial + tile0 * gpt * kTileM + 4 * lane;                   // key block nlo * gpt + k: at k * kTileM
+  const int n_out = g.band ? g.bpc : g.kb_total;
+  // key block k is column k + shift(r) of the tile's r-th query block (band layout: only the key blocks of its own chunk are stored)
+  auto shift = [&](int r) { return nlo * gpt - (g.band ? (g.row_off + ((i0 + r * RBS) / g.rcs) * g.rcs) / RBS : 0); };
+  int k_end = 0;                                         // blocks past the last one that any of the rows sees are zero (and not written by the GEMM)
+  if (i0 < g.rows_valid) {
     int lo, hi;
-    row_bounds(g, last, lo, hi);
-    const int vis = hi / RBS + 1 - nlo * gpt;
-    if (i0 >= g.rows_valid) k_end = 0;
-    else if (vis < k_end) k_end = vis;
+    row_bounds(g, i0 + kTileM - 1 < g.rows_valid - 1 ? i0 + kTileM - 1 : g.rows_valid - 1, lo, hi);
+    k_end = hi / RBS + 1 - nlo * gpt;
+    if (k_end > ncnt * gpt) k_end = ncnt * gpt;
   }
-  float4 p4[kAhead][RBS / 4];
-  auto fetch = [&](int kl0) {                              // the rows of outputs kl0 + u * kTeam; zeros outside the tiles
+  float4 p4[kLines];
+  float x[4];
+  auto fetch = [&](int k0) {                             // the rows of key blocks k0 .. and their (max, sum) in that tile
+    const int t = k0 >> by_gpt;
+    const float4 a = ld_written(ms + t * (kTileM / 2)), b = ld_written(ms + t * (kTileM / 2) + 1);
+    x[0] = a.x; x[1] = a.z; x[2] = b.x; x[3] = b.z;
+    const float4* line = reinterpret_cast<const float4*>(pp + static_cast<size_t>(k0) * kTileM);
+    if (k0 + kLines <= k_end) {
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      const int kl = kl0 + u * kTeam, k = cur + kl - nlo * gpt;
-      const bool in = kl < n_out && k >= 0 && k < k_end;
+      for (int j = 0; j < kLines; ++j) p4[j] = ld_written_once(line + j * (kTileM / 4));
+    } else {
 #pragma unroll
-      for (int j = 0; j < RBS / 4; ++j)
-        p4[u][j] = in ? ld_written_once(reinterpret_cast<const float4*>(pp + static_cast<size_t>(k) * kTileM) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int j = 0; j < kLines; ++j) p4[j] = k0 + j < k_end ? ld_written_once(line + j * (kTileM / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
-  fetch(tid);
-  float row_m, row_inv;                                    // of row tid % RBS
+  // (kVec == 0: few row tiles have their key blocks divided over several CTAs)
+  const int k_first = (warp + kWarps * blockIdx.z) * kLines, k_step = kWarps * kLines * gridDim.z;
+  if (k_first < k_end) fetch(k_first);
   {
-    const int row = tid % RBS, part = tid / RBS;
-    const bool valid = i0 + row < g.rows_valid;
-    float m = -INFINITY, l = 0.f;
-    auto add = [&](float xm, float xl) {
-      if (xm > -INFINITY) {
-        const float mn = fmaxf(m, xm);
-        l = l * exp2f(m - mn) + xl * exp2f(xm - mn);
-        m = mn;
-      }
-    };
-    if (valid) {
-#pragma unroll 4
-      for (int t = part; t < ncnt; t += kParts) {
-        const float2 x = ld_written(ms + t * kTileM + row);
-        add(x.x, x.y);
+    // per warp the rows' maxima and sums over its tiles, then a row per thread over the warps
+    float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, l[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (int t = warp; t < ncnt; t += kWarps) {
+      const float4 a = ld_written(ms + t * (kTileM / 2)), b = ld_written(ms + t * (kTileM / 2) + 1);
+      const float xm[4] = {a.x, a.z, b.x, b.z}, xl[4] = {a.y, a.w, b.y, b.w};
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float mn = fmaxf(m[r], xm[r]);
+        if (t == warp) l[r] = xl[r];
+        else if (xm[r] > -INFINITY) l[r] = l[r] * fast_exp2(m[r] - mn) + xl[r] * fast_exp2(xm[r] - mn);
+        m[r] = mn;
       }
     }
-#pragma unroll
-    for (int o = RBS; o < 32; o <<= 1) add(__shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, l, o));
-    if constexpr (kTeam > 32) {
-      if ((threadIdx.x & 31) < RBS) s_part[threadIdx.x >> 5][row] = make_float2(m, l);
-      __syncthreads();
-      m = -INFINITY;
-      l = 0.f;
-#pragma unroll
-      for (int w = 0; w < 4; ++w) add(s_part[w][row].x, s_part[w][row].y);
+    s_max[warp][lane] = make_float4(m[0], m[1], m[2], m[3]);
+    s_sum[warp][lane] = make_float4(l[0], l[1], l[2], l[3]);
+    __syncthreads();
+    if (threadIdx.x < kTileM) {
+      float* sm = reinterpret_cast<float*>(s_max) + threadIdx.x;
+      float* sl = reinterpret_cast<float*>(s_sum) + threadIdx.x;
+      const int parts = ncnt < kWarps ? ncnt : kWarps;
+      float rm = -INFINITY, rl = 0.f;
+      for (int w = 0; w < parts; ++w) rm = fmaxf(rm, sm[w * kTileM]);
+      if (rm > -INFINITY)
+        for (int w = 0; w < parts; ++w) rl += sl[w * kTileM] * fast_exp2(sm[w * kTileM] - rm);
+      *sm = rm;
+      *sl = rl > 0.f ? 1.f / rl : 0.f;
     }
-    row_m = m;
-    row_inv = l > 0.f ? 1.f / l : 0.f;
+    __syncthreads();
   }
-  float* out = sums + (static_cast<size_t>(bh) * g.qb_total + qb) * n_out;
+  const float4 rm4 = s_max[0][lane], ri4 = s_sum[0][lane];
+  const float row_m[4] = {rm4.x, rm4.y, rm4.z, rm4.w}, row_inv[4] = {ri4.x, ri4.y, ri4.z, ri4.w};
+  const int ql = lane / kShare, part = lane % kShare;    // this lane's query block, and its place among the lanes of it
+  const int own_shift = shift(ql);
+  float* out = nullptr;
+  if constexpr (kVec == 0) out = sums + (static_cast<size_t>(bh) * g.qb_total + i0 / RBS + ql) * n_out;
+  const bool real = i0 / RBS + ql < g.qb_total, whole = (reinterpret_cast<uintptr_t>(sums) & 15) == 0;
+  const bool aligned = whole && ((n_out | own_shift) & 7) == 0;
 #pragma unroll 1
-  for (int t0 = 0; t0 == 0 || t0 < ncnt; t0 += seg_tiles) {
-    const int t1 = t0 + seg_tiles < ncnt ? t0 + seg_tiles : ncnt;
-    if (t0 > 0) {
-      sync();
-      fetch(tid);
+  for (int k0 = k_first; k0 < k_end; k0 += k_step) {
+    float f[4], a[kLines];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) f[r] = row_inv[r] > 0.f ? fast_exp2(x[r] - row_m[r]) * row_inv[r] : 0.f;
+#pragma unroll
+    for (int j = 0; j < kLines; ++j) a[j] = p4[j].x * f[0] + p4[j].y * f[1] + p4[j].z * f[2] + p4[j].w * f[3];
+    if (k0 + k_step < k_end) fetch(k0 + k_step);
+    // The sums over a query block's lanes, by halves: a lane gives away half of its sums and receives the other lane's part of
+    // the half it keeps.
+    int n = kLines, base = 0;
+#pragma unroll
+    for (int o = kShare / 2; o > 0; o >>= 1) {
+      if (n > 1) {
+        n >>= 1;
+        const bool upper = (part & o) != 0;
+        if (upper) base += n;
+#pragma unroll
+        for (int j = 0; j < kLines / 2; ++j)
+          if (j < n) a[j] = (upper ? a[j + n] : a[j]) + __shfl_xor_sync(0xffffffffu, upper ? a[j] : a[j + n], o);
+      } else {
+        a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+      }
     }
-    for (int t = t0 + tid / RBS; t < t1; t += kParts) {
-      const float x = ld_written(ms + t * kTileM + tid % RBS).x;
-      s_f[(t - t0) * RBS + tid % RBS] = row_inv > 0.f && x > -INFINITY ? exp2f(x - row_m) * row_inv : 0.f;
+    const bool writer = kLines >= kShare || (part & (kShare / kLines - 1)) == 0;     // (more lanes than sums)
+    const int k = k0 + base;
+    if constexpr (kVec > 0) {
+      if (writer) store_sums<kLeft>(s_rows + ql * pitch + k, a);
+    } else if (writer && real) {
+      if (aligned) {
+        if (k + own_shift >= 0 && k + own_shift < n_out) store_sums<kLeft>(out + k + own_shift, a);
+      } else {
+#pragma unroll
+        for (int j = 0; j < kLeft; ++j)
+          if (k + j + own_shift >= 0 && k + j + own_shift < n_out) out[k + j + own_shift] = a[j];
+      }
     }
-    sync();
+  }
+  const int k_sums = k_end > 0 ? (k_end + kLines - 1) / kLines * kLines : 0;     // of which there are sums; the others are zero
+  if constexpr (kVec == 0) {
+    if (blockIdx.z != 0) return;
 #pragma unroll 1
-    for (int kl0 = tid; kl0 < n_out; kl0 += kAhead * kTeam) {
-      float acc[kAhead];
+    for (int r = warp; r < kTileM / RBS && i0 / RBS + r < g.qb_total; r += kWarps) {
+      float* row = sums + (static_cast<size_t>(bh) * g.qb_total + i0 / RBS + r) * n_out;
+      const int s = shift(r);
+      if (whole && ((n_out | s) & 7) == 0) {
+        for (int c = 4 * lane; c < n_out; c += 128)
+          if (c - s < 0 || c - s >= k_sums) *reinterpret_cast<float4*>(row + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        for (int c = lane; c < n_out; c += 32)
+          if (c - s < 0 || c - s >= k_sums) row[c] = 0.f;
+      }
+    }
+  } else {
+    __syncthreads();
+#pragma unroll 1
+    for (int r = warp; r < kTileM / RBS && i0 / RBS + r < g.qb_total; r += kWarps) {
+      const int w = bh * g.qb_total + i0 / RBS + r, s = shift(r);
+      float* row = sums + static_cast<size_t>(w) * n_out;
+      uint32_t v[4 * kVec];
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int k = cur + kl0 + u * kTeam - nlo * gpt, t = k >= 0 && k < k_end ? k / gpt : -1;
-        acc[u] = 0.f;
-        if (t >= t0 && t < t1) {
-          const float4* f4 = reinterpret_cast<const float4*>(s_f + (t - t0) * RBS);
-#pragma unroll
-          for (int j = 0; j < RBS / 4; ++j) {
-            const float4 f = f4[j];
-            acc[u] += p4[u][j].x * f.x + p4[u][j].y * f.y + p4[u][j].z * f.z + p4[u][j].w * f.w;
+      for (int u = 0; u < kVec; ++u) {
+        const int c = u * 128 + 4 * lane, k = c - s;
+        float e[4] = {0.f, 0.f, 0.f, 0.f};
+        if (sel.p.vec_in && (s & 3) == 0) {              // (multiples of four: columns, sums, and where the sums begin)
+          if (c < n_out && k >= 0 && k < k_sums) {
+            const float4 x4 = *reinterpret_cast<const float4*>(s_rows + r * pitch + k);
+            e[0] = x4.x; e[1] = x4.y; e[2] = x4.z; e[3] = x4.w;
           }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (c + q < n_out && k + q >= 0 && k + q < k_sums) e[q] = s_rows[r * pitch + k + q];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[4 * u + q] = __float_as_uint(e[q]);
+        if (sel.p.vec_in) {
+          if (c < n_out) *reinterpret_cast<float4*>(row + c) = make_float4(e[0], e[1], e[2], e[3]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (c + q < n_out) row[c + q] = e[q];
         }
       }
-      const int here = kl0;
-      if (kl0 + kAhead * kTeam < n_out) fetch(kl0 + kAhead * kTeam);
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int kl = here + u * kTeam, k = cur + kl - nlo * gpt, t = k >= 0 && k < k_end ? k / gpt : -1;
-        if (kl < n_out && ((t >= t0 && t < t1) || (t0 == 0 && t < 0))) out[kl] = acc[u];
-      }
+      select_values<kVec>(v, sel.p, sel.thr_per_head, sel.mask, sel.idx, sel.cnt, w, lane);
     }
-  }
-  if constexpr (kVec > 0) {
-    sync();
-    if (tid < 32) select_row<kVec>(sums, sel.p, sel.thr_per_head, sel.mask, sel.idx, sel.cnt, bh * g.qb_total + qb, threadIdx.x & 31);
   }
 }
 
@@ -1522,13 +1584,14 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // Block sums finished there can be selected on there, too: rows of up to 128 stored sums (four per lane), in clusters of four, or
   // where a CTA has tiles enough that the selection on one runs under the next.  Clusters of two do not gain: a CTA has the rows of
   // eight query blocks at stride 16, two rounds for its six warps (2100 tokens 35.4 us a call with it, 35.2 without).  Otherwise
-  // est_blocksum_kernel selects, rows of up to 512.
+  // est_blocksum_kernel selects, rows of up to 512 whose tile fits its shared memory.
   EstSelect sel;
   bool selecting = false;
   if (select) {
     const SelCall& c = *select;
     const int cols = g.band ? g.bpc : g.kb_total;
-    const bool here = direct ? !use_pairs && can_select(g.tile_n / 128, f32) && (g.split == 4 || (g.split == 1 && many)) && cols <= 128 : cols <= 512;
+    const bool here = direct ? !use_pairs && can_select(g.tile_n / 128, f32) && (g.split == 4 || (g.split == 1 && many)) && cols <= 128
+                             : cols <= 512 && static_cast<size_t>(kTileM / g.rbs) * (g.m_pitch * (g.tile_n / g.rbs) + 8) * sizeof(float) <= kSumSmem;
     if (here && c.k_blocks <= 1024 && c.attn_sums == attn_sums && c.batch == batch && c.heads == hq && c.q_blocks == g.qb_total &&
         c.k_blocks == g.kb_total && c.bpc == g.bpc && (c.band ? 1 : 0) == g.band) {
       if ((rc = select_params(c, sel.p))) return rc;
@@ -1685,28 +1748,30 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   if (rc) return rc;
   }
 
-  // A warp per query block where that fills the chip (32 warps per SM; 2528 query blocks: the estimate 58.6 us by one warp each, 57.5
-  // by four), otherwise four.  32 KiB of factors per CTA at most.
-  const long long items = static_cast<long long>(batch) * hq * g.qb_total;
-  const bool wide = items < 32LL * sm_count();
-  const int teams = wide ? 1 : kSumThreads / 32, seg_max = 32 * 1024 / (4 * g.rbs * teams);
-  const int seg_tiles = g.m_pitch < seg_max ? g.m_pitch : seg_max;
-  auto launch_sums = [&](auto kern, auto what) -> int {
-    return launch_dependent(kern, dim3(static_cast<unsigned>((items + teams - 1) / teams)), dim3(kSumThreads),
-                            static_cast<size_t>(teams) * seg_tiles * g.rbs * sizeof(float), stream, g, (const int*)tile_lo,
-                            (const int*)tile_prefix, (const float*)partial, (const float2*)mtile, attn_sums, seg_tiles, what);
+  const int gpt = g.tile_n / g.rbs, pitch = g.m_pitch * gpt + 8;        // (rows of sums in different banks)
+  const unsigned sum_ctas = static_cast<unsigned>(batch) * hq * g.n_mtiles;
+  // A row tile's key blocks over as many CTAs as it takes for two per SM (1024 tokens against 70000, 32 row tiles: 16 us by one CTA
+  // each, 7.0 by eight); not where they are selected on, for which all of them have to be in one.
+  unsigned parts = selecting ? 1u : 2u * sm_count() / sum_ctas;
+  parts = parts < 1 ? 1 : (parts > 8 ? 8 : parts);
+  auto launch_sums = [&](auto kern, int threads, auto what) -> int {
+    const size_t smem = selecting ? static_cast<size_t>(kTileM / g.rbs) * pitch * sizeof(float) : 0;
+    if (smem > 24 * 1024 && !allow_smem(kern, kSumSmem)) return XATTN_B200_ERR_CUDA;
+    return launch_dependent(kern, dim3(static_cast<unsigned>(batch) * hq, g.n_mtiles, parts), dim3(threads), smem, stream, g, (const int*)tile_lo,
+                            (const int*)tile_prefix, (const float*)partial, (const float2*)mtile, attn_sums, pitch, what);
   };
   // with the selection: the instantiation with just enough registers for a row of sums
-  auto launch_vec = [&](auto rbs, auto team) -> int {
-    constexpr int kRbs = decltype(rbs)::value, kTeam = decltype(team)::value;
+  auto launch_vec = [&](auto rbs, auto warps) -> int {
+    constexpr int kRbs = decltype(rbs)::value, kWarps = decltype(warps)::value;
     const int cols = g.band ? g.bpc : g.kb_total;
-    if (!selecting) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 0>, EstNothing());
-    if (cols <= 128) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 1>, sel);
-    if (cols <= 256) return launch_sums(est_blocksum_kernel<kRbs, kTeam, 2>, sel);
-    return launch_sums(est_blocksum_kernel<kRbs, kTeam, 4>, sel);
+    if (!selecting) return launch_sums(est_blocksum_kernel<kRbs, 0, kWarps>, 32 * kWarps, EstNothing());
+    if (cols <= 128) return launch_sums(est_blocksum_kernel<kRbs, 1, kWarps>, 32 * kWarps, sel);
+    if (cols <= 256) return launch_sums(est_blocksum_kernel<kRbs, 2, kWarps>, 32 * kWarps, sel);
+    return launch_sums(est_blocksum_kernel<kRbs, 4, kWarps>, 32 * kWarps, sel);
   };
+  // sixteen warps where that leaves no more than two CTAs per SM, otherwise eight
   auto launch_team = [&](auto rbs) -> int {
-    return wide ? launch_vec(rbs, std::integral_constant<int, 128>()) : launch_vec(rbs, std::integral_constant<int, 32>());
+    return sum_ctas <= 2u * sm_count() ? launch_vec(rbs, std::integral_constant<int, 16>()) : launch_vec(rbs, std::integral_constant<int, 8>());
   };
   switch (g.rbs) {
     case 4: return launch_team(std::integral_constant<int, 4>());

@@ -108,10 +108,10 @@ __device__ __forceinline__ void finish_row(const SelParams& p, int R, int cur, u
 }
 
 // Row w of the call by one warp: rows of up to 128 * kVec stored scores and up to 1024 key blocks, in registers; lane l holds
-// the columns 128 u + 4 l + e of the stored part (u < kVec, e < 4).
+// the columns 128 u + 4 l + e of the stored part (u < kVec, e < 4), zeros past its end.
 template <int kVec>
-__device__ __forceinline__ void select_row(const float* sums, const SelParams& p, const float* thr_per_head, uint8_t* mask_out,
-                                           int32_t* idx_out, int32_t* cnt_out, int w, int lane) {
+__device__ __forceinline__ void select_values(uint32_t (&v)[4 * kVec], const SelParams& p, const float* thr_per_head, uint8_t* mask_out,
+                                              int32_t* idx_out, int32_t* cnt_out, int w, int lane) {
   constexpr unsigned kAll = 0xffffffffu;
   const int bh = w / p.q_blocks;
   const int R = w - bh * p.q_blocks;
@@ -123,30 +123,8 @@ __device__ __forceinline__ void select_row(const float* sums, const SelParams& p
   const bool lag = n_forced == 1;
   const int n_read = p.band ? p.bpc : N;
   const int col0 = p.band ? cur : 0;
-  const float* x = sums + static_cast<size_t>(w) * n_read;
   const double thr = thr_per_head ? static_cast<double>(ld_written(thr_per_head + bh % p.heads)) : p.threshold;
 
-  // The row may be what this warp, or its CTA, has just stored: it is behind a barrier of theirs, and the compiler, which does not know
-  // what the loads read, keeps the stores in front of them.
-  asm volatile("" ::: "memory");
-  // ---- the row, once; scores as bit patterns (positive floats order like integers), forced and non-positive ones as 0
-  uint32_t v[4 * kVec];
-#pragma unroll
-  for (int u = 0; u < kVec; ++u) {
-    const int j = u * 128 + 4 * lane;
-    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.vec_in) {
-      const float4 in = ld_written(reinterpret_cast<const float4*>(x + (j < n_read ? j : 0)));      // (no branch per load)
-      if (j < n_read) q = in;
-    } else {
-      if (j < n_read) q.x = ld_written(x + j);
-      if (j + 1 < n_read) q.y = ld_written(x + j + 1);
-      if (j + 2 < n_read) q.z = ld_written(x + j + 2);
-      if (j + 3 < n_read) q.w = ld_written(x + j + 3);
-    }
-    v[4 * u] = __float_as_uint(q.x); v[4 * u + 1] = __float_as_uint(q.y);
-    v[4 * u + 2] = __float_as_uint(q.z); v[4 * u + 3] = __float_as_uint(q.w);
-  }
   // What the estimate returns is the scores in the inputs' type: written here, where the row is in registers anyway (a kernel of
   // its own read the sums once more: estimate and mask of 1003 tokens 25.0 -> 16.8 us, of 8192 49.4 -> 46.6, of 32768 119.2 ->
   // 114.8, of 131072 531 -> 515).
@@ -170,6 +148,7 @@ __device__ __forceinline__ void select_row(const float* sums, const SelParams& p
       }
     }
   }
+  // positive floats order like integers; forced and non-positive ones as 0
   double part = 0.0, fpart = 0.0;
   int m = 0;
 #pragma unroll
@@ -354,6 +333,36 @@ __device__ __forceinline__ void select_row(const float* sums, const SelParams& p
     o.cnt = cnt_out + row;
   }
   finish_row(p, R, cur, word, lane, o);
+}
+
+// The same for a row in memory.
+template <int kVec>
+__device__ __forceinline__ void select_row(const float* sums, const SelParams& p, const float* thr_per_head, uint8_t* mask_out,
+                                           int32_t* idx_out, int32_t* cnt_out, int w, int lane) {
+  const int n_read = p.band ? p.bpc : p.k_blocks;
+  const float* x = sums + static_cast<size_t>(w) * n_read;
+  // The row may be what this warp, or its CTA, has just stored: it is behind a barrier of theirs, and the compiler, which does not know
+  // what the loads read, keeps the stores in front of them.
+  asm volatile("" ::: "memory");
+  // ---- the row, once; scores as bit patterns
+  uint32_t v[4 * kVec];
+#pragma unroll
+  for (int u = 0; u < kVec; ++u) {
+    const int j = u * 128 + 4 * lane;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.vec_in) {
+      const float4 in = ld_written(reinterpret_cast<const float4*>(x + (j < n_read ? j : 0)));      // (no branch per load)
+      if (j < n_read) q = in;
+    } else {
+      if (j < n_read) q.x = ld_written(x + j);
+      if (j + 1 < n_read) q.y = ld_written(x + j + 1);
+      if (j + 2 < n_read) q.z = ld_written(x + j + 2);
+      if (j + 3 < n_read) q.w = ld_written(x + j + 3);
+    }
+    v[4 * u] = __float_as_uint(q.x); v[4 * u + 1] = __float_as_uint(q.y);
+    v[4 * u + 2] = __float_as_uint(q.z); v[4 * u + 3] = __float_as_uint(q.w);
+  }
+  select_values<kVec>(v, p, thr_per_head, mask_out, idx_out, cnt_out, w, lane);
 }
 
 // By a whole CTA, where sums were never finished (a device wait ran out): query blocks [qb0, qb0 + n) of a head select and list
