@@ -845,24 +845,31 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
 attn_order_kernel(const AttnParams p, const int32_t* __restrict__ block_cnt, int sms, int32_t* __restrict__ sorted) {
   __shared__ int hist[kOrderBuckets];
   __shared__ int warp_sum[kOrderThreads / 32];
-  __shared__ unsigned long long s_blocks;
+  __shared__ unsigned long long s_blocks[kOrderThreads / 32];
   __shared__ int s_long[3];           // very long units: of all heads, of the heads before this one, of this one
   pdl_launch_dependents();            // the attention kernel may take its place; it waits for this grid to end
   pdl_wait();
   const int tid = threadIdx.x;
   const int n_seg = static_cast<int>(p.by_units.d);                      // units of a (batch, kv head)
   const int n_heads = gridDim.x, first = blockIdx.x * n_seg;
-  if (tid == 0) s_blocks = 0;
   if (tid < 3) s_long[tid] = 0;
   for (int i = tid; i < kOrderBuckets; i += kOrderThreads) hist[i] = 0;
   __syncthreads();
   // blocks listed by the whole call; a unit with more than an eighth of one SM's share of them is a very long one
   const int rows = p.batch * p.hq * p.q_blocks;
   unsigned long long sum = 0;
+#pragma unroll 4
   for (int i = tid; i < rows; i += kOrderThreads) sum += static_cast<unsigned>(ld_written(block_cnt + i));
-  atomicAdd(&s_blocks, sum);
+  // (Warp by warp: an atomic addition of 64 bits in shared memory is a loop, and with all threads' going to one word this kernel took
+  // 47 us for 24 heads of 250 query blocks and 62 for 930; now 7 and 15.)
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((tid & 31) == 0) s_blocks[tid >> 5] = sum;
   __syncthreads();
-  unsigned long long lim64 = s_blocks / (8ull * sms);
+  sum = 0;
+#pragma unroll
+  for (int w = 0; w < kOrderThreads / 32; ++w) sum += s_blocks[w];
+  unsigned long long lim64 = sum / (8ull * sms);
   const int limit = lim64 < 64 ? 64 : (lim64 > kOrderBuckets - 2 ? kOrderBuckets - 2 : static_cast<int>(lim64));
   auto length = [&](int u) {
     const Tile t0 = unit_tile<false>(p, u, 0), t1 = unit_tile<false>(p, u, 1);
