@@ -135,6 +135,33 @@ def test_calls_in_a_row_without_a_pause():
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("dtype,out_dtype", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("hq,hkv,lq,lk", [(2, 1, 70 * 128, 70 * 128), (7, 7, 300, 8400), (4, 2, 1, 9000), (1, 1, 127, 128 * 70 + 1), (74, 37, 256, 8193)])
+def test_tiles_whose_streams_share_a_list(hq, hkv, lq, lk, dtype, out_dtype):
+    """Few tiles: of none, one, an odd and an even number of blocks, of more than a window of a list; several tiles per CTA with
+    the lists of the first ones the longest (dense), rows whose blocks are hidden from one stream altogether."""
+    from xattn_b200 import ops
+    q, k, v = _qkv(lq + hq, 1, hq, hkv, lq, lk, dtype)
+    qb, kb = (lq + 127) // 128, (lk + 127) // 128
+    g = torch.Generator().manual_seed(lk)
+    want_n = torch.randint(0, 6, (1, hq, qb, 1), generator=g)
+    want_n[:, :, ::3] = kb
+    mask = torch.rand(1, hq, qb, kb, generator=g).argsort(-1).argsort(-1) < want_n
+    rep = hq // hkv
+    qf, kf, vf = (x.to(torch.bfloat16).float() if dtype == torch.float32 else x.float() for x in (q, k, v))
+    kf, vf = kf.repeat_interleave(rep, 1), vf.repeat_interleave(rep, 1)
+    visible = torch.ones(lq, lk, dtype=torch.bool).tril(lk - lq)
+    idx, cnt = ops.mask_to_lists(mask.to(DEV), lq, lk, True)
+    for lists in (True, False):
+        out = ops.block_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), idx if lists else None, cnt if lists else None, True)
+        assert out.dtype == out_dtype
+        for h in range(0, hq, max(1, hq // 4)):
+            keep = visible & mask[0, h].repeat_interleave(128, 0)[:lq].repeat_interleave(128, 1)[:, :lk] if lists else visible
+            s = (qf[0, h] @ kf[0, h].T * 128 ** -0.5).masked_fill(~keep, float("-inf"))
+            want = torch.where(keep.any(1, keepdim=True), torch.softmax(s, -1).nan_to_num(0.0) @ vf[0, h], torch.zeros(()))
+            _close(out[0, h], want)
+
+
 @pytest.mark.parametrize("count", [2 ** 30, -5, 4])
 def test_counts_beyond_a_row_of_the_lists(count):
     """A count that no list can have is cut to the row of the lists (three blocks here), or to none."""

@@ -6,7 +6,8 @@
 // same kv head: two query heads of a kv group, or two neighbouring query blocks of one head.  The grid has a CTA per
 // unit, of which one per SM runs at a time and takes over further ones (cluster launch control).  Its two tiles are two
 // streams: each has its own Q tile in shared memory, its own score/probability buffer S and output accumulator O in
-// tensor memory and its own softmax warpgroup, so that one stream's softmax runs under the other's MMAs.  (Only the pass over
+// tensor memory and its own softmax warpgroup, so that one stream's softmax runs under the other's MMAs.  (Calls of few tiles: a
+// unit is a single tile, of whose list each stream walks every other block, and the epilogue adds the two parts of O.  Only the pass over
 // what the pair kernel leaves, whose length the host does not know, takes its units in strides of the grid instead.)
 //
 //   warps 0-3   softmax of stream 0  } one thread per query row.  A block's 128 scores leave TMEM once and stay in
@@ -78,10 +79,14 @@ __device__ __forceinline__ size_t tile_row(const AttnParams& p, const Tile& t) {
 // are, for each kv head, the pairs of query heads at hi, then those at hi-1, and for an odd group first one unit that takes
 // the last head at hi and hi-1.  Causal: super row by super row, the heaviest (last) first.  Non-causal: kv head by kv
 // head, so that the CTAs work on one head's K and V at a time.
-template <bool kList>
+// kSplit: unit u is the tile of that number in a tile list, both streams'.
+template <bool kList, bool kSplit = false>
 __device__ __forceinline__ Tile unit_tile(const AttnParams& p, int u, int s) {
   Tile t;
-  if (kList && p.tile_list) {
+  if constexpr (kSplit) {
+    const int rest = fast_div(u, p.by_hq, t.h);
+    t.qb = p.q_blocks - 1 - fast_div(rest, p.by_batch, t.b);
+  } else if (kList && p.tile_list) {
     t.b = t.h = 0;
     t.qb = -1;
     const int i = 2 * u + s < p.list_tiles ? ld_written(p.tile_list + 2 * u + s) : -1;
@@ -114,24 +119,30 @@ __device__ __forceinline__ int tile_count(const AttnParams& p, const int32_t* __
   const int n = last / 128 + 1;
   return n < p.list_k_blocks ? n : p.list_k_blocks;
 }
-// A tile's list as its walkers see it: walk position j maps to list[n - 1 - j].
+// Blocks of a tile of n that stream s walks (n < 0: no more units): all of them, or, split between the streams, every other one.
+template <bool kSplit>
+__device__ __forceinline__ int share(int n, int s) { return kSplit && n > 0 ? (n + 1 - s) >> 1 : n; }
+// A tile's list as its walkers see it: walk position j maps to list[n - 1 - j] (split: list[n - 1 - s - 2 j]).
 struct List {
-  const int32_t* last;     // its last entry; null in a dense call
-  int n;
+  const int32_t* last;     // the first entry walked; null in a dense call
+  int n, top;              // entries to walk; (split) place of the first one
 };
-__device__ __forceinline__ List tile_list(const AttnParams& p, const int32_t* __restrict__ block_idx, const Tile& t, int n) {
+template <bool kSplit>
+__device__ __forceinline__ List tile_list(const AttnParams& p, const int32_t* __restrict__ block_idx, const Tile& t, int n, int s) {
   List l;
-  l.last = block_idx ? block_idx + tile_row(p, t) * p.list_k_blocks + (n - 1) : nullptr;
-  l.n = n;
+  l.top = kSplit ? n - 1 - s : 0;
+  l.last = block_idx ? block_idx + tile_row(p, t) * p.list_k_blocks + (kSplit ? l.top : n - 1) : nullptr;
+  l.n = share<kSplit>(n, s);
   return l;
 }
 // entry j of the list, walking order
+template <bool kSplit>
 __device__ __forceinline__ int list_entry(const List& l, int j) {
   if (j >= l.n) return 0;
-  if (!l.last) return l.n - 1 - j;
+  if (!l.last) return kSplit ? l.top - 2 * j : l.n - 1 - j;
   // (its volatile asm also pins the issue point: a plain load would be sunk by the compiler to its first use, which turns
   // the intended prefetch into an exposed memory latency)
-  return ld_written(l.last - j);
+  return ld_written(l.last - (kSplit ? 2 * j : j));
 }
 
 // Reader of the published units.
@@ -160,7 +171,8 @@ struct Units {
 // kBf16: bf16 or fp16 (a template parameter: as a run-time switch every packed pair cost both conversions and a select).
 // kOutF32: the output is written as fp32.  kList: the units may come from a list.
 // kTwo: a CTA takes two units next to one another at a time (the causal numbering, no list of units), see the loader.
-template <bool kBf16, bool kOutF32, bool kList, bool kTwo>
+// kSplit: a unit is a single tile, of whose list each stream walks every other block; the epilogue puts the two together.
+template <bool kBf16, bool kOutF32, bool kList, bool kTwo, bool kSplit>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -283,7 +295,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           clc_try_cancel(smem_u32(answer), answer_full);
         }
         __syncwarp();
-        int wx = list_entry(l, 16 + wl);
+        int wx = list_entry<kSplit>(l, 16 + wl);
         bool fetched = false;
 #pragma unroll 1
         while (true) {
@@ -325,7 +337,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
             ++step;
             if (f && (++i & 15) == 0) {
               w = wx;
-              wx = list_entry(l, i + 16 + wl);
+              wx = list_entry<kSplit>(l, i + 16 + wl);
             }
             __syncwarp();
           } else if (fetched) {
@@ -350,14 +362,16 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
               }
               fence_proxy_async_smem();                 // read before the next answer is written
             }
+            int count = -1;                             // of the tile's blocks (split: of both streams)
             ln.n = -1;
             if (unit >= 0) {
-              tn = unit_tile<kList>(p, unit, s);
-              ln = tile_list(p, block_idx, tn, tile_count(p, block_cnt, tn));
-              wn = list_entry(ln, wl);
+              tn = unit_tile<kList, kSplit>(p, unit, s);
+              count = tile_count(p, block_cnt, tn);
+              ln = tile_list<kSplit>(p, block_idx, tn, count, s);
+              wn = list_entry<kSplit>(ln, wl);
             }
             if (!wait(unit_empty + 8 * (k % kUnitSlots), (k / kUnitSlots & 1) ^ 1)) { ok = false; break; }
-            if (wl == 0) reinterpret_cast<int4*>(unit_ring)[2 * (k % kUnitSlots) + s] = make_int4(tn.b, tn.h, tn.qb, ln.n);
+            if (wl == 0) reinterpret_cast<int4*>(unit_ring)[2 * (k % kUnitSlots) + s] = make_int4(tn.b, tn.h, tn.qb, count);
             __syncwarp();
             if (lane == 0) mbar_arrive(unit_full + 8 * (k % kUnitSlots));
           }
@@ -383,13 +397,13 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         // done: both tiles of the unit are first pulled into L2, so that the loads do not wait on HBM
         if (lane == 0) {
           if (t0.n > 0) tma_prefetch_l2_5d(&tmQ, 0, t0.qb * 128, 0, t0.h, t0.b);
-          if (t1.n > 0) tma_prefetch_l2_5d(&tmQ, 0, t1.qb * 128, 0, t1.h, t1.b);
+          if (!kSplit && t1.n > 0) tma_prefetch_l2_5d(&tmQ, 0, t1.qb * 128, 0, t1.h, t1.b);
         }
         __syncwarp();
 #pragma unroll 1
         for (int s = 0; s < 2; ++s) {
           const UnitTile t = s ? t1 : t0;
-          if (t.n == 0) continue;
+          if (share<kSplit>(t.n, s) == 0) continue;
           if (!__all_sync(0xffffffffu, mbar_wait(bar(s, Q_EMPTY), (m >> s & 1) ^ 1, abort_flag))) { ok = false; break; }
           if (lane == 0) {
             XB_TRACE_EV(0x10 + s, m);
@@ -533,7 +547,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     auto list_of = [&](const UnitTile& ut) -> List {
       Tile tt;
       tt.b = ut.b; tt.h = ut.h; tt.qb = ut.qb;
-      return tile_list(p, block_idx, tt, ut.n);
+      return tile_list<kSplit>(p, block_idx, tt, ut.n, s);
     };
     auto fetch = [&]() {
       if (!units.wait()) {
@@ -542,13 +556,13 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       }
       nt = units.tile(s);
       units.release(lane);
-      if (nt.n > 0) nwin = list_entry(list_of(nt), lane);
+      if (nt.n > 0) nwin = list_entry<kSplit>(list_of(nt), lane);
     };
     int m = 0;
     nt.n = 0;
 #pragma unroll 1
     while (ok && nt.n >= 0) {
-      if (nt.n == 0) {                                  // (at the start, too)
+      if (share<kSplit>(nt.n, s) == 0) {                // (at the start, too)
         fetch();
         continue;
       }
@@ -562,12 +576,12 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       int row_last_lo = p.k_len - 1;                    // the same for the first row of the warp
       if (p.causal && t.qb * 128 + quad * 32 + k_off < row_last_lo) row_last_lo = t.qb * 128 + quad * 32 + k_off;
       float m_used = -INFINITY, l = 0.f;
-      int w = nwin, w_next = list_entry(list, 32 + lane);
+      int w = nwin, w_next = list_entry<kSplit>(list, 32 + lane);
 #pragma unroll 1
       for (int j = 0; j < n; ++j, ++bc) {
         if (j > 0 && (j & 31) == 0) {
           w = w_next;
-          w_next = list_entry(list, j + 32 + lane);
+          w_next = list_entry<kSplit>(list, j + 32 + lane);
         }
         const int k0 = __shfl_sync(0xffffffffu, w, j & 31) * 128;
         if (lane == 0) XB_TRACE_EV(0x30, bc);
@@ -691,7 +705,16 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           unpack_f32x2(add_f32x2(add_f32x2(ls2[0], ls2[1]), add_f32x2(ls2[2], ls2[3])), a0, a1);
           l += a0 + a1;
         }
-        if (j == n - 1) s_l[(s * 2 + (m & 1)) * 128 + r] = l;   // read by the epilogue once this tile's last P.V is done
+        if (j == n - 1) {                               // read by the epilogue once this tile's last P.V is done
+          if constexpr (kSplit) {
+            // (the epilogue may still be waiting for the other stream's part of the tile before)
+            if (!__all_sync(0xffffffffu, mbar_wait(bar(s, O_EMPTY), (m & 1) ^ 1, abort_flag))) { ok = false; break; }
+            s_l[s * 2 * 128 + r] = l;
+            s_l[(s * 2 + 1) * 128 + r] = m_used;
+          } else {
+            s_l[(s * 2 + (m & 1)) * 128 + r] = l;
+          }
+        }
         half_ready(1);
         if (j == 0) fetch();
         if (lane == 0) XB_TRACE_EV(0x33, bc);
@@ -714,7 +737,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     UnitTile t1;
 #pragma unroll 1
     for (int i = 0; ok; ++i) {
-      const int s = i & 1;
+      const int s = kSplit ? 0 : i & 1;
       UnitTile t = t1;
       if (s == 0) {
         if (!units.wait()) break;
@@ -725,8 +748,25 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       const int n = t.n;
       if (n < 0) break;
       if (t.qb < 0) continue;
-      float inv = 0.f;
-      if (n > 0) {
+      float inv = 0.f, inv1 = 0.f;                      // what O is multiplied with; split: and the other stream's
+      if constexpr (kSplit) {
+#pragma unroll 1
+        for (int x = 0; x < 2 && x < n && ok; ++x) {
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(x, O_FULL), (done >> x) & 1, abort_flag));
+          done ^= 1u << x;
+        }
+        if (!ok) break;
+        tc_fence_after();
+        if (n > 0) {
+          // the two halves of the row against the larger of their maxima
+          const float l0 = s_l[r], m0 = s_l[128 + r], l1 = n > 1 ? s_l[2 * 128 + r] : 0.f, m1 = n > 1 ? s_l[3 * 128 + r] : -INFINITY;
+          const float top = fmaxf(m0, m1);
+          const float a0 = m0 == -INFINITY ? 0.f : fast_exp2(m0 - top), a1 = m1 == -INFINITY ? 0.f : fast_exp2(m1 - top);
+          const float sum = l0 * a0 + l1 * a1, over = sum > 0.f ? 1.f / sum : 0.f;
+          inv = a0 * over;
+          inv1 = a1 * over;
+        }
+      } else if (n > 0) {
         const uint32_t m = (done >> s) & 1;
         done ^= 1u << s;
         if (threadIdx.x == 256) XB_TRACE_EV(0x40 + s, m);
@@ -737,6 +777,32 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         inv = l > 0.f ? 1.f / l : 0.f;
       }
       const uint32_t tmem_o = tmem_base + 256 + s * 128 + lane_bits;
+      // 32 columns of O from `c` on, scaled (split: the two streams' parts added), as words
+      auto load_out = [&](int c, uint32_t (&v)[32]) {
+        tmem_ld32(tmem_o + c, v);
+        tc_wait_ld();
+#pragma unroll
+        for (int k = 0; k < 32; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * inv);
+        if constexpr (kSplit) {
+          if (n > 1) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              uint32_t y[16];
+              tmem_ld16(tmem_o + 128 + c + 16 * h, y);
+              tc_wait_ld();
+#pragma unroll
+              for (int k = 0; k < 16; ++k) v[16 * h + k] = __float_as_uint(__uint_as_float(v[16 * h + k]) + __uint_as_float(y[k]) * inv1);
+            }
+          }
+        }
+      };
+      auto o_read = [&]() {
+        if (n > 0) {
+          tc_fence_before();
+          mbar_arrive(bar(s, O_EMPTY));
+          if (kSplit && n > 1) mbar_arrive(bar(1, O_EMPTY));
+        }
+      };
       if constexpr (kOutF32) {
         const int q_row0 = t.qb * 128 + quad * 32;      // first row of this warp
         // 32 columns at a time through the two halves of the staging tile in turn
@@ -744,10 +810,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         for (int c = 0; c < 4; ++c) {
           uint32_t v[32];
           if (n > 0) {
-            tmem_ld32(tmem_o + c * 32, v);
-            tc_wait_ld();
-#pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * inv);
+            load_out(c * 32, v);
           } else {                                      // an empty list: zeros
 #pragma unroll
             for (int k = 0; k < 32; ++k) v[k] = 0u;
@@ -766,10 +829,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
             tma_store_commit();
           }
         }
-        if (n > 0) {
-          tc_fence_before();
-          mbar_arrive(bar(s, O_EMPTY));
-        }
+        o_read();
       } else {
         if (lane == 0) tma_store_wait_read();           // the staging tile's previous stores have read it
         __syncwarp();
@@ -778,11 +838,9 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           uint32_t pk[16];
           if (n > 0) {
             uint32_t v[32];
-            tmem_ld32(tmem_o + c * 32, v);
-            tc_wait_ld();
+            load_out(c * 32, v);
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
-              pk[k] = pack16t<kBf16>(__uint_as_float(v[2 * k]) * inv, __uint_as_float(v[2 * k + 1]) * inv);
+            for (int k = 0; k < 16; ++k) pk[k] = pack16t<kBf16>(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
           } else {                                      // an empty list: zeros
 #pragma unroll
             for (int k = 0; k < 16; ++k) pk[k] = 0u;
@@ -793,10 +851,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
             *reinterpret_cast<uint4*>(row + (((((c & 1) << 2) | q4) ^ (lane & 7)) << 4)) =
                 make_uint4(pk[4 * q4], pk[4 * q4 + 1], pk[4 * q4 + 2], pk[4 * q4 + 3]);
         }
-        if (n > 0) {
-          tc_fence_before();
-          mbar_arrive(bar(s, O_EMPTY));
-        }
+        o_read();
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
@@ -1026,20 +1081,30 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
   // stays out of the other calls: it cost dense ones 1 %.
   const bool two = causal && !dense && !rest && max_list > 0 && units >= 24 * sms && units >= max_list * sms &&
                    static_cast<long long>(batch) * hkv * p.list_k_blocks < 0x7fffffffLL;
-  const unsigned grid = static_cast<unsigned>(rest && units > sms ? sms : (two ? (units + 1) / 2 : units));
+  const long long tiles = static_cast<long long>(p.q_blocks) * batch * hq;
+  // Causal calls of few tiles give each a CTA of its own, whose streams share its list.  With lists, up to a tile per SM, and of more
+  // than 64 key blocks, where the lists may be long (us, two tiles per CTA and like this: 512 tokens against 30000, 75 blocks per row,
+  // 192 and 114, against 60000, 174 blocks, 372 and 230; against 300, two blocks, 12.1 and 12.1; with more tiles, where CTAs then take
+  // two, the chains of short lists come one after the other: 1024 tokens against 70000, three blocks, 13.0 and 15.5).  Dense ones up to
+  // two per SM (512 tokens 12.9 and 11.9, 1003 tokens 19.8 and 19.1, 1180 tokens of 28 heads 22.3 and 22.1).
+  const bool split = causal && !rest && (dense ? tiles <= 2 * sms : tiles <= sms && p.list_k_blocks > 64);
+  const unsigned grid = static_cast<unsigned>(rest && units > sms ? sms : (two ? (units + 1) / 2 : (split ? tiles : units)));
   auto launch = [&](auto kern) -> int {
     if (!allow_smem(kern, kAttnSmem))
       return XATTN_B200_ERR_CUDA;
     return launch_dependent(kern, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tmQ, tmK,
                             tmV, tmO, p, block_idx, block_cnt, rest, pair_header, min_share, status);
   };
-  auto launch_type = [&](auto list, auto pairs) -> int {
-    constexpr bool kList = decltype(list)::value, kTwo = decltype(pairs)::value;
-    return out_f32 ? launch(block_sparse_attn_kernel<true, true, kList, kTwo>)
-                   : (p.is_bf16 ? launch(block_sparse_attn_kernel<true, false, kList, kTwo>) : launch(block_sparse_attn_kernel<false, false, kList, kTwo>));
+  auto launch_type = [&](auto list, auto pairs, auto parts) -> int {
+    constexpr bool kList = decltype(list)::value, kTwo = decltype(pairs)::value, kSplit = decltype(parts)::value;
+    return out_f32 ? launch(block_sparse_attn_kernel<true, true, kList, kTwo, kSplit>)
+                   : (p.is_bf16 ? launch(block_sparse_attn_kernel<true, false, kList, kTwo, kSplit>) : launch(block_sparse_attn_kernel<false, false, kList, kTwo, kSplit>));
   };
-  if (p.tile_list || rest) return launch_type(std::true_type(), std::false_type());
-  return two ? launch_type(std::false_type(), std::true_type()) : launch_type(std::false_type(), std::false_type());
+  const auto yes = std::true_type();
+  const auto no = std::false_type();
+  if (p.tile_list || rest) return launch_type(yes, no, no);
+  if (two) return launch_type(no, yes, no);
+  return split ? launch_type(no, no, yes) : launch_type(no, no, no);
 }
 
 }  // namespace xb
