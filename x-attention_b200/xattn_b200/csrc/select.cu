@@ -482,6 +482,9 @@ int select_params(const SelCall& c, SelParams& p) {
   const long long rows = static_cast<long long>(c.batch) * c.heads * c.q_blocks;
   if (rows > 0x7fffffffLL) return XATTN_B200_ERR_LIMIT;
   p.rows_total = static_cast<int>(rows);
+  p.by_q_blocks = make_fast_div(c.q_blocks);
+  p.by_heads = make_fast_div(c.heads);
+  p.by_bpc = make_fast_div(c.bpc);
   return XATTN_B200_OK;
 }
 

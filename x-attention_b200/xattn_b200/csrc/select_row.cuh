@@ -37,6 +37,7 @@ struct SelParams {
   int band;           // score rows hold only the chunk's own key blocks [cur, cur + bpc)
   void* rounded;      // (rows in registers) the scores rounded to bf16 / fp16, same layout; null: not wanted
   int rounded_bf16;
+  FastDiv by_q_blocks, by_heads, by_bpc;
 };
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -86,8 +87,7 @@ __device__ __forceinline__ void finish_row(const SelParams& p, int R, int cur, u
       // last token of query block R sees keys up to this position (query end aligned to key end)
       int last_q = R * 128 + 127;
       if (last_q > p.list_q_len - 1) last_q = p.list_q_len - 1;
-      const long long lim = static_cast<long long>(last_q) + (p.list_k_len - p.list_q_len);
-      const int jm = lim < 0 ? -1 : static_cast<int>(lim / 128);
+      const int jm = (last_q + (p.list_k_len - p.list_q_len)) >> 7;      // (-1 and less: none)
       if (jm < hi_list) hi_list = jm;
     }
     uint32_t lw = word & bits_le(hi_list, lane);
@@ -113,17 +113,18 @@ template <int kVec>
 __device__ __forceinline__ void select_values(uint32_t (&v)[4 * kVec], const SelParams& p, const float* thr_per_head, uint8_t* mask_out,
                                               int32_t* idx_out, int32_t* cnt_out, int w, int lane) {
   constexpr unsigned kAll = 0xffffffffu;
-  const int bh = w / p.q_blocks;
-  const int R = w - bh * p.q_blocks;
+  int R, in_chunk, head;
+  const int bh = fast_div(w, p.by_q_blocks, R);
   const int N = p.k_blocks;
-  const int cur = p.block_offset + (R / p.bpc) * p.bpc;
-  const int d = cur + R % p.bpc;
+  const int cur = p.block_offset + fast_div(R, p.by_bpc, in_chunk) * p.bpc;
+  const int d = cur + in_chunk;
   const bool f0 = p.causal && cur != 0;            // block 0 forced
   const int n_forced = p.causal ? (f0 ? 2 : 1) : 0;
   const bool lag = n_forced == 1;
   const int n_read = p.band ? p.bpc : N;
   const int col0 = p.band ? cur : 0;
-  const double thr = thr_per_head ? static_cast<double>(ld_written(thr_per_head + bh % p.heads)) : p.threshold;
+  fast_div(bh, p.by_heads, head);
+  const double thr = thr_per_head ? static_cast<double>(ld_written(thr_per_head + head)) : p.threshold;
 
   // What the estimate returns is the scores in the inputs' type: written here, where the row is in registers anyway (a kernel of
   // its own read the sums once more: estimate and mask of 1003 tokens 25.0 -> 16.8 us, of 8192 49.4 -> 46.6, of 32768 119.2 ->
@@ -149,7 +150,8 @@ __device__ __forceinline__ void select_values(uint32_t (&v)[4 * kVec], const Sel
     }
   }
   // positive floats order like integers; forced and non-positive ones as 0
-  double part = 0.0, fpart = 0.0;
+  double part = 0.0;
+  uint32_t at_d = 0u, at_0 = 0u;                   // the forced scores, in the lanes that hold them
   int m = 0;
 #pragma unroll
   for (int k = 0; k < 4 * kVec; ++k) {
@@ -157,12 +159,14 @@ __device__ __forceinline__ void select_values(uint32_t (&v)[4 * kVec], const Sel
     const float f = __uint_as_float(v[k]);
     const double df = static_cast<double>(f);
     part += df;
-    const bool forced = p.causal && (jj == d || (f0 && jj == 0));
-    if (forced) fpart += df;
-    if (forced || !(f > 0.f)) v[k] = 0u;
+    const bool is_d = p.causal && jj == d, is_0 = f0 && jj == 0;
+    if (is_d) at_d = v[k];
+    if (is_0) at_0 = v[k];
+    if (is_d || is_0 || !(f > 0.f)) v[k] = 0u;
     m += v[k] != 0u;
   }
-  const double total = warp_sum(part), fsum = warp_sum(fpart);
+  const double total = warp_sum(part), fsum = static_cast<double>(__uint_as_float(__reduce_or_sync(kAll, at_d))) +
+                                            static_cast<double>(__uint_as_float(__reduce_or_sync(kAll, at_0)));
   const int M = __reduce_add_sync(kAll, m);
   const double req = total * thr;
 
