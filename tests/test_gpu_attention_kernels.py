@@ -135,6 +135,26 @@ def test_calls_in_a_row_without_a_pause():
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("blocks,items_per_sm,ordered", [(41, 4, True), (41, 3, False), (40, 4, False), (40, 16, True)])
+def test_which_non_causal_calls_are_ordered(blocks, items_per_sm, ordered):
+    """The units of a call with long lists and a few of them per SM are sorted first: one launch more, the same results."""
+    from xattn_b200 import _lib, ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    heads = -(-items_per_sm * sms // blocks) if ordered or blocks == 40 else items_per_sm * sms // blocks
+    L = blocks * 128 - 5
+    g = torch.Generator(device=DEV).manual_seed(blocks)
+    q, k, v = (torch.randn(1, heads, L, 128, device=DEV, generator=g).bfloat16() for _ in range(3))
+    mask = torch.rand(1, heads, blocks, blocks, device=DEV, generator=g) < 0.1
+    mask[:, :, -2:] = True
+    idx, cnt = ops.mask_to_lists(mask, L, L, False)
+    count = _lib.load().xattn_b200_launch_count
+    n0 = count()
+    got = ops.block_sparse_attention(q, k, v, idx, cnt, False)
+    n1 = count()
+    assert n1 - n0 == (2 if ordered else 1)
+    assert torch.equal(got, ops.block_sparse_attention(q, k, v, idx, cnt, False, use_workspace=False))
+
+
 @pytest.mark.parametrize("dtype,out_dtype", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16), (torch.float32, torch.float32)])
 @pytest.mark.parametrize("hq,hkv,lq,lk", [(2, 1, 70 * 128, 70 * 128), (7, 7, 300, 8400), (4, 2, 1, 9000), (1, 1, 127, 128 * 70 + 1), (74, 37, 256, 8193)])
 def test_tiles_whose_streams_share_a_list(hq, hkv, lq, lk, dtype, out_dtype):

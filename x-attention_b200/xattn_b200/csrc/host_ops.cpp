@@ -344,14 +344,17 @@ Tensor attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Ten
         "block_sparse_attn");
   return out;
 }
-// Non-causal calls: sorting the units by list length is one launch of a few microseconds; with only a few units per SM there
-// is nothing to balance.
-constexpr int64_t kOrderMinItemsPerSm = 16;
-bool default_workspace(bool causal, bool dense, const Tensor& q) {
+// Non-causal calls: sorting the units by list length is one launch of 5 to 15 us.  What it saves is the chain of a long list that would be
+// begun near the end, 1.5 us per block: worth it with many items per SM, or with a few whose lists may be long (24 heads, video
+// diffusion, us without and with it: 7400 tokens, 58 key blocks, 9 items per SM, 257 and 205; 11000 tokens, 14 items, 449 and 373; 12
+// heads of 7400, 5 items, 189 and 170; but 3800 tokens, 30 key blocks, 5 or 10 items, 138 and 142, 177 and 183).
+constexpr int64_t kOrderItemsPerSm = 16, kOrderFewItemsPerSm = 4, kOrderKeys = 40 * 128;
+bool default_workspace(bool causal, bool dense, const Tensor& q, int64_t k_len) {
   if (dense) return false;
   const char* forced = std::getenv("XATTN_B200_ATTN_WORKSPACE");       // "0" / "1": overrides the rule (for measurements)
   if (forced && (forced[0] == '0' || forced[0] == '1') && forced[1] == 0) return forced[0] == '1';
-  return !causal && q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) >= kOrderMinItemsPerSm * at::cuda::getDeviceProperties(q.get_device())->multiProcessorCount;
+  const int64_t per_sm = k_len > kOrderKeys ? kOrderFewItemsPerSm : kOrderItemsPerSm;
+  return !causal && q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) >= per_sm * at::cuda::getDeviceProperties(q.get_device())->multiProcessorCount;
 }
 
 void need_16bit_or_f32(const Tensor& q, const Tensor& k, const char* text) {
@@ -420,7 +423,7 @@ Tensor attention_any(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   const int64_t lqb = (q.size(2) + 127) / 128, lkb = (k.size(2) + 127) / 128;
   if (!dense && (idx.sizes() != at::IntArrayRef({q.size(0), q.size(1), lqb, lkb}) || cnt.sizes() != at::IntArrayRef({q.size(0), q.size(1), lqb})))
     fail(PyExc_ValueError, "block lists have the wrong shape");
-  const bool ws = dense ? false : use_workspace.value_or(default_workspace(causal, dense, q));
+  const bool ws = dense ? false : use_workspace.value_or(default_workspace(causal, dense, q, k.size(2)));
   return attention(q16, k16, v16, dense ? idx : idx.contiguous(), dense ? cnt : cnt.contiguous(), causal, scale, out, f32 && !out.defined(), ws, at_, max_blocks);
 }
 
@@ -521,7 +524,7 @@ PyObject* py_prefill(PyObject*, PyObject* const* pv, Py_ssize_t n) {
     check(xattn_b200_split_f32_terms(static_cast<const float*>(vc.data_ptr()), v.size(0), v.size(1), Lk, Lk, D, vc.stride(0), vc.stride(1),
                                      vc.stride(2), 1, v16.data_ptr(), at_.stream),
           "split_f32_terms");
-    return attention(q16, k16, v16, s.idx, s.cnt, e.causal, scale, out, true, default_workspace(e.causal, false, q), at_, max_blocks);
+    return attention(q16, k16, v16, s.idx, s.cnt, e.causal, scale, out, true, default_workspace(e.causal, false, q, Lk), at_, max_blocks);
   }));
   END_PY
 }

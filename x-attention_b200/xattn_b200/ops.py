@@ -205,7 +205,7 @@ def block_sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bl
     list of one or two blocks to a kernel of their own, provided those rows list at least `pair_split_share()` per cent
     of the blocks, which it finds out on the device; by default (None) no memory is offered.  Non-causal calls: the
     work is sorted by list length before it is handed to the SMs (one small kernel); offered by default from
-    16 items per SM on.  False: the general kernel alone, work in its natural order."""
+    16 items per SM on, with more than 40 key blocks from 4 on.  False: the general kernel alone, work in its natural order."""
     return _host.attention(q, k, v, block_idx, block_cnt, bool(causal), scale, out, use_workspace)
 
 
