@@ -54,11 +54,6 @@ __device__ __forceinline__ void xb_trace(int* status, uint32_t& n, int role, uin
 #define XB_TRACE_EV(tag, val) ((void)0)
 #endif
 
-template <int N, int kLaunchRegs> __device__ __forceinline__ void reg_set_from() {
-  if constexpr (N > kLaunchRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
-  if constexpr (N < kLaunchRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
-}
-
 // [128 bytes of columns, rows, column parts, heads, batch] of rows of 128 elements of `elem` bytes (2 or 4): one box
 // {128 bytes, `rows`, `parts`, 1, 1} moves `rows` rows of `parts` parts with a single TMA instruction, the parts one after
 // the other in shared memory (Q, K, V: both 64-column halves of 16-bit rows).

@@ -44,7 +44,12 @@ constexpr int kF32Smem = 224 * 1024;                         // terms and ring: 
 constexpr int kMaxUnits = 8;
 // Warps that split the units, every warp some rows of each: sixteen, or eight where the epilogue needs the registers.
 __host__ __device__ constexpr int convert_warps(int direct) { return direct ? 8 : 16; }
-__host__ __device__ constexpr int f32_threads(int direct) { return kGemmThreads + 32 * convert_warps(direct); }
+// Where the epilogue needs the registers it is a warpgroup of its own (warps 4-7), which takes over what the loading and issuing warps
+// (0-3) do not need; the converters follow.  (With 128 registers for all it stored 832 to 2750 bytes per thread to local memory, which is
+// L2 here, behind the last product of every tile.  fp32 inputs, 32 heads, estimate and mask, us: 2048 tokens at stride 8 52.2 -> 46.5,
+// 3000 at stride 16 in one chunk 80.0 -> 73.1, 4096 81.3 -> 76.0, 1003 30.8 -> 28.8, 4096 in chunks of 2048 59.7 -> 57.2.)
+__host__ __device__ constexpr bool own_registers(int direct, bool f32) { return f32 && direct > 0; }
+__host__ __device__ constexpr int f32_threads(int direct) { return direct ? 512 : kGemmThreads + 32 * convert_warps(direct); }
 
 // bf16 roundings of fp32 operands, [batch, heads, len, head_dim] contiguous, written on the way (null: not wanted)
 struct EstRounded {
@@ -542,7 +547,7 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int k_steps = g.S * g.d_chunks, ks0 = k_steps * rank / split, ks1 = k_steps * (rank + 1) / split;
   const bool interleave = g.tile_n == 128 && g.hq > g.hkv;      // streaming case only: see decode_tile
 
-  if (warp == 0) {
+  auto load_role = [&]() {
     // ------------------------------------------------------------ TMA producer (converged warp, one thread issues)
     {
       const uint32_t lead = elect_one() ? 1u : 0u;
@@ -586,7 +591,8 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       cluster_sync_all();
       cluster_sync_all();
     }
-  } else if (warp == 1) {
+  };
+  auto mma_role = [&]() {
     // ------------------------------------------------------------ MMA issuer (converged warp, one thread issues: see mma_ss_lead)
     {
       const uint32_t lead = elect_one() ? 1u : 0u;
@@ -637,13 +643,16 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       cluster_sync_all();
       cluster_sync_all();
     }
-  } else if (kF32 && warp >= kGemmThreads / 32) {
+  };
+  constexpr int kFirstConverter = own_registers(kDirect, kF32) ? 8 : kGemmThreads / 32;
+  auto convert_role = [&]() {
+    if constexpr (kF32) {
     // ------------------------------------------------------------ converters (fp32): some rows of each unit per warp
     // A lane takes eight columns (two 16-byte chunks) of one row of each group of eight.  Rows p and p ^ 5 next to one another:
     // neither the fp32 reads (chunks 2 col, 2 col + 1 of a swizzled row) nor the term writes (chunk col of a half) of a
     // quarter-warp then share a bank.
     constexpr int kGroups = kTileM / 8 / convert_warps(kDirect);
-    const int col = lane & 3, r7 = (lane >> 3) ^ ((lane >> 2 & 1) * 5), row0 = (warp - kGemmThreads / 32) * 8 * kGroups + r7;
+    const int col = lane & 3, r7 = (lane >> 3) ^ ((lane >> 2 & 1) * 5), row0 = (warp - kFirstConverter) * 8 * kGroups + r7;
     const uint32_t src0 = smem_u32(smem) + 3 * stage_bytes + row0 * 128, ch0 = ((2 * col) ^ r7) * 16, ch1 = ((2 * col + 1) ^ r7) * 16;
     const int row_vecs = g.head_dim / 8;
     int s = 0, half = 0;
@@ -707,7 +716,9 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       cluster_sync_all();
       cluster_sync_all();
     }
-  } else {
+    }
+  };
+  auto epilogue_role = [&]() {
     // ------------------------------------------------------------ epilogue (4 warps, thread = tile row)
     const int quad = warp & 3;                  // TMEM lane quarter this warp may access
     const int r = quad * 32 + lane;
@@ -813,6 +824,35 @@ est_gemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         est_epilogue_row<RBS>(g, taddr, n_chunks, clo, chi, true, partial + tile_at * kGroups + r, mtile + tile_at + r, release);
       }
     }
+  };
+
+  if constexpr (own_registers(kDirect, kF32)) {
+    constexpr int kRegEpilogue = 192, kRegLoadMma = 64;
+    static_assert(4 * kRegEpilogue + 4 * kRegLoadMma + 8 * 128 <= 16 * 128, "register budget of the roles");
+    if (warp < 4) {
+      reg_set_from<kRegLoadMma, 128>();
+      if (warp == 0) {
+        load_role();
+      } else if (warp == 1) {
+        mma_role();
+      } else if (split > 1) {
+        cluster_sync_all();
+        cluster_sync_all();
+      }
+    } else if (warp < 8) {
+      reg_set_from<kRegEpilogue, 128>();
+      epilogue_role();
+    } else {
+      convert_role();
+    }
+  } else if (warp == 0) {
+    load_role();
+  } else if (warp == 1) {
+    mma_role();
+  } else if (kF32 && warp >= kFirstConverter) {
+    convert_role();
+  } else {
+    epilogue_role();
   }
 
   // ---------------------------------------------------------------- teardown

@@ -105,6 +105,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return true;
 }
 
+// Registers per thread of a warpgroup, in a kernel launched with kLaunchRegs each (a multiple of 8; what is added here another warpgroup has
+// to give back).  All four warps execute the same one.
+template <int N, int kLaunchRegs> __device__ __forceinline__ void reg_set_from() {
+  if constexpr (N > kLaunchRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+  if constexpr (N < kLaunchRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 // ------------------------------------------------------------------ programmatic dependent launch
 // A kernel launched with the programmatic-stream-serialization attribute may start once every CTA of the kernel
 // before it in the stream has executed pdl_launch_dependents() or exited; what that kernel wrote is visible only
