@@ -212,6 +212,25 @@ def test_sums_off_a_16_byte_boundary(lq, lk, stride, chunk):
     assert torch.equal(sums.view(want.shape), want) and bool(memory[:1].isnan().all()) and bool(memory[1 + want.numel():].isnan().all())
 
 
+@pytest.mark.parametrize("stride,column,chunk,dtype", [(16, 256, 8192, torch.bfloat16), (16, 512, 16384, torch.bfloat16), (8, 768, 8192, torch.float32),
+                                                       (32, 256, 16384, torch.float16), (4, 512, 4096, torch.bfloat16)])
+def test_a_column_tile_that_shows_a_row_nothing_but_nan(stride, column, chunk, dtype):
+    """The last row sees one column of its last tile, and its scores there are NaN: that key block's sum is NaN, and the others are
+    those of the row without it."""
+    from xattn_b200 import ops
+    L = (column + 1) * stride
+    g = torch.Generator().manual_seed(stride)
+    q, k = (torch.randn(1, 2, L, 128, generator=g).to(dtype) for _ in range(2))
+    want = orc.estimate_block_sums(q.float(), k.float(), 128, stride, 1.0, chunk, True, "torch")
+    k[:, :, column * stride + 1, 7] = float("nan")
+    got = ops.estimate_block_sums(q.to(DEV), k.to(DEV), stride, 128, chunk, 1.0, True).cpu()
+    last = column * stride // 128                        # query and key block of the last row and its column
+    want, got = want[:, :, last], got[:, :, last]
+    assert bool(got[..., last].isnan().all())
+    want = want[..., :last] / (1 - want[..., last:last + 1])
+    assert torch.allclose(got[..., :last], want, rtol=RTOL, atol=ATOL), float((got[..., :last] - want).abs().max())
+
+
 @pytest.mark.parametrize("stride,chunk,lq,lk", [(16, 512, 4096, 4096), (16, 1536, 4608, 9216), (8, 512, 1536, 3072), (4, 1024, 5120, 5120), (32, 2560, 5120, 5120)])
 def test_row_tiles_that_span_chunks(stride, chunk, lq, lk):
     """The chunk band of row tiles of which every query block has a chunk of its own: the columns of it in the dense sums (which

@@ -1221,7 +1221,8 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const float mn = fmaxf(m[r], xm[r]);
-        if (t == warp) l[r] = xl[r];
+        // (a tile whose maximum is -inf shows the row nothing, or nothing but NaN, of which its sum would then make the row's)
+        if (t == warp) l[r] = xm[r] > -INFINITY ? xl[r] : 0.f;
         else if (xm[r] > -INFINITY) l[r] = l[r] * fast_exp2(m[r] - mn) + xl[r] * fast_exp2(xm[r] - mn);
         m[r] = mn;
       }
