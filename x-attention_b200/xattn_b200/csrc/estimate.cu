@@ -1168,7 +1168,7 @@ template <int RBS, int kVec, int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, kVec > 2 ? 24 / kWarps : 32 / kWarps)
 est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix, const float* __restrict__ partial,
                     const float2* __restrict__ mtile, float* __restrict__ sums, int pitch, const EstSelectIf<(kVec > 0)> sel) {
-  extern __shared__ float s_rows[];                      // (kVec > 0) [query block][pitch]
+  extern __shared__ __align__(16) float s_rows[];        // (kVec > 0) [query block][pitch], read and written as vectors of four
   __shared__ float4 s_max[kWarps][kTileM / 4], s_sum[kWarps][kTileM / 4];       // [warp][row] of the warp's tiles; [0]: of the whole row, and 1 / sum
   constexpr int kLines = RBS == 32 ? 4 : 8;              // key blocks that a warp has in flight (a divisor of a tile's)
   constexpr int kShare = RBS / 4, kLeft = kLines > kShare ? kLines / kShare : 1;      // lanes per query block; sums a lane ends up with
