@@ -76,6 +76,18 @@ def test_under_the_next_tiles(hq, hkv, L, stride, chunk, causal, dtype):
     _compare(hq, hkv, L, L, stride, chunk, dtype, causal, 0.93, launches=(mask, fused + 1 + extra))
 
 
+# Few row tiles: their query blocks, or where another kernel selects their key blocks, are divided over CTAs, and row tiles of
+# padding follow; of 1, 5, 8, 16, 17 and 32 query blocks in a tile.  The last: more than sixteen column tiles per row, whose sums are the same ones
+# whether a selection follows (eight warps) or not (sixteen).
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("hq,hkv,q_len,k_len,stride,chunk,causal", [
+    (2, 1, 2048, 30000, 32, 16384, True), (4, 4, 2047, 30000, 16, 16384, True), (3, 1, 1000, 20000, 8, 16384, False), (1, 1, 4200, 40000, 32, 8192, True),
+    (2, 2, 640, 9000, 16, 1024, True), (1, 1, 100, 20000, 16, 4096, True), (2, 1, 2176, 12000, 32, 2048, False), (1, 1, 2048, 30000, 4, 2048, True),
+    (2, 1, 2048, 65536, 16, 16384, True), (2, 1, 100, 62000, 8, 20480, True)])
+def test_row_tiles_in_parts(hq, hkv, q_len, k_len, stride, chunk, causal, dtype):
+    _compare(hq, hkv, q_len, k_len, stride, chunk, dtype, causal)
+
+
 # Calls of at least 32 query blocks per SM: the kernel of the block sums selects on its row tiles.  Bands of 128, 256 and 512 (the
 # prefill) and dense rows of as many (the mask), every stride, ragged lengths.
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])

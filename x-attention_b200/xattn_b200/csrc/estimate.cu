@@ -1147,11 +1147,14 @@ est_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // rows belong to one query block, whose lanes add by halves.  Bound by HBM where the partial sums do not stay in L2 (video diffusion,
 // 119K tokens: 1.33 GB), by latency otherwise.  A warp (or four) per query block read 64 bytes here and there of every key block and
 // loaded the next ones only when the ones before were added up.  us between the GEMM's end and the sums', before and now: 119K tokens
-// at stride 8 (24 heads) 521 and 284, 32768 at stride 8 17.1 and 12.1, 1024 tokens against 70000 16.5 and 7.0, 9973 9.4 and 5.7.
+// at stride 8 (24 heads) 521 and 284, 32768 at stride 8 17.1 and 12.1, 1024 tokens against 70000 16.7 and 7.9, 9973 9.4 and 5.7.
 // kVec > 0: and the selection on the tile's rows of sums, of up to 128 * kVec, from shared memory, a warp per row (select_values; as a
 // kernel of its own that is a launch and a hand-over between two kernels more): with the selection 32768 tokens at stride 16
 // 18.4 and 14.1, 9973 tokens at stride 8 13.6 and 8.1, 2500 tokens the call 24.8 and 21.0.
 // Rows of more than 512 sums go to the selection kernel, whose registers would leave too few warps here.
+// Up to two blocks of the selection's values, and the stream, take 64 registers and up to 44 bytes of local memory per thread; without
+// those (three quarters of the warps) 5000 tokens 24.6 -> 25.9 us, 8192 at stride 4 36.9 -> 39.0, 32768 at stride 8 244 and 243.
+constexpr int kSumGroups = 16;                           // of column tiles: tile t is in group t % 16
 constexpr size_t kSumSmem = 84 * 1024;                   // the tile's sums, for the selection: at most 32 rows of 512 and a few more
 
 template <int N>
@@ -1167,15 +1170,19 @@ __device__ __forceinline__ void store_sums(float* p, const float* a) {
 template <int RBS, int kVec, int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, kVec > 2 ? 24 / kWarps : 32 / kWarps)
 est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix, const float* __restrict__ partial,
-                    const float2* __restrict__ mtile, float* __restrict__ sums, int pitch, const EstSelectIf<(kVec > 0)> sel) {
+                    const float2* __restrict__ mtile, float* __restrict__ sums, int pitch, int split, const EstSelectIf<(kVec > 0)> sel) {
   extern __shared__ __align__(16) float s_rows[];        // (kVec > 0) [query block][pitch], read and written as vectors of four
-  __shared__ float4 s_max[kWarps][kTileM / 4], s_sum[kWarps][kTileM / 4];       // [warp][row] of the warp's tiles; [0]: of the whole row, and 1 / sum
+  __shared__ float4 s_max[kSumGroups][kTileM / 4], s_sum[kSumGroups][kTileM / 4];       // [group][row] of the group's tiles; [0]: of the whole row, and 1 / sum
   constexpr int kLines = RBS == 32 ? 4 : 8;              // key blocks that a warp has in flight (a divisor of a tile's)
   constexpr int kShare = RBS / 4, kLeft = kLines > kShare ? kLines / kShare : 1;      // lanes per query block; sums a lane ends up with
   pdl_launch_dependents();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mt = g.n_mtiles - 1 - blockIdx.y, bh = blockIdx.x;
+  // the longest row tiles first, in 2^split parts, then those of padding alone
+  const int y = blockIdx.y, bh = blockIdx.x, n_real = (g.rows_valid + kTileM - 1) / kTileM;
+  const bool pad = y >= n_real << split;
+  const int mt = pad ? y - (n_real << split) + n_real : n_real - 1 - (y >> split);
+  const int by_parts = pad ? 0 : split, z = y & ((1 << by_parts) - 1);
   const int i0 = mt * kTileM;
   const int nlo = g.tab_n ? g.tab[mt] : tile_lo[mt];
   const int ncnt = g.tab_n ? g.tab[kTabPrefix + mt + 1] - g.tab[kTabPrefix + mt] : tile_prefix[mt + 1] - tile_prefix[mt];
@@ -1208,36 +1215,42 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
       for (int j = 0; j < kLines; ++j) p4[j] = k0 + j < k_end ? ld_written_once(line + j * (kTileM / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
-  // (kVec == 0: few row tiles have their key blocks divided over several CTAs)
-  const int k_first = (warp + kWarps * blockIdx.z) * kLines, k_step = kWarps * kLines * gridDim.z;
+  // The parts of a row tile: of its key blocks, or (kVec > 0) of the query blocks that are selected on, for which each part adds up all.
+  const int k_first = (kVec > 0 ? warp : warp + kWarps * z) * kLines, k_step = (kVec > 0 ? kWarps : kWarps << by_parts) * kLines;
+  const int r_first = (warp << by_parts) + z, r_step = kWarps << by_parts;
   if (k_first < k_end) fetch(k_first);
   {
-    // per warp the rows' maxima and sums over its tiles, then a row per thread over the warps
-    float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, l[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-    for (int t = warp; t < ncnt; t += kWarps) {
-      const float4 a = ld_written(ms + t * (kTileM / 2)), b = ld_written(ms + t * (kTileM / 2) + 1);
-      const float xm[4] = {a.x, a.z, b.x, b.z}, xl[4] = {a.y, a.w, b.y, b.w};
+    // The rows' maxima and sums over the tiles, in as many groups whatever the number of warps (the sums do not depend on what else
+    // is in the call), then a row per thread over the groups.
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float mn = fmaxf(m[r], xm[r]);
-        // (a tile whose maximum is -inf shows the row nothing, or nothing but NaN, of which its sum would then make the row's)
-        if (t == warp) l[r] = xm[r] > -INFINITY ? xl[r] : 0.f;
-        else if (xm[r] > -INFINITY) l[r] = l[r] * fast_exp2(m[r] - mn) + xl[r] * fast_exp2(xm[r] - mn);
-        m[r] = mn;
+    for (int i = 0; i < kSumGroups / kWarps; ++i) {
+      const int group = warp + i * kWarps;
+      float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, l[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+      for (int t = group; t < ncnt; t += kSumGroups) {
+        const float4 a = ld_written(ms + t * (kTileM / 2)), b = ld_written(ms + t * (kTileM / 2) + 1);
+        const float xm[4] = {a.x, a.z, b.x, b.z}, xl[4] = {a.y, a.w, b.y, b.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float mn = fmaxf(m[r], xm[r]);
+          // (a tile whose maximum is -inf shows the row nothing, or nothing but NaN, of which its sum would then make the row's)
+          if (t == group) l[r] = xm[r] > -INFINITY ? xl[r] : 0.f;
+          else if (xm[r] > -INFINITY) l[r] = l[r] * fast_exp2(m[r] - mn) + xl[r] * fast_exp2(xm[r] - mn);
+          m[r] = mn;
+        }
       }
+      s_max[group][lane] = make_float4(m[0], m[1], m[2], m[3]);
+      s_sum[group][lane] = make_float4(l[0], l[1], l[2], l[3]);
     }
-    s_max[warp][lane] = make_float4(m[0], m[1], m[2], m[3]);
-    s_sum[warp][lane] = make_float4(l[0], l[1], l[2], l[3]);
     __syncthreads();
     if (threadIdx.x < kTileM) {
       float* sm = reinterpret_cast<float*>(s_max) + threadIdx.x;
       float* sl = reinterpret_cast<float*>(s_sum) + threadIdx.x;
-      const int parts = ncnt < kWarps ? ncnt : kWarps;
+      const int groups = ncnt < kSumGroups ? ncnt : kSumGroups;
       float rm = -INFINITY, rl = 0.f;
-      for (int w = 0; w < parts; ++w) rm = fmaxf(rm, sm[w * kTileM]);
+      for (int w = 0; w < groups; ++w) rm = fmaxf(rm, sm[w * kTileM]);
       if (rm > -INFINITY)
-        for (int w = 0; w < parts; ++w) rl += sl[w * kTileM] * fast_exp2(sm[w * kTileM] - rm);
+        for (int w = 0; w < groups; ++w) rl += sl[w * kTileM] * fast_exp2(sm[w * kTileM] - rm);
       *sm = rm;
       *sl = rl > 0.f ? 1.f / rl : 0.f;
     }
@@ -1291,9 +1304,8 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
   }
   const int k_sums = k_end > 0 ? (k_end + kLines - 1) / kLines * kLines : 0;     // of which there are sums; the others are zero
   if constexpr (kVec == 0) {
-    if (blockIdx.z != 0) return;
 #pragma unroll 1
-    for (int r = warp; r < kTileM / RBS && i0 / RBS + r < g.qb_total; r += kWarps) {
+    for (int r = r_first; r < kTileM / RBS && i0 / RBS + r < g.qb_total; r += r_step) {
       float* row = sums + (static_cast<size_t>(bh) * g.qb_total + i0 / RBS + r) * n_out;
       const int s = shift(r);
       if (whole && ((n_out | s) & 7) == 0) {
@@ -1307,7 +1319,7 @@ est_blocksum_kernel(const EstGeom g, const int* tile_lo, const int* tile_prefix,
   } else {
     __syncthreads();
 #pragma unroll 1
-    for (int r = warp; r < kTileM / RBS && i0 / RBS + r < g.qb_total; r += kWarps) {
+    for (int r = r_first; r < kTileM / RBS && i0 / RBS + r < g.qb_total; r += r_step) {
       const int w = bh * g.qb_total + i0 / RBS + r, s = shift(r);
       float* row = sums + static_cast<size_t>(w) * n_out;
       uint32_t v[4 * kVec];
@@ -1790,16 +1802,29 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   }
 
   const int gpt = g.tile_n / g.rbs, pitch = g.m_pitch * gpt + 8;        // (rows of sums in different banks)
-  const unsigned sum_ctas = static_cast<unsigned>(batch) * hq * g.n_mtiles;
-  // A row tile's key blocks over as many CTAs as it takes for two per SM (1024 tokens against 70000, 32 row tiles: 16 us by one CTA
-  // each, 7.0 by eight); not where they are selected on, for which all of them have to be in one.
-  unsigned parts = selecting ? 1u : 2u * sm_count() / sum_ctas;
-  parts = parts < 1 ? 1 : (parts > 8 ? 8 : parts);
+  // Few row tiles (of those that hold rows: a short piece of prompt is padded to a chunk) are divided over CTAs.  Where they are selected
+  // on, each part adds up all of the sums, which is little, and selects on some of the query blocks: a long selection by sixteen warps of
+  // one SM is slow.  As long as a part has more than four, and up to a CTA per SM, or two where there would be two rounds of warps.
+  // Otherwise a part has some of the key blocks, up to two CTAs per SM.  us a call, 32 heads, flat scores: one CTA per row tile and
+  // like this: 2048 tokens against 30000 at stride 32 53.9 and 43.6, at stride 8 53.6 and 41.2, 12000 at stride 32 58.9 and 48.6, 2048
+  // against 131072 56.5 and 54.7; 1024 against 70000 100 and 82 (padding counted and not).
+  const int real_tiles = (g.rows_valid + kTileM - 1) / kTileM;
+  const unsigned sum_ctas = static_cast<unsigned>(batch) * hq * real_tiles;
+  const int tile_rows = ((g.rows_valid < kTileM ? g.rows_valid : kTileM) + g.rbs - 1) / g.rbs;      // query blocks of a row tile
+  int split = 0;
+  if (selecting)
+    while (tile_rows > 4 << split && sum_ctas << (split + 1) <= (tile_rows > 16 << split ? 2u : 1u) * sms) ++split;
+  else
+    while (split < 3 && sum_ctas << (split + 1) <= 2u * sms) ++split;
+  // Sixteen warps where that leaves no more than two CTAs per SM, otherwise eight; eight, too, for a few sums in front of the selection
+  // kernel, whose CTAs then find registers free and set up under them (1024 tokens against 131072, 16 key blocks visible: 29.6 and 26.4;
+  // 512 against 300000, 2344 key blocks: 244 and 259).
+  const bool wide = sum_ctas <= 2u * sms && !(select && !selecting && pitch >> split <= 64);
   auto launch_sums = [&](auto kern, int threads, auto what) -> int {
     const size_t smem = selecting ? static_cast<size_t>(kTileM / g.rbs) * pitch * sizeof(float) : 0;
     if (smem > 24 * 1024 && !allow_smem(kern, kSumSmem)) return XATTN_B200_ERR_CUDA;
-    return launch_dependent(kern, dim3(static_cast<unsigned>(batch) * hq, g.n_mtiles, parts), dim3(threads), smem, stream, g, (const int*)tile_lo,
-                            (const int*)tile_prefix, (const float*)partial, (const float2*)mtile, attn_sums, pitch, what);
+    return launch_dependent(kern, dim3(static_cast<unsigned>(batch) * hq, (real_tiles << split) + g.n_mtiles - real_tiles), dim3(threads), smem, stream, g, (const int*)tile_lo,
+                            (const int*)tile_prefix, (const float*)partial, (const float2*)mtile, attn_sums, pitch, split, what);
   };
   // with the selection: the instantiation with just enough registers for a row of sums
   auto launch_vec = [&](auto rbs, auto warps) -> int {
@@ -1810,9 +1835,8 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
     if (cols <= 256) return launch_sums(est_blocksum_kernel<kRbs, 2, kWarps>, 32 * kWarps, sel);
     return launch_sums(est_blocksum_kernel<kRbs, 4, kWarps>, 32 * kWarps, sel);
   };
-  // sixteen warps where that leaves no more than two CTAs per SM, otherwise eight
   auto launch_team = [&](auto rbs) -> int {
-    return sum_ctas <= 2u * sm_count() ? launch_vec(rbs, std::integral_constant<int, 16>()) : launch_vec(rbs, std::integral_constant<int, 8>());
+    return wide ? launch_vec(rbs, std::integral_constant<int, 16>()) : launch_vec(rbs, std::integral_constant<int, 8>());
   };
   switch (g.rbs) {
     case 4: return launch_team(std::integral_constant<int, 4>());
