@@ -182,6 +182,17 @@ def test_tiles_whose_streams_share_a_list(hq, hkv, lq, lk, dtype, out_dtype):
             _close(out[0, h], want)
 
 
+def test_dense_calls_of_more_than_a_tile_per_sm_against_long_keys():
+    """Their tiles go in twos, as those of larger calls do: a sequence alone has the bits that it has in a batch."""
+    from xattn_b200 import ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    hq = 4 * (sms * 3 // 2 // 32)                        # of eight query blocks each: one and a half tiles per SM
+    q, k, v = (x.to(DEV) for x in _qkv(1, 2, hq, hq // 4, 1024, 4096))
+    assert sms < 8 * hq <= 2 * sms and 4 * hq <= sms
+    both = ops.block_sparse_attention(q, k, v, None, None, True)
+    assert torch.equal(ops.block_sparse_attention(q[:1], k[:1], v[:1], None, None, True), both[:1])
+
+
 @pytest.mark.parametrize("count", [2 ** 30, -5, 4])
 def test_counts_beyond_a_row_of_the_lists(count):
     """A count that no list can have is cut to the row of the lists (three blocks here), or to none."""

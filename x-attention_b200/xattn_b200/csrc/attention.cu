@@ -1049,7 +1049,8 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
   // 23.1, 2000 tokens at stride 8 36.7 and 36.0); with more than two units per SM it gains nothing (4096 tokens against 65536 51.9 and
   // 52.2, 32768 tokens 473 and 477).  Dense calls only up to one unit per SM (300 tokens 12.2 and 11.0, 1003 tokens 21.0 and 19.7): beyond
   // that other CTAs get hold of the units left over, and it goes either way (1100 tokens 23.0 and 22.6, 1400 28.3 and 28.9, 1530 31.4 and
-  // 31.9, 2000 45.6 and 45.4).
+  // 31.9, 2000 45.6 and 45.4).  Calls by single tiles gain up to two CTAs per SM, of which the second ones are short (without and with it: 1024
+  // tokens 20.4 and 19.4, of 28 heads 19.4 and 18.7, 1180 of 28 heads 23.1 and 22.3), and these have a unit per SM at most.
   p.early_next = units <= (dense ? 1LL : 2LL) * sm_count() ? 1 : 0;
   p.by_units = make_fast_div(causal ? batch * hq : super_rows * (hq / hkv));
   p.by_hq = make_fast_div(hq);
@@ -1082,12 +1083,19 @@ int block_sparse_attn_launch(const void* q, const void* k, const void* v, int dt
   const bool two = causal && !dense && !rest && max_list > 0 && units >= 24 * sms && units >= max_list * sms &&
                    static_cast<long long>(batch) * hkv * p.list_k_blocks < 0x7fffffffLL;
   const long long tiles = static_cast<long long>(p.q_blocks) * batch * hq;
-  // Causal calls of few tiles give each a CTA of its own, whose streams share its list.  With lists, up to a tile per SM, and of more
-  // than 64 key blocks, where the lists may be long (us, two tiles per CTA and like this: 512 tokens against 30000, 75 blocks per row,
-  // 192 and 114, against 60000, 174 blocks, 372 and 230; against 300, two blocks, 12.1 and 12.1; with more tiles, where CTAs then take
-  // two, the chains of short lists come one after the other: 1024 tokens against 70000, three blocks, 13.0 and 15.5).  Dense ones up to
-  // two per SM (512 tokens 12.9 and 11.9, 1003 tokens 19.8 and 19.1, 1180 tokens of 28 heads 22.3 and 22.1).
-  const bool split = causal && !rest && (dense ? tiles <= 2 * sms : tiles <= sms && p.list_k_blocks > 64);
+  // Causal calls of few tiles give each a CTA of its own, whose streams share its list: up to a tile per SM, dense ones and those with
+  // lists of more than 64 key blocks (us, 32 heads, two tiles per CTA and like this; dense, 512 tokens 12.9 and 12.4, against 4096 58 and 38,
+  // against 65536 857 and 513; lists of half of the blocks, 512 tokens against 8315 86 and 48, against 65531 580 and 281; of five blocks 24.1
+  // and 17.8, 28.0 and 21.9; of two 11.9 in either form.  Shorter rows gain, too: against 2555, 20 blocks, 33.8 and 22.4).
+  // With more tiles an SM takes two of them one after the other, which is as many blocks as two at a time, and loads K and V for each: lists
+  // go by units of two (1024 tokens against 70000, three blocks, 13.0 and 15.5), and dense calls (1024 against 4096 66 and 71, against 65536
+  // 976 and 1184; 900 against 32768 492 and 578), but for two kinds: keys little longer than the queries, where the tiles are of so
+  // different lengths that the longest first even the call out (1024 tokens 20.2 and 19.4, 3000 of 12 heads 47.8 and 41.5, against 3750 60.9 and
+  // 55.3, 1150 of 28 heads 21.6 and 20.9, 500 of 28 heads in a batch of two 13.3 and 13.2, but against 625 15.6 and 16.3), and more units
+  // than SMs, as odd numbers of query blocks make them: the units left over are fetched ahead by CTAs that have one (1150 tokens against
+  // 32768 851 and 533, six sequences of 100 against 8192 211 and 150, of which five, 160 tiles, are done in one round, 111 and 150).
+  const bool even = 4LL * p.k_len <= 5LL * p.q_len || (units > sms && 4 * tiles > 5 * sms);
+  const bool split = causal && !rest && (dense ? tiles <= sms || (tiles <= 2 * sms && even) : tiles <= sms && p.list_k_blocks > 64);
   const unsigned grid = static_cast<unsigned>(rest && units > sms ? sms : (two ? (units + 1) / 2 : (split ? tiles : units)));
   auto launch = [&](auto kern) -> int {
     if (!allow_smem(kern, kAttnSmem))
