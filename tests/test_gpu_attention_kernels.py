@@ -158,8 +158,8 @@ def test_which_non_causal_calls_are_ordered(blocks, items_per_sm, ordered):
 @pytest.mark.parametrize("dtype,out_dtype", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16), (torch.float32, torch.float32)])
 @pytest.mark.parametrize("hq,hkv,lq,lk", [(2, 1, 70 * 128, 70 * 128), (7, 7, 300, 8400), (4, 2, 1, 9000), (1, 1, 127, 128 * 70 + 1), (74, 37, 256, 8193)])
 def test_tiles_whose_streams_share_a_list(hq, hkv, lq, lk, dtype, out_dtype):
-    """Few tiles: of none, one, an odd and an even number of blocks, of more than a window of a list; several tiles per CTA with
-    the lists of the first ones the longest (dense), rows whose blocks are hidden from one stream altogether."""
+    """Up to a tile per SM: of none, one, an odd and an even number of blocks, of more than a window of a list; rows whose blocks are
+    hidden from one stream altogether."""
     from xattn_b200 import ops
     q, k, v = _qkv(lq + hq, 1, hq, hkv, lq, lk, dtype)
     qb, kb = (lq + 127) // 128, (lk + 127) // 128
@@ -180,6 +180,40 @@ def test_tiles_whose_streams_share_a_list(hq, hkv, lq, lk, dtype, out_dtype):
             s = (qf[0, h] @ kf[0, h].T * 128 ** -0.5).masked_fill(~keep, float("-inf"))
             want = torch.where(keep.any(1, keepdim=True), torch.softmax(s, -1).nan_to_num(0.0) @ vf[0, h], torch.zeros(()))
             _close(out[0, h], want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("batch,hq,hkv,ragged", [(1, 28, 4, 100), (1, 2, 1, 3), (2, 12, 4, 127), (1, 7, 7, 0)])
+def test_second_tiles_of_a_cta(batch, hq, hkv, ragged, dtype):
+    """Dense prompts of one to two tiles per SM: a CTA takes a second tile, shorter than its first or of a single block, behind which a
+    stream has none."""
+    from xattn_b200 import ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    nb = 19 * sms // (10 * batch * hq)
+    L = nb * 128 - ragged
+    assert sms < nb * batch * hq <= 2 * sms
+    q, k, v = (x.to(DEV) for x in _qkv(L, batch, hq, hkv, L, L, dtype))
+    out = ops.block_sparse_attention(q, k, v, None, None, True)
+    assert out.dtype == dtype
+    qf, kf, vf = (x.to(torch.bfloat16).float() if dtype == torch.float32 else x.float() for x in (q, k, v))
+    visible = torch.ones(L, L, dtype=torch.bool, device=DEV).tril()
+    for b, h in {(0, 0), (batch - 1, hq - 1), (0, hq // 2)}:
+        s = (qf[b, h] @ kf[b, h * hkv // hq].T * 128 ** -0.5).masked_fill(~visible, float("-inf"))
+        _close(out[b, h], (torch.softmax(s, -1) @ vf[b, h * hkv // hq]).cpu())
+
+
+def test_lists_of_a_batch_shared_by_the_streams():
+    """Up to a tile per SM and more than 64 key blocks: a sequence alone has the bits that it has in a batch of two."""
+    from xattn_b200 import ops
+    q, k, v = (x.to(DEV) for x in _qkv(4, 2, 4, 2, 300, 8400))
+    mask = torch.rand(2, 4, 3, 66, generator=torch.Generator().manual_seed(1)) < 0.3
+    idx, cnt = ops.mask_to_lists(mask.to(DEV), 300, 8400, True)
+    both = ops.block_sparse_attention(q, k, v, idx, cnt, True)
+    for b in range(2):
+        s = slice(b, b + 1)
+        assert torch.equal(ops.block_sparse_attention(q[s], k[s], v[s], idx[s], cnt[s], True), both[s])
+    want = orc.block_sparse_attention_oracle(q.cpu(), k.cpu(), v.cpu(), mask, True)
+    _close(both, want)
 
 
 def test_dense_calls_of_more_than_a_tile_per_sm_against_long_keys():

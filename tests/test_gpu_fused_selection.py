@@ -88,24 +88,25 @@ def test_row_tiles_in_parts(hq, hkv, q_len, k_len, stride, chunk, causal, dtype)
     _compare(hq, hkv, q_len, k_len, stride, chunk, dtype, causal)
 
 
-# Calls of at least 32 query blocks per SM: the kernel of the block sums selects on its row tiles.  Bands of 128, 256 and 512 (the
-# prefill) and dense rows of as many (the mask), every stride, ragged lengths.
+# The kernel of the block sums selects on its row tiles: sixteen warps up to two row tiles per SM (the first three), eight beyond.  Bands
+# of 128, 256 and 512 (the prefill) and dense rows of as many (the mask), every stride, ragged lengths.
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("hq,hkv,L,stride,chunk,causal", [
-    (32, 8, 32768, 8, 16384, True), (32, 8, 40955, 16, 2048, True), (40, 8, 15400, 16, 4096, True), (40, 40, 16384, 4, 16384, True), (20, 4, 32768, 32, 32768, True),
-    (20, 20, 32760, 16, 8192, True), (20, 5, 31000, 16, 32768, True), (10, 5, 62000, 16, 4096, True), (10, 2, 65536, 8, 65536, True),
-    (40, 8, 15400, 16, 2048, False), (10, 10, 61000, 8, 2048, False)])
-def test_a_warp_per_query_block(hq, hkv, L, stride, chunk, causal, dtype):
+@pytest.mark.parametrize("hq,hkv,L,stride,chunk,causal,few", [
+    (4, 2, 16384, 8, 16384, True, True), (4, 2, 32768, 16, 32768, True, True), (2, 1, 65536, 16, 65536, True, True),
+    (32, 8, 32768, 8, 16384, True, False), (32, 8, 40955, 16, 2048, True, False), (40, 8, 15400, 16, 4096, True, False),
+    (40, 40, 16384, 4, 16384, True, False), (20, 4, 32768, 32, 32768, True, True), (20, 20, 32760, 16, 8192, True, False),
+    (20, 5, 31000, 16, 32768, True, False), (10, 5, 62000, 16, 4096, True, False), (10, 2, 65536, 8, 65536, True, False),
+    (40, 8, 15400, 16, 2048, False, False), (10, 10, 61000, 8, 2048, False, False)])
+def test_row_tiles_selected_on_behind_the_gemm(hq, hkv, L, stride, chunk, causal, few, dtype):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    blocks = hq * (-(-L // chunk) * chunk // 128)
-    if blocks < 32 * sms:
-        pytest.skip("needs 32 query blocks per SM")
+    if (hq * -(-L // (128 * stride)) <= 2 * sms) != few:
+        pytest.skip("meant for another number of SMs")
     gemm = 1 if -(-L // chunk) * chunk // stride <= 64 * 128 else 2     # (long calls: the tile tables are a kernel of their own)
     for sink, recent in ((False, False), (True, True)):
         extra = 0 if causal else 1                     # (the ordered list of units of a non-causal attention)
         _compare(hq, hkv, L, L, stride, chunk, dtype, causal, 0.93, sink, recent, launches=(gemm + 1, gemm + 2 + extra))
 
 
-def test_a_warp_per_query_block_in_fp32():
+def test_row_tiles_selected_on_behind_the_fp32_gemm():
     """fp32 inputs take the same kernel of the block sums behind a GEMM of their own."""
     _compare(40, 8, 15400, 15400, 16, 4096, torch.float32)

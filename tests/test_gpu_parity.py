@@ -657,6 +657,22 @@ def test_query_chunk_shards_equal_the_full_call():
             _assert_same_up_to_body_choice(o, full[:, :, c * 4096:(c + 1) * 4096], msg=str(("rows 4096", r, c)))
 
 
+def test_a_piece_against_many_key_blocks_equals_the_full_call():
+    """A piece against more than 64 key blocks, and a head shard of it, have few enough tiles for each to be shared by the two
+    streams of a CTA; the full call has its tiles in twos."""
+    import xattn_b200
+    from xattn_b200 import synth
+    from xattn_b200.sharding import prefill_sharded
+    q, k, v, w = synth.make_inputs("llama3_8b_128k", seed=10, heads_limit=4, seq_len=12288)
+    dq, dk, dv = q.to(DEV), k.to(DEV), v.to(DEV)
+    full = xattn_b200.Xattention_prefill(dq, dk, dv, 16, threshold=0.9, chunk_size=2048)
+    piece = xattn_b200.Xattention_prefill(dq[:, :, 10240:], dk, dv, 16, threshold=0.9, chunk_size=2048)
+    _assert_same_up_to_body_choice(piece, full[:, :, 10240:])
+    parts = [prefill_sharded(dq[:, :, 10240:], dk, dv, xattn_b200.Xattention_prefill, 4, r, threshold=0.9, stride=16, chunk_size=2048) for r in range(4)]
+    assert parts[0].shape[1] * 16 <= torch.cuda.get_device_properties(0).multi_processor_count < piece.shape[1] * 16
+    _assert_same_up_to_body_choice(torch.cat(parts, dim=1), full[:, :, 10240:])
+
+
 def test_prefill_against_a_longer_key_cache():
     """q shorter than k (chunked prefill against a cache): masks vs the oracle, outputs vs the oracle's
     attention under the GPU mask, queries aligned to the end of the keys."""
