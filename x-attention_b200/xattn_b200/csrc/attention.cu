@@ -193,7 +193,7 @@ block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     return;
   }
   uint8_t* stage_base = smem + kAttnSmemTiles;
-  float* s_l = reinterpret_cast<float*>(stage_base + kStageBytes);                 // [stream][2][128] final row sums
+  float* s_l = reinterpret_cast<float*>(stage_base + kStageBytes);                 // [stream][2][128] final row sums of two tiles (split: of one, and the maxima they are against)
   volatile int* ring = reinterpret_cast<volatile int*>(s_l + 2 * 2 * 128);         // [step]
   UnitTile* unit_ring = reinterpret_cast<UnitTile*>(s_l + 2 * 2 * 128 + kRingEntries);         // [slot][stream]
   uint8_t* answer = reinterpret_cast<uint8_t*>(unit_ring + 2 * kUnitSlots);                    // of the request for a unit

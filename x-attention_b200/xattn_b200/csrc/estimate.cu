@@ -42,7 +42,8 @@ constexpr int kF32Cols = 32;
 constexpr int kF32Unit = kTileM * kF32Cols * 4;              // 16 KiB
 constexpr int kF32Smem = 224 * 1024;                         // terms and ring: 3 x 32 KiB and 8 units, or 3 x 48 KiB and 5
 constexpr int kMaxUnits = 8;
-// Warps that split the units, every warp some rows of each: sixteen, or eight where the epilogue needs the registers.
+// Warps that split the units, every warp some rows of each: sixteen of up to 88 registers, or, where the epilogue has registers of its own,
+// eight of 128, with which the sixteen warps of the CTA make up the register file.
 __host__ __device__ constexpr int convert_warps(int direct) { return direct ? 8 : 16; }
 // Where the epilogue needs the registers it is a warpgroup of its own (warps 4-7), which takes over what the loading and issuing warps
 // (0-3) do not need; the converters follow.  (With 128 registers for all it stored 832 to 2750 bytes per thread to local memory, which is
@@ -93,7 +94,7 @@ struct EstGeom {
   int bpc;                     // key blocks per chunk
   // Scratch layout: tile by tile, m_pitch tiles per row tile; a tile holds tile_n / rbs partial block sums and one (max, sum)
   // pair of each of its 128 rows, the rows of a block sum next to one another (the epilogue's lanes are rows, and
-  // est_blocksum_kernel reads the rows of a query block).  Dense: every column tile.  Compact (left_blank: a row only ever
+  // est_blocksum_kernel reads a block sum's 128 rows as one line).  Dense: every column tile.  Compact (left_blank: a row only ever
   // touches the tiles of its own chunk): the column tiles [tile_lo, tile_lo + m_pitch) of the row tile.
   int compact, m_pitch;
   // Lengths that are no multiple of the stride: the last stride group lacks the tokens of offset >= len % stride, which
@@ -477,7 +478,7 @@ __device__ __forceinline__ uint4 next_term(unsigned long long (&v)[4]) {
 // them back (32 heads of 4096 tokens, chunks of 2048: split 56 us + GEMM 46 -> 44; the prefill, whose attention phase takes the
 // bf16 roundings written here, 151 -> 114 us, 2 us of them for the proxy fence of every unit).  Bound by the latency of a
 // converter's step (waits, shared-memory traffic next to the MMAs', three dependent roundings); with loads alone it runs in 30
-// us.  Sixteen converter warps, or eight where the epilogue of a single tile needs the registers.
+// us.  Sixteen converter warps, or eight beside an epilogue with registers of its own (own_registers).
 // kSelect: and selects on its rows (can_select)
 template <int RBS, int kDirect, bool kF32, bool kSelect>
 __global__ void __launch_bounds__(kF32 ? f32_threads(kDirect) : kGemmThreads, 1)
