@@ -344,10 +344,12 @@ Tensor attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Ten
         "block_sparse_attn");
   return out;
 }
-// Non-causal calls: sorting the units by list length is one launch of 5 to 15 us.  What it saves is the chain of a long list that would be
+// Non-causal calls: sorting the units by list length is one launch of 4 to 15 us.  What it saves is the chain of a long list that would be
 // begun near the end, 1.5 us per block: worth it with many items per SM, or with a few whose lists may be long (24 heads, video
-// diffusion, us without and with it: 7400 tokens, 58 key blocks, 9 items per SM, 257 and 205; 11000 tokens, 14 items, 449 and 373; 12
-// heads of 7400, 5 items, 189 and 170; but 3800 tokens, 30 key blocks, 5 or 10 items, 138 and 142, 177 and 183).
+// diffusion, us without and with it: 7456 tokens, 58 key blocks, 9 items per SM, 250 and 199; 11056 tokens, 14 items, 430 and 349; 12
+// heads of 7400, 5 items, 189 and 170; but 3800 tokens, 30 key blocks, 5 or 10 items, 138 and 142, 177 and 183).  Lists that are all
+// alike, whose lengths the host does not know, gain nothing (lists of two blocks or so, the whole prefill: 5500 tokens 62 and 67, 7400 93 and
+// 100, 11000 163 and 169, 12 heads of 7400 51.5 and 56; the attention alone, two full rows of lists among those of five blocks, 200 and 128).
 constexpr int64_t kOrderItemsPerSm = 16, kOrderFewItemsPerSm = 4, kOrderKeys = 40 * 128;
 bool default_workspace(bool causal, bool dense, const Tensor& q, int64_t k_len) {
   if (dense) return false;
