@@ -1805,16 +1805,18 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   const int gpt = g.tile_n / g.rbs, pitch = g.m_pitch * gpt + 8;        // (rows of sums in different banks)
   // Few row tiles (of those that hold rows: a short piece of prompt is padded to a chunk) are divided over CTAs.  Where they are selected
   // on, each part adds up all of the sums, which is little, and selects on some of the query blocks: a long selection by sixteen warps of
-  // one SM is slow.  As long as a part has more than four, and up to a CTA per SM, or two where there would be two rounds of warps.
-  // Otherwise a part has some of the key blocks, up to two CTAs per SM.  us a call, 32 heads, flat scores: one CTA per row tile and
-  // like this: 2048 tokens against 30000 at stride 32 53.9 and 43.6, at stride 8 53.6 and 41.2, 12000 at stride 32 58.9 and 48.6, 2048
-  // against 131072 56.5 and 54.7; 1024 against 70000 100 and 82 (padding counted and not).
+  // one SM is slow.  As long as a part has more than four (rows of up to 128 sums: eight, which are done soon, and the attention
+  // kernel sets up on the SMs left: 2048 tokens of 28 heads at stride 8 35.7 us with four, 35.1), and up to a CTA per SM, or two where there
+  // would be two rounds of warps.  Otherwise a part has some of the key blocks, up to two CTAs per SM.  us a call, 32 heads, flat scores, one CTA
+  // per row tile and like this: 2048 tokens against 30000 at stride 32 53.9 and 43.4, at stride 8 53.6 and 41.2, 12000 at stride 32 58.4 and 49.0, 2048
+  // against 131072 56.7 and 54.6; 1024 against 70000 100 and 82 (padding counted and not).
   const int real_tiles = (g.rows_valid + kTileM - 1) / kTileM;
   const unsigned sum_ctas = static_cast<unsigned>(batch) * hq * real_tiles;
   const int tile_rows = ((g.rows_valid < kTileM ? g.rows_valid : kTileM) + g.rbs - 1) / g.rbs;      // query blocks of a row tile
+  const int cols = g.band ? g.bpc : g.kb_total;
   int split = 0;
   if (selecting)
-    while (tile_rows > 4 << split && sum_ctas << (split + 1) <= (tile_rows > 16 << split ? 2u : 1u) * sms) ++split;
+    while (tile_rows > (cols > 128 ? 4 : 8) << split && sum_ctas << (split + 1) <= (tile_rows > 16 << split ? 2u : 1u) * sms) ++split;
   else
     while (split < 3 && sum_ctas << (split + 1) <= 2u * sms) ++split;
   // Sixteen warps where that leaves no more than two CTAs per SM, otherwise eight; eight, too, for a few sums in front of the selection
@@ -1830,7 +1832,6 @@ int estimate_launch(const void* q, const void* k, int dtype, int batch, int hq, 
   // with the selection: the instantiation with just enough registers for a row of sums
   auto launch_vec = [&](auto rbs, auto warps) -> int {
     constexpr int kRbs = decltype(rbs)::value, kWarps = decltype(warps)::value;
-    const int cols = g.band ? g.bpc : g.kb_total;
     if (!selecting) return launch_sums(est_blocksum_kernel<kRbs, 0, kWarps>, 32 * kWarps, EstNothing());
     if (cols <= 128) return launch_sums(est_blocksum_kernel<kRbs, 1, kWarps>, 32 * kWarps, sel);
     if (cols <= 256) return launch_sums(est_blocksum_kernel<kRbs, 2, kWarps>, 32 * kWarps, sel);
